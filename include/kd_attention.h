@@ -69,6 +69,9 @@ typedef struct kd_meta {
   int32_t causal;     /* used only when rules == 0 (original_kernel.py:512-515) */
   int32_t rules;      /* 1 when any of attention_mask/in_span/span_id/is_prefix was given
                          (the negation of FAST_PATH_NO_RULES, original_kernel.py:422) */
+  uint32_t* status_mirror; /* NULL, or a word of host memory the device can write (pinned, unified addressing):
+                         whatever a kernel puts into the plan's status word it also puts here, so that the
+                         host sees a failure without a copy or a synchronisation */
 } kd_meta;
 
 /* Byte offsets of the pieces of a plan inside the caller's plan buffer. */
@@ -87,7 +90,7 @@ typedef struct kd_plan_layout {
   size_t off_order;      /* uint8  [B][3][NT]    tiles sorted by decreasing work: [0] forward q tile
                                                  pairs, [1] dQ q tiles, [2] dK/dV k tiles */
   size_t off_stats;      /* uint32 [B][2]        number of FULL and of PARTIAL tiles */
-  size_t off_status;     /* uint32               device status word (0 = ok) */
+  size_t off_status;     /* uint32               device status word (0 = ok); at +8 the address of its host mirror */
   size_t total;          /* bytes the caller must provide (256-byte aligned base) */
 } kd_plan_layout;
 

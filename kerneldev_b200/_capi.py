@@ -33,7 +33,7 @@ class KdMeta(Structure):
         ("B", c_int32), ("T", c_int32),
         ("in_span", c_void_p), ("span_id", c_void_p), ("is_prefix", c_void_p), ("lens", c_void_p),
         ("in_span_stride_b", c_int64), ("span_id_stride_b", c_int64), ("is_prefix_stride_b", c_int64),
-        ("causal", c_int32), ("rules", c_int32),
+        ("causal", c_int32), ("rules", c_int32), ("status_mirror", c_void_p),
     ]
 
 

@@ -16,6 +16,8 @@ PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "_lib"
 LIB_PATH = LIB_DIR / "libkd_attention.so"
+HOST_PATH = LIB_DIR / "kd_host.so"      # the host extension: links against libtorch, gets the library's addresses at run time
+HOST_SOURCE = CSRC / "host.cpp"
 INCLUDE_DIR = PKG_DIR.parent / "include"
 
 SOURCES = ["capi.cu", "plan.cu", "attn_fwd.cu", "attn_bwd.cu", "attn_bwd_fused.cu", "hadamard.cu", "metadata.cu", "cocktail.cu"]
@@ -44,6 +46,29 @@ def _stale() -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
+def build_host(force: bool = False) -> Path:
+    """Compiles the host extension (csrc/host.cpp) against the installed torch."""
+    deps = [HOST_SOURCE, INCLUDE_DIR / "kd_attention.h"]
+    if not force and HOST_PATH.exists() and all(d.stat().st_mtime <= HOST_PATH.stat().st_mtime for d in deps):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    torch_dir = Path(torch.__file__).resolve().parent
+    cuda_home = Path(_nvcc()).resolve().parent.parent
+    inc = [torch_dir / "include", torch_dir / "include" / "torch" / "csrc" / "api" / "include", cuda_home / "include",
+           sysconfig.get_paths()["include"]]
+    LIB_DIR.mkdir(exist_ok=True)
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=kd_host",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *[f"-I{p}" for p in inc], str(HOST_SOURCE), "-o", str(HOST_PATH), f"-L{torch_dir / 'lib'}",
+           "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{torch_dir / 'lib'}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host.cpp:\n{r.stdout}\n{r.stderr}")
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False, extra_flags=(), name=None) -> Path:
     """Compiles every CUDA source for sm_100a and links the shared library. Returns its path.
 
@@ -56,8 +81,10 @@ def build(force: bool = False, verbose: bool = False, extra_flags=(), name=None)
         deps = [CSRC / s for s in SOURCES + HEADERS] + [INCLUDE_DIR / "kd_attention.h"]
         if not force and lib_path.exists() and all(d.stat().st_mtime <= lib_path.stat().st_mtime for d in deps):
             return lib_path
-    elif not force and not _stale():
-        return LIB_PATH
+    else:
+        build_host(force)
+        if not force and not _stale():
+            return LIB_PATH
     LIB_DIR.mkdir(exist_ok=True)
     obj_dir = LIB_DIR / (f"obj_{name}" if name else "obj")
     obj_dir.mkdir(exist_ok=True)

@@ -924,8 +924,9 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
  
   auto kq = attn_bwd_dq_kernel<HD, kBf16>;
   auto kk = attn_bwd_dkdv_kernel<HD, kBf16>;
-  cudaError_t e = cudaFuncSetAttribute(kq, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_ALLOC);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kk, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_ALLOC);
+  static SmemOptIn opt_in_q, opt_in_k;
+  cudaError_t e = opt_in_q(kq, C::SMEM_ALLOC);
+  if (e == cudaSuccess) e = opt_in_k(kk, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "bwd smem attribute: %s", cudaGetErrorString(e));
   dim3 grid((p.H + a.G - 1) / a.G, p.B, L.NT);
   const int phases = (p.bwd_phases & 3) ? (p.bwd_phases & 3) : 3;

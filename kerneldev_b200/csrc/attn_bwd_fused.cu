@@ -651,7 +651,8 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   int rc = encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, C::HD, KD_TILE, "dq_acc");
   if (rc != 0) return rc;
   auto kern = attn_bwd_fused_kernel<kBf16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_ALLOC);
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd smem attribute: %s", cudaGetErrorString(e));
   // The warps re-divide the registers the CTA was launched with; a request beyond that pool would block for ever,
   // so a build whose per-thread count is below the one the division assumes is refused here.

@@ -2,6 +2,8 @@
 // descriptors (so the single MMA-issuing thread spends two integer adds per MMA, not a 64-bit
 // descriptor build), work-list staging, 16-bit row stores.
 #pragma once
+#include <atomic>
+
 #include "common.cuh"
 #include "mask_rule.cuh"
 #include "sm100_prims.cuh"
@@ -180,6 +182,23 @@ inline int heads_per_cta(int B, int H, int items_per_batch, int forced, int per_
   if (g > H) g = H;
   return static_cast<int>(g);
 }
+
+// Raises a kernel's dynamic shared-memory limit, once per device (one instance per kernel): the attribute call
+// costs about a microsecond of host time, which a small launch would pay every time.
+struct SmemOptIn {
+  std::atomic<uint64_t> done{0};   // bit d: set on device d
+  template <typename Kernel>
+  cudaError_t operator()(Kernel kern, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? uint64_t(1) << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+};
 
 // bounded wait used while unwinding after an abort: lets a TMA copy that is already in flight land
 __device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {

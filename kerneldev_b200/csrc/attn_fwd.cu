@@ -661,7 +661,8 @@ static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   a.test_drop_load = (drop != nullptr && atoi(drop) != 0) ? 1 : 0;
 #endif
   auto kern = attn_fwd_kernel<HD, kBf16>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_ALLOC);
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
   dim3 grid((p.H + a.G - 1) / a.G, p.B, L.NP);
   kern<<<grid, C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, a);

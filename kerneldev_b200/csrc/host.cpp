@@ -1,0 +1,548 @@
+// Host path of the operator as a torch extension: argument checks, the plan cache, allocations, the autograd
+// node and the calls into libkd_attention.so, without a Python frame between flash_attention() and the launches.
+//
+// A forward or backward of a small problem is a few microseconds of kernels; the same path written in Python
+// (ctypes structures, an autograd.Function whose backward takes the interpreter lock on the engine's thread) cost
+// 65 us per forward and 185 us per backward whatever the size. The C ABI stays the boundary to the kernels: this
+// file holds no device code and gets the library's entry points as addresses (bind), so that a test can bind
+// another build of the library.
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include <list>
+#include <mutex>
+#include <unordered_map>
+
+#include "../../include/kd_attention.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+// ---- the library -----------------------------------------------------------------------------------------------
+
+struct Library {
+  decltype(&kd_plan_layout_get) plan_layout_get = nullptr;
+  decltype(&kd_classify) classify = nullptr;
+  decltype(&kd_attn_fwd) attn_fwd = nullptr;
+  decltype(&kd_attn_bwd) attn_bwd = nullptr;
+  decltype(&kd_hadamard) hadamard = nullptr;
+  decltype(&kd_metadata_from_tokens) metadata_from_tokens = nullptr;
+  decltype(&kd_last_error) last_error = nullptr;
+};
+Library lib;
+
+template <typename F>
+void take(F& slot, const py::dict& addresses, const char* name) {
+  slot = reinterpret_cast<F>(addresses[name].cast<uintptr_t>());
+}
+
+void bind(const py::dict& a) {
+  take(lib.plan_layout_get, a, "kd_plan_layout_get");
+  take(lib.classify, a, "kd_classify");
+  take(lib.attn_fwd, a, "kd_attn_fwd");
+  take(lib.attn_bwd, a, "kd_attn_bwd");
+  take(lib.hadamard, a, "kd_hadamard");
+  take(lib.metadata_from_tokens, a, "kd_metadata_from_tokens");
+  take(lib.last_error, a, "kd_last_error");
+}
+
+// an entry point rejected its arguments or a CUDA call failed (raised in Python as _capi.KdError)
+struct LibraryError : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
+
+void check(int rc) {
+  if (rc != 0) throw LibraryError("libkd_attention: error " + std::to_string(rc) + ": " + lib.last_error());
+}
+
+#define KD_VALUE(cond, ...) TORCH_CHECK_VALUE(cond, __VA_ARGS__)
+
+// ---- plans -----------------------------------------------------------------------------------------------------
+
+constexpr uint32_t kStatusTimeout = KD_STATUS_TIMEOUT, kStatusSpanRange = KD_STATUS_SPAN_RANGE;
+
+// Status mirrors of the plans: one pinned block handed out in rotation (pinning is a slow, device-wide call).
+// 1024 words: a collision would need more than 1024 live plans and could only make a reported failure show up on
+// two of them.
+Tensor pinned_word() {
+  static std::mutex m;
+  static Tensor block;
+  static int next = 0;
+  std::lock_guard<std::mutex> lock(m);
+  if (!block.defined()) block = at::zeros({1024}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+  Tensor w = block.narrow(0, next, 1);
+  next = (next + 1) % 1024;
+  *w.data_ptr<int32_t>() = 0;
+  return w;
+}
+
+bool check_every_launch() {
+  const char* e = std::getenv("KD_CHECK_STATUS");
+  return e != nullptr && e[0] == '1' && e[1] == 0;
+}
+
+struct Plan {
+  int64_t B, T;
+  at::Device device;
+  kd_plan_layout layout;
+  Tensor buf, status_dev, status_host;
+  volatile uint32_t* host_word;
+  std::vector<Tensor> keep;   // the caller's metadata and its converted copies, alive as long as the plan is cached
+  at::cuda::CUDAStream built_on;
+  at::cuda::CUDAEvent built;
+
+  Plan(int64_t B_, int64_t T_, at::Device dev, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix,
+       const OptTensor& lens, bool causal, bool rules)
+      : B(B_), T(T_), device(dev), built_on(at::cuda::getCurrentCUDAStream(dev.index())) {
+    check(lib.plan_layout_get(static_cast<int32_t>(B), static_cast<int32_t>(T), &layout));
+    // the caching allocator returns 512-byte aligned blocks, which covers the 256 the ABI asks for
+    buf = at::empty({static_cast<int64_t>(layout.total)}, at::TensorOptions().dtype(at::kByte).device(dev));
+    kd_meta meta{};
+    meta.B = layout.B;
+    meta.T = layout.T;
+    meta.in_span = static_cast<const uint8_t*>(per_token(in_span, at::kBool, "in_span", &meta.in_span_stride_b));
+    meta.span_id = static_cast<const int64_t*>(per_token(span_id, at::kLong, "span_id", &meta.span_id_stride_b));
+    meta.is_prefix = static_cast<const uint8_t*>(per_token(is_prefix, at::kBool, "is_prefix", &meta.is_prefix_stride_b));
+    if (lens.has_value()) {
+      KD_VALUE(lens->scalar_type() == at::kInt && lens->dim() == 1 && lens->size(0) == B, "lens must be an int32 tensor of shape (B,)");
+      keep.push_back(*lens);
+      Tensor l = lens->contiguous();
+      keep.push_back(l);
+      meta.lens = l.data_ptr<int32_t>();
+    }
+    meta.causal = causal;
+    meta.rules = rules;
+    const int64_t off = static_cast<int64_t>(layout.off_status);
+    status_dev = buf.narrow(0, off, 4).view(at::kInt);
+    status_host = pinned_word();
+    host_word = reinterpret_cast<volatile uint32_t*>(status_host.data_ptr<int32_t>());
+    meta.status_mirror = const_cast<uint32_t*>(host_word);
+    c10::cuda::CUDAGuard guard(dev);
+    check(lib.classify(&meta, buf.data_ptr(), built_on.stream()));
+    built.record(built_on);
+    if (check_every_launch()) check_status();
+  }
+
+  const void* per_token(const OptTensor& o, at::ScalarType dtype, const char* name, int64_t* stride_b) {
+    if (!o.has_value()) return nullptr;
+    Tensor t = *o;
+    KD_VALUE(t.dim() == 2 && t.size(0) == B && t.size(1) == T, name, " must have shape (B, T) = (", B, ", ", T, "), got ", t.sizes());
+    KD_VALUE(t.device() == device, name, " must live on ", device);
+    keep.push_back(t);
+    if (dtype == at::kBool) KD_VALUE(t.scalar_type() == at::kBool, name, " must be a torch.bool tensor (the rule negates it logically)");
+    if (t.scalar_type() != dtype) t = t.to(dtype);
+    if (t.stride(1) != 1) t = t.contiguous();
+    keep.push_back(t);
+    *stride_b = t.stride(0);
+    return t.data_ptr();
+  }
+
+  // Orders the current stream after the classifier when the plan was built on another one.
+  void use_on_current_stream() {
+    auto cur = at::cuda::getCurrentCUDAStream(device.index());
+    if (cur == built_on) return;
+    built.block(cur);
+    buf.record_stream(cur);
+  }
+
+  // Raises if a finished launch has reported a status to the host mirror. Never synchronises.
+  void poll() {
+    const uint32_t s = *host_word;
+    if (s != 0) report(s);
+  }
+
+  // Synchronises the current stream, reads the device status word and raises if it is set.
+  void check_status() {
+    const uint32_t s = static_cast<uint32_t>(status_dev.item<int32_t>());
+    if (s != 0) report(s);
+  }
+
+  [[noreturn]] void report(uint32_t s) {
+    // both copies are cleared, so that one event is reported once and later launches start clean
+    status_dev.zero_();
+    *host_word = 0;
+    TORCH_CHECK_VALUE((s & kStatusSpanRange) == 0, "span_id values must fit in 24 signed bits (|span_id| < 2**23)");
+    char hex[16], site[16];
+    snprintf(hex, sizeof hex, "0x%08x", s);
+    snprintf(site, sizeof site, "0x%x", s & 0xFFFFu);
+    TORCH_CHECK((s & kStatusTimeout) == 0, "a device-side wait timed out (status ", hex, ", wait site ", site,
+                "); the results of that launch are invalid");
+    TORCH_CHECK(false, "device status ", hex);
+  }
+
+  void after_launch() {
+    if (check_every_launch()) check_status();
+  }
+};
+using PlanPtr = std::shared_ptr<Plan>;
+
+// The cache key: identity, version and geometry of the metadata tensors (the plan keeps them alive, so an address
+// cannot be reused while its plan is cached) and the flags of the mask.
+struct PlanKey {
+  struct Slot {
+    const void* ptr = nullptr;
+    uint32_t version = 0;
+    int64_t s0 = 0, s1 = 0, st0 = 0, st1 = 0;
+    int32_t dtype = -1, dim = 0;
+    bool operator==(const Slot& o) const {
+      return ptr == o.ptr && version == o.version && s0 == o.s0 && s1 == o.s1 && st0 == o.st0 && st1 == o.st1 && dtype == o.dtype && dim == o.dim;
+    }
+  };
+  int64_t B, T;
+  int32_t device, flags;
+  Slot slot[4];
+  bool operator==(const PlanKey& o) const {
+    return B == o.B && T == o.T && device == o.device && flags == o.flags && slot[0] == o.slot[0] && slot[1] == o.slot[1] &&
+           slot[2] == o.slot[2] && slot[3] == o.slot[3];
+  }
+};
+struct PlanKeyHash {
+  size_t operator()(const PlanKey& k) const {
+    size_t h = static_cast<size_t>(k.B * 1000003 + k.T) * 31 + static_cast<size_t>(k.device * 4 + k.flags);
+    for (const auto& s : k.slot) h = (h ^ reinterpret_cast<uintptr_t>(s.ptr) ^ s.version) * 0x9E3779B97F4A7C15ull;
+    return h;
+  }
+};
+
+class PlanCache {
+ public:
+  static constexpr size_t kSize = 64;
+  PlanPtr find(const PlanKey& key) {
+    std::lock_guard<std::mutex> lock(m_);
+    auto it = map_.find(key);
+    if (it == map_.end()) return nullptr;
+    order_.splice(order_.end(), order_, it->second);
+    return it->second->second;
+  }
+  void insert(const PlanKey& key, PlanPtr plan) {
+    PlanPtr evicted;   // destroyed after the lock is released
+    std::lock_guard<std::mutex> lock(m_);
+    if (map_.count(key)) return;
+    order_.emplace_back(key, std::move(plan));
+    map_[key] = std::prev(order_.end());
+    if (order_.size() > kSize) {
+      evicted = std::move(order_.front().second);
+      map_.erase(order_.front().first);
+      order_.pop_front();
+    }
+  }
+  std::vector<PlanPtr> values() {
+    std::lock_guard<std::mutex> lock(m_);
+    std::vector<PlanPtr> v;
+    for (auto& e : order_) v.push_back(e.second);
+    return v;
+  }
+  void clear() {
+    std::list<std::pair<PlanKey, PlanPtr>> gone;
+    std::lock_guard<std::mutex> lock(m_);
+    map_.clear();
+    gone.swap(order_);
+  }
+
+ private:
+  std::mutex m_;
+  std::list<std::pair<PlanKey, PlanPtr>> order_;   // least recently used first
+  std::unordered_map<PlanKey, std::list<std::pair<PlanKey, PlanPtr>>::iterator, PlanKeyHash> map_;
+};
+PlanCache& cache() {
+  static PlanCache* c = new PlanCache;   // never destroyed: at exit the CUDA context may be gone before it
+  return *c;
+}
+
+bool fill_slot(PlanKey::Slot& s, const OptTensor& t) {
+  if (!t.has_value()) return true;
+  if (t->is_inference()) return false;   // no version counter: a rewrite could not be told from the original
+  s.ptr = t->data_ptr();
+  s.version = static_cast<uint32_t>(t->_version());
+  s.dim = static_cast<int32_t>(t->dim());
+  s.dtype = static_cast<int32_t>(t->scalar_type());
+  if (s.dim > 0) { s.s0 = t->size(0); s.st0 = t->stride(0); }
+  if (s.dim > 1) { s.s1 = t->size(1); s.st1 = t->stride(1); }
+  return true;
+}
+
+PlanPtr get_plan(int64_t B, int64_t T, at::Device device, const OptTensor& in_span, const OptTensor& span_id,
+                 const OptTensor& is_prefix, const OptTensor& lens, bool causal, bool rules) {
+  if (!device.has_index()) device = at::Device(device.type(), at::cuda::current_device());
+  PlanKey key{B, T, device.index(), (causal ? 1 : 0) | (rules ? 2 : 0), {}};
+  const bool keyed = fill_slot(key.slot[0], in_span) && fill_slot(key.slot[1], span_id) && fill_slot(key.slot[2], is_prefix) &&
+                     fill_slot(key.slot[3], lens);
+  if (keyed) {
+    if (PlanPtr p = cache().find(key)) {
+      p->use_on_current_stream();
+      p->poll();
+      return p;
+    }
+  }
+  auto p = std::make_shared<Plan>(B, T, device, in_span, span_id, is_prefix, lens, causal, rules);
+  if (keyed) cache().insert(key, p);
+  return p;
+}
+
+// ---- kernel calls ----------------------------------------------------------------------------------------------
+
+int dtype_code(at::ScalarType t) { return t == at::kHalf ? KD_F16 : t == at::kBFloat16 ? KD_BF16 : KD_F32; }
+
+kd_tensor desc(const Tensor& t) { return kd_tensor{t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
+
+// t itself when TMA can describe it (unit stride along D, 16-byte aligned rows), else one contiguous copy
+Tensor usable(const Tensor& t) {
+  const int64_t es = t.element_size();
+  bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  for (int i = 0; i < 3; ++i) ok = ok && (t.stride(i) * es) % 16 == 0 && t.stride(i) > 0;
+  return ok ? t : t.contiguous();
+}
+
+Tensor empty_out(const Tensor& like, bool like_input) {
+  // empty_like keeps the strides of a dense tensor, e.g. (B,T,H,D) memory seen as (B,H,T,D)
+  return like_input ? at::empty_like(like) : at::empty(like.sizes(), like.options());
+}
+
+kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Plan& plan,
+                      double sm_scale, int heads_per_cta) {
+  kd_attn_params p{};
+  p.B = static_cast<int32_t>(q.size(0));
+  p.H = static_cast<int32_t>(q.size(1));
+  p.T = static_cast<int32_t>(q.size(2));
+  p.D = static_cast<int32_t>(q.size(3));
+  p.dtype = dtype_code(q.scalar_type());
+  p.sm_scale = static_cast<float>(sm_scale);
+  p.q = desc(q);
+  p.k = desc(k);
+  p.v = desc(v);
+  p.o = desc(o);
+  p.lse = lse.data_ptr<float>();
+  p.plan = plan.buf.data_ptr();
+  p.heads_per_cta = heads_per_cta;
+  return p;
+}
+
+std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const PlanPtr& plan, double sm_scale,
+                                   bool like_input, int heads_per_cta) {
+  const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
+  Tensor o = empty_out(q, like_input);
+  Tensor lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
+  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
+  plan->poll();
+  c10::cuda::CUDAGuard guard(q.device());
+  check(lib.attn_fwd(&p, at::cuda::getCurrentCUDAStream()));
+  plan->after_launch();
+  return {o, lse};
+}
+
+// `phases` selects a part of the backward (kd_attn_params.bwd_phases); defined tensors among dq .. dq_acc are reused.
+std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o, const Tensor& lse,
+                                            const Tensor& d_o_, const PlanPtr& plan, double sm_scale, int phases, Tensor dq, Tensor dk,
+                                            Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic,
+                                            int heads_per_cta) {
+  const Tensor q = usable(q_), k = usable(k_), v = usable(v_), d_o = usable(d_o_);
+  if (!dq.defined()) {
+    dq = empty_out(q, like_input);
+    dk = empty_out(k, like_input);
+    dv = empty_out(v, like_input);
+  }
+  const auto f32 = q.options().dtype(at::kFloat);
+  if (!delta.defined()) delta = at::empty({q.size(0), q.size(1), q.size(2)}, f32);
+  const bool fused = !deterministic && q.size(3) <= 64;
+  // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
+  if (fused && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), 64}, f32);
+  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
+  p.d_o = desc(d_o);
+  p.dq = desc(dq);
+  p.dk = desc(dk);
+  p.dv = desc(dv);
+  p.delta = delta.data_ptr<float>();
+  p.bwd_phases = phases;
+  if (fused) {
+    p.bwd_mode = KD_BWD_FUSED;
+    p.dq_acc = dq_acc.data_ptr<float>();
+  }
+  plan->poll();
+  c10::cuda::CUDAGuard guard(q.device());
+  check(lib.attn_bwd(&p, at::cuda::getCurrentCUDAStream()));
+  plan->after_launch();
+  return {dq, dk, dv};
+}
+
+Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
+  const Tensor x = usable(x_);
+  Tensor y = at::empty(x.sizes(), x.options());
+  const kd_tensor xs = desc(x), ys = desc(y);
+  c10::cuda::CUDAGuard guard(x.device());
+  check(lib.hadamard(&xs, &ys, static_cast<int32_t>(x.size(0)), static_cast<int32_t>(x.size(1)), static_cast<int32_t>(x.size(2)),
+                     static_cast<int32_t>(x.size(3)), dtype_code(x.scalar_type()), signs.has_value() ? signs->data_ptr<float>() : nullptr,
+                     inverse ? 1 : 0, at::cuda::getCurrentCUDAStream()));
+  return y;
+}
+
+// ---- autograd --------------------------------------------------------------------------------------------------
+
+struct Options {
+  double sm_scale;
+  bool like_input, deterministic;
+  int heads_per_cta;
+};
+
+// dQ, dK, dV of one flash_attention call. Saves the operands the kernels read: for float32 tensors their float16
+// copies, with incoherent processing the transformed Q and K.
+struct AttentionBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable q, k, v, o, lse;
+  PlanPtr plan;
+  Options opt;
+  OptTensor signs;
+  bool widen;   // float32 tensors: gradients go back as float32
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list out(3);
+    if (!grads[0].defined()) return out;
+    Tensor tq, tk, tv, to, tlse;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      tq = q.unpack();
+      tk = k.unpack();
+      tv = v.unpack();
+      to = o.unpack(shared_from_this());
+      tlse = lse.unpack();
+    }
+    at::NoGradGuard no_grad;
+    const Tensor d_o = widen ? grads[0].to(at::kHalf) : grads[0];
+    auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
+                                 opt.heads_per_cta);
+    if (signs.has_value()) {
+      // y = x diag(s) W / sqrt(D) with W symmetric, so dx = dy W / sqrt(D) diag(s)
+      dq = hadamard(dq, signs, true);
+      dk = hadamard(dk, signs, true);
+    }
+    if (widen) {
+      dq = dq.to(at::kFloat);
+      dk = dk.to(at::kFloat);
+      dv = dv.to(at::kFloat);
+    }
+    out[0] = dq;
+    out[1] = dk;
+    out[2] = dv;
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    q.reset_data();
+    k.reset_data();
+    v.reset_data();
+    o.reset_data();
+    lse.reset_data();
+  }
+  std::string name() const override { return "FlashAttentionBackward"; }
+};
+
+void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v) {
+  KD_VALUE(q.dim() == 4, "q, k, v must be (batch, heads, time, head_dim)");
+  KD_VALUE(q.sizes() == k.sizes() && q.sizes() == v.sizes(), "q, k, v must have the same shape, got ", q.sizes(), ", ", k.sizes(), ", ", v.sizes());
+  TORCH_CHECK(q.is_cuda(), "flash_attention runs on CUDA sm_100 devices only; there is no CPU path");
+  const auto t = q.scalar_type();
+  KD_VALUE((t == at::kHalf || t == at::kBFloat16 || t == at::kFloat) && k.scalar_type() == t && v.scalar_type() == t,
+           "q, k, v must share dtype float16, bfloat16 or float32");
+  KD_VALUE(q.size(3) % 16 == 0 && q.size(3) >= 16 && q.size(3) <= 128, "head_dim ", q.size(3), " is not supported (a multiple of 16 from 16 to 128)");
+  KD_VALUE(k.device() == q.device() && v.device() == q.device(), "q, k, v must be on the same device");
+}
+
+std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& lens, std::optional<double> sm_scale,
+                                     bool causal, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix, bool rules,
+                                     const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta) {
+  check_inputs(q, k, v);
+  const double scale = sm_scale.has_value() ? *sm_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
+  KD_VALUE(scale > 0.0 && std::isfinite(scale), "sm_scale must be positive and finite");
+  PlanPtr plan = get_plan(q.size(0), q.size(2), q.device(), in_span, span_id, is_prefix, lens, causal, rules);
+  const bool track = at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
+  const bool f32 = q.scalar_type() == at::kFloat;
+  Tensor o, lse, q2, k2, v2, o16;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    q2 = f32 ? q.to(at::kHalf) : q;
+    k2 = f32 ? k.to(at::kHalf) : k;
+    v2 = f32 ? v.to(at::kHalf) : v;
+    if (signs.has_value()) {
+      q2 = hadamard(q2, signs, false);
+      k2 = hadamard(k2, signs, false);
+    }
+    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, heads_per_cta);
+    o = f32 ? o16.to(at::kFloat) : o16;
+  }
+  if (track) {
+    auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
+    node->plan = std::move(plan);
+    node->opt = Options{scale, like_input, deterministic, heads_per_cta};
+    node->signs = signs;
+    node->widen = f32;
+    torch::autograd::set_history(o, node);
+    node->q = torch::autograd::SavedVariable(q2, false);
+    node->k = torch::autograd::SavedVariable(k2, false);
+    node->v = torch::autograd::SavedVariable(v2, false);
+    node->o = torch::autograd::SavedVariable(o16, !f32);   // for float32 tensors o16 is a copy of its own, not the output
+    node->lse = torch::autograd::SavedVariable(lse, false);
+  }
+  return {o, lse};
+}
+
+// ---- metadata --------------------------------------------------------------------------------------------------
+
+std::tuple<Tensor, Tensor, Tensor> metadata_from_tokens(const Tensor& tokens_, int64_t tok_span, int64_t tok_es, int64_t tok_cls, int64_t tok_maskq) {
+  const Tensor tokens = tokens_.stride(1) == 1 ? tokens_ : tokens_.contiguous();
+  const int64_t B = tokens.size(0), T = tokens.size(1);
+  Tensor in_span = at::empty({B, T}, tokens.options().dtype(at::kBool));
+  Tensor span_id = at::empty({B, T}, tokens.options());
+  Tensor is_prefix = at::empty({B, T}, tokens.options().dtype(at::kBool));
+  c10::cuda::CUDAGuard guard(tokens.device());
+  check(lib.metadata_from_tokens(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(T, 1), static_cast<int32_t>(B),
+                                 static_cast<int32_t>(T), tok_span, tok_es, tok_cls, tok_maskq, static_cast<uint8_t*>(in_span.data_ptr()),
+                                 span_id.data_ptr<int64_t>(), static_cast<uint8_t*>(is_prefix.data_ptr()), at::cuda::getCurrentCUDAStream()));
+  return {in_span, span_id, is_prefix};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.doc() = "host path of the attention operator";
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const LibraryError& e) {
+      PyErr_SetString(py::module_::import("kerneldev_b200._capi").attr("KdError").ptr(), e.what());
+    } catch (const c10::ValueError& e) {
+      PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
+    } catch (const c10::Error& e) {
+      PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    }
+  });
+  py::class_<Plan, PlanPtr>(m, "Plan")
+      .def(py::init<int64_t, int64_t, at::Device, const OptTensor&, const OptTensor&, const OptTensor&, const OptTensor&, bool, bool>())
+      .def_readonly("B", &Plan::B)
+      .def_readonly("T", &Plan::T)
+      .def_readonly("device", &Plan::device)
+      .def_readonly("buf", &Plan::buf)
+      .def_readonly("status_dev", &Plan::status_dev)
+      .def_readonly("status_host", &Plan::status_host)
+      .def("use_on_current_stream", &Plan::use_on_current_stream);
+  m.def("bind", &bind);
+  m.def("get_plan", &get_plan);
+  m.def("cached_plans", [] { return cache().values(); });
+  m.def("clear_plans", [] { cache().clear(); });
+  m.def("forward", &forward);
+  m.def("backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, const PlanPtr& plan,
+                       double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic, int heads_per_cta) {
+    Tensor b[5];
+    for (size_t i = 0; i < bufs.size() && i < 5; ++i) b[i] = bufs[i];
+    return backward(q, k, v, o, lse, d_o, plan, sm_scale, phases, b[0], b[1], b[2], b[3], b[4], like_input, deterministic, heads_per_cta);
+  });
+  m.def("hadamard", &hadamard);
+  m.def("attention", &attention);
+  m.def("metadata_from_tokens", &metadata_from_tokens);
+}

@@ -13,6 +13,8 @@ namespace kd {
 __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
   const int tile = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int t = tile * KD_TILE + tid;
+  // for the reports of later kernels; this kernel's own use the argument
+  if (tile == 0 && b == 0 && tid == 0) *reinterpret_cast<uint32_t**>(pv.status + 2) = m.status_mirror;
   int n_b = m.T;
   if (m.lens != nullptr) n_b = min(m.lens[b], m.T);
   const bool alive = t < n_b;
@@ -22,7 +24,10 @@ __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
       const bool ins = m.in_span ? (m.in_span[b * m.in_span_stride_b + t] != 0) : false;
       const bool pre = m.is_prefix ? (m.is_prefix[b * m.is_prefix_stride_b + t] != 0) : false;
       const int64_t sid = m.span_id ? m.span_id[b * m.span_id_stride_b + t] : 0;
-      if (sid >= (1 << 23) || sid < -(1 << 23)) atomicOr(pv.status, KD_STATUS_SPAN_RANGE);
+      if (sid >= (1 << 23) || sid < -(1 << 23)) {
+        atomicOr(pv.status, KD_STATUS_SPAN_RANGE);
+        if (m.status_mirror != nullptr) *const_cast<volatile uint32_t*>(m.status_mirror) = KD_STATUS_SPAN_RANGE;
+      }
       d = pack_token(ins, pre, sid, true);
     } else {
       // no metadata: causal = every token is context; otherwise every token is prefix

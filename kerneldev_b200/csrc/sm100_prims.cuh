@@ -82,6 +82,18 @@ struct AbortFlag {
   volatile uint32_t v;
 };
 
+// Records `value` in the plan's status word (the first report wins) and in its host mirror, whose address the
+// plan keeps eight bytes behind the word. Only failing launches get here, so a successful one costs the host
+// neither a copy nor a synchronisation.
+__device__ __forceinline__ void report_status(uint32_t* status, uint32_t value) {
+  if (atomicCAS(status, KD_DEV_OK, value) != KD_DEV_OK) return;
+  uint32_t* mirror = *reinterpret_cast<uint32_t* volatile*>(status + 2);
+  if (mirror != nullptr) {
+    *const_cast<volatile uint32_t*>(mirror) = value;
+    __threadfence_system();
+  }
+}
+
 #ifndef KD_WAIT_LIMIT_NS
 #define KD_WAIT_LIMIT_NS 400000000ull  // 0.4 s: far above any legitimate wait in these kernels
 #endif
@@ -113,7 +125,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFl
     if (abort_flag->v != 0u) return false;
     if (globaltimer_ns() - t0 > KD_WAIT_LIMIT_NS) {
       abort_flag->v = 1u;
-      atomicCAS(status, KD_DEV_OK, KD_DEV_TIMEOUT | site);
+      report_status(status, KD_DEV_TIMEOUT | site);
       return false;
     }
   }

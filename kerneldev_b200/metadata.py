@@ -10,7 +10,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _capi
+from . import _host
 
 #: ids of the reference tokenizer's special tokens (data_builder.py:44-51)
 SPECIAL_TOKENS = {"[PAD]": 0, "[CLS]": 1, "[MASK]": 2, "[SPAN]": 3, "[ES]": 4, "[MASKQ]": 5}
@@ -24,15 +24,4 @@ def metadata_from_tokens(tokens: torch.Tensor, special_tokens=None):
     if not tokens.is_cuda:
         raise RuntimeError("metadata_from_tokens runs on CUDA devices only; there is no CPU path")
     st = SPECIAL_TOKENS if special_tokens is None else special_tokens
-    if tokens.stride(1) != 1:
-        tokens = tokens.contiguous()
-    B, T = tokens.shape
-    in_span = torch.empty((B, T), dtype=torch.bool, device=tokens.device)
-    span_id = torch.empty((B, T), dtype=torch.int64, device=tokens.device)
-    is_prefix = torch.empty((B, T), dtype=torch.bool, device=tokens.device)
-    stream = torch.cuda.current_stream(tokens.device).cuda_stream
-    with torch.cuda.device(tokens.device):
-        _capi.check(_capi.load().kd_metadata_from_tokens(
-            tokens.data_ptr(), tokens.stride(0) if B > 1 else max(T, 1), B, T, st["[SPAN]"], st["[ES]"], st["[CLS]"],
-            st["[MASKQ]"], in_span.data_ptr(), span_id.data_ptr(), is_prefix.data_ptr(), stream))
-    return in_span, span_id, is_prefix
+    return _host.load().metadata_from_tokens(tokens, st["[SPAN]"], st["[ES]"], st["[CLS]"], st["[MASKQ]"])

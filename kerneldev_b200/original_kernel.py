@@ -20,19 +20,16 @@ Differences from the reference, all deliberate:
 """
 from __future__ import annotations
 
-import ctypes
-import math
-import os
-
 import torch
 
-from . import _capi
+from . import _capi, _host
 from .plan import AttentionPlan, get_plan
 
-_capi.load()  # fail at import time, loudly, when the CUDA library has not been built
+_ext = _host.load()  # fails at import time, loudly, when the CUDA library or the host extension has not been built
 
 __all__ = ["flash_attention", "generate_hadamard_signs", "hadamard_transform"]
 
+_HADAMARD_DIMS = (16, 32, 64, 128)
 _DTYPES = {torch.float16: _capi.KD_F16, torch.bfloat16: _capi.KD_BF16}
 
 # Heads a CTA handles one after the other (kd_attn_params.heads_per_cta): 0 lets the library choose from
@@ -42,30 +39,6 @@ HEADS_PER_CTA = 0
 
 def _kd_tensor(t: torch.Tensor) -> _capi.KdTensor:
     return _capi.KdTensor(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
-
-
-def _usable(t: torch.Tensor) -> torch.Tensor:
-    """Returns t itself when TMA can describe it (unit stride along D, 16-byte aligned rows),
-    else one contiguous copy."""
-    es = t.element_size()
-    ok = (t.stride(3) == 1 and t.data_ptr() % 16 == 0
-          and all((t.stride(i) * es) % 16 == 0 and t.stride(i) > 0 for i in range(3)))
-    return t if ok else t.contiguous()
-
-
-def _check_inputs(q, k, v):
-    if q.dim() != 4:
-        raise ValueError("q, k, v must be (batch, heads, time, head_dim)")
-    if not (q.shape == k.shape == v.shape):
-        raise ValueError(f"q, k, v must have the same shape, got {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
-    if not q.is_cuda:
-        raise RuntimeError("flash_attention runs on CUDA sm_100 devices only; there is no CPU path")
-    if q.dtype not in _DTYPES or k.dtype != q.dtype or v.dtype != q.dtype:
-        raise ValueError("q, k, v must share dtype float16, bfloat16 or float32")
-    if q.shape[-1] % 16 != 0 or not 16 <= q.shape[-1] <= 128:
-        raise ValueError(f"head_dim {q.shape[-1]} is not supported (a multiple of 16 from 16 to 128)")
-    if not (k.device == q.device and v.device == q.device):
-        raise ValueError("q, k, v must be on the same device")
 
 
 def _params(q, k, v, o, lse, plan, sm_scale):
@@ -81,30 +54,10 @@ def _params(q, k, v, o, lse, plan, sm_scale):
     return p
 
 
-def _after_launch(plan: AttentionPlan) -> None:
-    """Device-side failures (a bounded wait that gave up) are written to the plan's status word. The word
-    follows every launch to a pinned host mirror; ``plan.poll()`` at the next call raises from it without
-    a synchronisation. KD_CHECK_STATUS=1 synchronises and checks after every launch instead."""
-    plan.mirror_status()
-    if os.environ.get("KD_CHECK_STATUS") == "1":
-        plan.check_status()
-
-
 def _forward(q, k, v, plan: AttentionPlan, sm_scale: float, like_input: bool = False):
-    """One kd_attn_fwd call: returns (O, LSE) for inputs that passed _check_inputs. ``like_input``: O in the
+    """One kd_attn_fwd call: returns (O, LSE) for inputs flash_attention would accept. ``like_input``: O in the
     memory layout of q instead of contiguous."""
-    q, k, v = _usable(q), _usable(k), _usable(v)
-    B, H, T, D = q.shape
-    # empty_like keeps the strides of a dense q, e.g. (B,T,H,D) memory seen as (B,H,T,D)
-    o = torch.empty_like(q) if like_input else torch.empty((B, H, T, D), dtype=q.dtype, device=q.device)
-    lse = torch.empty((B, H, T), dtype=torch.float32, device=q.device)
-    p = _params(q, k, v, o, lse, plan, sm_scale)
-    stream = torch.cuda.current_stream(q.device).cuda_stream
-    plan.poll()
-    with torch.cuda.device(q.device):
-        _capi.check(_capi.load().kd_attn_fwd(ctypes.byref(p), stream))
-    _after_launch(plan)
-    return o, lse
+    return _ext.forward(q, k, v, plan._core, sm_scale, like_input, HEADS_PER_CTA)
 
 
 def _backward(q, k, v, o, lse, d_o, plan: AttentionPlan, sm_scale: float, phases: int = 0, bufs=None,
@@ -113,70 +66,11 @@ def _backward(q, k, v, o, lse, d_o, plan: AttentionPlan, sm_scale: float, phases
     kd_attn_params.bwd_phases); ``bufs`` = (dq, dk, dv, delta[, dq_acc]) reuses buffers.
     ``deterministic=False`` selects the fused backward where it exists (head_dim <= 64): one pass over the
     tiles instead of two, dQ accumulated with fp32 atomics in a (B,H,T,D) scratch."""
-    q, k, v, d_o = _usable(q), _usable(k), _usable(v), _usable(d_o)
-    B, H, T, D = q.shape
-    if bufs is None:
-        if like_input:   # each gradient in its input's layout
-            dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        else:
-            dq = torch.empty((B, H, T, D), dtype=q.dtype, device=q.device)
-            dk = torch.empty_like(dq)
-            dv = torch.empty_like(dq)
-        delta = torch.empty((B, H, T), dtype=torch.float32, device=q.device)
-        dq_acc = None
-    else:
-        dq, dk, dv, delta = bufs[:4]
-        dq_acc = bufs[4] if len(bufs) > 4 else None
-    fused = (not deterministic) and D <= 64
-    if fused and dq_acc is None:   # rows as wide as the kernel's tile (kd_workspace_bytes_fused)
-        dq_acc = torch.empty((B, H, T, 64), dtype=torch.float32, device=q.device)
-    p = _params(q, k, v, o, lse, plan, sm_scale)
-    p.d_o = _kd_tensor(d_o)
-    p.dq, p.dk, p.dv = _kd_tensor(dq), _kd_tensor(dk), _kd_tensor(dv)
-    p.delta = delta.data_ptr()
-    p.bwd_phases = phases
-    if fused:
-        p.bwd_mode = _capi.KD_BWD_FUSED
-        p.dq_acc = dq_acc.data_ptr()
-    stream = torch.cuda.current_stream(q.device).cuda_stream
-    plan.poll()
-    with torch.cuda.device(q.device):
-        _capi.check(_capi.load().kd_attn_bwd(ctypes.byref(p), stream))
-    _after_launch(plan)
-    return dq, dk, dv
-
-
-class _FlashAttentionFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, plan, sm_scale, like_input=False, deterministic=False):
-        o, lse = _forward(q, k, v, plan, sm_scale, like_input)
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.plan = plan
-        ctx.sm_scale = sm_scale
-        ctx.like_input = like_input
-        ctx.deterministic = deterministic
-        ctx.mark_non_differentiable(lse)
-        return o, lse
-
-    @staticmethod
-    def backward(ctx, d_o, _d_lse):
-        q, k, v, o, lse = ctx.saved_tensors
-        dq, dk, dv = _backward(q, k, v, o, lse, d_o, ctx.plan, ctx.sm_scale, like_input=ctx.like_input,
-                               deterministic=ctx.deterministic)
-        return dq, dk, dv, None, None, None, None
+    return _ext.backward(q, k, v, o, lse, d_o, plan._core, sm_scale, phases, list(bufs or ()), like_input, deterministic, HEADS_PER_CTA)
 
 
 def _hadamard_call(x: torch.Tensor, signs, inverse: bool) -> torch.Tensor:
-    x = _usable(x)
-    B, H, T, D = x.shape
-    y = torch.empty((B, H, T, D), dtype=x.dtype, device=x.device)
-    xs, ys = _kd_tensor(x), _kd_tensor(y)
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        _capi.check(_capi.load().kd_hadamard(ctypes.byref(xs), ctypes.byref(ys), B, H, T, D, _DTYPES[x.dtype],
-                                             signs.data_ptr() if signs is not None else None,
-                                             1 if inverse else 0, stream))
-    return y
+    return _ext.hadamard(x, signs, inverse)
 
 
 class _HadamardFn(torch.autograd.Function):
@@ -202,15 +96,19 @@ def generate_hadamard_signs(n_heads: int, head_dim: int, seed: int = 0, device="
     return s.to(torch.float32).to(device)
 
 
+def _check_signs(signs: torch.Tensor, n_heads: int, head_dim: int, device) -> torch.Tensor:
+    if signs.shape != (n_heads, head_dim):
+        raise ValueError("signs must have shape (heads, head_dim)")
+    return signs.to(device=device, dtype=torch.float32).contiguous()
+
+
 def hadamard_transform(x: torch.Tensor, signs: torch.Tensor | None = None) -> torch.Tensor:
     """``WHT(x * signs[h]) / sqrt(D)`` over the last dimension of a (B, H, T, D) tensor, with the
     Walsh-Hadamard matrix in natural (Sylvester) order; differentiable."""
-    if x.dim() != 4 or x.shape[-1] not in (16, 32, 64, 128) or x.dtype not in _DTYPES or not x.is_cuda:
+    if x.dim() != 4 or x.shape[-1] not in _HADAMARD_DIMS or x.dtype not in _DTYPES or not x.is_cuda:
         raise ValueError("hadamard_transform expects a CUDA (B, H, T, D) fp16/bf16 tensor with D in {16, 32, 64, 128}")
     if signs is not None:
-        if signs.shape != (x.shape[1], x.shape[3]):
-            raise ValueError("signs must have shape (heads, head_dim)")
-        signs = signs.to(device=x.device, dtype=torch.float32).contiguous()
+        signs = _check_signs(signs, x.shape[1], x.shape[3], x.device)
     return _HadamardFn.apply(x, signs)
 
 
@@ -261,38 +159,22 @@ def flash_attention(
 
     Returns O, or (O, LSE) with return_lse, or (that, mask[B,H,T,T] bool) with return_attention_mask.
     """
-    if q.dtype is torch.float32 and k.dtype is torch.float32 and v.dtype is torch.float32:
-        if precision == "ieee":
-            raise ValueError("float32 inputs with precision='ieee' are not supported: the tensor cores take 16-bit operands here "
-                             "(precision='tf32' rounds the operands to tf32's 10-bit mantissa)")
-        res = flash_attention(q.to(torch.float16), k.to(torch.float16), v.to(torch.float16), lens, sm_scale, causal, autotune,
-                              return_lse, prescale_qk, precision, attention_mask, in_span, span_id, is_prefix,
-                              return_attention_mask, hadamard_signs, out_layout, deterministic)
-        widen = lambda x: x.to(torch.float32) if torch.is_tensor(x) and x.dtype is torch.float16 else x
-        if return_attention_mask:
-            first, mask = res
-            first = tuple(widen(x) for x in first) if isinstance(first, tuple) else widen(first)
-            return first, mask
-        return tuple(widen(x) for x in res) if isinstance(res, tuple) else widen(res)
-    _check_inputs(q, k, v)
-    B, H, T, D = q.shape
-    if sm_scale is None:
-        sm_scale = D ** -0.5
-    sm_scale = float(sm_scale)
-    if not (sm_scale > 0.0 and math.isfinite(sm_scale)):
-        raise ValueError("sm_scale must be positive and finite")
-    rules = any(t is not None for t in (attention_mask, in_span, span_id, is_prefix))
-    plan = get_plan(B, T, q.device, in_span, span_id, is_prefix, lens, causal, rules)
-
-    if hadamard_signs is not None:
-        q = hadamard_transform(q, hadamard_signs)
-        k = hadamard_transform(k, hadamard_signs)
-
+    if precision == "ieee" and q.dtype is torch.float32 and k.dtype is torch.float32 and v.dtype is torch.float32:
+        raise ValueError("float32 inputs with precision='ieee' are not supported: the tensor cores take 16-bit operands here "
+                         "(precision='tf32' rounds the operands to tf32's 10-bit mantissa)")
     if out_layout not in ("contiguous", "input"):
         raise ValueError("out_layout must be 'contiguous' or 'input'")
-    o, lse = _FlashAttentionFn.apply(q, k, v, plan, sm_scale, out_layout == "input", bool(deterministic))
+    rules = attention_mask is not None or in_span is not None or span_id is not None or is_prefix is not None
+    if hadamard_signs is not None and q.dim() == 4:
+        if q.shape[-1] not in _HADAMARD_DIMS:
+            raise ValueError("hadamard_signs needs a head_dim in {16, 32, 64, 128}")
+        hadamard_signs = _check_signs(hadamard_signs, q.shape[1], q.shape[3], q.device)
+    o, lse = _ext.attention(q, k, v, lens, sm_scale, bool(causal), in_span, span_id, is_prefix, rules, hadamard_signs,
+                            out_layout == "input", bool(deterministic), HEADS_PER_CTA)
 
     if return_attention_mask:
+        B, H, T, _ = q.shape
+        plan = get_plan(B, T, q.device, in_span, span_id, is_prefix, lens, causal, rules)
         mask = plan.dense_mask().unsqueeze(1).expand(B, H, T, T)
         if return_lse:
             return (o, lse), mask

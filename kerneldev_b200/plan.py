@@ -10,49 +10,25 @@ reused while its plan is cached). Metadata rewritten in place through raw pointe
 kd_metadata_from_tokens into preallocated buffers, or through ``.data`` -- does not change a tensor's
 version: call ``clear_plan_cache()`` after such a write.
 
+The plans and their cache live in the host extension (csrc/host.cpp); ``AttentionPlan`` is the view of one
+of them from Python.
+
 Device status. Kernels report problems (a bounded wait that ran out, a span id out of range) in the
-plan's status word. After every launch the word is copied to a pinned host mirror with an
-asynchronous copy on the launching stream; the next call that uses the plan (or ``poll()``) looks at
-the mirror without synchronising and raises, so a failed launch surfaces one call later at the
-latest -- normally at the backward of the same step. ``KD_CHECK_STATUS=1`` makes every call
-synchronise and check at once.
+plan's status word and, in the same breath, in a pinned host mirror whose address the plan carries; the
+next call that uses the plan (or ``poll()``) looks at the mirror without synchronising and raises, so a
+failed launch surfaces one call later at the latest -- normally at the backward of the same step. A
+launch that succeeds costs no copy. ``KD_CHECK_STATUS=1`` makes every call synchronise and check at once.
 """
 from __future__ import annotations
 
 import ctypes
-import os
-from collections import OrderedDict
+import weakref
 
-import numpy as np
 import torch
 
-from . import _capi
+from . import _capi, _host
 
-_CACHE: "OrderedDict[tuple, AttentionPlan]" = OrderedDict()
-_CACHE_SIZE = 64
-
-
-def _tensor_key(t):
-    if t is None:
-        return None
-    return (t.data_ptr(), t._version, tuple(t.shape), tuple(t.stride()), str(t.dtype))
-
-
-_PINNED_WORDS = None
-_PINNED_NEXT = 0
-
-
-def _pinned_status_word() -> torch.Tensor:
-    """One int32 of pinned host memory for a plan's status mirror. Pinning memory is a slow, device-wide
-    call, so the words come from one pinned block handed out in rotation (1024 slots: a collision would
-    need more than 1024 live plans, and could only make a reported failure show up on two of them)."""
-    global _PINNED_WORDS, _PINNED_NEXT
-    if _PINNED_WORDS is None:
-        _PINNED_WORDS = torch.zeros(1024, dtype=torch.int32).pin_memory()
-    w = _PINNED_WORDS[_PINNED_NEXT:_PINNED_NEXT + 1]
-    _PINNED_NEXT = (_PINNED_NEXT + 1) % 1024
-    w.zero_()
-    return w
+_ext = _host.load()
 
 
 class AttentionPlan:
@@ -60,58 +36,27 @@ class AttentionPlan:
 
     def __init__(self, B, T, device, in_span=None, span_id=None, is_prefix=None, lens=None,
                  causal=True, rules=False):
-        self.B, self.T, self.device = B, T, device
-        self.layout = _capi.plan_layout(B, T)
+        device = torch.device(device)
+        if device.index is None:
+            device = torch.device(device.type, torch.cuda.current_device())
+        self._bind(_ext.Plan(B, T, device, in_span, span_id, is_prefix, lens, bool(causal), bool(rules)))
+
+    def _bind(self, core):
+        self._core = core
+        self.B, self.T, self.device, self.buf = core.B, core.T, core.device, core.buf
+        self.layout = _capi.plan_layout(self.B, self.T)
         self.NT, self.NP = self.layout.NT, self.layout.NP
-        # torch's caching allocator returns 512-byte aligned blocks, which covers the 256 the ABI asks for
-        self.buf = torch.empty(self.layout.total, dtype=torch.uint8, device=device)
-        meta = _capi.KdMeta()
-        meta.B, meta.T = B, T
-        keep = []
+        self._status_dev, self._status_host = core.status_dev, core.status_host
 
-        def prep(t, dtype, name):
-            if t is None:
-                return None, 0
-            if t.shape != (B, T):
-                raise ValueError(f"{name} must have shape (B, T) = ({B}, {T}), got {tuple(t.shape)}")
-            if t.device != device:
-                raise ValueError(f"{name} must live on {device}")
-            if dtype is torch.bool and t.dtype is not torch.bool:
-                raise ValueError(f"{name} must be a torch.bool tensor (the rule negates it logically)")
-            if dtype is torch.int64 and t.dtype is not torch.int64:
-                t = t.to(torch.int64)
-            if t.stride(1) != 1:
-                t = t.contiguous()
-            keep.append(t)
-            return t.data_ptr(), t.stride(0)
-
-        meta.in_span, meta.in_span_stride_b = prep(in_span, torch.bool, "in_span")
-        meta.span_id, meta.span_id_stride_b = prep(span_id, torch.int64, "span_id")
-        meta.is_prefix, meta.is_prefix_stride_b = prep(is_prefix, torch.bool, "is_prefix")
-        if lens is not None:
-            if lens.dtype is not torch.int32 or lens.shape != (B,):
-                raise ValueError("lens must be an int32 tensor of shape (B,)")
-            lens = lens.contiguous()
-            keep.append(lens)
-            meta.lens = lens.data_ptr()
-        meta.causal = 1 if causal else 0
-        meta.rules = 1 if rules else 0
-        # the caller's tensors and their converted copies stay alive while the plan is cached, so none of
-        # the addresses in the cache key can be handed to another tensor
-        self._keep = keep + [x for x in (in_span, span_id, is_prefix, lens) if x is not None]
-        off = self.layout.off_status
-        self._status_dev = self.buf[off:off + 4].view(torch.int32)
-        self._status_host = _pinned_status_word()
-        cur = torch.cuda.current_stream(device)
-        with torch.cuda.device(device):
-            _capi.check(_capi.load().kd_classify(ctypes.byref(meta), self.buf.data_ptr(), cur.cuda_stream))
-        # a plan used later from another stream must wait for the classifier
-        self._built_on = cur
-        self._built = torch.cuda.Event()
-        self._built.record(cur)
-        self.mirror_status()
-        if os.environ.get("KD_CHECK_STATUS") == "1":
-            self.check_status()
+    @classmethod
+    def _of(cls, core):
+        """The one Python view of a plan of the extension (while somebody holds it)."""
+        plan = _VIEWS.get(core)
+        if plan is None:
+            plan = object.__new__(cls)
+            plan._bind(core)
+            _VIEWS[core] = plan
+        return plan
 
     # ---- views into the plan buffer -------------------------------------------------------------
     def _view(self, off, nbytes, dtype, shape):
@@ -147,16 +92,14 @@ class AttentionPlan:
 
     def use_on_current_stream(self) -> None:
         """Orders the current stream after the classifier when the plan was built on another one."""
-        cur = torch.cuda.current_stream(self.device)
-        if cur != self._built_on:
-            cur.wait_event(self._built)
+        self._core.use_on_current_stream()
 
     def status(self) -> int:
         """Reads the device status word (synchronises the current stream)."""
         return int(self._status_dev.item()) & 0xFFFFFFFF
 
     def mirror_status(self) -> None:
-        """Enqueues a copy of the status word to the pinned host mirror behind the work just launched."""
+        """Enqueues a copy of the status word to the pinned host mirror (kernels write the mirror themselves)."""
         self._status_host.copy_(self._status_dev, non_blocking=True)
 
     def poll(self) -> None:
@@ -195,22 +138,30 @@ class AttentionPlan:
         return int(self.stats.sum().item())
 
 
+# the core is alive as long as its view is (the view holds it), so its hash cannot be reused while it is a key
+_VIEWS: "weakref.WeakValueDictionary" = weakref.WeakValueDictionary()
+
+
+class _PlanCacheView:
+    """The extension's plan cache seen from Python: the cached plans, least recently used first."""
+
+    def values(self):
+        return [AttentionPlan._of(core) for core in _ext.cached_plans()]
+
+    def clear(self):
+        _ext.clear_plans()
+
+    def __len__(self):
+        return len(_ext.cached_plans())
+
+
+_CACHE = _PlanCacheView()
+
+
 def get_plan(B, T, device, in_span=None, span_id=None, is_prefix=None, lens=None, causal=True,
              rules=False) -> AttentionPlan:
     """Returns a cached plan for this metadata, classifying on the device if it is new."""
-    key = (B, T, str(device), _tensor_key(in_span), _tensor_key(span_id), _tensor_key(is_prefix),
-           _tensor_key(lens), bool(causal), bool(rules))
-    plan = _CACHE.get(key)
-    if plan is not None:
-        _CACHE.move_to_end(key)
-        plan.use_on_current_stream()
-        plan.poll()
-        return plan
-    plan = AttentionPlan(B, T, device, in_span, span_id, is_prefix, lens, causal, rules)
-    _CACHE[key] = plan
-    while len(_CACHE) > _CACHE_SIZE:
-        _CACHE.popitem(last=False)
-    return plan
+    return AttentionPlan._of(_ext.get_plan(B, T, torch.device(device), in_span, span_id, is_prefix, lens, bool(causal), bool(rules)))
 
 
 def clear_plan_cache() -> None:
