@@ -116,14 +116,15 @@ typedef struct kd_attn_params {
                          kernel; 2: the dK/dV kernel alone (reads delta of an earlier pass 1).
                          Lets a caller time the two large kernels separately. */
   int32_t bwd_mode;   /* kd_attn_bwd only. KD_BWD_SPLIT (0): a dQ kernel and a dK/dV kernel as in the reference
-                         (original_kernel.py:1173-1336, :1339-1525), results bit-reproducible. KD_BWD_FUSED (1),
-                         D = 64 only: one kernel forms S and dP once per tile and adds its dQ partials to dq_acc
+                         (original_kernel.py:1173-1336, :1339-1525), results bit-reproducible. KD_BWD_FUSED (1):
+                         one kernel forms S and dP once per tile and adds its dQ partials to dq_acc
                          with fp32 atomics (dQ then differs in the last bits from run to run). With
                          KD_BWD_FUSED, bwd_phases 1 runs the delta kernel alone and 2 the fused kernel. */
-  float* dq_acc;      /* KD_BWD_FUSED: (B,H,T,D) contiguous fp32 scratch (kd_workspace_bytes_fused gives its
-                         size); the library zeroes it itself. Ignored otherwise. */
+  float* dq_acc;      /* KD_BWD_FUSED: (B,H,T,W) contiguous fp32 scratch, W = 64 for D <= 64 and 128 above
+                         (kd_workspace_bytes_fused gives its size); the library zeroes it itself. Ignored otherwise. */
   int32_t heads_per_cta; /* 0: chosen by the library from the grid size. n >= 1: every CTA handles n heads
-                         one after the other (they share the plan's work list); a tuning and test knob. */
+                         one after the other (they share the plan's work list); a tuning and test knob. The fused
+                         backward takes its work items dynamically and ignores it. */
 } kd_attn_params;
 
 /* Size and layout of a plan for B sequences of T tokens. */

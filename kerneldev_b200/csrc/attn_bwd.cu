@@ -193,7 +193,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int h = h0 + hh, fb = hh % C::NFIX;
         if (hh >= C::NFIX) {   // the buffer's previous head must have been consumed by both M1 issuers
-          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, a.status, W_Q_FIXEMPTY);
+          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, W_Q_FIXEMPTY);
           if (!ok) break;
         }
         mbar_arrive_expect_tx(smem_u32(&bar_fix_full[fb]), 2 * C::TILE_BYTES);
@@ -206,7 +206,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int s = issued % C::STAGES;
           const uint32_t ph = (issued / C::STAGES) & 1;
           const int kt = sAct[e] & 0xFF;
-          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, a.status, W_Q_RINGEMPTY);
+          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, W_Q_RINGEMPTY);
           if (!ok) break;
           mbar_arrive_expect_tx(smem_u32(&bar_ring_full[s]), 2 * C::TILE_BYTES);
           const uint32_t dst = sRing + s * 2 * C::TILE_BYTES;
@@ -235,7 +235,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       uint32_t ring_parity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int fb = hh % C::NFIX;
-        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, a.status, W_Q_FIXFULL);
+        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, W_Q_FIXFULL);
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // dO or Q
         uint64_t adesc[HD / 16];   // A descriptors of the head's k-steps
@@ -251,11 +251,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, a.status, W_Q_M2ISSUED);
+            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, W_Q_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its K and V tiles must have landed
-            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, a.status, W_Q_RINGFULL);
+            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, W_Q_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -280,7 +280,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       uint32_t round_parity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         if (hh > 0) {   // the previous head's dQ must have been read out of the accumulator
-          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, a.status, W_Q_ACCFREE);
+          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, W_Q_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -295,7 +295,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             bdesc[kk] = desc64(kb + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, a.status, W_Q_PFULL);
+          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_Q_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           mma_ts64_p(tAcc, aop[0], bdesc[0], idesc_m2, u > 0 ? 1u : 0u);
@@ -396,7 +396,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           prefetch_kd(ent_next);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, a.status, W_Q_SFULL);
+        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, W_Q_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -439,7 +439,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
       // epilogue of this head: warpgroup g stores EC columns of dQ from column g * EC
       if (na > 0) {
-        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, a.status, W_Q_ACCFULL);
+        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, W_Q_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -477,6 +477,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tbase, 512);
+  if (tid == 0) report_abort(&abortf, a.status);
 }
 
 // =========================================================================================
@@ -554,7 +555,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int h = h0 + hh, fb = hh % C::NFIX;
         if (hh >= C::NFIX) {
-          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, a.status, W_K_FIXEMPTY);
+          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, W_K_FIXEMPTY);
           if (!ok) break;
         }
         mbar_arrive_expect_tx(smem_u32(&bar_fix_full[fb]), 2 * C::TILE_BYTES);
@@ -567,7 +568,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           const int s = issued % C::STAGES;
           const uint32_t ph = (issued / C::STAGES) & 1;
           const int qt = list[e] & 0xFF;
-          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, a.status, W_K_RINGEMPTY);
+          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, W_K_RINGEMPTY);
           if (!ok) break;
           mbar_arrive_expect_tx(smem_u32(&bar_ring_full[s]), 2 * C::TILE_BYTES);
           const uint32_t dst = sRing + s * 2 * C::TILE_BYTES;
@@ -596,7 +597,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       uint32_t ring_parity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int fb = hh % C::NFIX;
-        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, a.status, W_K_FIXFULL);
+        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, W_K_FIXFULL);
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // V or K
         uint64_t adesc[HD / 16];   // A descriptors of the head's k-steps
@@ -612,11 +613,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, a.status, W_K_M2ISSUED);
+            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, W_K_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its Q and dO tiles must have landed
-            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, a.status, W_K_RINGFULL);
+            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, W_K_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -641,7 +642,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       uint32_t round_parity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         if (hh > 0) {   // the previous head's dK and dV must have been read out of the accumulators
-          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, a.status, W_K_ACCFREE);
+          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, W_K_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -659,7 +660,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             bdo[kk] = desc64(dob + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, a.status, W_K_PFULL);
+          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_K_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           // dV += P^T_u dO_u   (P^T_u on top of S^T_u)
@@ -786,7 +787,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           prefetch(ent_next, h + 1);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, a.status, W_K_SFULL);
+        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, W_K_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -848,7 +849,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
       // epilogue of this head: warpgroup g stores EC columns of dK and dV from column g * EC
       if (n > 0) {
-        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, a.status, W_K_ACCFULL);
+        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, W_K_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -894,6 +895,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tbase, 512);
+  if (tid == 0) report_abort(&abortf, a.status);
 }
 
 template <int HD, bool kBf16>
@@ -939,9 +941,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   }
   if (fused) {
     // bwd_phases 1: the delta kernel alone (it also zeroes dq_acc); 2: the fused kernel and the conversion
-    if constexpr (HD == 64) {
-      if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, grid, stream);
-    }
+    if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, stream);
   } else if (phases & 2) {
     kk<<<grid, C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, a);
   }

@@ -24,7 +24,7 @@ struct BwdArgs {
   int64_t do_sb, do_sh, do_st;
   const float* lse;
   float* delta;
-  float* dq_acc;     // fp32 (B,H,T,D) dQ accumulation scratch of the fused backward, else null
+  float* dq_acc;     // fp32 (B,H,T,tile width) dQ accumulation scratch of the fused backward, else null
   void* dq;
   int64_t dq_sb, dq_sh, dq_st;
   void* dk;
@@ -33,9 +33,9 @@ struct BwdArgs {
   int64_t dv_sb, dv_sh, dv_st;
 };
 
-// Fused backward for head dim 64 (attn_bwd_fused.cu): one key-tile-major kernel that forms S and dP once per
-// tile, accumulates dK and dV in TMEM and adds its dQ partials to a.dq_acc, then a conversion kernel.
+// Fused backward (attn_bwd_fused.cu): one key-tile-major kernel that forms S and dP once per tile, accumulates dK and
+// dV in TMEM and adds its dQ partials to a.dq_acc, then a conversion kernel.
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                     const BwdArgs& a, int dtype, dim3 grid, cudaStream_t stream);
+                     const BwdArgs& a, int dtype, cudaStream_t stream);
 
 }  // namespace kd

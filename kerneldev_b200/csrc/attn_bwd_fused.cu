@@ -1,630 +1,986 @@
-// Fused backward for head dim 64 on sm_100a: dK, dV and dQ from ONE pass over the non-empty tiles.
+// Fused backward on sm_100a: dK, dV and dQ from ONE pass over the non-empty tiles (head dims up to 128).
 //
 // The two-kernel backward (attn_bwd.cu) follows the reference's split into a dQ worker and a dK/dV
 // worker (original_kernel.py:1173-1336, :1339-1525) and so forms S = Q K^T, dP = dO V^T and the
 // exponentials twice per tile: 7 matrix products and two exponential passes. This kernel is key-tile
 // major like the dK/dV worker and forms them once: per (query tile, key tile)
-//     S^T = K Q^T, dP^T = V dO^T                           (smem x smem -> TMEM, in two halves of 64 queries)
+//     S^T = K Q^T, dP^T = V dO^T                           (smem x smem -> TMEM)
 //     P^T = exp2(S^T c - LSE), dS^T = P^T (dP^T - delta)   (compute warps; 16-bit results)
 //     dV += P^T dO                                         (P^T read from TMEM as the A operand)
 //     dK += dS^T Q,  dQ_tile = dS K                        (dS^T written to shared memory once and read by
 //                                                           the tensor core K-major for dK, MN-major for dQ)
 // 5 products and one exponential pass. dK and dV stay in TMEM for the whole key tile; the dQ partial of
-// every tile is added to an fp32 scratch (B,H,T,64) by a TMA bulk reduction (cp.reduce.async.bulk.tensor
+// every tile is added to an fp32 scratch (B,H,T,HD) by TMA bulk reductions (cp.reduce.async.bulk.tensor
 // .add, fp32 adds performed in L2 on whole 128-byte lines; the additions of different key tiles arrive in
 // no fixed order, so dQ is not bit-reproducible from run to run) and a bandwidth-bound kernel converts
 // the scratch to the output dtype afterwards. The delta kernel, which runs first anyway, zeroes the
-// scratch. The dQ tile is staged for the reduction in the shared-memory buffer its own dS^T came from,
-// which the products have finished reading by then.
+// scratch.
 //
-// Pipeline. P^T has its own TMEM columns and dS^T goes to shared memory, so the S^T / dP^T columns are free
-// again as soon as the compute warps have LOADED them. The tile's 128 query columns are two halves with
-// their own barriers throughout: warpgroups 0-1 own the first half, 2-3 the second, the S^T / dP^T products
-// of a half (N = 64) are issued as soon as that half's columns have been loaded, and dV and dK take a half's
-// 64 queries of their inner dimension as soon as that half's P^T / dS^T are written. The two pairs of
-// warpgroups therefore run as two pipelines that drift apart in time, and the accumulating products of a
-// tile run while the compute warps work on the next one. Every TMEM region is single-buffered (S^T 128 +
-// dP^T 128 + P^T 64 + dK 64 + dV 64 + dQ 64 = 512 columns); only dS^T in shared memory is double-buffered.
+// What bounds it. No single unit. Per tile at HD = 64 (cycles of an SM): products 1,540, exponentials 1,024, shared
+// memory 2,450 of its 128 bytes a cycle (1,408 of them the products' operands), instruction issue 1,350 of each
+// scheduler; a tile takes 3,150 with full lists. Taking any one of these out of the kernel changes it by 3 to 8 %.
+//  * Shared memory is kept free by the layout of the compute warps' registers: they read S^T and dP^T from TMEM in the
+//    16x256b shape, in which a thread owns four key rows and a quarter of the columns, as in an mma fragment, so that a
+//    warp needs LSE and delta of a column once and not 32 times; P^T goes back in the 16x128b shape and dS^T leaves
+//    through stmatrix without bank conflicts. Arithmetic on column pairs uses the packed f32x2 instructions.
+//  * The instruction cache: sixteen warps in six roles run different loops at the same time. With the waits' time-out
+//    code inlined and more unrolling this kernel was 120 KB and took 5,600 cycles a tile (a loop back-edge cost 580);
+//    at 75 KB the same schedule took 3,600. Loops of the issuing and dQ warps are therefore rolled where they can be.
+//  * The products are issued by whole warps with warp-uniform operands (mma_ss_uniform).
 //
-// Heads. A CTA handles several heads of its (batch, key tile) one after the other, and nothing drains between
-// them: the ring of Q / dO tiles runs on into the next head; K has two buffers (the next head's K is requested
-// a head ahead by the dK / dQ issuer, when the last dQ product of the head before has released the buffer) and
-// V one (requested by the S^T / dP^T issuer right after the head's last dP^T product, about a tile before the
-// head ends), so the next head's first products are issued while this head's last tile is still in the compute
-// warps; dK and dV of the finished head leave through the dQ warps, and only the next head's first
-// accumulating products wait for that.
+// Schedule at HD = 64. The compute warps form P^T of tile t and dS^T of tile t - 1 in one instruction stream (see there).
+//   warp 1   S^T(t), dP^T(t - 1) as soon as S^T(t - 1) and dP^T(t - 2) have been loaded; also requests the next item's V
+//   warp 3   dV += P^T(t) dO, a half of 64 queries at a time
+//   warp 2   dK += dS^T(t - 1) Q by halves, dQ(t - 1)
+// TMEM: S^T 128, dP^T 128, dV 64, dK 64, dQ 64, P^T 64 columns.
+// Schedule at HD = 128. S^T, dP^T, dV and dK fill TMEM, so P^T lies over the S^T it was made from and dQ takes the columns
+// of dP^T; the compute warps form P^T(t) while dQ(t - 1) is read out and dP^T(t) formed, then dS^T(t).
+//   warp 1   dV += P^T(t) dO, then S^T(t + 1) over P^T(t) (the tensor pipe executes in issue order)
+//   warp 2   dQ(t), dK += dS^T(t) Q; when dQ(t) has been read out, dP^T(t + 1); also requests the next item's K and V
 //
-// 768 threads: warp 0 producer (lane 0 issues the TMA loads of Q and dO; all lanes copy LSE, delta, token
-// descriptors and mask words of the stage's 128 queries to shared memory, so that compute warps find them
-// there and issue no global loads); warp 3 issues S^T and dP^T; warp 1 issues dV and warp 2 dK and dQ (24
-// products per tile from one thread would make that thread the slowest stage); warps 4-19 are four compute
-// warpgroups (32 query columns each, a key row per thread); warps 20-23 move finished dQ tiles from TMEM to
-// the scratch and write dK and dV at the end of each head.
+// Work items. An item is one (batch, head, key tile). The grid has a CTA per item, but a CTA that is running takes
+// further items by cancelling CTAs that have not been launched yet (clusterlaunchcontrol) and works on them without
+// draining its pipeline: the rings of Q and dO tiles run on into the next item, K has two buffers at HD = 64
+// (shared memory holds one at HD = 128), and dK and dV of the finished item leave through the dQ warps while the
+// next item's first products run. Starting a CTA costs some 12,000 cycles (launch, TMEM, first loads, pipeline fill,
+// drain), and a (batch, head, key tile) has around ten tiles.
+// Items are numbered in chunks of heads whose scratch and operands fit L2 together (FusedArgs::chunk), inside a
+// chunk by decreasing list length, so that the CTAs on the machine at one time add to dQ lines that stay in L2 and
+// the last items are short.
+//
+// 512 threads: warp 0 takes items and streams Q and dO (lane 0 issues the TMA loads; all lanes copy LSE, delta, token
+// descriptors and mask words of the tile's 128 queries to shared memory); warps 1-3 as above; warps 4-11 are two compute
+// warpgroups (64 query columns each); warps 12-15 move finished dQ tiles from TMEM to the scratch (each warp stages and
+// reduces its own 32 rows) and write dK and dV of finished items.
+//
+// Measured against the two forms before it (us, delta and conversion kernels included): a fused kernel with a row per
+// thread, sixteen compute warps and heads per CTA (HD = 64) and the two-kernel form (HD = 128):
+//   bf16 B16 H16 T4096 D64 hierarchical 1291 -> 1175-1230    bf16 B8 H16 T2048 D64 causal 338 -> 298
+//   bf16 B8 H16 T2048 D128 causal 644 -> 441                 fp16 B4 H32 T8192 D128 hierarchical 3944 -> 2540
 #include <algorithm>
+#include <type_traits>
 
 #include "attn_bwd.cuh"
 
 namespace kd {
 
+struct FusedArgs {
+  BwdArgs b;
+  int chunk;   // (batch, head) pairs per chunk of items
+};
+
+template <int HD_>
 struct FusedCfg {
-  static constexpr int HD = 64;
+  static constexpr int HD = HD_;
+  static constexpr int KBLK = HD / 64;               // 64-element blocks along D
   static constexpr int TILE_BYTES = KD_TILE * HD * 2;
-  static constexpr int STAGES = 3;                   // ring of streamed (Q, dO) tile pairs: a stage is held from its TMA load until
-                                                     // the tile's dV and dK products have completed, about two tile periods
-  // resident tiles of the CTA's key tile: K in two buffers (head hh in buffer hh % 2), V in one. V's last reader in a head
-  // is a dP^T product, issued about one tile before the head ends, so the next head's V lands in time without a second
-  // buffer; K's last reader is the head's last dQ product, so the next head's K has to be there already.
+  static constexpr int NK = (HD == 64) ? 2 : 1;      // K buffers (head hh in buffer hh % NK)
+  static constexpr int QS = (HD == 64) ? 4 : 2;      // ring stages of Q tiles: held from S^T of a tile to its dK
+  static constexpr int OS = (HD == 64) ? 2 : 1;      // ring stages of dO tiles: held from dP^T to dV
   static constexpr int SMEM_K = 0;
-  static constexpr int SMEM_V = SMEM_K + 2 * TILE_BYTES;
-  static constexpr int SMEM_RING = SMEM_V + TILE_BYTES;
-  static constexpr int SMEM_DS = SMEM_RING + STAGES * 2 * TILE_BYTES;   // 2 x dS^T of a query tile: two [128 keys][64 queries] blocks
-  // per ring stage, beside the tiles: LSE, delta and token descriptor of the stage's 128 queries and the 32 mask words of
-  // the query tile, copied there by the producer warp
-  static constexpr int SIDE_WORDS = 3 * KD_TILE + 32;
-  static constexpr int SMEM_SIDE = SMEM_DS + 2 * 2 * TILE_BYTES;
-  static constexpr int SMEM_LIST = SMEM_SIDE + STAGES * SIDE_WORDS * 4;
-  static constexpr int SMEM_TOTAL = SMEM_LIST + 128 * 2;
-  static constexpr int SMEM_ALLOC = SMEM_TOTAL + 1024;
-  static constexpr int THREADS = 768;
-  static constexpr uint32_t TM_S = 0, TM_DP = 128, TM_PT = 256, TM_DK = 320, TM_DV = 384, TM_DQ = 448;
-  static_assert(TM_DQ + HD <= 512, "TMEM budget");
+  static constexpr int SMEM_V = SMEM_K + NK * TILE_BYTES;
+  static constexpr int SMEM_Q = SMEM_V + TILE_BYTES;
+  static constexpr int SMEM_DO = SMEM_Q + QS * TILE_BYTES;
+  static constexpr int SMEM_DS = SMEM_DO + OS * TILE_BYTES;   // dS^T: two blocks [128 keys][64 queries]
+  static constexpr int SMEM_STG = SMEM_DS + 2 * 16384;        // dQ staging: per dQ warp two boxes [32 rows][32 floats]
+  // per Q stage: LSE and delta of the 128 queries, the 32 mask words of the query tile and its list entry (4 words with
+  // padding); HD = 64 also the queries' token descriptors (HD = 128 has no room: its compute warps fetch them)
+  static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + 32, SIDE_DESC = SIDE_ENT + 4;
+  static constexpr int SIDE_WORDS = (HD == 64) ? SIDE_DESC + KD_TILE : SIDE_DESC;
+  static constexpr int SMEM_SIDE = SMEM_STG + 4 * 2 * 4096;
+  static constexpr int NITEM = 4;                    // ring of item headers
+  static constexpr int SMEM_ITEM = SMEM_SIDE + QS * SIDE_WORDS * 4;   // NITEM x {batch, head, key tile | first entry << 16, entries}
+  static constexpr int SMEM_CLC = SMEM_ITEM + NITEM * 16;             // response of a cancellation
+  static constexpr int SMEM_BAR = SMEM_CLC + 16;
+  // barriers (8 bytes each)
+  static constexpr int NH = (HD == 64) ? 2 : 1;      // halves of 64 queries with barriers of their own
+  static constexpr int B_KFULL = 0, B_KEMPTY = B_KFULL + NK, B_VFULL = B_KEMPTY + NK, B_VEMPTY = B_VFULL + 1, B_QFULL = B_VEMPTY + 1,
+                       B_QEMPTY = B_QFULL + QS, B_DOFULL = B_QEMPTY + QS, B_DOEMPTY = B_DOFULL + OS, B_SFULL = B_DOEMPTY + OS,
+                       B_SFREE = B_SFULL + NH, B_PFULL = B_SFREE + NH, B_PFREE = B_PFULL + NH, B_DPFULL = B_PFREE + NH,
+                       B_DSFULL = B_DPFULL + 1, B_DSFREE = B_DSFULL + 1, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
+                       B_ACCFULL = B_DQEMPTY + 1, B_ACCFREE = B_ACCFULL + 1, B_ITEMFULL = B_ACCFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
+                       B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;
+  static constexpr int ITEM_READERS = (HD == 64) ? 15 : 14;   // warps that read item headers
+  static constexpr int SMEM_ALLOC = SMEM_BAR + NBAR * 8 + 16;   // + TMEM base, abort flag
+  static constexpr int THREADS = 512;
+  // TMEM columns
+  static constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = TM_DV + HD, TM_DQ = (HD == 64) ? TM_DK + HD : TM_DP,
+                            TM_P = (HD == 64) ? TM_DQ + HD : TM_S;
+  static constexpr uint32_t P_STRIDE = (HD == 64) ? 32 : 64;   // packed columns between the two warpgroups' P^T
+  static_assert(TM_DK + HD <= 512 && TM_DQ + HD <= 512 && TM_P + P_STRIDE + 32 <= 512, "TMEM budget");
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
-  // registers: 80 per thread at launch; light warps release down to 56, the dQ warps to 72, compute warps take 88
-  static constexpr int REGS_LIGHT = 56, REGS_DQ = 72, REGS_COMPUTE = 88;
-  static constexpr int REGS_LAUNCH = 80;             // per thread at launch: 6 warps per scheduler x 32 x 80 fit its 16384 registers
-  static_assert(4 * 32 * REGS_LIGHT + 4 * 32 * REGS_DQ + 16 * 32 * REGS_COMPUTE <= THREADS * REGS_LAUNCH, "register pool");
-  static_assert(THREADS == 768, "a 25th warp would put 7 warps on one scheduler and cut the launch count to 72 registers");
+  // registers: 128 per thread at launch; light warps release down to 80, the dQ warps to 96, compute warps take 168
+  static constexpr int REGS_LAUNCH = 128, REGS_LIGHT = (HD == 64) ? 88 : 72, REGS_DQ = (HD == 64) ? 56 : 120, REGS_COMPUTE = (HD == 64) ? 184 : 160;
+  static_assert(4 * 32 * REGS_LIGHT + 4 * 32 * REGS_DQ + 8 * 32 * REGS_COMPUTE <= THREADS * REGS_LAUNCH, "register pool");
 };
 
 enum : uint32_t {
-  W_U_FIXFULL = 0x401, W_U_RINGEMPTY = 0x402, W_U_RINGFULL = 0x403, W_U_PFULL = 0x404, W_U_SFULL = 0x405,
-  W_U_ACCFULL = 0x406, W_U_SPFREE = 0x407, W_U_FIXEMPTY = 0x408, W_U_ACCFREE = 0x409, W_U_DQFULL = 0x40A,
-  W_U_DQEMPTY = 0x40B, W_U_DSEMPTY = 0x40C, W_U_PTFREE = 0x40D, W_U_SFULL1 = 0x40E, W_U_SPFREE1 = 0x40F, W_U_VFULL = 0x410,
+  W_U_KFULL = 0x401, W_U_VFULL = 0x402, W_U_QFULL = 0x403, W_U_DOFULL = 0x404, W_U_QEMPTY = 0x405, W_U_DOEMPTY = 0x406, W_U_ITEMEMPTY = 0x407,
+  W_U_SFULL = 0x408, W_U_SFREE = 0x409, W_U_PFULL = 0x40A, W_U_PFREE = 0x40B, W_U_DPFULL = 0x40C, W_U_DSFULL = 0x40D,
+  W_U_DSFREE = 0x40E, W_U_DQFULL = 0x40F, W_U_DQEMPTY = 0x410, W_U_ACCFULL = 0x411, W_U_ACCFREE = 0x412, W_U_ALIGN = 0x413,
+  W_U_ITEMFULL = 0x414, W_U_CLC = 0x415, W_U_KEMPTY = 0x416, W_U_VEMPTY = 0x417,
 };
 
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-template <bool kBf16>
-__global__ void __launch_bounds__(FusedCfg::THREADS, 1)
+// Two consecutive floats as two 4-byte loads. The lanes of a warp read four such pairs, eight lanes each: as 8-byte loads that
+// took more than five shared-memory wavefronts, 690 of the 1,480 of a tile; a 4-byte load takes one.
+__device__ __forceinline__ uint64_t ld_shared_pair(const float* p) {
+  uint32_t lo, hi;
+  const uint32_t a = smem_u32(p);
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(lo) : "r"(a));
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(hi) : "r"(a + 4u));
+  return pack_u32x2(lo, hi);
+}
+
+template <int HD_, bool kBf16>
+__global__ void __launch_bounds__(FusedCfg<HD_>::THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                      const __grid_constant__ CUtensorMap tmAcc, const BwdArgs a) {
-  using C = FusedCfg;
-  constexpr int HD = C::HD;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t sK = smem_u32(smem + C::SMEM_K);        // K of head hh at + (hh % 2) TILE_BYTES
-  const uint32_t sV = smem_u32(smem + C::SMEM_V);
-  const uint32_t sRing = smem_u32(smem + C::SMEM_RING);  // stage s: Q at +0, dO at +TILE_BYTES
-  const uint32_t sDS = smem_u32(smem + C::SMEM_DS);      // buffer t: block 0 (queries 0-63) at +0, block 1 at +TILE_BYTES
-  uint32_t* sSide = reinterpret_cast<uint32_t*>(smem + C::SMEM_SIDE);
-  uint16_t* sList = reinterpret_cast<uint16_t*>(smem + C::SMEM_LIST);
+                      const __grid_constant__ CUtensorMap tmAcc, const __grid_constant__ CUtensorMap tmDK,
+                      const __grid_constant__ CUtensorMap tmDV, const FusedArgs fa) {
+  using C = FusedCfg<HD_>;
+  const BwdArgs& a = fa.b;
+  constexpr int HD = C::HD, TILE = C::TILE_BYTES;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t s0 = smem_u32(smem);
+  const uint32_t sK = s0 + C::SMEM_K, sV = s0 + C::SMEM_V, sQ = s0 + C::SMEM_Q, sDO = s0 + C::SMEM_DO, sDS = s0 + C::SMEM_DS;
+  int4* items = reinterpret_cast<int4*>(smem + C::SMEM_ITEM);
+  float* sSide = reinterpret_cast<float*>(smem + C::SMEM_SIDE);
+  uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + C::SMEM_BAR + C::NBAR * 8);
+  AbortFlag* abortf = reinterpret_cast<AbortFlag*>(tmem_base_s + 1);
+  auto bar = [&](int i) -> uint32_t { return s0 + C::SMEM_BAR + i * 8; };
 
-  __shared__ __align__(8) uint64_t bar_k_full[2], bar_k_empty[2], bar_v_full, bar_v_empty, bar_ring_full[C::STAGES],
-      bar_ring_empty[C::STAGES], bar_s_full[2], bar_sp_free[2], bar_p_full[2][2], bar_pt_free[2], bar_acc_full, bar_acc_free[2],
-      bar_dq_full, bar_dq_empty, bar_ds_empty[2];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ AbortFlag abortf;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h0 = blockIdx.x * a.G, b = blockIdx.y;
-  const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
-  const int kt = a.order[((size_t)b * 3 + 2) * a.NT + blockIdx.z];   // longest lists first
-  const int n = a.bwd_cnt[b * a.NT + kt];
-
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  if ((s0 & 1023u) != 0u) {   // the swizzled tiles need it; the launch asks for it, so this never happens
+    if (tid == 0) report_status(a.status, KD_DEV_TIMEOUT | W_U_ALIGN);
+    return;
+  }
   if (tid == 0) {
-    abortf.v = 0;
-    for (int f = 0; f < 2; ++f) {
-      mbar_init(smem_u32(&bar_k_full[f]), 1);
-      mbar_init(smem_u32(&bar_k_empty[f]), 1);   // the head's last dQ product has read K (its S^T products were issued, and so
-                                                 // completed, before it: the tensor pipe runs in issue order)
+    abortf->v = 0;
+    for (int i = 0; i < C::NBAR; ++i) {
+      uint32_t count = 1;
+      if (i >= C::B_QFULL && i < C::B_QEMPTY) count = 33;        // the TMA load and the producer lanes' own copies
+      if (i >= C::B_DOEMPTY && i < C::B_SFULL) count = 2;        // dP^T and dV have read the tile
+      if (i == C::B_DSFULL || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
+      if (i == C::B_DQEMPTY) count = 4;                          // one per dQ warp
+      if (i == C::B_ACCFULL) count = 2;                          // the head's last dV and dK
+      if (i == C::B_ACCFREE || i == C::B_ACCFREE + 1) count = 4; // dV, dK have been read out of TMEM
+      if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = C::ITEM_READERS;
+      mbar_init(bar(i), count);
     }
-    mbar_init(smem_u32(&bar_v_full), 1);
-    mbar_init(smem_u32(&bar_v_empty), 1);        // the head's last dP^T product has read V
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(smem_u32(&bar_ring_full[s]), 2);    // the TMA loads (with their byte count) and the producer warp's own copies
-      mbar_init(smem_u32(&bar_ring_empty[s]), 2);   // the dV issuer and the dK / dQ issuer are done with the stage
-    }
-    // S^T and dP^T are produced and released in two halves of 64 query columns
-    mbar_init(smem_u32(&bar_s_full[0]), 1);
-    mbar_init(smem_u32(&bar_s_full[1]), 1);
-    // the warps of a role arrive once each (lane 0, after a warp-wide sync): hundreds of single-thread arrivals on one
-    // barrier would serialise in the shared-memory atomic unit
-    // every barrier of a half is used by the two compute warpgroups (8 warps) that own the half
-    mbar_init(smem_u32(&bar_sp_free[0]), 8);   // the warps have loaded their S^T and dP^T columns
-    mbar_init(smem_u32(&bar_sp_free[1]), 8);
-    // P^T of the half is in TMEM and its dS^T block in shared memory. Two barriers per half, used by even and odd tiles: with
-    // two dS^T buffers the compute warps may finish two tiles before the dK / dQ issuer has looked at the first, and a parity
-    // wait on a single barrier cannot tell "two phases on" from "not yet"
-    for (int f = 0; f < 4; ++f) mbar_init(smem_u32(&bar_p_full[f >> 1][f & 1]), 8);
-    mbar_init(smem_u32(&bar_pt_free[0]), 1);   // the dV products have read the half's P^T
-    mbar_init(smem_u32(&bar_pt_free[1]), 1);
-    mbar_init(smem_u32(&bar_dq_full), 1);
-    mbar_init(smem_u32(&bar_dq_empty), 4);     // the dQ warps have read the dQ tile out of TMEM
-    mbar_init(smem_u32(&bar_ds_empty[0]), 1);  // a dS^T buffer is free: its products and the reduction staged in it are done
-    mbar_init(smem_u32(&bar_ds_empty[1]), 1);
-    mbar_init(smem_u32(&bar_acc_full), 2);       // both accumulating issuers have committed the head's last products
-    mbar_init(smem_u32(&bar_acc_free[0]), 4);  // the dQ warps have read dV out of TMEM
-    mbar_init(smem_u32(&bar_acc_free[1]), 4);  // ... and dK
     fence_barrier_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(tmem_base_s), 512);
     tmem_relinquish();
-  }
-  if (warp == 2) {
-    const uint16_t* glist = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
-    for (int e = lane; e < n; e += 32) sList[e] = glist[e];
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tbase = tmem_base_s;
-  const uint16_t* list = sList;
+  // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
+  auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
+  };
+  // two barriers of which both are complete as a rule: their tests overlap
+  auto wait2 = [&](int i, uint32_t pi, uint32_t site_i, int j, uint32_t pj, uint32_t site_j) -> bool {
+    const bool ri = mbar_try_wait(bar(i), pi), rj = mbar_try_wait(bar(j), pj);
+    if (__all_sync(0xffffffffu, ri && rj)) return true;
+    return wait(i, pi, site_i) && wait(j, pj, site_j);
+  };
+
+  // header of this CTA's k-th item with entries; entries < 0: there is none. The redux makes the fields warp-uniform for the compiler.
+  auto next_item = [&](int k, int4& it) -> bool {
+    const int slot = k % C::NITEM;
+    if (!wait(C::B_ITEMFULL + slot, (k / C::NITEM) & 1, W_U_ITEMFULL)) return false;
+    const int4 v = items[slot];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(C::B_ITEMEMPTY + slot));
+    it.x = __reduce_max_sync(0xffffffffu, v.x);
+    it.y = __reduce_max_sync(0xffffffffu, v.y);
+    it.z = __reduce_max_sync(0xffffffffu, v.z);
+    it.w = __reduce_max_sync(0xffffffffu, v.w);
+    return it.w >= 0;
+  };
+
+  // one thread: requests tile `tile` of (b, h); the barrier expects its bytes
+  auto load_tile = [&](const CUtensorMap* tm, uint32_t dst, int full, int tile, int h, int b) {
+    mbar_arrive_expect_tx(bar(full), TILE);
+    for (int kb = 0; kb < C::KBLK; ++kb) tma_load_4d(dst + kb * 16384, tm, bar(full), kb * 64, tile * KD_TILE, h, b);
+  };
 
   if (warp < 4) {
     reg_dealloc<C::REGS_LIGHT>();
-    if (warp == 0 && n > 0) {
+    if (warp == 0) {
       // ------------------------------ producer warp ------------------------------
-      // lane 0 issues the TMA loads; all lanes copy the per-query scalars of the stage (4 queries each) and the tile's
-      // mask words (one each) with plain loads, so that the compute warps find everything about a tile in shared memory
       if (lane == 0) {
         tma_prefetch_desc(&tmQ);
+        tma_prefetch_desc(&tmDO);
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
-        tma_prefetch_desc(&tmDO);
       }
-      int issued = 0;   // ring entries requested so far, over all heads
-      bool ok = true;
-      if (lane == 0) {
-        // K and V of the first head and K of the second; later heads' tiles are requested by the issuing threads that see
-        // the buffers fall free (the dK / dQ issuer for K, the S^T / dP^T issuer for V)
-        mbar_arrive_expect_tx(smem_u32(&bar_k_full[0]), C::TILE_BYTES);
-        tma_load_4d(sK, &tmK, smem_u32(&bar_k_full[0]), 0, kt * KD_TILE, h0, b);
-        mbar_arrive_expect_tx(smem_u32(&bar_v_full), C::TILE_BYTES);
-        tma_load_4d(sV, &tmV, smem_u32(&bar_v_full), 0, kt * KD_TILE, h0, b);
-        if (nh > 1) {
-          mbar_arrive_expect_tx(smem_u32(&bar_k_full[1]), C::TILE_BYTES);
-          tma_load_4d(sK + C::TILE_BYTES, &tmK, smem_u32(&bar_k_full[1]), 0, kt * KD_TILE, h0 + 1, b);
+      int q_tiles = 0, do_tiles = 0, k_loads = 0, k = 0;   // Q / dO / K tiles requested and items published so far
+      bool ok = true, pending = false;
+      // decodes item number `idx` of the launch
+      auto decode = [&](int idx) -> int4 {
+        const int per_chunk = fa.chunk * a.NT;
+        const int c = idx / per_chunk, rem = idx - c * per_chunk;
+        const int heads = min(fa.chunk, a.B * a.H - c * fa.chunk);   // (batch, head) pairs of this chunk
+        const int rank = rem / heads, bh = c * fa.chunk + (rem - rank * heads);
+        int4 it;
+        it.x = bh / a.H;
+        it.y = bh - it.x * a.H;
+        const int kt = a.order[((size_t)it.x * 3 + 2) * a.NT + rank];   // longest lists first
+        it.w = a.bwd_cnt[it.x * a.NT + kt];
+        it.z = kt | (static_cast<int>(a.bwd_list[((size_t)it.x * a.NT + kt) * a.NT]) << 16);
+        return it;
+      };
+      int asked = 0;   // cancellations asked for
+      auto ask = [&]() {   // for the item after the one in hand
+        if (lane == 0) {
+          fence_proxy_async_smem();   // the previous response has been read
+          mbar_arrive_expect_tx(bar(C::B_CLC), 16);
+          clc_try_cancel(s0 + C::SMEM_CLC, bar(C::B_CLC));
         }
+        ++asked;
+        pending = true;
+      };
+      // dK = dV = 0 for an item without entries: no other warp hears of it
+      auto write_zeros = [&](const int4& z) {
+        const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0), cpr = a.d_real / 8;   // 16-byte chunks of a row
+        uint16_t* dk = reinterpret_cast<uint16_t*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
+        uint16_t* dv = reinterpret_cast<uint16_t*>(a.dv) + (size_t)z.x * a.dv_sb + (size_t)z.y * a.dv_sh;
+        for (int i = lane; i < rows * cpr; i += 32) {
+          const int r = i / cpr, c = (i - r * cpr) * 8;
+          *reinterpret_cast<uint4*>(dk + (size_t)(row0 + r) * a.dk_st + c) = make_uint4(0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(dv + (size_t)(row0 + r) * a.dv_st + c) = make_uint4(0u, 0u, 0u, 0u);
+        }
+      };
+      // the next item that has entries (nx.w < 0: there is none); its successor has been asked for
+      auto take_next = [&](int4& nx) -> bool {
+        while (true) {
+          if (!wait(C::B_CLC, (asked - 1) & 1, W_U_CLC)) return false;
+          pending = false;
+          const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
+          if (idx < 0) {
+            nx.w = -1;
+            return true;
+          }
+          nx = decode(idx);
+          ask();
+          if (nx.w > 0) return true;
+          write_zeros(nx);
+        }
+      };
+      int4 it = decode(blockIdx.x);
+      ask();
+      if (it.w == 0) {
+        write_zeros(it);
+        ok = take_next(it);
       }
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const int h = h0 + hh;
-        const float* lse_row = a.lse + ((size_t)b * a.H + h) * a.T;
-        const float* delta_row = a.delta + ((size_t)b * a.H + h) * a.T;
+      int qs = 0, os = 0;
+      uint32_t q_parity = 1u, do_parity = 1u;   // of the stages' "empty" phases
+      while (ok) {
+        const int slot = k % C::NITEM;
+        if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_U_ITEMEMPTY))) break;
+        if (lane == 0) {
+          items[slot] = it;
+          mbar_arrive(bar(C::B_ITEMFULL + slot));
+        }
+        __syncwarp();
+        if (it.w < 0) break;
+        const int b = it.x, h = it.y, kt = it.z & 0xFFFF, n = it.w;
+        // K into the buffer of the item before the last (HD = 64; at HD = 128 the issuing warps request K as well as V)
+        if (HD == 64 || k == 0) {
+          if (!(ok = wait(C::B_KEMPTY + k % C::NK, ((k / C::NK) & 1) ^ 1, W_U_KEMPTY))) break;
+          if (lane == 0) load_tile(&tmK, sK + (k % C::NK) * TILE, C::B_KFULL + k % C::NK, kt, h, b);
+          ++k_loads;
+        }
+        if (k == 0 && lane == 0) load_tile(&tmV, sV, C::B_VFULL, kt, h, b);
+        ++k;
+        const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
+        const size_t row = ((size_t)b * a.H + h) * a.T;
+        const bool aligned = (row & 3) == 0;
+        uint32_t ent = static_cast<uint32_t>(it.z) >> 16;
+        int4 nx = it;
+#pragma unroll 1
         for (int e = 0; e < n; ++e) {
-          const int s = issued % C::STAGES;
-          const uint32_t ph = (issued / C::STAGES) & 1;
-          const int qt = list[e] & 0xFF;
-          // the scalars are requested before the wait for the stage: the wait covers their latency
-          // (a query at or beyond the sequence length reads the last row's scalars: its descriptor is 0, so the tile is
-          // PARTIAL and the mask removes it)
-          const int q = qt * KD_TILE + 4 * lane;
-          float4 l4, d4;
-          l4.x = lse_row[min(q + 0, a.T - 1)]; l4.y = lse_row[min(q + 1, a.T - 1)];
-          l4.z = lse_row[min(q + 2, a.T - 1)]; l4.w = lse_row[min(q + 3, a.T - 1)];
-          d4.x = delta_row[min(q + 0, a.T - 1)]; d4.y = delta_row[min(q + 1, a.T - 1)];
-          d4.z = delta_row[min(q + 2, a.T - 1)]; d4.w = delta_row[min(q + 3, a.T - 1)];
+          const uint32_t this_ent = ent;
+          if (e + 1 < n) ent = list[e + 1];
+          const int qt = this_ent & 0xFF;
+          if (!(ok = wait(C::B_QEMPTY + qs, q_parity, W_U_QEMPTY))) break;
+          const uint32_t side = s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4);
           if (lane == 0) {
-            ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, a.status, W_U_RINGEMPTY);
-            if (ok) {
-              mbar_arrive_expect_tx(smem_u32(&bar_ring_full[s]), 2 * C::TILE_BYTES);
-              const uint32_t dst = sRing + s * 2 * C::TILE_BYTES;
-              tma_load_4d(dst, &tmQ, smem_u32(&bar_ring_full[s]), 0, qt * KD_TILE, h, b);
-              tma_load_4d(dst + C::TILE_BYTES, &tmDO, smem_u32(&bar_ring_full[s]), 0, qt * KD_TILE, h, b);
+            st_shared_u32(side + C::SIDE_ENT * 4, this_ent);   // published by the arrival that goes with the load
+            load_tile(&tmQ, sQ + qs * TILE, C::B_QFULL + qs, qt, h, b);
+          }
+          // the scalars of four queries and one mask word per lane, copied asynchronously: the barrier counts the lanes' copies
+          // (a query at or beyond the sequence length takes the last row's scalars: its descriptor is 0, so the tile is PARTIAL
+          // and the mask removes it)
+          const int q = qt * KD_TILE + 4 * lane;
+          if (aligned && q + 3 < a.T) {
+            cp_async16(side + 16 * lane, a.lse + row + q);
+            cp_async16(side + KD_TILE * 4 + 16 * lane, a.delta + row + q);
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j) {
+              const size_t r = row + min(q + j, a.T - 1);
+              cp_async4(side + 16 * lane + 4 * j, a.lse + r);
+              cp_async4(side + KD_TILE * 4 + 16 * lane + 4 * j, a.delta + r);
             }
           }
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) break;
-          // (descriptors and mask words are fetched after the wait: held across it they would not fit this warp's registers)
-          const uint4 c4 = *reinterpret_cast<const uint4*>(a.desc + (size_t)b * a.Tpad + q);   // the descriptor rows are padded to whole tiles
-          const uint32_t tbw = a.tilebits[((size_t)b * a.NT + qt) * 32 + lane];
-          uint32_t* side = sSide + s * C::SIDE_WORDS;
-          *reinterpret_cast<float4*>(side + 4 * lane) = l4;
-          *reinterpret_cast<float4*>(side + KD_TILE + 4 * lane) = d4;
-          *reinterpret_cast<uint4*>(side + 2 * KD_TILE + 4 * lane) = c4;
-          side[3 * KD_TILE + lane] = tbw;
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&bar_ring_full[s]));
-          ++issued;
+          cp_async4(side + (C::SIDE_BITS + lane) * 4, a.tilebits + ((size_t)b * a.NT + qt) * 32 + lane);
+          if constexpr (HD == 64) cp_async16(side + C::SIDE_DESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + q);   // padded to whole tiles
+          cp_async_mbar_arrive(bar(C::B_QFULL + qs));
+          ++q_tiles;
+          if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
+          if (!(ok = wait(C::B_DOEMPTY + os, do_parity, W_U_DOEMPTY))) break;
+          if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, qt, h, b);
+          ++do_tiles;
+          if (++os == C::OS) { os = 0; do_parity ^= 1u; }
+          if (e == 0 && !(ok = take_next(nx))) break;
         }
+        it = nx;
       }
-      if (lane == 0 && abortf.v != 0) {   // let the copies in flight land before the CTA exits
-        for (int e = max(0, issued - C::STAGES); e < issued; ++e) drain_wait(smem_u32(&bar_ring_full[e % C::STAGES]), (e / C::STAGES) & 1);
-        drain_wait(smem_u32(&bar_k_full[0]), 0);
-        drain_wait(smem_u32(&bar_v_full), 0);
-        if (nh > 1) drain_wait(smem_u32(&bar_k_full[1]), 0);
+      if (lane == 0 && abortf->v != 0) {   // let the copies in flight land before the CTA exits
+        for (int f = max(0, k_loads - C::NK); f < k_loads; ++f) drain_wait(bar(C::B_KFULL + f % C::NK), (f / C::NK) & 1);
+        if (k > 0) drain_wait(bar(C::B_VFULL), 0);
+        for (int f = max(0, q_tiles - C::QS); f < q_tiles; ++f) drain_wait(bar(C::B_QFULL + f % C::QS), (f / C::QS) & 1);
+        for (int f = max(0, do_tiles - C::OS); f < do_tiles; ++f) drain_wait(bar(C::B_DOFULL + f % C::OS), (f / C::OS) & 1);
+        if (pending) drain_wait(bar(C::B_CLC), (asked - 1) & 1);
       }
-    } else if (warp == 3 && lane == 0 && n > 0) {
-      // ------- M1 issuer: per half of 64 queries, S^T = K Q^T and dP^T = V dO^T into columns 64 half .. 64 half + 63 -------
-      const uint32_t idesc_m1 = make_idesc_f16(kBf16, 0, 0, KD_TILE, KD_TILE / 2);
+    } else {
+      // ------------------------------ issuing warps ------------------------------
+      // All lanes follow the control flow and one elected lane issues (mma_ss_uniform).
       const uint32_t hi = desc_hi_sw128();
-      const uint32_t loRingK = desc_lo_kmajor(sRing);
+      const uint32_t idesc_s = make_idesc_f16(kBf16, 0, 0, KD_TILE, KD_TILE);   // S^T, dP^T (of a half)
+      const uint32_t idesc_dv = make_idesc_f16(kBf16, 0, 1, KD_TILE, a.d_real);      // dV, dK: B = dO / Q rows, MN-major
+      const uint32_t idesc_dq = make_idesc_f16(kBf16, 1, 1, KD_TILE, a.d_real);      // A = dS^T read MN-major (M = queries)
+      const uint32_t lo_k0 = desc_lo_kmajor(sK), lo_v = desc_lo_kmajor(sV), lo_q0 = desc_lo_kmajor(sQ), lo_do0 = desc_lo_kmajor(sDO);
+      const uint32_t k_mn0 = desc_lo_mnmajor(sK), q_mn0 = desc_lo_mnmajor(sQ), do_mn0 = desc_lo_mnmajor(sDO);
+      const uint32_t ds_k = desc_lo_kmajor(sDS), ds_mn = desc_lo_mnmajor(sDS);
+      constexpr uint32_t T16 = TILE >> 4;
       bool ok = true;
-      int t = 0, stage = 0;   // tiles so far and ring stage, running on across the heads
-      uint32_t ring_parity = 0;
-      int v_loads = 1;        // V tiles requested so far (the first by the producer)
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        ok = mbar_wait(smem_u32(&bar_k_full[hh & 1]), (hh >> 1) & 1, &abortf, a.status, W_U_FIXFULL);
-        if (!ok) break;
-        const uint32_t loK = desc_lo_kmajor(sK + (hh & 1) * C::TILE_BYTES), loV = desc_lo_kmajor(sV);
-        bool v_ready = false;
-        for (int e = 0; e < n && ok; ++e) {
+      int4 it;
+      int k = 0, m = 0, t = 0;   // headers read; current item; tiles so far
+      bool have = false;
+      auto advance = [&]() { have = next_item(k++, it); };
+      auto product_kmajor = [&](uint32_t d, uint32_t a_lo, uint32_t b_lo) {   // d = A B^T over the head dim
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            // rows 64 half .. of the stage's Q and dO tiles (128 bytes per row)
-            const uint32_t qlo = loRingK + stage * (2 * C::TILE_BYTES >> 4) + half * (C::TILE_BYTES >> 5), dolo = qlo + (C::TILE_BYTES >> 4);
-            const uint32_t tS = tbase + C::TM_S + half * 64, tDP = tbase + C::TM_DP + half * 64;
-            if (t > 0) {   // the compute warps must have loaded the previous tile's columns of this half
-              ok = mbar_wait(smem_u32(&bar_sp_free[half]), (t - 1) & 1, &abortf, a.status, half ? W_U_SPFREE1 : W_U_SPFREE);
-              if (!ok) break;
+        for (int kk = 0; kk < HD / 16; ++kk)
+          mma_ss_uniform(d, a_lo + koff_kmajor(kk), b_lo + koff_kmajor(kk), hi, idesc_s, kk > 0 ? 1u : 0u);
+      };
+      auto product_dv = [&](int w, uint32_t do_mn, bool first) {   // dV += P^T dO over queries 64 w .. 64 w + 63
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          mma_ts_uniform(C::TM_DV, C::TM_P + w * C::P_STRIDE + kk * 8, do_mn + w * koff_mnmajor(4) + koff_mnmajor(kk), hi, idesc_dv, (kk > 0 || !first) ? 1u : 0u);
+      };
+      auto product_dk = [&](int w, uint32_t q_mn, bool first) {    // dK += dS^T Q over the same
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          mma_ss_uniform(C::TM_DK, ds_k + w * koff_kmajor(4) + koff_kmajor(kk), q_mn + w * koff_mnmajor(4) + koff_mnmajor(kk), hi, idesc_dv, (kk > 0 || !first) ? 1u : 0u);
+      };
+      auto product_dq = [&](uint32_t k_mn) {                                  // dQ = dS K
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) mma_ss_uniform(C::TM_DQ, ds_mn + koff_mnmajor(kk), k_mn + koff_mnmajor(kk), hi, idesc_dq, kk > 0 ? 1u : 0u);
+      };
+      if constexpr (HD == 64) {
+        if (warp == 1) {
+          // ---- S^T(t) and dP^T(t - 1), a half at a time, as soon as the half's S^T(t - 1) and dP^T(t - 2) have been loaded ----
+          int q_stage = 0, do_stage = 0;
+          uint32_t q_parity = 0, do_parity = 0;
+          advance();
+          bool p_first = false, p_last = false;   // tile t - 1 is its item's first / last
+          int e = 0, v_loads = 1;
+          while (ok) {
+            const bool s_there = have, dp_there = t > 0;
+            if (!s_there && !dp_there) break;
+            const bool last = e == it.w - 1;
+            if (s_there) {
+              if (e == 0 && !(ok = wait(C::B_KFULL + (m & 1), (m >> 1) & 1, W_U_KFULL))) break;
+              if (!(ok = wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL))) break;
             }
-            if (half == 0) {
-              ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, a.status, W_U_RINGFULL);
+            if (dp_there) {   // V of tile t - 1's item: waited for at the item's first dP^T
+              if (p_first && !(ok = wait(C::B_VFULL, ((s_there && e > 0) ? m : m - 1) & 1, W_U_VFULL))) break;
+              if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
+            }
+            if (dp_there && !(ok = wait2(C::B_SFREE, (t - 1) & 1, W_U_SFREE, C::B_SFREE + 1, (t - 1) & 1, W_U_SFREE))) break;
+            tc_fence_after_sync();
+            if (s_there) product_kmajor(C::TM_S, lo_k0 + (m & 1) * T16, lo_q0 + q_stage * T16);
+            if (dp_there) product_kmajor(C::TM_DP, lo_v, lo_do0 + do_stage * T16);
+            commit_uniform(bar(C::B_SFULL));
+            commit_uniform(bar(C::B_SFULL + 1));
+            if (dp_there) {
+              commit_uniform(bar(C::B_DOEMPTY + do_stage));
+              if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
+            }
+            if (!s_there) break;   // that was the last dP^T
+            if (dp_there && p_last) {
+              // That was V's last reader in its item: the next item's V goes into the same buffer. This warp has nothing else to
+              // do before the next S^T can be formed, and the load has an iteration to land.
+              commit_uniform(bar(C::B_VEMPTY));
+              if (!(ok = wait(C::B_VEMPTY, (m - 1) & 1, W_U_VEMPTY))) break;
+              if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
+              v_loads = m + 1;
+            }
+            if (++q_stage == C::QS) { q_stage = 0; q_parity ^= 1u; }
+            p_first = e == 0;
+            p_last = last;
+            ++t;
+            ++e;
+            if (last) {
+              advance();
+              ++m;
+              e = 0;
+            }
+          }
+          if (lane == 0 && abortf->v != 0 && v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
+        } else if (warp == 3) {
+          // ---- dV, a half at a time ----
+          int do_stage = 0;
+          uint32_t do_parity = 0;
+          advance();
+          while (have && ok) {
+            const int n = it.w;
+            for (int e = 0; e < n && ok; ++e, ++t) {
+              if (e == 0 && m > 0 && !(ok = wait(C::B_ACCFREE, (m - 1) & 1, W_U_ACCFREE))) break;
+              if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;   // P^T does not imply it
+#pragma unroll 1
+              for (int w = 0; w < 2; ++w) {
+                if (!(ok = wait(C::B_PFULL + w, t & 1, W_U_PFULL))) break;
+                tc_fence_after_sync();
+                product_dv(w, do_mn0 + do_stage * T16, e == 0 && w == 0);
+                commit_uniform(bar(C::B_PFREE + w));
+              }
               if (!ok) break;
+              commit_uniform(bar(C::B_DOEMPTY + do_stage));
+              if (e == n - 1) commit_uniform(bar(C::B_ACCFULL));
+              if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
+            }
+            ++m;
+            if (ok) advance();
+          }
+        } else {
+          // ---- dK(t - 1), a half at a time, and dQ(t - 1), as dS^T(t - 1) is written in the compute warps' iteration t ----
+          int q_stage = 0;
+          bool first = false, last = false;   // of tile t - 1
+          auto accumulate = [&](int item) -> bool {
+            if (first && item > 0 && !wait(C::B_ACCFREE + 1, (item - 1) & 1, W_U_ACCFREE)) return false;
+#pragma unroll 1
+            for (int w = 0; w < 2; ++w) {
+              if (!wait(C::B_PFULL + w, t & 1, W_U_PFULL)) return false;
+              tc_fence_after_sync();
+              product_dk(w, q_mn0 + q_stage * T16, first && w == 0);
+            }
+            if (t > 1 && !wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY)) return false;
+            tc_fence_after_sync();
+            product_dq(k_mn0 + (item & 1) * T16);
+            commit_uniform(bar(C::B_DQFULL));
+            commit_uniform(bar(C::B_DSFREE));
+            commit_uniform(bar(C::B_QEMPTY + q_stage));
+            if (last) {
+              commit_uniform(bar(C::B_ACCFULL));
+              commit_uniform(bar(C::B_KEMPTY + (item & 1)));
+            }
+            if (++q_stage == C::QS) q_stage = 0;
+            return true;
+          };
+          int e = 0;
+          advance();
+          while (have || t > 0) {
+            if (t == 0) {
+              if (!(ok = wait(C::B_PFULL, 0, W_U_PFULL) && wait(C::B_PFULL + 1, 0, W_U_PFULL))) break;
+            } else if (!(ok = accumulate((have && e > 0) ? m : m - 1))) {
+              break;
+            }
+            if (!have) break;   // that was the last tile
+            first = e == 0;
+            last = e == it.w - 1;
+            ++t;
+            ++e;
+            if (last) {
+              advance();
+              ++m;
+              e = 0;
+            }
+          }
+        }
+      } else if (warp == 1) {
+        // ---- issuing warp A: S^T and dV ----
+        int q_stage = 0, do_stage = 0;
+        uint32_t q_parity = 0, do_parity = 0;
+        auto issue_s = [&]() {
+          tc_fence_after_sync();
+          product_kmajor(C::TM_S, lo_k0, lo_q0 + q_stage * T16);
+          commit_uniform(bar(C::B_SFULL));
+          if (++q_stage == C::QS) { q_stage = 0; q_parity ^= 1u; }
+        };
+        advance();
+        if (have && (ok = wait(C::B_KFULL, 0, W_U_KFULL) && wait(C::B_QFULL, 0, W_U_QFULL))) issue_s();
+        while (have && ok) {
+          const int n = it.w;
+          for (int e = 0; e < n; ++e, ++t) {
+            const bool last = (e == n - 1);
+            if (e == 0 && m > 0 && !(ok = wait(C::B_ACCFREE, (m - 1) & 1, W_U_ACCFREE))) break;
+            // (P^T does not imply that dO has landed)
+            if (!(ok = wait2(C::B_PFULL, t & 1, W_U_PFULL, C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
+            tc_fence_after_sync();
+#pragma unroll 1
+            for (int w = 0; w < 2; ++w) product_dv(w, do_mn0 + do_stage * T16, e == 0 && w == 0);
+            commit_uniform(bar(C::B_DOEMPTY + do_stage));
+            if (last) commit_uniform(bar(C::B_ACCFULL));
+            if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
+            if (last) advance();
+            if (have) {   // S^T of the next tile over P^T, whose reader precedes it in the pipe
+              if (last && !(ok = wait(C::B_KFULL, (m + 1) & 1, W_U_KFULL))) break;
+              if (!(ok = wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL))) break;
+              issue_s();
+            }
+          }
+          ++m;
+        }
+      } else if (warp == 2) {
+        // ---- issuing warp B: dP^T, dK and dQ ----
+        int q_stage = 0, do_stage = 0, k_loads = 1, v_loads = 1;
+        uint32_t do_parity = 0;
+        auto issue_dp = [&]() {
+          tc_fence_after_sync();
+          product_kmajor(C::TM_DP, lo_v, lo_do0 + do_stage * T16);
+          commit_uniform(bar(C::B_DPFULL));
+          commit_uniform(bar(C::B_DOEMPTY + do_stage));
+          if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
+        };
+        advance();
+        if (have && (ok = wait(C::B_VFULL, 0, W_U_VFULL) && wait(C::B_DOFULL, 0, W_U_DOFULL))) issue_dp();
+        while (have && ok) {
+          const int n = it.w;
+          for (int e = 0; e < n; ++e, ++t) {
+            const bool last = (e == n - 1);
+            if (e == 0 && m > 0 && !(ok = wait(C::B_ACCFREE + 1, (m - 1) & 1, W_U_ACCFREE))) break;
+            if (!(ok = wait(C::B_DSFULL, t & 1, W_U_DSFULL))) break;
+            // V's last reader in this item, dP^T(t), is done: the next item's V goes into the same buffer, before the products
+            // below if that item is known
+            bool v_asked = false;
+            if (last && __all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) {
+              advance();
+              v_asked = true;
+              if (have) {
+                if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
+                ++v_loads;
+              }
             }
             tc_fence_after_sync();
-            mma_ss64<false>(tS, desc64(loK, hi), desc64(qlo, hi), idesc_m1);
-#pragma unroll
-            for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(tS, desc64(loK + koff_kmajor(kk), hi), desc64(qlo + koff_kmajor(kk), hi), idesc_m1);
-            if (!v_ready) {   // the head's V is requested late (below), so it is waited for only where it is first needed
-              ok = mbar_wait(smem_u32(&bar_v_full), hh & 1, &abortf, a.status, W_U_VFULL);
-              if (!ok) break;
-              v_ready = true;
+            product_dq(k_mn0);   // over dP^T(t), which dS^T(t) was made from
+            commit_uniform(bar(C::B_DQFULL));
+#pragma unroll 1
+            for (int w = 0; w < 2; ++w) product_dk(w, q_mn0 + q_stage * T16, e == 0 && w == 0);
+            commit_uniform(bar(C::B_DSFREE));
+            commit_uniform(bar(C::B_QEMPTY + q_stage));
+            if (++q_stage == C::QS) q_stage = 0;
+            if (last) {
+              commit_uniform(bar(C::B_ACCFULL));
+              if (!v_asked) {
+                advance();
+                if (have) {
+                  if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
+                  ++v_loads;
+                }
+              }
+              if (have) {   // one K buffer: the next item's K can only be requested when the products above are done
+                if (!(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
+                if (elect_one()) load_tile(&tmK, sK, C::B_KFULL, it.z & 0xFFFF, it.y, it.x);
+                ++k_loads;
+              }
             }
-            mma_ss64<false>(tDP, desc64(loV, hi), desc64(dolo, hi), idesc_m1);
-#pragma unroll
-            for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(tDP, desc64(loV + koff_kmajor(kk), hi), desc64(dolo + koff_kmajor(kk), hi), idesc_m1);
-            mma_commit(smem_u32(&bar_s_full[half]));
-          }
-          ++t;
-          if (++stage == C::STAGES) { stage = 0; ring_parity ^= 1; }
-        }
-        if (!ok) break;
-        mma_commit(smem_u32(&bar_v_empty));           // the head's dP^T products no longer read V
-        if (hh + 1 < nh) {
-          // The next head's V goes into the same buffer: this thread waits for its own last products (a few hundred cycles,
-          // during which it has nothing else to issue: the next S^T needs columns the compute warps are still reading)
-          // and requests the tile.
-          ok = mbar_wait(smem_u32(&bar_v_empty), hh & 1, &abortf, a.status, W_U_FIXEMPTY);
-          if (!ok) break;
-          mbar_arrive_expect_tx(smem_u32(&bar_v_full), C::TILE_BYTES);
-          tma_load_4d(sV, &tmV, smem_u32(&bar_v_full), 0, kt * KD_TILE, h0 + hh + 1, b);
-          v_loads = hh + 2;
-        }
-      }
-      if (abortf.v != 0 && v_loads > 1) drain_wait(smem_u32(&bar_v_full), (v_loads - 1) & 1);   // let a copy in flight land
-    } else if (warp == 1 && lane == 0 && n > 0) {
-      // ------- dV issuer: per tile dV += P^T dO (A from TMEM) -------
-      const uint32_t idesc_dv = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);   // B = dO rows, MN-major
-      const uint32_t tDV = tbase + C::TM_DV, tPT = tbase + C::TM_PT;
-      const uint32_t hi = desc_hi_sw128();
-      const uint32_t loRingMN = desc_lo_mnmajor(sRing);
-      bool ok = true;
-      int t = 0, stage = 0;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        if (hh > 0) {   // the previous head's dK and dV must have been read out of the accumulators
-          ok = mbar_wait(smem_u32(&bar_acc_free[0]), (hh - 1) & 1, &abortf, a.status, W_U_ACCFREE);
-          if (!ok) break;
-        }
-        for (int e = 0; e < n && ok; ++e) {
-          const uint32_t dob = loRingMN + stage * (2 * C::TILE_BYTES >> 4) + (C::TILE_BYTES >> 4);
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {   // 64 queries of the product's inner dimension at a time
-            ok = mbar_wait(smem_u32(&bar_p_full[half][t & 1]), (t >> 1) & 1, &abortf, a.status, W_U_PFULL);
-            if (!ok) break;
-            tc_fence_after_sync();
-#pragma unroll
-            for (int kk = 4 * half; kk < 4 * half + 4; ++kk)
-              mma_ts_split(tDV, tPT + kk * 8, dob + koff_mnmajor(kk), hi, idesc_dv, (e > 0 || kk > 0) ? 1u : 0u);
-            if (half == 0 && t >= 1) {
-              // bar_pt_free of tile t also tells the compute warps that the dS^T buffer of tile t + 1 is free, i.e. that the
-              // dK / dQ products and the dQ reduction of tile t - 1 are done with it (normally long before this point)
-              ok = mbar_wait(smem_u32(&bar_ds_empty[(t + 1) & 1]), ((t - 1) >> 1) & 1, &abortf, a.status, W_U_DSEMPTY);
-              if (!ok) break;
+            if (have) {
+              if (!(ok = wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY))) break;
+              if (last && !(ok = wait(C::B_VFULL, (m + 1) & 1, W_U_VFULL))) break;
+              if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
+              issue_dp();
             }
-            mma_commit(smem_u32(&bar_pt_free[half]));
           }
-          if (!ok) break;
-          mma_commit(smem_u32(&bar_ring_empty[stage]));   // one of two: dO of the stage is no longer read
-          ++t;
-          if (++stage == C::STAGES) stage = 0;
+          ++m;
         }
-        if (ok) mma_commit(smem_u32(&bar_acc_full));
-      }
-    } else if (warp == 2 && lane == 0 && n > 0) {
-      // ------- dK / dQ issuer: per tile dK += dS^T Q and dQ_tile = dS K (A = dS^T from shared memory) -------
-      const uint32_t idesc_dk = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);   // A = dS^T rows (keys) K-major, B = Q rows, MN-major
-      const uint32_t idesc_dq = make_idesc_f16(kBf16, 1, 1, KD_TILE, HD);   // A = dS^T read MN-major (M = queries), B = K rows, MN-major
-      const uint32_t tDK = tbase + C::TM_DK, tDQ = tbase + C::TM_DQ;
-      const uint32_t hi = desc_hi_sw128();
-      const uint32_t loRingMN = desc_lo_mnmajor(sRing);
-      bool ok = true;
-      int t = 0, stage = 0;
-      int k_loads = 2;   // K tiles requested so far (the first two by the producer)
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const uint32_t loK = desc_lo_mnmajor(sK + (hh & 1) * C::TILE_BYTES);
-        ok = mbar_wait(smem_u32(&bar_k_full[hh & 1]), (hh >> 1) & 1, &abortf, a.status, W_U_FIXFULL);
-        if (!ok) break;
-        if (hh > 0) {
-          ok = mbar_wait(smem_u32(&bar_acc_free[1]), (hh - 1) & 1, &abortf, a.status, W_U_ACCFREE);
-          if (!ok) break;
+        if (lane == 0 && abortf->v != 0) {   // let this warp's own copies in flight land before the CTA exits
+          if (k_loads > 1) drain_wait(bar(C::B_KFULL), (k_loads - 1) & 1);
+          if (v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
         }
-        for (int e = 0; e < n && ok; ++e) {
-          const int tb = t & 1;
-          const uint32_t qb = loRingMN + stage * (2 * C::TILE_BYTES >> 4);
-          const uint32_t dsK = desc_lo_kmajor(sDS + tb * (2 * C::TILE_BYTES));     // dS^T as [keys][queries]: K-major A of dK
-          const uint32_t dsMN = desc_lo_mnmajor(sDS + tb * (2 * C::TILE_BYTES));   // the same bytes as MN-major A of dQ
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            ok = mbar_wait(smem_u32(&bar_p_full[half][t & 1]), (t >> 1) & 1, &abortf, a.status, W_U_PFULL);
-            if (!ok) break;
-            tc_fence_after_sync();
-#pragma unroll
-            for (int kk = 4 * half; kk < 4 * half + 4; ++kk)
-              mma_ss_split(tDK, dsK + koff_kmajor(kk), qb + koff_mnmajor(kk), hi, idesc_dk, (e > 0 || kk > 0) ? 1u : 0u);
-          }
-          if (!ok) break;
-          mma_commit(smem_u32(&bar_ring_empty[stage]));   // two of two: Q of the stage is no longer read
-          if (t > 0) {   // the dQ warpgroup must have read the previous tile's dQ out of TMEM
-            ok = mbar_wait(smem_u32(&bar_dq_empty), (t - 1) & 1, &abortf, a.status, W_U_DQEMPTY);
-            if (!ok) break;
-            tc_fence_after_sync();
-          }
-          mma_ss_split(tDQ, dsMN, loK, hi, idesc_dq, 0u);
-#pragma unroll
-          for (int kk = 1; kk < KD_TILE / 16; ++kk) mma_ss_split(tDQ, dsMN + koff_mnmajor(kk), loK + koff_mnmajor(kk), hi, idesc_dq, 1u);
-          mma_commit(smem_u32(&bar_dq_full));   // issued after the dK product by the same thread: it covers both
-          ++t;
-          if (++stage == C::STAGES) stage = 0;
-        }
-        if (!ok) break;
-        mma_commit(smem_u32(&bar_acc_full));
-        mma_commit(smem_u32(&bar_k_empty[hh & 1]));   // the head's dQ products no longer read K
-        if (hh + 2 < nh) {
-          // The K of the head after next goes into this head's buffer: this thread waits for its own last products (it has
-          // nothing to issue before the next tile's dS^T is written) and requests the tile, a whole head ahead of its use.
-          ok = mbar_wait(smem_u32(&bar_k_empty[hh & 1]), (hh >> 1) & 1, &abortf, a.status, W_U_FIXEMPTY);
-          if (!ok) break;
-          mbar_arrive_expect_tx(smem_u32(&bar_k_full[hh & 1]), C::TILE_BYTES);
-          tma_load_4d(sK + (hh & 1) * C::TILE_BYTES, &tmK, smem_u32(&bar_k_full[hh & 1]), 0, kt * KD_TILE, h0 + hh + 2, b);
-          k_loads = hh + 3;
-        }
-      }
-      // let copies in flight land before the CTA exits: the last two requests of this thread
-      if (abortf.v != 0) {
-        for (int f = max(2, k_loads - 2); f < k_loads; ++f) drain_wait(smem_u32(&bar_k_full[f & 1]), (f >> 1) & 1);
       }
     }
-  } else if (warp < 20) {
+  } else if (warp < 12) {
     reg_alloc<C::REGS_COMPUTE>();
     // ------------------------------ compute warpgroups ------------------------------
-    // warpgroup g handles queries 32 g .. 32 g + 31 of every tile, a key row per thread. Warpgroups 0 and 1 own the first half of
-    // the tile's columns, 2 and 3 the second; the halves have their own barriers throughout, so the two pairs of warpgroups run
-    // as independent pipelines that drift apart in time: one does arithmetic while the other waits, loads or stores.
-    const int g = (warp - 4) >> 2;
-    const int half = g >> 1;
-    const int wq = warp & 3;
-    const int row = wq * 32 + lane;
-    const int kj = kt * KD_TILE + row;   // this thread's key
+    // Warpgroup w handles queries 64 w .. 64 w + 63 of every tile, a warp 32 keys of it in two halves of 16. In a half, this
+    // thread holds keys lane / 4 and lane / 4 + 8 and, of every 8 queries, queries 2 (lane % 4) and + 1.
+    const int w = (warp - 4) >> 2, wq = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const float c = a.scale_log2;
-    const uint32_t kdesc = a.desc[(size_t)b * a.Tpad + kj];
-    // this thread's 64 bytes of its key's row in dS^T block g / 2: 16-byte chunks 4 (g % 2) .. + 3, swizzled with the row
-    const uint32_t ds_row = static_cast<uint32_t>(half) * C::TILE_BYTES + static_cast<uint32_t>(row) * 128u;
-    const uint32_t ds_sw = static_cast<uint32_t>(row & 7);
+    const uint32_t tS = lane_base + C::TM_S + w * 64, tDP = lane_base + C::TM_DP + w * 64, tP = lane_base + C::TM_P + w * C::P_STRIDE;
+    constexpr uint32_t ROW16 = 16u << 16;
+    const uint64_t nc2 = pack_f32x2(-a.scale_log2, -a.scale_log2), minus1 = pack_f32x2(-1.f, -1.f);
+    const int qcol = w * 64 + 2 * (lane & 3);       // this thread's first query
+    // stmatrix: matrix m of four = (rows 8 (m & 1) .., 16-byte chunk n + (m >> 1)); lane l gives the address of row l % 8 of matrix l / 8
+    const uint32_t ds_row = sDS + static_cast<uint32_t>(w) * 16384u + static_cast<uint32_t>(wq * 32 + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u;
+    const uint32_t ds_sw = static_cast<uint32_t>((lane >> 4) ^ (lane & 7)) << 4;
     bool ok = true;
-
-    int stage = 0;
-    int t = 0;   // tiles so far, over all heads
-    const uint32_t tS = tbase + lane_base + C::TM_S + g * 32, tP = tbase + lane_base + C::TM_DP + g * 32;
-    const uint32_t tPT = tbase + lane_base + C::TM_PT + g * 16;
-    const uint32_t b_sfull = smem_u32(&bar_s_full[half]), b_spfree = smem_u32(&bar_sp_free[half]), b_pfull = smem_u32(&bar_p_full[half][0]),
-                   b_ptfree = smem_u32(&bar_pt_free[half]);
-
-    for (int hh = 0; hh < nh && ok; ++hh) {
-      for (int e = 0; e < n; ++e) {
-        const uint32_t ent = list[e];
-        const uint32_t cls = ent >> 8;
-        // The stage's scalars and mask words were written by the producer warp before its arrival on the stage's barrier;
-        // the issuer of S^T waited for that barrier before the products whose completion is awaited here, so no separate
-        // wait for the stage is taken.
-        ok = mbar_wait(b_sfull, t & 1, &abortf, a.status, half ? W_U_SFULL1 : W_U_SFULL);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+    int t = 0, qs = 0;
+    int4 it;
+    // visibility of this lane's key for the warpgroup's 64 queries
+    auto mask_words = [&](const float* side, uint32_t kdesc, int kj, int i0, uint32_t qd0, uint32_t qd1, uint32_t (&mk)[2]) {
+      const uint32_t* tb = reinterpret_cast<const uint32_t*>(side) + C::SIDE_BITS + 2 * w;   // words 2 w, 2 w + 1 of every mask
+      key_row_mask<2>(kdesc, kj, i0, tb + 4 * TB_SEES_PRE, tb + 4 * TB_SEES_CTX, tb + 4 * TB_SEES_INS, tb + 4 * TB_CTX, mk);
+      if ((tb[4 * TB_SIDPOS] | tb[4 * TB_SIDPOS + 1]) != 0u) {
+        // "same span": one round per distinct span among the warp's 32 keys, each a ballot over the queries
+        const uint32_t my_key = span_key_of_key(kdesc);
+        uint32_t todo = __ballot_sync(0xffffffffu, (kdesc & TD_INS) != 0u);
+        while (todo != 0u) {
+          const uint32_t kk = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
+          const uint32_t hit0 = __ballot_sync(0xffffffffu, span_match_query(kk, qd0) != 0u);
+          const uint32_t hit1 = __ballot_sync(0xffffffffu, span_match_query(kk, qd1) != 0u);
+          const bool mine = (my_key == kk);
+          if (mine) { mk[0] |= hit0; mk[1] |= hit1; }
+          todo &= ~__ballot_sync(0xffffffffu, mine);
+        }
+      }
+    };
+    // zeroes the hidden ones among this thread's 32 values of half hf
+    auto apply_mask = [&](uint32_t (&p)[32], const uint32_t (&mk)[2], int hf) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int src = hf * 16 + r * 8 + (lane >> 2);   // the lane that formed this key's mask
+        const uint32_t m0 = __shfl_sync(0xffffffffu, mk[0], src) >> (2 * (lane & 3));
+        const uint32_t m1 = __shfl_sync(0xffffffffu, mk[1], src) >> (2 * (lane & 3));
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const uint32_t m = j < 4 ? m0 : m1;
+          if ((m & (1u << (8 * (j & 3)))) == 0u) p[4 * j + 2 * r] = 0u;
+          if ((m & (2u << (8 * (j & 3)))) == 0u) p[4 * j + 2 * r + 1] = 0u;
+        }
+      }
+    };
+    if constexpr (HD == 64) {
+      // Iteration t forms P^T of tile t and dS^T of tile t - 1 in one instruction stream: the exponentials' special-function
+      // pipe and the multiply-adds, conversions and stores of dS^T overlap, and neither product is ever waited for in a
+      // chain: S^T(t + 1) and dP^T(t) are issued as soon as S^T(t) and dP^T(t - 1) have been loaded. The two warpgroups
+      // have barriers of their own and drift apart, so that one does arithmetic while the other waits, loads or stores:
+      //   SFULL  S^T(t) and dP^T(t - 1) of the half are there      SFREE   they have been loaded
+      //   PFULL  its P^T(t) and dS^T(t - 1) have been written      PFREE   dV has read P^T(t);  DSFREE  dK and dQ have read dS^T(t)
+      // P^T stays in registers as fp32 for a tile; results are stored at the end of the iteration, when the products that
+      // read their predecessors are done.
+      uint32_t p[2][32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) { p[0][j] = 0u; p[1][j] = 0u; }
+      const float* side_prev = sSide;
+      bool s_ready = false;
+      // One body for all iterations: the first one's dS^T and the last one's P^T are computed from whatever is there and
+      // read by nobody.
+      for (int k = 0;;) {
+        const bool more = next_item(k++, it);
+        if (!more && t == 0) break;
+        const int b = it.x, kt = it.z & 0xFFFF, n = more ? it.w : 1;
+        const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
+        const uint32_t kdesc = more ? a.desc[(size_t)b * a.Tpad + kj] : 0u;
+#pragma unroll 1
+        for (int e = 0; e < n; ++e, ++t) {
+          if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
+          tc_fence_after_sync();
+          const float* side = sSide + qs * C::SIDE_WORDS;
+          bool out_ready = false;
+          uint32_t pk_ds[2][16];
+          uint64_t lse[4], delta[4];
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {   // 16 keys x 32 queries at a time
+            const int hf = c & 1, ch = c >> 1;
+            uint32_t s[16], dp[16];
+            tmem_ld16x256_x4(tS + hf * ROW16 + ch * 32, s);
+            tmem_ld16x256_x4(tDP + hf * ROW16 + ch * 32, dp);
+            if (hf == 0) {   // both halves of the keys see the same queries
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                lse[j] = ld_shared_pair(side + qcol + 32 * ch + 8 * j);
+                delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 32 * ch + 8 * j);
+              }
+            }
+            tmem_wait_ld();
+            if (c == 3) {   // all loaded
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(C::B_SFREE + w));
+              // The barriers of the stores below, and of the next iteration further down, are tested ahead: a test takes some 150
+              // cycles under this load, and as a rule it finds the phase complete.
+              out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1) && mbar_test_wait(bar(C::B_DSFREE), t & 1);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                uint32_t& p0 = p[hf][16 * ch + 4 * j + 2 * r];
+                uint32_t& p1 = p[hf][16 * ch + 4 * j + 2 * r + 1];
+                const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dp[4 * j + 2 * r], dp[4 * j + 2 * r + 1]));
+                const uint64_t x = mul_f32x2(pack_u32x2(p0, p1), d);
+                pk_ds[hf][8 * ch + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+                const uint64_t y = fma_f32x2(pack_u32x2(s[4 * j + 2 * r], s[4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
+                p0 = __float_as_uint(fast_exp2(-lo_f32x2(y)));
+                p1 = __float_as_uint(fast_exp2(-hi_f32x2(y)));
+              }
+            }
+          }
+          const uint32_t* side_u = reinterpret_cast<const uint32_t*>(side);
+          const uint32_t ent = side_u[C::SIDE_ENT];
+          if (more && (ent >> 8) == KD_TILE_PARTIAL) {
+            uint32_t mk[2];
+            mask_words(side, kdesc, kj, (ent & 0xFF) * KD_TILE + w * 64, side_u[C::SIDE_DESC + w * 64 + lane], side_u[C::SIDE_DESC + w * 64 + 32 + lane], mk);
+            apply_mask(p[0], mk, 0);
+            apply_mask(p[1], mk, 1);
+          }
+          // (in the last iteration too: it must not complete a phase of PFULL ahead of the dV issuer)
+          if (!__all_sync(0xffffffffu, out_ready)) {
+            if (t > 0 && !(ok = wait(C::B_PFREE + w, (t - 1) & 1, W_U_PFREE))) break;
+            if (t > 1 && !(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
+          }
+          tc_fence_after_sync();
+          s_ready = mbar_test_wait(bar(C::B_SFULL + w), (t + 1) & 1);
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(p[hf][2 * j]), __uint_as_float(p[hf][2 * j + 1]));
+            tmem_st16x128_x8(tP + hf * ROW16, pk);
+          }
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+            for (int j = 0; j < 8; j += 2)
+              stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(j) << 4) ^ ds_sw), pk_ds[hf][2 * j], pk_ds[hf][2 * j + 1], pk_ds[hf][2 * j + 2], pk_ds[hf][2 * j + 3]);
+          fence_proxy_async_smem();   // the dK and dQ products read dS^T through the async proxy
+          tmem_wait_st();
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(C::B_PFULL + w));
+          side_prev = side;
+          if (++qs == C::QS) qs = 0;
+        }
+        if (!ok || !more) break;
+      }
+    } else {
+    for (int k = 0; ok && next_item(k, it); ++k) {
+      const int b = it.x, kt = it.z & 0xFFFF, n = it.w;
+      const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
+      const uint32_t kdesc = a.desc[(size_t)b * a.Tpad + kj];
+      const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
+      uint32_t ent_next = static_cast<uint32_t>(it.z) >> 16;
+      for (int e = 0; e < n; ++e, ++t) {
+        const uint32_t ent = ent_next;
+        if (e + 1 < n) ent_next = list[e + 1];
+        const bool partial = (ent >> 8) == KD_TILE_PARTIAL;
+        const int i0 = (ent & 0xFF) * KD_TILE + w * 64;
+        uint32_t qd0 = 0u, qd1 = 0u;
+        if (partial) {   // query descriptors for the same-span ballots, requested ahead of the wait
+          qd0 = a.desc[(size_t)b * a.Tpad + i0 + lane];
+          qd1 = a.desc[(size_t)b * a.Tpad + i0 + 32 + lane];
+        }
+        // LSE, delta and mask words of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here
+        if (!(ok = wait(C::B_SFULL, t & 1, W_U_SFULL))) break;
         tc_fence_after_sync();
-        const uint32_t* side = sSide + stage * C::SIDE_WORDS + g * 32;   // this warpgroup's 32 queries
-        if (++stage == C::STAGES) stage = 0;
-        uint32_t mk = 0xFFFFFFFFu;   // visibility of this key for the 32 queries
-        if (cls == KD_TILE_PARTIAL) {
-          const uint32_t* tbw = side - g * 32 + 3 * KD_TILE + g;   // word g of every query-side class mask
-          const int i0 = (ent & 0xFF) * KD_TILE + g * 32;          // first query handled here
-          key_row_mask<1>(kdesc, kj, i0, tbw + 4 * TB_SEES_PRE, tbw + 4 * TB_SEES_CTX, tbw + 4 * TB_SEES_INS, tbw + 4 * TB_CTX, &mk);
-          if (tbw[4 * TB_SIDPOS] != 0u) {
-            // "same span": lane L holds the descriptor of query number L of this warpgroup; one round per distinct span among
-            // the warp's 32 keys, each a ballot over the queries
-            const uint32_t qd_lane = side[2 * KD_TILE + lane];
-            const uint32_t my_key = span_key_of_key(kdesc);
-            uint32_t todo = __ballot_sync(0xffffffffu, (kdesc & TD_INS) != 0u);
-            while (todo != 0u) {
-              const uint32_t kk = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-              const uint32_t hit = __ballot_sync(0xffffffffu, span_match_query(kk, qd_lane) != 0u);
-              const bool mine = (my_key == kk);
-              if (mine) mk |= hit;
-              todo &= ~__ballot_sync(0xffffffffu, mine);
+        const float* side = sSide + qs * C::SIDE_WORDS;
+        if (++qs == C::QS) qs = 0;
+        uint32_t s[2][32];
+        tmem_ld16x256_x8(tS, s[0]);
+        tmem_ld16x256_x8(tS + ROW16, s[1]);
+        uint64_t col[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) col[j] = ld_shared_pair(side + qcol + 8 * j);   // LSE of this thread's columns
+        tmem_wait_ld();
+        uint32_t mk[2] = {0u, 0u};
+        if (partial) mask_words(side, kdesc, kj, i0, qd0, qd1, mk);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {   // 16 keys at a time
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const uint64_t x = fma_f32x2(pack_u32x2(s[hf][4 * j + 2 * r], s[hf][4 * j + 2 * r + 1]), nc2, col[j]);   // LSE - c S
+              s[hf][4 * j + 2 * r] = __float_as_uint(fast_exp2(-lo_f32x2(x)));
+              s[hf][4 * j + 2 * r + 1] = __float_as_uint(fast_exp2(-hi_f32x2(x)));
             }
           }
+          if (partial) apply_mask(s[hf], mk, hf);
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(s[hf][2 * j]), __uint_as_float(s[hf][2 * j + 1]));
+          tmem_st16x128_x8(tP + hf * ROW16, pk);
         }
-        const int tb = t & 1;
-        const uint32_t ds_base = sDS + tb * (2 * C::TILE_BYTES) + ds_row;
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {   // 16 queries at a time
-          uint32_t pk_p[8], pk_ds[8];
-          uint32_t rs[16], rp[16];
-          tmem_ld16(tS + hf * 16, rs);
-          tmem_ld16(tP + hf * 16, rp);
-          tmem_wait_ld();
-          if (hf == 1) {   // all of this warp's values are in registers: the next tile's S^T and dP^T may overwrite the half's columns
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(b_spfree);
-          }
-          const uint32_t mh = mk >> (hf * 16);
-#pragma unroll
-          for (int j = 0; j < 16; j += 4) {
-            const float4 l4 = *reinterpret_cast<const float4*>(side + hf * 16 + j);             // LSE of 4 queries
-            const float4 d4 = *reinterpret_cast<const float4*>(side + KD_TILE + hf * 16 + j);   // delta of 4 queries
-            const float lw[4] = {l4.x, l4.y, l4.z, l4.w}, dw[4] = {d4.x, d4.y, d4.z, d4.w};
-            float pv[4], ds[4];
-#pragma unroll
-            for (int u2 = 0; u2 < 4; ++u2) pv[u2] = fast_exp2(fmaf(__uint_as_float(rs[j + u2]), c, -lw[u2]));
-            if (cls == KD_TILE_PARTIAL) {   // warp-uniform
-#pragma unroll
-              for (int u2 = 0; u2 < 4; ++u2)
-                if ((mh & (1u << (j + u2))) == 0u) pv[u2] = 0.f;
-            }
-#pragma unroll
-            for (int u2 = 0; u2 < 4; ++u2) ds[u2] = pv[u2] * (__uint_as_float(rp[j + u2]) - dw[u2]);
-            pk_p[j / 2] = pack2<kBf16>(pv[0], pv[1]);
-            pk_p[j / 2 + 1] = pack2<kBf16>(pv[2], pv[3]);
-            pk_ds[j / 2] = pack2<kBf16>(ds[0], ds[1]);
-            pk_ds[j / 2 + 1] = pack2<kBf16>(ds[2], ds[3]);
-          }
-          if (hf == 0 && t > 0) {
-            // P^T and dS^T may leave the registers once the products that read their previous contents are done: the
-            // previous tile's dV, and the dK / dQ / reduction of the tile before that. The dV issuer waits for the latter
-            // itself before it signals the former, so one barrier stands for both.
-            ok = mbar_wait(b_ptfree, (t - 1) & 1, &abortf, a.status, W_U_PTFREE);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after_sync();
-          }
-          tmem_st8(tPT + hf * 8, pk_p);
-          const uint32_t ch = static_cast<uint32_t>(4 * (g & 1) + 2 * hf);
-          st_shared_v4(ds_base + (((ch + 0u) ^ ds_sw) << 4), pk_ds[0], pk_ds[1], pk_ds[2], pk_ds[3]);
-          st_shared_v4(ds_base + (((ch + 1u) ^ ds_sw) << 4), pk_ds[4], pk_ds[5], pk_ds[6], pk_ds[7]);
-        }
-        if (!ok) break;
-        fence_proxy_async_smem();   // the dK and dQ products read these shared-memory writes through the async proxy
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(b_pfull + (t & 1) * 8);
-        ++t;
+        if (lane == 0) mbar_arrive(bar(C::B_PFULL));
+
+#pragma unroll
+        for (int j = 0; j < 8; ++j) col[j] = ld_shared_pair(side + KD_TILE + qcol + 8 * j);   // delta
+        // dP^T, and the products that read the previous tile's dS^T are done (long before, as a rule)
+        if (!(ok = t == 0 ? wait(C::B_DPFULL, 0, W_U_DPFULL) : wait2(C::B_DPFULL, t & 1, W_U_DPFULL, C::B_DSFREE, (t - 1) & 1, W_U_DSFREE))) break;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t dp[32];
+          tmem_ld16x256_x8(tDP + hf * ROW16, dp);
+          tmem_wait_ld();
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const uint64_t d = fma_f32x2(col[j], minus1, pack_u32x2(dp[4 * j + 2 * r], dp[4 * j + 2 * r + 1]));
+              const uint64_t x = mul_f32x2(pack_u32x2(s[hf][4 * j + 2 * r], s[hf][4 * j + 2 * r + 1]), d);
+              pk[2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 8; j += 2)
+            stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(j) << 4) ^ ds_sw), pk[2 * j], pk[2 * j + 1], pk[2 * j + 2], pk[2 * j + 3]);
+        }
+        fence_proxy_async_smem();   // the dK and dQ products read these shared-memory writes through the async proxy
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::B_DSFULL));
       }
+    }
     }
   } else {
     reg_dealloc<C::REGS_DQ>();
-    // ------------------------------ dQ warpgroup: TMEM -> shared memory -> bulk reduction into the fp32 scratch ------------------------------
+    // ------------------------------ dQ warps: TMEM -> shared memory -> bulk reduction into the fp32 scratch ------------------------------
     const int wq = warp & 3;
-    const int row = wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t st_row = static_cast<uint32_t>(row) * 128u, st_sw = static_cast<uint32_t>(row & 7);
-    const bool leader = (warp == 20 && lane == 0);
-    if (leader) tma_prefetch_desc(&tmAcc);
-    const uint32_t tDQ = tbase + lane_base + C::TM_DQ;
+    const uint32_t stg = s0 + C::SMEM_STG + wq * 8192, st_row = static_cast<uint32_t>(lane) * 128u, st_sw = static_cast<uint32_t>(lane & 7);
+    if (lane == 0) {
+      tma_prefetch_desc(&tmAcc);
+      tma_prefetch_desc(&tmDK);
+      tma_prefetch_desc(&tmDV);
+    }
     bool ok = true;
     int t = 0;
-    const int kj = kt * KD_TILE + row;   // this thread's key: it also writes that key's rows of dK and dV
-    // dK and dV of head number hd leave through these warps as well (a whole 128-byte row per thread): the compute warps
-    // go straight on to the next head's tiles, whose S^T / dP^T are already waiting, and the accumulating issuers wait for
-    // bar_acc_free before they overwrite the accumulators.
-    auto write_out = [&](int hd) -> bool {
-      if (n > 0) {
-        ok = mbar_wait(smem_u32(&bar_acc_full), hd & 1, &abortf, a.status, W_U_ACCFULL);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) return false;
-        tc_fence_after_sync();
-      }
-      const int h = h0 + hd;
-      uint16_t* krow = reinterpret_cast<uint16_t*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st;
-      uint16_t* vrow = reinterpret_cast<uint16_t*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st;
-#pragma unroll
-      for (int part = 0; part < 4; ++part) {   // dV columns 0-31, 32-63, then dK: the next head's first dV product is the
-                                               // one the compute warps wait for, so dV is released first
-        uint32_t r[32];
-        const bool is_k = part >= 2;
-        if (n > 0) {
-          tmem_ld32(tbase + lane_base + (is_k ? C::TM_DK : C::TM_DV) + (part & 1) * 32, r);
+    const int np = (a.d_real + 31) / 32;   // 32-column pieces of a dQ tile
+    // Writes dV, then dK (the next item's first dV product comes first) of the item: 32 rows of a warp as boxes of 64 columns
+    // through the staging buffers and TMA stores. m: number of the item; kt: its key tile.
+    auto write_out = [&](int b, int h, int kt, int m) -> bool {
+      if (!wait(C::B_ACCFULL, m & 1, W_U_ACCFULL)) return false;
+      tc_fence_after_sync();
+      const int key0 = kt * KD_TILE + wq * 32;
+#pragma unroll 1
+      for (int part = 0; part < 2 * HD / 64; ++part) {
+        const bool is_k = part >= HD / 64;
+        const int col = (part % (HD / 64)) * 64;
+        const uint32_t buf = stg + (part & 1) * 4096;
+        const float f = is_k ? a.sm_scale : 1.0f;
+        if ((part & 1) == 0) {
+          if (lane == 0) bulk_wait_group_read0();   // the staging buffers have been read
+          __syncwarp();
+        }
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+          uint32_t r[32], pk[16];
+          tmem_ld32(lane_base + (is_k ? C::TM_DK : C::TM_DV) + col + half * 32, r);
           tmem_wait_ld();
-          if (part & 1) {   // the accumulator is in registers: the next head's first product may overwrite it
+          if (col + 64 == HD && half == 1) {   // the accumulator is in registers: the next item's first product may overwrite it
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_free[is_k ? 1 : 0]));
+            if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + (is_k ? 1 : 0)));
           }
-        } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = 0u;
+          for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(r[2 * j]) * f, __uint_as_float(r[2 * j + 1]) * f);
+#pragma unroll
+          for (int cch = 0; cch < 4; ++cch)
+            st_shared_v4(buf + st_row + ((static_cast<uint32_t>(4 * half + cch) ^ st_sw) << 4), pk[4 * cch], pk[4 * cch + 1], pk[4 * cch + 2], pk[4 * cch + 3]);
         }
-        if (kj < a.T) store_row32_upto<kBf16>((is_k ? krow : vrow) + (part & 1) * 32, r, is_k ? a.sm_scale : 1.0f, (part & 1) * 32, a.d_real);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && key0 < a.T && col < a.d_real) {
+          tma_store_4d(is_k ? &tmDK : &tmDV, buf, col, key0, h, b);
+          bulk_commit_group();
+        }
       }
       return true;
     };
-    for (int hh = 0; hh < nh && ok; ++hh) {
-      const int bh = b * a.H + h0 + hh;
-      if (n == 0) write_out(hh);
-      for (int e = 0; e < n; ++e) {
-        const int tb = t & 1;
-        const int q0 = (list[e] & 0xFF) * KD_TILE;
-        ok = mbar_wait(smem_u32(&bar_dq_full), t & 1, &abortf, a.status, W_U_DQFULL);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+    int4 it;
+    int m = 0;
+    for (int k = 0; ok && next_item(k, it); ++k) {
+      const int b = it.x, h = it.y, kt = it.z & 0xFFFF, n = it.w;
+      const int bh = b * a.H + h;
+      const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
+      uint32_t ent_next = static_cast<uint32_t>(it.z) >> 16;
+      for (int e = 0; e < n; ++e, ++t) {
+        const int q0 = (ent_next & 0xFF) * KD_TILE + wq * 32;
+        if (e + 1 < n) ent_next = list[e + 1];
+        if (!(ok = wait(C::B_DQFULL, t & 1, W_U_DQFULL))) break;
         tc_fence_after_sync();
-        // The dQ product was the last reader of this tile's dS^T buffer (the dK product was issued before it by the same
-        // thread): its 32 KB now stage the dQ tile as two [128 rows][32 floats] boxes in the 128-byte-swizzled layout the
-        // tensor map expects.
-        const uint32_t stage = sDS + tb * (2 * C::TILE_BYTES);
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-          uint32_t r[32];
-          tmem_ld32(tDQ + hf * 32, r);
-          tmem_wait_ld();
-          if (hf == 1) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_dq_empty));   // the next tile's dQ product may overwrite the TMEM columns
-          }
+        const uint32_t tDQ = lane_base + C::TM_DQ;
+        auto drained = [&]() {   // the tile is in registers: the columns may be overwritten
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(C::B_DQEMPTY));
+        };
+        auto stage = [&](int buf, const uint32_t (&r)[32]) {   // 32 columns as a box [32 rows][32 columns]
 #pragma unroll
           for (int cch = 0; cch < 8; ++cch)
-            st_shared_v4(stage + hf * C::TILE_BYTES + st_row + ((static_cast<uint32_t>(cch) ^ st_sw) << 4), r[4 * cch], r[4 * cch + 1],
-                         r[4 * cch + 2], r[4 * cch + 3]);
+            st_shared_v4(stg + buf * 4096 + st_row + ((static_cast<uint32_t>(cch) ^ st_sw) << 4), r[4 * cch], r[4 * cch + 1], r[4 * cch + 2], r[4 * cch + 3]);
+        };
+        auto reduce = [&](int g) {   // both boxes: columns 64 g .. 64 g + 63
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && q0 < a.T) {
+            if (g * 2 < np) tma_reduce_add_3d(&tmAcc, stg, g * 64, q0, bh);
+            if (g * 2 + 1 < np) tma_reduce_add_3d(&tmAcc, stg + 4096, g * 64 + 32, q0, bh);
+            bulk_commit_group();
+          }
+        };
+        if (lane == 0) bulk_wait_group_read0();   // the staging buffers have been read
+        __syncwarp();
+        if constexpr (HD == 64) {
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            uint32_t r[32];
+            tmem_ld32(tDQ + p * 32, r);
+            tmem_wait_ld();
+            if (p == 1) drained();
+            stage(p, r);
+          }
+          reduce(0);
+        } else {   // the next dP^T waits for these columns: the second half goes into registers before the first leaves
+          uint32_t r[2][32];
+          tmem_ld32(tDQ, r[0]);
+          tmem_ld32(tDQ + 32, r[1]);
+          tmem_wait_ld();
+          stage(0, r[0]);
+          stage(1, r[1]);
+          tmem_ld32(tDQ + 64, r[0]);
+          tmem_ld32(tDQ + 96, r[1]);
+          tmem_wait_ld();
+          drained();
+          reduce(0);
+          if (lane == 0) bulk_wait_group_read0();
+          __syncwarp();
+          stage(0, r[0]);
+          stage(1, r[1]);
+          reduce(1);
         }
-        fence_proxy_async_smem();
-        named_bar_sync(1, 128);
-        if (leader) {
-          tma_reduce_add_3d(&tmAcc, stage, 0, q0, bh);
-          tma_reduce_add_3d(&tmAcc, stage + C::TILE_BYTES, 32, q0, bh);
-          bulk_commit_group();
-        }
-        // after the head's last tile its dK and dV are complete (their last products were issued before the dQ product
-        // this warpgroup has just consumed): they are written while the bulk reduction reads the staged tile
-        if (e == n - 1 && !write_out(hh)) break;
-        if (leader) {
-          bulk_wait_group_read0();
-          mbar_arrive(smem_u32(&bar_ds_empty[tb]));    // compute warps may write the tile after next's dS^T here
-        }
-        ++t;
+        if (e == n - 1 && !(ok = write_out(b, h, kt, m++))) break;
       }
     }
-    if (leader) bulk_wait_group0();
+    if (lane == 0) bulk_wait_group0();
   }
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tbase, 512);
+  if (warp == 1) tmem_dealloc(0, 512);
+  if (tid == 0) report_abort(abortf, a.status);
 }
 
-// dq[b, h, t, :] = dq_acc[b, h, t, :] * sm_scale in the output dtype; 8 threads per row, 32 bytes in and 16 out each
-template <bool kBf16>
+// dq[b, h, t, :] = dq_acc[b, h, t, :] * sm_scale in the output dtype; HD / 8 threads per row, 32 bytes in and 16 out each
+template <int HD, bool kBf16>
 __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs a) {
-  constexpr int HD = FusedCfg::HD, TPR = HD / 8;
+  constexpr int TPR = HD / 8;
   const size_t rows = (size_t)a.B * a.H * a.T;
   const int sub = threadIdx.x % TPR;
   for (size_t r = (size_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR; r < rows; r += (size_t)gridDim.x * (256 / TPR)) {
@@ -643,14 +999,26 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
   }
 }
 
-template <bool kBf16>
+template <int HD, bool kBf16>
 static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                          const BwdArgs& a, dim3 grid, cudaStream_t stream) {
-  using C = FusedCfg;
-  CUtensorMap tmAcc;
-  int rc = encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, C::HD, KD_TILE, "dq_acc");
+                          const BwdArgs& a, int dtype, cudaStream_t stream) {
+  using C = FusedCfg<HD>;
+  CUtensorMap tmAcc, tmDK, tmDV;
+  int rc = encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
+  const kd_tensor dk = {a.dk, a.dk_sb, a.dk_sh, a.dk_st}, dv = {a.dv, a.dv_sb, a.dv_sh, a.dv_st};
+  if (rc == 0) rc = encode_tensor_map(&tmDK, dk, a.B, a.H, a.T, a.d_real, dtype, 32, "dk");
+  if (rc == 0) rc = encode_tensor_map(&tmDV, dv, a.B, a.H, a.T, a.d_real, dtype, 32, "dv");
   if (rc != 0) return rc;
-  auto kern = attn_bwd_fused_kernel<kBf16>;
+  const long long n_items = (long long)a.B * a.H * a.NT;
+  if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
+  FusedArgs fa;
+  fa.b = a;
+  // (batch, head) pairs whose Q, K, V, dO and dQ scratch take about 64 MB of the 126 MB L2 together, and enough of them that
+  // a chunk holds two items per SM
+  const double pair_bytes = (double)a.T * (4.0 * a.d_real * 2 + HD * 4.0);
+  fa.chunk = static_cast<int>(std::min<double>((double)a.B * a.H, std::max(1.0, 64e6 / pair_bytes)));
+  while ((long long)fa.chunk * a.NT < 296 && fa.chunk < a.B * a.H) ++fa.chunk;
+  auto kern = attn_bwd_fused_kernel<HD, kBf16>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd smem attribute: %s", cudaGetErrorString(e));
@@ -664,19 +1032,21 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
     launch_regs = fa.numRegs;
   }
   if (launch_regs < C::REGS_LAUNCH) return set_error(KD_ERR_DEVICE, "fused bwd was built with %d registers per thread, needs %d", launch_regs, C::REGS_LAUNCH);
-  kern<<<grid, C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, tmAcc, a);
+  kern<<<static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
   const size_t rows = (size_t)a.B * a.H * a.T;
-  const int blocks = static_cast<int>(std::min<size_t>((rows + 31) / 32, size_t(148) * 32));
-  attn_bwd_dq_convert_kernel<kBf16><<<blocks, 256, 0, stream>>>(a);
+  const int rows_per_block = 256 / (HD / 8);
+  const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
+  attn_bwd_dq_convert_kernel<HD, kBf16><<<blocks, 256, 0, stream>>>(a);
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }
 
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                     const BwdArgs& a, int dtype, dim3 grid, cudaStream_t stream) {
-  return dtype == KD_BF16 ? launch_fused_t<true>(tmQ, tmK, tmV, tmDO, a, grid, stream)
-                          : launch_fused_t<false>(tmQ, tmK, tmV, tmDO, a, grid, stream);
+                     const BwdArgs& a, int dtype, cudaStream_t stream) {
+  if (a.d_real <= 64)
+    return dtype == KD_BF16 ? launch_fused_t<64, true>(tmQ, tmK, tmV, tmDO, a, dtype, stream) : launch_fused_t<64, false>(tmQ, tmK, tmV, tmDO, a, dtype, stream);
+  return dtype == KD_BF16 ? launch_fused_t<128, true>(tmQ, tmK, tmV, tmDO, a, dtype, stream) : launch_fused_t<128, false>(tmQ, tmK, tmV, tmDO, a, dtype, stream);
 }
 
 }  // namespace kd

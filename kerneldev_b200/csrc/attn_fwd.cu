@@ -253,7 +253,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       bool ok = true;
       auto load_q = [&](int hh) -> bool {   // Q pair of head h0 + hh into buffer hh % NQ
         const int qb = hh % C::NQ, qround = hh / C::NQ;
-        if (qround > 0 && !mbar_wait(smem_u32(&bar_q_empty[qb]), (qround - 1) & 1, &abortf, a.status, W_F_QEMPTY)) return false;
+        if (qround > 0 && !mbar_wait(smem_u32(&bar_q_empty[qb]), (qround - 1) & 1, &abortf, W_F_QEMPTY)) return false;
         mbar_arrive_expect_tx(smem_u32(&bar_q_full[qb]), ntile_q * C::TILE_BYTES);
         for (int t = 0; t < ntile_q; ++t)
           for (int kb = 0; kb < C::KBLK; ++kb)
@@ -282,7 +282,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #endif
           {
             const int s = k_cnt % C::KST;
-            ok = mbar_wait(smem_u32(&bar_k_empty[s]), ((k_cnt / C::KST) & 1) ^ 1, &abortf, a.status, W_F_KEMPTY);
+            ok = mbar_wait(smem_u32(&bar_k_empty[s]), ((k_cnt / C::KST) & 1) ^ 1, &abortf, W_F_KEMPTY);
             if (!ok) break;
             mbar_arrive_expect_tx(smem_u32(&bar_k_full[s]), C::TILE_BYTES);
             for (int kb = 0; kb < C::KBLK; ++kb)
@@ -291,7 +291,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           {
             const int s = v_cnt % C::VST;
-            ok = mbar_wait(smem_u32(&bar_v_empty[s]), ((v_cnt / C::VST) & 1) ^ 1, &abortf, a.status, W_F_VEMPTY);
+            ok = mbar_wait(smem_u32(&bar_v_empty[s]), ((v_cnt / C::VST) & 1) ^ 1, &abortf, W_F_VEMPTY);
             if (!ok) break;
             mbar_arrive_expect_tx(smem_u32(&bar_v_full[s]), C::TILE_BYTES);
             for (int kb = 0; kb < C::KBLK; ++kb)
@@ -321,7 +321,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       uint32_t kparity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int qb = hh % C::NQ;
-        ok = mbar_wait(smem_u32(&bar_q_full[qb]), (hh / C::NQ) & 1, &abortf, a.status, W_F_QFULL);
+        ok = mbar_wait(smem_u32(&bar_q_full[qb]), (hh / C::NQ) & 1, &abortf, W_F_QFULL);
         const uint32_t q_off = qb * (2 * C::TILE_BYTES >> 4);
         for (int u = 0; u < U && ok; ++u) {
           const uint4 c = sCmd[2 * u];
@@ -336,11 +336,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           }
           if (round > 0) {
             // the buffer is free once P V of the unit that used it in the previous round has been issued
-            ok = mbar_wait(smem_u32(&bar_pv_issued[buf]), (round - 1) & 1, &abortf, a.status, W_F_PVISSUED);
+            ok = mbar_wait(smem_u32(&bar_pv_issued[buf]), (round - 1) & 1, &abortf, W_F_PVISSUED);
             if (!ok) break;
           }
           if (c.z & CMD_WAIT) {
-            ok = mbar_wait(smem_u32(&bar_k_full[kstage]), kparity, &abortf, a.status, W_F_KFULL);
+            ok = mbar_wait(smem_u32(&bar_k_full[kstage]), kparity, &abortf, W_F_KFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -379,10 +379,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             vdesc[kk] = desc64(vlo + koff_mnmajor(kk), hi);
             pop[kk] = aP + kk * 8;   // P of 16 keys = 8 packed columns at the start of the score buffer
           }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, a.status, W_F_PFULL);
+          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_F_PFULL);
           if (!ok) break;
           if (c.z & CMD_WAIT) {
-            ok = mbar_wait(smem_u32(&bar_v_full[vstage]), vparity, &abortf, a.status, W_F_VFULL);
+            ok = mbar_wait(smem_u32(&bar_v_full[vstage]), vparity, &abortf, W_F_VFULL);
             if (!ok) break;
           }
           const uint32_t i = (c.z & CMD_TILE1) ? 1u : 0u;
@@ -390,7 +390,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (acc0 == 0u && hh > 0) {
             // first product of this query tile for a new head overwrites O_i: the softmax warpgroup must
             // have read the previous head's result out of it
-            ok = mbar_wait(smem_u32(&bar_o_free[i]), (hh - 1) & 1, &abortf, a.status, W_F_OFREE);
+            ok = mbar_wait(smem_u32(&bar_o_free[i]), (hh - 1) & 1, &abortf, W_F_OFREE);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -472,7 +472,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int buf = wcmd_buf(cmd) + buf_off;
       if (buf >= C::NBUF) buf -= C::NBUF;
       const uint32_t tS = tbase + lane_base + buf * 128;
-      ok = mbar_wait(smem_u32(&bar_s_full[2 * buf + i]), (sfull_par >> buf) & 1u, &abortf, a.status, W_F_SFULL);
+      ok = mbar_wait(smem_u32(&bar_s_full[2 * buf + i]), (sfull_par >> buf) & 1u, &abortf, W_F_SFULL);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       sfull_par ^= 1u << buf;
@@ -572,7 +572,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (nact > 0) {
         // O_i may be touched only after the previous P V product of this query tile has completed;
         // the wait is taken for every unit so that no phase of the barrier goes unobserved
-        ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, a.status, W_F_PVDONE);
+        ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, W_F_PVDONE);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -602,7 +602,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
     // epilogue of this head: normalise, convert, store this thread's share of O, and LSE
     if (nact > 0) {
-      ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, a.status, W_F_PVDONE);
+      ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, W_F_PVDONE);
       ok = __all_sync(0xffffffffu, ok);
     }
     if (ok && tile_valid && qi < a.T) {
@@ -637,6 +637,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tbase, 512);
+  if (tid == 0) report_abort(&abortf, a.status);
 }
 
 template <int HD, bool kBf16>

@@ -109,7 +109,6 @@ static int check_attn(const kd_attn_params* p, bool backward) {
     if (!p->delta) return set_error(KD_ERR_ARG, "delta scratch is null");
     if (p->bwd_mode != KD_BWD_SPLIT && p->bwd_mode != KD_BWD_FUSED) return set_error(KD_ERR_ARG, "bwd_mode %d unknown", p->bwd_mode);
     if (p->bwd_mode == KD_BWD_FUSED) {
-      if (p->D > 64) return set_error(KD_ERR_ARG, "the fused backward (KD_BWD_FUSED) supports head dims up to 64 only, got %d", p->D);
       if (!p->dq_acc || (reinterpret_cast<uintptr_t>(p->dq_acc) & 15u)) return set_error(KD_ERR_ARG, "dq_acc scratch is null or not 16-byte aligned");
     }
     const kd_tensor* outs[3] = {&p->dq, &p->dk, &p->dv};
@@ -212,8 +211,8 @@ int kd_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, size_t* bytes
 
 int kd_workspace_bytes_fused(int32_t B, int32_t H, int32_t T, int32_t D, size_t* bytes) {
   if (!bytes || B < 1 || H < 1 || T < 1 || D < 1) return set_error(KD_ERR_ARG, "bad workspace query");
-  (void)D;   // rows of the scratch are as wide as the kernel's tile (64 columns) whatever the head dim
-  *bytes = (size_t)B * H * T * 64 * sizeof(float);
+  // rows of the scratch are as wide as the kernel's tile
+  *bytes = (size_t)B * H * T * (D <= 64 ? 64 : 128) * sizeof(float);
   return 0;
 }
 

@@ -351,9 +351,9 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   }
   const auto f32 = q.options().dtype(at::kFloat);
   if (!delta.defined()) delta = at::empty({q.size(0), q.size(1), q.size(2)}, f32);
-  const bool fused = !deterministic && q.size(3) <= 64;
+  const bool fused = !deterministic;
   // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
-  if (fused && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), 64}, f32);
+  if (fused && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, f32);
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
   p.d_o = desc(d_o);
   p.dq = desc(dq);

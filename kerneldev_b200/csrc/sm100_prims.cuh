@@ -25,12 +25,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
@@ -77,7 +71,23 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Shared by all roles of a CTA: once set, every bounded wait returns false at once.
+// the same without suspending the thread: is the phase complete now?
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// Shared by all roles of a CTA: once set (to KD_DEV_TIMEOUT | site of the wait that gave up first), every bounded wait
+// returns false at once; report_abort passes it on when the CTA has unwound.
 struct AbortFlag {
   volatile uint32_t v;
 };
@@ -94,13 +104,23 @@ __device__ __forceinline__ void report_status(uint32_t* status, uint32_t value) 
   }
 }
 
+// called by one thread at the end of a kernel, behind a block-wide barrier
+__device__ __forceinline__ void report_abort(const AbortFlag* abort_flag, uint32_t* status) {
+  if (abort_flag->v != 0u) report_status(status, abort_flag->v);
+}
+
 #ifndef KD_WAIT_LIMIT_NS
 #define KD_WAIT_LIMIT_NS 400000000ull  // 0.4 s: far above any legitimate wait in these kernels
 #endif
+// in SM cycles, at two a nanosecond: the clock is below that, so the limit is never shorter than stated
+constexpr uint32_t KD_WAIT_LIMIT_CYCLES = static_cast<uint32_t>(KD_WAIT_LIMIT_NS * 2);
+static_assert(KD_WAIT_LIMIT_NS * 2 < 0x80000000ull, "the limit is measured with a 32-bit cycle counter");
 
-// Waits for the phase with the given parity. Returns true when the phase completed.
-// On time-out (or when another role already aborted) returns false after recording
-// KD_DEV_TIMEOUT|site in *status (first writer wins) and raising the CTA abort flag.
+__device__ __forceinline__ uint32_t clock32() {
+  uint32_t c;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+  return c;
+}
 // try_wait that lets the hardware suspend the thread for up to `ns` nanoseconds while the phase is
 // pending: a waiting thread then takes no issue slots from the warps that share its scheduler
 __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t parity, uint32_t ns) {
@@ -116,21 +136,26 @@ __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t par
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFlag* abort_flag,
-                                          uint32_t* status, uint32_t site) {
+// marks the CTA as aborted (the first wait that gives up wins)
+__device__ __forceinline__ void raise_abort(AbortFlag* abort_flag, uint32_t site) {
+  atomicCAS(const_cast<uint32_t*>(&abort_flag->v), 0u, KD_DEV_TIMEOUT | site);
+}
+// Waits for the phase with the given parity. Returns true when the phase completed, false when the limit ran out or
+// another role has aborted. This is inlined dozens of times per kernel, between hot loops that compete for the
+// instruction cache, so the slow path is a few instructions: a 32-bit cycle count, and the status word is left to the
+// end of the kernel (with the reporting inlined here the fused backward was 120 KB of code).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFlag* abort_flag, uint32_t site) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  while (true) {
-    if (mbar_try_wait_suspend(bar, parity, 20000u)) return true;
+  const uint32_t t0 = clock32();
+  while (!mbar_try_wait_suspend(bar, parity, 20000u)) {
     if (abort_flag->v != 0u) return false;
-    if (globaltimer_ns() - t0 > KD_WAIT_LIMIT_NS) {
-      abort_flag->v = 1u;
-      report_status(status, KD_DEV_TIMEOUT | site);
+    if (clock32() - t0 > KD_WAIT_LIMIT_CYCLES) {
+      raise_abort(abort_flag, site);
       return false;
     }
   }
+  return true;
 }
-
 // ---------------------------------------------------------------------------------------
 // TMA (plain per-CTA tile loads; completion reported on an mbarrier as bytes)
 // ---------------------------------------------------------------------------------------
@@ -154,6 +179,21 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm,
       : "memory");
 }
 
+// asynchronous 4- and 16-byte copies global -> shared, and this thread's arrival on an mbarrier when its copies so far
+// have landed (counted like any other arrival)
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_mbar_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_shared_u32(uint32_t saddr, uint32_t v) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory");
+}
+
 // Adds a shared-memory tile to global memory through TMA (fp32 add in L2); completion is tracked by the
 // issuing thread's bulk async-group. Rows outside the tensor are clipped.
 __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tm, uint32_t src, int c0, int c1, int c2) {
@@ -161,11 +201,42 @@ __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* tm, uint32_
                ::"l"(tm), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
 }
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* tm, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+               ::"l"(tm), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all of this thread's bulk groups have finished READING their shared-memory source
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// ... all but the most recent one
+__device__ __forceinline__ void bulk_wait_group_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // ... and have completed altogether
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// Cluster launch control: asks the hardware to cancel a CTA of this grid that has not been launched yet, so that the
+// asking CTA can do its work. The 16-byte response is written to shared memory and counted on the mbarrier. After a
+// response without a CTA no further request may be made.
+__device__ __forceinline__ void clc_try_cancel(uint32_t dst, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(dst), "r"(bar) : "memory");
+}
+// blockIdx.x of the cancelled CTA, or -1
+__device__ __forceinline__ int clc_first_ctaid_x(uint32_t src) {
+  uint32_t x;
+  asm volatile(
+      "{\n"
+      ".reg .b128 r;\n"
+      ".reg .pred p;\n"
+      "ld.shared.b128 r, [%1];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+      "mov.u32 %0, 0xffffffff;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n"
+      "}\n"
+      : "=r"(x)
+      : "r"(src)
+      : "memory");
+  return static_cast<int>(x);
+}
 
 // Byte offset of element (row, 16-byte chunk) inside a tile whose rows are 128 bytes and
 // which was written by TMA with the 128-byte swizzle (tile base 1024-byte aligned):
@@ -333,6 +404,45 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 
+// 16 lanes x 64 columns in mma-fragment order: per 8 columns, registers 0-1 hold columns 2 (lane % 4) and + 1 of row
+// lane / 4, registers 2-3 the same columns of row lane / 4 + 8. The address's lane field is a multiple of 16.
+__device__ __forceinline__ void tmem_ld16x256_x8(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+// the same for 32 columns
+__device__ __forceinline__ void tmem_ld16x256_x4(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 16 lanes x 32 columns, the 16-bit counterpart: per 4 columns (8 packed pairs' halves), register 0 is column lane % 4 of row
+// lane / 4 and register 1 the same column of row lane / 4 + 8
+__device__ __forceinline__ void tmem_st16x128_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// four 8x8 matrices of 16-bit elements to shared memory; lane l gives the address of row l % 8 of matrix l / 8
+__device__ __forceinline__ void stmatrix_x4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
 // TMEM address: lane in bits [16,32), column in bits [0,16).
 __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, uint32_t lane, uint32_t col) {
   return base + (lane << 16) + col;
@@ -345,6 +455,25 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// two fp32 values in one 64-bit register and the packed arithmetic on them
+__device__ __forceinline__ uint64_t pack_u32x2(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) { return pack_u32x2(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ float lo_f32x2(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v)); }
+__device__ __forceinline__ float hi_f32x2(uint64_t v) { return __uint_as_float(static_cast<uint32_t>(v >> 32)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
 }
 // packs (lo, hi) as two 16-bit floats: element with the lower index in the low half
 template <bool kBf16>

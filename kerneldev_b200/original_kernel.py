@@ -64,8 +64,8 @@ def _backward(q, k, v, o, lse, d_o, plan: AttentionPlan, sm_scale: float, phases
               like_input: bool = False, deterministic: bool = False):
     """One kd_attn_bwd call: returns (dQ, dK, dV). ``phases`` selects a part of the backward (see
     kd_attn_params.bwd_phases); ``bufs`` = (dq, dk, dv, delta[, dq_acc]) reuses buffers.
-    ``deterministic=False`` selects the fused backward where it exists (head_dim <= 64): one pass over the
-    tiles instead of two, dQ accumulated with fp32 atomics in a (B,H,T,D) scratch."""
+    ``deterministic=False`` selects the fused backward: one pass over the tiles instead of two, dQ accumulated
+    with fp32 additions in a scratch (kd_workspace_bytes_fused)."""
     return _ext.backward(q, k, v, o, lse, d_o, plan._core, sm_scale, phases, list(bufs or ()), like_input, deterministic, HEADS_PER_CTA)
 
 
@@ -149,8 +149,8 @@ def flash_attention(
     of (B,T,H,D) memory (model.py:76-78) the ``transpose(1, 2).contiguous()`` after the call
     (model.py:95) and its counterpart in the backward then copy nothing. The drop-in module uses it.
     deterministic (extension, default False): True forces the two-kernel backward, whose results are
-    bit-identical from run to run; by default head_dim <= 64 takes the fused backward, which forms S and dP
-    once per tile and adds dQ partials with fp32 atomics (dQ then varies in its last bits between runs).
+    bit-identical from run to run; the default is the fused backward, which forms S and dP once per tile and
+    adds dQ partials in fp32 in no fixed order (dQ then varies in its last bits between runs).
 
     float32 q, k, v (the reference's default ``precision="tf32"`` path, original_kernel.py:2106): the tensors
     are rounded to float16 operands -- the 10-bit mantissa tf32 keeps -- the products accumulate in fp32 as
