@@ -8,13 +8,9 @@
 #include "mask_rule.cuh"
 #include "sm100_prims.cuh"
 
-// Register split between the four light warps (producer, MMA issuer, list builder, idle) and the
-// eight compute warps: 4*32*ISSUE + 8*32*COMPUTE must not exceed 65536.
+// Registers of the light warps (producer, MMA issuers) of the two-kernel backward.
 #ifndef KD_REGS_ISSUE
 #define KD_REGS_ISSUE 56
-#endif
-#ifndef KD_REGS_COMPUTE
-#define KD_REGS_COMPUTE 224
 #endif
 // The backward kernels run sixteen compute warps (640 threads, 96 registers each at launch):
 // 4*32*(96 - ISSUE) released registers cover 16*32*(COMPUTE_BWD - 96).

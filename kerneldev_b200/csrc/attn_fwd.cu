@@ -62,13 +62,15 @@ struct FwdCfg {
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
   static constexpr int SMEM_LIST = SMEM_V + VST * TILE_BYTES;      // the pair's work list (<= 128 entries)
   static constexpr int SMEM_UNITS = SMEM_LIST + 128 * 2;           // unit list (<= 256 units)
-  static constexpr int SMEM_CMD = SMEM_UNITS + 256 * 2;            // 256 x {S command, P V command} (uint4 each)
-  static constexpr int SMEM_WCMD = SMEM_CMD + 256 * 2 * 16;        // 2 x 256 softmax commands (u32 each)
+  static constexpr int SMEM_CMD = SMEM_UNITS + 256 * 2;            // 256 issuer commands (u32 each)
+  static constexpr int SMEM_WCMD = SMEM_CMD + 256 * 4;        // 2 x 256 softmax commands (u32 each)
   static constexpr int SMEM_TOTAL = SMEM_WCMD + 2 * 256 * 4;
   static constexpr int SMEM_ALLOC = SMEM_TOTAL + 1024;   // slack for 1024-byte alignment
   static constexpr int CW = KD_TILE;                     // score columns per softmax thread: a whole row
   static constexpr int THREADS = 384;                    // four light warps + one softmax warpgroup per query tile
-  static constexpr int REGS_COMPUTE = KD_REGS_COMPUTE;
+  // registers: 168 per thread at launch; light warps release down to 88, softmax warps take 208
+  static constexpr int REGS_LIGHT = 88, REGS_COMPUTE = 208;
+  static_assert(4 * 32 * REGS_LIGHT + 8 * 32 * REGS_COMPUTE <= THREADS * 168, "register pool");
   // TMEM columns: NBUF score buffers of 128, then O0 and O1 (HD each)
   static constexpr uint32_t TM_O0 = NBUF * 128, TM_O1 = NBUF * 128 + HD;
   static_assert(TM_O1 + HD <= 512, "TMEM budget");
@@ -80,7 +82,7 @@ __device__ __forceinline__ int unit_entry(uint32_t u) { return u & 0x7F; }
 __device__ __forceinline__ int unit_tile(uint32_t u) { return (u >> 7) & 1; }
 __device__ __forceinline__ uint32_t unit_class(uint32_t u) { return (u >> 8) & 3; }
 
-// command flags (word z of a command)
+// command flags
 constexpr uint32_t CMD_WAIT = 8u, CMD_RELEASE = 16u, CMD_ACC = 32u, CMD_TILE1 = 64u;
 // softmax command of a warpgroup's k-th unit: key tile | class << 8 | (unit index mod NBUF) << 10
 __device__ __forceinline__ int wcmd_kt(uint32_t c) { return c & 0xFF; }
@@ -105,7 +107,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t sV = smem_u32(smem + C::SMEM_V);
   uint16_t* sList = reinterpret_cast<uint16_t*>(smem + C::SMEM_LIST);
   uint16_t* sUnits = reinterpret_cast<uint16_t*>(smem + C::SMEM_UNITS);
-  uint4* sCmd = reinterpret_cast<uint4*>(smem + C::SMEM_CMD);   // [u][0] = S command, [u][1] = P V command
+  uint32_t* sCmd = reinterpret_cast<uint32_t*>(smem + C::SMEM_CMD);   // command of every unit
   uint32_t* sWcmd = reinterpret_cast<uint32_t*>(smem + C::SMEM_WCMD);   // [tile][k]
 
   __shared__ __align__(8) uint64_t bar_q_full[C::NQ], bar_q_empty[C::NQ], bar_k_full[C::KST], bar_k_empty[C::KST],
@@ -115,7 +117,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __shared__ int n_units_s, n_own_s[2];
   __shared__ AbortFlag abortf;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   // blockIdx.z walks the pairs from the longest list to the shortest, so the CTAs that take
   // longest are dispatched first
   const int h0 = blockIdx.x * a.G, b = blockIdx.y;
@@ -178,8 +181,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     if (lane == 0) n_units_s = nu;
     __syncwarp();
-    // per-unit commands for the two issuers and for the softmax warpgroups
-    const uint32_t loQ0 = desc_lo_kmajor(sQ), loK0 = desc_lo_kmajor(sK), loV0 = desc_lo_mnmajor(sV);
+    // per-unit commands for the issuers and for the softmax warpgroups
     int cnt_key[2 * C::NBUF];   // units seen so far per (buffer, tile)
 #pragma unroll
     for (int j = 0; j < 2 * C::NBUF; ++j) cnt_key[j] = 0;
@@ -210,20 +212,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (valid) {
         const bool first_of_entry = (u == 0) || unit_entry(sUnits[u - 1]) != e;
         const bool last_of_entry = (u + 1 >= nu) || unit_entry(sUnits[u + 1]) != e;
-        uint4 cs, cp;
         // ring stages and barrier parities run on across heads, so the issuers keep them in counters;
         // the commands carry what is the same for every head
-        cs.x = loQ0 + i * (C::TILE_BYTES >> 4);
-        cs.y = loK0;
-        cs.z = (first_of_entry ? CMD_WAIT : 0u) | (last_of_entry ? CMD_RELEASE : 0u) | (i ? CMD_TILE1 : 0u);
-        cs.w = 0u;
-        cp.x = 0u;
-        cp.y = loV0;
-        cp.z = (first_of_entry ? CMD_WAIT : 0u) | (last_of_entry ? CMD_RELEASE : 0u) | (rank_tile == 0 ? 0u : CMD_ACC) |
-               (i ? CMD_TILE1 : 0u);
-        cp.w = 0u;
-        sCmd[2 * u] = cs;
-        sCmd[2 * u + 1] = cp;
+        sCmd[u] = (first_of_entry ? CMD_WAIT : 0u) | (last_of_entry ? CMD_RELEASE : 0u) | (rank_tile == 0 ? 0u : CMD_ACC) | (i ? CMD_TILE1 : 0u);
         sWcmd[i * 256 + rank_tile] = (sList[e] & 0xFFu) | (unit_class(un) << 8) | (static_cast<uint32_t>(buf) << 10);
         (void)rank_key;
       }
@@ -239,11 +230,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tbase = tmem_base_s;
+  // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   const int U = n_units_s;
+  auto wait = [&](uint64_t& b64, uint32_t parity, uint32_t site) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(smem_u32(&b64), parity, &abortf, site));
+  };
 
   if (warp < 4) {
-    reg_dealloc<KD_REGS_ISSUE>();
+    reg_dealloc<C::REGS_LIGHT>();
     if (warp == 0 && lane == 0 && n > 0) {
       // ------------------------------ TMA producer ------------------------------
       tma_prefetch_desc(&tmQ);
@@ -311,45 +305,31 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int e = max(0, v_cnt - C::VST); e < v_cnt; ++e) drain_wait(smem_u32(&bar_v_full[e % C::VST]), (e / C::VST) & 1);
         for (int hh = max(0, q_loaded - C::NQ); hh < q_loaded; ++hh) drain_wait(smem_u32(&bar_q_full[hh % C::NQ]), (hh / C::NQ) & 1);
       }
-    } else if (warp == 3 && lane == 0 && U > 0) {
+    } else if (warp == 3 && U > 0) {
       // ------------------------------ S issuer ------------------------------
+      // (both issuers: all lanes follow the control flow and one elected lane issues, see mma_ss_uniform)
       const uint32_t idesc_s = make_idesc_f16(kBf16, 0, 0, KD_TILE, KD_TILE);
-      const uint32_t hi = desc_hi_sw128();
+      const uint32_t hi = desc_hi_sw128(), lo_q = desc_lo_kmajor(sQ), lo_k = desc_lo_kmajor(sK);
+      constexpr uint32_t T16 = C::TILE_BYTES >> 4;
       bool ok = true;
       int buf = 0, round = 0;      // the g-th unit over all heads uses buffer g % NBUF in round g / NBUF
       int kstage = 0;
       uint32_t kparity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
         const int qb = hh % C::NQ;
-        ok = mbar_wait(smem_u32(&bar_q_full[qb]), (hh / C::NQ) & 1, &abortf, W_F_QFULL);
-        const uint32_t q_off = qb * (2 * C::TILE_BYTES >> 4);
-        for (int u = 0; u < U && ok; ++u) {
-          const uint4 c = sCmd[2 * u];
-          // operands of the unit, formed ahead of the waits
-          const uint32_t d = tbase + buf * 128;
-          const uint32_t qlo = c.x + q_off, klo = c.y + kstage * (C::TILE_BYTES >> 4);
-          uint64_t qdesc[HD / 16], kdesc[HD / 16];
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) {
-            qdesc[kk] = desc64(qlo + koff_kmajor(kk), hi);
-            kdesc[kk] = desc64(klo + koff_kmajor(kk), hi);
-          }
-          if (round > 0) {
-            // the buffer is free once P V of the unit that used it in the previous round has been issued
-            ok = mbar_wait(smem_u32(&bar_pv_issued[buf]), (round - 1) & 1, &abortf, W_F_PVISSUED);
-            if (!ok) break;
-          }
-          if (c.z & CMD_WAIT) {
-            ok = mbar_wait(smem_u32(&bar_k_full[kstage]), kparity, &abortf, W_F_KFULL);
-            if (!ok) break;
-          }
+        if (!(ok = wait(bar_q_full[qb], (hh / C::NQ) & 1, W_F_QFULL))) break;
+        for (int u = 0; u < U; ++u) {
+          const uint32_t z = __reduce_or_sync(0xffffffffu, sCmd[u]);
+          // the buffer is free once P V of the unit that used it in the previous round has been issued
+          if (round > 0 && !(ok = wait(bar_pv_issued[buf], (round - 1) & 1, W_F_PVISSUED))) break;
+          if ((z & CMD_WAIT) && !(ok = wait(bar_k_full[kstage], kparity, W_F_KFULL))) break;
           tc_fence_after_sync();
-          mma_ss64<false>(d, qdesc[0], kdesc[0], idesc_s);
+          const uint32_t qlo = lo_q + qb * (2 * T16) + ((z & CMD_TILE1) ? T16 : 0u), klo = lo_k + kstage * T16;
 #pragma unroll
-          for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(d, qdesc[kk], kdesc[kk], idesc_s);
-          mma_commit(smem_u32(&bar_s_full[2 * buf + ((c.z & CMD_TILE1) ? 1 : 0)]));
-          if (c.z & CMD_RELEASE) {
-            mma_commit(smem_u32(&bar_k_empty[kstage]));
+          for (int kk = 0; kk < HD / 16; ++kk) mma_ss_uniform(buf * 128, qlo + koff_kmajor(kk), klo + koff_kmajor(kk), hi, idesc_s, kk > 0 ? 1u : 0u);
+          commit_uniform(smem_u32(&bar_s_full[2 * buf + ((z & CMD_TILE1) ? 1 : 0)]));
+          if (z & CMD_RELEASE) {
+            commit_uniform(smem_u32(&bar_k_empty[kstage]));
             if (++kstage == C::KST) { kstage = 0; kparity ^= 1; }
           }
           if (++buf == C::NBUF) {
@@ -357,55 +337,38 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             ++round;
           }
         }
-        if (ok) mma_commit(smem_u32(&bar_q_empty[qb]));   // Q of this head is no longer read once the MMAs above are done
+        if (ok) commit_uniform(smem_u32(&bar_q_empty[qb]));   // Q of this head is no longer read once the MMAs above are done
       }
-    } else if (warp == 1 && lane == 0 && U > 0) {
+    } else if (warp == 1 && U > 0) {
       // ------------------------------ P V issuer ------------------------------
       const uint32_t idesc_o = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);
-      const uint32_t hi = desc_hi_sw128();
+      const uint32_t hi = desc_hi_sw128(), lo_v = desc_lo_mnmajor(sV);
+      constexpr uint32_t T16 = C::TILE_BYTES >> 4;
       bool ok = true;
       int buf = 0, vstage = 0;
       uint32_t round_parity = 0, vparity = 0;
       for (int hh = 0; hh < nh && ok; ++hh) {
-        for (int u = 0; u < U && ok; ++u) {
-          const uint4 c = sCmd[2 * u + 1];
-          // operands of the unit, formed ahead of the waits
-          const uint32_t vlo = c.y + vstage * (C::TILE_BYTES >> 4);
-          const uint32_t aP = tbase + buf * 128;
-          uint64_t vdesc[KD_TILE / 16];
-          uint32_t pop[KD_TILE / 16];
-#pragma unroll
-          for (int kk = 0; kk < KD_TILE / 16; ++kk) {
-            vdesc[kk] = desc64(vlo + koff_mnmajor(kk), hi);
-            pop[kk] = aP + kk * 8;   // P of 16 keys = 8 packed columns at the start of the score buffer
-          }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_F_PFULL);
-          if (!ok) break;
-          if (c.z & CMD_WAIT) {
-            ok = mbar_wait(smem_u32(&bar_v_full[vstage]), vparity, &abortf, W_F_VFULL);
-            if (!ok) break;
-          }
-          const uint32_t i = (c.z & CMD_TILE1) ? 1u : 0u;
-          const uint32_t acc0 = (c.z & CMD_ACC) ? 1u : 0u;
-          if (acc0 == 0u && hh > 0) {
-            // first product of this query tile for a new head overwrites O_i: the softmax warpgroup must
-            // have read the previous head's result out of it
-            ok = mbar_wait(smem_u32(&bar_o_free[i]), (hh - 1) & 1, &abortf, W_F_OFREE);
-            if (!ok) break;
-          }
+        for (int u = 0; u < U; ++u) {
+          const uint32_t z = __reduce_or_sync(0xffffffffu, sCmd[u]);
+          const uint32_t i = (z & CMD_TILE1) ? 1u : 0u;
+          if ((z & CMD_WAIT) && !(ok = wait(bar_v_full[vstage], vparity, W_F_VFULL))) break;
+          // first product of this query tile for a new head overwrites O_i: the softmax warpgroup must have read the previous
+          // head's result out of it
+          if ((z & CMD_ACC) == 0u && hh > 0 && !(ok = wait(bar_o_free[i], (hh - 1) & 1, W_F_OFREE))) break;
+          if (!(ok = wait(bar_p_full[buf], round_parity, W_F_PFULL))) break;
           tc_fence_after_sync();
-          const uint32_t dO = tbase + C::TM_O0 + i * HD;
-          mma_ts64_p(dO, pop[0], vdesc[0], idesc_o, acc0);
+          const uint32_t vlo = lo_v + vstage * T16, dO = C::TM_O0 + i * HD, acc0 = (z & CMD_ACC) ? 1u : 0u;
 #pragma unroll
-          for (int kk = 1; kk < KD_TILE / 16; ++kk) mma_ts64<true>(dO, pop[kk], vdesc[kk], idesc_o);
-          mma_commit(smem_u32(&bar_pv_done[i]));
-          if (c.z & CMD_RELEASE) {
-            mma_commit(smem_u32(&bar_v_empty[vstage]));
+          for (int kk = 0; kk < KD_TILE / 16; ++kk)   // P of 16 keys = 8 packed columns at the start of the score buffer
+            mma_ts_uniform(dO, buf * 128 + kk * 8, vlo + koff_mnmajor(kk), hi, idesc_o, kk > 0 ? 1u : acc0);
+          commit_uniform(smem_u32(&bar_pv_done[i]));
+          if (z & CMD_RELEASE) {
+            commit_uniform(smem_u32(&bar_v_empty[vstage]));
             if (++vstage == C::VST) { vstage = 0; vparity ^= 1; }
           }
           // hand the buffer back to the S issuer, ordered after the MMAs above
           tc_fence_before_sync();
-          mbar_arrive(smem_u32(&bar_pv_issued[buf]));
+          if (elect_one()) mbar_arrive(smem_u32(&bar_pv_issued[buf]));
           if (++buf == C::NBUF) {
             buf = 0;
             round_parity ^= 1;
@@ -425,8 +388,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int qi = qtile * KD_TILE + row;  // token index of this thread's query
     const bool tile_valid = qtile < a.NT;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t tO = tbase + lane_base + (i == 0 ? C::TM_O0 : C::TM_O1);   // this thread's row of O
+    const uint32_t tO = lane_base + (i == 0 ? C::TM_O0 : C::TM_O1);   // this thread's row of O
     const float c = a.scale_log2;
+    const uint64_t c2 = pack_f32x2(c, c);
 
     const uint32_t qd = tile_valid ? a.desc[(size_t)b * a.Tpad + qi] : 0u;
     bool ok = true;
@@ -471,10 +435,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int kt = wcmd_kt(cmd);
       int buf = wcmd_buf(cmd) + buf_off;
       if (buf >= C::NBUF) buf -= C::NBUF;
-      const uint32_t tS = tbase + lane_base + buf * 128;
-      ok = mbar_wait(smem_u32(&bar_s_full[2 * buf + i]), (sfull_par >> buf) & 1u, &abortf, W_F_SFULL);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      const uint32_t tS = lane_base + buf * 128;
+      if (!(ok = wait(bar_s_full[2 * buf + i], (sfull_par >> buf) & 1u, W_F_SFULL))) break;
       sfull_par ^= 1u << buf;
       tc_fence_after_sync();
 
@@ -543,38 +505,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * c);
       const bool need_rescale = (nact > 0) && (m_new != m);
-      const float neg_mc = -m_use * c;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[CW / 2];
+      const uint64_t neg_mc2 = pack_f32x2(-m_use * c, -m_use * c);
+      uint64_t sum2[2] = {0u, 0u};
 #pragma unroll
-      for (int j = 0; j < CW; j += 4) {
-        const float p0 = fast_exp2(fmaf(sc[j], c, neg_mc));
-        const float p1 = fast_exp2(fmaf(sc[j + 1], c, neg_mc));
-        const float p2 = fast_exp2(fmaf(sc[j + 2], c, neg_mc));
-        const float p3 = fast_exp2(fmaf(sc[j + 3], c, neg_mc));
-        sum4[0] += p0;
-        sum4[1] += p1;
-        sum4[2] += p2;
-        sum4[3] += p3;
-        pk[j / 2] = pack2<kBf16>(p0, p1);
-        pk[j / 2 + 1] = pack2<kBf16>(p2, p3);
+      for (int cb = 0; cb < NW; ++cb) {   // 32 columns at a time; P over the start of this thread's own score columns
+        uint32_t pk[16];
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const uint64_t x = fma_f32x2(pack_f32x2(sc[cb * 32 + j], sc[cb * 32 + j + 1]), c2, neg_mc2);
+          const float p0 = fast_exp2(lo_f32x2(x)), p1 = fast_exp2(hi_f32x2(x));
+          sum2[(j / 2) & 1] = add_f32x2(sum2[(j / 2) & 1], pack_f32x2(p0, p1));
+          pk[j / 2] = pack2<kBf16>(p0, p1);
+        }
+        tmem_st16(tS + cb * 16, pk);
       }
-      const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      l = l * alpha + sum;
+      const uint64_t sum_pair = add_f32x2(sum2[0], sum2[1]);
+      l = l * alpha + (lo_f32x2(sum_pair) + hi_f32x2(sum_pair));
       m = m_new;
-#pragma unroll
-      for (int cb = 0; cb < CW / 64; ++cb) {
-        uint32_t r[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = pk[cb * 32 + j];
-        tmem_st32(tS + cb * 32, r);   // P over the start of this thread's own score columns
-      }
       if (nact > 0) {
         // O_i may be touched only after the previous P V product of this query tile has completed;
         // the wait is taken for every unit so that no phase of the barrier goes unobserved
-        ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, W_F_PVDONE);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        if (!(ok = wait(bar_pv_done[i], (pv_seen - 1) & 1, W_F_PVDONE))) break;
       }
       if (__any_sync(0xffffffffu, need_rescale)) {
         tc_fence_after_sync();
@@ -602,8 +553,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
     // epilogue of this head: normalise, convert, store this thread's share of O, and LSE
     if (nact > 0) {
-      ok = mbar_wait(smem_u32(&bar_pv_done[i]), (pv_seen - 1) & 1, &abortf, W_F_PVDONE);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = wait(bar_pv_done[i], (pv_seen - 1) & 1, W_F_PVDONE);
     }
     if (ok && tile_valid && qi < a.T) {
       a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
@@ -636,7 +586,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tbase, 512);
+  if (warp == 1) tmem_dealloc(0, 512);
   if (tid == 0) report_abort(&abortf, a.status);
 }
 
