@@ -123,8 +123,9 @@ typedef struct kd_attn_params {
   float* dq_acc;      /* KD_BWD_FUSED: (B,H,T,W) contiguous fp32 scratch, W = 64 for D <= 64 and 128 above
                          (kd_workspace_bytes_fused gives its size); the library zeroes it itself. Ignored otherwise. */
   int32_t heads_per_cta; /* 0: chosen by the library from the grid size. n >= 1: every CTA handles n heads
-                         one after the other (they share the plan's work list); a tuning and test knob. The fused
-                         backward takes its work items dynamically and ignores it. */
+                         one after the other (they share the plan's work list); a tuning and test knob of the
+                         deterministic backward. The forward and the fused backward take their work items
+                         dynamically and ignore it. */
 } kd_attn_params;
 
 /* Size and layout of a plan for B sequences of T tokens. */
