@@ -217,6 +217,28 @@ int kd_span_mean(int32_t backward, const void* a, int64_t a_sb, int64_t a_st, vo
                  int32_t B, int32_t T, int32_t C, int32_t S, int32_t dtype, const int32_t* starts,
                  const int32_t* ends, const int32_t* n_starts, const int32_t* n_ends, void* stream);
 
+/* Scores of the cocktail-party head and their gradient, from markers ranked before (model.py:258-296):
+ *   scores[b, j] = <x[b, first_mask[b], :], h[b, j, :]> with h as for kd_span_mean; 0 without a [MASK]. */
+typedef struct {
+  const void* x;         /* forward: (B,T,C) with element strides x_sb, x_st and unit stride along C */
+  int64_t x_sb, x_st;
+  int32_t B, T, C, S;    /* S: padded span count, the largest n_starts of the batch */
+  int32_t dtype;         /* KD_F16 / KD_BF16 / KD_F32, of x, scores and gx; sums in fp32 */
+  const int32_t *starts, *ends, *n_starts, *n_ends, *first_mask;   /* of kd_cocktail_index */
+  void* scores;          /* (B,S) contiguous: forward out; backward in: the gradient of the scores */
+  float* h;              /* (B,S+1,C) contiguous fp32: the means and, as row S, the embedding at the [MASK]. Forward out
+                            (null: not needed, there will be no backward); backward in */
+  void* gx;              /* backward out: (B,T,C) contiguous */
+} kd_cocktail;
+
+/* kd_span_index, which also writes the [SPAN] counts to counts_host (B int32 of pinned host memory; they are there once
+ * the stream has been synchronised). */
+int kd_cocktail_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span, int64_t tok_es,
+                      int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
+                      int32_t* first_mask, int32_t* counts_host, void* stream);
+int kd_cocktail_scores(const kd_cocktail* p, void* stream);
+int kd_cocktail_grad(const kd_cocktail* p, void* stream);
+
 /* Message for the last negative return value on this host thread. */
 const char* kd_last_error(void);
 

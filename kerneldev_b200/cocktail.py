@@ -6,15 +6,15 @@ the tokens between the j-th [SPAN] and the j-th [ES], ``scores = einsum('bd,bnd-
 markers with ``.nonzero()`` / ``torch.unique`` and fills ``h_spans`` in a Python double loop over rows
 and spans (one small ``mean`` kernel and several host synchronisations per span).
 
-``span_means`` does the marker ranking and the means with three kernels (one of them only in the
-backward) and a single host read (the padded span count, which fixes the output shape as in the
-reference); ``cocktail_scores`` is the whole block. Both are differentiable with respect to x_embed.
+``cocktail_scores`` is the whole block: the markers' ranking and the scores are one kernel each, the gradient is a
+third, and the host waits once, for the padded span count that fixes the output shape (as in the reference).
+``span_means`` gives the means alone. Both are differentiable with respect to x_embed.
 """
 from __future__ import annotations
 
 import torch
 
-from . import _capi
+from . import _capi, _host
 from .metadata import SPECIAL_TOKENS
 
 _DT = {torch.float16: _capi.KD_F16, torch.bfloat16: _capi.KD_BF16, torch.float32: _capi.KD_F32}
@@ -92,9 +92,5 @@ def span_means(x_embed: torch.Tensor, tokens: torch.Tensor, special_tokens=None,
 def cocktail_scores(x_embed: torch.Tensor, tokens: torch.Tensor, special_tokens=None):
     """scores (batch, max_spans) of model.py:262-296: <embedding at the row's first [MASK], mean embedding
     of each of its spans>; rows without a [MASK] score 0."""
-    index = span_index(tokens, special_tokens)
-    h_spans = span_means(x_embed, tokens, special_tokens, index)
-    first_mask = index[4].long()
-    rows = torch.arange(x_embed.shape[0], device=x_embed.device)
-    h_context = x_embed[rows, first_mask.clamp(min=0)] * (first_mask >= 0).unsqueeze(1).to(x_embed.dtype)
-    return torch.einsum("bd,bnd->bn", h_context, h_spans)
+    st = SPECIAL_TOKENS if special_tokens is None else special_tokens
+    return _host.load().cocktail_scores(x_embed, tokens, st["[SPAN]"], st["[ES]"], st["[MASK]"])

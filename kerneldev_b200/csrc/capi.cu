@@ -244,9 +244,9 @@ int kd_metadata_from_tokens(const int64_t* tokens, int64_t stride_b, int32_t B, 
                          static_cast<cudaStream_t>(stream));
 }
 
-int kd_span_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span, int64_t tok_es,
-                  int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
-                  int32_t* first_mask, void* stream) {
+int kd_cocktail_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span, int64_t tok_es,
+                      int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
+                      int32_t* first_mask, int32_t* counts_host, void* stream) {
   if (B < 0 || T < 0) return set_error(KD_ERR_ARG, "bad shape B=%d T=%d", B, T);
   if (B == 0 || T == 0) return 0;
   if (!tokens || !starts || !ends || !n_starts || !n_ends || !first_mask) return set_error(KD_ERR_ARG, "null pointer");
@@ -254,7 +254,38 @@ int kd_span_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T,
   int rc = check_device();
   if (rc) return rc;
   return launch_span_index(tokens, stride_b, B, T, tok_span, tok_es, tok_mask, starts, ends, n_starts, n_ends, first_mask,
-                           static_cast<cudaStream_t>(stream));
+                           counts_host, static_cast<cudaStream_t>(stream));
+}
+
+int kd_span_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span, int64_t tok_es,
+                  int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
+                  int32_t* first_mask, void* stream) {
+  return kd_cocktail_index(tokens, stride_b, B, T, tok_span, tok_es, tok_mask, starts, ends, n_starts, n_ends, first_mask, nullptr, stream);
+}
+
+static int check_cocktail(const kd_cocktail* p, bool backward) {
+  if (!p) return set_error(KD_ERR_ARG, "params is null");
+  if (p->B < 0 || p->T < 0 || p->C < 0 || p->S < 0) return set_error(KD_ERR_ARG, "bad shape B=%d T=%d C=%d S=%d", p->B, p->T, p->C, p->S);
+  if (p->B > 65535) return set_error(KD_ERR_LIMIT, "B=%d exceeds 65535", p->B);
+  if (p->dtype != KD_F16 && p->dtype != KD_BF16 && p->dtype != KD_F32) return set_error(KD_ERR_ARG, "dtype %d not supported", p->dtype);
+  const bool empty = p->B == 0 || p->T == 0 || p->C == 0 || p->S == 0;
+  if (!empty && (!p->starts || !p->ends || !p->n_starts || !p->n_ends || !p->first_mask || !p->scores || (backward ? !p->h || !p->gx : !p->x)))
+    return set_error(KD_ERR_ARG, "null pointer");
+  return empty ? 1 : 0;
+}
+
+int kd_cocktail_scores(const kd_cocktail* p, void* stream) {
+  int rc = check_cocktail(p, false);
+  if (rc) return rc > 0 ? 0 : rc;
+  if ((rc = check_device()) != 0) return rc;
+  return launch_cocktail(false, *p, static_cast<cudaStream_t>(stream));
+}
+
+int kd_cocktail_grad(const kd_cocktail* p, void* stream) {
+  int rc = check_cocktail(p, true);
+  if (rc) return rc > 0 ? 0 : rc;
+  if ((rc = check_device()) != 0) return rc;
+  return launch_cocktail(true, *p, static_cast<cudaStream_t>(stream));
 }
 
 int kd_span_mean(int32_t backward, const void* a, int64_t a_sb, int64_t a_st, void* out, int64_t o_sb, int64_t o_st,

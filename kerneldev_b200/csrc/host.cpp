@@ -35,6 +35,9 @@ struct Library {
   decltype(&kd_attn_bwd) attn_bwd = nullptr;
   decltype(&kd_hadamard) hadamard = nullptr;
   decltype(&kd_metadata_from_tokens) metadata_from_tokens = nullptr;
+  decltype(&kd_cocktail_index) cocktail_index = nullptr;
+  decltype(&kd_cocktail_scores) cocktail_scores = nullptr;
+  decltype(&kd_cocktail_grad) cocktail_grad = nullptr;
   decltype(&kd_last_error) last_error = nullptr;
 };
 Library lib;
@@ -51,6 +54,9 @@ void bind(const py::dict& a) {
   take(lib.attn_bwd, a, "kd_attn_bwd");
   take(lib.hadamard, a, "kd_hadamard");
   take(lib.metadata_from_tokens, a, "kd_metadata_from_tokens");
+  take(lib.cocktail_index, a, "kd_cocktail_index");
+  take(lib.cocktail_scores, a, "kd_cocktail_scores");
+  take(lib.cocktail_grad, a, "kd_cocktail_grad");
   take(lib.last_error, a, "kd_last_error");
 }
 
@@ -507,6 +513,109 @@ std::tuple<Tensor, Tensor, Tensor> metadata_from_tokens(const Tensor& tokens_, i
   return {in_span, span_id, is_prefix};
 }
 
+// ---- cocktail-party head ---------------------------------------------------------------------------------------
+
+// gradient of cocktail_scores: one kernel that writes every row of grad_x
+struct CocktailBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable h, index;
+  kd_cocktail p;   // shapes, type and the index pointers (into `index`)
+  Tensor like;     // an empty tensor with x's options
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list out(1);
+    if (!grads[0].defined()) return out;
+    Tensor th, ti;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      th = h.unpack();
+      ti = index.unpack();
+    }
+    at::NoGradGuard no_grad;
+    const Tensor ds = grads[0].contiguous();
+    // without a span nothing reaches x, and there is no kernel to write the zeros
+    Tensor gx = p.S == 0 ? at::zeros({p.B, p.T, p.C}, like.options()) : at::empty({p.B, p.T, p.C}, like.options());
+    kd_cocktail q = p;
+    q.scores = ds.data_ptr();
+    q.h = th.data_ptr<float>();
+    q.gx = gx.data_ptr();
+    c10::cuda::CUDAGuard guard(gx.device());
+    check(lib.cocktail_grad(&q, at::cuda::getCurrentCUDAStream()));
+    out[0] = gx;
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    h.reset_data();
+    index.reset_data();
+  }
+  std::string name() const override { return "CocktailScoresBackward"; }
+};
+
+Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span, int64_t tok_es, int64_t tok_mask) {
+  KD_VALUE(tokens_.dim() == 2 && tokens_.scalar_type() == at::kLong, "tokens must be an int64 tensor of shape (batch, time)");
+  TORCH_CHECK(tokens_.is_cuda(), "span_index runs on CUDA devices only; there is no CPU path");
+  const auto t = x_.scalar_type();
+  KD_VALUE(x_.dim() == 3 && (t == at::kHalf || t == at::kBFloat16 || t == at::kFloat), "x_embed must be (batch, time, dim) in float16, bfloat16 or float32");
+  TORCH_CHECK(x_.is_cuda(), "span_means runs on CUDA devices only; there is no CPU path");
+  KD_VALUE(x_.size(0) == tokens_.size(0) && x_.size(1) == tokens_.size(1) && x_.device() == tokens_.device(),
+           "x_embed and tokens must have the same batch, time and device");
+  const int64_t B = x_.size(0), T = x_.size(1), C = x_.size(2);
+  const bool track = at::GradMode::is_enabled() && x_.requires_grad();
+  Tensor scores, h, index;
+  kd_cocktail p{};
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor tokens = tokens_.stride(1) == 1 ? tokens_ : tokens_.contiguous();
+    const Tensor x = x_.stride(2) == 1 ? x_ : x_.contiguous();
+    index = at::empty({2 * B * T + 3 * B}, tokens.options().dtype(at::kInt));
+    int32_t* words = index.data_ptr<int32_t>();
+    int32_t *starts = words, *ends = words + B * T, *n_starts = words + 2 * B * T, *n_ends = n_starts + B, *first_mask = n_ends + B;
+    Tensor counts = at::empty({B}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    c10::cuda::CUDAGuard guard(x.device());
+    auto stream = at::cuda::getCurrentCUDAStream();
+    check(lib.cocktail_index(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(T, 1), static_cast<int32_t>(B),
+                             static_cast<int32_t>(T), tok_span, tok_es, tok_mask, starts, ends, n_starts, n_ends, first_mask,
+                             counts.data_ptr<int32_t>(), stream));
+    int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
+    if (B > 0 && T > 0) {
+      {
+        py::gil_scoped_release release;
+        C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+      }
+      for (int64_t b = 0; b < B; ++b) S = std::max(S, counts.data_ptr<int32_t>()[b]);
+    }
+    scores = C == 0 ? at::zeros({B, S}, x.options()) : at::empty({B, S}, x.options());
+    if (track) h = at::empty({B, S + 1, C}, x.options().dtype(at::kFloat));
+    p.x = x.data_ptr();
+    p.x_sb = x.stride(0);
+    p.x_st = x.stride(1);
+    p.B = static_cast<int32_t>(B);
+    p.T = static_cast<int32_t>(T);
+    p.C = static_cast<int32_t>(C);
+    p.S = S;
+    p.dtype = t == at::kFloat ? KD_F32 : dtype_code(t);
+    p.starts = starts;
+    p.ends = ends;
+    p.n_starts = n_starts;
+    p.n_ends = n_ends;
+    p.first_mask = first_mask;
+    p.scores = scores.data_ptr();
+    p.h = track ? h.data_ptr<float>() : nullptr;
+    check(lib.cocktail_scores(&p, stream));
+  }
+  if (track) {
+    auto node = std::shared_ptr<CocktailBackward>(new CocktailBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x_));
+    node->p = p;
+    node->p.x = nullptr;
+    node->like = at::empty({0}, x_.options());
+    torch::autograd::set_history(scores, node);
+    node->h = torch::autograd::SavedVariable(h, false);
+    node->index = torch::autograd::SavedVariable(index, false);
+  }
+  return scores;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -545,4 +654,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("hadamard", &hadamard);
   m.def("attention", &attention);
   m.def("metadata_from_tokens", &metadata_from_tokens);
+  m.def("cocktail_scores", &cocktail_scores);
 }
