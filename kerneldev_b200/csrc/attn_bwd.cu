@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
   constexpr int RPB = 256 / TPR;   // rows per block and iteration
   const size_t rows = (size_t)a.B * a.H * a.T;
   const int sub = threadIdx.x % TPR;
+  pdl_wait();
+  pdl_launch_dependents();
   // the loop bound is the same for every thread of the block: the shuffles below need full warps
   for (size_t base = (size_t)blockIdx.x * RPB; base < rows; base += (size_t)gridDim.x * RPB) {
     const size_t r = base + threadIdx.x / TPR;
@@ -177,6 +179,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();
+  pdl_launch_dependents();
   const uint32_t tbase = tmem_base_s;
   const int na = n_act_s;
 
@@ -539,6 +543,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();
+  pdl_launch_dependents();
   const uint32_t tbase = tmem_base_s;
   const uint16_t* list = sList;
 
@@ -936,16 +942,15 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
     const size_t rows = (size_t)p.B * p.H * p.T;
     const int rows_per_block = 256 / (HD / 8);
     const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-    attn_bwd_delta_kernel<HD, kBf16><<<blocks, 256, 0, stream>>>(a);
-    if (!fused) kq<<<grid, C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, a);
+    e = launch(attn_bwd_delta_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
+    if (!fused && e == cudaSuccess) e = launch(kq, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
-  if (fused) {
+  if (fused && e == cudaSuccess) {
     // bwd_phases 1: the delta kernel alone (it also zeroes dq_acc); 2: the fused kernel and the conversion
     if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, stream);
-  } else if (phases & 2) {
-    kk<<<grid, C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, a);
+  } else if ((phases & 2) && e == cudaSuccess) {
+    e = launch(kk, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
-  e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }

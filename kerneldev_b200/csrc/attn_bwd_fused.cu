@@ -181,6 +181,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();
+  pdl_launch_dependents();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
     return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
@@ -983,6 +985,8 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
   constexpr int TPR = HD / 8;
   const size_t rows = (size_t)a.B * a.H * a.T;
   const int sub = threadIdx.x % TPR;
+  pdl_wait();
+  pdl_launch_dependents();
   for (size_t r = (size_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR; r < rows; r += (size_t)gridDim.x * (256 / TPR)) {
     const int t = static_cast<int>(r % a.T);
     const int h = static_cast<int>((r / a.T) % a.H);
@@ -1032,12 +1036,11 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
     launch_regs = fa.numRegs;
   }
   if (launch_regs < C::REGS_LAUNCH) return set_error(KD_ERR_DEVICE, "fused bwd was built with %d registers per thread, needs %d", launch_regs, C::REGS_LAUNCH);
-  kern<<<static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
+  e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
   const size_t rows = (size_t)a.B * a.H * a.T;
   const int rows_per_block = 256 / (HD / 8);
   const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-  attn_bwd_dq_convert_kernel<HD, kBf16><<<blocks, 256, 0, stream>>>(a);
-  e = cudaGetLastError();
+  if (e == cudaSuccess) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }

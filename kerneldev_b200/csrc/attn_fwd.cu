@@ -149,6 +149,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_wait();
+  pdl_launch_dependents();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
     return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
@@ -664,8 +666,7 @@ static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
-  kern<<<static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream>>>(tmQ, tmK, tmV, a);
-  e = cudaGetLastError();
+  e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_fwd_kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }

@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "sm100_prims.cuh"
 
 namespace kd {
 
@@ -29,6 +30,8 @@ __global__ void __launch_bounds__(SI_THREADS)
 span_index_kernel(const int64_t* __restrict__ tokens, int64_t stride_b, int T, int64_t tok_span, int64_t tok_es,
                   int64_t tok_mask, int32_t* __restrict__ starts, int32_t* __restrict__ ends, int32_t* __restrict__ n_starts,
                   int32_t* __restrict__ n_ends, int32_t* __restrict__ first_mask, int32_t* __restrict__ counts_host) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ int s_span[SI_WARPS], s_es[SI_WARPS], s_mask[SI_WARPS];
   const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t* x = tokens + (size_t)b * stride_b;
@@ -138,6 +141,8 @@ cocktail_scores_kernel(const E* __restrict__ x, int64_t x_sb, int64_t x_st, int 
                        const int32_t* __restrict__ starts, const int32_t* __restrict__ ends, const int32_t* __restrict__ n_starts,
                        const int32_t* __restrict__ n_ends, const int32_t* __restrict__ first_mask, E* __restrict__ scores,
                        float* __restrict__ h) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float part[CK_SCORE_THREADS * V];   // [group][column of the chunk]
   __shared__ float s_dot[CK_SCORE_THREADS / 32];
   const int j = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
@@ -198,6 +203,8 @@ __global__ void __launch_bounds__(CK_THREADS)
 cocktail_grad_kernel(const E* __restrict__ ds, const float* __restrict__ h, int S, int T, int C, int tpr,
                      const int32_t* __restrict__ starts, const int32_t* __restrict__ ends, const int32_t* __restrict__ n_starts,
                      const int32_t* __restrict__ n_ends, const int32_t* __restrict__ first_mask, E* __restrict__ gx) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float coef[CK_TOKENS];
   const int b = blockIdx.y, tb = blockIdx.x * CK_TOKENS, tid = threadIdx.x;
   const int n = min(min(n_starts[b], n_ends[b]), S), fm = first_mask[b];
@@ -246,6 +253,8 @@ __global__ void __launch_bounds__(CK_THREADS)
 span_mean_fwd_kernel(const E* __restrict__ x, int64_t x_sb, int64_t x_st, int T, int C, const int32_t* __restrict__ starts,
                      const int32_t* __restrict__ ends, const int32_t* __restrict__ n_starts,
                      const int32_t* __restrict__ n_ends, E* __restrict__ h, int S) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int j = blockIdx.x, b = blockIdx.y;
   int st = 0, ed = 0;
   const bool live = span_pair(starts, ends, n_starts, n_ends, b, j, T, st, ed);
@@ -267,6 +276,8 @@ __global__ void __launch_bounds__(CK_THREADS)
 span_mean_bwd_kernel(const E* __restrict__ gh, int S, int T, int C, const int32_t* __restrict__ starts,
                      const int32_t* __restrict__ ends, const int32_t* __restrict__ n_starts,
                      const int32_t* __restrict__ n_ends, E* __restrict__ gx, int64_t gx_sb, int64_t gx_st) {
+  pdl_wait();
+  pdl_launch_dependents();
   constexpr int TT = 8;
   const int b = blockIdx.y, tb = blockIdx.x * TT;
   const int n = min(min(n_starts[b], n_ends[b]), S);
@@ -300,9 +311,8 @@ int launch_span_index(const int64_t* tokens, int64_t stride_b, int B, int T, int
                       int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
                       int32_t* first_mask, int32_t* counts_host, cudaStream_t stream) {
   if (B == 0 || T == 0) return 0;
-  span_index_kernel<<<B, SI_THREADS, 0, stream>>>(tokens, stride_b, T, tok_span, tok_es, tok_mask, starts, ends, n_starts,
+  const cudaError_t e = launch(span_index_kernel, B, SI_THREADS, 0, stream, tokens, stride_b, T, tok_span, tok_es, tok_mask, starts, ends, n_starts,
                                                   n_ends, first_mask, counts_host);
-  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "span_index_kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -315,16 +325,16 @@ static int threads_per_row(int C, int V, int most) {
 }
 
 template <typename E, int V>
-static void scores_t(const kd_cocktail& p, cudaStream_t stream) {
+static cudaError_t scores_t(const kd_cocktail& p, cudaStream_t stream) {
   const int tpr = threads_per_row(p.C, V, CK_SCORE_THREADS);
   const int threads = std::min(CK_SCORE_THREADS, std::max(32, tpr * 32));   // at most 32 groups: they are added up one by one
-  cocktail_scores_kernel<E, V><<<dim3(p.S, p.B), threads, 0, stream>>>(
+  return launch(cocktail_scores_kernel<E, V>, dim3(p.S, p.B), threads, 0, stream,
       static_cast<const E*>(p.x), p.x_sb, p.x_st, p.T, p.C, p.S, tpr, p.starts, p.ends, p.n_starts, p.n_ends, p.first_mask,
       static_cast<E*>(p.scores), p.h);
 }
 template <typename E, int V>
-static void grad_t(const kd_cocktail& p, cudaStream_t stream) {
-  cocktail_grad_kernel<E, V><<<dim3((p.T + CK_TOKENS - 1) / CK_TOKENS, p.B), CK_THREADS, 0, stream>>>(
+static cudaError_t grad_t(const kd_cocktail& p, cudaStream_t stream) {
+  return launch(cocktail_grad_kernel<E, V>, dim3((p.T + CK_TOKENS - 1) / CK_TOKENS, p.B), CK_THREADS, 0, stream,
       static_cast<const E*>(p.scores), p.h, p.S, p.T, p.C, threads_per_row(p.C, V, CK_THREADS), p.starts, p.ends, p.n_starts, p.n_ends,
       p.first_mask, static_cast<E*>(p.gx));
 }
@@ -337,15 +347,14 @@ int launch_cocktail(bool backward, const kd_cocktail& p, cudaStream_t stream) {
   auto run = [&](auto e, auto v) {
     using E = decltype(e);
     constexpr int W = decltype(v)::value;
-    if (backward) grad_t<E, W>(p, stream); else scores_t<E, W>(p, stream);
+    return backward ? grad_t<E, W>(p, stream) : scores_t<E, W>(p, stream);
   };
   using One = std::integral_constant<int, 1>;
   using Four = std::integral_constant<int, 4>;
   using Eight = std::integral_constant<int, 8>;
-  if (p.dtype == KD_F32) { if (wide) run(float(), Four()); else run(float(), One()); }
-  else if (p.dtype == KD_F16) { if (wide) run(__half(), Eight()); else run(__half(), One()); }
-  else { if (wide) run(__nv_bfloat16(), Eight()); else run(__nv_bfloat16(), One()); }
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = p.dtype == KD_F32   ? (wide ? run(float(), Four()) : run(float(), One()))
+                        : p.dtype == KD_F16 ? (wide ? run(__half(), Eight()) : run(__half(), One()))
+                                            : (wide ? run(__nv_bfloat16(), Eight()) : run(__nv_bfloat16(), One()));
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "cocktail kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -354,14 +363,11 @@ template <typename E>
 static int span_mean_t(bool backward, const void* a, int64_t a_sb, int64_t a_st, void* out, int64_t o_sb, int64_t o_st, int B,
                        int T, int C, int S, const int32_t* starts, const int32_t* ends, const int32_t* n_starts,
                        const int32_t* n_ends, cudaStream_t stream) {
-  if (!backward) {
-    span_mean_fwd_kernel<E><<<dim3(S, B), CK_THREADS, 0, stream>>>(static_cast<const E*>(a), a_sb, a_st, T, C, starts, ends,
-                                                                   n_starts, n_ends, static_cast<E*>(out), S);
-  } else {
-    span_mean_bwd_kernel<E><<<dim3((T + 7) / 8, B), CK_THREADS, 0, stream>>>(static_cast<const E*>(a), S, T, C, starts, ends,
-                                                                             n_starts, n_ends, static_cast<E*>(out), o_sb, o_st);
-  }
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e =
+      backward ? launch(span_mean_bwd_kernel<E>, dim3((T + 7) / 8, B), CK_THREADS, 0, stream, static_cast<const E*>(a), S, T, C, starts, ends, n_starts,
+                        n_ends, static_cast<E*>(out), o_sb, o_st)
+               : launch(span_mean_fwd_kernel<E>, dim3(S, B), CK_THREADS, 0, stream, static_cast<const E*>(a), a_sb, a_st, T, C, starts, ends, n_starts,
+                        n_ends, static_cast<E*>(out), S);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "span_mean kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }

@@ -24,6 +24,7 @@ struct PlanView {
   uint32_t* tilebits;
   uint8_t* order;
   uint32_t* stats;
+  uint32_t* done;   // [B] CTAs of the classifier that have finished
   uint32_t* status;
 };
 
@@ -43,8 +44,28 @@ inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
   v.tilebits = reinterpret_cast<uint32_t*>(base + L.off_tilebits);
   v.order = reinterpret_cast<uint8_t*>(base + L.off_order);
   v.stats = reinterpret_cast<uint32_t*>(base + L.off_stats);
+  v.done = v.stats + 2 * (size_t)L.B;
   v.status = reinterpret_cast<uint32_t*>(base + L.off_status);
   return v;
+}
+
+// Launches a kernel whose blocks may become resident while the kernel before it on the stream still runs (programmatic
+// stream serialisation). Every kernel of this library is launched like this and begins with pdl_wait(), which returns when
+// the kernels before it are complete and their writes visible: launch latency, barrier set-up and the TMEM allocation then
+// overlap the predecessor, which is what a chain of short kernels consists of.
+template <typename... P, typename... A>
+inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // records a printf-style message for kd_last_error() and returns `code`

@@ -23,6 +23,8 @@ __global__ void __launch_bounds__(256) hadamard_kernel(const uint16_t* x, int64_
   const int sub = threadIdx.x % TPR;
   const long long rows = (long long)B * H * T;
   const float norm = rsqrtf(static_cast<float>(HD));
+  pdl_wait();
+  pdl_launch_dependents();
   // the loop bound is the same for every thread of a warp: the shuffles below need all lanes
   for (long long base = (long long)blockIdx.x * RPB; base < rows; base += (long long)gridDim.x * RPB) {
     const long long row = base + threadIdx.x / TPR;
@@ -124,9 +126,10 @@ int launch_hadamard(const kd_tensor& x, const kd_tensor& y, int B, int H, int T,
   const unsigned blocks = static_cast<unsigned>(std::min<long long>((rows + rows_per_block - 1) / rows_per_block, 148LL * 32));
   const uint16_t* xp = static_cast<const uint16_t*>(x.ptr);
   uint16_t* yp = static_cast<uint16_t*>(y.ptr);
+  cudaError_t e;
 #define KD_LAUNCH_H(HD, BF)                                                                             \
-  hadamard_kernel<HD, BF><<<blocks, 256, 0, stream>>>(xp, x.stride_b, x.stride_h, x.stride_t, yp,       \
-                                                      y.stride_b, y.stride_h, y.stride_t, B, H, T, signs, inverse)
+  e = launch(hadamard_kernel<HD, BF>, blocks, 256, 0, stream, xp, x.stride_b, x.stride_h, x.stride_t, yp, y.stride_b,           \
+             y.stride_h, y.stride_t, B, H, T, signs, inverse)
   if (D == 16 && dtype == KD_BF16) KD_LAUNCH_H(16, true);
   else if (D == 16) KD_LAUNCH_H(16, false);
   else if (D == 32 && dtype == KD_BF16) KD_LAUNCH_H(32, true);
@@ -136,7 +139,6 @@ int launch_hadamard(const kd_tensor& x, const kd_tensor& y, int B, int H, int T,
   else if (D == 128 && dtype == KD_BF16) KD_LAUNCH_H(128, true);
   else KD_LAUNCH_H(128, false);
 #undef KD_LAUNCH_H
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "hadamard_kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }

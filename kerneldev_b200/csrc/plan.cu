@@ -1,7 +1,8 @@
-// Plan construction: token descriptors, exact 128x128 tile classification, work lists,
+// Plan construction (two kernels: token descriptors; exact 128x128 tile classification with the work lists)
 // and the dense-mask materialiser. Integer-only kernels; HBM traffic is a few hundred KB.
 #include "common.cuh"
 #include "mask_rule.cuh"
+#include "sm100_prims.cuh"
 
 namespace kd {
 
@@ -13,21 +14,23 @@ namespace kd {
 __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
   const int tile = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
   const int t = tile * KD_TILE + tid;
-  // for the reports of later kernels; this kernel's own use the argument
-  if (tile == 0 && b == 0 && tid == 0) *reinterpret_cast<uint32_t**>(pv.status + 2) = m.status_mirror;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (tile == 0 && b == 0 && tid == 0) {
+    *pv.status = 0u;   // raised by the next kernel at the earliest
+    *reinterpret_cast<uint32_t**>(pv.status + 2) = m.status_mirror;
+  }
   int n_b = m.T;
   if (m.lens != nullptr) n_b = min(m.lens[b], m.T);
   const bool alive = t < n_b;
   uint32_t d = 0;
+  bool bad_id = false;
   if (alive) {
     if (m.rules) {
       const bool ins = m.in_span ? (m.in_span[b * m.in_span_stride_b + t] != 0) : false;
       const bool pre = m.is_prefix ? (m.is_prefix[b * m.is_prefix_stride_b + t] != 0) : false;
       const int64_t sid = m.span_id ? m.span_id[b * m.span_id_stride_b + t] : 0;
-      if (sid >= (1 << 23) || sid < -(1 << 23)) {
-        atomicOr(pv.status, KD_STATUS_SPAN_RANGE);
-        if (m.status_mirror != nullptr) *const_cast<volatile uint32_t*>(m.status_mirror) = KD_STATUS_SPAN_RANGE;
-      }
+      bad_id = sid >= (1 << 23) || sid < -(1 << 23);
       d = pack_token(ins, pre, sid, true);
     } else {
       // no metadata: causal = every token is context; otherwise every token is prefix
@@ -37,13 +40,13 @@ __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
   pv.desc[(size_t)b * pv.Tpad + t] = d;
   {
     // 128-bit class masks of the tile: bit t of mask k = descriptor bit k of token t
-    // (bits 0..2 = classes as a key, bits 5..7 = classes seen as a query, bit 4 = same-span armed)
+    // (bits 0..2 = classes as a key, bits 5..7 = classes seen as a query, bit 4 = same-span armed); mask 7: span id out of range
     const uint32_t src_bit[8] = {TD_PRE, TD_CTX, TD_INS, TD_PRE << TD_SEES_SHIFT, TD_CTX << TD_SEES_SHIFT,
                                  TD_INS << TD_SEES_SHIFT, TD_SIDPOS, 0u};
     uint32_t* tb = pv.tilebits + ((size_t)b * pv.NT + tile) * 32;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const uint32_t bal = __ballot_sync(0xffffffffu, (d & src_bit[k]) != 0u);
+      const uint32_t bal = __ballot_sync(0xffffffffu, k < 7 ? (d & src_bit[k]) != 0u : bad_id);
       if ((tid & 31) == 0) tb[k * 4 + (tid >> 5)] = bal;
     }
   }
@@ -79,119 +82,155 @@ __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
     if (tile == 0) {
       pv.stats[b * 2 + 0] = 0;
       pv.stats[b * 2 + 1] = 0;
+      pv.done[b] = 0;
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------
-// 2. classify: one warp per (b, q_tile, k_tile)
+// 2. classify and lists: one CTA per (b, pair of query tiles) and per (b, key tile)
 // ---------------------------------------------------------------------------------------
 // Tiles whose 128 query tokens share one flag combination and whose 128 key tokens share one
 // are decided from the summaries; everything else is decided by evaluating the rule on all
 // 128x128 pairs. Both routes give the exact reduction of the dense mask.
-__global__ void __launch_bounds__(128) classify_kernel(PlanView pv, int B) {
-  __shared__ uint32_t s_k[4][KD_TILE];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long total = (long long)B * pv.NT * pv.NT;
-  const long long item = (long long)blockIdx.x * 4 + warp;
-  if (item >= total) return;
-  const int kt = static_cast<int>(item % pv.NT);
-  const int qt = static_cast<int>((item / pv.NT) % pv.NT);
-  const int b = static_cast<int>(item / ((long long)pv.NT * pv.NT));
+//
+// A CTA classifies the tiles of its row pair (or of its column) and writes their list at once, so every tile is
+// classified twice; in exchange the lists need no kernel of their own that walks the classes serially. The last CTA of a
+// sequence sorts its items. All of it is latency: a step on 8 x 2048 tokens spent 21 us in a memset and three kernels, of
+// which the serial lists took 8, and evaluating a tile pair by pair 5 (now a row's 128 bits are a few word operations).
+constexpr int CL_THREADS = 512, CL_WARPS = CL_THREADS / 32;
 
-  const uint32_t* sq = pv.summary + ((size_t)b * pv.NT + qt) * 4;
-  const uint32_t* sk = pv.summary + ((size_t)b * pv.NT + kt) * 4;
-  const uint32_t q_or = sq[0], q_and = sq[1], k_or = sk[0], k_and = sk[1];
-  int cls = -1;
-  if (q_or == 0u || k_or == 0u) {
-    cls = KD_TILE_EMPTY;  // all queries or all keys are beyond the sequence length
-  } else if (q_or == q_and && k_or == k_and) {
-    // flags only; the span id is handled below
-    if (k_or & sees_of_flags(q_or)) {
-      cls = KD_TILE_FULL;
-    } else if ((k_or & q_or & TD_CTX) != 0u) {
-      cls = qt > kt ? KD_TILE_FULL : (qt < kt ? KD_TILE_EMPTY : KD_TILE_PARTIAL);
-    } else if ((q_or & TD_SIDPOS) && (k_or & TD_INS)) {
-      const int32_t qmin = (int32_t)sq[2], qmax = (int32_t)sq[3];
-      const int32_t kmin = (int32_t)sk[2], kmax = (int32_t)sk[3];
-      if (qmin == qmax && kmin == kmax) cls = (qmin == kmin) ? KD_TILE_FULL : KD_TILE_EMPTY;
-      else if (qmax < kmin || kmax < qmin) cls = KD_TILE_EMPTY;  // disjoint id ranges
-    } else {
-      cls = KD_TILE_EMPTY;
-    }
+// exact class of tile (qt, kt) from all its pairs; one warp
+__device__ __forceinline__ int classify_exact(const PlanView& pv, int b, int qt, int kt, int lane) {
+  const uint32_t* dq = pv.desc + (size_t)b * pv.Tpad + (size_t)qt * KD_TILE;
+  const uint32_t* dk = pv.desc + (size_t)b * pv.Tpad + (size_t)kt * KD_TILE;
+  const uint32_t* tb = pv.tilebits + ((size_t)b * pv.NT + kt) * 32;
+  uint32_t pre[4], ctx[4], ins[4], kd[4], qd[4];
+  uint32_t any_ins = 0u;
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    pre[w] = tb[TB_PRE * 4 + w];
+    ctx[w] = tb[TB_CTX * 4 + w];
+    ins[w] = tb[TB_INS * 4 + w];
+    any_ins |= ins[w];
+    kd[w] = dk[w * 32 + lane];
+    qd[w] = dq[w * 32 + lane];
   }
-  if (cls < 0) {
-    const uint32_t* dq = pv.desc + (size_t)b * pv.Tpad + (size_t)qt * KD_TILE;
-    const uint32_t* dk = pv.desc + (size_t)b * pv.Tpad + (size_t)kt * KD_TILE;
-    for (int j = lane; j < KD_TILE; j += 32) s_k[warp][j] = dk[j];
-    __syncwarp();
-    bool any_on = false, any_off = false;
-    for (int r = 0; r < 4; ++r) {
-      const int i = qt * KD_TILE + r * 32 + lane;
-      const uint32_t qd = dq[r * 32 + lane];
-      for (int j = 0; j < KD_TILE; ++j) {
-        const bool a = rule_allowed(qd, i, s_k[warp][j], kt * KD_TILE + j);
-        any_on |= a;
-        any_off |= !a;
+  uint32_t on = 0u, off = 0u;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    uint32_t mk[4];
+    query_row_mask<4>(qd[r], qt * KD_TILE + r * 32 + lane, kt * KD_TILE, pre, ctx, ins, mk);
+    // "same span": one round per distinct span among the 32 queries; a ballot gives the keys of that span
+    const uint32_t my_key = span_key_of_query(qd[r]);
+    uint32_t todo = any_ins != 0u ? __ballot_sync(0xffffffffu, (qd[r] & TD_SIDPOS) != 0u) : 0u;
+    while (todo != 0u) {
+      const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
+      const bool mine = my_key == kq;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd[w]) != 0u);
+        if (mine) mk[w] |= hit;
       }
-      const bool w_on = __any_sync(0xffffffffu, any_on);
-      const bool w_off = __any_sync(0xffffffffu, any_off);
-      if (w_on && w_off) break;
+      todo &= ~__ballot_sync(0xffffffffu, mine);
     }
-    const bool w_on = __any_sync(0xffffffffu, any_on);
-    const bool w_off = __any_sync(0xffffffffu, any_off);
-    cls = w_on ? (w_off ? KD_TILE_PARTIAL : KD_TILE_FULL) : KD_TILE_EMPTY;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      on |= mk[w];
+      off |= ~mk[w];
+    }
   }
-  if (lane == 0) {
-    pv.cls[((size_t)b * pv.NT + qt) * pv.NT + kt] = static_cast<uint8_t>(cls);
-    if (cls == KD_TILE_FULL) atomicAdd(&pv.stats[b * 2 + 0], 1u);
-    if (cls == KD_TILE_PARTIAL) atomicAdd(&pv.stats[b * 2 + 1], 1u);
-  }
+  const bool w_on = __any_sync(0xffffffffu, on != 0u), w_off = __any_sync(0xffffffffu, off != 0u);
+  return w_on ? (w_off ? KD_TILE_PARTIAL : KD_TILE_FULL) : KD_TILE_EMPTY;
 }
 
-// ---------------------------------------------------------------------------------------
-// 3. work lists
-// ---------------------------------------------------------------------------------------
-// forward: per (b, pair p of query tiles 2p, 2p+1) the key tiles that are non-empty for either
-// backward: per (b, key tile) the query tiles that are non-empty
-// order:    per b, the pairs / query tiles / key tiles sorted by decreasing list length, so that the
-//           kernels can schedule the longest work items first
-__global__ void __launch_bounds__(128) lists_kernel(PlanView pv) {
+// class of tile (qt, kt) from the summaries of the two runs of tokens, or -1
+__device__ __forceinline__ int classify_summary(uint4 q, uint4 k, int qt, int kt) {
+  if (q.x == 0u || k.x == 0u) return KD_TILE_EMPTY;   // all queries or all keys are beyond the sequence length
+  if (q.x != q.y || k.x != k.y) return -1;
+  // flags only; the span id is handled below
+  if (k.x & sees_of_flags(q.x)) return KD_TILE_FULL;
+  if ((k.x & q.x & TD_CTX) != 0u) return qt > kt ? KD_TILE_FULL : (qt < kt ? KD_TILE_EMPTY : KD_TILE_PARTIAL);
+  if ((q.x & TD_SIDPOS) && (k.x & TD_INS)) {
+    const int32_t qmin = (int32_t)q.z, qmax = (int32_t)q.w, kmin = (int32_t)k.z, kmax = (int32_t)k.w;
+    if (qmin == qmax && kmin == kmax) return (qmin == kmin) ? KD_TILE_FULL : KD_TILE_EMPTY;
+    return (qmax < kmin || kmax < qmin) ? KD_TILE_EMPTY : -1;   // disjoint id ranges
+  }
+  return KD_TILE_EMPTY;
+}
+
+// forward list: per (b, pair p of query tiles 2p, 2p+1) the key tiles that are non-empty for either
+// backward list: per (b, key tile) the query tiles that are non-empty
+// order: per b, the pairs / query tiles / key tiles sorted by decreasing list length, so that the
+//        kernels can schedule the longest work items first
+__global__ void __launch_bounds__(CL_THREADS) classify_kernel(PlanView pv) {
+  __shared__ uint4 s_sum[128];        // summaries of all tiles of the sequence
+  __shared__ uint8_t s_cls[2][128];   // [query tile of the pair][key tile], or [0][query tile]
   __shared__ int s_cnt[3][128];
-  const int b = blockIdx.x;
-  for (int w = threadIdx.x; w < pv.NP + 2 * pv.NT; w += blockDim.x) {
-    if (w < pv.NP) {
-      const int p = w, q0 = 2 * p, q1 = 2 * p + 1;
-      uint16_t* list = pv.fwd_list + ((size_t)b * pv.NP + p) * pv.NT;
-      int n = 0;
-      for (int kt = 0; kt < pv.NT; ++kt) {
-        const uint32_t c0 = pv.cls[((size_t)b * pv.NT + q0) * pv.NT + kt];
-        const uint32_t c1 = q1 < pv.NT ? pv.cls[((size_t)b * pv.NT + q1) * pv.NT + kt] : KD_TILE_EMPTY;
-        if (c0 | c1) list[n++] = static_cast<uint16_t>(kt | (c0 << 8) | (c1 << 10));
-      }
-      pv.fwd_cnt[b * pv.NP + p] = n;
-      s_cnt[0][p] = n;
-    } else if (w < pv.NP + pv.NT) {
-      const int kt = w - pv.NP;
-      uint16_t* list = pv.bwd_list + ((size_t)b * pv.NT + kt) * pv.NT;
-      int n = 0;
-      for (int qt = 0; qt < pv.NT; ++qt) {
-        const uint32_t c = pv.cls[((size_t)b * pv.NT + qt) * pv.NT + kt];
-        if (c) list[n++] = static_cast<uint16_t>(qt | (c << 8));
-      }
-      pv.bwd_cnt[b * pv.NT + kt] = n;
-      s_cnt[2][kt] = n;
-    } else {
-      const int qt = w - pv.NP - pv.NT;
-      int n = 0;
-      for (int kt = 0; kt < pv.NT; ++kt) n += pv.cls[((size_t)b * pv.NT + qt) * pv.NT + kt] != KD_TILE_EMPTY;
-      s_cnt[1][qt] = n;
+  __shared__ int s_last;
+  const int item = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int NT = pv.NT, NP = pv.NP;
+  const bool is_pair = item < NP;
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int t = tid; t < NT; t += CL_THREADS) s_sum[t] = *reinterpret_cast<const uint4*>(pv.summary + ((size_t)b * NT + t) * 4);
+  __syncthreads();
+  const int rows = is_pair ? min(2, NT - 2 * item) : 1, total = rows * NT;
+  for (int e = warp; e < total; e += CL_WARPS) {
+    const int r = e / NT, c = e - r * NT;
+    const int qt = is_pair ? 2 * item + r : c, kt = is_pair ? c : item - NP;
+    int cls = classify_summary(s_sum[qt], s_sum[kt], qt, kt);
+    if (cls < 0) cls = classify_exact(pv, b, qt, kt, lane);
+    if (lane == 0) {
+      s_cls[r][c] = static_cast<uint8_t>(cls);
+      if (is_pair) pv.cls[((size_t)b * NT + qt) * NT + kt] = static_cast<uint8_t>(cls);
     }
   }
   __syncthreads();
-  for (int w = threadIdx.x; w < 3 * pv.NT; w += blockDim.x) {
-    const int kind = w / pv.NT, t = w % pv.NT;
-    const int n_items = kind == 0 ? pv.NP : pv.NT;
+  if (warp == 0) {
+    int n = 0, full = 0, partial = 0;
+    uint16_t* list = is_pair ? pv.fwd_list + ((size_t)b * NP + item) * NT : pv.bwd_list + ((size_t)b * NT + item - NP) * NT;
+    for (int base = 0; base < NT; base += 32) {
+      const int t = base + lane;
+      const uint32_t c0 = t < NT ? s_cls[0][t] : KD_TILE_EMPTY, c1 = t < NT && rows == 2 ? s_cls[1][t] : KD_TILE_EMPTY;
+      const uint32_t any = __ballot_sync(0xffffffffu, (c0 | c1) != 0u);
+      if ((c0 | c1) != 0u) list[n + __popc(any & ((1u << lane) - 1u))] = static_cast<uint16_t>(t | (c0 << 8) | (c1 << 10));
+      n += __popc(any);
+      full += __popc(__ballot_sync(0xffffffffu, c0 == KD_TILE_FULL)) + __popc(__ballot_sync(0xffffffffu, c1 == KD_TILE_FULL));
+      partial += __popc(__ballot_sync(0xffffffffu, c0 == KD_TILE_PARTIAL)) + __popc(__ballot_sync(0xffffffffu, c1 == KD_TILE_PARTIAL));
+    }
+    if (lane == 0) {
+      if (is_pair) {
+        pv.fwd_cnt[b * NP + item] = n;
+        atomicAdd(&pv.stats[b * 2 + 0], static_cast<uint32_t>(full));
+        atomicAdd(&pv.stats[b * 2 + 1], static_cast<uint32_t>(partial));
+      } else {
+        pv.bwd_cnt[b * NT + item - NP] = n;
+        // span ids that do not fit the descriptors, found while packing
+        const uint32_t* tb = pv.tilebits + ((size_t)b * NT + item - NP) * 32 + 28;
+        if ((tb[0] | tb[1] | tb[2] | tb[3]) != 0u) report_status(pv.status, KD_STATUS_SPAN_RANGE);
+      }
+    }
+  }
+  // the last CTA of the sequence sorts its items
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&pv.done[b], 1u) == static_cast<uint32_t>(NP + NT - 1);
+  __syncthreads();
+  if (s_last == 0) return;
+  __threadfence();
+  for (int t = tid; t < NP; t += CL_THREADS) s_cnt[0][t] = __ldcg(pv.fwd_cnt + b * NP + t);
+  for (int t = tid; t < NT; t += CL_THREADS) s_cnt[2][t] = __ldcg(pv.bwd_cnt + b * NT + t);
+  for (int qt = warp; qt < NT; qt += CL_WARPS) {
+    int n = 0;
+    for (int kt = lane; kt < NT; kt += 32) n += __ldcg(pv.cls + ((size_t)b * NT + qt) * NT + kt) != KD_TILE_EMPTY;
+    n = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) s_cnt[1][qt] = n;
+  }
+  __syncthreads();
+  for (int w = tid; w < 3 * NT; w += CL_THREADS) {
+    const int kind = w / NT, t = w % NT;
+    const int n_items = kind == 0 ? NP : NT;
     if (t >= n_items) continue;
     const int mine = s_cnt[kind][t];
     int rank = 0;
@@ -199,14 +238,16 @@ __global__ void __launch_bounds__(128) lists_kernel(PlanView pv) {
       const int other = s_cnt[kind][u];
       rank += (other > mine) || (other == mine && u < t);
     }
-    pv.order[((size_t)b * 3 + kind) * pv.NT + rank] = static_cast<uint8_t>(t);
+    pv.order[((size_t)b * 3 + kind) * NT + rank] = static_cast<uint8_t>(t);
   }
 }
 
 // ---------------------------------------------------------------------------------------
-// 4. dense mask materialiser
+// 3. dense mask materialiser
 // ---------------------------------------------------------------------------------------
 __global__ void mask_dense_kernel(PlanView pv, int T, uint8_t* out) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int b = blockIdx.z, i = blockIdx.y;
   const uint32_t* d = pv.desc + (size_t)b * pv.Tpad;
   const uint32_t qd = d[i];
@@ -221,13 +262,8 @@ int launch_classify(const kd_meta& m, void* plan, cudaStream_t stream) {
   kd_plan_layout L;
   if (kd_plan_layout_get(m.B, m.T, &L) != 0) return KD_ERR_ARG;
   PlanView pv = make_plan_view(plan, L);
-  cudaError_t e = cudaMemsetAsync(pv.status, 0, sizeof(uint32_t), stream);
-  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "cudaMemsetAsync(status): %s", cudaGetErrorString(e));
-  pack_kernel<<<dim3(L.NT, m.B), KD_TILE, 0, stream>>>(m, pv);
-  const long long tiles = (long long)m.B * L.NT * L.NT;
-  classify_kernel<<<(unsigned)((tiles + 3) / 4), 128, 0, stream>>>(pv, m.B);
-  lists_kernel<<<m.B, 128, 0, stream>>>(pv);
-  e = cudaGetLastError();
+  cudaError_t e = launch(pack_kernel, dim3(L.NT, m.B), KD_TILE, 0, stream, m, pv);
+  if (e == cudaSuccess) e = launch(classify_kernel, dim3(L.NP + L.NT, m.B), CL_THREADS, 0, stream, pv);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "plan kernels: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -238,8 +274,7 @@ int launch_mask_dense(const void* plan, int B, int T, uint8_t* out, cudaStream_t
   PlanView pv = make_plan_view(const_cast<void*>(plan), L);
   dim3 grid((T + 255) / 256, T, B);
   if (grid.x > 16) grid.x = 16;
-  mask_dense_kernel<<<grid, 256, 0, stream>>>(pv, T, out);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch(mask_dense_kernel, grid, 256, 0, stream, pv, T, out);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "mask_dense_kernel: %s", cudaGetErrorString(e));
   return 0;
 }

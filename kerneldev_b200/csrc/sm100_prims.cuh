@@ -156,6 +156,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFl
   }
   return true;
 }
+// Programmatic dependent launch. pdl_wait: returns when every kernel before this one on the stream has completed and its
+// writes are visible; before it, a kernel touches nothing but its arguments, shared memory and TMEM. pdl_launch_dependents:
+// the next kernel's blocks may be scheduled once every block of this one has called it (or exited).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------
 // TMA (plain per-CTA tile loads; completion reported on an mbarrier as bytes)
 // ---------------------------------------------------------------------------------------

@@ -8,6 +8,7 @@ import torch
 
 sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden"))
 from cocktail_inputs import cocktail_rows, embeddings  # noqa: E402
+sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from oracle import attention_oracle as ao  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +43,46 @@ def test_cocktail_scores_and_gradient(B, T, C, dtype):
     top = float(ds.abs().double().sum(1).max() * max(h.detach().abs().max(), e_ref.detach().abs().max()))
     err = (e_dev.grad.double().cpu() - e_ref.grad).abs()
     assert bool((err <= 2 * eps * e_ref.grad.abs() + (S + T + 8) * 2.0**-24 * top).all())
+
+
+# More items than SMs, so that CTAs take several one after the other. `lens` makes runs of empty items longer than the ring of
+# item headers between items with work (both tile widths; an odd number of query tiles; a last tile of 1 and of 127 tokens)
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.float16), (80, torch.bfloat16)])
+@pytest.mark.parametrize("T,n_full", [(513, 1), (895, 2), (1280, 5)])
+def test_many_items_per_cta_with_empty_ones_between(T, n_full, D, dtype, deterministic):
+    from tests.helpers import assert_close, random_meta
+    from kerneldev_b200 import flash_attention
+    B, H = 12, 24
+    ins, sid, pre = random_meta(T + D, B, T)
+    lens = np.array([T if b % (B // n_full) == 0 else (0, 3, 129)[b % 3] for b in range(B)], np.int32)
+    meta = {"in_span": torch.as_tensor(ins, device=DEV), "span_id": torch.as_tensor(sid, device=DEV),
+            "is_prefix": torch.as_tensor(pre, device=DEV), "lens": torch.as_tensor(lens, device=DEV)}
+    g = torch.Generator(device=DEV).manual_seed(T)
+    q, k, v, do = (torch.randn((B, H, T, D), generator=g, device=DEV).to(dtype) for _ in range(4))
+    for x in (q, k, v):
+        x.requires_grad_()
+    o = flash_attention(q, k, v, deterministic=deterministic, **meta)
+    grads = torch.autograd.grad(o, (q, k, v), do)
+    mask = torch.as_tensor(ao.dense_mask(T, ins, sid, pre, lens))
+    for b, h in [(0, 0), (0, H - 1), (1, 3), (2, 5), (B - 1, H - 1), (B - B // n_full, 7)]:
+        sl = lambda x: x.detach()[b:b + 1, h:h + 1].float().cpu()
+        want = ao.attention_fwd_bwd(sl(q), sl(k), sl(v), sl(do), mask[b:b + 1])
+        # the operands P and dS are rounded to 16 bits before their products: the repository's tolerance for that
+        assert_close("O", sl(o), want[0])
+        for name, got, ref in zip(("dQ", "dK", "dV"), grads, want[-3:]):
+            assert_close(name, sl(got), ref)
+
+
+# a row of exactly one chunk of 4096 tokens, one more, and several: first [CLS] in the first, a later, or no chunk
+@pytest.mark.parametrize("T", [1, 127, 4096, 4097, 12289])
+def test_metadata_chunks(T):
+    from kerneldev_b200 import metadata_from_tokens
+    rng = np.random.default_rng(T)
+    x = rng.integers(6, 300, size=(4, T))
+    marks = rng.random((4, T)) < 0.05
+    x[marks] = rng.integers(2, 6, size=int(marks.sum()))
+    x[0, T - 1] = x[1, T // 2] = x[2, 0] = 1
+    got = [t.cpu().numpy() for t in metadata_from_tokens(torch.as_tensor(x, device=DEV))]
+    for g, w in zip(got, ao.metadata_from_tokens(x)):
+        assert np.array_equal(g, w)
