@@ -184,6 +184,12 @@ int kd_workspace_bytes_fused(int32_t B, int32_t H, int32_t T, int32_t D, size_t*
 int kd_hadamard(const kd_tensor* x, const kd_tensor* y, int32_t B, int32_t H, int32_t T, int32_t D,
                 int32_t dtype, const float* signs, int32_t inverse, void* stream);
 
+/* Converts n (at most KD_CAST_MAX) tensors of one shape in one launch: float32 to float16 (widen = 0, round to nearest) or
+ * float16 to float32 (widen = 1). D a multiple of 8; pointers and byte strides multiples of 16. */
+#define KD_CAST_MAX 3
+int kd_cast(const kd_tensor* src, const kd_tensor* dst, int32_t n, int32_t B, int32_t H, int32_t T, int32_t D, int32_t widen,
+            void* stream);
+
 /* Per-token mask metadata from token ids, on the device (replaces the fallback of
  * GPTModel.forward, model.py:203-238: two cumulative sums plus a host loop with one .nonzero() /
  * .item() synchronisation per row).

@@ -26,6 +26,7 @@ EXPORTS = (
     "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_static", "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard",
     "kd_metadata_from_tokens", "kd_span_index", "kd_span_mean",
     "kd_cocktail_index", "kd_cocktail_scores", "kd_cocktail_grad",
+    "kd_cast",
 )
 
 

@@ -231,6 +231,22 @@ int kd_hadamard(const kd_tensor* x, const kd_tensor* y, int32_t B, int32_t H, in
   return launch_hadamard(*x, *y, B, H, T, D, dtype, signs, inverse, static_cast<cudaStream_t>(stream));
 }
 
+int kd_cast(const kd_tensor* src, const kd_tensor* dst, int32_t n, int32_t B, int32_t H, int32_t T, int32_t D, int32_t widen,
+            void* stream) {
+  if (!src || !dst || n < 1 || n > KD_CAST_MAX) return set_error(KD_ERR_ARG, "bad tensor count %d", n);
+  if (B < 1 || H < 1 || T < 1 || D < 8 || D % 8 != 0) return set_error(KD_ERR_ARG, "bad shape B=%d H=%d T=%d D=%d", B, H, T, D);
+  for (int i = 0; i < 2 * n; ++i) {
+    const kd_tensor& t = i < n ? src[i] : dst[i - n];
+    const int es = (i < n) == (widen != 0) ? 2 : 4;
+    if (!t.ptr) return set_error(KD_ERR_ARG, "src / dst is null");
+    if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) || ((t.stride_b * es) & 15) || ((t.stride_h * es) & 15) || ((t.stride_t * es) & 15))
+      return set_error(KD_ERR_ALIGN, "pointers and byte strides must be multiples of 16");
+  }
+  int rc = check_device();
+  if (rc) return rc;
+  return launch_cast(src, dst, n, B, H, T, D, widen != 0, static_cast<cudaStream_t>(stream));
+}
+
 int kd_metadata_from_tokens(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span,
                             int64_t tok_es, int64_t tok_cls, int64_t tok_maskq, uint8_t* in_span,
                             int64_t* span_id, uint8_t* is_prefix, void* stream) {

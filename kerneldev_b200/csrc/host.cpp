@@ -38,6 +38,7 @@ struct Library {
   decltype(&kd_cocktail_index) cocktail_index = nullptr;
   decltype(&kd_cocktail_scores) cocktail_scores = nullptr;
   decltype(&kd_cocktail_grad) cocktail_grad = nullptr;
+  decltype(&kd_cast) cast = nullptr;
   decltype(&kd_last_error) last_error = nullptr;
 };
 Library lib;
@@ -57,6 +58,7 @@ void bind(const py::dict& a) {
   take(lib.cocktail_index, a, "kd_cocktail_index");
   take(lib.cocktail_scores, a, "kd_cocktail_scores");
   take(lib.cocktail_grad, a, "kd_cocktail_grad");
+  take(lib.cast, a, "kd_cast");
   take(lib.last_error, a, "kd_last_error");
 }
 
@@ -378,6 +380,37 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   return {dq, dk, dv};
 }
 
+// float32 <-> float16 copies of up to three tensors of one shape, in the memory order of the originals, by one kernel.
+// Tensors whose strides it cannot address go through the library's conversion.
+std::array<Tensor, KD_CAST_MAX> cast(std::initializer_list<Tensor> in, at::ScalarType to) {
+  std::array<Tensor, KD_CAST_MAX> out;
+  kd_tensor src[KD_CAST_MAX], dst[KD_CAST_MAX];
+  int n = 0, slot = 0;
+  auto aligned = [](const Tensor& t) {
+    const int64_t es = t.element_size();
+    bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+    for (int i = 0; i < 3; ++i) ok = ok && (t.stride(i) * es) % 16 == 0;
+    return ok;
+  };
+  const Tensor& first = *in.begin();
+  for (const Tensor& x : in) {
+    Tensor y = at::empty_like(x, x.options().dtype(to));
+    if (x.numel() > 0 && x.scalar_type() != to && aligned(x) && aligned(y)) {
+      src[n] = desc(x);
+      dst[n++] = desc(y);
+    } else {
+      y = x.to(to);
+    }
+    out[slot++] = y;
+  }
+  if (n > 0) {
+    c10::cuda::CUDAGuard guard(first.device());
+    check(lib.cast(src, dst, n, static_cast<int32_t>(first.size(0)), static_cast<int32_t>(first.size(1)), static_cast<int32_t>(first.size(2)),
+                   static_cast<int32_t>(first.size(3)), to == at::kFloat ? 1 : 0, at::cuda::getCurrentCUDAStream()));
+  }
+  return out;
+}
+
 Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
   const Tensor x = usable(x_);
   Tensor y = at::empty(x.sizes(), x.options());
@@ -419,7 +452,7 @@ struct AttentionBackward : torch::autograd::Node {
       tlse = lse.unpack();
     }
     at::NoGradGuard no_grad;
-    const Tensor d_o = widen ? grads[0].to(at::kHalf) : grads[0];
+    const Tensor d_o = widen ? cast({grads[0]}, at::kHalf)[0] : grads[0];
     auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
                                  opt.heads_per_cta);
     if (signs.has_value()) {
@@ -428,9 +461,10 @@ struct AttentionBackward : torch::autograd::Node {
       dk = hadamard(dk, signs, true);
     }
     if (widen) {
-      dq = dq.to(at::kFloat);
-      dk = dk.to(at::kFloat);
-      dv = dv.to(at::kFloat);
+      auto wide = cast({dq, dk, dv}, at::kFloat);
+      dq = wide[0];
+      dk = wide[1];
+      dv = wide[2];
     }
     out[0] = dq;
     out[1] = dk;
@@ -471,15 +505,22 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
   Tensor o, lse, q2, k2, v2, o16;
   {
     at::AutoDispatchBelowADInplaceOrView below;
-    q2 = f32 ? q.to(at::kHalf) : q;
-    k2 = f32 ? k.to(at::kHalf) : k;
-    v2 = f32 ? v.to(at::kHalf) : v;
+    if (f32) {
+      auto half = cast({q, k, v}, at::kHalf);
+      q2 = half[0];
+      k2 = half[1];
+      v2 = half[2];
+    } else {
+      q2 = q;
+      k2 = k;
+      v2 = v;
+    }
     if (signs.has_value()) {
       q2 = hadamard(q2, signs, false);
       k2 = hadamard(k2, signs, false);
     }
     std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, heads_per_cta);
-    o = f32 ? o16.to(at::kFloat) : o16;
+    o = f32 ? cast({o16}, at::kFloat)[0] : o16;
   }
   if (track) {
     auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
