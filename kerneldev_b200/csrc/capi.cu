@@ -37,6 +37,16 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// The encoder wants a current context, which a host thread that has not used the runtime yet (a new autograd worker whose
+// allocations all came from a cache) does not have: it is bound then, and the call repeated.
+template <typename F>
+static CUresult with_context(F encode) {
+  CUresult r = encode();
+  int dev = 0;
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  return r;
+}
+
 int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype,
                       int box_rows, const char* name) {
   EncodeTiledFn enc = encode_fn();
@@ -56,9 +66,9 @@ int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T,
     if (strides[i] & 15) strides[i] = (strides[i] + 15) & ~cuuint64_t(15);
   cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
   cuuint32_t es[4] = {1, 1, 1, 1};
-  CUresult r = enc(out, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+  const CUresult r = with_context([&] { return enc(out, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                    t.ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return set_error(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
   return 0;
 }
@@ -71,8 +81,8 @@ int encode_tensor_map_f32_rows(CUtensorMap* out, float* base, int slices, int T,
   cuuint64_t strides[2] = {(cuuint64_t)D * 4, (cuuint64_t)D * 4 * (cuuint64_t)T};
   cuuint32_t box[3] = {32, (cuuint32_t)box_rows, 1};
   cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUresult r = with_context([&] { return enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return set_error(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
   return 0;
 }

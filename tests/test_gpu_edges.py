@@ -86,3 +86,25 @@ def test_metadata_chunks(T):
     got = [t.cpu().numpy() for t in metadata_from_tokens(torch.as_tensor(x, device=DEV))]
     for g, w in zip(got, ao.metadata_from_tokens(x)):
         assert np.array_equal(g, w)
+
+
+def test_host_thread_without_a_cuda_context():
+    """A forward and backward whose every allocation comes from the cache, in a host thread that has not used CUDA before."""
+    import threading
+    from kerneldev_b200 import flash_attention
+    q, k, v, do = (torch.randn(1, 2, 200, 64, device=DEV, dtype=torch.bfloat16) for _ in range(4))
+    out = []
+
+    def run():
+        a, b, c = (x.detach().requires_grad_() for x in (q, k, v))
+        o = flash_attention(a, b, c)
+        out.append((o.detach(), *torch.autograd.grad(o, (a, b, c), do)))
+
+    run()
+    first = out.pop()
+    worker = threading.Thread(target=run)
+    worker.start()
+    worker.join()
+    assert len(out) == 1
+    for x, y in zip(first, out[0]):
+        assert torch.allclose(x.float(), y.float(), atol=1e-2, rtol=1e-2)
