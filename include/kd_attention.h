@@ -126,6 +126,8 @@ typedef struct kd_attn_params {
                          one after the other (they share the plan's work list); a tuning and test knob of the
                          deterministic backward. The forward and the fused backward take their work items
                          dynamically and ignore it. */
+  int32_t plan_ready;    /* 1: an earlier launch on the same stream has used this plan, which lets kd_attn_fwd look up its
+                         work before the kernel ahead of it on the stream has finished. 0 is always correct. */
 } kd_attn_params;
 
 /* Size and layout of a plan for B sequences of T tokens. */

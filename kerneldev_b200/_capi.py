@@ -60,7 +60,7 @@ class KdAttnParams(Structure):
         ("q", KdTensor), ("k", KdTensor), ("v", KdTensor), ("o", KdTensor), ("d_o", KdTensor),
         ("dq", KdTensor), ("dk", KdTensor), ("dv", KdTensor),
         ("lse", c_void_p), ("delta", c_void_p), ("plan", c_void_p), ("bwd_phases", c_int32), ("bwd_mode", c_int32),
-        ("dq_acc", c_void_p), ("heads_per_cta", c_int32),
+        ("dq_acc", c_void_p), ("heads_per_cta", c_int32), ("plan_ready", c_int32),
     ]
 
 

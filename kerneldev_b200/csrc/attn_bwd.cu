@@ -947,7 +947,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   }
   if (fused && e == cudaSuccess) {
     // bwd_phases 1: the delta kernel alone (it also zeroes dq_acc); 2: the fused kernel and the conversion
-    if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, stream);
+    if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, (phases & 1) != 0, stream);
   } else if ((phases & 2) && e == cudaSuccess) {
     e = launch(kk, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }

@@ -36,6 +36,6 @@ struct BwdArgs {
 // Fused backward (attn_bwd_fused.cu): one key-tile-major kernel that forms S and dP once per tile, accumulates dK and
 // dV in TMEM and adds its dQ partials to a.dq_acc, then a conversion kernel.
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                     const BwdArgs& a, int dtype, cudaStream_t stream);
+                     const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream);
 
 }  // namespace kd

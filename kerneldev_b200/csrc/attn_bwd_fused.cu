@@ -67,6 +67,7 @@ namespace kd {
 struct FusedArgs {
   BwdArgs b;
   int chunk;   // (batch, head) pairs per chunk of items
+  int after_delta;   // the delta kernel of the same call is the kernel before this one on the stream
 };
 
 template <int HD_>
@@ -159,19 +160,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (tid == 0) report_status(a.status, KD_DEV_TIMEOUT | W_U_ALIGN);
     return;
   }
-  if (tid == 0) {
-    abortf->v = 0;
-    for (int i = 0; i < C::NBAR; ++i) {
-      uint32_t count = 1;
-      if (i >= C::B_QFULL && i < C::B_QEMPTY) count = 33;        // the TMA load and the producer lanes' own copies
-      if (i >= C::B_DOEMPTY && i < C::B_SFULL) count = 2;        // dP^T and dV have read the tile
-      if (i == C::B_DSFULL || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
-      if (i == C::B_DQEMPTY) count = 4;                          // one per dQ warp
-      if (i == C::B_ACCFULL) count = 2;                          // the head's last dV and dK
-      if (i == C::B_ACCFREE || i == C::B_ACCFREE + 1) count = 4; // dV, dK have been read out of TMEM
-      if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = C::ITEM_READERS;
-      mbar_init(bar(i), count);
-    }
+  if (tid == 0) abortf->v = 0;
+  if (tid < C::NBAR) {   // a thread each: one after the other they took 900 cycles of a CTA's start
+    const int i = tid;
+    uint32_t count = 1;
+    if (i >= C::B_QFULL && i < C::B_QEMPTY) count = 33;        // the TMA load and the producer lanes' own copies
+    if (i >= C::B_DOEMPTY && i < C::B_SFULL) count = 2;        // dP^T and dV have read the tile
+    if (i == C::B_DSFULL || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
+    if (i == C::B_DQEMPTY) count = 4;                          // one per dQ warp
+    if (i == C::B_ACCFULL) count = 2;                          // the head's last dV and dK
+    if (i == C::B_ACCFREE || i == C::B_ACCFREE + 1) count = 4; // dV, dK have been read out of TMEM
+    if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = C::ITEM_READERS;
+    mbar_init(bar(i), count);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -181,8 +181,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  pdl_wait();
-  pdl_launch_dependents();
+  // With the delta kernel directly before this one, everything but delta and the zeroed dQ scratch was complete before that
+  // kernel let this one start: the plan, Q, K, V, dO and LSE may be read, and dK and dV written, before the wait.
+  if (!fa.after_delta) pdl_wait();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
     return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
@@ -241,7 +242,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         return it;
       };
       int asked = 0;   // cancellations asked for
-      auto ask = [&]() {   // for the item after the one in hand
+      // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), which hides the
+      // answer and the look-up of its list, and no earlier: an item held in reserve by a CTA with a long list is one that an idle CTA cannot take.
+      auto ask = [&]() {
         if (lane == 0) {
           fence_proxy_async_smem();   // the previous response has been read
           mbar_arrive_expect_tx(bar(C::B_CLC), 16);
@@ -250,7 +253,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ++asked;
         pending = true;
       };
-      // dK = dV = 0 for an item without entries: no other warp hears of it
+      // dK = dV = 0 for an item without entries
       auto write_zeros = [&](const int4& z) {
         const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0), cpr = a.d_real / 8;   // 16-byte chunks of a row
         uint16_t* dk = reinterpret_cast<uint16_t*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
@@ -261,31 +264,26 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           *reinterpret_cast<uint4*>(dv + (size_t)(row0 + r) * a.dv_st + c) = make_uint4(0u, 0u, 0u, 0u);
         }
       };
-      // the next item that has entries (nx.w < 0: there is none); its successor has been asked for
+      // the answer (nx.w < 0: there is no further item)
       auto take_next = [&](int4& nx) -> bool {
-        while (true) {
-          if (!wait(C::B_CLC, (asked - 1) & 1, W_U_CLC)) return false;
-          pending = false;
-          const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
-          if (idx < 0) {
-            nx.w = -1;
-            return true;
-          }
+        if (!wait(C::B_CLC, (asked - 1) & 1, W_U_CLC)) return false;
+        pending = false;
+        const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
+        __syncwarp();   // every lane has read the response that the next request overwrites
+        nx.w = -1;
+        if (idx >= 0) {
           nx = decode(idx);
-          ask();
-          if (nx.w > 0) return true;
-          write_zeros(nx);
+          if (nx.w <= 2) ask();
         }
+        return true;
       };
       int4 it = decode(blockIdx.x);
-      ask();
-      if (it.w == 0) {
-        write_zeros(it);
-        ok = take_next(it);
-      }
+      if (it.w <= 2) ask();
       int qs = 0, os = 0;
       uint32_t q_parity = 1u, do_parity = 1u;   // of the stages' "empty" phases
       while (ok) {
+        const int b = it.x, h = it.y, kt = it.z & 0xFFFF, n = it.w;
+        if (n != 0) {   // (no other warp hears of an item without entries)
         const int slot = k % C::NITEM;
         if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_U_ITEMEMPTY))) break;
         if (lane == 0) {
@@ -293,23 +291,33 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           mbar_arrive(bar(C::B_ITEMFULL + slot));
         }
         __syncwarp();
-        if (it.w < 0) break;
-        const int b = it.x, h = it.y, kt = it.z & 0xFFFF, n = it.w;
+        if (n < 0) break;
         // K into the buffer of the item before the last (HD = 64; at HD = 128 the issuing warps request K as well as V)
         if (HD == 64 || k == 0) {
           if (!(ok = wait(C::B_KEMPTY + k % C::NK, ((k / C::NK) & 1) ^ 1, W_U_KEMPTY))) break;
           if (lane == 0) load_tile(&tmK, sK + (k % C::NK) * TILE, C::B_KFULL + k % C::NK, kt, h, b);
           ++k_loads;
         }
-        if (k == 0 && lane == 0) load_tile(&tmV, sV, C::B_VFULL, kt, h, b);
+        if (k == 0) {
+          if (lane == 0) load_tile(&tmV, sV, C::B_VFULL, kt, h, b);
+          pdl_wait();   // delta is read from here on
+          pdl_launch_dependents();
+        }
         ++k;
+        }
         const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
         const size_t row = ((size_t)b * a.H + h) * a.T;
         const bool aligned = (row & 3) == 0;
         uint32_t ent = static_cast<uint32_t>(it.z) >> 16;
         int4 nx = it;
 #pragma unroll 1
-        for (int e = 0; e < n; ++e) {
+        for (int e = 0; e < max(n, 1); ++e) {
+          if (n > 2 && e == n - 3) ask();
+          if (e >= n - 1 && !(ok = take_next(nx))) break;   // its list is looked up while this item's last tile waits for a slot
+          if (n == 0) {
+            write_zeros(it);
+            break;
+          }
           const uint32_t this_ent = ent;
           if (e + 1 < n) ent = list[e + 1];
           const int qt = this_ent & 0xFF;
@@ -343,7 +351,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, qt, h, b);
           ++do_tiles;
           if (++os == C::OS) { os = 0; do_parity ^= 1u; }
-          if (e == 0 && !(ok = take_next(nx))) break;
         }
         it = nx;
       }
@@ -853,6 +860,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   } else {
     reg_dealloc<C::REGS_DQ>();
     // ------------------------------ dQ warps: TMEM -> shared memory -> bulk reduction into the fp32 scratch ------------------------------
+    pdl_wait();   // the scratch has been zeroed
     const int wq = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t stg = s0 + C::SMEM_STG + wq * 8192, st_row = static_cast<uint32_t>(lane) * 128u, st_sw = static_cast<uint32_t>(lane & 7);
@@ -1005,7 +1013,7 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
 
 template <int HD, bool kBf16>
 static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                          const BwdArgs& a, int dtype, cudaStream_t stream) {
+                          const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   using C = FusedCfg<HD>;
   CUtensorMap tmAcc, tmDK, tmDV;
   int rc = encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
@@ -1017,6 +1025,7 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
   FusedArgs fa;
   fa.b = a;
+  fa.after_delta = after_delta;
   // (batch, head) pairs whose Q, K, V, dO and dQ scratch take about 64 MB of the 126 MB L2 together, and enough of them that
   // a chunk holds two items per SM
   const double pair_bytes = (double)a.T * (4.0 * a.d_real * 2 + HD * 4.0);
@@ -1046,10 +1055,10 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
 }
 
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                     const BwdArgs& a, int dtype, cudaStream_t stream) {
+                     const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   if (a.d_real <= 64)
-    return dtype == KD_BF16 ? launch_fused_t<64, true>(tmQ, tmK, tmV, tmDO, a, dtype, stream) : launch_fused_t<64, false>(tmQ, tmK, tmV, tmDO, a, dtype, stream);
-  return dtype == KD_BF16 ? launch_fused_t<128, true>(tmQ, tmK, tmV, tmDO, a, dtype, stream) : launch_fused_t<128, false>(tmQ, tmK, tmV, tmDO, a, dtype, stream);
+    return dtype == KD_BF16 ? launch_fused_t<64, true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream) : launch_fused_t<64, false>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
+  return dtype == KD_BF16 ? launch_fused_t<128, true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream) : launch_fused_t<128, false>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
 }
 
 }  // namespace kd

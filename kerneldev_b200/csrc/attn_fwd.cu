@@ -41,6 +41,7 @@ struct FwdArgs {
   const uint16_t* fwd_list;
   const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length
   uint32_t* status;
+  int plan_ready;
   void* o;
   int64_t o_sb, o_sh, o_st;
   float* lse;
@@ -130,16 +131,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (tid == 0) report_status(a.status, KD_DEV_TIMEOUT | W_F_ALIGN);
     return;
   }
-  if (tid == 0) {
-    abortf->v = 0;
-    for (int i = 0; i < C::NBAR; ++i) {
-      uint32_t count = 1;
-      // One "scores ready" barrier per (buffer, query tile): each softmax warpgroup then sees every phase of the barriers it
-      // waits on, which is what makes a parity wait sound. P and O barriers: one arrival per softmax warp.
-      if ((i >= C::B_PFULL && i < C::B_PVDONE) || (i >= C::B_OFREE && i < C::B_ITEMFULL)) count = 4;
-      if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = 9;   // the issuer and eight softmax warps
-      mbar_init(bar(i), count);
-    }
+  if (tid == 0) abortf->v = 0;
+  if (tid < C::NBAR) {   // a thread each: one after the other they took 900 cycles of a CTA's start
+    const int i = tid;
+    uint32_t count = 1;
+    // One "scores ready" barrier per (buffer, query tile): each softmax warpgroup then sees every phase of the barriers it
+    // waits on, which is what makes a parity wait sound. P and O barriers: one arrival per softmax warp.
+    if ((i >= C::B_PFULL && i < C::B_PVDONE) || (i >= C::B_OFREE && i < C::B_ITEMFULL)) count = 4;
+    if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = 9;   // the issuer and eight softmax warps
+    mbar_init(bar(i), count);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -149,8 +149,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  pdl_wait();
-  pdl_launch_dependents();
+  // A plan that an earlier launch on this stream has used was complete when the kernel before this one let it start (a kernel
+  // lets its successor start only when its own predecessors are complete): its lists and descriptors may be read before the
+  // wait, which hides three dependent look-ups under the predecessor (in a stack of layers, 2 us of each kernel's 9 at T = 173).
+  // They are read past L1, which the start of a kernel that overlaps another need not have cleaned.
+  if (!a.plan_ready) pdl_wait();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
     return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
@@ -189,15 +192,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         int4 it;
         it.x = io.b;
         it.y = io.h;
-        it.z = a.order[((size_t)io.b * 3 + 0) * a.NT + io.rank];
-        it.w = a.fwd_cnt[io.b * a.NP + it.z];
+        it.z = __ldcg(a.order + ((size_t)io.b * 3 + 0) * a.NT + io.rank);
         const uint16_t* list = a.fwd_list + ((size_t)io.b * a.NP + it.z) * a.NT;
+        it.w = __ldcg(a.fwd_cnt + io.b * a.NP + it.z);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < it.w ? list[r * 32 + lane] : 0u;
+        for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
+#pragma unroll
+        for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < it.w ? lst[r] : 0u;
         return it;
       };
-      // The next item is asked for two tiles before the end of this one, which the rings hide, and no earlier: an item held
-      // in reserve by a CTA with a long list is one that an idle CTA cannot take (claimed two ahead: 575 us for 519).
+      // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), which hides the
+      // answer and the look-up of its list, and no earlier: an item held in reserve by a CTA with a long list is one that an idle CTA cannot take (claimed two
+      // items ahead: 575 us for 519 with hierarchical masks at 16 x 16 x 4096 x 64).
       auto ask = [&]() {
         if (lane == 0) {
           fence_proxy_async_smem();   // the previous response has been read
@@ -212,10 +218,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         pending = false;
         const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
         __syncwarp();   // every lane has read the response that the next request overwrites
-        if (idx < 0) {
-          nx.w = -1;
-        } else {
+        nx.w = -1;
+        if (idx >= 0) {
           nx = decode(idx);
+          if (nx.w <= 2) ask();
         }
         return true;
       };
@@ -225,6 +231,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int kb = 0; kb < C::KBLK; ++kb) tma_load_4d(dst + kb * 16384, tm, bar(full), kb * 64, tile * KD_TILE, h, b);
       };
       int4 it = decode(blockIdx.x);
+      if (it.w <= 2) ask();
       while (ok) {
         const int slot = k % C::NITEM;
         if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_F_ITEMEMPTY))) break;
@@ -240,6 +247,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_ITEMFULL + slot));
         if (n < 0) break;
+        if (k == 0) {   // Q, K and V are read from here on
+          pdl_wait();
+          pdl_launch_dependents();
+        }
         ++k;
         const int ntile_q = (2 * pair + 1 < a.NT) ? 2 : 1;
         auto load_q = [&](int t) -> bool {
@@ -251,9 +262,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         };
         if (!(ok = load_q(0))) break;
         int4 nx = it;
-        if (n == 0) ask();
 #pragma unroll 1
-        for (int e = 0; e < n; ++e) {
+        for (int e = 0; e < max(n, 1); ++e) {
+          if (n > 2 && e == n - 3) ask();
+          if (e >= n - 1 && !(ok = take_next(nx))) break;   // its list is looked up while this item's last tiles wait for slots
+          if (n == 0) {
+            if (ntile_q == 2) ok = load_q(1);
+            break;
+          }
           const int kt = sList[slot * 128 + e] & 0xFF;
 #ifdef KD_TEST_DROP_LOAD
           // Test build only: this one K tile is never requested (no copy, no expected bytes), so the S issuer's
@@ -268,7 +284,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             load_tile(&tmK, sK + s * TILE, C::B_KFULL + s, kt, h, b);
             ++kv_cnt;
           }
-          if (e == max(0, n - 2)) ask();
           if (e == 0 && ntile_q == 2 && !(ok = load_q(1))) break;
           {
             const int s = v_cnt % C::VST;
@@ -277,7 +292,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             ++v_cnt;
           }
         }
-        if (!ok || (n == 0 && ntile_q == 2 && !(ok = load_q(1))) || !(ok = take_next(nx))) break;
         it = nx;
       }
       if (abortf->v != 0 && lane == 0) {
@@ -428,7 +442,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int qtile = 2 * it.z + i;
     const int qi = qtile * KD_TILE + row;  // token index of this thread's query
     const bool tile_valid = qtile < a.NT;
-    const uint32_t qd = tile_valid ? a.desc[(size_t)b * a.Tpad + qi] : 0u;
+    const uint32_t qd = tile_valid ? __ldcg(a.desc + (size_t)b * a.Tpad + qi) : 0u;
     uint32_t lst[4];   // the list, 32 entries per register
 #pragma unroll
     for (int r = 0; r < 4; ++r) lst[r] = sList[(k % C::NITEM) * 128 + r * 32 + lane];
@@ -461,18 +475,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const uint32_t* src = a.desc + (size_t)b * a.Tpad + (size_t)kt * KD_TILE;
         const uint4* tbp = reinterpret_cast<const uint4*>(a.tilebits + ((size_t)b * a.NT + kt) * 32);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) kd_pre[w] = src[w * 32 + lane];
+        for (int w = 0; w < NW; ++w) kd_pre[w] = __ldcg(src + w * 32 + lane);
         static_assert(NW == 4, "a class mask of a tile is four words: one 16-byte load each");
         constexpr int cls3[3] = {TB_PRE, TB_CTX, TB_INS};
 #pragma unroll
         for (int k3 = 0; k3 < 3; ++k3) {
-          const uint4 m4 = tbp[cls3[k3]];
+          const uint4 m4 = __ldcg(tbp + cls3[k3]);
           tb_pre[k3][0] = m4.x; tb_pre[k3][1] = m4.y; tb_pre[k3][2] = m4.z; tb_pre[k3][3] = m4.w;
         }
       }
     };
     find_next();
     if (n_own > 0) prefetch_kd(ent_next);
+    if (k == 0) pdl_wait();   // O and LSE are written from here on
     float m = -INFINITY, l = 0.f;
     int nact = 0;
 #pragma unroll 1
@@ -654,6 +669,7 @@ static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   while ((long long)a.chunk * L.NP < 296 && a.chunk < p.B * p.H) ++a.chunk;
   const int n_chunks = (p.B * p.H) / a.chunk;   // equal chunks, none smaller: a small last one would leave SMs idle
   a.chunk = (p.B * p.H + n_chunks - 1) / n_chunks;
+  a.plan_ready = p.plan_ready;
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
   a.order = pv.order; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;

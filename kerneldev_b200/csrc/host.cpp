@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
+#include <atomic>
 #include <list>
 #include <mutex>
 #include <unordered_map>
@@ -106,6 +107,18 @@ struct Plan {
   std::vector<Tensor> keep;   // the caller's metadata and its converted copies, alive as long as the plan is cached
   at::cuda::CUDAStream built_on;
   at::cuda::CUDAEvent built;
+  std::atomic<cudaStream_t> used_on{reinterpret_cast<cudaStream_t>(-1)};   // the stream of the plan's last eager launch
+
+  // kd_attn_params.plan_ready for a launch on `stream`. A captured launch says nothing about the stream it was captured from.
+  bool ready_on(cudaStream_t stream) const {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    return used_on.load() == stream && cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+  }
+  void launched_on(cudaStream_t stream) {
+    if (used_on.load() == stream) return;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) used_on.store(stream);
+  }
 
   Plan(int64_t B_, int64_t T_, at::Device dev, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix,
        const OptTensor& lens, bool causal, bool rules)
@@ -341,7 +354,10 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Ten
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
-  check(lib.attn_fwd(&p, at::cuda::getCurrentCUDAStream()));
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  p.plan_ready = plan->ready_on(stream) ? 1 : 0;
+  check(lib.attn_fwd(&p, stream));
+  plan->launched_on(stream);
   plan->after_launch();
   return {o, lse};
 }
