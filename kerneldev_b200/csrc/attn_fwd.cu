@@ -5,11 +5,16 @@
 // that have not been launched yet (clusterlaunchcontrol) and works on them without draining its pipeline. Items are
 // numbered in chunks of heads that fit L2 together, inside a chunk by decreasing list length. (With one CTA per item or
 // group of heads, a fifth of the time went into CTA starts and a last wave that was nearly empty.)
-// Roles (warp-specialised, 384 threads):
+// Roles (warp-specialised, 640 threads):
 //   warp 0      takes items, stages their lists, loads Q tiles and the K and V rings by TMA
 //   warp 1      issues S = Q_i K^T (smem x smem -> TMEM) and O_i += P V (TMEM x smem -> TMEM)
-//   warps 4-7   softmax of query tile 0: TMEM -> registers, rule on PARTIAL tiles, online
-//   warps 8-11  softmax of query tile 1  softmax in base 2, P back to TMEM as 16-bit operand
+//   warps 4-11  softmax of query tile 0: TMEM -> registers, rule on PARTIAL tiles, online softmax in base 2, P back to TMEM as
+//   warps 12-19 softmax of query tile 1  16-bit operand. Two warps share 32 rows, 64 columns each, and exchange row maxima.
+//
+// What bounds it. An exponential per score: 1,024 cycles of the special-function units per 128 x 128 tile, twice what the
+// tensor cores need at D = 64. With one warp per 32 rows (eight softmax warps) the units were busy 65 % of the time, because
+// while a warp loads, masks and reduces its 128 columns only one other warp of its scheduler can compute exponentials. Two
+// warps to a row spend half as long outside the exponentials, at the price of one exchange of row maxima per unit.
 //
 // A "unit" is one (key tile, query tile) product that is not EMPTY. Units are numbered in list
 // order over all items; unit u computes its scores into TMEM buffer u % NBUF (128 fp32 columns), and P (64
@@ -58,26 +63,28 @@ struct FwdCfg {
   static constexpr int KST = NBUF;                       // K ring stages
   static constexpr int VST = (HD == 64) ? 3 : 2;         // V ring stages
   static constexpr int NQ = (HD == 64) ? 4 : 3;          // ring of Q tiles (two per item): the next item's Q loads while this one computes
-  static constexpr int NPART = 2;                        // parts of P that are handed over one by one
-  static constexpr int NITEM = 4;                        // ring of item headers and lists
+  static constexpr int NPART = 2;                        // P is handed over in two parts: the first, then the second 32 columns of each half
+  static constexpr int NITEM = (HD == 64) ? 4 : 2;       // ring of item headers and lists
+  static constexpr int NXB = (HD == 64) ? 2 : 1;         // buffers of the row maxima that two warps exchange (see there)
   static constexpr int SMEM_Q = 0;
   static constexpr int SMEM_K = SMEM_Q + NQ * TILE_BYTES;
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
   static constexpr int SMEM_LIST = SMEM_V + VST * TILE_BYTES;      // NITEM x <= 128 list entries
   static constexpr int SMEM_ITEM = SMEM_LIST + NITEM * 128 * 2;    // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16}
-  static constexpr int SMEM_CLC = SMEM_ITEM + NITEM * 16;
+  static constexpr int SMEM_XCH = SMEM_ITEM + NITEM * 16;          // NXB x [query tile][half][row] fp32
+  static constexpr int SMEM_CLC = SMEM_XCH + NXB * 4 * KD_TILE * 4;
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
   // barriers (8 bytes each)
   static constexpr int B_QFULL = 0, B_QEMPTY = B_QFULL + NQ, B_KFULL = B_QEMPTY + NQ, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST,
                        B_VEMPTY = B_VFULL + VST, B_SFULL = B_VEMPTY + VST, B_PFULL = B_SFULL + 2 * NBUF,
-                       B_PVDONE = B_PFULL + NPART * NBUF, B_OFREE = B_PVDONE + 2, B_ITEMFULL = B_OFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
+                       B_PVDONE = B_PFULL + NPART * NBUF, B_OFREE = B_PVDONE + 4, B_ITEMFULL = B_OFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
                        B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;
   static constexpr int SMEM_ALLOC = SMEM_BAR + NBAR * 8 + 16;
-  static constexpr int CW = KD_TILE;                     // score columns per softmax thread: a whole row
-  static constexpr int THREADS = 384;                    // four light warps + one softmax warpgroup per query tile
-  // registers: 168 per thread at launch; light warps release down to 88, softmax warps take 208
-  static constexpr int REGS_LIGHT = 88, REGS_COMPUTE = 208;
-  static_assert(4 * 32 * REGS_LIGHT + 8 * 32 * REGS_COMPUTE <= THREADS * 168, "register pool");
+  static constexpr int CW = KD_TILE / 2;                 // score columns per softmax thread: half a row
+  static constexpr int THREADS = 640;                    // four light warps + eight softmax warps per query tile
+  // registers: 96 per thread at launch; light warps release down to 56, softmax warps take 104
+  static constexpr int REGS_LIGHT = 56, REGS_COMPUTE = 104;
+  static_assert(4 * 32 * REGS_LIGHT + 16 * 32 * REGS_COMPUTE <= THREADS * 96, "register pool");
   // TMEM columns: NBUF score buffers of 128, then O0 and O1 (HD each)
   static constexpr uint32_t TM_O0 = NBUF * 128, TM_O1 = NBUF * 128 + HD;
   static_assert(TM_O1 + HD <= 512, "TMEM budget");
@@ -91,7 +98,8 @@ enum : uint32_t {
   W_F_ITEMFULL = 0x10C, W_F_ITEMEMPTY = 0x10D, W_F_CLC = 0x10E, W_F_ALIGN = 0x10F,
 };
 
-// list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10
+// list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10; in shared memory also
+// | score buffer of the entry's first unit << 12
 __device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
 
 // Items of the launch in order: chunks of `chunk` (batch, head) pairs; inside a chunk rank by rank (longest lists first), and
@@ -137,8 +145,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint32_t count = 1;
     // One "scores ready" barrier per (buffer, query tile): each softmax warpgroup then sees every phase of the barriers it
     // waits on, which is what makes a parity wait sound. P and O barriers: one arrival per softmax warp.
-    if ((i >= C::B_PFULL && i < C::B_PVDONE) || (i >= C::B_OFREE && i < C::B_ITEMFULL)) count = 4;
-    if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = 9;   // the issuer and eight softmax warps
+    if ((i >= C::B_PFULL && i < C::B_PVDONE) || (i >= C::B_OFREE && i < C::B_ITEMFULL)) count = 8;
+    if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = 17;   // the issuer and sixteen softmax warps
     mbar_init(bar(i), count);
     fence_barrier_init();
   }
@@ -186,6 +194,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       int q_cnt = 0, kv_cnt = 0, v_cnt = 0, k = 0, asked = 0;   // Q, K, V tiles requested, items published, cancellations asked for
       int k_dropped = -1;   // index of a K tile that was never requested (test builds only)
       bool ok = true, pending = false;
+      const uint32_t below = (1u << lane) - 1u;
+      uint32_t unit0 = 0u;  // score buffer of the next item's first unit
       uint32_t lst[4];      // the next item's list, 32 entries per register
       auto decode = [&](int idx) -> int4 {
         const ItemOrder io(idx, a.chunk, a.NP, a.B, a.H);
@@ -239,10 +249,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         int units[2] = {0, 0};
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          sList[slot * 128 + r * 32 + lane] = static_cast<uint16_t>(lst[r]);
-          units[0] += __popc(__ballot_sync(0xffffffffu, entry_class(lst[r], 0) != 0u));
-          units[1] += __popc(__ballot_sync(0xffffffffu, entry_class(lst[r], 1) != 0u));
+          const uint32_t has0 = __ballot_sync(0xffffffffu, entry_class(lst[r], 0) != 0u), has1 = __ballot_sync(0xffffffffu, entry_class(lst[r], 1) != 0u);
+          const uint32_t first = (unit0 + units[0] + units[1] + __popc(has0 & below) + __popc(has1 & below)) % C::NBUF;
+          sList[slot * 128 + r * 32 + lane] = static_cast<uint16_t>(lst[r] | (first << 12));
+          units[0] += __popc(has0);
+          units[1] += __popc(has1);
         }
+        unit0 = (unit0 + units[0] + units[1]) % C::NBUF;
         if (lane == 0) items[slot] = make_int4(b, h, pair, n < 0 ? -1 : (n | (units[0] << 8) | (units[1] << 16)));
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(C::B_ITEMFULL + slot));
@@ -310,71 +323,91 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t idesc_s = make_idesc_f16(kBf16, 0, 0, KD_TILE, KD_TILE), idesc_o = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);
       const uint32_t hi = desc_hi_sw128(), lo_q = desc_lo_kmajor(sQ), lo_k = desc_lo_kmajor(sK), lo_v = desc_lo_mnmajor(sV);
       constexpr uint32_t T16 = TILE >> 4;
-      // place in the stream of units: item k with n entries, `e` entries of it begun, tile `i` next of entry `ent`
-      int k = 0, n = 0, e = 0, i = 2, kstage = -1, q_cnt = 0, ntile_q = 0;
-      uint32_t ent = 0, kparity = 1u, left = 0, q_there = 0;   // units left of tile 0 | of tile 1 << 8; bit i: Q tile i has landed
-      bool open = false;   // item k is being worked on
-      int n_flight = 0;    // units whose scores have been issued and whose P V has not
+      // A wait costs this warp 150-200 cycles even when the phase is complete, for it shares its scheduler with softmax warps; with
+      // five of them one after the other and a walk over the list by entry and tile a unit took 1,550 cycles, more than the
+      // exponentials. So the tests of an iteration are issued together, and the next list entry is fetched one entry ahead.
+      // place in the stream of units: item k with n entries, `e` of them begun; unit = tile `i` of entry `ent`
+      int k = 0, n = 0, e = 0, i = 1, kstage = -1, q_cnt = 0, ntile_q = 0;
+      uint32_t ent = 0, ent_ahead = 0, kparity = 1u, left = 0, q_there = 0;   // units left of tile 0 | of tile 1 << 8; bit i: Q tile i has landed
+      bool open = false;    // item k is being worked on
+      bool new_k = false;   // the unit is the first of its entry
+      int n_flight = 0;     // units whose scores have been issued and whose P V has not
       enum : int { UNIT, STALLED, ENDED, ABORTED };
       auto wait_q = [&](int t) -> bool {
         q_there |= 1u << t;
         const int g = q_cnt + t;
         return wait(C::B_QFULL + g % C::NQ, (g / C::NQ) & 1, W_F_QFULL);
       };
-      // Moves to the next unit and waits for its operands. With units in flight it does not wait for an item's header, for
-      // the producer may need them to be finished to publish it (a run of empty items longer than the ring of headers).
-      auto advance = [&]() -> int {
+      // Closes the item in hand and opens the next one that has entries. With units in flight it does not wait for a header,
+      // for the producer may need them to be finished to publish it (a run of empty items longer than the ring of headers).
+      auto next_list = [&]() -> int {
         for (;;) {
-          if (i < 2) {
-            if (entry_class(ent, i) != 0u) return ((q_there >> i) & 1u) != 0u || wait_q(i) ? UNIT : ABORTED;
-            ++i;
-          } else if (e < n) {
-            ent = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(sList[(k % C::NITEM) * 128 + e]));
-            ++e;
-            i = 0;
-            if (++kstage == C::KST) kstage = 0;
-            if (kstage == 0) kparity ^= 1u;
-            if (!wait(C::B_KFULL + kstage, kparity, W_F_KFULL)) return ABORTED;
-          } else {
-            if (open) {
-              for (int t = 0; t < ntile_q; ++t) {   // tiles without units
-                if ((q_there >> t) & 1u) continue;
-                if (!wait_q(t)) return ABORTED;
-                if (elect_one()) mbar_arrive(bar(C::B_QEMPTY + (q_cnt + t) % C::NQ));
-              }
-              q_cnt += ntile_q;
-              item_done(k);
-              open = false;
-              ++k;
+          if (open) {
+            for (int t = 0; t < ntile_q; ++t) {   // tiles without units
+              if ((q_there >> t) & 1u) continue;
+              if (!wait_q(t)) return ABORTED;
+              if (elect_one()) mbar_arrive(bar(C::B_QEMPTY + (q_cnt + t) % C::NQ));
             }
-            if (n_flight > 0 && !__all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) return STALLED;
-            int4 it;
-            if (!next_item(k, it)) return abortf->v == 0u ? ENDED : ABORTED;
-            n = it.w & 0xFF;
-            left = static_cast<uint32_t>(it.w) >> 8;
-            ntile_q = (2 * it.z + 1 < a.NT) ? 2 : 1;
-            e = 0;
-            q_there = 0u;
-            open = true;
+            q_cnt += ntile_q;
+            item_done(k);
+            open = false;
+            ++k;
           }
+          if (n_flight > 0 && !__all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) return STALLED;
+          int4 it;
+          if (!next_item(k, it)) return abortf->v == 0u ? ENDED : ABORTED;
+          n = it.w & 0xFF;
+          left = static_cast<uint32_t>(it.w) >> 8;
+          ntile_q = (2 * it.z + 1 < a.NT) ? 2 : 1;
+          e = 0;
+          q_there = 0u;
+          open = true;
+          ent_ahead = sList[(k % C::NITEM) * 128];
+          if (n > 0) return UNIT;
         }
       };
       // What P V needs to know of the units whose scores are in flight, oldest in the low byte
       constexpr uint32_t U_TILE = 1u, U_FIRST = 2u, U_NEW_V = 4u, U_LAST_V = 8u;
-      uint32_t flight = 0u, used = 0u, used_par = 0u, vparity = 1u, pparity = 0u, began = 0u;
+      uint32_t flight = 0u, pv_issued = 0u, used = 0u, used_par = 0u, vparity = 1u, pparity = 0u, began = 0u;
       int sbuf = 0, pbuf = 0, vstage = -1;
       for (;;) {
-        const int next = __reduce_max_sync(0xffffffffu, advance());
-        if (next == ABORTED) break;
-        if (n_flight == C::NBUF || (next != UNIT && n_flight > 0)) {
-          const uint32_t t = flight & U_TILE;
-          if (flight & U_NEW_V) {
-            if (++vstage == C::VST) vstage = 0;
-            if (vstage == 0) vparity ^= 1u;
-            if (!wait(C::B_VFULL + vstage, vparity, W_F_VFULL)) break;
+        int next = UNIT;
+        if (i == 0 && entry_class(ent, 1) != 0u) {
+          i = 1;
+          new_k = false;
+        } else {
+          if (e == n) next = __reduce_max_sync(0xffffffffu, next_list());
+          if (next == ABORTED) break;
+          if (next == UNIT) {
+            if (e == 0) began = 0u;
+            ent = __reduce_or_sync(0xffffffffu, ent_ahead);
+            ++e;
+            ent_ahead = sList[(k % C::NITEM) * 128 + min(e, 127)];
+            i = entry_class(ent, 0) != 0u ? 0 : 1;
+            new_k = true;
+            if (++kstage == C::KST) kstage = 0;
+            if (kstage == 0) kparity ^= 1u;
           }
+        }
+        const bool s_now = next == UNIT, pv_now = n_flight == C::NBUF || (!s_now && n_flight > 0), new_v = pv_now && (flight & U_NEW_V) != 0u;
+        if (new_v) {
+          if (++vstage == C::VST) vstage = 0;
+          if (vstage == 0) vparity ^= 1u;
+        }
+        bool there = true;
+        if (s_now && new_k) there = mbar_test_wait(bar(C::B_KFULL + kstage), kparity);
+        if (new_v) there &= mbar_test_wait(bar(C::B_VFULL + vstage), vparity);
+        if (pv_now) there &= mbar_test_wait(bar(C::B_PFULL + C::NPART * pbuf), pparity);
+        if (!__all_sync(0xffffffffu, there)) {
+          if (s_now && new_k && !wait(C::B_KFULL + kstage, kparity, W_F_KFULL)) break;
+          if (new_v && !wait(C::B_VFULL + vstage, vparity, W_F_VFULL)) break;
+          if (pv_now && !wait(C::B_PFULL + C::NPART * pbuf, pparity, W_F_PFULL)) break;
+        }
+        if (s_now && ((q_there >> i) & 1u) == 0u && !wait_q(i)) break;
+        if (pv_now) {
+          const uint32_t t = flight & U_TILE;
           if (flight & U_FIRST) {
-            // the first product of a query tile overwrites O: the softmax warpgroup must have read the previous item's result
+            // the first product of a query tile overwrites O: the softmax warps must have read the previous item's result
             if ((used >> t) & 1u) {
               if (!wait(C::B_OFREE + t, (used_par >> t) & 1u, W_F_OFREE)) break;
               used_par ^= 1u << t;
@@ -382,86 +415,107 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             used |= 1u << t;
           }
           const uint32_t vlo = lo_v + vstage * T16, dO = C::TM_O0 + t * HD, acc0 = (flight & U_FIRST) ? 0u : 1u;
-          bool there = true;
+          tc_fence_after_sync();
 #pragma unroll
           for (int part = 0; part < C::NPART; ++part) {
-            if (!(there = wait(C::B_PFULL + C::NPART * pbuf + part, pparity, W_F_PFULL))) break;
-            tc_fence_after_sync();
-            constexpr int STEPS = KD_TILE / 16 / C::NPART;
+            if (part > 0) {
+              if (!(there = wait(C::B_PFULL + C::NPART * pbuf + part, pparity, W_F_PFULL))) break;
+              tc_fence_after_sync();
+            }
+            // P of 16 keys = 8 packed columns; a warp's 64 keys begin at the first of its score columns
 #pragma unroll
-            for (int kk = part * STEPS; kk < (part + 1) * STEPS; ++kk)   // P of 16 keys = 8 packed columns at the start of the score buffer
-              mma_ts_uniform(dO, pbuf * 128 + kk * 8, vlo + koff_mnmajor(kk), hi, idesc_o, kk > 0 ? 1u : acc0);
+            for (int kk = 0; kk < KD_TILE / 16; ++kk) {
+              if (((kk >> 1) & 1) != part) continue;
+              mma_ts_uniform(dO, pbuf * 128 + (kk >> 2) * C::CW + (kk & 3) * 8, vlo + koff_mnmajor(kk), hi, idesc_o, kk > 0 ? 1u : acc0);
+            }
           }
           if (!there) break;
-          commit_uniform(bar(C::B_PVDONE + t));
+          commit_uniform(bar(C::B_PVDONE + 2 * t + ((pv_issued >> t) & 1u)));
+          pv_issued ^= 1u << t;
           if (flight & U_LAST_V) commit_uniform(bar(C::B_VEMPTY + vstage));
           if (++pbuf == C::NBUF) { pbuf = 0; pparity ^= 1u; }
           flight >>= 8;
           --n_flight;
         }
-        if (next == ENDED && n_flight == 0) break;
-        if (next != UNIT) continue;
-        const uint32_t qlo = lo_q + ((q_cnt + i) % C::NQ) * T16, klo = lo_k + kstage * T16;
+        if (s_now) {
+          const uint32_t qlo = lo_q + ((q_cnt + i) % C::NQ) * T16, klo = lo_k + kstage * T16;
+          tc_fence_after_sync();
 #pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) mma_ss_uniform(sbuf * 128, qlo + koff_kmajor(kk), klo + koff_kmajor(kk), hi, idesc_s, kk > 0 ? 1u : 0u);
-        commit_uniform(bar(C::B_SFULL + 2 * sbuf + i));
-        const bool last_of_entry = i == 1 || entry_class(ent, 1) == 0u;
-        if (last_of_entry) commit_uniform(bar(C::B_KEMPTY + kstage));
-        left -= 1u << (8 * i);
-        if (((left >> (8 * i)) & 0xFFu) == 0u) commit_uniform(bar(C::B_QEMPTY + (q_cnt + i) % C::NQ));   // the tile's last product
-        if (e == 1 && (i == 0 || entry_class(ent, 0) == 0u)) began = 0u;   // first unit of the item
-        flight |= (static_cast<uint32_t>(i) | (((began >> i) & 1u) ? 0u : U_FIRST) | ((i == 0 || entry_class(ent, 0) == 0u) ? U_NEW_V : 0u) |
-                   (last_of_entry ? U_LAST_V : 0u)) << (8 * n_flight);
-        began |= 1u << i;
-        ++n_flight;
-        if (++sbuf == C::NBUF) sbuf = 0;
-        ++i;
+          for (int kk = 0; kk < HD / 16; ++kk) mma_ss_uniform(sbuf * 128, qlo + koff_kmajor(kk), klo + koff_kmajor(kk), hi, idesc_s, kk > 0 ? 1u : 0u);
+          commit_uniform(bar(C::B_SFULL + 2 * sbuf + i));
+          const bool last_of_entry = i == 1 || entry_class(ent, 1) == 0u;
+          if (last_of_entry) commit_uniform(bar(C::B_KEMPTY + kstage));
+          left -= 1u << (8 * i);
+          if (((left >> (8 * i)) & 0xFFu) == 0u) commit_uniform(bar(C::B_QEMPTY + (q_cnt + i) % C::NQ));   // the tile's last product
+          flight |= (static_cast<uint32_t>(i) | (((began >> i) & 1u) ? 0u : U_FIRST) | (new_k ? U_NEW_V : 0u) | (last_of_entry ? U_LAST_V : 0u)) << (8 * n_flight);
+          began |= 1u << i;
+          ++n_flight;
+          if (++sbuf == C::NBUF) sbuf = 0;
+        } else if (next == ENDED && n_flight == 0) {
+          break;
+        }
       }
     }
   } else {
     reg_alloc<C::REGS_COMPUTE>();
     // ------------------------------ softmax warpgroups ------------------------------
-    // One warpgroup per query tile; each thread owns one row of 128 scores.
+    // Two warpgroups per query tile; each thread owns half a row, 64 scores.
     constexpr int CW = C::CW, NW = CW / 32;
-    const int i = (warp - 4) >> 2;        // warpgroup = query tile of the pair
+    const int i = (warp - 4) >> 3;        // query tile of the pair
+    const int half = ((warp - 4) >> 2) & 1;   // columns 64 * half .. 64 * half + 63
     const int wq = warp & 3;              // TMEM lane quadrant of this warp
     const int row = wq * 32 + lane;       // row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t tO = lane_base + (i == 0 ? C::TM_O0 : C::TM_O1);   // this thread's row of O
+    const uint32_t tO = lane_base + (i == 0 ? C::TM_O0 : C::TM_O1) + half * (HD / 2);   // this thread's half of its row of O
+    float* xch = reinterpret_cast<float*>(smem + C::SMEM_XCH) + i * (2 * KD_TILE) + row;
+    // Both warps of 32 rows: hands over a value and takes the partner's; false: some role has aborted. The barrier cannot
+    // hang: a warp that gives up arrives there once more (below), and the partner sees the abort behind the barrier.
+    // With two buffers a slot is written again two exchanges later, when the partner, which has been to the barrier in between,
+    // has read it. Where shared memory has room for one only (HD = 128), other synchronisation lies between two exchanges.
+    const uint32_t pair_bar = 1 + i * 4 + wq;
+    int exchanges = 0;
+    auto exchange = [&](float mine, float& other) -> bool {
+      float* x = xch + (C::NXB == 2 ? (exchanges++ & 1) * (4 * KD_TILE) : 0);
+      x[half * KD_TILE] = mine;
+      named_bar_sync(pair_bar, 64);
+      other = x[(half ^ 1) * KD_TILE];
+      return __all_sync(0xffffffffu, abortf->v == 0u);
+    };
     const float c = a.scale_log2;
     const uint64_t c2 = pack_f32x2(c, c);
     bool ok = true;
     // state that runs on across the items of this CTA
-    int buf = 0;                // buffer of the next unit of either query tile
     uint32_t sfull_par = 0;     // bit j: parity of the next phase of this tile's score barrier on buffer j
-    int pv_seen = 0;            // P V products of this query tile issued so far (phases of bar_pv_done[i])
+    int pv_seen = 0;            // P V products of this query tile handed over so far
+    int last_buf = 0;           // buffer of this tile's last unit
+    // Waits for the last of them (back = 1), or the one before. Not for every unit: a product signals on one of two barriers in
+    // turn. A parity wait is sound while the barrier's phase before the awaited one is complete, that is the tile's product two
+    // before it. Once the scores of the tile's next unit are ready it is (products and scores execute in issue order, and at
+    // most NBUF - 1 products precede those scores unfinished); at the end of an item it is after a wait with back = 2.
+    auto pv_done = [&](int back) -> bool {
+      const int c = pv_seen - back;
+      return c < 0 || wait(C::B_PVDONE + 2 * i + (c & 1), (c >> 1) & 1, W_F_PVDONE);
+    };
     int4 it;
 
     for (int k = 0; ok && next_item(k, it); ++k) {
-    const int b = it.x, h = it.y, n = it.w & 0xFF, n_own = (it.w >> (8 + 8 * i)) & 0xFF;
+    const int b = it.x, h = it.y, n_own = (it.w >> (8 + 8 * i)) & 0xFF;
     const int qtile = 2 * it.z + i;
     const int qi = qtile * KD_TILE + row;  // token index of this thread's query
     const bool tile_valid = qtile < a.NT;
     const uint32_t qd = tile_valid ? __ldcg(a.desc + (size_t)b * a.Tpad + qi) : 0u;
-    uint32_t lst[4];   // the list, 32 entries per register
-#pragma unroll
-    for (int r = 0; r < 4; ++r) lst[r] = sList[(k % C::NITEM) * 128 + r * 32 + lane];
-    item_done(k);
-    // this query tile's next unit: sets ent_next and, in buf_next, its buffer; `e` is the entry after it
-    int e = 0;
-    uint32_t ent_next = 0u;
-    int buf_next = 0;
+    const uint16_t* list = sList + (k % C::NITEM) * 128;
+    // this query tile's next unit, of which there is one: sets ent_next and, in buf_next, its buffer
+    uint32_t ent_next = 0u, fetched = n_own > 0 ? list[0] : 0u;   // fetched: entry e, read one step ahead
+    int e = 0, buf_next = 0;
     auto find_next = [&]() {
-      while (e < n) {
-        const uint32_t r = e < 64 ? (e < 32 ? lst[0] : lst[1]) : (e < 96 ? lst[2] : lst[3]);
-        ent_next = __shfl_sync(0xffffffffu, r, e & 31);
+      do {
+        ent_next = __reduce_or_sync(0xffffffffu, fetched);
         ++e;
-        const bool u0 = entry_class(ent_next, 0) != 0u, u1 = entry_class(ent_next, 1) != 0u;
-        buf_next = buf;
-        if (u0) { if (i == 1 && ++buf_next == C::NBUF) buf_next = 0; if (++buf == C::NBUF) buf = 0; }
-        if (u1 && ++buf == C::NBUF) buf = 0;
-        if (i == 0 ? u0 : u1) return;
-      }
+        fetched = list[min(e, 127)];
+      } while (entry_class(ent_next, i) == 0u);
+      buf_next = static_cast<int>(ent_next >> 12) + ((i == 1 && entry_class(ent_next, 0) != 0u) ? 1 : 0);
+      if (buf_next >= C::NBUF) buf_next -= C::NBUF;
     };
     // Key descriptors (lane L holds keys L, 32 + L, ...) and class masks of PARTIAL tiles are fetched one unit ahead
     // into registers, so their global-memory latency overlaps the previous tile's softmax.
@@ -473,20 +527,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (entry_class(ent, i) == KD_TILE_PARTIAL) {
         const int kt = ent & 0xFF;
         const uint32_t* src = a.desc + (size_t)b * a.Tpad + (size_t)kt * KD_TILE;
-        const uint4* tbp = reinterpret_cast<const uint4*>(a.tilebits + ((size_t)b * a.NT + kt) * 32);
+        const uint2* tbp = reinterpret_cast<const uint2*>(a.tilebits + ((size_t)b * a.NT + kt) * 32);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) kd_pre[w] = __ldcg(src + w * 32 + lane);
-        static_assert(NW == 4, "a class mask of a tile is four words: one 16-byte load each");
+        for (int w = 0; w < NW; ++w) kd_pre[w] = __ldcg(src + half * CW + w * 32 + lane);
+        static_assert(NW == 2, "a class mask of half a tile is two words: one 8-byte load each");
         constexpr int cls3[3] = {TB_PRE, TB_CTX, TB_INS};
 #pragma unroll
         for (int k3 = 0; k3 < 3; ++k3) {
-          const uint4 m4 = __ldcg(tbp + cls3[k3]);
-          tb_pre[k3][0] = m4.x; tb_pre[k3][1] = m4.y; tb_pre[k3][2] = m4.z; tb_pre[k3][3] = m4.w;
+          const uint2 m2 = __ldcg(tbp + cls3[k3] * 2 + half);
+          tb_pre[k3][0] = m2.x; tb_pre[k3][1] = m2.y;
         }
       }
     };
-    find_next();
-    if (n_own > 0) prefetch_kd(ent_next);
+    if (n_own > 0) {
+      find_next();
+      prefetch_kd(ent_next);
+    }
     if (k == 0) pdl_wait();   // O and LSE are written from here on
     float m = -INFINITY, l = 0.f;
     int nact = 0;
@@ -495,7 +551,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t ent = ent_next;
       const uint32_t cls = entry_class(ent, i);
       const int kt = ent & 0xFF, sbuf = buf_next;
-      const uint32_t tS = lane_base + sbuf * 128;
+      const uint32_t tS = lane_base + sbuf * 128 + half * CW;
       if (!(ok = wait(C::B_SFULL + 2 * sbuf + i, (sfull_par >> sbuf) & 1u, W_F_SFULL))) break;
       sfull_par ^= 1u << sbuf;
       tc_fence_after_sync();
@@ -508,11 +564,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int j = 0; j < 32; ++j) sc[cb * 32 + j] = __uint_as_float(r[j]);
       }
+      if (u + 1 < n_own) find_next();   // while the scores are on their way
       tmem_wait_ld();
       if (cls == KD_TILE_PARTIAL) {
         // The row's visibility mask comes from the tile's class masks with a few word-wide
         // operations; only the "same span" term needs the individual key descriptors.
-        const int j0 = kt * KD_TILE;
+        const int j0 = kt * KD_TILE + half * CW;
         uint32_t mk[NW];
         query_row_mask<NW>(qd, qi, j0, tb_pre[0], tb_pre[1], tb_pre[2], mk);
         uint32_t any_ins = 0u;
@@ -540,7 +597,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if ((mk[w] & (1u << j)) == 0u) sc[w * 32 + j] = -INFINITY;
         }
       }
-      find_next();   // (after the item's last unit it runs over the rest of the list, which counts the other tile's buffers)
       if (u + 1 < n_own) prefetch_kd(ent_next);
       // four independent chains for the row maximum and for the row sum: a single chain of
       // dependent operations would be latency-bound
@@ -555,6 +611,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
       for (int k4 = 0; k4 < 4; ++k4) mx4[k4] = fmaxf(mx4[k4], sc[CW - 4 + k4]);
       float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      if (C::NXB == 1 && nact > 0 && sbuf != last_buf) {
+        // Consecutive units of one tile: the scores can be ready before the partner has read this warp's last maximum, which
+        // it does before it hands over its P. (Otherwise they have been issued behind that P's product.)
+        if (!(ok = pv_done(1))) break;
+      }
+      last_buf = sbuf;
+      float mx_other;
+      if (!(ok = exchange(mx, mx_other))) break;
+      mx = fmaxf(mx, mx_other);
       // The running maximum is refreshed only when it would grow by more than 2^8 in the
       // exponent; until then the stale value is used consistently for P, l and O, which leaves
       // the normalised result unchanged and skips most O rescales.
@@ -563,16 +628,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * c);
       const bool need_rescale = (nact > 0) && (m_new != m);
-      if (nact > 0) {
-        // O_i may be touched only after the previous P V product of this query tile has completed;
-        // the wait is taken for every unit so that no phase of the barrier goes unobserved
-        if (!(ok = wait(C::B_PVDONE + i, (pv_seen - 1) & 1, W_F_PVDONE))) break;
-      }
-      if (__any_sync(0xffffffffu, need_rescale)) {
+      if (__any_sync(0xffffffffu, need_rescale)) {   // O may be touched only after the tile's previous product
+        if (!(ok = pv_done(1))) break;
         tc_fence_after_sync();
         const float f = need_rescale ? alpha : 1.f;
 #pragma unroll 1
-        for (int cb = 0; cb < HD / 16; ++cb) {   // rare; 16 columns at a time, for the scores are still in registers
+        for (int cb = 0; cb < HD / 32; ++cb) {   // rare; 16 columns at a time, for the scores are still in registers
           uint32_t r[16];
           tmem_ld16(tO + cb * 16, r);
           tmem_wait_ld();
@@ -594,12 +655,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           pk[j / 2] = pack2<kBf16>(p0, p1);
         }
         tmem_st16(tS + cb * 16, pk);
-        if ((cb + 1) % (NW / C::NPART) == 0) {   // this part of P is complete: its product runs under the next exponentials
-          tmem_wait_st();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(C::B_PFULL + C::NPART * sbuf + cb / (NW / C::NPART)));
-        }
+        // this part of P is complete: its product runs under the next exponentials
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::B_PFULL + C::NPART * sbuf + cb));
       }
       const uint64_t sum_pair = add_f32x2(sum2[0], sum2[1]);
       l = l * alpha + (lo_f32x2(sum_pair) + hi_f32x2(sum_pair));
@@ -608,20 +668,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       ++pv_seen;
     }
     if (!ok) break;
+    item_done(k);
 
     // epilogue of this item: normalise, convert, store this thread's share of O, and LSE
-    if (nact > 0) {
-      ok = wait(C::B_PVDONE + i, (pv_seen - 1) & 1, W_F_PVDONE);
+    if (nact > 0 && !(ok = pv_done(2) && pv_done(1))) break;
+    float l_other;
+    if (!(ok = exchange(l, l_other))) break;
+    if constexpr (C::NXB == 1) {   // both have read the sums: the slot may be written again
+      named_bar_sync(pair_bar, 64);
+      if (!(ok = __all_sync(0xffffffffu, abortf->v == 0u))) break;
     }
-    if (ok && tile_valid && qi < a.T) {
+    l += l_other;
+    if (half == 0 && tile_valid && qi < a.T) {
       a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
     }
-    if (ok) {
+    {
       tc_fence_after_sync();
       const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
       uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)qi * a.o_st;
 #pragma unroll
-      for (int cb = 0; cb < HD / 32; ++cb) {
+      for (int cb = 0; cb < HD / 64; ++cb) {
         uint32_t r[32];
         if (nact > 0) {
           tmem_ld32(tO + cb * 32, r);
@@ -630,16 +696,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = 0u;
         }
-        if (cb == HD / 32 - 1 && nact > 0) {
+        if (cb == HD / 64 - 1 && nact > 0) {
           // this thread's share of O_i has been read out: the next item's first product may overwrite it
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(C::B_OFREE + i));
         }
-        if (tile_valid && qi < a.T) store_row32_upto<kBf16>(orow + cb * 32, r, inv_l, cb * 32, a.d_real);
+        if (tile_valid && qi < a.T) store_row32_upto<kBf16>(orow + half * (HD / 2) + cb * 32, r, inv_l, half * (HD / 2) + cb * 32, a.d_real);
       }
     }
     }  // items
+    if (abortf->v != 0u) named_bar_arrive(pair_bar, 64);
   }
 
   tc_fence_before_sync();

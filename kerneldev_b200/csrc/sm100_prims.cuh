@@ -514,6 +514,9 @@ __device__ __forceinline__ float2 unpack2(uint32_t v) {
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
+__device__ __forceinline__ void named_bar_arrive(uint32_t id, uint32_t nthreads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
+}
 
 template <uint32_t kRegs>
 __device__ __forceinline__ void reg_dealloc() {
