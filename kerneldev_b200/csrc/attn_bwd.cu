@@ -133,6 +133,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __shared__ AbortFlag abortf;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (!a.plan_ready) pdl_wait();
   const int h0 = blockIdx.x * a.G, b = blockIdx.y;
   const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
   const int qt = a.order[((size_t)b * 3 + 1) * a.NT + blockIdx.z];   // longest lists first
@@ -508,6 +509,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __shared__ AbortFlag abortf;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (!a.plan_ready) pdl_wait();
   const int h0 = blockIdx.x * a.G, b = blockIdx.y;
   const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
   const int kt = a.order[((size_t)b * 3 + 2) * a.NT + blockIdx.z];   // longest lists first
@@ -924,6 +926,8 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.d_o = p.d_o.ptr; a.do_sb = p.d_o.stride_b; a.do_sh = p.d_o.stride_h; a.do_st = p.d_o.stride_t;
   a.lse = p.lse; a.delta = p.delta;
+  // with the delta kernel ahead of them in this call, the plan was complete before the kernels may start
+  a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
   a.dq_acc = fused ? p.dq_acc : nullptr;
   a.dq = p.dq.ptr; a.dq_sb = p.dq.stride_b; a.dq_sh = p.dq.stride_h; a.dq_st = p.dq.stride_t;

@@ -22,6 +22,7 @@ struct BwdArgs {
   int64_t o_sb, o_sh, o_st;
   const void* d_o;
   int64_t do_sb, do_sh, do_st;
+  int plan_ready;    // the plan may be read before the wait for the kernel ahead
   const float* lse;
   float* delta;
   float* dq_acc;     // fp32 (B,H,T,tile width) dQ accumulation scratch of the fused backward, else null

@@ -182,7 +182,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after_sync();
   // With the delta kernel directly before this one, everything but delta and the zeroed dQ scratch was complete before that
-  // kernel let this one start: the plan, Q, K, V, dO and LSE may be read, and dK and dV written, before the wait.
+  // kernel let this one start: the plan, Q, K, V, dO and LSE may be read, and dK and dV written, before the wait (plain reads
+  // past L1, which the start of a kernel that overlaps another need not have cleaned).
   if (!fa.after_delta) pdl_wait();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
@@ -236,9 +237,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         int4 it;
         it.x = bh / a.H;
         it.y = bh - it.x * a.H;
-        const int kt = a.order[((size_t)it.x * 3 + 2) * a.NT + rank];   // longest lists first
-        it.w = a.bwd_cnt[it.x * a.NT + kt];
-        it.z = kt | (static_cast<int>(a.bwd_list[((size_t)it.x * a.NT + kt) * a.NT]) << 16);
+        const int kt = __ldcg(a.order + ((size_t)it.x * 3 + 2) * a.NT + rank);   // longest lists first
+        it.w = __ldcg(a.bwd_cnt + it.x * a.NT + kt);
+        it.z = kt | (static_cast<int>(__ldcg(a.bwd_list + ((size_t)it.x * a.NT + kt) * a.NT)) << 16);
         return it;
       };
       int asked = 0;   // cancellations asked for
@@ -635,6 +636,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t ds_sw = static_cast<uint32_t>((lane >> 4) ^ (lane & 7)) << 4;
     bool ok = true;
     int t = 0, qs = 0;
+    uint32_t q_parity = 0u;   // of the Q stage's "full" phase
     int4 it;
     // visibility of this lane's key for the warpgroup's 64 queries
     auto mask_words = [&](const float* side, uint32_t kdesc, int kj, int i0, uint32_t qd0, uint32_t qd1, uint32_t (&mk)[2]) {
@@ -690,7 +692,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!more && t == 0) break;
         const int b = it.x, kt = it.z & 0xFFFF, n = more ? it.w : 1;
         const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
-        const uint32_t kdesc = more ? a.desc[(size_t)b * a.Tpad + kj] : 0u;
+        const uint32_t kdesc = more ? __ldcg(a.desc + (size_t)b * a.Tpad + kj) : 0u;
 #pragma unroll 1
         for (int e = 0; e < n; ++e, ++t) {
           if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
@@ -777,24 +779,31 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int k = 0; ok && next_item(k, it); ++k) {
       const int b = it.x, kt = it.z & 0xFFFF, n = it.w;
       const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
-      const uint32_t kdesc = a.desc[(size_t)b * a.Tpad + kj];
+      const uint32_t kdesc = __ldcg(a.desc + (size_t)b * a.Tpad + kj);
       const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
       uint32_t ent_next = static_cast<uint32_t>(it.z) >> 16;
       for (int e = 0; e < n; ++e, ++t) {
         const uint32_t ent = ent_next;
-        if (e + 1 < n) ent_next = list[e + 1];
+        if (e + 1 < n) ent_next = __ldcg(list + e + 1);
         const bool partial = (ent >> 8) == KD_TILE_PARTIAL;
         const int i0 = (ent & 0xFF) * KD_TILE + w * 64;
         uint32_t qd0 = 0u, qd1 = 0u;
         if (partial) {   // query descriptors for the same-span ballots, requested ahead of the wait
-          qd0 = a.desc[(size_t)b * a.Tpad + i0 + lane];
-          qd1 = a.desc[(size_t)b * a.Tpad + i0 + 32 + lane];
+          qd0 = __ldcg(a.desc + (size_t)b * a.Tpad + i0 + lane);
+          qd1 = __ldcg(a.desc + (size_t)b * a.Tpad + i0 + 32 + lane);
         }
         // LSE, delta and mask words of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here
+        const float* side = sSide + qs * C::SIDE_WORDS;
+        bool masked = false;
+        uint32_t mk[2] = {0u, 0u};
+        if (partial) {   // before the wait for the scores, from what came with the Q tile (many a block of such a tile is visible as a whole)
+          if (!(ok = wait(C::B_QFULL + qs, q_parity, W_U_QFULL))) break;
+          mask_words(side, kdesc, kj, i0, qd0, qd1, mk);
+          masked = __any_sync(0xffffffffu, (mk[0] & mk[1]) != 0xFFFFFFFFu);
+        }
         if (!(ok = wait(C::B_SFULL, t & 1, W_U_SFULL))) break;
         tc_fence_after_sync();
-        const float* side = sSide + qs * C::SIDE_WORDS;
-        if (++qs == C::QS) qs = 0;
+        if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
         uint32_t s[2][32];
         tmem_ld16x256_x8(tS, s[0]);
         tmem_ld16x256_x8(tS + ROW16, s[1]);
@@ -802,8 +811,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
         for (int j = 0; j < 8; ++j) col[j] = ld_shared_pair(side + qcol + 8 * j);   // LSE of this thread's columns
         tmem_wait_ld();
-        uint32_t mk[2] = {0u, 0u};
-        if (partial) mask_words(side, kdesc, kj, i0, qd0, qd1, mk);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {   // 16 keys at a time
 #pragma unroll
@@ -815,7 +822,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               s[hf][4 * j + 2 * r + 1] = __float_as_uint(fast_exp2(-hi_f32x2(x)));
             }
           }
-          if (partial) apply_mask(s[hf], mk, hf);
+          if (masked) apply_mask(s[hf], mk, hf);
           uint32_t pk[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(s[hf][2 * j]), __uint_as_float(s[hf][2 * j + 1]));
