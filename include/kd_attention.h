@@ -107,7 +107,7 @@ typedef struct kd_attn_params {
   kd_tensor o;       /* forward: output; backward: input */
   kd_tensor d_o;     /* backward input dO */
   kd_tensor dq, dk, dv; /* backward outputs */
-  float* lse;        /* (B,H,T) contiguous, base-2 log-sum-exp: m + log2(l)
+  float* lse;        /* (B,H,T) contiguous, base-2 log-sum-exp (kd_attn_fwd: may be NULL, it is not written then): m + log2(l)
                         (original_kernel.py:603-604); forward output, backward input */
   float* delta;      /* (B,H,T) contiguous fp32 scratch of the backward: rowsum(O * dO)
                         (kd_workspace_bytes gives its size) */

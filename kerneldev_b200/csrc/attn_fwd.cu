@@ -691,7 +691,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (!(ok = __all_sync(0xffffffffu, abortf->v == 0u))) break;
     }
     l += l_other;
-    if (half == 0 && qi < a.T) {
+    if (half == 0 && qi < a.T && a.lse != nullptr) {
       a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
     }
     {

@@ -111,7 +111,7 @@ static int check_attn(const kd_attn_params* p, bool backward) {
   if (!(p->sm_scale > 0.f) || !(p->sm_scale < 1e30f)) return set_error(KD_ERR_ARG, "sm_scale must be positive and finite");
   if (p->heads_per_cta < 0) return set_error(KD_ERR_ARG, "heads_per_cta must be 0 (automatic) or positive");
   if (!p->plan) return set_error(KD_ERR_ARG, "plan is null (call kd_classify first)");
-  if (!p->lse) return set_error(KD_ERR_ARG, "lse is null");
+  if (backward && !p->lse) return set_error(KD_ERR_ARG, "lse is null");
   if (!p->o.ptr) return set_error(KD_ERR_ARG, "o is null");
   if ((reinterpret_cast<uintptr_t>(p->o.ptr) & 15u) || ((p->o.stride_t * 2) & 15) || ((p->o.stride_h * 2) & 15) || ((p->o.stride_b * 2) & 15))
     return set_error(KD_ERR_ALIGN, "o: pointer and byte strides must be multiples of 16");

@@ -81,16 +81,16 @@ constexpr uint32_t kStatusTimeout = KD_STATUS_TIMEOUT, kStatusSpanRange = KD_STA
 // Status mirrors of the plans: one pinned block handed out in rotation (pinning is a slow, device-wide call).
 // 1024 words: a collision would need more than 1024 live plans and could only make a reported failure show up on
 // two of them.
-Tensor pinned_word() {
+std::pair<Tensor, int> pinned_word() {   // the block and the word's index in it
   static std::mutex m;
   static Tensor block;
   static int next = 0;
   std::lock_guard<std::mutex> lock(m);
   if (!block.defined()) block = at::zeros({1024}, at::TensorOptions().dtype(at::kInt)).pin_memory();
-  Tensor w = block.narrow(0, next, 1);
+  const int word = next;
   next = (next + 1) % 1024;
-  *w.data_ptr<int32_t>() = 0;
-  return w;
+  block.data_ptr<int32_t>()[word] = 0;
+  return {block, word};
 }
 
 bool check_every_launch() {
@@ -102,8 +102,12 @@ struct Plan {
   int64_t B, T;
   at::Device device;
   kd_plan_layout layout;
-  Tensor buf, status_dev, status_host;
+  Tensor buf;
+  std::pair<Tensor, int> mirror;   // the status word's copy in host memory
   volatile uint32_t* host_word;
+  // the status word and its mirror as tensors: views cost more than a launch, and only reports and tests want them
+  Tensor status_dev() const { return buf.narrow(0, static_cast<int64_t>(layout.off_status), 4).view(at::kInt); }
+  Tensor status_host() const { return mirror.first.narrow(0, mirror.second, 1); }
   std::vector<Tensor> keep;   // the caller's metadata and its converted copies, alive as long as the plan is cached
   at::cuda::CUDAStream built_on;
   at::cuda::CUDAEvent built;
@@ -141,10 +145,8 @@ struct Plan {
     }
     meta.causal = causal;
     meta.rules = rules;
-    const int64_t off = static_cast<int64_t>(layout.off_status);
-    status_dev = buf.narrow(0, off, 4).view(at::kInt);
-    status_host = pinned_word();
-    host_word = reinterpret_cast<volatile uint32_t*>(status_host.data_ptr<int32_t>());
+    mirror = pinned_word();
+    host_word = reinterpret_cast<volatile uint32_t*>(mirror.first.data_ptr<int32_t>() + mirror.second);
     meta.status_mirror = const_cast<uint32_t*>(host_word);
     c10::cuda::CUDAGuard guard(dev);
     check(lib.classify(&meta, buf.data_ptr(), built_on.stream()));
@@ -182,13 +184,13 @@ struct Plan {
 
   // Synchronises the current stream, reads the device status word and raises if it is set.
   void check_status() {
-    const uint32_t s = static_cast<uint32_t>(status_dev.item<int32_t>());
+    const uint32_t s = static_cast<uint32_t>(status_dev().item<int32_t>());
     if (s != 0) report(s);
   }
 
   [[noreturn]] void report(uint32_t s) {
     // both copies are cleared, so that one event is reported once and later launches start clean
-    status_dev.zero_();
+    status_dev().zero_();
     *host_word = 0;
     TORCH_CHECK_VALUE((s & kStatusSpanRange) == 0, "span_id values must fit in 24 signed bits (|span_id| < 2**23)");
     char hex[16], site[16];
@@ -340,17 +342,17 @@ kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const T
   p.k = desc(k);
   p.v = desc(v);
   p.o = desc(o);
-  p.lse = lse.data_ptr<float>();
+  p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
   p.plan = plan.buf.data_ptr();
   p.heads_per_cta = heads_per_cta;
   return p;
 }
 
 std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const PlanPtr& plan, double sm_scale,
-                                   bool like_input, int heads_per_cta) {
+                                   bool like_input, int heads_per_cta, bool want_lse = true) {
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
-  Tensor o = empty_out(q, like_input);
-  Tensor lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
+  Tensor o = empty_out(q, like_input), lse;
+  if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
@@ -511,7 +513,7 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v) {
 
 std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& lens, std::optional<double> sm_scale,
                                      bool causal, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix, bool rules,
-                                     const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta) {
+                                     const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta, bool return_lse) {
   check_inputs(q, k, v);
   const double scale = sm_scale.has_value() ? *sm_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
   KD_VALUE(scale > 0.0 && std::isfinite(scale), "sm_scale must be positive and finite");
@@ -535,7 +537,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
       q2 = hadamard(q2, signs, false);
       k2 = hadamard(k2, signs, false);
     }
-    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, heads_per_cta);
+    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, heads_per_cta, return_lse || track);
     o = f32 ? cast({o16}, at::kFloat)[0] : o16;
   }
   if (track) {
@@ -694,14 +696,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readonly("T", &Plan::T)
       .def_readonly("device", &Plan::device)
       .def_readonly("buf", &Plan::buf)
-      .def_readonly("status_dev", &Plan::status_dev)
-      .def_readonly("status_host", &Plan::status_host)
+      .def_property_readonly("status_dev", &Plan::status_dev)
+      .def_property_readonly("status_host", &Plan::status_host)
       .def("use_on_current_stream", &Plan::use_on_current_stream);
   m.def("bind", &bind);
   m.def("get_plan", &get_plan);
   m.def("cached_plans", [] { return cache().values(); });
   m.def("clear_plans", [] { cache().clear(); });
-  m.def("forward", &forward);
+  m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const PlanPtr& plan, double sm_scale, bool like_input, int heads_per_cta) {
+    return forward(q, k, v, plan, sm_scale, like_input, heads_per_cta);
+  });
   m.def("backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, const PlanPtr& plan,
                        double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic, int heads_per_cta) {
     Tensor b[5];

@@ -170,7 +170,7 @@ def flash_attention(
             raise ValueError("hadamard_signs needs a head_dim in {16, 32, 64, 128}")
         hadamard_signs = _check_signs(hadamard_signs, q.shape[1], q.shape[3], q.device)
     o, lse = _ext.attention(q, k, v, lens, sm_scale, bool(causal), in_span, span_id, is_prefix, rules, hadamard_signs,
-                            out_layout == "input", bool(deterministic), HEADS_PER_CTA)
+                            out_layout == "input", bool(deterministic), HEADS_PER_CTA, bool(return_lse))
 
     if return_attention_mask:
         B, H, T, _ = q.shape
