@@ -2,6 +2,7 @@
 // descriptors (so the single MMA-issuing thread spends two integer adds per MMA, not a 64-bit
 // descriptor build), work-list staging, 16-bit row stores.
 #pragma once
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -191,6 +192,32 @@ inline int heads_per_cta(int B, int H, int items_per_batch, int forced, int per_
   if (g > H) g = H;
   return static_cast<int>(g);
 }
+
+// Order of a launch's items (tiles of one (batch, head) pair): chunks of heads whose tensors share L2, inside a chunk rank by
+// rank (longest lists first) and for a rank head by head. The chunks differ by one head at most: each begins with its longest
+// items, and a small last one gets them when the SMs run out of work (hier 8 x 16 x 2048 x 64: backward 207 us, 198 with even
+// chunks).
+struct ItemOrder {
+  int heads, big;   // (batch, head) pairs of a chunk; the first `big` chunks have one more
+  __device__ __forceinline__ void decode(int idx, int per_head, int& bh, int& rank) const {
+    const int in_big = big * (heads + 1) * per_head;
+    const bool second = idx >= in_big;
+    const int n = second ? heads : heads + 1, rest = second ? idx - in_big : idx;
+    const int c = rest / (n * per_head), r = rest - c * n * per_head;
+    rank = r / n;
+    bh = (second ? big * (heads + 1) : 0) + c * n + (r - rank * n);
+  }
+  // as many (batch, head) pairs to a chunk as take l2_bytes, and enough of them that it holds two items per SM
+  static ItemOrder make(int pairs, int per_head, double pair_bytes, double l2_bytes) {
+    long long chunk = static_cast<long long>(std::min<double>(pairs, std::max(1.0, l2_bytes / pair_bytes)));
+    chunk = std::min<long long>(pairs, std::max<long long>(chunk, (296 + per_head - 1) / per_head));
+    const int n = static_cast<int>(pairs / chunk);
+    ItemOrder o;
+    o.heads = pairs / n;
+    o.big = pairs % n;
+    return o;
+  }
+};
 
 // Raises a kernel's dynamic shared-memory limit, once per device (one instance per kernel): the attribute call
 // costs about a microsecond of host time, which a small launch would pay every time.

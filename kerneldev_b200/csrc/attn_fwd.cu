@@ -37,7 +37,7 @@ namespace kd {
 
 struct FwdArgs {
   int B, H, T, NT, NP, Tpad;
-  int chunk;         // (batch, head) pairs per chunk of items
+  ItemOrder order_of;
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
   const uint32_t* desc;
@@ -101,21 +101,6 @@ enum : uint32_t {
 // list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10; in shared memory also
 // | score buffer of the entry's first unit << 12
 __device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
-
-// Items of the launch in order: chunks of `chunk` (batch, head) pairs; inside a chunk rank by rank (longest lists first), and
-// for a rank head by head.
-struct ItemOrder {
-  int b, h, rank;
-  __device__ __forceinline__ ItemOrder(int idx, int chunk, int per_head, int B, int H) {
-    const int per_chunk = chunk * per_head;
-    const int c = idx / per_chunk, rem = idx - c * per_chunk;
-    const int heads = min(chunk, B * H - c * chunk);   // (batch, head) pairs of this chunk
-    rank = rem / heads;
-    const int bh = c * chunk + (rem - rank * heads);
-    b = bh / H;
-    h = bh - b * H;
-  }
-};
 
 template <int HD, bool kBf16>
 __global__ void __launch_bounds__(FwdCfg<HD>::THREADS, 1)
@@ -198,13 +183,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       uint32_t unit0 = 0u;  // score buffer of the next item's first unit
       uint32_t lst[4];      // the next item's list, 32 entries per register
       auto decode = [&](int idx) -> int4 {
-        const ItemOrder io(idx, a.chunk, a.NP, a.B, a.H);
         int4 it;
-        it.x = io.b;
-        it.y = io.h;
-        it.z = __ldcg(a.order + ((size_t)io.b * 3 + 0) * a.NT + io.rank);
-        const uint16_t* list = a.fwd_list + ((size_t)io.b * a.NP + it.z) * a.NT;
-        it.w = __ldcg(a.fwd_cnt + io.b * a.NP + it.z);
+        int rank;
+        a.order_of.decode(idx, a.NP, it.x, rank);
+        it.y = it.x % a.H;
+        it.x = it.x / a.H;
+        it.z = __ldcg(a.order + ((size_t)it.x * 3 + 0) * a.NT + rank);
+        const uint16_t* list = a.fwd_list + ((size_t)it.x * a.NP + it.z) * a.NT;
+        it.w = __ldcg(a.fwd_cnt + it.x * a.NP + it.z);
 #pragma unroll
         for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
 #pragma unroll
@@ -741,13 +727,8 @@ static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   a.scale_log2 = p.sm_scale * 1.4426950408889634f;
   const long long n_items = (long long)p.B * p.H * L.NP;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 256) exceeds 2^31 - 1");
-  // (batch, head) pairs whose Q, K, V and O take about 64 MB of the 126 MB L2 together, and enough of them that a chunk
-  // holds two items per SM
-  const double pair_bytes = (double)p.T * p.D * 2 * 4;
-  a.chunk = static_cast<int>(std::min<double>((double)p.B * p.H, std::max(1.0, 64e6 / pair_bytes)));
-  while ((long long)a.chunk * L.NP < 296 && a.chunk < p.B * p.H) ++a.chunk;
-  const int n_chunks = (p.B * p.H) / a.chunk;   // equal chunks, none smaller: a small last one would leave SMs idle
-  a.chunk = (p.B * p.H + n_chunks - 1) / n_chunks;
+  // Q, K, V and O. (64 and 110 MB: no difference outside the noise)
+  a.order_of = ItemOrder::make(p.B * p.H, L.NP, (double)p.T * p.D * 2 * 4, 64e6);
   a.plan_ready = p.plan_ready;
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
   a.order = pv.order; a.tilebits = pv.tilebits;
