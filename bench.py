@@ -18,7 +18,7 @@ The one JSON line printed by rank 0:
              backward per element of a non-empty tile (BASELINE.json's "unmasked-tile" count; PARTIAL
              tiles count in full, recomputation is not counted). `flops_exact_pairs` gives the same
              figure with 14*D*H * (allowed (query, key) pairs) instead.
-  plan       time of the tile classifier (3 launches per new metadata batch) and `value_with_plan`, the
+  plan       time of the tile classifier (2 launches per new metadata batch) and `value_with_plan`, the
              headline figure when a new plan is built every step instead of being reused.
   e2e        the same metric through flash_attention() + autograd with HOST (pinned) buffers: every
              step copies Q, K, V, dO host->device and O, dQ, dK, dV device->host; `copy_ceiling_ms` is
@@ -247,8 +247,7 @@ class Workload:
         self.f_eff = 14.0 * self.D * self.H * 128.0 * 128.0 * self.nonempty
         self.bufs = (torch.empty_like(self.q), torch.empty_like(self.q), torch.empty_like(self.q),
                      torch.empty((self.B, self.H, self.L), dtype=torch.float32, device=dev),
-                     torch.empty(shape, dtype=torch.float32, device=dev) if self.D == 64 else None)
-        self.fused = self.D == 64
+                     torch.empty((self.B, self.H, self.L, 64 if self.D <= 64 else 128), dtype=torch.float32, device=dev))
         self.launches_per_step = 4 + (4 if self.signs is not None else 0)
 
     def new_plan(self, cached=True):
@@ -305,17 +304,11 @@ def kernel_times(w, iters):
     per_pair = w.D * w.H * 128.0 * 128.0 * w.nonempty
     ms_fwd = time_call(lambda: _forward(qq, kk, w.v, w.plan, w.sm_scale), iters)
     bw = lambda ph: time_call(lambda: _backward(qq, kk, w.v, o, lse, w.do, w.plan, w.sm_scale, ph, w.bufs), iters)
-    if w.fused:
-        return {
-            # name: (ms, algorithmic FLOPs per launch, executed MMA FLOPs per launch)
-            "attn_fwd_kernel": (ms_fwd, 4 * per_pair, 4 * per_pair),
-            "attn_bwd_delta_kernel": (bw(1), 0.0, 0.0),
-            "attn_bwd_fused_kernel": (bw(2), 10 * per_pair, 10 * per_pair),   # S, dP, dV, dK, dQ (+ the dQ conversion kernel)
-        }
     return {
+        # name: (ms, algorithmic FLOPs per launch, executed MMA FLOPs per launch)
         "attn_fwd_kernel": (ms_fwd, 4 * per_pair, 4 * per_pair),
-        "attn_bwd_dq_kernel": (bw(1), 6 * per_pair, 6 * per_pair),        # delta; S, dP, dQ
-        "attn_bwd_dkdv_kernel": (bw(2), 4 * per_pair, 8 * per_pair),      # dV, dK (+ recomputed S, dP)
+        "attn_bwd_delta_kernel": (bw(1), 0.0, 0.0),
+        "attn_bwd_fused_kernel": (bw(2), 10 * per_pair, 10 * per_pair),   # S, dP, dV, dK, dQ (+ the dQ conversion kernel)
     }
 
 
@@ -427,14 +420,13 @@ def run_ours(args, cfg):
         "kernels_ms": {n: kernels[n][0] for n in kernels},
         "kernels_algorithmic_tflops": {n: kernels[n][1] / (kernels[n][0] * 1e-3) / 1e12 for n in kernels},
     }
-    if w.fused:
-        red_bytes = w.nonempty * w.H * 128.0 * w.D * 4.0     # one fp32 dQ tile per non-empty tile and head
-        ms_f = kernels["attn_bwd_fused_kernel"][0]
-        roofline["dq_accumulate"] = {
-            "reduce_bytes_per_launch": red_bytes, "GBps": red_bytes / (ms_f * 1e-3) / 1e9,
-            "hbm_peak_GBps": peak_hbm,
-            "note": "fp32 bytes of the dQ tiles the TMA bulk reductions add into the scratch, over the fused kernel's time; the adds run in L2, "
-                    "HBM sees the scratch once zeroed, once written back and once read by the conversion kernel"}
+    red_bytes = w.nonempty * w.H * 128.0 * w.D * 4.0     # one fp32 dQ tile per non-empty tile and head
+    ms_f = kernels["attn_bwd_fused_kernel"][0]
+    roofline["dq_accumulate"] = {
+        "reduce_bytes_per_launch": red_bytes, "GBps": red_bytes / (ms_f * 1e-3) / 1e9,
+        "hbm_peak_GBps": peak_hbm,
+        "note": "fp32 bytes of the dQ tiles the TMA bulk reductions add into the scratch, over the fused kernel's time; the adds run in L2, "
+                "HBM sees the scratch once zeroed, once written back and once read by the conversion kernel"}
 
     # ---- end to end: public API with host buffers ------------------------------------------------
     e2e = None
@@ -524,7 +516,7 @@ def run_ours(args, cfg):
             "config": {"workload": cfg["name"], "per_gpu_batch": B, "heads": H, "seq_len": L, "head_dim": D,
                        "sharding": "one config-shaped batch per GPU, (batch, head) pairs independent, no collective",
                        "l2": "inputs larger than L2 (Q, K, V, dO are %d MB each)" % (B * H * L * D * 2 // 2 ** 20),
-                       "backward": "fused (dQ accumulated in fp32 with atomics)" if D == 64 else "two kernels (dQ, dK/dV)",
+                       "backward": "fused (dQ accumulated in fp32 with atomics)",
                        "nonempty_tile_fraction": frac, "full_tiles": stats[0], "partial_tiles": stats[1]},
             "per_gpu_tflops": per_gpu,
             "pct_of_bf16_peak": {"burst": 100 * per_gpu / peak_tf, "sustained": 100 * per_gpu / peak_sus, "peaks": peak_kind},

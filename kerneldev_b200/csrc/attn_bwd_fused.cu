@@ -55,8 +55,8 @@
 //
 // Measured against the two forms before it (us, delta and conversion kernels included): a fused kernel with a row per
 // thread, sixteen compute warps and heads per CTA (HD = 64) and the two-kernel form (HD = 128):
-//   bf16 B16 H16 T4096 D64 hierarchical 1291 -> 1175-1230    bf16 B8 H16 T2048 D64 causal 338 -> 298
-//   bf16 B8 H16 T2048 D128 causal 644 -> 441                 fp16 B4 H32 T8192 D128 hierarchical 3944 -> 2540
+//   bf16 B16 H16 T4096 D64 hierarchical 1291 -> 1175-1230    bf16 B8 H16 T2048 D64 causal 338 -> 284
+//   bf16 B8 H16 T2048 D128 causal 644 -> 415                 fp16 B4 H32 T8192 D128 hierarchical 3944 -> 2420
 #include <algorithm>
 #include <type_traits>
 

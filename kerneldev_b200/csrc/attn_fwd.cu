@@ -16,11 +16,16 @@
 // while a warp loads, masks and reduces its 128 columns only one other warp of its scheduler can compute exponentials. Two
 // warps to a row spend half as long outside the exponentials, at the price of one exchange of row maxima per unit.
 //
-// A "unit" is one (key tile, query tile) product that is not EMPTY. Units are numbered in list
-// order over all items; unit u computes its scores into TMEM buffer u % NBUF (128 fp32 columns), and P (64
-// columns of packed pairs) is written over the same buffer. S(u + NBUF) is issued directly after P(u) V, so a softmax warpgroup that finishes unit u finds the scores of its next unit already in
-// TMEM, and the tensor core works on other units while it computes. The tensor pipe executes
-// in issue order, which is what allows S(u + NBUF) to overwrite the buffer P(u) was read from.
+// A "unit" is one (key tile, query tile) product that is not EMPTY. Units are numbered in list order over all items; unit u
+// computes its scores into TMEM buffer u % NBUF (128 fp32 columns), and P (32 columns of packed pairs for each half of the
+// keys) is written over the same buffer. S(u + NBUF) is issued directly after P(u) V, so that a softmax warp that finishes
+// unit u finds the scores of its tile's next unit in TMEM (at D = 64, where there are three buffers) or under way (at
+// D = 128, where O takes the room of the third). The tensor pipe executes in issue order, which is what allows S(u + NBUF) to
+// overwrite the buffer P(u) was read from.
+// Measured, bf16: hierarchical masks 16 x 16 x 4096 x 64 483 us (560 with a group of heads per CTA, two issuing warps and
+// eight softmax warps), causal 8 x 16 x 2048 x 64 119 us (147), x 128 152 us (207): 1,800 cycles a tile at D = 64, 2,400 at 128.
+// At D = 128 the chain P -> P V -> S -> P of a tile is what is left: both tiles wait a quarter of their time for scores.
+// Tried and slower: a quarter of the exponentials as polynomials on the FMA pipe (5-9 %).
 // EMPTY tiles never appear in the list: they are neither loaded nor multiplied.
 //
 // Replaces _flash_attn_fwd (original_kernel.py:278-626): same math (scores scaled by
