@@ -462,6 +462,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// permute whose selector nibbles with the top bit set replicate a byte's sign over the byte
+__device__ __forceinline__ uint32_t prmt_sign(uint32_t v, uint32_t selector) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %1, %2;" : "=r"(d) : "r"(v), "r"(selector));
+  return d;
+}
 // two fp32 values in one 64-bit register and the packed arithmetic on them
 __device__ __forceinline__ uint64_t pack_u32x2(uint32_t lo, uint32_t hi) {
   uint64_t d;
