@@ -574,10 +574,22 @@ std::tuple<Tensor, Tensor, Tensor> metadata_from_tokens(const Tensor& tokens_, i
 
 // ---- cocktail-party head ---------------------------------------------------------------------------------------
 
+// the marker index of a batch as one int32 tensor: starts and ends (B,T each), their counts and the first [MASK] (B each)
+int64_t index_words(int64_t B, int64_t T) { return 2 * B * T + 3 * B; }
+void point_into_index(kd_cocktail& p, const Tensor& index) {
+  const int64_t rows = static_cast<int64_t>(p.B) * p.T;
+  const int32_t* words = index.data_ptr<int32_t>();
+  p.starts = words;
+  p.ends = words + rows;
+  p.n_starts = words + 2 * rows;
+  p.n_ends = p.n_starts + p.B;
+  p.first_mask = p.n_ends + p.B;
+}
+
 // gradient of cocktail_scores: one kernel that writes every row of grad_x
 struct CocktailBackward : torch::autograd::Node {
   torch::autograd::SavedVariable h, index;
-  kd_cocktail p;   // shapes, type and the index pointers (into `index`)
+  kd_cocktail p{};   // shapes and type; the pointers are those of the unpacked tensors, which need not be the saved ones
   Tensor like;     // an empty tensor with x's options
 
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
@@ -594,6 +606,9 @@ struct CocktailBackward : torch::autograd::Node {
     // without a span nothing reaches x, and there is no kernel to write the zeros
     Tensor gx = p.S == 0 ? at::zeros({p.B, p.T, p.C}, like.options()) : at::empty({p.B, p.T, p.C}, like.options());
     kd_cocktail q = p;
+    ti = ti.contiguous();
+    th = th.contiguous();
+    point_into_index(q, ti);
     q.scores = ds.data_ptr();
     q.h = th.data_ptr<float>();
     q.gx = gx.data_ptr();
@@ -626,14 +641,18 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor tokens = tokens_.stride(1) == 1 ? tokens_ : tokens_.contiguous();
     const Tensor x = x_.stride(2) == 1 ? x_ : x_.contiguous();
-    index = at::empty({2 * B * T + 3 * B}, tokens.options().dtype(at::kInt));
-    int32_t* words = index.data_ptr<int32_t>();
-    int32_t *starts = words, *ends = words + B * T, *n_starts = words + 2 * B * T, *n_ends = n_starts + B, *first_mask = n_ends + B;
+    index = at::empty({index_words(B, T)}, tokens.options().dtype(at::kInt));
+    p.B = static_cast<int32_t>(B);
+    p.T = static_cast<int32_t>(T);
+    p.C = static_cast<int32_t>(C);
+    p.dtype = t == at::kFloat ? KD_F32 : dtype_code(t);
+    point_into_index(p, index);
+    auto out = [](const int32_t* words) { return const_cast<int32_t*>(words); };
     Tensor counts = at::empty({B}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     c10::cuda::CUDAGuard guard(x.device());
     auto stream = at::cuda::getCurrentCUDAStream();
     check(lib.cocktail_index(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(T, 1), static_cast<int32_t>(B),
-                             static_cast<int32_t>(T), tok_span, tok_es, tok_mask, starts, ends, n_starts, n_ends, first_mask,
+                             static_cast<int32_t>(T), tok_span, tok_es, tok_mask, out(p.starts), out(p.ends), out(p.n_starts), out(p.n_ends), out(p.first_mask),
                              counts.data_ptr<int32_t>(), stream));
     int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
     if (B > 0 && T > 0) {
@@ -648,16 +667,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     p.x = x.data_ptr();
     p.x_sb = x.stride(0);
     p.x_st = x.stride(1);
-    p.B = static_cast<int32_t>(B);
-    p.T = static_cast<int32_t>(T);
-    p.C = static_cast<int32_t>(C);
     p.S = S;
-    p.dtype = t == at::kFloat ? KD_F32 : dtype_code(t);
-    p.starts = starts;
-    p.ends = ends;
-    p.n_starts = n_starts;
-    p.n_ends = n_ends;
-    p.first_mask = first_mask;
     p.scores = scores.data_ptr();
     p.h = track ? h.data_ptr<float>() : nullptr;
     check(lib.cocktail_scores(&p, stream));
@@ -665,8 +675,11 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
   if (track) {
     auto node = std::shared_ptr<CocktailBackward>(new CocktailBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x_));
-    node->p = p;
-    node->p.x = nullptr;
+    node->p.B = p.B;
+    node->p.T = p.T;
+    node->p.C = p.C;
+    node->p.S = p.S;
+    node->p.dtype = p.dtype;
     node->like = at::empty({0}, x_.options());
     torch::autograd::set_history(scores, node);
     node->h = torch::autograd::SavedVariable(h, false);
