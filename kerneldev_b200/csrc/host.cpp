@@ -138,6 +138,7 @@ struct Plan {
     meta.is_prefix = static_cast<const uint8_t*>(per_token(is_prefix, at::kBool, "is_prefix", &meta.is_prefix_stride_b));
     if (lens.has_value()) {
       KD_VALUE(lens->scalar_type() == at::kInt && lens->dim() == 1 && lens->size(0) == B, "lens must be an int32 tensor of shape (B,)");
+      KD_VALUE(lens->device() == device, "lens must live on ", device);
       keep.push_back(*lens);
       Tensor l = lens->contiguous();
       keep.push_back(l);

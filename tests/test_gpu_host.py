@@ -33,3 +33,11 @@ def test_cocktail_gradient_when_hooks_replace_the_saved_tensors():
     (got,) = torch.autograd.grad(scores, x, ds)
     del rubbish
     assert torch.equal(got, want)
+
+
+def test_lens_on_another_device_is_refused():
+    """The kernels read lens on the device: an address of host memory must not reach them."""
+    from kerneldev_b200 import flash_attention
+    q = torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="lens must live on"):
+        flash_attention(q, q, q, lens=torch.tensor([100], dtype=torch.int32))
