@@ -306,7 +306,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
         const size_t row = ((size_t)b * a.H + h) * a.T;
-        const bool aligned = (row & 3) == 0;
+        // the rows of four scalars that the lanes copy begin on 16 bytes (the arrays need no alignment beyond a float's)
+        const bool aligned = ((reinterpret_cast<uintptr_t>(a.lse + row) | reinterpret_cast<uintptr_t>(a.delta + row)) & 15u) == 0;
         uint32_t ent = static_cast<uint32_t>(it.z) >> 16;
         int4 nx = it;
 #pragma unroll 1

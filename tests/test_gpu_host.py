@@ -41,3 +41,27 @@ def test_lens_on_another_device_is_refused():
     q = torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16)
     with pytest.raises(ValueError, match="lens must live on"):
         flash_attention(q, q, q, lens=torch.tensor([100], dtype=torch.int32))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lse_off,delta_off", [(1, 0), (0, 2), (3, 1)])
+def test_fused_backward_with_scalars_off_16_bytes(D, lse_off, delta_off):
+    """LSE and delta need no alignment beyond a float's: their rows are copied 16 bytes at a time only where they begin on
+    16 bytes. Bit-equal dK and dV (fixed order of sums), dQ within the rounding of its unordered fp32 sums."""
+    from kerneldev_b200.original_kernel import _backward, _forward
+    from kerneldev_b200.plan import AttentionPlan
+    B, H, T = 2, 3, 388
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v, do = (torch.randn((B, H, T, D), generator=g, device=DEV).to(torch.bfloat16) for _ in range(4))
+    plan = AttentionPlan(B, T, DEV)
+    o, lse = _forward(q, k, v, plan, D ** -0.5)
+    want = _backward(q, k, v, o, lse, do, plan, D ** -0.5)
+    n = B * H * T
+    shifted = torch.empty(n + 4, device=DEV)[lse_off:lse_off + n].view(B, H, T).copy_(lse)
+    delta = torch.empty(n + 4, device=DEV)[delta_off:delta_off + n].view(B, H, T)
+    assert shifted.data_ptr() % 16 == 4 * lse_off and delta.data_ptr() % 16 == 4 * delta_off
+    bufs = [torch.empty_like(q), torch.empty_like(q), torch.empty_like(q), delta, torch.empty((B, H, T, 64 if D <= 64 else 128), device=DEV)]
+    got = _backward(q, k, v, o, shifted, do, plan, D ** -0.5, 0, bufs)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    # at most four key tiles add up in another order, then one rounding to bf16, whose neighbours differ by 2^-7 of the value at most
+    assert torch.allclose(got[0].float(), want[0].float(), rtol=2.0**-7, atol=1e-4)
