@@ -133,10 +133,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __shared__ AbortFlag abortf;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // With the delta kernel ahead the plan may be read before the wait, past L1: the start of a kernel that overlaps another
+  // need not have cleaned it, and a plan's memory may have held another one.
   if (!a.plan_ready) pdl_wait();
   const int h0 = blockIdx.x * a.G, b = blockIdx.y;
   const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
-  const int qt = a.order[((size_t)b * 3 + 1) * a.NT + blockIdx.z];   // longest lists first
+  const int qt = __ldcg(a.order + ((size_t)b * 3 + 1) * a.NT + blockIdx.z);   // longest lists first
   const int pair = qt >> 1, ip = qt & 1;
 
   if (tid == 0) {
@@ -164,12 +166,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   if (warp == 2) {
     // compact the pair's list down to the entries that are non-empty for this query tile
-    const int n = a.fwd_cnt[b * a.NP + pair];
+    const int n = __ldcg(a.fwd_cnt + b * a.NP + pair);
     const uint16_t* list = a.fwd_list + ((size_t)b * a.NP + pair) * a.NT;
     int na = 0;
     for (int base = 0; base < n; base += 32) {
       const int e = base + lane;
-      const uint32_t ent = e < n ? list[e] : 0u;
+      const uint32_t ent = e < n ? __ldcg(list + e) : 0u;
       const uint32_t cls = (ent >> (8 + 2 * ip)) & 3u;
       const uint32_t bal = __ballot_sync(0xffffffffu, cls != 0u);
       if (cls != 0u) sAct[na + __popc(bal & ((1u << lane) - 1u))] = static_cast<uint16_t>((ent & 0xFFu) | (cls << 8));
@@ -509,11 +511,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __shared__ AbortFlag abortf;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!a.plan_ready) pdl_wait();
+  if (!a.plan_ready) pdl_wait();   // reads ahead of the wait below go past L1, as in the dQ kernel
   const int h0 = blockIdx.x * a.G, b = blockIdx.y;
   const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
-  const int kt = a.order[((size_t)b * 3 + 2) * a.NT + blockIdx.z];   // longest lists first
-  const int n = a.bwd_cnt[b * a.NT + kt];
+  const int kt = __ldcg(a.order + ((size_t)b * 3 + 2) * a.NT + blockIdx.z);   // longest lists first
+  const int n = __ldcg(a.bwd_cnt + b * a.NT + kt);
 
   if (tid == 0) {
     abortf.v = 0;
@@ -540,7 +542,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   if (warp == 2) {
     const uint16_t* glist = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
-    for (int e = lane; e < n; e += 32) sList[e] = glist[e];
+    for (int e = lane; e < n; e += 32) sList[e] = __ldcg(glist + e);
   }
   tc_fence_before_sync();
   __syncthreads();

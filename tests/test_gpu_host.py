@@ -65,3 +65,33 @@ def test_fused_backward_with_scalars_off_16_bytes(D, lse_off, delta_off):
     assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
     # at most four key tiles add up in another order, then one rounding to bf16, whose neighbours differ by 2^-7 of the value at most
     assert torch.allclose(got[0].float(), want[0].float(), rtol=2.0**-7, atol=1e-4)
+
+
+def test_deterministic_backward_with_plans_at_reused_addresses(monkeypatch):
+    """Plans of very different masks one after the other in the same memory, without a synchronisation between: each launch
+    has to see the plan of its own call, whatever an SM may hold of the one before."""
+    from kerneldev_b200 import clear_plan_cache, flash_attention
+    monkeypatch.setenv("KD_CHECK_STATUS", "0")
+    B, H, T, D = 2, 4, 1024, 64
+    g = torch.Generator(device=DEV).manual_seed(5)
+    q, k, v, do = (torch.randn((B, H, T, D), generator=g, device=DEV).to(torch.bfloat16) for _ in range(4))
+    for x in (q, k, v):
+        x.requires_grad_()
+    spans = torch.zeros((B, T), dtype=torch.bool, device=DEV)
+    spans[:, 300:900] = True
+    ids = (torch.arange(T, device=DEV) // 96 + 1).expand(B, T) * spans
+    masks = [dict(causal=True), dict(causal=False), dict(in_span=spans, span_id=ids), dict(lens=torch.tensor([130, T], dtype=torch.int32, device=DEV))]
+
+    def run(m):
+        clear_plan_cache()   # the plan of the call before goes back to the allocator
+        o = flash_attention(q, k, v, deterministic=True, **m)
+        return torch.autograd.grad(o, (q, k, v), do)
+
+    want = []
+    for m in masks:
+        want.append(run(m))
+        torch.cuda.synchronize()
+    order = np.random.default_rng(0).integers(0, len(masks), 60)
+    got = [run(masks[i]) for i in order]
+    for i, grads in zip(order, got):
+        assert all(torch.equal(a, b) for a, b in zip(grads, want[i]))
