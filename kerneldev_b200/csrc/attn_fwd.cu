@@ -40,6 +40,20 @@
 
 namespace kd {
 
+#ifdef KD_TEST_DROP_LOAD
+// Test build only: a caller's kernel that lets the next one start at once and goes on for `ns` nanoseconds.
+__global__ void test_busy_kernel(uint64_t ns) {
+  pdl_launch_dependents();
+  auto now = [] {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+  };
+  const uint64_t t0 = now();
+  for (uint32_t i = 0; i < (1u << 20) && now() - t0 < ns; ++i) __nanosleep(1000);
+}
+#endif
+
 struct FwdArgs {
   int B, H, T, NT, NP, Tpad;
   ItemOrder order_of;
@@ -347,6 +361,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (n_flight > 0 && !__all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) return STALLED;
           int4 it;
           if (!next_item(k, it)) return abortf->v == 0u ? ENDED : ABORTED;
+          // The waits for Q and K that follow are bounded, and the loads they wait for are issued behind the producer's wait for the
+          // kernel ahead: the limit must not run while that kernel does (a caller's may let this one start early and take long).
+          if (k == 0) pdl_wait();
           n = it.w & 0xFF;
           left = static_cast<uint32_t>(it.w) >> 8;
           ntile_q = (2 * it.z + 1 < a.NT) ? 2 : 1;
@@ -762,3 +779,10 @@ int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
 }
 
 }  // namespace kd
+
+#ifdef KD_TEST_DROP_LOAD
+extern "C" int kd_test_busy(uint64_t ns, void* stream) {
+  kd::test_busy_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(ns);
+  return static_cast<int>(cudaGetLastError());
+}
+#endif

@@ -68,3 +68,37 @@ def test_wait_timeout_unwinds_reports_and_recovers():
     env.pop("KD_CHECK_STATUS", None)     # the default, asynchronous reporting is what is under test
     r = subprocess.run([sys.executable, "-c", CHILD % {"root": ROOT}], env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "unwound and recovered" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+CHILD_EARLY_START = r"""
+import ctypes, os, sys
+sys.path.insert(0, %(root)r)
+import torch
+from kerneldev_b200 import _capi, flash_attention
+from kerneldev_b200 import plan as plan_module
+assert "waittest" in str(_capi.LIB_PATH)
+busy = _capi.load().kd_test_busy
+busy.argtypes = [ctypes.c_uint64, ctypes.c_void_p]
+dev = torch.device("cuda:0")
+for D in (64, 128):
+    q, k, v = (torch.randn((1, 4, 384, D), device=dev).to(torch.bfloat16) for _ in range(3))
+    want = [flash_attention(q, k, v, causal=True) for _ in range(2)][1]   # the stream has used the plan: the next launch looks it up early
+    torch.cuda.synchronize()
+    assert busy(100_000_000, torch.cuda.current_stream().cuda_stream) == 0
+    got = flash_attention(q, k, v, causal=True)
+    torch.cuda.synchronize()
+    assert all(p.status() == 0 for p in plan_module._CACHE.values())
+    assert torch.equal(got, want)
+print("no time-out")
+"""
+
+
+def test_waits_do_not_run_while_the_kernel_ahead_does():
+    """A kernel of the caller's that lets its successor start at once and goes on for 100 ms, five times the wait limit of the
+    test build: the forward's CTAs are resident all that time and must not count it against their waits."""
+    from kerneldev_b200.build import build
+    lib = build(name="waittest", extra_flags=WAITTEST_FLAGS)
+    env = dict(os.environ, KD_LIB_PATH=str(lib))
+    env.pop("KD_CHECK_STATUS", None)
+    r = subprocess.run([sys.executable, "-c", CHILD_EARLY_START % {"root": ROOT}], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and "no time-out" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
