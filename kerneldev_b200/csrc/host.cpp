@@ -11,6 +11,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
@@ -63,9 +64,10 @@ void bind(const py::dict& a) {
   take(lib.last_error, a, "kd_last_error");
 }
 
-// an entry point rejected its arguments or a CUDA call failed (raised in Python as _capi.KdError)
-struct LibraryError : std::runtime_error {
-  using std::runtime_error::runtime_error;
+// an entry point rejected its arguments or a CUDA call failed: _capi.KdError in Python, from the autograd engine's threads too
+struct LibraryError : torch::PyTorchError {
+  using torch::PyTorchError::PyTorchError;
+  PyObject* python_type() override { return py::module_::import("kerneldev_b200._capi").attr("KdError").ptr(); }
 };
 
 void check(int rc) {
@@ -693,15 +695,14 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "host path of the attention operator";
-  py::register_exception_translator([](std::exception_ptr p) {
+  // torch's own translation (out of memory, Python errors raised in hooks, LibraryError), for this module's functions alone
+  py::register_local_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
-    } catch (const LibraryError& e) {
-      PyErr_SetString(py::module_::import("kerneldev_b200._capi").attr("KdError").ptr(), e.what());
-    } catch (const c10::ValueError& e) {
-      PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
-    } catch (const c10::Error& e) {
-      PyErr_SetString(PyExc_RuntimeError, e.what_without_backtrace());
+    } catch (const py::builtin_exception&) {
+      throw;
+    } catch (const std::exception&) {
+      torch::translate_exception_to_python(std::current_exception());
     }
   });
   py::class_<Plan, PlanPtr>(m, "Plan")

@@ -95,3 +95,57 @@ def test_deterministic_backward_with_plans_at_reused_addresses(monkeypatch):
     got = [run(masks[i]) for i in order]
     for i, grads in zip(order, got):
         assert all(torch.equal(a, b) for a, b in zip(grads, want[i]))
+
+
+def _out_of_memory(call):
+    """call() with the allocator limited to what it holds."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 2**23) / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_out_of_memory_keeps_its_type():
+    from kerneldev_b200 import cocktail_scores, flash_attention
+    q = torch.zeros((4, 16, 2048, 64), device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    _out_of_memory(lambda: flash_attention(q, q, q))
+    o = flash_attention(q, q, q)
+    _out_of_memory(lambda: torch.autograd.grad(o, q, torch.zeros_like(o)))
+    x = torch.zeros((8, 4096, 512), device=DEV, requires_grad=True)
+    tokens = torch.full((8, 4096), 3, dtype=torch.int64, device=DEV)   # a row of spans: the saved means are as large as x
+    _out_of_memory(lambda: cocktail_scores(x, tokens))
+
+
+def test_library_errors_in_the_backward_keep_their_type():
+    """A hook that gives O back off a 16-byte boundary: kd_attn_bwd refuses it on the host."""
+    from kerneldev_b200 import _capi, flash_attention
+    q, k, v = (torch.randn((1, 2, 200, 64), device=DEV).to(torch.bfloat16).requires_grad_() for _ in range(3))
+    n = q.numel()
+
+    def unpack(t):
+        if t.dtype != torch.bfloat16:
+            return t
+        return torch.empty(n + 8, dtype=t.dtype, device=DEV)[4:4 + n].view(t.shape).copy_(t)
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach().clone(), unpack):
+        o = flash_attention(q, k, v)
+    with pytest.raises(_capi.KdError, match="multiples of 16"):
+        torch.autograd.grad(o, (q, k, v), torch.ones_like(o))
+
+
+def test_errors_of_saved_tensor_hooks_come_through():
+    from kerneldev_b200 import flash_attention
+
+    class Stop(Exception):
+        pass
+
+    def pack(t):
+        raise Stop
+
+    q = torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    with pytest.raises(Stop), torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        flash_attention(q, q, q)
