@@ -12,6 +12,7 @@
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/FunctionsManual.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
 
@@ -503,6 +504,12 @@ struct AttentionBackward : torch::autograd::Node {
   std::string name() const override { return "FlashAttentionBackward"; }
 };
 
+// The nodes of this file have no formula for tangents: without this check they would be lost without a word.
+void refuse_forward_ad(const char* name, std::initializer_list<Tensor> inputs) {
+  for (const Tensor& t : inputs)
+    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(t), name, " does not support forward mode AD");
+}
+
 void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v) {
   KD_VALUE(q.dim() == 4, "q, k, v must be (batch, heads, time, head_dim)");
   KD_VALUE(q.sizes() == k.sizes() && q.sizes() == v.sizes(), "q, k, v must have the same shape, got ", q.sizes(), ", ", k.sizes(), ", ", v.sizes());
@@ -518,6 +525,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
                                      bool causal, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix, bool rules,
                                      const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta, bool return_lse) {
   check_inputs(q, k, v);
+  refuse_forward_ad("flash_attention", {q, k, v});
   const double scale = sm_scale.has_value() ? *sm_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
   KD_VALUE(scale > 0.0 && std::isfinite(scale), "sm_scale must be positive and finite");
   PlanPtr plan = get_plan(q.size(0), q.size(2), q.device(), in_span, span_id, is_prefix, lens, causal, rules);
@@ -636,6 +644,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
   TORCH_CHECK(x_.is_cuda(), "span_means runs on CUDA devices only; there is no CPU path");
   KD_VALUE(x_.size(0) == tokens_.size(0) && x_.size(1) == tokens_.size(1) && x_.device() == tokens_.device(),
            "x_embed and tokens must have the same batch, time and device");
+  refuse_forward_ad("cocktail_scores", {x_});
   const int64_t B = x_.size(0), T = x_.size(1), C = x_.size(2);
   const bool track = at::GradMode::is_enabled() && x_.requires_grad();
   Tensor scores, h, index;

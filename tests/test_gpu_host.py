@@ -149,3 +149,18 @@ def test_errors_of_saved_tensor_hooks_come_through():
     q = torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16, requires_grad=True)
     with pytest.raises(Stop), torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
         flash_attention(q, q, q)
+
+
+@pytest.mark.parametrize("arg", [0, 1, 2])
+def test_forward_mode_ad_is_refused(arg):
+    """There is no formula for tangents; a result without one would read as a derivative of zero."""
+    import torch.autograd.forward_ad as fwd
+    from kerneldev_b200 import cocktail_scores, flash_attention
+    qkv = [torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16) for _ in range(3)]
+    x = torch.zeros((1, 64, 16), device=DEV)
+    with fwd.dual_level():
+        qkv[arg] = fwd.make_dual(qkv[arg], torch.ones_like(qkv[arg]))
+        with pytest.raises(NotImplementedError, match="forward mode AD"):
+            flash_attention(*qkv)
+        with pytest.raises(NotImplementedError, match="forward mode AD"):
+            cocktail_scores(fwd.make_dual(x, torch.ones_like(x)), _span_tokens(1, 64))
