@@ -10,11 +10,13 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/FunctionsManual.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 #include <list>
@@ -504,6 +506,13 @@ struct AttentionBackward : torch::autograd::Node {
   std::string name() const override { return "FlashAttentionBackward"; }
 };
 
+// A trace would hold the allocation of the results and not the kernels that fill them.
+void refuse_tracing(const char* name) {
+  using c10::impl::TorchDispatchModeTLS;
+  TORCH_CHECK(!torch::jit::tracer::isTracing() && !TorchDispatchModeTLS::get_mode(c10::impl::TorchDispatchModeKey::PROXY).has_value(), name,
+              " cannot be traced: its kernels are not recorded");
+}
+
 // The nodes of this file have no formula for tangents: without this check they would be lost without a word.
 void refuse_forward_ad(const char* name, std::initializer_list<Tensor> inputs) {
   for (const Tensor& t : inputs)
@@ -526,6 +535,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
                                      const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta, bool return_lse) {
   check_inputs(q, k, v);
   refuse_forward_ad("flash_attention", {q, k, v});
+  refuse_tracing("flash_attention");
   const double scale = sm_scale.has_value() ? *sm_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
   KD_VALUE(scale > 0.0 && std::isfinite(scale), "sm_scale must be positive and finite");
   PlanPtr plan = get_plan(q.size(0), q.size(2), q.device(), in_span, span_id, is_prefix, lens, causal, rules);
@@ -645,6 +655,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
   KD_VALUE(x_.size(0) == tokens_.size(0) && x_.size(1) == tokens_.size(1) && x_.device() == tokens_.device(),
            "x_embed and tokens must have the same batch, time and device");
   refuse_forward_ad("cocktail_scores", {x_});
+  refuse_tracing("cocktail_scores");
   const int64_t B = x_.size(0), T = x_.size(1), C = x_.size(2);
   const bool track = at::GradMode::is_enabled() && x_.requires_grad();
   Tensor scores, h, index;

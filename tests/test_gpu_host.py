@@ -164,3 +164,16 @@ def test_forward_mode_ad_is_refused(arg):
             flash_attention(*qkv)
         with pytest.raises(NotImplementedError, match="forward mode AD"):
             cocktail_scores(fwd.make_dual(x, torch.ones_like(x)), _span_tokens(1, 64))
+
+
+def test_tracing_is_refused():
+    """A trace would hold the allocation of the results without the kernels that fill them."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from kerneldev_b200 import cocktail_scores, flash_attention
+    q = torch.zeros((1, 1, 128, 64), device=DEV, dtype=torch.bfloat16)
+    x, tokens = torch.zeros((1, 64, 16), device=DEV), _span_tokens(1, 64)
+    for trace in (lambda f, a: make_fx(f)(a), torch.jit.trace):
+        with pytest.raises(RuntimeError, match="cannot be traced"):
+            trace(lambda a: flash_attention(a, a, a), q)
+        with pytest.raises(RuntimeError, match="cannot be traced"):
+            trace(lambda a: cocktail_scores(a, tokens), x)
