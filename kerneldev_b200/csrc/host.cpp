@@ -465,7 +465,6 @@ struct AttentionBackward : torch::autograd::Node {
 
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     torch::autograd::variable_list out(3);
-    if (!grads[0].defined()) return out;
     Tensor tq, tk, tv, to, tlse;
     {
       std::lock_guard<std::mutex> lock(mutex_);
@@ -476,7 +475,8 @@ struct AttentionBackward : torch::autograd::Node {
       tlse = lse.unpack();
     }
     at::NoGradGuard no_grad;
-    const Tensor d_o = widen ? cast({grads[0]}, at::kHalf)[0] : grads[0];
+    // a gradient that a later node left undefined counts as zeros, as for autograd.Function
+    const Tensor d_o = !grads[0].defined() ? at::zeros_like(to) : widen ? cast({grads[0]}, at::kHalf)[0] : grads[0];
     auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
                                  opt.heads_per_cta);
     if (signs.has_value()) {
@@ -615,7 +615,6 @@ struct CocktailBackward : torch::autograd::Node {
 
   torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
     torch::autograd::variable_list out(1);
-    if (!grads[0].defined()) return out;
     Tensor th, ti;
     {
       std::lock_guard<std::mutex> lock(mutex_);
@@ -623,7 +622,7 @@ struct CocktailBackward : torch::autograd::Node {
       ti = index.unpack();
     }
     at::NoGradGuard no_grad;
-    const Tensor ds = grads[0].contiguous();
+    const Tensor ds = grads[0].defined() ? grads[0].contiguous() : at::zeros({p.B, p.S}, like.options());
     // without a span nothing reaches x, and there is no kernel to write the zeros
     Tensor gx = p.S == 0 ? at::zeros({p.B, p.T, p.C}, like.options()) : at::empty({p.B, p.T, p.C}, like.options());
     kd_cocktail q = p;

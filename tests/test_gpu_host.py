@@ -177,3 +177,23 @@ def test_tracing_is_refused():
             trace(lambda a: flash_attention(a, a, a), q)
         with pytest.raises(RuntimeError, match="cannot be traced"):
             trace(lambda a: cocktail_scores(a, tokens), x)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_undefined_gradients_count_as_zeros(dtype):
+    from kerneldev_b200 import cocktail_scores, flash_attention
+
+    class NoGradient(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    q, k, v = (torch.randn((1, 2, 150, 64), device=DEV).to(dtype).requires_grad_() for _ in range(3))
+    x = torch.randn((1, 64, 16), device=DEV).to(dtype).requires_grad_()
+    o, s = NoGradient.apply(flash_attention(q, k, v)), NoGradient.apply(cocktail_scores(x, _span_tokens(1, 64)))
+    for g, t in zip(torch.autograd.grad(o.sum() + s.sum(), (q, k, v, x)), (q, k, v, x)):
+        assert g.shape == t.shape and g.dtype == dtype and not g.any()
