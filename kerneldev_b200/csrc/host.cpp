@@ -678,10 +678,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
                              counts.data_ptr<int32_t>(), stream));
     int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
     if (B > 0 && T > 0) {
-      {
-        py::gil_scoped_release release;
-        C10_CUDA_CHECK(cudaStreamSynchronize(stream));
-      }
+      C10_CUDA_CHECK(cudaStreamSynchronize(stream));
       for (int64_t b = 0; b < B; ++b) S = std::max(S, counts.data_ptr<int32_t>()[b]);
     }
     scores = C == 0 ? at::zeros({B, S}, x.options()) : at::empty({B, S}, x.options());
@@ -724,30 +721,33 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       torch::translate_exception_to_python(std::current_exception());
     }
   });
+  // Everything that allocates, launches or waits runs without the interpreter lock: a launch waits while the stream's queue is
+  // full, and other threads go on meanwhile.
+  using NoGil = py::call_guard<py::gil_scoped_release>;
   py::class_<Plan, PlanPtr>(m, "Plan")
-      .def(py::init<int64_t, int64_t, at::Device, const OptTensor&, const OptTensor&, const OptTensor&, const OptTensor&, bool, bool>())
+      .def(py::init<int64_t, int64_t, at::Device, const OptTensor&, const OptTensor&, const OptTensor&, const OptTensor&, bool, bool>(), NoGil())
       .def_readonly("B", &Plan::B)
       .def_readonly("T", &Plan::T)
       .def_readonly("device", &Plan::device)
       .def_readonly("buf", &Plan::buf)
       .def_property_readonly("status_dev", &Plan::status_dev)
       .def_property_readonly("status_host", &Plan::status_host)
-      .def("use_on_current_stream", &Plan::use_on_current_stream);
+      .def("use_on_current_stream", &Plan::use_on_current_stream, NoGil());
   m.def("bind", &bind);
-  m.def("get_plan", &get_plan);
+  m.def("get_plan", &get_plan, NoGil());
   m.def("cached_plans", [] { return cache().values(); });
   m.def("clear_plans", [] { cache().clear(); });
   m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const PlanPtr& plan, double sm_scale, bool like_input, int heads_per_cta) {
     return forward(q, k, v, plan, sm_scale, like_input, heads_per_cta);
-  });
+  }, NoGil());
   m.def("backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, const PlanPtr& plan,
                        double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic, int heads_per_cta) {
     Tensor b[5];
     for (size_t i = 0; i < bufs.size() && i < 5; ++i) b[i] = bufs[i];
     return backward(q, k, v, o, lse, d_o, plan, sm_scale, phases, b[0], b[1], b[2], b[3], b[4], like_input, deterministic, heads_per_cta);
-  });
-  m.def("hadamard", &hadamard);
-  m.def("attention", &attention);
-  m.def("metadata_from_tokens", &metadata_from_tokens);
-  m.def("cocktail_scores", &cocktail_scores);
+  }, NoGil());
+  m.def("hadamard", &hadamard, NoGil());
+  m.def("attention", &attention, NoGil());
+  m.def("metadata_from_tokens", &metadata_from_tokens, NoGil());
+  m.def("cocktail_scores", &cocktail_scores, NoGil());
 }

@@ -197,3 +197,29 @@ def test_undefined_gradients_count_as_zeros(dtype):
     o, s = NoGradient.apply(flash_attention(q, k, v)), NoGradient.apply(cocktail_scores(x, _span_tokens(1, 64)))
     for g, t in zip(torch.autograd.grad(o.sum() + s.sum(), (q, k, v, x)), (q, k, v, x)):
         assert g.shape == t.shape and g.dtype == dtype and not g.any()
+
+
+def test_other_threads_run_while_the_host_waits(monkeypatch):
+    """KD_CHECK_STATUS=1 waits for the device in every call: here behind a busy stream."""
+    import threading
+    import time
+    from kerneldev_b200 import flash_attention
+    monkeypatch.setenv("KD_CHECK_STATUS", "1")
+    q = torch.zeros((1, 2, 128, 64), device=DEV, dtype=torch.bfloat16)
+    flash_attention(q, q, q)
+    steps, stop = [0], threading.Event()
+
+    def work():
+        while not stop.is_set():
+            steps[0] += 1
+            time.sleep(0.001)
+
+    worker = threading.Thread(target=work)
+    worker.start()
+    torch.cuda._sleep(500_000_000)   # a quarter of a second or more
+    before, t0 = steps[0], time.perf_counter()
+    flash_attention(q, q, q)
+    waited, done = time.perf_counter() - t0, steps[0] - before
+    stop.set()
+    worker.join()
+    assert waited > 0.1 and done > 20
