@@ -19,6 +19,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
+#include <deque>
 #include <list>
 #include <mutex>
 #include <unordered_map>
@@ -83,19 +84,35 @@ void check(int rc) {
 
 constexpr uint32_t kStatusTimeout = KD_STATUS_TIMEOUT, kStatusSpanRange = KD_STATUS_SPAN_RANGE;
 
-// Status mirrors of the plans: one pinned block handed out in rotation (pinning is a slow, device-wide call).
-// 1024 words: a collision would need more than 1024 live plans and could only make a reported failure show up on
-// two of them.
-std::pair<Tensor, int> pinned_word() {   // the block and the word's index in it
-  static std::mutex m;
-  static Tensor block;
-  static int next = 0;
-  std::lock_guard<std::mutex> lock(m);
-  if (!block.defined()) block = at::zeros({1024}, at::TensorOptions().dtype(at::kInt)).pin_memory();
-  const int word = next;
-  next = (next + 1) % 1024;
-  block.data_ptr<int32_t>()[word] = 0;
-  return {block, word};
+// Status mirrors of the plans: words of pinned blocks of 1024 (pinning is a slow, device-wide call). A word belongs to one plan
+// as long as that lives. Words that come back go to the end of the queue: a kernel of a plan that is gone may still report.
+class StatusWords {
+ public:
+  using Word = std::pair<Tensor, int>;   // the block and the word's index in it
+  Word take() {
+    std::lock_guard<std::mutex> lock(m_);
+    if (free_.empty()) {
+      const Tensor block = at::zeros({kBlock}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+      for (int i = 0; i < kBlock; ++i) free_.emplace_back(block, i);
+    }
+    Word w = std::move(free_.front());
+    free_.pop_front();
+    w.first.data_ptr<int32_t>()[w.second] = 0;
+    return w;
+  }
+  void give_back(Word w) {
+    std::lock_guard<std::mutex> lock(m_);
+    free_.push_back(std::move(w));
+  }
+
+ private:
+  static constexpr int kBlock = 1024;
+  std::mutex m_;
+  std::deque<Word> free_;
+};
+StatusWords& status_words() {
+  static StatusWords* w = new StatusWords;   // never destroyed: plans outlive the statics of this file
+  return *w;
 }
 
 bool check_every_launch() {
@@ -108,11 +125,14 @@ struct Plan {
   at::Device device;
   kd_plan_layout layout;
   Tensor buf;
-  std::pair<Tensor, int> mirror;   // the status word's copy in host memory
+  struct Mirror {                  // the status word's copy in host memory
+    StatusWords::Word word = status_words().take();
+    ~Mirror() { status_words().give_back(std::move(word)); }
+  } mirror;
   volatile uint32_t* host_word;
   // the status word and its mirror as tensors: views cost more than a launch, and only reports and tests want them
   Tensor status_dev() const { return buf.narrow(0, static_cast<int64_t>(layout.off_status), 4).view(at::kInt); }
-  Tensor status_host() const { return mirror.first.narrow(0, mirror.second, 1); }
+  Tensor status_host() const { return mirror.word.first.narrow(0, mirror.word.second, 1); }
   std::vector<Tensor> keep;   // the caller's metadata and its converted copies, alive as long as the plan is cached
   at::cuda::CUDAStream built_on;
   at::cuda::CUDAEvent built;
@@ -151,8 +171,7 @@ struct Plan {
     }
     meta.causal = causal;
     meta.rules = rules;
-    mirror = pinned_word();
-    host_word = reinterpret_cast<volatile uint32_t*>(mirror.first.data_ptr<int32_t>() + mirror.second);
+    host_word = reinterpret_cast<volatile uint32_t*>(mirror.word.first.data_ptr<int32_t>() + mirror.word.second);
     meta.status_mirror = const_cast<uint32_t*>(host_word);
     c10::cuda::CUDAGuard guard(dev);
     check(lib.classify(&meta, buf.data_ptr(), built_on.stream()));

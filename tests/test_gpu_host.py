@@ -223,3 +223,17 @@ def test_other_threads_run_while_the_host_waits(monkeypatch):
     stop.set()
     worker.join()
     assert waited > 0.1 and done > 20
+
+
+def test_a_live_plan_keeps_its_status_word():
+    """A report that waits in a plan's host word survives any number of further plans, and no two live plans share one."""
+    from kerneldev_b200 import _capi
+    from kerneldev_b200.plan import AttentionPlan
+    plan = AttentionPlan(1, 128, DEV)
+    plan._status_host.fill_(_capi.KD_STATUS_TIMEOUT | 0x104)
+    for _ in range(1100):
+        AttentionPlan(1, 16, DEV)
+    with pytest.raises(RuntimeError, match="timed out"):
+        plan.poll()
+    live = [AttentionPlan(1, 16, DEV) for _ in range(1100)]
+    assert len({p._status_host.data_ptr() for p in live + [plan]}) == 1101
