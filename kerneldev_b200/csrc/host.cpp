@@ -670,7 +670,9 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
   const auto t = x_.scalar_type();
   KD_VALUE(x_.dim() == 3 && (t == at::kHalf || t == at::kBFloat16 || t == at::kFloat), "x_embed must be (batch, time, dim) in float16, bfloat16 or float32");
   TORCH_CHECK(x_.is_cuda(), "span_means runs on CUDA devices only; there is no CPU path");
-  KD_VALUE(x_.size(0) == tokens_.size(0) && x_.size(1) == tokens_.size(1) && x_.device() == tokens_.device(),
+  // one row may have more embeddings than tokens: the rest belongs to no span
+  KD_VALUE(x_.size(0) == tokens_.size(0) && (x_.size(1) == tokens_.size(1) || (x_.size(0) == 1 && x_.size(1) > tokens_.size(1))) &&
+               x_.device() == tokens_.device(),
            "x_embed and tokens must have the same batch, time and device");
   refuse_forward_ad("cocktail_scores", {x_});
   refuse_tracing("cocktail_scores");
@@ -692,11 +694,12 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     Tensor counts = at::empty({B}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     c10::cuda::CUDAGuard guard(x.device());
     auto stream = at::cuda::getCurrentCUDAStream();
-    check(lib.cocktail_index(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(T, 1), static_cast<int32_t>(B),
-                             static_cast<int32_t>(T), tok_span, tok_es, tok_mask, out(p.starts), out(p.ends), out(p.n_starts), out(p.n_ends), out(p.first_mask),
+    const int64_t n_tokens = tokens.size(1);
+    check(lib.cocktail_index(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(n_tokens, 1), static_cast<int32_t>(B),
+                             static_cast<int32_t>(n_tokens), tok_span, tok_es, tok_mask, out(p.starts), out(p.ends), out(p.n_starts), out(p.n_ends), out(p.first_mask),
                              counts.data_ptr<int32_t>(), stream));
     int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
-    if (B > 0 && T > 0) {
+    if (B > 0 && n_tokens > 0) {
       C10_CUDA_CHECK(cudaStreamSynchronize(stream));
       for (int64_t b = 0; b < B; ++b) S = std::max(S, counts.data_ptr<int32_t>()[b]);
     }

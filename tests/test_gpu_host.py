@@ -237,3 +237,19 @@ def test_a_live_plan_keeps_its_status_word():
         plan.poll()
     live = [AttentionPlan(1, 16, DEV) for _ in range(1100)]
     assert len({p._status_host.data_ptr() for p in live + [plan]}) == 1101
+
+
+def test_one_row_may_have_more_embeddings_than_tokens():
+    from kerneldev_b200 import cocktail_scores
+    T, more, C = 130, 37, 24
+    tokens = _span_tokens(1, T)
+    x = torch.randn((1, T + more, C), generator=torch.Generator(device=DEV).manual_seed(2), device=DEV)
+    a, b = x.clone().requires_grad_(), x[:, :T].clone().requires_grad_()
+    sa, sb = cocktail_scores(a, tokens), cocktail_scores(b, tokens)
+    assert sa.shape == (1, 2) and torch.equal(sa, sb)
+    (ga,), (gb,) = torch.autograd.grad(sa.sum(), a), torch.autograd.grad(sb.sum(), b)
+    assert torch.equal(ga[:, :T], gb) and not ga[:, T:].any()
+    with pytest.raises(ValueError):
+        cocktail_scores(x[:, :T - 1], tokens)
+    with pytest.raises(ValueError):
+        cocktail_scores(x.expand(2, -1, -1), tokens.expand(2, -1))
