@@ -206,6 +206,7 @@ cocktail_grad_kernel(const E* __restrict__ ds, const float* __restrict__ h, int 
   pdl_wait();
   pdl_launch_dependents();
   __shared__ float coef[CK_TOKENS];
+  __shared__ bool covered[CK_TOKENS];   // by a pair; a coefficient of zero does not say that (0 times an infinity is not 0)
   const int b = blockIdx.y, tb = blockIdx.x * CK_TOKENS, tid = threadIdx.x;
   const int n = min(min(n_starts[b], n_ends[b]), S), fm = first_mask[b];
   const int32_t *row_st = starts + (size_t)b * T, *row_en = ends + (size_t)b * T;
@@ -223,6 +224,7 @@ cocktail_grad_kernel(const E* __restrict__ ds, const float* __restrict__ h, int 
     float c = 0.f;
     for (int j = lo; j < lo2; ++j) c += to_f<E>(row_ds[j]) / static_cast<float>(row_en[j] - row_st[j] - 1);
     coef[tid] = c;
+    covered[tid] = lo < lo2;
   }
   const int groups = CK_THREADS / tpr, g = tid / tpr, cols = tpr * V, mine = (tid - g * tpr) * V;
   __syncthreads();
@@ -234,12 +236,17 @@ cocktail_grad_kernel(const E* __restrict__ ds, const float* __restrict__ h, int 
       const float w = coef[k];
       float f[V];
 #pragma unroll
-      for (int i = 0; i < V; ++i) f[i] = w != 0.f ? w * ctx[i] : 0.f;
+      for (int i = 0; i < V; ++i) f[i] = covered[k] ? w * ctx[i] : 0.f;
       if (tb + k == fm) {
         for (int j = 0; j < n; ++j) {
           const float d = to_f<E>(row_ds[j]);
 #pragma unroll
           for (int i = 0; i < V; ++i) f[i] = fmaf(d, hb[(size_t)j * C + c + i], f[i]);
+        }
+        for (int j = n; j < S; ++j) {   // the row's missing pairs, whose means are zero: what their gradients may add is a NaN
+          const float none = 0.f * to_f<E>(row_ds[j]);
+#pragma unroll
+          for (int i = 0; i < V; ++i) f[i] += none;
         }
       }
       Vec<E, V>::store(gx + ((size_t)b * T + tb + k) * C + c, f);

@@ -253,3 +253,22 @@ def test_one_row_may_have_more_embeddings_than_tokens():
         cocktail_scores(x[:, :T - 1], tokens)
     with pytest.raises(ValueError):
         cocktail_scores(x.expand(2, -1, -1), tokens.expand(2, -1))
+
+
+@pytest.mark.parametrize("C", [16, 17])
+def test_cocktail_gradient_of_infinities(C):
+    """0 times an infinity is not 0: in the tokens of a span whose gradient is zero, and from the padding of a row with
+    fewer spans than the widest into its [MASK] row."""
+    from kerneldev_b200 import cocktail_scores
+    tokens = _span_tokens(2, 64)
+    tokens[1, 32:50] = 50    # one span only
+    x = torch.randn((2, 64, C), generator=torch.Generator(device=DEV).manual_seed(4), device=DEV)
+    x[0, 2, 3] = float("inf")
+    x.requires_grad_()
+    ds = torch.tensor([[0.0, 0.0], [1.0, float("inf")]], device=DEV)
+    (g,) = torch.autograd.grad(cocktail_scores(x, tokens), x, ds)
+    nan = torch.zeros((2, 64, C), dtype=torch.bool)
+    nan[0, 6:9, 3] = nan[0, 33:49, 3] = True
+    nan[1, 2] = True
+    assert torch.equal(g.isnan().cpu(), nan)
+    assert torch.allclose(g[1, 7], x.detach()[1, 2] / 3, rtol=2.0**-22, atol=0) and not g[1, 33:50].any()
