@@ -626,6 +626,57 @@ void point_into_index(kd_cocktail& p, const Tensor& index) {
   p.first_mask = p.n_ends + p.B;
 }
 
+// Gradient of the gradient. With h(x) the means and the [MASK]'s embedding of x, which are linear in x, gx is linear in ds and in
+// h(x), and so is what comes back for a gradient v of gx: gx's own formula with h(v) for x, and for ds_j
+// <h_ctx(x), h_j(v)> + <h_ctx(v), h_j(x)>.
+struct CocktailDoubleBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable ds, h, index;
+  kd_cocktail p{};   // shapes and type
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    torch::autograd::variable_list out(2);
+    if (!grads[0].defined()) return out;
+    Tensor tds, th, ti;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);
+      tds = ds.unpack();
+      th = h.unpack();
+      ti = index.unpack();
+    }
+    at::NoGradGuard no_grad;
+    const Tensor v = grads[0].contiguous();
+    tds = tds.contiguous();
+    ti = ti.contiguous();
+    Tensor unused = at::empty_like(tds), hv = at::empty({p.B, p.S + 1, p.C}, v.options().dtype(at::kFloat)), gx = at::empty_like(v);
+    c10::cuda::CUDAGuard guard(v.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+    kd_cocktail q = p;
+    point_into_index(q, ti);
+    q.x = v.data_ptr();
+    q.x_sb = v.stride(0);
+    q.x_st = v.stride(1);
+    q.scores = unused.data_ptr();
+    q.h = hv.data_ptr<float>();
+    check(lib.cocktail_scores(&q, stream));
+    q.scores = tds.data_ptr();
+    q.gx = gx.data_ptr();
+    check(lib.cocktail_grad(&q, stream));
+    auto dots = [&](const Tensor& ctx, const Tensor& means) {   // (B,S)
+      return (ctx.narrow(1, p.S, 1) * means.narrow(1, 0, p.S)).sum(2);
+    };
+    out[0] = (dots(th, hv) + dots(hv, th)).to(tds.scalar_type());
+    out[1] = gx;
+    return out;
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    ds.reset_data();
+    h.reset_data();
+    index.reset_data();
+  }
+  std::string name() const override { return "CocktailScoresDoubleBackward"; }
+};
+
 // gradient of cocktail_scores: one kernel that writes every row of grad_x
 struct CocktailBackward : torch::autograd::Node {
   torch::autograd::SavedVariable h, index;
@@ -640,6 +691,7 @@ struct CocktailBackward : torch::autograd::Node {
       th = h.unpack();
       ti = index.unpack();
     }
+    const bool again = at::GradMode::is_enabled() && p.S > 0 && p.T > 0 && p.C > 0;   // create_graph: gx is differentiated in its turn
     at::NoGradGuard no_grad;
     const Tensor ds = grads[0].defined() ? grads[0].contiguous() : at::zeros({p.B, p.S}, like.options());
     // without a span nothing reaches x, and there is no kernel to write the zeros
@@ -653,6 +705,15 @@ struct CocktailBackward : torch::autograd::Node {
     q.gx = gx.data_ptr();
     c10::cuda::CUDAGuard guard(gx.device());
     check(lib.cocktail_grad(&q, at::cuda::getCurrentCUDAStream()));
+    if (again) {
+      auto node = std::shared_ptr<CocktailDoubleBackward>(new CocktailDoubleBackward(), torch::autograd::deleteNode);
+      node->set_next_edges({grads[0].defined() ? torch::autograd::impl::gradient_edge(grads[0]) : torch::autograd::Edge(), next_edge(0)});
+      node->p = p;
+      torch::autograd::set_history(gx, node);
+      node->ds = torch::autograd::SavedVariable(ds, false);
+      node->h = torch::autograd::SavedVariable(th, false);
+      node->index = torch::autograd::SavedVariable(ti, false);
+    }
     out[0] = gx;
     return out;
   }

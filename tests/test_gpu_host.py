@@ -272,3 +272,27 @@ def test_cocktail_gradient_of_infinities(C):
     nan[1, 2] = True
     assert torch.equal(g.isnan().cpu(), nan)
     assert torch.allclose(g[1, 7], x.detach()[1, 2] / 3, rtol=2.0**-22, atol=0) and not g[1, 33:50].any()
+
+
+@pytest.mark.parametrize("through_ds", [False, True])
+def test_second_derivatives_of_the_cocktail_scores(through_ds):
+    """A gradient penalty on the embeddings, against the oracle in 64 bits; with the scores' gradient a constant or itself a
+    function of the embeddings. Sums of at most T + C fp32 products in each of the four passes."""
+    from kerneldev_b200 import cocktail_scores
+    from oracle import attention_oracle as ao
+    B, T, C = 2, 70, 20
+    tokens = _span_tokens(B, T)
+    tokens[1, 5:10] = 50    # the second row has one span
+    x0 = torch.randn((B, T, C), generator=torch.Generator().manual_seed(6))
+    w0 = torch.randn((B, 2), generator=torch.Generator().manual_seed(7))
+
+    def penalty(scores, x, w):
+        (g,) = torch.autograd.grad((scores.tanh() if through_ds else scores).mul(w).sum(), x, create_graph=True)
+        return (g * g).sum() + (x * x).sum()
+
+    x = x0.to(DEV).requires_grad_()
+    (got,) = torch.autograd.grad(penalty(cocktail_scores(x, tokens), x, w0.to(DEV)), x)
+    y = x0.double().requires_grad_()
+    (want,) = torch.autograd.grad(penalty(ao.cocktail_scores(y, tokens.cpu())[0], y, w0.double()), y)
+    assert (want - 2 * y).abs().max() > 0.1
+    assert torch.allclose(got.double().cpu(), want, rtol=4 * (T + C) * 2.0**-24, atol=4 * (T + C) * 2.0**-24 * float(want.abs().max()))
