@@ -465,8 +465,8 @@ def test_backward_phases_and_delta_scratch(D):
 @pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.float16)])
 @pytest.mark.parametrize("G", [2, 3, 8])
 def test_head_groups_per_cta(monkeypatch, D, dtype, G):
-    """A CTA handles G heads one after the other (the work list is shared, the pipeline runs on across
-    heads). Small problems get G = 1 by themselves, so the group size is forced here: H = 5 is not a
+    """A CTA of the deterministic backward handles G heads one after the other (the work list is shared, the pipeline runs on
+    across heads). Small problems get G = 1 by themselves, so the group size is forced here: H = 5 is not a
     multiple of 2 or 3, a sequence is empty and one ends inside a tile."""
     from kerneldev_b200 import original_kernel
     monkeypatch.setattr(original_kernel, "HEADS_PER_CTA", G)
@@ -474,7 +474,7 @@ def test_head_groups_per_cta(monkeypatch, D, dtype, G):
     ins, sid, pre = random_meta(17 + G, B, T)
     lens = np.array([T, 0, T - 77], np.int32)
     q, k, v, do = rand_inputs(B, H, T, D, dtype, seed=40 + G)
-    got = run_op(q, k, v, do, ins, sid, pre, lens)
+    got = run_op(q, k, v, do, ins, sid, pre, lens, deterministic=True)
     compare(q, k, v, do, ao.dense_mask(T, ins, sid, pre, lens), got)
 
 
@@ -514,15 +514,14 @@ def test_max_sequence_length_sampled_rows(D, dtype):
     assert torch.allclose(k2.grad.float(), 2 * k.grad.float(), rtol=0, atol=2e-3)
 
 
+@pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("T,G", [(128, 0), (333, 0), (520, 3), (1100, 2)])
-def test_fused_backward_matches_oracle_and_split_backward(monkeypatch, dtype, T, G):
-    """Head dim 64 takes the fused backward by default (S and dP once per tile, dQ partials added to an fp32
-    scratch with atomics). Against the fp32 oracle at the stated tolerance; dK and dV also bit-equal across two
+@pytest.mark.parametrize("T", [128, 333, 520, 1100])
+def test_fused_backward_matches_oracle_and_split_backward(dtype, T, D):
+    """The fused backward is the default (S and dP once per tile, dQ partials added to an fp32
+    scratch in no fixed order). Against the fp32 oracle at the stated tolerance; dK and dV also bit-equal across two
     runs (their accumulation order is fixed), dQ within 1e-2 of the two-kernel backward's."""
-    from kerneldev_b200 import original_kernel
-    monkeypatch.setattr(original_kernel, "HEADS_PER_CTA", G)
-    B, H, D = 3, 5, 64
+    B, H = 3, 5
     ins, sid, pre = random_meta(90 + T, B, T)
     lens = np.array([T, 0, max(1, T - 77)], np.int32)
     q, k, v, do = rand_inputs(B, H, T, D, dtype, seed=T)
@@ -535,22 +534,23 @@ def test_fused_backward_matches_oracle_and_split_backward(monkeypatch, dtype, T,
     assert torch.allclose(got[2].float(), split[2].float(), atol=1e-2, rtol=1e-2)
 
 
-@pytest.mark.parametrize("T", [128, 300, 700])
-def test_fused_backward_many_heads_per_cta_short_lists(monkeypatch, T):
-    """A CTA of the fused backward hands its pipeline from head to head without draining it: K lives in two buffers
-    requested a head ahead, V is reloaded as soon as its last reader of a head is done, dK and dV leave through
-    other warps than the ones that go on computing. With one to six tiles per head and eight heads per CTA every
-    hand-over is two or three tiles after the one before, the case in which a barrier could be lapped or a buffer
-    refilled while still being read. Repeated runs must neither time out nor differ in dK and dV (whose
-    accumulation order is fixed), and must agree with the two-kernel backward."""
-    from kerneldev_b200 import original_kernel
-    monkeypatch.setattr(original_kernel, "HEADS_PER_CTA", 8)
-    B, H, D = 2, 16, 64
+# B * H * ceil(T / 128) items: five to ten for every SM, all of them with one to six tiles
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,T", [(12, 64, 128), (6, 64, 300), (4, 64, 700)])
+def test_fused_backward_hand_over_of_short_items(B, H, T, D):
+    """A CTA of the fused backward goes from item to item without draining its pipeline: K and V of the next one are requested
+    while the last products of this one run, dK and dV leave through other warps than the ones that go on computing. With
+    lists of one to six tiles every hand-over is a few tiles after the one before, the case in which a barrier could be
+    lapped or a buffer refilled while still being read. Repeated runs must neither time out nor differ in dK and dV (whose
+    accumulation order is fixed), and must agree with the two-kernel backward and, in sampled pairs, with the oracle."""
     ins, sid, pre = random_meta(7 + T, B, T)
-    lens = np.array([T, max(1, T - 40)], np.int32)
+    lens = np.array([T - 40 * (b % 2) for b in range(B)], np.int32)
     q, k, v, do = rand_inputs(B, H, T, D, torch.bfloat16, seed=3 * T)
     first = run_op(q, k, v, do, ins, sid, pre, lens)
-    compare(q, k, v, do, ao.dense_mask(T, ins, sid, pre, lens), first)
+    mask = ao.dense_mask(T, ins, sid, pre, lens)
+    for b, h in [(0, 0), (1, H - 1), (B // 2, H // 2), (B - 1, 1)]:
+        sl = lambda x: x[b:b + 1, h:h + 1]
+        compare(sl(q), sl(k), sl(v), sl(do), mask[b:b + 1], tuple(sl(x).contiguous() for x in first))
     split = run_op(q, k, v, do, ins, sid, pre, lens, deterministic=True)
     assert torch.allclose(first[2].float(), split[2].float(), atol=1e-2, rtol=1e-2)
     assert torch.allclose(first[3].float(), split[3].float(), atol=2e-2, rtol=1e-2)
@@ -579,7 +579,7 @@ def test_fused_backward_full_size_config2():
 def test_head_dims_below_the_tile_width(D, dtype, deterministic):
     """The reference takes head dims 16, 32, 64, 128 and 256 (original_kernel.py:1720). Dims that are not 64 or
     128 run on the next wider kernels with the missing tile columns zero-filled by TMA; outputs have the real
-    width. Both backward forms where they exist (fused for D <= 64)."""
+    width. Both backward forms."""
     B, H, T = 2, 3, 333
     ins, sid, pre = random_meta(D, B, T)
     lens = np.array([T, T - 50], np.int32)
