@@ -110,7 +110,8 @@ struct FusedCfg {
   static constexpr uint32_t P_STRIDE = (HD == 64) ? 32 : 64;   // packed columns between the two warpgroups' P^T
   static_assert(TM_DK + HD <= 512 && TM_DQ + HD <= 512 && TM_P + P_STRIDE + 32 <= 512, "TMEM budget");
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
-  // registers: 128 per thread at launch; light warps release down to 80, the dQ warps to 96, compute warps take 168
+  // registers: 128 per thread at launch; the light warps and the dQ warps release theirs down to REGS_LIGHT and REGS_DQ, the compute
+  // warps take REGS_COMPUTE
   static constexpr int REGS_LAUNCH = 128, REGS_LIGHT = (HD == 64) ? 88 : 72, REGS_DQ = (HD == 64) ? 56 : 120, REGS_COMPUTE = (HD == 64) ? 184 : 160;
   static_assert(4 * 32 * REGS_LIGHT + 4 * 32 * REGS_DQ + 8 * 32 * REGS_COMPUTE <= THREADS * REGS_LAUNCH, "register pool");
 };

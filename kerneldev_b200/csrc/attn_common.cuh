@@ -207,7 +207,8 @@ struct ItemOrder {
     rank = r / n;
     bh = (second ? big * (heads + 1) : 0) + c * n + (r - rank * n);
   }
-  // as many (batch, head) pairs to a chunk as take l2_bytes, and enough of them that it holds two items per SM
+  // As many (batch, head) pairs to a chunk as take l2_bytes, and enough of them that it holds two items per SM of 148. The number of
+  // chunks is rounded down, so that a chunk takes up to twice as much.
   static ItemOrder make(int pairs, int per_head, double pair_bytes, double l2_bytes) {
     long long chunk = static_cast<long long>(std::min<double>(pairs, std::max(1.0, l2_bytes / pair_bytes)));
     chunk = std::min<long long>(pairs, std::max<long long>(chunk, (296 + per_head - 1) / per_head));

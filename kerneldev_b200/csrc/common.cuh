@@ -50,9 +50,10 @@ inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
 }
 
 // Launches a kernel whose blocks may become resident while the kernel before it on the stream still runs (programmatic
-// stream serialisation). Every kernel of this library is launched like this and begins with pdl_wait(), which returns when
-// the kernels before it are complete and their writes visible: launch latency, barrier set-up and the TMEM allocation then
-// overlap the predecessor, which is what a chain of short kernels consists of.
+// stream serialisation). Every kernel of this library is launched like this and executes pdl_wait(), which returns when
+// the kernels before it are complete and their writes visible, before it reads or writes anything that they may write or read;
+// most begin with it. Launch latency, barrier set-up, the TMEM allocation and in some the look-up of the work then overlap the
+// predecessor, which is what a chain of short kernels consists of.
 template <typename... P, typename... A>
 inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
   cudaLaunchAttribute attr[1];

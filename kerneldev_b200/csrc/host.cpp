@@ -355,7 +355,7 @@ Tensor empty_out(const Tensor& like, bool like_input) {
 }
 
 kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Plan& plan,
-                      double sm_scale, int heads_per_cta) {
+                      double sm_scale) {
   kd_attn_params p{};
   p.B = static_cast<int32_t>(q.size(0));
   p.H = static_cast<int32_t>(q.size(1));
@@ -369,16 +369,15 @@ kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const T
   p.o = desc(o);
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
   p.plan = plan.buf.data_ptr();
-  p.heads_per_cta = heads_per_cta;
   return p;
 }
 
 std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const PlanPtr& plan, double sm_scale,
-                                   bool like_input, int heads_per_cta, bool want_lse = true) {
+                                   bool like_input, bool want_lse = true) {
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
   Tensor o = empty_out(q, like_input), lse;
   if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
-  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
+  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
@@ -405,7 +404,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   const bool fused = !deterministic;
   // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
   if (fused && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, f32);
-  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale, heads_per_cta);
+  kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
+  p.heads_per_cta = heads_per_cta;
   p.d_o = desc(d_o);
   p.dq = desc(dq);
   p.dk = desc(dk);
@@ -470,7 +470,7 @@ Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
 struct Options {
   double sm_scale;
   bool like_input, deterministic;
-  int heads_per_cta;
+  int heads_per_cta;   // of the deterministic backward
 };
 
 // dQ, dK, dV of one flash_attention call. Saves the operands the kernels read: for float32 tensors their float16
@@ -577,7 +577,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
       q2 = hadamard(q2, signs, false);
       k2 = hadamard(k2, signs, false);
     }
-    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, heads_per_cta, return_lse || track);
+    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, return_lse || track);
     o = f32 ? cast({o16}, at::kFloat)[0] : o16;
   }
   if (track) {
@@ -820,8 +820,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("get_plan", &get_plan, NoGil());
   m.def("cached_plans", [] { return cache().values(); });
   m.def("clear_plans", [] { cache().clear(); });
-  m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const PlanPtr& plan, double sm_scale, bool like_input, int heads_per_cta) {
-    return forward(q, k, v, plan, sm_scale, like_input, heads_per_cta);
+  m.def("forward", [](const Tensor& q, const Tensor& k, const Tensor& v, const PlanPtr& plan, double sm_scale, bool like_input) {
+    return forward(q, k, v, plan, sm_scale, like_input);
   }, NoGil());
   m.def("backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, const PlanPtr& plan,
                        double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic, int heads_per_cta) {

@@ -157,8 +157,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFl
   return true;
 }
 // Programmatic dependent launch. pdl_wait: returns when every kernel before this one on the stream has completed and its
-// writes are visible; before it, a kernel touches nothing but its arguments, shared memory and TMEM. pdl_launch_dependents:
-// the next kernel's blocks may be scheduled once every block of this one has called it (or exited).
+// writes are visible. Ahead of it a kernel touches its arguments, shared memory and TMEM, and, past L1, what was complete before
+// the kernel ahead let it start (see there: the plan, and the operands behind the delta kernel). pdl_launch_dependents: the next
+// kernel's blocks may be scheduled once every block of this one has called it (or exited).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -176,15 +177,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* tm,
       ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
-                                            int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(tm), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-
 // asynchronous 4- and 16-byte copies global -> shared, and this thread's arrival on an mbarrier when its copies so far
 // have landed (counted like any other arrival)
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
@@ -215,8 +207,6 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* tm, uint32_t src
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all of this thread's bulk groups have finished READING their shared-memory source
 __device__ __forceinline__ void bulk_wait_group_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... all but the most recent one
-__device__ __forceinline__ void bulk_wait_group_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // ... and have completed altogether
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 

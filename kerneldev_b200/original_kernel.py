@@ -32,8 +32,9 @@ __all__ = ["flash_attention", "generate_hadamard_signs", "hadamard_transform"]
 _HADAMARD_DIMS = (16, 32, 64, 128)
 _DTYPES = {torch.float16: _capi.KD_F16, torch.bfloat16: _capi.KD_BF16}
 
-# Heads a CTA handles one after the other (kd_attn_params.heads_per_cta): 0 lets the library choose from
-# the grid size. Small problems get 1 by themselves, so the tests of the multi-head path set this.
+# Heads a CTA of the deterministic backward handles one after the other (kd_attn_params.heads_per_cta): 0 lets the library
+# choose from the grid size. Small problems get 1 by themselves, so the tests of the multi-head path set this. The forward
+# and the fused backward take their work items one by one and have no use for it.
 HEADS_PER_CTA = 0
 
 
@@ -57,7 +58,7 @@ def _params(q, k, v, o, lse, plan, sm_scale):
 def _forward(q, k, v, plan: AttentionPlan, sm_scale: float, like_input: bool = False):
     """One kd_attn_fwd call: returns (O, LSE) for inputs flash_attention would accept. ``like_input``: O in the
     memory layout of q instead of contiguous."""
-    return _ext.forward(q, k, v, plan._core, sm_scale, like_input, HEADS_PER_CTA)
+    return _ext.forward(q, k, v, plan._core, sm_scale, like_input)
 
 
 def _backward(q, k, v, o, lse, d_o, plan: AttentionPlan, sm_scale: float, phases: int = 0, bufs=None,
