@@ -13,9 +13,9 @@ Differences from the reference, all deliberate:
     metadata is given (original_kernel.py:1202-1204, :1368-1371);
   * a query row that sees no key gets O = 0, LSE = -inf and no gradient (the reference's default
     path produces NaN there, original_kernel.py:554-561);
-  * CUDA sm_100 only, fp16 / bf16, head_dim a multiple of 16 up to 128 (the reference also takes 256 and
-    fp32 tensors). There is no Triton, no autotuning and no
-    CPU path: unsupported inputs raise.
+  * CUDA sm_100 only, fp16 / bf16 (fp32 tensors as fp16 operands), head_dim a multiple of 16 up to 128 (the reference also
+    takes 256). There is no Triton, no autotuning and no CPU path: unsupported inputs raise, as do forward-mode AD and
+    tracing.
 ``autotune``, ``prescale_qk`` and ``precision`` are accepted and ignored.
 """
 from __future__ import annotations
@@ -150,8 +150,9 @@ def flash_attention(
     of (B,T,H,D) memory (model.py:76-78) the ``transpose(1, 2).contiguous()`` after the call
     (model.py:95) and its counterpart in the backward then copy nothing. The drop-in module uses it.
     deterministic (extension, default False): True forces the two-kernel backward, whose results are
-    bit-identical from run to run; the default is the fused backward, which forms S and dP once per tile and
-    adds dQ partials in fp32 in no fixed order (dQ then varies in its last bits between runs).
+    bit-identical from run to run and which needs no scratch beyond 4 bytes a row; the default, at every head dim, is the
+    fused backward, which forms S and dP once per tile and adds dQ partials in fp32 in no fixed order (dQ then varies in its
+    last bits between runs) to a scratch of batch * heads * time rows of 64 floats (head_dim <= 64) or 128 (above).
 
     float32 q, k, v (the reference's default ``precision="tf32"`` path, original_kernel.py:2106): the tensors
     are rounded to float16 operands -- the 10-bit mantissa tf32 keeps -- the products accumulate in fp32 as
