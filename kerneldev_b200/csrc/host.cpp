@@ -8,15 +8,14 @@
 // another build of the library.
 #include <torch/extension.h>
 
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/FunctionsManual.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
-#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
 #include <deque>
@@ -528,14 +527,14 @@ struct AttentionBackward : torch::autograd::Node {
 // A trace would hold the allocation of the results and not the kernels that fill them.
 void refuse_tracing(const char* name) {
   using c10::impl::TorchDispatchModeTLS;
-  TORCH_CHECK(!torch::jit::tracer::isTracing() && !TorchDispatchModeTLS::get_mode(c10::impl::TorchDispatchModeKey::PROXY).has_value(), name,
-              " cannot be traced: its kernels are not recorded");
+  const bool recorded = TorchDispatchModeTLS::any_modes_set() && TorchDispatchModeTLS::get_mode(c10::impl::TorchDispatchModeKey::PROXY).has_value();
+  TORCH_CHECK(!at::tracer::impl::is_dispatch_enabled() && !recorded, name, " cannot be traced: its kernels are not recorded");
 }
 
 // The nodes of this file have no formula for tangents: without this check they would be lost without a word.
-void refuse_forward_ad(const char* name, std::initializer_list<Tensor> inputs) {
-  for (const Tensor& t : inputs)
-    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(t), name, " does not support forward mode AD");
+template <typename... T>
+void refuse_forward_ad(const char* name, const T&... inputs) {
+  TORCH_CHECK_NOT_IMPLEMENTED(!(inputs._fw_grad(/*level=*/0).defined() || ...), name, " does not support forward mode AD");
 }
 
 void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v) {
@@ -553,7 +552,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
                                      bool causal, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix, bool rules,
                                      const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta, bool return_lse) {
   check_inputs(q, k, v);
-  refuse_forward_ad("flash_attention", {q, k, v});
+  refuse_forward_ad("flash_attention", q, k, v);
   refuse_tracing("flash_attention");
   const double scale = sm_scale.has_value() ? *sm_scale : 1.0 / std::sqrt(static_cast<double>(q.size(3)));
   KD_VALUE(scale > 0.0 && std::isfinite(scale), "sm_scale must be positive and finite");
@@ -735,7 +734,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
   KD_VALUE(x_.size(0) == tokens_.size(0) && (x_.size(1) == tokens_.size(1) || (x_.size(0) == 1 && x_.size(1) > tokens_.size(1))) &&
                x_.device() == tokens_.device(),
            "x_embed and tokens must have the same batch, time and device");
-  refuse_forward_ad("cocktail_scores", {x_});
+  refuse_forward_ad("cocktail_scores", x_);
   refuse_tracing("cocktail_scores");
   const int64_t B = x_.size(0), T = x_.size(1), C = x_.size(2);
   const bool track = at::GradMode::is_enabled() && x_.requires_grad();
