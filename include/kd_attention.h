@@ -31,9 +31,11 @@
 extern "C" {
 #endif
 
+#define KD_INTERFACE_VERSION 2
+
 #define KD_F16 0
 #define KD_BF16 1
-#define KD_F32 2   /* kd_span_mean only */
+#define KD_F32 2   /* kd_span_mean and kd_cocktail only */
 
 #define KD_TILE 128 /* mask classification and kernel tile edge (tokens) */
 
@@ -110,7 +112,7 @@ typedef struct kd_attn_params {
   float* lse;        /* (B,H,T) contiguous, base-2 log-sum-exp (kd_attn_fwd: may be NULL, it is not written then): m + log2(l)
                         (original_kernel.py:603-604); forward output, backward input */
   float* delta;      /* (B,H,T) contiguous fp32 scratch of the backward: rowsum(O * dO)
-                        (kd_workspace_bytes gives its size) */
+                        (kd_workspace_bytes gives its size). lse and delta need the alignment of a float. */
   const void* plan;  /* filled by kd_classify for the same (B,T) */
   int32_t bwd_phases; /* kd_attn_bwd only. 0 or 3: all kernels; 1: the delta kernel and the dQ
                          kernel; 2: the dK/dV kernel alone (reads delta of an earlier pass 1).
@@ -250,6 +252,8 @@ int kd_cocktail_grad(const kd_cocktail* p, void* stream);
 /* Message for the last negative return value on this host thread. */
 const char* kd_last_error(void);
 
+/* KD_INTERFACE_VERSION of the library: it changes with the structures above, and a binding written for another one must not call
+ * the entry points that take them. 2: kd_meta.status_mirror and kd_attn_params.plan_ready. */
 int kd_version(void);
 
 #ifdef __cplusplus

@@ -11,6 +11,7 @@ from ctypes import (POINTER, Structure, c_char_p, c_float, c_int32, c_int64, c_s
                     c_void_p)
 from pathlib import Path
 
+KD_INTERFACE_VERSION = 2
 KD_F16, KD_BF16, KD_F32 = 0, 1, 2
 KD_TILE = 128
 KD_TILE_EMPTY, KD_TILE_FULL, KD_TILE_PARTIAL = 0, 1, 2
@@ -82,6 +83,9 @@ def load() -> ctypes.CDLL:
             "(needs nvcc; cross-compiles for sm_100a). This package has no other compute path.")
     lib = ctypes.CDLL(str(LIB_PATH))
     lib.kd_version.restype = c_int32
+    if lib.kd_version() != KD_INTERFACE_VERSION:
+        raise ImportError(f"{LIB_PATH} has interface version {lib.kd_version()}, this package needs {KD_INTERFACE_VERSION}: "
+                          "build it again with `python -m kerneldev_b200.build --force`")
     lib.kd_last_error.restype = c_char_p
     lib.kd_plan_layout_get.argtypes = [c_int32, c_int32, POINTER(KdPlanLayout)]
     lib.kd_classify.argtypes = [POINTER(KdMeta), c_void_p, c_void_p]

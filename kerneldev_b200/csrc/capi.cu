@@ -137,7 +137,7 @@ using namespace kd;
 
 extern "C" {
 
-int kd_version(void) { return 1; }
+int kd_version(void) { return KD_INTERFACE_VERSION; }
 
 const char* kd_last_error(void) { return g_last_error; }
 

@@ -166,3 +166,13 @@ def test_reference_model_binds_the_dropin_operator():
         "print('bound')\n")
     r = subprocess.run([os.sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "bound" in r.stdout, r.stdout + r.stderr
+
+
+def test_interface_version_changes_with_the_structures():
+    """kd_meta ends in status_mirror and kd_attn_params in plan_ready since version 2: a binding with the shorter structures
+    has to be able to tell, for the library reads what lies behind them."""
+    from kerneldev_b200 import _capi
+    header = open(os.path.join(ROOT, "include", "kd_attention.h")).read()
+    declared = int(re.search(r"#define KD_INTERFACE_VERSION (\d+)", header).group(1))
+    assert _capi.KdMeta._fields_[-1][0] == "status_mirror" and _capi.KdAttnParams._fields_[-1][0] == "plan_ready"
+    assert declared == _capi.KD_INTERFACE_VERSION == _capi.load().kd_version() == 2
