@@ -24,7 +24,8 @@
 // overwrite the buffer P(u) was read from.
 // Measured, bf16: hierarchical masks 16 x 16 x 4096 x 64 483 us (560 with a group of heads per CTA, two issuing warps and
 // eight softmax warps), causal 8 x 16 x 2048 x 64 119 us (147), x 128 152 us (207): 1,800 cycles a tile at D = 64, 2,400 at 128.
-// At D = 128 the chain P -> P V -> S -> P of a tile is what is left: both tiles wait a quarter of their time for scores.
+// At D = 128 the chain P -> P V -> S -> P of a tile is what is left: with long lists (hierarchical, 32 heads x 8192) the tensor
+// pipe is busy 54 % of the time and the special-function units 55 %.
 // Tried and slower: a quarter of the exponentials as polynomials on the FMA pipe (5-9 %).
 // EMPTY tiles never appear in the list: they are neither loaded nor multiplied.
 //
