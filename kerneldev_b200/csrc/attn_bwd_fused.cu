@@ -18,7 +18,7 @@
 //
 // What bounds it. No single unit. Per tile at HD = 64 (cycles of an SM): products 1,540, exponentials 1,024, shared
 // memory 2,450 of its 128 bytes a cycle (1,408 of them the products' operands), instruction issue 1,350 of each
-// scheduler; a tile takes 3,150 with full lists. Taking any one of these out of the kernel changes it by 3 to 8 %.
+// scheduler; a tile takes 3,000 with full lists. Taking any one of these out of the kernel changes it by 3 to 8 %.
 //  * Shared memory is kept free by the layout of the compute warps' registers: they read S^T and dP^T from TMEM in the
 //    16x256b shape, in which a thread owns four key rows and a quarter of the columns, as in an mma fragment, so that a
 //    warp needs LSE and delta of a column once and not 32 times; P^T goes back in the 16x128b shape and dS^T leaves
@@ -703,22 +703,30 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           const float* side = sSide + qs * C::SIDE_WORDS;
           bool out_ready = false;
           uint32_t pk_ds[2][16];
-          uint64_t lse[4], delta[4];
+          // 16 keys x 16 queries at a time, both halves of the keys for a group of queries. The next block is loaded while one is
+          // worked on: with two warps to a scheduler a TMEM load of some 150 cycles that is waited for at once is not covered. (Four
+          // blocks of 32 queries, each loaded and awaited: causal 8 x 16 x 1000 x 64 84.0 -> 80.7 us, 8 x 16 x 2048 241 -> 230.)
+          uint64_t lse[2], delta[2];
+          uint32_t sb[2][8], dpb[2][8];
+          auto load_block = [&](int c) {
+            tmem_ld16x256_x2(tS + (c & 1) * ROW16 + (c >> 1) * 16, sb[c & 1]);
+            tmem_ld16x256_x2(tDP + (c & 1) * ROW16 + (c >> 1) * 16, dpb[c & 1]);
+          };
+          auto load_scalars = [&](int g) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {   // 16 keys x 32 queries at a time
-            const int hf = c & 1, ch = c >> 1;
-            uint32_t s[16], dp[16];
-            tmem_ld16x256_x4(tS + hf * ROW16 + ch * 32, s);
-            tmem_ld16x256_x4(tDP + hf * ROW16 + ch * 32, dp);
-            if (hf == 0) {   // both halves of the keys see the same queries
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                lse[j] = ld_shared_pair(side + qcol + 32 * ch + 8 * j);
-                delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 32 * ch + 8 * j);
-              }
+            for (int j = 0; j < 2; ++j) {
+              lse[j] = ld_shared_pair(side + qcol + 16 * g + 8 * j);
+              delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 16 * g + 8 * j);
             }
+          };
+          load_block(0);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const int hf = c & 1, g = c >> 1;
+            if (hf == 0) load_scalars(g);
             tmem_wait_ld();
-            if (c == 3) {   // all loaded
+            if (c < 7) load_block(c + 1);
+            if (c == 7) {   // all loaded
               tc_fence_before_sync();
               __syncwarp();
               if (lane == 0) mbar_arrive(bar(C::B_SFREE + w));
@@ -727,15 +735,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1) && mbar_test_wait(bar(C::B_DSFREE), t & 1);
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 2; ++j) {
 #pragma unroll
               for (int r = 0; r < 2; ++r) {
-                uint32_t& p0 = p[hf][16 * ch + 4 * j + 2 * r];
-                uint32_t& p1 = p[hf][16 * ch + 4 * j + 2 * r + 1];
-                const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dp[4 * j + 2 * r], dp[4 * j + 2 * r + 1]));
+                uint32_t& p0 = p[hf][8 * g + 4 * j + 2 * r];
+                uint32_t& p1 = p[hf][8 * g + 4 * j + 2 * r + 1];
+                const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dpb[hf][4 * j + 2 * r], dpb[hf][4 * j + 2 * r + 1]));
                 const uint64_t x = mul_f32x2(pack_u32x2(p0, p1), d);
-                pk_ds[hf][8 * ch + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
-                const uint64_t y = fma_f32x2(pack_u32x2(s[4 * j + 2 * r], s[4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
+                pk_ds[hf][4 * g + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+                const uint64_t y = fma_f32x2(pack_u32x2(sb[hf][4 * j + 2 * r], sb[hf][4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
                 p0 = __float_as_uint(fast_exp2(-lo_f32x2(y)));
                 p1 = __float_as_uint(fast_exp2(-hi_f32x2(y)));
               }
@@ -809,13 +817,13 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
         uint32_t s[2][32];
         tmem_ld16x256_x8(tS, s[0]);
-        tmem_ld16x256_x8(tS + ROW16, s[1]);
         uint64_t col[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) col[j] = ld_shared_pair(side + qcol + 8 * j);   // LSE of this thread's columns
-        tmem_wait_ld();
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {   // 16 keys at a time
+          tmem_wait_ld();
+          if (hf == 0) tmem_ld16x256_x8(tS + ROW16, s[1]);   // under the first half's arithmetic
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
 #pragma unroll
@@ -841,19 +849,24 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // dP^T, and the products that read the previous tile's dS^T are done (long before, as a rule)
         if (!(ok = t == 0 ? wait(C::B_DPFULL, 0, W_U_DPFULL) : wait2(C::B_DPFULL, t & 1, W_U_DPFULL, C::B_DSFREE, (t - 1) & 1, W_U_DSFREE))) break;
         tc_fence_after_sync();
+        // 16 keys x 32 queries at a time; the next block is loaded while one is worked on (causal 1 x 16 x 16384 x 128, whole backward: 2750 -> 2640 us)
+        uint32_t dp[2][16];
+        tmem_ld16x256_x4(tDP, dp[0]);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-          uint32_t dp[32];
-          tmem_ld16x256_x8(tDP + hf * ROW16, dp);
-          tmem_wait_ld();
           uint32_t pk[16];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
+          for (int ch = 0; ch < 2; ++ch) {
+            tmem_wait_ld();
+            if (hf + ch < 2) tmem_ld16x256_x4(tDP + (ch == 0 ? hf : 1) * ROW16 + (ch == 0 ? 32 : 0), dp[ch ^ 1]);
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              const uint64_t d = fma_f32x2(col[j], minus1, pack_u32x2(dp[4 * j + 2 * r], dp[4 * j + 2 * r + 1]));
-              const uint64_t x = mul_f32x2(pack_u32x2(s[hf][4 * j + 2 * r], s[hf][4 * j + 2 * r + 1]), d);
-              pk[2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+            for (int j = 0; j < 4; ++j) {
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const uint64_t d = fma_f32x2(col[4 * ch + j], minus1, pack_u32x2(dp[ch][4 * j + 2 * r], dp[ch][4 * j + 2 * r + 1]));
+                const uint64_t x = mul_f32x2(pack_u32x2(s[hf][16 * ch + 4 * j + 2 * r], s[hf][16 * ch + 4 * j + 2 * r + 1]), d);
+                pk[8 * ch + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+              }
             }
           }
 #pragma unroll

@@ -424,6 +424,13 @@ __device__ __forceinline__ void tmem_ld16x256_x4(uint32_t taddr, uint32_t (&r)[1
       : "r"(taddr)
       : "memory");
 }
+// the same for 16 columns
+__device__ __forceinline__ void tmem_ld16x256_x2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // 16 lanes x 32 columns, the 16-bit counterpart: per 4 columns (8 packed pairs' halves), register 0 is column lane % 4 of row
 // lane / 4 and register 1 the same column of row lane / 4 + 8
 __device__ __forceinline__ void tmem_st16x128_x8(uint32_t taddr, const uint32_t (&r)[16]) {
