@@ -20,7 +20,7 @@ HOST_PATH = LIB_DIR / "kd_host.so"      # the host extension: links against libt
 HOST_SOURCE = CSRC / "host.cpp"
 INCLUDE_DIR = PKG_DIR.parent / "include"
 
-SOURCES = ["capi.cu", "plan.cu", "attn_fwd.cu", "attn_bwd.cu", "attn_bwd_fused.cu", "hadamard.cu", "metadata.cu", "cocktail.cu", "cast.cu"]
+SOURCES = ["capi.cu", "plan.cu", "attn_fwd.cu", "attn_fwd_wide.cu", "attn_bwd.cu", "attn_bwd_fused.cu", "hadamard.cu", "metadata.cu", "cocktail.cu", "cast.cu"]
 HEADERS = sorted(p.name for p in (Path(__file__).resolve().parent / "csrc").glob("*.cuh"))
 
 NVCC_FLAGS = [

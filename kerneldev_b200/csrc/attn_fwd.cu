@@ -1,4 +1,4 @@
-// Forward kernel: O = softmax(mask(Q K^T * scale)) V and base-2 LSE, for sm_100a.
+// Forward kernel for head dims up to 64, and the dispatch: O = softmax(mask(Q K^T * scale)) V and base-2 LSE, for sm_100a.
 //
 // A work item is a pair of 128-row query tiles of one (batch, head); it walks the plan's list of key tiles that are
 // non-empty for either of them. The grid has a CTA per item, but a running CTA takes further items by cancelling CTAs
@@ -19,14 +19,14 @@
 // A "unit" is one (key tile, query tile) product that is not EMPTY. Units are numbered in list order over all items; unit u
 // computes its scores into TMEM buffer u % NBUF (128 fp32 columns), and P (32 columns of packed pairs for each half of the
 // keys) is written over the same buffer. S(u + NBUF) is issued directly after P(u) V, so that a softmax warp that finishes
-// unit u finds the scores of its tile's next unit in TMEM (at D = 64, where there are three buffers) or under way (at
-// D = 128, where O takes the room of the third). The tensor pipe executes in issue order, which is what allows S(u + NBUF) to
-// overwrite the buffer P(u) was read from.
-// Measured, bf16: hierarchical masks 16 x 16 x 4096 x 64 483 us (560 with a group of heads per CTA, two issuing warps and
-// eight softmax warps), causal 8 x 16 x 2048 x 64 119 us (147), x 128 152 us (207): 1,800 cycles a tile at D = 64, 2,400 at 128.
-// At D = 128 the chain P -> P V -> S -> P of a tile is what is left: with long lists (hierarchical, 32 heads x 8192) the tensor
-// pipe is busy 54 % of the time and the special-function units 55 %.
-// Tried and slower: a quarter of the exponentials as polynomials on the FMA pipe (5-9 %).
+// unit u finds the scores of its tile's next unit in TMEM. The tensor pipe executes in issue order, which is what allows
+// S(u + NBUF) to overwrite the buffer P(u) was read from.
+// Measured, bf16: hierarchical masks 16 x 16 x 4096 x 64 425 us, causal 8 x 16 x 2048 x 64 110 us; 1,400 cycles a tile with full lists, of
+// which the special-function units are busy 1,024 and the issuing warp all: its steps take 1,430 one after the other.
+// Tried and slower: a quarter of the exponentials as polynomials on the FMA pipe (5-9 %); an issuing warp per query tile, or one for
+// the scores and one for P V (the issuing warp's order is what keeps the exponentials of the two tiles apart: in phase, full lists
+// 1,600, short ones +10 %); the first half of the exponentials before the exchange of maxima (1,550); the next scores loaded
+// ahead (1,650); eight softmax warps with a thread per row, as above head dim 64 (1,465, short lists +10 %).
 // EMPTY tiles never appear in the list: they are neither loaded nor multiplied.
 //
 // Replaces _flash_attn_fwd (original_kernel.py:278-626): same math (scores scaled by
@@ -34,7 +34,7 @@
 // LSE = -inf.
 #include <algorithm>
 
-#include "attn_common.cuh"
+#include "attn_fwd.cuh"
 #ifdef KD_TEST_DROP_LOAD
 #include <stdlib.h>
 #endif
@@ -55,37 +55,17 @@ __global__ void test_busy_kernel(uint64_t ns) {
 }
 #endif
 
-struct FwdArgs {
-  int B, H, T, NT, NP, Tpad;
-  ItemOrder order_of;
-  int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
-  float scale_log2;  // sm_scale * log2(e)
-  const uint32_t* desc;
-  const uint32_t* tilebits;   // [B][NT][8][4] class masks of every 128-token tile
-  const int32_t* fwd_cnt;
-  const uint16_t* fwd_list;
-  const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length
-  uint32_t* status;
-  int plan_ready;
-  void* o;
-  int64_t o_sb, o_sh, o_st;
-  float* lse;
-#ifdef KD_TEST_DROP_LOAD
-  int test_drop_load;   // wait time-out test build: the producer of CTA 0 leaves out its first K tile load
-#endif
-};
-
-template <int HD>
 struct FwdCfg {
+  static constexpr int HD = 64;
   static constexpr int KBLK = HD / 64;                   // 64-element blocks along D
   static constexpr int TILE_BYTES = KD_TILE * HD * 2;    // one Q / K / V tile
-  static constexpr int NBUF = (HD == 64) ? 3 : 2;        // score buffers in TMEM
+  static constexpr int NBUF = 3;                         // score buffers in TMEM
   static constexpr int KST = NBUF;                       // K ring stages
-  static constexpr int VST = (HD == 64) ? 3 : 2;         // V ring stages
-  static constexpr int NQ = (HD == 64) ? 4 : 3;          // ring of Q tiles (two per item): the next item's Q loads while this one computes
+  static constexpr int VST = 3;                          // V ring stages
+  static constexpr int NQ = 4;                           // ring of Q tiles (two per item): the next item's Q loads while this one computes
   static constexpr int NPART = 2;                        // P is handed over in two parts: the first, then the second 32 columns of each half
-  static constexpr int NITEM = (HD == 64) ? 4 : 2;       // ring of item headers and lists
-  static constexpr int NXB = (HD == 64) ? 2 : 1;         // buffers of the row maxima that two warps exchange (see there)
+  static constexpr int NITEM = 4;                        // ring of item headers and lists
+  static constexpr int NXB = 2;                          // buffers of the row maxima that two warps exchange (see there)
   static constexpr int SMEM_Q = 0;
   static constexpr int SMEM_K = SMEM_Q + NQ * TILE_BYTES;
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
@@ -111,23 +91,12 @@ struct FwdCfg {
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
-// wait-site codes reported in the status word
-enum : uint32_t {
-  W_F_QFULL = 0x101, W_F_KEMPTY = 0x102, W_F_VEMPTY = 0x103, W_F_KFULL = 0x104, W_F_VFULL = 0x105,
-  W_F_PFULL = 0x106, W_F_SFULL = 0x107, W_F_PVDONE = 0x108, W_F_QEMPTY = 0x10A, W_F_OFREE = 0x10B,
-  W_F_ITEMFULL = 0x10C, W_F_ITEMEMPTY = 0x10D, W_F_CLC = 0x10E, W_F_ALIGN = 0x10F,
-};
-
-// list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10; in shared memory also
-// | score buffer of the entry's first unit << 12
-__device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
-
-template <int HD, bool kBf16>
-__global__ void __launch_bounds__(FwdCfg<HD>::THREADS, 1)
+template <bool kBf16>
+__global__ void __launch_bounds__(FwdCfg::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
-  using C = FwdCfg<HD>;
-  constexpr int TILE = C::TILE_BYTES;
+  using C = FwdCfg;
+  constexpr int HD = C::HD, TILE = C::TILE_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t s0 = smem_u32(smem);
   const uint32_t sQ = s0 + C::SMEM_Q, sK = s0 + C::SMEM_K, sV = s0 + C::SMEM_V;
@@ -191,68 +160,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     reg_dealloc<C::REGS_LIGHT>();
     if (warp == 0) {
       // ------------------------------ producer warp ------------------------------
-      if (lane == 0) {
-        tma_prefetch_desc(&tmQ);
-        tma_prefetch_desc(&tmK);
-        tma_prefetch_desc(&tmV);
-      }
-      int q_cnt = 0, kv_cnt = 0, v_cnt = 0, k = 0, asked = 0;   // Q, K, V tiles requested, items published, cancellations asked for
-      int k_dropped = -1;   // index of a K tile that was never requested (test builds only)
-      bool ok = true, pending = false;
       const uint32_t below = (1u << lane) - 1u;
       uint32_t unit0 = 0u;  // score buffer of the next item's first unit
-      uint32_t lst[4];      // the next item's list, 32 entries per register
-      auto decode = [&](int idx) -> int4 {
-        int4 it;
-        int rank;
-        a.order_of.decode(idx, a.NP, it.x, rank);
-        it.y = it.x % a.H;
-        it.x = it.x / a.H;
-        it.z = __ldcg(a.order + ((size_t)it.x * 3 + 0) * a.NT + rank);
-        const uint16_t* list = a.fwd_list + ((size_t)it.x * a.NP + it.z) * a.NT;
-        it.w = __ldcg(a.fwd_cnt + it.x * a.NP + it.z);
-#pragma unroll
-        for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
-#pragma unroll
-        for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < it.w ? lst[r] : 0u;
-        return it;
-      };
-      // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), which hides the
-      // answer and the look-up of its list, and no earlier: an item held in reserve by a CTA with a long list is one that an idle CTA cannot take (claimed two
-      // items ahead: 575 us for 519 with hierarchical masks at 16 x 16 x 4096 x 64).
-      auto ask = [&]() {
-        if (lane == 0) {
-          fence_proxy_async_smem();   // the previous response has been read
-          mbar_arrive_expect_tx(bar(C::B_CLC), 16);
-          clc_try_cancel(s0 + C::SMEM_CLC, bar(C::B_CLC));
-        }
-        ++asked;
-        pending = true;
-      };
-      auto take_next = [&](int4& nx) -> bool {
-        if (!wait(C::B_CLC, (asked - 1) & 1, W_F_CLC)) return false;
-        pending = false;
-        const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
-        __syncwarp();   // every lane has read the response that the next request overwrites
-        nx.w = -1;
-        if (idx >= 0) {
-          nx = decode(idx);
-          if (nx.w <= 2) ask();
-        }
-        return true;
-      };
-      auto load_tile = [&](const CUtensorMap* tm, uint32_t dst, int full, int tile, int h, int b) {
-        if (lane != 0) return;
-        mbar_arrive_expect_tx(bar(full), TILE);
-        for (int kb = 0; kb < C::KBLK; ++kb) tma_load_4d(dst + kb * 16384, tm, bar(full), kb * 64, tile * KD_TILE, h, b);
-      };
-      int4 it = decode(blockIdx.x);
-      if (it.w <= 2) ask();
-      while (ok) {
-        const int slot = k % C::NITEM;
-        if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_F_ITEMEMPTY))) break;
-        const int b = it.x, h = it.y, pair = it.z, n = it.w;
-        int units[2] = {0, 0};
+      // in shared memory an entry has the score buffer of its first unit << 12 as well
+      auto publish = [&](int slot, const uint32_t (&lst)[4], int, int (&units)[2]) {
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const uint32_t has0 = __ballot_sync(0xffffffffu, entry_class(lst[r], 0) != 0u), has1 = __ballot_sync(0xffffffffu, entry_class(lst[r], 1) != 0u);
@@ -262,65 +173,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           units[1] += __popc(has1);
         }
         unit0 = (unit0 + units[0] + units[1]) % C::NBUF;
-        if (lane == 0) items[slot] = make_int4(b, h, pair, n < 0 ? -1 : (n | (units[0] << 8) | (units[1] << 16)));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(C::B_ITEMFULL + slot));
-        if (n < 0) break;
-        if (k == 0) {   // Q, K and V are read from here on
-          pdl_wait();
-          pdl_launch_dependents();
-        }
-        ++k;
-        const int ntile_q = (2 * pair + 1 < a.NT) ? 2 : 1;
-        auto load_q = [&](int t) -> bool {
-          const int s = q_cnt % C::NQ;
-          if (!wait(C::B_QEMPTY + s, ((q_cnt / C::NQ) & 1) ^ 1, W_F_QEMPTY)) return false;
-          load_tile(&tmQ, sQ + s * TILE, C::B_QFULL + s, 2 * pair + t, h, b);
-          ++q_cnt;
-          return true;
-        };
-        if (!(ok = load_q(0))) break;
-        int4 nx = it;
-#pragma unroll 1
-        for (int e = 0; e < max(n, 1); ++e) {
-          if (n > 2 && e == n - 3) ask();
-          if (e >= n - 1 && !(ok = take_next(nx))) break;   // its list is looked up while this item's last tiles wait for slots
-          if (n == 0) {
-            if (ntile_q == 2) ok = load_q(1);
-            break;
-          }
-          const int kt = sList[slot * 128 + e] & 0xFF;
-#ifdef KD_TEST_DROP_LOAD
-          // Test build only: this one K tile is never requested (no copy, no expected bytes), so the S issuer's
-          // bounded wait for it runs out and the CTA has to unwind. Nothing is left in flight for the stage.
-          if (a.test_drop_load && blockIdx.x == 0 && kv_cnt == 0) {
-            k_dropped = kv_cnt++;
-          } else
-#endif
-          {
-            const int s = kv_cnt % C::KST;
-            if (!(ok = wait(C::B_KEMPTY + s, ((kv_cnt / C::KST) & 1) ^ 1, W_F_KEMPTY))) break;
-            load_tile(&tmK, sK + s * TILE, C::B_KFULL + s, kt, h, b);
-            ++kv_cnt;
-          }
-          if (e == 0 && ntile_q == 2 && !(ok = load_q(1))) break;
-          {
-            const int s = v_cnt % C::VST;
-            if (!(ok = wait(C::B_VEMPTY + s, ((v_cnt / C::VST) & 1) ^ 1, W_F_VEMPTY))) break;
-            load_tile(&tmV, sV + s * TILE, C::B_VFULL + s, kt, h, b);
-            ++v_cnt;
-          }
-        }
-        it = nx;
-      }
-      if (abortf->v != 0 && lane == 0) {
-        // unwinding: let every copy already in flight land (bounded) before the CTA exits
-        for (int e = max(0, kv_cnt - C::KST); e < kv_cnt; ++e)
-          if (e != k_dropped) drain_wait(bar(C::B_KFULL + e % C::KST), (e / C::KST) & 1);
-        for (int e = max(0, v_cnt - C::VST); e < v_cnt; ++e) drain_wait(bar(C::B_VFULL + e % C::VST), (e / C::VST) & 1);
-        for (int e = max(0, q_cnt - C::NQ); e < q_cnt; ++e) drain_wait(bar(C::B_QFULL + e % C::NQ), (e / C::NQ) & 1);
-        if (pending) drain_wait(bar(C::B_CLC), (asked - 1) & 1);
-      }
+      };
+      fwd_producer<C>(tmQ, tmK, tmV, a, smem, abortf, lane, wait, publish);
     } else if (warp == 1) {
       // ------------------------------ issuer ------------------------------
       // All lanes follow the control flow and one elected lane issues (mma_ss_uniform). One warp issues both products: the
@@ -479,12 +333,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float* xch = reinterpret_cast<float*>(smem + C::SMEM_XCH) + i * (2 * KD_TILE) + row;
     // Both warps of 32 rows: hands over a value and takes the partner's; false: some role has aborted. The barrier cannot
     // hang: a warp that gives up arrives there once more (below), and the partner sees the abort behind the barrier.
-    // With two buffers a slot is written again two exchanges later, when the partner, which has been to the barrier in between,
-    // has read it. Where shared memory has room for one only (HD = 128), other synchronisation lies between two exchanges.
+    // A slot is written again two exchanges later, when the partner, which has been to the barrier in between, has read it.
     const uint32_t pair_bar = 1 + i * 4 + wq;
     int exchanges = 0;
     auto exchange = [&](float mine, float& other) -> bool {
-      float* x = xch + (C::NXB == 2 ? (exchanges++ & 1) * (4 * KD_TILE) : 0);
+      float* x = xch + (exchanges++ % C::NXB) * (4 * KD_TILE);
       x[half * KD_TILE] = mine;
       named_bar_sync(pair_bar, 64);
       other = x[(half ^ 1) * KD_TILE];
@@ -496,7 +349,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // state that runs on across the items of this CTA
     uint32_t sfull_par = 0;     // bit j: parity of the next phase of this tile's score barrier on buffer j
     int pv_seen = 0;            // P V products of this query tile handed over so far
-    int last_buf = 0;           // buffer of this tile's last unit
     // Waits for the last of them (back = 1), or the one before. Not for every unit: a product signals on one of two barriers in
     // turn. A parity wait is sound while the barrier's phase before the awaited one is complete, that is the tile's product two
     // before it. Once the scores of the tile's next unit are ready it is (products and scores execute in issue order, and at
@@ -631,12 +483,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
       for (int k4 = 0; k4 < 4; ++k4) mx4[k4] = fmaxf(mx4[k4], sc[CW - 4 + k4]);
       float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      if (C::NXB == 1 && nact > 0 && sbuf != last_buf) {
-        // Consecutive units of one tile: the scores can be ready before the partner has read this warp's last maximum, which
-        // it does before it hands over its P. (Otherwise they have been issued behind that P's product.)
-        if (!(ok = pv_done(1))) break;
-      }
-      last_buf = sbuf;
       float mx_other;
       if (!(ok = exchange(mx, mx_other))) break;
       mx = fmaxf(mx, mx_other);
@@ -695,10 +541,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (nact > 0 && !(ok = pv_done(2) && pv_done(1))) break;
     float l_other;
     if (!(ok = exchange(l, l_other))) break;
-    if constexpr (C::NXB == 1) {   // both have read the sums: the slot may be written again
-      named_bar_sync(pair_bar, 64);
-      if (!(ok = __all_sync(0xffffffffu, abortf->v == 0u))) break;
-    }
     l += l_other;
     if (half == 0 && qi < a.T && a.lse != nullptr) {
       a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
@@ -736,9 +578,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (tid == 0) report_abort(abortf, a.status);
 }
 
-template <int HD, bool kBf16>
-static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
-  using C = FwdCfg<HD>;
+template <bool kBf16>
+static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, cudaStream_t stream) {
+  auto kern = attn_fwd_kernel<kBf16>;
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in(kern, FwdCfg::SMEM_ALLOC);
+  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
+  e = launch(kern, static_cast<unsigned>(n_items), FwdCfg::THREADS, FwdCfg::SMEM_ALLOC, stream, tmQ, tmK, tmV, a);
+  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_fwd_kernel launch: %s", cudaGetErrorString(e));
+  return 0;
+}
+
+int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
+  kd_plan_layout L;
+  if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
+  const PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
   CUtensorMap tmQ, tmK, tmV;
   int rc;
   if ((rc = encode_tensor_map(&tmQ, p.q, p.B, p.H, p.T, p.D, p.dtype, KD_TILE, "q")) != 0) return rc;
@@ -761,22 +615,9 @@ static int launch_fwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   const char* drop = getenv("KD_TEST_DROP_LOAD");
   a.test_drop_load = (drop != nullptr && atoi(drop) != 0) ? 1 : 0;
 #endif
-  auto kern = attn_fwd_kernel<HD, kBf16>;
-  static SmemOptIn opt_in;
-  cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
-  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
-  e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, a);
-  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_fwd_kernel launch: %s", cudaGetErrorString(e));
-  return 0;
-}
-
-int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
-  kd_plan_layout L;
-  if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
-  PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
-  // head dims below the tile width run on the next wider instantiation: TMA zero-fills the missing columns
-  if (p.D <= 64) return p.dtype == KD_BF16 ? launch_fwd_t<64, true>(p, L, pv, stream) : launch_fwd_t<64, false>(p, L, pv, stream);
-  return p.dtype == KD_BF16 ? launch_fwd_t<128, true>(p, L, pv, stream) : launch_fwd_t<128, false>(p, L, pv, stream);
+  // head dims below the tile width run on the next wider kernel: TMA zero-fills the missing columns
+  if (p.D > 64) return launch_attn_fwd_wide(n_items, a, p.dtype, tmQ, tmK, tmV, stream);
+  return p.dtype == KD_BF16 ? launch_fwd_t<true>(n_items, a, tmQ, tmK, tmV, stream) : launch_fwd_t<false>(n_items, a, tmQ, tmK, tmV, stream);
 }
 
 }  // namespace kd

@@ -75,6 +75,32 @@ def test_many_items_per_cta_with_empty_ones_between(monkeypatch, T, n_full, D, d
             assert_close(name, sl(got), ref)
 
 
+# Forward above head dim 64: an issuing warp per query tile walks a common list. A tile of prefix tokens in the middle of the
+# sequence sees the prefix only, its pair's other tile nearly everything: runs of entries of one tile, longer than the rings of
+# K and V tiles, for tile 1 of a pair (tile 8) and for tile 0 (tile 13); a tile beyond the sequence length; an odd number of tiles;
+# scores whose maximum grows from tile to tile (O is rescaled)
+@pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (80, torch.float16)])
+@pytest.mark.parametrize("T,length", [(128 * 14, 128 * 14), (128 * 15 - 127, 128 * 14 + 1), (128 * 14 + 5, 128 * 12)])
+def test_forward_wide_unequal_lists_of_a_pair(T, length, D, dtype):
+    from tests.helpers import assert_close, assert_lse_close
+    from kerneldev_b200 import flash_attention
+    B, H = 2, 3
+    ins, sid, pre = np.zeros((B, T), bool), np.zeros((B, T), np.int64), np.zeros((B, T), bool)
+    for tile in (0, 8, 13):
+        pre[:, tile * 128:(tile + 1) * 128] = True
+    lens = np.array([length, T], np.int32)
+    g = torch.Generator(device=DEV).manual_seed(T + D)
+    q, k, v = (torch.randn((B, H, T, D), generator=g, device=DEV) for _ in range(3))
+    k *= torch.linspace(0.2, 4.0, T, device=DEV)[:, None]
+    q, k, v = (x.to(dtype) for x in (q, k, v))
+    with torch.no_grad():
+        o, lse = flash_attention(q, k, v, return_lse=True, in_span=torch.as_tensor(ins, device=DEV), span_id=torch.as_tensor(sid, device=DEV),
+                                 is_prefix=torch.as_tensor(pre, device=DEV), lens=torch.as_tensor(lens, device=DEV))
+    want_o, want_lse = ao.attention_forward(q.float().cpu(), k.float().cpu(), v.float().cpu(), torch.as_tensor(ao.dense_mask(T, ins, sid, pre, lens)))[:2]
+    assert_close("O", o, want_o)   # P is rounded to 16 bits before its product: the repository's tolerance for that
+    assert_lse_close(lse, want_lse)
+
+
 # a row of exactly one chunk of 4096 tokens, one more, and several: first [CLS] in the first, a later, or no chunk
 @pytest.mark.parametrize("T", [1, 127, 4096, 4097, 12289])
 def test_metadata_chunks(T):
