@@ -21,8 +21,9 @@
 // keys) is written over the same buffer. S(u + NBUF) is issued directly after P(u) V, so that a softmax warp that finishes
 // unit u finds the scores of its tile's next unit in TMEM. The tensor pipe executes in issue order, which is what allows
 // S(u + NBUF) to overwrite the buffer P(u) was read from.
-// Measured, bf16: hierarchical masks 16 x 16 x 4096 x 64 425 us, causal 8 x 16 x 2048 x 64 110 us; 1,400 cycles a tile with full lists, of
-// which the special-function units are busy 1,024 and the issuing warp all: its steps take 1,430 one after the other.
+// Measured, bf16: hierarchical masks 8 x 16 x 4096 x 64 215 us, causal 8 x 16 x 1000 x 64 38.9; 1,400 cycles a tile with full lists, of
+// which the special-function units are busy 1,024. (The issuing warp's steps take as long one after the other, but a loop a fifth
+// shorter, with what it needs of a unit in one byte, changed nothing.)
 // Tried and slower: a quarter of the exponentials as polynomials on the FMA pipe (5-9 %); an issuing warp per query tile, or one for
 // the scores and one for P V (the issuing warp's order is what keeps the exponentials of the two tiles apart: in phase, full lists
 // 1,600, short ones +10 %); the first half of the exponentials before the exchange of maxima (1,550); the next scores loaded
@@ -239,7 +240,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           i = 1;
           new_k = false;
         } else {
-          if (e == n) next = __reduce_max_sync(0xffffffffu, next_list());
+          // (with every buffer taken a P V comes first: closing and opening an item takes this warp up to 1,800 cycles, which the
+          // units in flight would wait for, to no purpose)
+          if (e == n) next = n_flight == C::NBUF ? static_cast<int>(STALLED) : __reduce_max_sync(0xffffffffu, next_list());
           if (next == ABORTED) break;
           if (next == UNIT) {
             if (e == 0) began = 0u;
@@ -331,17 +334,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t tO = lane_base + (i == 0 ? C::TM_O0 : C::TM_O1) + half * (HD / 2);   // this thread's half of its row of O
     float* xch = reinterpret_cast<float*>(smem + C::SMEM_XCH) + i * (2 * KD_TILE) + row;
-    // Both warps of 32 rows: hands over a value and takes the partner's; false: some role has aborted. The barrier cannot
-    // hang: a warp that gives up arrives there once more (below), and the partner sees the abort behind the barrier.
+    // Both warps of 32 rows: hands over a value and takes the partner's. Whether some role has aborted is read behind the barrier and
+    // looked at before the next exchange, off the chain. The barrier cannot hang: a warp that gives up arrives there once more
+    // (below), and the partner sees the abort behind it.
     // A slot is written again two exchanges later, when the partner, which has been to the barrier in between, has read it.
     const uint32_t pair_bar = 1 + i * 4 + wq;
     int exchanges = 0;
-    auto exchange = [&](float mine, float& other) -> bool {
+    uint32_t aborted = 0u;   // looked at before the next exchange
+    auto exchange = [&](float mine, float& other) {
       float* x = xch + (exchanges++ % C::NXB) * (4 * KD_TILE);
       x[half * KD_TILE] = mine;
       named_bar_sync(pair_bar, 64);
       other = x[(half ^ 1) * KD_TILE];
-      return __all_sync(0xffffffffu, abortf->v == 0u);
+      aborted = abortf->v;
     };
     const float c = a.scale_log2;
     const uint64_t c2 = pack_f32x2(c, c);
@@ -484,30 +489,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int k4 = 0; k4 < 4; ++k4) mx4[k4] = fmaxf(mx4[k4], sc[CW - 4 + k4]);
       float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx_other;
-      if (!(ok = exchange(mx, mx_other))) break;
+      exchange(mx, mx_other);
       mx = fmaxf(mx, mx_other);
-      // The running maximum is refreshed only when it would grow by more than 2^8 in the
-      // exponent; until then the stale value is used consistently for P, l and O, which leaves
-      // the normalised result unchanged and skips most O rescales.
-      float m_new = m;
-      if (m == -INFINITY || (mx - m) * c > 8.0f) m_new = fmaxf(m, mx);
-      const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-      const float alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * c);
-      const bool need_rescale = (nact > 0) && (m_new != m);
-      if (__any_sync(0xffffffffu, need_rescale)) {   // O may be touched only after the tile's previous product
-        if (!(ok = pv_done(1))) break;
-        tc_fence_after_sync();
-        const float f = need_rescale ? alpha : 1.f;
+      // The running maximum is refreshed only when it would grow by more than 2^8 in the exponent (or is -inf: the difference is then
+      // inf); until then the stale value is used consistently for P, l and O, which leaves the normalised result unchanged, skips
+      // most O rescales and keeps the refresh out of the chain.
+      const bool grow = (mx - m) * c > 8.0f;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float m_new = grow ? mx : m, alpha = (m == -INFINITY) ? 0.f : fast_exp2((m - m_new) * c);
+        if (nact > 0 && __any_sync(0xffffffffu, grow && m != -INFINITY)) {   // O may be touched only after the tile's previous product
+          if (!(ok = pv_done(1))) break;
+          tc_fence_after_sync();
+          const float f = grow ? alpha : 1.f;
 #pragma unroll 1
-        for (int cb = 0; cb < HD / 32; ++cb) {   // rare; 16 columns at a time, for the scores are still in registers
-          uint32_t r[16];
-          tmem_ld16(tO + cb * 16, r);
-          tmem_wait_ld();
+          for (int cb = 0; cb < HD / 32; ++cb) {   // rare; 16 columns at a time, for the scores are still in registers
+            uint32_t r[16];
+            tmem_ld16(tO + cb * 16, r);
+            tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
-          tmem_st16(tO + cb * 16, r);
+            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
+            tmem_st16(tO + cb * 16, r);
+          }
         }
+        if (grow) l *= alpha;
+        m = m_new;
       }
+      const float m_use = (m == -INFINITY) ? 0.f : m;
       const uint64_t neg_mc2 = pack_f32x2(-m_use * c, -m_use * c);
       uint64_t sum2[2] = {0u, 0u};
 #pragma unroll
@@ -528,10 +535,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (lane == 0) mbar_arrive(bar(C::B_PFULL + C::NPART * sbuf + cb));
       }
       const uint64_t sum_pair = add_f32x2(sum2[0], sum2[1]);
-      l = l * alpha + (lo_f32x2(sum_pair) + hi_f32x2(sum_pair));
-      m = m_new;
+      l += lo_f32x2(sum_pair) + hi_f32x2(sum_pair);
       ++nact;
       ++pv_seen;
+      if (!(ok = __all_sync(0xffffffffu, aborted == 0u))) break;
     }
     if (!ok) break;
     item_done(k);
@@ -540,7 +547,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     // epilogue of this item: normalise, convert, store this thread's share of O, and LSE
     if (nact > 0 && !(ok = pv_done(2) && pv_done(1))) break;
     float l_other;
-    if (!(ok = exchange(l, l_other))) break;
+    exchange(l, l_other);
+    if (!(ok = __all_sync(0xffffffffu, aborted == 0u))) break;
     l += l_other;
     if (half == 0 && qi < a.T && a.lse != nullptr) {
       a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
