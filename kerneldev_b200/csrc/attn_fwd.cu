@@ -71,7 +71,7 @@ struct FwdCfg {
   static constexpr int SMEM_K = SMEM_Q + NQ * TILE_BYTES;
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
   static constexpr int SMEM_LIST = SMEM_V + VST * TILE_BYTES;      // NITEM x <= 128 list entries
-  static constexpr int SMEM_ITEM = SMEM_LIST + NITEM * 128 * 2;    // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16}
+  static constexpr int SMEM_ITEM = SMEM_LIST + NITEM * 128 * 2;    // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16 | the item's only tile + 1 << 24}
   static constexpr int SMEM_XCH = SMEM_ITEM + NITEM * 16;          // NXB x [query tile][half][row] fp32
   static constexpr int SMEM_CLC = SMEM_XCH + NXB * 4 * KD_TILE * 4;
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
@@ -165,11 +165,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       uint32_t unit0 = 0u;  // score buffer of the next item's first unit
       // in shared memory an entry has the score buffer of its first unit << 12 as well
       auto publish = [&](int slot, const uint32_t (&lst)[4], int, int (&units)[2]) {
+        int e = 0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const uint32_t has0 = __ballot_sync(0xffffffffu, entry_class(lst[r], 0) != 0u), has1 = __ballot_sync(0xffffffffu, entry_class(lst[r], 1) != 0u);
           const uint32_t first = (unit0 + units[0] + units[1] + __popc(has0 & below) + __popc(has1 & below)) % C::NBUF;
-          sList[slot * 128 + r * 32 + lane] = static_cast<uint16_t>(lst[r] | (first << 12));
+          if (lst[r] != 0u) sList[slot * 128 + e + __popc((has0 | has1) & below)] = static_cast<uint16_t>(lst[r] | (first << 12));
+          e += __popc(has0 | has1);
           units[0] += __popc(has0);
           units[1] += __popc(has1);
         }
@@ -404,8 +406,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
-      qi_next = qtile * KD_TILE + row;
-      qd_next = qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
+      const int only = it.w >> 24;
+      const bool mine = only == 0 || only == i + 1;
+      qi_next = mine ? qtile * KD_TILE + row : INT_MAX;   // (written by the other item of the pair)
+      qd_next = mine && qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
       list = sList + (k % C::NITEM) * 128;
       e = 0;
       if (n_next > 0) {
@@ -610,10 +614,11 @@ int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
   a.B = p.B; a.H = p.H; a.T = p.T; a.NT = L.NT; a.NP = L.NP; a.Tpad = L.NT * KD_TILE;
   a.d_real = p.D;
   a.scale_log2 = p.sm_scale * 1.4426950408889634f;
-  const long long n_items = (long long)p.B * p.H * L.NP;
+  a.split = split_pairs(static_cast<int>(std::min<long long>((long long)p.B * p.H * L.NP, INT_MAX / 2)), L.NT);
+  const long long n_items = ((long long)p.B * p.H * L.NP) << a.split;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 256) exceeds 2^31 - 1");
   // Q, K, V and O. (64 and 110 MB: no difference outside the noise)
-  a.order_of = ItemOrder::make(p.B * p.H, L.NP, (double)p.T * p.D * 2 * 4, 64e6);
+  a.order_of = ItemOrder::make(p.B * p.H, L.NP << a.split, (double)p.T * p.D * 2 * 4, 64e6);
   a.plan_ready = p.plan_ready;
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
   a.order = pv.order; a.tilebits = pv.tilebits;

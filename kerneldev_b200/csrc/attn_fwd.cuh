@@ -16,6 +16,7 @@ struct FwdArgs {
   const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length
   uint32_t* status;
   int plan_ready;
+  int split;         // 1: an item is one query tile of a pair (see split_pairs)
   void* o;
   int64_t o_sb, o_sh, o_st;
   float* lse;
@@ -34,9 +35,16 @@ enum : uint32_t {
 // list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10
 __device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
 
+// Pairs of query tiles are split into items of one tile each while those have an SM each: two tiles' exponentials on one SM take turns
+// at its special-function units, and the other SMs have nothing to do. A call in a stream of them, pairs -> tiles (us, bf16): causal
+// 1 x 16 x 256 x 64 7.1 -> 6.2, 1 x 8 x 1000 x 64 18.7 -> 14.8, 1 x 4 x 4096 x 64 48.4 -> 37.7, 1 x 8 x 1024 x 128 18.2 -> 16.4, 74 pairs of T = 500 10.8 -> 9.5
+// (D = 64) and, 64 of them, 12.3 -> 12.3 (D = 128). With more pairs some SMs would have two items to others' one.
+inline int split_pairs(int pairs, int tiles_per_head) { return tiles_per_head > 1 && 2 * pairs <= 148 ? 1 : 0; }
+
 // The producer warp: takes items (see the head of attn_fwd.cu), publishes their headers and lists and loads Q tiles and the rings of
 // K and V tiles by TMA. C: the kernel's configuration. wait(barrier, parity, site): a warp's bounded wait. publish(slot, lst, n,
-// units): writes the list of an item with n entries, 32 per register and lane, to its slot and counts the units of both query tiles.
+// units): writes the list of an item with n entries, 32 per register and lane (in a split pair with gaps: zeros), to its slot and counts
+// the units of both query tiles.
 template <typename C, typename Wait, typename Publish>
 __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const FwdArgs& a, uint8_t* smem,
                                              AbortFlag* abortf, int lane, const Wait& wait, const Publish& publish) {
@@ -57,16 +65,25 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
   auto decode = [&](int idx) -> int4 {
     int4 it;
     int rank;
-    a.order_of.decode(idx, a.NP, it.x, rank);
+    a.order_of.decode(idx, a.NP << a.split, it.x, rank);
     it.y = it.x % a.H;
     it.x = it.x / a.H;
-    it.z = __ldcg(a.order + ((size_t)it.x * 3 + 0) * a.NT + rank);
-    const uint16_t* list = a.fwd_list + ((size_t)it.x * a.NP + it.z) * a.NT;
-    it.w = __ldcg(a.fwd_cnt + it.x * a.NP + it.z);
+    const int pair = __ldcg(a.order + ((size_t)it.x * 3 + 0) * a.NT + (rank >> a.split)), only = a.split ? 1 + (rank & 1) : 0;
+    it.z = pair | (only << 16);
+    const uint16_t* list = a.fwd_list + ((size_t)it.x * a.NP + pair) * a.NT;
+    it.w = __ldcg(a.fwd_cnt + it.x * a.NP + pair);
 #pragma unroll
     for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
 #pragma unroll
     for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < it.w ? lst[r] : 0u;
+    if (only != 0) {   // the entries that are not EMPTY for the one tile
+      it.w = 0;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        lst[r] = entry_class(lst[r], only - 1) != 0u ? lst[r] & (only == 1 ? 0x3FFu : 0xCFFu) : 0u;
+        it.w += __popc(__ballot_sync(0xffffffffu, lst[r] != 0u));
+      }
+    }
     return it;
   };
   // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), which hides the
@@ -103,10 +120,10 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
   while (ok) {
     const int slot = k % C::NITEM;
     if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_F_ITEMEMPTY))) break;
-    const int b = it.x, h = it.y, pair = it.z, n = it.w;
+    const int b = it.x, h = it.y, pair = it.z & 0xFFFF, only = it.z >> 16, n = it.w;
     int units[2] = {0, 0};
     publish(slot, lst, n, units);
-    if (lane == 0) items[slot] = make_int4(b, h, pair, n < 0 ? -1 : (n | (units[0] << 8) | (units[1] << 16)));
+    if (lane == 0) items[slot] = make_int4(b, h, pair, n < 0 ? -1 : (n | (units[0] << 8) | (units[1] << 16) | (only << 24)));
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(C::B_ITEMFULL + slot));
     if (n < 0) break;

@@ -38,7 +38,7 @@ struct FwdWideCfg {
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
   static constexpr int SMEM_LIST = SMEM_V + VST * TILE_BYTES;      // NITEM x <= 128 list entries
   static constexpr int SMEM_OWN = SMEM_LIST + NITEM * 128 * 2;     // NITEM x the units of query tile 0, then of tile 1: key tile | PARTIAL << 8
-  static constexpr int SMEM_ITEM = SMEM_OWN + NITEM * 256 * 2;     // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16}
+  static constexpr int SMEM_ITEM = SMEM_OWN + NITEM * 256 * 2;     // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16 | the item's only tile + 1 << 24}
   static constexpr int SMEM_CLC = SMEM_ITEM + NITEM * 16;
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
   // barriers (8 bytes each)
@@ -124,9 +124,12 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const uint32_t below = (1u << lane) - 1u;
       // the list for the issuers, and each query tile's own for its softmax warps
       auto publish = [&](int slot, const uint32_t (&lst)[4], int, int (&units)[2]) {
+        int e = 0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-          sList[slot * 128 + r * 32 + lane] = static_cast<uint16_t>(lst[r]);
+          const uint32_t any = __ballot_sync(0xffffffffu, lst[r] != 0u);
+          if (lst[r] != 0u) sList[slot * 128 + e + __popc(any & below)] = static_cast<uint16_t>(lst[r]);
+          e += __popc(any);
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const uint32_t cls = entry_class(lst[r], i), has = __ballot_sync(0xffffffffu, cls != 0u);
@@ -283,8 +286,10 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
-      qi_next = qtile * KD_TILE + row;
-      qd_next = qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
+      const int only = it.w >> 24;
+      const bool mine = only == 0 || only == i + 1;
+      qi_next = mine ? qtile * KD_TILE + row : INT_MAX;   // (written by the other item of the pair)
+      qd_next = mine && qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
       list = sOwn + (k % C::NITEM) * 256 + i * 128;
       if (n_next > 0) ent_next = list[0];
       return true;

@@ -101,6 +101,26 @@ def test_forward_wide_unequal_lists_of_a_pair(T, length, D, dtype):
     assert_lse_close(lse, want_lse)
 
 
+# Forward items of one query tile (up to 74 pairs of tiles in a call) and of two (75): pairs with a second tile, without one (T = 300),
+# and with entries of the list that are EMPTY for one of them; rows beyond the sequence length; one tile per head is not split
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (112, torch.float16)])
+@pytest.mark.parametrize("B,H,T", [(2, 37, 200), (3, 25, 200), (1, 37, 300), (2, 2, 128 * 9 + 1), (74, 1, 100)])
+def test_forward_items_of_one_tile(B, H, T, D, dtype):
+    from tests.helpers import assert_close, assert_lse_close, random_meta, rand_inputs
+    from kerneldev_b200 import flash_attention
+    ins, sid, pre = random_meta(T + D, B, T)
+    ins[:, 128:256], pre[:, 128:256], sid[:, 128:256] = False, True, 0   # a tile of prefix tokens: sees few others
+    lens = np.array([T if b % 2 == 0 else T // 2 for b in range(B)], np.int32)
+    q, k, v, _ = rand_inputs(B, H, T, D, dtype, T + H)
+    with torch.no_grad():
+        o, lse = flash_attention(q.to(DEV), k.to(DEV), v.to(DEV), return_lse=True, in_span=torch.as_tensor(ins, device=DEV),
+                                 span_id=torch.as_tensor(sid, device=DEV), is_prefix=torch.as_tensor(pre, device=DEV),
+                                 lens=torch.as_tensor(lens, device=DEV))
+    want_o, want_lse = ao.attention_forward(q, k, v, torch.as_tensor(ao.dense_mask(T, ins, sid, pre, lens)))
+    assert_close("O", o, want_o)   # P is rounded to 16 bits before its product: the repository's tolerance for that
+    assert_lse_close(lse, want_lse)
+
+
 # a row of exactly one chunk of 4096 tokens, one more, and several: first [CLS] in the first, a later, or no chunk
 @pytest.mark.parametrize("T", [1, 127, 4096, 4097, 12289])
 def test_metadata_chunks(T):
