@@ -121,6 +121,26 @@ def test_forward_items_of_one_tile(B, H, T, D, dtype):
     assert_lse_close(lse, want_lse)
 
 
+# deterministic backward: one head per CTA up to 739 tiles, two from 740 (an odd number of heads leaves a CTA with one)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H", [(9, 41), (10, 37)])
+def test_deterministic_backward_heads_per_cta(B, H, D):
+    from tests.helpers import assert_close, rand_inputs, random_meta
+    from kerneldev_b200 import flash_attention
+    T = 200
+    ins, sid, pre = random_meta(D, B, T)
+    q, k, v, do = rand_inputs(B, H, T, D, torch.bfloat16, D + B)
+    dev = [x.to(DEV).requires_grad_() for x in (q, k, v)]
+    o = flash_attention(*dev, deterministic=True, in_span=torch.as_tensor(ins, device=DEV), span_id=torch.as_tensor(sid, device=DEV),
+                        is_prefix=torch.as_tensor(pre, device=DEV))
+    grads = torch.autograd.grad(o, dev, do.to(DEV))
+    mask = torch.as_tensor(ao.dense_mask(T, ins, sid, pre))
+    for b, h in [(0, 0), (1, H - 1), (B - 1, 1), (B - 1, H - 1)]:
+        want = ao.attention_fwd_bwd(*(x[b:b + 1, h:h + 1].float() for x in (q, k, v, do)), mask[b:b + 1])
+        for name, got, ref in zip(("dQ", "dK", "dV"), grads, want[-3:]):
+            assert_close(name, got[b:b + 1, h:h + 1], ref)   # P and dS are rounded to 16 bits: the repository's tolerance for that
+
+
 # a row of exactly one chunk of 4096 tokens, one more, and several: first [CLS] in the first, a later, or no chunk
 @pytest.mark.parametrize("T", [1, 127, 4096, 4097, 12289])
 def test_metadata_chunks(T):
