@@ -38,7 +38,9 @@ __device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (e
 // Pairs of query tiles are split into items of one tile each while those have an SM each: two tiles' exponentials on one SM take turns
 // at its special-function units, and the other SMs have nothing to do. A call in a stream of them, pairs -> tiles (us, bf16): causal
 // 1 x 16 x 256 x 64 7.1 -> 6.2, 1 x 8 x 1000 x 64 18.7 -> 14.8, 1 x 4 x 4096 x 64 48.4 -> 37.7, 1 x 8 x 1024 x 128 18.2 -> 16.4, 74 pairs of T = 500 10.8 -> 9.5
-// (D = 64) and, 64 of them, 12.3 -> 12.3 (D = 128). With more pairs some SMs would have two items to others' one.
+// (D = 64) and, 64 of them, 12.3 -> 12.3 (D = 128). With 75 to 148 pairs some
+// SMs have two items to others' one: unequal lists still gain (causal, 80 and 128 pairs of T = 1000: 19.0 -> 15.5, 19.6 -> 16.1), equal ones lose
+// (no mask: 20.6 -> 25.6, 21.1 -> 26.6), and the lists are on the device. From 192 pairs on both lose.
 inline int split_pairs(int pairs, int tiles_per_head) { return tiles_per_head > 1 && 2 * pairs <= 148 ? 1 : 0; }
 
 // The producer warp: takes items (see the head of attn_fwd.cu), publishes their headers and lists and loads Q tiles and the rings of
