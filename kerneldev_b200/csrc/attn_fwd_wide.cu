@@ -212,6 +212,13 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             next_v();
             continue;
           }
+          // The two tiles of a CTA's first item would compute exponentials at the same time, with the special-function units idle
+          // between; half a unit apart they take turns. (With long lists that comes by itself, and the wait costs causal 8 x 16 x 2048 x 128
+          // 0.7 %.)
+          if (i == 1 && k == 0 && e == 0 && n <= 2) {
+            const uint32_t t0 = clock32();
+            while (clock32() - t0 < 900u) {}
+          }
           tc_fence_after_sync();
           const uint32_t klo = lo_k + kstage * T16;
 #pragma unroll
@@ -247,8 +254,8 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int c = n_seen - back;
       return c < 0 || wait(C::B_PVDONE + 2 * i + (c & 1), (c >> 1) & 1, W_F_PVDONE);
     };
-    // The next item's header, query descriptor and first unit are fetched before the epilogue of the item in hand, which hides their
-    // latency.
+    // The next item's header, query descriptor and first unit's mask are fetched before the epilogue of the item in hand, and for the first
+    // item before the wait for the kernel ahead, which hides their latency.
     int4 it = make_int4(0, 0, 0, 0);
     int n_next = 0, qi_next = 0;
     uint32_t qd_next = 0u, ent_next = 0u;   // the query descriptor and the first (then: the next) unit's entry
@@ -282,6 +289,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         todo &= ~__ballot_sync(0xffffffffu, mine);
       }
     };
+    uint32_t mk[NW] = {0u, 0u, 0u, 0u};   // of the coming unit, where it is PARTIAL
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
@@ -291,7 +299,10 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       qi_next = mine ? qtile * KD_TILE + row : INT_MAX;   // (written by the other item of the pair)
       qd_next = mine && qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
       list = sOwn + (k % C::NITEM) * 256 + i * 128;
-      if (n_next > 0) ent_next = list[0];
+      if (n_next > 0) {
+        ent_next = list[0];
+        if (ent_next & 0x100u) row_mask(ent_next & 0xFF, qd_next, qi_next, mk);
+      }
       return true;
     };
 
@@ -305,9 +316,6 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int u = 0; u < n_own; ++u) {
         const uint32_t ent = ent_next;
         if (u + 1 < n_own) ent_next = list[u + 1];
-        // the mask of a PARTIAL tile is formed while the scores are: the tile's products take longer
-        uint32_t mk[NW];
-        if (ent & 0x100u) row_mask(ent & 0xFF, qd, qi, mk);
         if (!(ok = wait(C::B_SFULL + i, n_seen & 1, W_F_SFULL))) break;
         tc_fence_after_sync();
         float sc[KD_TILE];
@@ -386,6 +394,8 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint64_t sum_pair = add_f32x2(sum2[0], sum2[1]);
         l += lo_f32x2(sum_pair) + hi_f32x2(sum_pair);
         ++n_seen;
+        // the mask of a PARTIAL tile is formed while its scores are: the tile's products take longer
+        if (u + 1 < n_own && (ent_next & 0x100u) != 0u) row_mask(ent_next & 0xFF, qd, qi, mk);
       }
       if (!ok) break;
       item_done(k);
@@ -393,27 +403,28 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
       // epilogue of this item: normalise, convert, store this thread's row of O, and LSE
       if (n_own > 0 && !(ok = pv_done(2) && pv_done(1))) break;
-      if (qi < a.T && a.lse != nullptr) a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
-      tc_fence_after_sync();
-      const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
-      uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)qi * a.o_st;
+      uint32_t r[HD / 32][32];   // (the scores' registers)
+      if (n_own > 0) {
+        tc_fence_after_sync();
 #pragma unroll
-      for (int cb = 0; cb < HD / 32; ++cb) {
-        uint32_t r[32];
-        if (n_own > 0) {
-          tmem_ld32(tO + cb * 32, r);
-          tmem_wait_ld();
-        } else {
+        for (int cb = 0; cb < HD / 32; ++cb) tmem_ld32(tO + cb * 32, r[cb]);
+        tmem_wait_ld();
+        // this thread's row of O_i has been read out: the next item's first product may overwrite it
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::B_OFREE + i));
+      } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = 0u;
-        }
-        if (cb == HD / 32 - 1 && n_own > 0) {
-          // this thread's row of O_i has been read out: the next item's first product may overwrite it
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(C::B_OFREE + i));
-        }
-        if (qi < a.T) store_row32_upto<kBf16>(orow + cb * 32, r, inv_l, cb * 32, a.d_real);
+        for (int cb = 0; cb < HD / 32; ++cb)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[cb][j] = 0u;
+      }
+      if (qi < a.T) {
+        const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
+        uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)qi * a.o_st;
+#pragma unroll
+        for (int cb = 0; cb < HD / 32; ++cb) store_row32_upto<kBf16>(orow + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
+        if (a.lse != nullptr) a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
       }
     }  // items
   }
