@@ -63,7 +63,8 @@ struct FwdCfg {
   static constexpr int NBUF = 3;                         // score buffers in TMEM
   static constexpr int KST = NBUF;                       // K ring stages
   static constexpr int VST = 3;                          // V ring stages
-  static constexpr int NQ = 4;                           // ring of Q tiles (two per item): the next item's Q loads while this one computes
+  using QR = FwdQRing;                                   // ring of Q tiles (two per item): four slots, the next item's Q loads while this one computes
+  static constexpr int NQ = QR::SLOTS;
   static constexpr int NPART = 2;                        // P is handed over in two parts: the first, then the second 32 columns of each half
   static constexpr int NITEM = 4;                        // ring of item headers and lists
   static constexpr int NXB = 2;                          // buffers of the row maxima that two warps exchange (see there)
@@ -76,7 +77,7 @@ struct FwdCfg {
   static constexpr int SMEM_CLC = SMEM_XCH + NXB * 4 * KD_TILE * 4;
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
   // barriers (8 bytes each)
-  static constexpr int B_QFULL = 0, B_QEMPTY = B_QFULL + NQ, B_KFULL = B_QEMPTY + NQ, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST,
+  static constexpr int B_QFULL = 0, B_QEMPTY = B_QFULL + QR::FULL, B_KFULL = B_QEMPTY + NQ, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST,
                        B_VEMPTY = B_VFULL + VST, B_SFULL = B_VEMPTY + VST, B_PFULL = B_SFULL + 2 * NBUF,
                        B_PVDONE = B_PFULL + NPART * NBUF, B_OFREE = B_PVDONE + 4, B_ITEMFULL = B_OFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
                        B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;

@@ -1,6 +1,7 @@
 // Declarations and the producer warp shared by the forward kernels (attn_fwd.cu for head dims up to 64, attn_fwd_wide.cu above).
 #pragma once
 #include "attn_common.cuh"
+#include "fwd_rules.cuh"
 
 namespace kd {
 
@@ -61,6 +62,8 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
     tma_prefetch_desc(&tmV);
   }
   int q_cnt = 0, kv_cnt = 0, v_cnt = 0, k = 0, asked = 0;   // Q, K, V tiles requested, items published, cancellations asked for
+  PhaseBits q_phases;   // of the Q tiles' "full" barriers
+  uint32_t q_used = 0u;
   int k_dropped = -1;   // index of a K tile that was never requested (test builds only)
   bool ok = true, pending = false;
   uint32_t lst[4];      // the next item's list, 32 entries per register
@@ -136,9 +139,11 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
     ++k;
     const int ntile_q = (2 * pair + 1 < a.NT) ? 2 : 1;
     auto load_q = [&](int t) -> bool {
-      const int s = q_cnt % C::NQ;
-      if (!wait(C::B_QEMPTY + s, ((q_cnt / C::NQ) & 1) ^ 1, W_F_QEMPTY)) return false;
-      load_tile(&tmQ, sQ + s * TILE, C::B_QFULL + s, 2 * pair + t, h, b);
+      const int s = C::QR::slot(q_cnt), full = C::QR::full(q_cnt, t);
+      if (!wait(C::B_QEMPTY + s, C::QR::empty_parity(q_cnt), W_F_QEMPTY)) return false;
+      load_tile(&tmQ, sQ + s * TILE, C::B_QFULL + full, 2 * pair + t, h, b);
+      q_phases.take(full);
+      q_used |= 1u << full;
       ++q_cnt;
       return true;
     };
@@ -181,7 +186,8 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
     for (int e = max(0, kv_cnt - C::KST); e < kv_cnt; ++e)
       if (e != k_dropped) drain_wait(bar(C::B_KFULL + e % C::KST), (e / C::KST) & 1);
     for (int e = max(0, v_cnt - C::VST); e < v_cnt; ++e) drain_wait(bar(C::B_VFULL + e % C::VST), (e / C::VST) & 1);
-    for (int e = max(0, q_cnt - C::NQ); e < q_cnt; ++e) drain_wait(bar(C::B_QFULL + e % C::NQ), (e / C::NQ) & 1);
+    for (int f = 0; f < C::QR::FULL; ++f)
+      if ((q_used >> f) & 1u) drain_wait(bar(C::B_QFULL + f), q_phases.last(f));
     if (pending) drain_wait(bar(C::B_CLC), (asked - 1) & 1);
   }
 }

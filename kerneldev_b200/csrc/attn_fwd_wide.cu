@@ -30,7 +30,8 @@ struct FwdWideCfg {
   static constexpr int KBLK = HD / 64;                   // 64-element blocks along D
   static constexpr int TILE_BYTES = KD_TILE * HD * 2;    // one Q / K / V tile
   static constexpr int KST = 2, VST = 2;                 // K and V ring stages
-  static constexpr int NQ = 3;                           // ring of Q tiles (two per item)
+  using QR = FwdWideQRing;                               // ring of Q tiles (two per item): three slots, a "full" barrier per slot and issuing warp
+  static constexpr int NQ = QR::SLOTS;
   static constexpr int NPART = 2;                        // P is handed over in two halves of the keys
   static constexpr int NITEM = 2;                        // ring of item headers and lists
   static constexpr int SMEM_Q = 0;
@@ -42,7 +43,7 @@ struct FwdWideCfg {
   static constexpr int SMEM_CLC = SMEM_ITEM + NITEM * 16;
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
   // barriers (8 bytes each)
-  static constexpr int B_QFULL = 0, B_QEMPTY = B_QFULL + NQ, B_KFULL = B_QEMPTY + NQ, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST,
+  static constexpr int B_QFULL = 0, B_QEMPTY = B_QFULL + QR::FULL, B_KFULL = B_QEMPTY + NQ, B_KEMPTY = B_KFULL + KST, B_VFULL = B_KEMPTY + KST,
                        B_VEMPTY = B_VFULL + VST, B_SFULL = B_VEMPTY + VST, B_PFULL = B_SFULL + 2, B_PVDONE = B_PFULL + NPART * 2,
                        B_OFREE = B_PVDONE + 4, B_ITEMFULL = B_OFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM, B_CLC = B_ITEMEMPTY + NITEM,
                        NBAR = B_CLC + 1;
@@ -150,6 +151,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       constexpr uint32_t T16 = TILE >> 4;
       int kstage = 0, vstage = 0, q_cnt = 0;
       uint32_t kparity = 0u, vparity = 0u, pv_cnt = 0u, o_cnt = 0u;   // P V products issued; items with units
+      PhaseBits q_phases;   // of this query tile's barriers
       bool first = false;   // no P V of the item has been issued
       auto next_k = [&]() { if (++kstage == C::KST) { kstage = 0; kparity ^= 1u; } };
       auto next_v = [&]() { if (++vstage == C::VST) { vstage = 0; vparity ^= 1u; } };
@@ -183,9 +185,10 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (k == 0) pdl_wait();
         const int n = it.w & 0xFF, ntile_q = (2 * it.z + 1 < a.NT) ? 2 : 1;
         int left = (it.w >> (8 + 8 * i)) & 0xFF;   // units without scores
-        const int q_slot = (q_cnt + i) % C::NQ;
+        const int q_slot = C::QR::slot(q_cnt + i);
         if (i < ntile_q) {
-          if (!(ok = wait(C::B_QFULL + q_slot, ((q_cnt + i) / C::NQ) & 1, W_F_QFULL))) break;
+          const int full = C::QR::full(q_cnt + i, i);
+          if (!(ok = wait(C::B_QFULL + full, q_phases.take(full), W_F_QFULL))) break;
           if (left == 0 && elect_one()) mbar_arrive(bar(C::B_QEMPTY + q_slot));
         }
         q_cnt += ntile_q;

@@ -101,6 +101,31 @@ def test_forward_wide_unequal_lists_of_a_pair(T, length, D, dtype):
     assert_lse_close(lse, want_lse)
 
 
+# Forward above head dim 64 with more items than SMs, whose lists hold 0, 1 or 2 entries (T = 256) or up to 3 (T = 300: a pair without a second
+# tile) and whose tile 1 often has none: the ring of Q tiles passes from one query tile's issuing warp to the other's. Repeats give the same bits
+@pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (80, torch.float16)])
+@pytest.mark.parametrize("T", [256, 300])
+def test_forward_wide_ring_of_query_tiles(T, D, dtype):
+    from tests.helpers import assert_close, assert_lse_close
+    from kerneldev_b200 import flash_attention
+    B, H = 40, 37
+    lens = np.array([(T, 100, 0, 129)[b % 4] for b in range(B)], np.int32)
+    g = torch.Generator(device=DEV).manual_seed(T + D)
+    q, k, v = (torch.randn((B, H, T, D), generator=g, device=DEV).to(dtype) for _ in range(3))
+    call = lambda: flash_attention(q, k, v, return_lse=True, lens=torch.as_tensor(lens, device=DEV))
+    with torch.no_grad():
+        o, lse = call()
+        for _ in range(20):
+            o2, lse2 = call()
+            assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    pick = [(b, h) for b in range(4) for h in (0, 18, H - 1)] + [(B - 1, H - 1)]
+    sel = lambda x: torch.stack([x[b, h] for b, h in pick])[:, None].float().cpu()
+    mask = torch.as_tensor(ao.dense_mask(T, lens=lens, causal=True))
+    want_o, want_lse = ao.attention_forward(sel(q), sel(k), sel(v), torch.stack([mask[b] for b, _ in pick]))
+    assert_close("O", sel(o), want_o)   # P is rounded to 16 bits before its product: the repository's tolerance for that
+    assert_lse_close(sel(lse), want_lse)
+
+
 # Forward items of one query tile (up to 74 pairs of tiles in a call) and of two (75): pairs with a second tile, without one (T = 300),
 # and with entries of the list that are EMPTY for one of them; rows beyond the sequence length; one tile per head is not split
 @pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (112, torch.float16)])
