@@ -33,9 +33,6 @@ enum : uint32_t {
   W_F_ITEMFULL = 0x10C, W_F_ITEMEMPTY = 0x10D, W_F_CLC = 0x10E, W_F_ALIGN = 0x10F,
 };
 
-// list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10
-__device__ __forceinline__ uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
-
 // Pairs of query tiles are split into items of one tile each while those have an SM each: two tiles' exponentials on one SM take turns
 // at its special-function units, and the other SMs have nothing to do. A call in a stream of them, pairs -> tiles (us, bf16): causal
 // 1 x 16 x 256 x 64 7.1 -> 6.2, 1 x 8 x 1000 x 64 18.7 -> 14.8, 1 x 4 x 4096 x 64 48.4 -> 37.7, 1 x 8 x 1024 x 128 18.2 -> 16.4, 74 pairs of T = 500 10.8 -> 9.5
@@ -85,7 +82,7 @@ __device__ __forceinline__ void fwd_producer(const CUtensorMap& tmQ, const CUten
       it.w = 0;
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
-        lst[r] = entry_class(lst[r], only - 1) != 0u ? lst[r] & (only == 1 ? 0x3FFu : 0xCFFu) : 0u;
+        lst[r] = entry_of_tile(lst[r], only - 1);
         it.w += __popc(__ballot_sync(0xffffffffu, lst[r] != 0u));
       }
     }

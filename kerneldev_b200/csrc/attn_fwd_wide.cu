@@ -215,10 +215,9 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             next_v();
             continue;
           }
-          // The two tiles of a CTA's first item would compute exponentials at the same time, with the special-function units idle
-          // between; half a unit apart they take turns. (With long lists that comes by itself, and the wait costs causal 8 x 16 x 2048 x 128
-          // 0.7 %.)
-          if (i == 1 && k == 0 && e == 0 && n <= 2) {
+          // Tile 1's exponentials half a unit behind tile 0's. (With long lists that comes by itself, and the wait costs causal
+          // 8 x 16 x 2048 x 128 0.7 %.)
+          if (i == 1 && k == 0 && e == 0 && tiles_take_turns(ent, n)) {
             const uint32_t t0 = clock32();
             while (clock32() - t0 < 900u) {}
           }

@@ -37,6 +37,17 @@ struct PhaseBits {
   KD_HOST_DEVICE uint32_t last(int j) const { return ((next >> j) & 1u) ^ 1u; }   // of the phase taken last
 };
 
+// A list entry: key tile | class for query tile 0 << 8 | class for query tile 1 << 10 (class 0: EMPTY).
+KD_HOST_DEVICE uint32_t entry_class(uint32_t ent, int i) { return (ent >> (8 + 2 * i)) & 3u; }
+// What is left of an entry in an item of query tile i alone: 0 where that tile does not need it.
+KD_HOST_DEVICE uint32_t entry_of_tile(uint32_t ent, int i) { return entry_class(ent, i) != 0u ? ent & (i == 0 ? 0x3FFu : 0xCFFu) : 0u; }
+
+// Head dims above 64: do the two tiles of a CTA's first item, of n entries with `first` ahead, begin half a unit apart? With lists of
+// one or two entries they would compute their exponentials at the same time, with the special-function units idle before and after.
+// Where only one tile begins with the entry there is nothing to take turns with, and the half unit would be lost (20 calls in a graph, items of
+// one tile, us a call: causal 1 x 16 x 173 x 128 7.4 -> 6.9, no mask 1 x 16 x 256 x 128 7.6 -> 7.1, hierarchical 2 x 16 x 256 x 96 6.3 -> 5.9).
+KD_HOST_DEVICE bool tiles_take_turns(uint32_t first, int n) { return n <= 2 && entry_class(first, 0) != 0u && entry_class(first, 1) != 0u; }
+
 using FwdWideQRing = QRing<3, 2>;   // head dims above 64 (shared memory has room for three tiles)
 using FwdQRing = QRing<4, 1>;       // head dims up to 64
 

@@ -1,9 +1,10 @@
-// Host-side model of the Q tile hand-over in the forward kernel for head dims above 64 (fwd_rules.cuh, attn_fwd.cuh, attn_fwd_wide.cu):
-// the producer, two issuing warps that run ahead of each other, and copies that land in any order. Every product must read
+// Host-side checks of the forward kernels' rules (fwd_rules.cuh). Built and run by tests/test_host_logic.py (host code only; no GPU needed).
+//
+// 1. A model of the Q tile hand-over in the kernel for head dims above 64 (attn_fwd.cuh, attn_fwd_wide.cu): the producer, two issuing warps that run ahead of each other, and copies that land in any order. Every product must read
 // the tile it is meant for, landed, and no slot may be released or filled before that. Random schedules of random items, among
 // them items whose tiles have no units, odd last tiles and lists of up to four entries. With one "full" barrier per slot, which a warp
 // then does not see all phases of, the model must find the wrong product (the check of the model itself).
-// Built and run by tests/test_host_logic.py (host code only; no GPU needed).
+// 2. Entries of an item of one query tile, and which items' tiles begin half a unit apart.
 #include <cstdio>
 #include <cstdint>
 #include <vector>
@@ -145,8 +146,24 @@ static const char* run(uint64_t seed) {   // nullptr: no fault
   return nullptr;
 }
 
+static int list_rules() {   // mistakes
+  int bad = 0;
+  for (uint32_t kt = 0; kt < 128; ++kt)
+    for (uint32_t c0 = 0; c0 < 3; ++c0)
+      for (uint32_t c1 = 0; c1 < 3; ++c1) {
+        const uint32_t ent = kt | (c0 << 8) | (c1 << 10), cls[2] = {c0, c1};
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t one = entry_of_tile(ent, i);
+          bad += cls[i] == 0u ? one != 0u : (one & 0xFFu) != kt || entry_class(one, i) != cls[i] || entry_class(one, 1 - i) != 0u;
+          for (int n = 1; n <= 3; ++n) bad += tiles_take_turns(one, n);   // alone on its SM
+        }
+        for (int n = 1; n <= 3; ++n) bad += tiles_take_turns(ent, n) != (n <= 2 && c0 != 0u && c1 != 0u);
+      }
+  return bad;
+}
+
 int main() {
-  int bad = 0, found = 0;
+  int bad = list_rules(), found = 0;
   for (uint64_t seed = 1; seed <= 20000; ++seed) {
     const char* e = run<AsBuilt>(seed);
     if (e != nullptr && bad++ == 0) printf("seed %llu: %s\n", static_cast<unsigned long long>(seed), e);
