@@ -920,7 +920,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   BwdArgs a;
   a.B = p.B; a.H = p.H; a.T = p.T; a.NT = L.NT; a.NP = L.NP; a.Tpad = L.NT * KD_TILE;
   a.d_real = p.D;
-  a.scale_log2 = p.sm_scale * 1.4426950408889634f;
+  a.scale_log2 = scale_log2_of(p.sm_scale);
   a.sm_scale = p.sm_scale;
   a.G = heads_per_cta(p.B, p.H, L.NT, p.heads_per_cta);
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;

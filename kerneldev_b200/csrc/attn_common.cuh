@@ -4,6 +4,7 @@
 #pragma once
 #include <algorithm>
 #include <atomic>
+#include <cfloat>
 
 #include "common.cuh"
 #include "mask_rule.cuh"
@@ -20,6 +21,10 @@
 #endif
 
 namespace kd {
+
+// The factor of the scores in base 2. The kernels flush numbers below FLT_MIN to zero, and a factor of zero makes NaN of a hidden
+// score and of a row maximum without keys (-inf both); raised to FLT_MIN it leaves every exponential at 1, as the smaller one would.
+inline float scale_log2_of(float sm_scale) { return std::max(sm_scale * 1.4426950408889634f, FLT_MIN); }
 
 // High words of the two descriptor kinds used here (layout, version, stride byte offset 1024);
 // the low word carries the start address and the leading byte offset.

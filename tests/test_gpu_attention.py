@@ -106,6 +106,16 @@ def test_explicit_scale(scale):
     compare(q, k, v, do, ao.dense_mask(T, ins, sid, pre), run_op(q, k, v, do, ins, sid, pre, scale=scale), scale)
 
 
+# a scale that the kernels' arithmetic flushes to zero: uniform attention over the visible keys
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.float16)])
+@pytest.mark.parametrize("causal,deterministic", [(False, False), (True, False), (True, True)])
+def test_subnormal_scale(D, dtype, causal, deterministic):
+    B, H, T = 2, 2, 300
+    q, k, v, do = rand_inputs(B, H, T, D, dtype, seed=D)
+    got = run_op(q, k, v, do, causal=causal, scale=1e-40, deterministic=deterministic)
+    compare(q, k, v, do, ao.dense_mask(T, causal=causal, B=B), got, 1e-40)
+
+
 def test_medium_hierarchical_config2_like():
     B, H, T, D = 2, 4, 2048, 64
     ins, sid, pre, lens = ao.batch_metadata(4, B, T, **ao.CONFIG_RANGES[4])
