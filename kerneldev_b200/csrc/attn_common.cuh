@@ -177,6 +177,15 @@ __device__ __forceinline__ void store_row16_upto(uint16_t* dst, const uint32_t (
   if (col < d_real) store_row16<kBf16>(dst, r, f);
 }
 
+// SMs of the device that was current at the first call (the devices of a machine are alike: the library runs on sm_100 alone).
+inline int sm_count() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
+  }();
+  return n;
+}
+
 // Heads a CTA handles one after the other (they share the plan's work list, so the list staging,
 // the TMEM allocation and the pipeline fill are paid once): as many as keeps about per_sm CTAs per SM,
 // at most g_max (the longest-first dispatch order keeps the SMs balanced with that few). Measured best for the
@@ -187,15 +196,9 @@ __device__ __forceinline__ void store_row16_upto(uint16_t* dst, const uint32_t (
 // 5.2: 142 -> 131, 6.9: 191 -> 175, 10.4: 302 -> 279; causal T = 1000, D = 64, 3.5: 81 -> 72, 6.9: 156 -> 147.
 inline int heads_per_cta(int B, int H, int items_per_batch, int forced, int per_sm = 6, int g_max = 8) {
   if (forced >= 1) return forced < H ? forced : H;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-      sm_count = 148;
-  }
-  const long long ctas = (long long)B * H * items_per_batch;
-  long long g = ctas / ((long long)sm_count * per_sm);
-  if (g < 2) g = ctas >= 5LL * sm_count ? 2 : 1;
+  const long long ctas = (long long)B * H * items_per_batch, sms = sm_count();
+  long long g = ctas / (sms * per_sm);
+  if (g < 2) g = ctas >= 5 * sms ? 2 : 1;
   if (g > g_max) g = g_max;
   if (g > H) g = H;
   return static_cast<int>(g);

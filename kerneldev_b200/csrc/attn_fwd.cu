@@ -615,7 +615,7 @@ int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
   a.B = p.B; a.H = p.H; a.T = p.T; a.NT = L.NT; a.NP = L.NP; a.Tpad = L.NT * KD_TILE;
   a.d_real = p.D;
   a.scale_log2 = scale_log2_of(p.sm_scale);
-  a.split = split_pairs(static_cast<int>(std::min<long long>((long long)p.B * p.H * L.NP, INT_MAX / 2)), L.NT);
+  a.split = split_pairs((long long)p.B * p.H * L.NP, L.NT, sm_count());
   const long long n_items = ((long long)p.B * p.H * L.NP) << a.split;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 256) exceeds 2^31 - 1");
   // Q, K, V and O. (64 and 110 MB: no difference outside the noise)

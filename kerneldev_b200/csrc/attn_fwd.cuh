@@ -2,6 +2,7 @@
 #pragma once
 #include "attn_common.cuh"
 #include "fwd_rules.cuh"
+#include "launch_rules.cuh"
 
 namespace kd {
 
@@ -17,7 +18,7 @@ struct FwdArgs {
   const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length
   uint32_t* status;
   int plan_ready;
-  int split;         // 1: an item is one query tile of a pair (see split_pairs)
+  int split;         // 1: an item is one query tile of a pair (see launch_rules.cuh)
   void* o;
   int64_t o_sb, o_sh, o_st;
   float* lse;
@@ -32,14 +33,6 @@ enum : uint32_t {
   W_F_PFULL = 0x106, W_F_SFULL = 0x107, W_F_PVDONE = 0x108, W_F_QEMPTY = 0x10A, W_F_OFREE = 0x10B,
   W_F_ITEMFULL = 0x10C, W_F_ITEMEMPTY = 0x10D, W_F_CLC = 0x10E, W_F_ALIGN = 0x10F,
 };
-
-// Pairs of query tiles are split into items of one tile each while those have an SM each: two tiles' exponentials on one SM take turns
-// at its special-function units, and the other SMs have nothing to do. A call in a stream of them, pairs -> tiles (us, bf16): causal
-// 1 x 16 x 256 x 64 7.1 -> 6.2, 1 x 8 x 1000 x 64 18.7 -> 14.8, 1 x 4 x 4096 x 64 48.4 -> 37.7, 1 x 8 x 1024 x 128 18.2 -> 16.4, 74 pairs of T = 500 10.8 -> 9.5
-// (D = 64) and, 64 of them, 12.3 -> 12.3 (D = 128). With 75 to 148 pairs some
-// SMs have two items to others' one: unequal lists still gain (causal, 80 and 128 pairs of T = 1000: 19.0 -> 15.5, 19.6 -> 16.1), equal ones lose
-// (no mask: 20.6 -> 25.6, 21.1 -> 26.6), and the lists are on the device. From 192 pairs on both lose.
-inline int split_pairs(int pairs, int tiles_per_head) { return tiles_per_head > 1 && 2 * pairs <= 148 ? 1 : 0; }
 
 // The producer warp: takes items (see the head of attn_fwd.cu), publishes their headers and lists and loads Q tiles and the rings of
 // K and V tiles by TMA. C: the kernel's configuration. wait(barrier, parity, site): a warp's bounded wait. publish(slot, lst, n,

@@ -5,10 +5,13 @@
 // them items whose tiles have no units, odd last tiles and lists of up to four entries. With one "full" barrier per slot, which a warp
 // then does not see all phases of, the model must find the wrong product (the check of the model itself).
 // 2. Entries of an item of one query tile, and which items' tiles begin half a unit apart.
+// 3. Which calls have items of one query tile (launch_rules.cuh): never more items than SMs, and none beyond half of the SMs where the
+//    lists are short.
 #include <cstdio>
 #include <cstdint>
 #include <vector>
 #include "../kerneldev_b200/csrc/fwd_rules.cuh"
+#include "../kerneldev_b200/csrc/launch_rules.cuh"
 
 using namespace kd;
 
@@ -162,8 +165,20 @@ static int list_rules() {   // mistakes
   return bad;
 }
 
+static int split_rule() {   // mistakes
+  int bad = 0;
+  for (long long pairs = 1; pairs <= 400; ++pairs)
+    for (int tiles = 1; tiles <= 128; ++tiles) {
+      const long long items = 2 * pairs;
+      const int split = split_pairs(pairs, tiles, 148);
+      bad += split && (tiles == 1 || items > 148 || (tiles < 5 && items > 74));
+      bad += !split && tiles > 1 && items <= (tiles < 5 ? 74 : 148);
+    }
+  return bad + split_pairs(1LL << 40, 128, 148);
+}
+
 int main() {
-  int bad = list_rules(), found = 0;
+  int bad = list_rules() + split_rule(), found = 0;
   for (uint64_t seed = 1; seed <= 20000; ++seed) {
     const char* e = run<AsBuilt>(seed);
     if (e != nullptr && bad++ == 0) printf("seed %llu: %s\n", static_cast<unsigned long long>(seed), e);

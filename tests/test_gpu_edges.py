@@ -126,10 +126,12 @@ def test_forward_wide_ring_of_query_tiles(T, D, dtype):
     assert_lse_close(sel(lse), want_lse)
 
 
-# Forward items of one query tile (up to 74 pairs of tiles in a call) and of two (75): pairs with a second tile, without one (T = 300),
-# and with entries of the list that are EMPTY for one of them; rows beyond the sequence length; one tile per head is not split
+# Forward items of one query tile (up to 37 pairs of tiles in a call, from five tiles per head on up to 74) and of two (38; 75): pairs with a
+# second tile, without one (T = 300, 640), and with entries of the list that are EMPTY for one of them; rows beyond the sequence length; one tile
+# per head is not split
 @pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (112, torch.float16)])
-@pytest.mark.parametrize("B,H,T", [(2, 37, 200), (3, 25, 200), (1, 37, 300), (2, 2, 128 * 9 + 1), (74, 1, 100)])
+@pytest.mark.parametrize("B,H,T", [(1, 37, 200), (2, 19, 200), (2, 37, 200), (3, 25, 200), (1, 18, 300), (1, 37, 300), (4, 6, 640), (2, 7, 128 * 9 + 1),
+                                   (3, 5, 128 * 9 + 1), (2, 2, 128 * 9 + 1), (74, 1, 100)])
 def test_forward_items_of_one_tile(B, H, T, D, dtype):
     from tests.helpers import assert_close, assert_lse_close, random_meta, rand_inputs
     from kerneldev_b200 import flash_attention
