@@ -922,7 +922,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   a.d_real = p.D;
   a.scale_log2 = scale_log2_of(p.sm_scale);
   a.sm_scale = p.sm_scale;
-  a.G = heads_per_cta(p.B, p.H, L.NT, p.heads_per_cta);
+  a.G = heads_per_cta((long long)p.B * p.H, p.H, L.NT, p.heads_per_cta, sm_count());
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
   a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;

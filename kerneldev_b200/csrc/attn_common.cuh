@@ -7,6 +7,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "launch_rules.cuh"
 #include "mask_rule.cuh"
 #include "sm100_prims.cuh"
 
@@ -184,24 +185,6 @@ inline int sm_count() {
     return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
   }();
   return n;
-}
-
-// Heads a CTA handles one after the other (they share the plan's work list, so the list staging,
-// the TMEM allocation and the pipeline fill are paid once): as many as keeps about per_sm CTAs per SM,
-// at most g_max (the longest-first dispatch order keeps the SMs balanced with that few). Measured best for the
-// deterministic backward: 6 per SM, up to 8 heads. Fewer CTAs than that lose more to imbalance between sequences of
-// different section lengths than the shared pipeline fill saves; but two heads pay from five tiles per SM on, that is with 2.5 CTAs
-// per SM, for a CTA's start and drain (6 us) are as long as its work there. Whole backward, one head -> two (us): hierarchical
-// T = 2048, D = 64, with 3.5 tiles per SM 66 -> 77, 4.3: 79 -> 78, 5.2: 92 -> 84, 6.9: 124 -> 111, 10.4: 198 -> 178; D = 128, 3.5: 101 -> 121,
-// 5.2: 142 -> 131, 6.9: 191 -> 175, 10.4: 302 -> 279; causal T = 1000, D = 64, 3.5: 81 -> 72, 6.9: 156 -> 147.
-inline int heads_per_cta(int B, int H, int items_per_batch, int forced, int per_sm = 6, int g_max = 8) {
-  if (forced >= 1) return forced < H ? forced : H;
-  const long long ctas = (long long)B * H * items_per_batch, sms = sm_count();
-  long long g = ctas / (sms * per_sm);
-  if (g < 2) g = ctas >= 5 * sms ? 2 : 1;
-  if (g > g_max) g = g_max;
-  if (g > H) g = H;
-  return static_cast<int>(g);
 }
 
 // Order of a launch's items (tiles of one (batch, head) pair): chunks of heads whose tensors share L2, inside a chunk rank by

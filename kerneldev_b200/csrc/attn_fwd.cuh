@@ -2,7 +2,6 @@
 #pragma once
 #include "attn_common.cuh"
 #include "fwd_rules.cuh"
-#include "launch_rules.cuh"
 
 namespace kd {
 

@@ -1,4 +1,4 @@
-// Host-side checks of the forward kernels' rules (fwd_rules.cuh). Built and run by tests/test_host_logic.py (host code only; no GPU needed).
+// Host-side checks of the kernels' rules (fwd_rules.cuh, launch_rules.cuh). Built and run by tests/test_host_logic.py (host code only; no GPU needed).
 //
 // 1. A model of the Q tile hand-over in the kernel for head dims above 64 (attn_fwd.cuh, attn_fwd_wide.cu): the producer, two issuing warps that run ahead of each other, and copies that land in any order. Every product must read
 // the tile it is meant for, landed, and no slot may be released or filled before that. Random schedules of random items, among
@@ -7,6 +7,8 @@
 // 2. Entries of an item of one query tile, and which items' tiles begin half a unit apart.
 // 3. Which calls have items of one query tile (launch_rules.cuh): never more items than SMs, and none beyond half of the SMs where the
 //    lists are short.
+// 4. Heads per CTA of the deterministic backward (launch_rules.cuh): one or two up to twelve tiles per SM, and two only where lists are short
+//    or the tiles many.
 #include <cstdio>
 #include <cstdint>
 #include <vector>
@@ -177,8 +179,21 @@ static int split_rule() {   // mistakes
   return bad + split_pairs(1LL << 40, 128, 148);
 }
 
+static int heads_rule() {   // mistakes
+  int bad = 0;
+  for (int tiles = 1; tiles <= 128; ++tiles)
+    for (long long pairs = 1; pairs * tiles < 12 * 148; ++pairs) {
+      const int g = heads_per_cta(pairs, 16, tiles, 0, 148);
+      const long long ctas = pairs * tiles;
+      bad += g < 1 || g > 2 || (g == 2 && (ctas < 740 || tiles > 32 || (tiles > 20 && ctas < 1036)));
+      bad += g == 1 && tiles <= 20 && ctas >= 740;
+      bad += heads_per_cta(pairs, 1, tiles, 0, 148) != 1 || heads_per_cta(pairs, 16, tiles, 3, 148) != 3 || heads_per_cta(pairs, 2, tiles, 3, 148) != 2;
+    }
+  return bad + (heads_per_cta(1LL << 24, 16, 128, 0, 148) != 8);
+}
+
 int main() {
-  int bad = list_rules() + split_rule(), found = 0;
+  int bad = list_rules() + split_rule() + heads_rule(), found = 0;
   for (uint64_t seed = 1; seed <= 20000; ++seed) {
     const char* e = run<AsBuilt>(seed);
     if (e != nullptr && bad++ == 0) printf("seed %llu: %s\n", static_cast<unsigned long long>(seed), e);

@@ -92,10 +92,10 @@ def test_bit_parallel_rule_equals_per_element_rule(tmp_path):
 
 
 @pytest.mark.skipif(shutil.which("nvcc") is None and not os.path.exists("/usr/local/cuda/bin/nvcc"), reason="needs nvcc to compile host code")
-def test_forward_rules_and_q_tile_hand_over_in_any_landing_order(tmp_path):
+def test_launch_rules_and_q_tile_hand_over_in_any_landing_order(tmp_path):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    exe = tmp_path / "fwd_rules_check"
-    r = subprocess.run([nvcc, "-O1", "-o", str(exe), os.path.join(ROOT, "tests", "fwd_rules_check.cu")], capture_output=True, text=True)
+    exe = tmp_path / "launch_rules_check"
+    r = subprocess.run([nvcc, "-O1", "-o", str(exe), os.path.join(ROOT, "tests", "launch_rules_check.cu")], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
