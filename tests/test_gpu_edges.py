@@ -78,13 +78,15 @@ def test_many_items_per_cta_with_empty_ones_between(monkeypatch, T, n_full, D, d
 # Forward above head dim 64: an issuing warp per query tile walks a common list. A tile of prefix tokens in the middle of the
 # sequence sees the prefix only, its pair's other tile nearly everything: runs of entries of one tile, longer than the rings of
 # K and V tiles, for tile 1 of a pair (tile 8) and for tile 0 (tile 13); a tile beyond the sequence length; an odd number of tiles;
-# scores whose maximum grows from tile to tile (O is rescaled)
+# scores whose maximum grows from tile to tile (O is rescaled). With six heads a call has 84 or 96 pairs, which are its items; with three, 42 or
+# 48, whose tiles are items of their own
+@pytest.mark.parametrize("H", [6, 3])
 @pytest.mark.parametrize("D,dtype", [(128, torch.bfloat16), (80, torch.float16)])
 @pytest.mark.parametrize("T,length", [(128 * 14, 128 * 14), (128 * 15 - 127, 128 * 14 + 1), (128 * 14 + 5, 128 * 12)])
-def test_forward_wide_unequal_lists_of_a_pair(T, length, D, dtype):
+def test_forward_wide_unequal_lists_of_a_pair(T, length, D, dtype, H):
     from tests.helpers import assert_close, assert_lse_close
     from kerneldev_b200 import flash_attention
-    B, H = 2, 3
+    B = 2
     ins, sid, pre = np.zeros((B, T), bool), np.zeros((B, T), np.int64), np.zeros((B, T), bool)
     for tile in (0, 8, 13):
         pre[:, tile * 128:(tile + 1) * 128] = True
