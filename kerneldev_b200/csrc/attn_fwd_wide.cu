@@ -13,7 +13,8 @@
 // What bounds it: with long lists the power limit (bf16 causal 16 x 16384 x 128 runs at 1,600 MHz) and the chain above, of which 1,024
 // cycles are the products and 1,024 the exponentials of a tile. A thread per row needs no exchange of row maxima and executes three
 // quarters of the instructions that two threads per row do, and an issuing warp per tile does not make one tile's products wait
-// for the other tile's P. Against sixteen softmax warps and one issuing warp (us, at 1,600-1,680 MHz under the power limit):
+// for the other tile's P. Against sixteen softmax warps and one issuing warp (us, normally distributed inputs, at 1,600-1,680 MHz under the power
+// limit; with outliers, whose sparse P draws less power, hierarchical 4 x 32 x 8192 x 128 955 -> 963):
 //   bf16 causal 16 x 16384 x 128 977 -> 916          fp16 hierarchical 4 x 32 x 8192 x 128 1363 -> 1290
 //   bf16 full 2 x 16 x 4096 x 128 280 -> 260         bf16 causal 8 x 16 x 2048 x 128 156 -> 157
 // Masks formed after the scores had been loaded, from descriptors held in registers since the unit before: 916 -> 942 (registers).
