@@ -155,6 +155,22 @@ int kd_attn_fwd(const kd_attn_params* p, void* stream);
  * with its dQ and dK/dV workers (:713-838, :1173-1525). */
 int kd_attn_bwd(const kd_attn_params* p, void* stream);
 
+/* float32 tensors of a call whose operands are float16 copies (p->dtype KD_F16; see kd_cast): what the kernels of the call read or
+ * write of them directly, in place of a conversion before or behind. Pointers and byte strides multiples of 16. No counterpart in the
+ * reference, whose float32 path multiplies in tf32. */
+typedef struct kd_attn_f32 {
+  kd_tensor o;          /* kd_attn_fwd_f32: out, not rounded to 16 bits */
+  kd_tensor d_o;        /* kd_attn_bwd_f32: in; ptr NULL when p->d_o holds dO in 16 bits already */
+  kd_tensor dq, dk, dv; /* kd_attn_bwd_f32: out */
+} kd_attn_f32;
+
+/* kd_attn_fwd with O written as float32. p->o may have a NULL ptr: the 16-bit O, which a backward wants, is not written then. */
+int kd_attn_fwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream);
+
+/* kd_attn_bwd with dO read and dQ, dK, dV written as float32; p->dq, p->dk and p->dv are ignored. With f->d_o, p->d_o is a 16-bit
+ * scratch tensor that the delta kernel (bwd_phases 1 or 0) fills. KD_BWD_FUSED adds dQ into f->dq itself and needs no dq_acc. */
+int kd_attn_bwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream);
+
 /* kd_attn_bwd without any caller-provided scratch. This entry point has no counterpart in the
  * reference. It is for hosts that are not allowed to allocate device memory where they call the
  * backward -- an engine that reserves all of HBM for its own arena at start-up and bans cudaMalloc

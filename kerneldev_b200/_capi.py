@@ -24,7 +24,7 @@ LIB_PATH = Path(os.environ.get("KD_LIB_PATH") or Path(__file__).resolve().parent
 
 EXPORTS = (
     "kd_version", "kd_last_error", "kd_plan_layout_get", "kd_classify", "kd_mask_dense",
-    "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_static", "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard",
+    "kd_attn_fwd", "kd_attn_bwd", "kd_attn_fwd_f32", "kd_attn_bwd_f32", "kd_attn_bwd_static", "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard",
     "kd_metadata_from_tokens", "kd_span_index", "kd_span_mean",
     "kd_cocktail_index", "kd_cocktail_scores", "kd_cocktail_grad",
     "kd_cast",

@@ -68,7 +68,9 @@ enum : uint32_t {
 // each tensor per thread, so a warp reads whole 128-byte lines; bound by HBM bandwidth. For the fused
 // backward it also zeroes the row of the fp32 dQ accumulation scratch (8 floats per thread).
 // =========================================================================================
-template <int HD, bool kBf16>
+// A float32 call (kF32) leaves two more passes to it: dO is rounded to the 16-bit operand on the way, and dQ, into which the fused
+// backward then adds, is zeroed in place of a scratch.
+template <int HD, bool kBf16, bool kF32 = false>
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
   constexpr int TPR = HD / 8;   // threads per row
   constexpr int RPB = 256 / TPR;   // rows per block and iteration
@@ -86,7 +88,21 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
       const int h = static_cast<int>((r / a.T) % a.H);
       const int b = static_cast<int>(r / ((size_t)a.T * a.H));
       const uint4 ov = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)t * a.o_st + sub * 8);
-      const uint4 dv = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.d_o) + (size_t)b * a.do_sb + (size_t)h * a.do_sh + (size_t)t * a.do_st + sub * 8);
+      uint4* dp = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.d_o) + (size_t)b * a.do_sb + (size_t)h * a.do_sh + (size_t)t * a.do_st + sub * 8);
+      uint4 dv;
+      if (kF32 && a.d_o32 != nullptr) {
+        const float4* src = reinterpret_cast<const float4*>(a.d_o32 + (size_t)b * a.do32_sb + (size_t)h * a.do32_sh + (size_t)t * a.do32_st + sub * 8);
+        const float4 x = src[0], y = src[1];
+        dv = make_uint4(pack2<kBf16>(x.x, x.y), pack2<kBf16>(x.z, x.w), pack2<kBf16>(y.x, y.y), pack2<kBf16>(y.z, y.w));
+        *dp = dv;
+      } else {
+        dv = *dp;
+      }
+      if (kF32 && a.zero_dq) {
+        float4* z = reinterpret_cast<float4*>(static_cast<float*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + (size_t)t * a.dq_st + sub * 8);
+        z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+        z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
       const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, dw[4] = {dv.x, dv.y, dv.z, dv.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -474,8 +490,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (q_valid) {
 #pragma unroll
         for (int cb = 0; cb < EC / ECH; ++cb) {
-          if constexpr (ECH == 16) store_row16_upto<kBf16>(drow + cb * ECH, r[cb], a.sm_scale, g * EC + cb * ECH, a.d_real);
-          else store_row32_upto<kBf16>(drow + cb * ECH, r[cb], a.sm_scale, g * EC + cb * ECH, a.d_real);
+          const int col = g * EC + cb * ECH;
+          if (!kBf16 && a.grads_f32) {
+            float* wide = static_cast<float*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + (size_t)qi * a.dq_st + col;
+            if constexpr (ECH == 16) store_row16_f32_upto(wide, r[cb], a.sm_scale, col, a.d_real);
+            else store_row32_f32_upto(wide, r[cb], a.sm_scale, col, a.d_real);
+          } else if constexpr (ECH == 16) {
+            store_row16_upto<kBf16>(drow + cb * ECH, r[cb], a.sm_scale, col, a.d_real);
+          } else {
+            store_row32_upto<kBf16>(drow + cb * ECH, r[cb], a.sm_scale, col, a.d_real);
+          }
         }
       }
     }
@@ -889,7 +913,18 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
           for (int j = 0; j < ECH; ++j) { rk[j] = 0u; rv[j] = 0u; }
         }
-        if (k_valid) {
+        const int col = g * EC + cb * ECH;
+        if (k_valid && !kBf16 && a.grads_f32) {
+          float* kw = static_cast<float*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st + col;
+          float* vw = static_cast<float*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st + col;
+          if constexpr (ECH == 16) {
+            store_row16_f32_upto(kw, rk, a.sm_scale, col, a.d_real);
+            store_row16_f32_upto(vw, rv, 1.0f, col, a.d_real);
+          } else {
+            store_row32_f32_upto(kw, rk, a.sm_scale, col, a.d_real);
+            store_row32_f32_upto(vw, rv, 1.0f, col, a.d_real);
+          }
+        } else if (k_valid) {
           if constexpr (ECH == 16) {
             store_row16_upto<kBf16>(krow + cb * ECH, rk, a.sm_scale, g * EC + cb * ECH, a.d_real);
             store_row16_upto<kBf16>(vrow + cb * ECH, rv, 1.0f, g * EC + cb * ECH, a.d_real);
@@ -909,7 +944,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 template <int HD, bool kBf16>
-static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
+static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
   using C = BwdCfg<HD>;
   CUtensorMap tmQ, tmK, tmV, tmDO;
   int rc;
@@ -931,10 +966,15 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
   // with the delta kernel ahead of them in this call, the plan was complete before the kernels may start
   a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
-  a.dq_acc = fused ? p.dq_acc : nullptr;
-  a.dq = p.dq.ptr; a.dq_sb = p.dq.stride_b; a.dq_sh = p.dq.stride_h; a.dq_st = p.dq.stride_t;
-  a.dk = p.dk.ptr; a.dk_sb = p.dk.stride_b; a.dk_sh = p.dk.stride_h; a.dk_st = p.dk.stride_t;
-  a.dv = p.dv.ptr; a.dv_sb = p.dv.stride_b; a.dv_sh = p.dv.stride_h; a.dv_st = p.dv.stride_t;
+  a.grads_f32 = f32 != nullptr;
+  a.zero_dq = f32 != nullptr && fused;
+  a.dq_acc = fused && !f32 ? p.dq_acc : nullptr;
+  const kd_tensor &dq = f32 ? f32->dq : p.dq, &dk = f32 ? f32->dk : p.dk, &dv = f32 ? f32->dv : p.dv;
+  a.dq = dq.ptr; a.dq_sb = dq.stride_b; a.dq_sh = dq.stride_h; a.dq_st = dq.stride_t;
+  a.dk = dk.ptr; a.dk_sb = dk.stride_b; a.dk_sh = dk.stride_h; a.dk_st = dk.stride_t;
+  a.dv = dv.ptr; a.dv_sb = dv.stride_b; a.dv_sh = dv.stride_h; a.dv_st = dv.stride_t;
+  a.d_o32 = f32 ? static_cast<const float*>(f32->d_o.ptr) : nullptr;
+  if (f32) { a.do32_sb = f32->d_o.stride_b; a.do32_sh = f32->d_o.stride_h; a.do32_st = f32->d_o.stride_t; }
  
   auto kq = attn_bwd_dq_kernel<HD, kBf16>;
   auto kk = attn_bwd_dkdv_kernel<HD, kBf16>;
@@ -948,7 +988,10 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_plan_layout& L, const 
     const size_t rows = (size_t)p.B * p.H * p.T;
     const int rows_per_block = 256 / (HD / 8);
     const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-    e = launch(attn_bwd_delta_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
+    if constexpr (!kBf16) {
+      if (f32) e = launch(attn_bwd_delta_kernel<HD, kBf16, true>, blocks, 256, 0, stream, a);
+    }
+    if (!f32) e = launch(attn_bwd_delta_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
     if (!fused && e == cudaSuccess) e = launch(kq, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
   if (fused && e == cudaSuccess) {
@@ -1002,13 +1045,13 @@ int static_delta_address(size_t rows_needed, float** out) {
   return 0;
 }
 
-int launch_attn_bwd(const kd_attn_params& p, cudaStream_t stream) {
+int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream) {
   kd_plan_layout L;
   if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
   PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
   if (!p.d_o.ptr) return set_error(KD_ERR_ARG, "d_o is null");
-  if (p.D <= 64) return p.dtype == KD_BF16 ? launch_bwd_t<64, true>(p, L, pv, stream) : launch_bwd_t<64, false>(p, L, pv, stream);
-  return p.dtype == KD_BF16 ? launch_bwd_t<128, true>(p, L, pv, stream) : launch_bwd_t<128, false>(p, L, pv, stream);
+  if (p.D <= 64) return p.dtype == KD_BF16 ? launch_bwd_t<64, true>(p, f32, L, pv, stream) : launch_bwd_t<64, false>(p, f32, L, pv, stream);
+  return p.dtype == KD_BF16 ? launch_bwd_t<128, true>(p, f32, L, pv, stream) : launch_bwd_t<128, false>(p, f32, L, pv, stream);
 }
 
 }  // namespace kd

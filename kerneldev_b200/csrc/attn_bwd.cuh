@@ -20,12 +20,16 @@ struct BwdArgs {
   uint32_t* status;
   const void* o;
   int64_t o_sb, o_sh, o_st;
-  const void* d_o;
+  void* d_o;         // with d_o32: written by the delta kernel
   int64_t do_sb, do_sh, do_st;
+  const float* d_o32;   // null, or dO of a float32 call
+  int64_t do32_sb, do32_sh, do32_st;
   int plan_ready;    // the plan may be read before the wait for the kernel ahead
   const float* lse;
   float* delta;
   float* dq_acc;     // fp32 (B,H,T,tile width) dQ accumulation scratch of the fused backward, else null
+  bool grads_f32;    // dq, dk, dv are float32 (the fused backward then adds its dQ tiles into dq itself)
+  bool zero_dq;      // ... and the delta kernel zeroes it
   void* dq;
   int64_t dq_sb, dq_sh, dq_st;
   void* dk;

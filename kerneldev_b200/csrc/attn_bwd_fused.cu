@@ -137,7 +137,9 @@ __device__ __forceinline__ uint64_t ld_shared_pair(const float* p) {
   return pack_u32x2(lo, hi);
 }
 
-template <int HD_, bool kBf16>
+// kF32: dQ, dK and dV are float32 tensors (of a float32 call). The dQ tiles are then scaled and added into dQ itself, which the delta kernel
+// has zeroed: no scratch and no conversion (2 x 4 x 256 x 64: forward and backward 8 launches -> 4, 105 -> 86 us).
+template <int HD_, bool kBf16, bool kF32>
 __global__ void __launch_bounds__(FusedCfg<HD_>::THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -255,11 +257,13 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       };
       // dK = dV = 0 for an item without entries
       auto write_zeros = [&](const int4& z) {
-        const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0), cpr = a.d_real / 8;   // 16-byte chunks of a row
-        uint16_t* dk = reinterpret_cast<uint16_t*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
-        uint16_t* dv = reinterpret_cast<uint16_t*>(a.dv) + (size_t)z.x * a.dv_sb + (size_t)z.y * a.dv_sh;
+        using Out = std::conditional_t<kF32, float, uint16_t>;
+        constexpr int per = 16 / sizeof(Out);   // elements of a 16-byte chunk
+        const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0), cpr = a.d_real / per;
+        Out* dk = reinterpret_cast<Out*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
+        Out* dv = reinterpret_cast<Out*>(a.dv) + (size_t)z.x * a.dv_sb + (size_t)z.y * a.dv_sh;
         for (int i = lane; i < rows * cpr; i += 32) {
-          const int r = i / cpr, c = (i - r * cpr) * 8;
+          const int r = i / cpr, c = (i - r * cpr) * per;
           *reinterpret_cast<uint4*>(dk + (size_t)(row0 + r) * a.dk_st + c) = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(dv + (size_t)(row0 + r) * a.dv_st + c) = make_uint4(0u, 0u, 0u, 0u);
         }
@@ -895,6 +899,16 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     bool ok = true;
     int t = 0;
     const int np = (a.d_real + 31) / 32;   // 32-column pieces of a dQ tile
+    auto stage_box = [&](int buf, const uint32_t (&r)[32]) {   // 32 columns as a box [32 rows][32 columns]
+#pragma unroll
+      for (int cch = 0; cch < 8; ++cch)
+        st_shared_v4(stg + buf * 4096 + st_row + ((static_cast<uint32_t>(cch) ^ st_sw) << 4), r[4 * cch], r[4 * cch + 1], r[4 * cch + 2], r[4 * cch + 3]);
+    };
+    auto stage_scaled = [&](int buf, uint32_t (&r)[32], float f) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
+      stage_box(buf, r);
+    };
     // Writes dV, then dK (the next item's first dV product comes first) of the item: 32 rows of a warp as boxes of 64 columns
     // through the staging buffers and TMA stores. m: number of the item; kt: its key tile.
     auto write_out = [&](int b, int h, int kt, int m) -> bool {
@@ -905,15 +919,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int part = 0; part < 2 * HD / 64; ++part) {
         const bool is_k = part >= HD / 64;
         const int col = (part % (HD / 64)) * 64;
-        const uint32_t buf = stg + (part & 1) * 4096;
+        const uint32_t buf = kF32 ? stg : stg + (part & 1) * 4096;   // 64 columns of float32 are two boxes
         const float f = is_k ? a.sm_scale : 1.0f;
-        if ((part & 1) == 0) {
+        if (kF32 || (part & 1) == 0) {
           if (lane == 0) bulk_wait_group_read0();   // the staging buffers have been read
           __syncwarp();
         }
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
-          uint32_t r[32], pk[16];
+          uint32_t r[32];
           tmem_ld32(lane_base + (is_k ? C::TM_DK : C::TM_DV) + col + half * 32, r);
           tmem_wait_ld();
           if (col + 64 == HD && half == 1) {   // the accumulator is in registers: the next item's first product may overwrite it
@@ -921,16 +935,22 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + (is_k ? 1 : 0)));
           }
+          if constexpr (kF32) {
+            stage_scaled(half, r, f);
+          } else {
+            uint32_t pk[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(r[2 * j]) * f, __uint_as_float(r[2 * j + 1]) * f);
+            for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(r[2 * j]) * f, __uint_as_float(r[2 * j + 1]) * f);
 #pragma unroll
-          for (int cch = 0; cch < 4; ++cch)
-            st_shared_v4(buf + st_row + ((static_cast<uint32_t>(4 * half + cch) ^ st_sw) << 4), pk[4 * cch], pk[4 * cch + 1], pk[4 * cch + 2], pk[4 * cch + 3]);
+            for (int cch = 0; cch < 4; ++cch)
+              st_shared_v4(buf + st_row + ((static_cast<uint32_t>(4 * half + cch) ^ st_sw) << 4), pk[4 * cch], pk[4 * cch + 1], pk[4 * cch + 2], pk[4 * cch + 3]);
+          }
         }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && key0 < a.T && col < a.d_real) {
           tma_store_4d(is_k ? &tmDK : &tmDV, buf, col, key0, h, b);
+          if (kF32 && col + 32 < a.d_real) tma_store_4d(is_k ? &tmDK : &tmDV, buf + 4096, col + 32, key0, h, b);
           bulk_commit_group();
         }
       }
@@ -954,17 +974,20 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(C::B_DQEMPTY));
         };
-        auto stage = [&](int buf, const uint32_t (&r)[32]) {   // 32 columns as a box [32 rows][32 columns]
-#pragma unroll
-          for (int cch = 0; cch < 8; ++cch)
-            st_shared_v4(stg + buf * 4096 + st_row + ((static_cast<uint32_t>(cch) ^ st_sw) << 4), r[4 * cch], r[4 * cch + 1], r[4 * cch + 2], r[4 * cch + 3]);
+        auto stage = [&](int buf, uint32_t (&r)[32]) {
+          if constexpr (kF32) stage_scaled(buf, r, a.sm_scale);
+          else stage_box(buf, r);
         };
         auto reduce = [&](int g) {   // both boxes: columns 64 g .. 64 g + 63
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && q0 < a.T) {
-            if (g * 2 < np) tma_reduce_add_3d(&tmAcc, stg, g * 64, q0, bh);
-            if (g * 2 + 1 < np) tma_reduce_add_3d(&tmAcc, stg + 4096, g * 64 + 32, q0, bh);
+            auto add = [&](uint32_t src, int col) {
+              if constexpr (kF32) tma_reduce_add_4d(&tmAcc, src, col, q0, h, b);
+              else tma_reduce_add_3d(&tmAcc, src, col, q0, bh);
+            };
+            if (g * 2 < np) add(stg, g * 64);
+            if (g * 2 + 1 < np) add(stg + 4096, g * 64 + 32);
             bulk_commit_group();
           }
         };
@@ -1034,15 +1057,18 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
   }
 }
 
-template <int HD, bool kBf16>
+template <int HD, bool kBf16, bool kF32>
 static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                           const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   using C = FusedCfg<HD>;
   CUtensorMap tmAcc, tmDK, tmDV;
-  int rc = encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
-  const kd_tensor dk = {a.dk, a.dk_sb, a.dk_sh, a.dk_st}, dv = {a.dv, a.dv_sb, a.dv_sh, a.dv_st};
-  if (rc == 0) rc = encode_tensor_map(&tmDK, dk, a.B, a.H, a.T, a.d_real, dtype, 32, "dk");
-  if (rc == 0) rc = encode_tensor_map(&tmDV, dv, a.B, a.H, a.T, a.d_real, dtype, 32, "dv");
+  const kd_tensor dq = {a.dq, a.dq_sb, a.dq_sh, a.dq_st}, dk = {a.dk, a.dk_sb, a.dk_sh, a.dk_st}, dv = {a.dv, a.dv_sb, a.dv_sh, a.dv_st};
+  auto encode_out = [&](CUtensorMap* tm, const kd_tensor& t, const char* name) {
+    return kF32 ? encode_tensor_map_f32(tm, t, a.B, a.H, a.T, a.d_real, 32, name) : encode_tensor_map(tm, t, a.B, a.H, a.T, a.d_real, dtype, 32, name);
+  };
+  int rc = kF32 ? encode_out(&tmAcc, dq, "dq") : encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
+  if (rc == 0) rc = encode_out(&tmDK, dk, "dk");
+  if (rc == 0) rc = encode_out(&tmDV, dv, "dv");
   if (rc != 0) return rc;
   const long long n_items = (long long)a.B * a.H * a.NT;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
@@ -1051,7 +1077,7 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   fa.after_delta = after_delta;
   // Q, K, V, dO and the dQ scratch. (64 MB: hier T = 8192, D = 128 2470 us instead of 2409; without chunks 3540)
   fa.order_of = ItemOrder::make(a.B * a.H, a.NT, (double)a.T * (4.0 * a.d_real * 2 + HD * 4.0), 90e6);
-  auto kern = attn_bwd_fused_kernel<HD, kBf16>;
+  auto kern = attn_bwd_fused_kernel<HD, kBf16, kF32>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd smem attribute: %s", cudaGetErrorString(e));
@@ -1069,16 +1095,18 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   const size_t rows = (size_t)a.B * a.H * a.T;
   const int rows_per_block = 256 / (HD / 8);
   const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-  if (e == cudaSuccess) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
+  if (e == cudaSuccess && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }
 
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                      const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
-  if (a.d_real <= 64)
-    return dtype == KD_BF16 ? launch_fused_t<64, true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream) : launch_fused_t<64, false>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
-  return dtype == KD_BF16 ? launch_fused_t<128, true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream) : launch_fused_t<128, false>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
+  auto run = [&](auto launch_fn) { return launch_fn(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream); };
+  const bool narrow = a.d_real <= 64;
+  if (a.grads_f32) return narrow ? run(launch_fused_t<64, false, true>) : run(launch_fused_t<128, false, true>);
+  if (dtype == KD_BF16) return narrow ? run(launch_fused_t<64, true, false>) : run(launch_fused_t<128, true, false>);
+  return narrow ? run(launch_fused_t<64, false, false>) : run(launch_fused_t<128, false, false>);
 }
 
 }  // namespace kd

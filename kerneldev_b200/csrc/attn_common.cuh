@@ -173,6 +173,19 @@ __device__ __forceinline__ void store_row32_upto(uint16_t* dst, const uint32_t (
     }
   }
 }
+// The same columns of a float32 row. (Four lanes' 16-byte stores fill a line between them in L2.)
+__device__ __forceinline__ void store_row32_f32_upto(float* dst, const uint32_t (&r)[32], float f, int col, int d_real) {
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    if (col + j < d_real)   // 16 columns at a time, as d_real
+      *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]) * f, __uint_as_float(r[j + 1]) * f, __uint_as_float(r[j + 2]) * f, __uint_as_float(r[j + 3]) * f);
+}
+__device__ __forceinline__ void store_row16_f32_upto(float* dst, const uint32_t (&r)[16], float f, int col, int d_real) {
+  if (col >= d_real) return;
+#pragma unroll
+  for (int j = 0; j < 16; j += 4)
+    *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(r[j]) * f, __uint_as_float(r[j + 1]) * f, __uint_as_float(r[j + 2]) * f, __uint_as_float(r[j + 3]) * f);
+}
 template <bool kBf16>
 __device__ __forceinline__ void store_row16_upto(uint16_t* dst, const uint32_t (&r)[16], float f, int col, int d_real) {
   if (col < d_real) store_row16<kBf16>(dst, r, f);

@@ -578,7 +578,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(C::B_OFREE + i));
         }
-        if (qi < a.T) store_row32_upto<kBf16>(orow + half * (HD / 2) + cb * 32, r, inv_l, half * (HD / 2) + cb * 32, a.d_real);
+        const int col = half * (HD / 2) + cb * 32;
+        if (qi < a.T && (kBf16 || a.o != nullptr)) store_row32_upto<kBf16>(orow + col, r, inv_l, col, a.d_real);
+        if (!kBf16 && qi < a.T && a.o32 != nullptr)
+          store_row32_f32_upto(a.o32 + (size_t)b * a.o32_sb + (size_t)h * a.o32_sh + (size_t)qi * a.o32_st + col, r, inv_l, col, a.d_real);
       }
     }
     }  // items
@@ -602,7 +605,7 @@ static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& 
   return 0;
 }
 
-int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
+int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream) {
   kd_plan_layout L;
   if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
   const PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
@@ -624,6 +627,8 @@ int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream) {
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
   a.order = pv.order; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
+  a.o32 = f32 ? static_cast<float*>(f32->o.ptr) : nullptr;
+  if (f32) { a.o32_sb = f32->o.stride_b; a.o32_sh = f32->o.stride_h; a.o32_st = f32->o.stride_t; }
   a.lse = p.lse;
 #ifdef KD_TEST_DROP_LOAD
   const char* drop = getenv("KD_TEST_DROP_LOAD");

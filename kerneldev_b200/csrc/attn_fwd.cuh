@@ -18,8 +18,10 @@ struct FwdArgs {
   uint32_t* status;
   int plan_ready;
   int split;         // 1: an item is one query tile of a pair (see launch_rules.cuh)
-  void* o;
+  void* o;           // null: O is wanted as float32 alone
   int64_t o_sb, o_sh, o_st;
+  float* o32;        // null, or O of a float32 call
+  int64_t o32_sb, o32_sh, o32_st;
   float* lse;
 #ifdef KD_TEST_DROP_LOAD
   int test_drop_load;   // wait time-out test build: the producer of CTA 0 leaves out its first K tile load

@@ -438,7 +438,11 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
         uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)qi * a.o_st;
 #pragma unroll
-        for (int cb = 0; cb < HD / 32; ++cb) store_row32_upto<kBf16>(orow + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
+        for (int cb = 0; cb < HD / 32; ++cb) {
+          if (kBf16 || a.o != nullptr) store_row32_upto<kBf16>(orow + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
+          if (!kBf16 && a.o32 != nullptr)
+            store_row32_f32_upto(a.o32 + (size_t)b * a.o32_sb + (size_t)h * a.o32_sh + (size_t)qi * a.o32_st + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
+        }
         if (a.lse != nullptr) a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
       }
     }  // items

@@ -47,30 +47,38 @@ static CUresult with_context(F encode) {
   return r;
 }
 
-int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype,
-                      int box_rows, const char* name) {
+// a box is 128 bytes wide, whatever D is
+static int encode_4d(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, CUtensorMapDataType type, int es,
+                     int box_rows, const char* name) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return set_error(KD_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
   if (t.ptr == nullptr) return set_error(KD_ERR_ARG, "tensor %s is null", name);
   if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) != 0) return set_error(KD_ERR_ALIGN, "tensor %s: base pointer not 16-byte aligned", name);
-  const int64_t sb = t.stride_b * 2, sh = t.stride_h * 2, st = t.stride_t * 2;  // bytes
+  const int64_t sb = t.stride_b * es, sh = t.stride_h * es, st = t.stride_t * es;  // bytes
   if (st <= 0 || (st & 15) || (H > 1 && (sh <= 0 || (sh & 15))) || (B > 1 && (sb <= 0 || (sb & 15))))
     return set_error(KD_ERR_ALIGN, "tensor %s: byte strides (%lld, %lld, %lld) must be positive multiples of 16",
                      name, (long long)sb, (long long)sh, (long long)st);
-  // the box is 64 elements wide whatever D is: for D < 64 (or the second box of 64 < D < 128) the elements
-  // beyond the tensor are filled with zeros, which leaves every product of the kernels unchanged
+  // For a D that is no multiple of the box (64 elements of 16 bits) the elements beyond the tensor are filled with zeros, which
+  // leaves every product of the kernels unchanged, and not written by stores.
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
   // a stride of a size-1 dimension is never used for addressing but must still be valid
   cuuint64_t strides[3] = {(cuuint64_t)st, (cuuint64_t)(H > 1 ? sh : st * T), (cuuint64_t)(B > 1 ? sb : (H > 1 ? sh * H : st * T))};
   for (int i = 0; i < 3; ++i)
     if (strides[i] & 15) strides[i] = (strides[i] + 15) & ~cuuint64_t(15);
-  cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
-  cuuint32_t es[4] = {1, 1, 1, 1};
-  const CUresult r = with_context([&] { return enc(out, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                   t.ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  cuuint32_t box[4] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows, 1, 1};
+  cuuint32_t step[4] = {1, 1, 1, 1};
+  const CUresult r = with_context([&] { return enc(out, type, 4, t.ptr, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return set_error(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
   return 0;
+}
+
+int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype, int box_rows, const char* name) {
+  return encode_4d(out, t, B, H, T, D, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, box_rows, name);
+}
+
+int encode_tensor_map_f32(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int box_rows, const char* name) {
+  return encode_4d(out, t, B, H, T, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, box_rows, name);
 }
 
 int encode_tensor_map_f32_rows(CUtensorMap* out, float* base, int slices, int T, int D, int box_rows, const char* name) {
@@ -101,7 +109,11 @@ static int check_device() {
   return 0;
 }
 
-static int check_attn(const kd_attn_params* p, bool backward) {
+static bool aligned16(const kd_tensor& t, int es) {
+  return ((reinterpret_cast<uintptr_t>(t.ptr) | (t.stride_t * es) | (t.stride_h * es) | (t.stride_b * es)) & 15u) == 0;
+}
+
+static int check_attn(const kd_attn_params* p, bool backward, const kd_attn_f32* f32 = nullptr) {
   if (!p) return set_error(KD_ERR_ARG, "params is null");
   if (p->B < 1 || p->H < 1 || p->T < 1) return set_error(KD_ERR_ARG, "bad shape B=%d H=%d T=%d", p->B, p->H, p->T);
   if (p->D < 16 || p->D > 128 || (p->D % 16) != 0) return set_error(KD_ERR_ARG, "head dim %d not supported (a multiple of 16 from 16 to 128)", p->D);
@@ -112,17 +124,26 @@ static int check_attn(const kd_attn_params* p, bool backward) {
   if (p->heads_per_cta < 0) return set_error(KD_ERR_ARG, "heads_per_cta must be 0 (automatic) or positive");
   if (!p->plan) return set_error(KD_ERR_ARG, "plan is null (call kd_classify first)");
   if (backward && !p->lse) return set_error(KD_ERR_ARG, "lse is null");
-  if (!p->o.ptr) return set_error(KD_ERR_ARG, "o is null");
+  if (f32) {
+    if (p->dtype != KD_F16) return set_error(KD_ERR_ARG, "float32 tensors take part as float16 operands, dtype is %d", p->dtype);
+    const kd_tensor* t[4] = {backward ? &f32->d_o : &f32->o, &f32->dq, &f32->dk, &f32->dv};
+    for (int i = 0; i < (backward ? 4 : 1); ++i) {
+      if (!t[i]->ptr && !(backward && i == 0)) return set_error(KD_ERR_ARG, "a float32 tensor is null");
+      if (t[i]->ptr && !aligned16(*t[i], 4)) return set_error(KD_ERR_ALIGN, "float32 tensors: pointers and byte strides must be multiples of 16");
+    }
+    if (backward && !aligned16(p->d_o, 2)) return set_error(KD_ERR_ALIGN, "d_o: pointer and byte strides must be multiples of 16");
+  }
+  if (!p->o.ptr && (backward || !f32)) return set_error(KD_ERR_ARG, "o is null");
   if ((reinterpret_cast<uintptr_t>(p->o.ptr) & 15u) || ((p->o.stride_t * 2) & 15) || ((p->o.stride_h * 2) & 15) || ((p->o.stride_b * 2) & 15))
     return set_error(KD_ERR_ALIGN, "o: pointer and byte strides must be multiples of 16");
   if (backward) {
     if (!p->delta) return set_error(KD_ERR_ARG, "delta scratch is null");
     if (p->bwd_mode != KD_BWD_SPLIT && p->bwd_mode != KD_BWD_FUSED) return set_error(KD_ERR_ARG, "bwd_mode %d unknown", p->bwd_mode);
-    if (p->bwd_mode == KD_BWD_FUSED) {
+    if (p->bwd_mode == KD_BWD_FUSED && !f32) {
       if (!p->dq_acc || (reinterpret_cast<uintptr_t>(p->dq_acc) & 15u)) return set_error(KD_ERR_ARG, "dq_acc scratch is null or not 16-byte aligned");
     }
     const kd_tensor* outs[3] = {&p->dq, &p->dk, &p->dv};
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < (f32 ? 0 : 3); ++i) {
       if (!outs[i]->ptr) return set_error(KD_ERR_ARG, "dq/dk/dv is null");
       if ((reinterpret_cast<uintptr_t>(outs[i]->ptr) & 15u) || ((outs[i]->stride_t * 2) & 15) || ((outs[i]->stride_h * 2) & 15) || ((outs[i]->stride_b * 2) & 15))
         return set_error(KD_ERR_ALIGN, "dq/dk/dv: pointer and byte strides must be multiples of 16");
@@ -186,14 +207,30 @@ int kd_attn_fwd(const kd_attn_params* p, void* stream) {
   int rc = check_attn(p, false);
   if (rc) return rc;
   if ((rc = check_device()) != 0) return rc;
-  return launch_attn_fwd(*p, static_cast<cudaStream_t>(stream));
+  return launch_attn_fwd(*p, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int kd_attn_bwd(const kd_attn_params* p, void* stream) {
   int rc = check_attn(p, true);
   if (rc) return rc;
   if ((rc = check_device()) != 0) return rc;
-  return launch_attn_bwd(*p, static_cast<cudaStream_t>(stream));
+  return launch_attn_bwd(*p, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int kd_attn_fwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream) {
+  if (!f) return set_error(KD_ERR_ARG, "float32 tensors are null");
+  int rc = check_attn(p, false, f);
+  if (rc) return rc;
+  if ((rc = check_device()) != 0) return rc;
+  return launch_attn_fwd(*p, f, static_cast<cudaStream_t>(stream));
+}
+
+int kd_attn_bwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream) {
+  if (!f) return set_error(KD_ERR_ARG, "float32 tensors are null");
+  int rc = check_attn(p, true, f);
+  if (rc) return rc;
+  if ((rc = check_device()) != 0) return rc;
+  return launch_attn_bwd(*p, f, static_cast<cudaStream_t>(stream));
 }
 
 int kd_attn_bwd_static(const kd_attn_params* p, void* stream) {
@@ -209,7 +246,7 @@ int kd_attn_bwd_static(const kd_attn_params* p, void* stream) {
   q.delta = scratch;
   q.bwd_mode = KD_BWD_SPLIT;   // the fused backward needs a second, much larger scratch
   if ((rc = check_attn(&q, true)) != 0) return rc;
-  return launch_attn_bwd(q, static_cast<cudaStream_t>(stream));
+  return launch_attn_bwd(q, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int kd_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, size_t* bytes) {

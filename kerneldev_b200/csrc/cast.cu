@@ -1,7 +1,7 @@
 // Conversion between float32 tensors and the 16-bit operands of the kernels: all tensors of a call in one launch.
-// float32 Q, K, V take part as float16 operands (the mantissa of tf32), and O, dQ, dK, dV go back as float32. Bound by HBM
-// traffic (6 bytes per element), for small calls by launches: one for Q, K and V and one for the three gradients instead
-// of a library kernel each took 40 us off the 131 of a forward and backward of 2 x 4 x 256 x 64.
+// float32 Q, K, V take part as float16 operands (the mantissa of tf32). O, dO and the gradients need no pass of their own (kd_attn_f32),
+// but with incoherent processing, whose transform of dQ and dK works on 16-bit tensors, dO and the gradients come here as well.
+// Bound by HBM traffic (6 bytes per element), for small calls by launches.
 #include <algorithm>
 
 #include "common.cuh"

@@ -81,10 +81,14 @@ int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T,
 // one slice), 128-byte swizzle: the target of the fused backward's bulk reductions of dQ tiles.
 int encode_tensor_map_f32_rows(CUtensorMap* out, float* base, int slices, int T, int D, int box_rows, const char* name);
 
+// 4-D tensor map over a float32 (B,H,T,D) tensor with box (32 elements along D, `box_rows` tokens), 128-byte swizzle
+int encode_tensor_map_f32(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int box_rows, const char* name);
+
 int launch_classify(const kd_meta& m, void* plan, cudaStream_t stream);
 int launch_mask_dense(const void* plan, int B, int T, uint8_t* out, cudaStream_t stream);
-int launch_attn_fwd(const kd_attn_params& p, cudaStream_t stream);
-int launch_attn_bwd(const kd_attn_params& p, cudaStream_t stream);
+// f32: NULL, or the call's float32 tensors (kd_attn_f32)
+int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream);
+int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream);
 int static_delta_address(size_t rows_needed, float** out);
 int launch_hadamard(const kd_tensor& x, const kd_tensor& y, int B, int H, int T, int D, int dtype,
                     const float* signs, int inverse, cudaStream_t stream);

@@ -38,6 +38,8 @@ struct Library {
   decltype(&kd_classify) classify = nullptr;
   decltype(&kd_attn_fwd) attn_fwd = nullptr;
   decltype(&kd_attn_bwd) attn_bwd = nullptr;
+  decltype(&kd_attn_fwd_f32) attn_fwd_f32 = nullptr;
+  decltype(&kd_attn_bwd_f32) attn_bwd_f32 = nullptr;
   decltype(&kd_hadamard) hadamard = nullptr;
   decltype(&kd_metadata_from_tokens) metadata_from_tokens = nullptr;
   decltype(&kd_cocktail_index) cocktail_index = nullptr;
@@ -58,6 +60,8 @@ void bind(const py::dict& a) {
   take(lib.classify, a, "kd_classify");
   take(lib.attn_fwd, a, "kd_attn_fwd");
   take(lib.attn_bwd, a, "kd_attn_bwd");
+  take(lib.attn_fwd_f32, a, "kd_attn_fwd_f32");
+  take(lib.attn_bwd_f32, a, "kd_attn_bwd_f32");
   take(lib.hadamard, a, "kd_hadamard");
   take(lib.metadata_from_tokens, a, "kd_metadata_from_tokens");
   take(lib.cocktail_index, a, "kd_cocktail_index");
@@ -340,18 +344,25 @@ int dtype_code(at::ScalarType t) { return t == at::kHalf ? KD_F16 : t == at::kBF
 
 kd_tensor desc(const Tensor& t) { return kd_tensor{t.data_ptr(), t.stride(0), t.stride(1), t.stride(2)}; }
 
-// t itself when TMA can describe it (unit stride along D, 16-byte aligned rows), else one contiguous copy
-Tensor usable(const Tensor& t) {
+// rows of 16-byte pieces: unit stride along D, pointer and strides multiples of 16 bytes
+bool aligned(const Tensor& t) {
   const int64_t es = t.element_size();
   bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
-  for (int i = 0; i < 3; ++i) ok = ok && (t.stride(i) * es) % 16 == 0 && t.stride(i) > 0;
-  return ok ? t : t.contiguous();
+  for (int i = 0; i < 3; ++i) ok = ok && (t.stride(i) * es) % 16 == 0;
+  return ok;
 }
+// ... which TMA can describe: positive strides
+bool tma_ready(const Tensor& t) { return aligned(t) && t.stride(0) > 0 && t.stride(1) > 0 && t.stride(2) > 0; }
 
-Tensor empty_out(const Tensor& like, bool like_input) {
+// t itself when TMA can describe it, else one contiguous copy
+Tensor usable(const Tensor& t) { return tma_ready(t) ? t : t.contiguous(); }
+
+Tensor empty_out(const Tensor& like, bool like_input, at::ScalarType type) {
   // empty_like keeps the strides of a dense tensor, e.g. (B,T,H,D) memory seen as (B,H,T,D)
-  return like_input ? at::empty_like(like) : at::empty(like.sizes(), like.options());
+  const auto options = like.options().dtype(type);
+  return like_input ? at::empty_like(like, options) : at::empty(like.sizes(), options);
 }
+Tensor empty_out(const Tensor& like, bool like_input) { return empty_out(like, like_input, like.scalar_type()); }
 
 kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Plan& plan,
                       double sm_scale) {
@@ -365,59 +376,79 @@ kd_attn_params params(const Tensor& q, const Tensor& k, const Tensor& v, const T
   p.q = desc(q);
   p.k = desc(k);
   p.v = desc(v);
-  p.o = desc(o);
+  if (o.defined()) p.o = desc(o);
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
   p.plan = plan.buf.data_ptr();
   return p;
 }
 
+// `o32`: receives O as float32 (of a float32 call); the 16-bit O is undefined then unless it is wanted.
 std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const PlanPtr& plan, double sm_scale,
-                                   bool like_input, bool want_lse = true) {
+                                   bool like_input, bool want_lse = true, Tensor* o32 = nullptr, bool want_o16 = true) {
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
-  Tensor o = empty_out(q, like_input), lse;
+  Tensor o, lse;
+  if (want_o16) o = empty_out(q, like_input);
+  kd_attn_f32 f{};
+  if (o32 != nullptr) {
+    *o32 = empty_out(q, like_input, at::kFloat);
+    f.o = desc(*o32);
+  }
   if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   p.plan_ready = plan->ready_on(stream) ? 1 : 0;
-  check(lib.attn_fwd(&p, stream));
+  check(o32 != nullptr ? lib.attn_fwd_f32(&p, &f, stream) : lib.attn_fwd(&p, stream));
   plan->launched_on(stream);
   plan->after_launch();
   return {o, lse};
 }
 
+// f32: of a float32 call; dO may be float32, and dQ, dK and dV are.
 // `phases` selects a part of the backward (kd_attn_params.bwd_phases); defined tensors among dq .. dq_acc are reused.
 std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o, const Tensor& lse,
                                             const Tensor& d_o_, const PlanPtr& plan, double sm_scale, int phases, Tensor dq, Tensor dk,
                                             Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic,
-                                            int heads_per_cta) {
-  const Tensor q = usable(q_), k = usable(k_), v = usable(v_), d_o = usable(d_o_);
-  if (!dq.defined()) {
-    dq = empty_out(q, like_input);
-    dk = empty_out(k, like_input);
-    dv = empty_out(v, like_input);
+                                            int heads_per_cta, bool f32 = false) {
+  const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
+  kd_attn_f32 f{};
+  Tensor d_o;
+  if (!f32 || d_o_.scalar_type() != at::kFloat) {
+    d_o = usable(d_o_);
+  } else if (Tensor copy = at::empty_like(d_o_, d_o_.options().dtype(at::kHalf)); aligned(d_o_) && tma_ready(copy)) {
+    d_o = copy;   // filled by the delta kernel
+    f.d_o = desc(d_o_);
+  } else {
+    d_o = usable(d_o_.to(at::kHalf));
   }
-  const auto f32 = q.options().dtype(at::kFloat);
-  if (!delta.defined()) delta = at::empty({q.size(0), q.size(1), q.size(2)}, f32);
+  if (!dq.defined()) {
+    const auto type = f32 ? at::kFloat : q.scalar_type();
+    dq = empty_out(q, like_input, type);
+    dk = empty_out(k, like_input, type);
+    dv = empty_out(v, like_input, type);
+  }
+  const auto f32_options = q.options().dtype(at::kFloat);
+  if (!delta.defined()) delta = at::empty({q.size(0), q.size(1), q.size(2)}, f32_options);
   const bool fused = !deterministic;
   // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
-  if (fused && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, f32);
+  if (fused && !f32 && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, f32_options);
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
   p.heads_per_cta = heads_per_cta;
   p.d_o = desc(d_o);
-  p.dq = desc(dq);
-  p.dk = desc(dk);
-  p.dv = desc(dv);
+  (f32 ? f.dq : p.dq) = desc(dq);
+  (f32 ? f.dk : p.dk) = desc(dk);
+  (f32 ? f.dv : p.dv) = desc(dv);
   p.delta = delta.data_ptr<float>();
   p.bwd_phases = phases;
   if (fused) {
     p.bwd_mode = KD_BWD_FUSED;
-    p.dq_acc = dq_acc.data_ptr<float>();
+    if (!f32) p.dq_acc = dq_acc.data_ptr<float>();
   }
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
-  check(lib.attn_bwd(&p, at::cuda::getCurrentCUDAStream()));
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  check(f32 ? lib.attn_bwd_f32(&p, &f, stream) : lib.attn_bwd(&p, stream));
   plan->after_launch();
   return {dq, dk, dv};
 }
@@ -428,12 +459,6 @@ std::array<Tensor, KD_CAST_MAX> cast(std::initializer_list<Tensor> in, at::Scala
   std::array<Tensor, KD_CAST_MAX> out;
   kd_tensor src[KD_CAST_MAX], dst[KD_CAST_MAX];
   int n = 0, slot = 0;
-  auto aligned = [](const Tensor& t) {
-    const int64_t es = t.element_size();
-    bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
-    for (int i = 0; i < 3; ++i) ok = ok && (t.stride(i) * es) % 16 == 0;
-    return ok;
-  };
   const Tensor& first = *in.begin();
   for (const Tensor& x : in) {
     Tensor y = at::empty_like(x, x.options().dtype(to));
@@ -494,15 +519,16 @@ struct AttentionBackward : torch::autograd::Node {
     }
     at::NoGradGuard no_grad;
     // a gradient that a later node left undefined counts as zeros, as for autograd.Function
-    const Tensor d_o = !grads[0].defined() ? at::zeros_like(to) : widen ? cast({grads[0]}, at::kHalf)[0] : grads[0];
+    const bool direct = widen && !signs.has_value();   // the transform of dQ and dK works on 16-bit tensors
+    const Tensor d_o = !grads[0].defined() ? at::zeros_like(to) : widen && !direct ? cast({grads[0]}, at::kHalf)[0] : grads[0];
     auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
-                                 opt.heads_per_cta);
+                                 opt.heads_per_cta, direct);
     if (signs.has_value()) {
       // y = x diag(s) W / sqrt(D) with W symmetric, so dx = dy W / sqrt(D) diag(s)
       dq = hadamard(dq, signs, true);
       dk = hadamard(dk, signs, true);
     }
-    if (widen) {
+    if (widen && !direct) {
       auto wide = cast({dq, dk, dv}, at::kFloat);
       dq = wide[0];
       dk = wide[1];
@@ -576,8 +602,8 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
       q2 = hadamard(q2, signs, false);
       k2 = hadamard(k2, signs, false);
     }
-    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, return_lse || track);
-    o = f32 ? cast({o16}, at::kFloat)[0] : o16;
+    std::tie(o16, lse) = forward(q2, k2, v2, plan, scale, like_input, return_lse || track, f32 ? &o : nullptr, !f32 || track);
+    if (!f32) o = o16;
   }
   if (track) {
     auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);

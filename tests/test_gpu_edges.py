@@ -10,6 +10,7 @@ sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "gol
 from cocktail_inputs import cocktail_rows, embeddings  # noqa: E402
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from oracle import attention_oracle as ao  # noqa: E402
+from helpers import rand_inputs  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -204,3 +205,36 @@ def test_host_thread_without_a_cuda_context():
     assert len(out) == 1
     for x, y in zip(first, out[0]):
         assert torch.allclose(x.float(), y.float(), atol=1e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("B,H,T,D,layout", [(1, 1, 1, 16, "bhtd"), (2, 3, 129, 48, "bthd"), (1, 2, 300, 80, "bhtd"), (2, 2, 257, 64, "bthd"), (1, 3, 640, 128, "bthd"), (1, 2, 383, 112, "bhtd")])
+def test_float32_results_are_not_rounded_to_16_bits(B, H, T, D, layout, deterministic):
+    """float32 O, dQ, dK and dV are written by the attention kernels: rows and columns at the edges of tiles and boxes, memory orders,
+    sequences that end early (rows without keys, key tiles without queries). Errors are those of the float16 operands alone."""
+    from kerneldev_b200 import flash_attention
+    q, k, v, do = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.float32, seed=T + D))
+    if layout == "bthd":
+        q, k, v, do = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (q, k, v, do))
+    lens = torch.tensor([T] + [T // 2] * (B - 1), dtype=torch.int32, device=DEV)
+    qg, kg, vg = (x.detach().clone(memory_format=torch.preserve_format).requires_grad_() for x in (q, k, v))
+    o = flash_attention(qg, kg, vg, lens=lens, causal=True, out_layout="input", deterministic=deterministic)
+    grads = torch.autograd.grad(o, (qg, kg, vg), do, retain_graph=True)
+    mask = ao.dense_mask(T, None, None, None, lens.cpu().numpy(), causal=True, B=B)
+    half = [x.half().float().cpu() for x in (q, k, v, do)]
+    ro, _, *rg = ao.attention_fwd_bwd(*half, mask)
+    for got, ref, like in zip((o, *grads), (ro, *rg), (q, q, k, v)):
+        assert got.dtype == torch.float32 and got.stride() == like.stride()
+        # P, dS and O inside delta are float16 (2^-11 relative each); a handful of such terms of the size of the result. With one
+        # token dQ and dK are the difference of two equal fp32 sums of products of size 1 (2^-24 each).
+        assert float((got.detach().cpu() - ref).norm()) <= 4 * 2.0**-11 * float(ref.norm()) + D * 2.0**-22
+        if T > 1:
+            assert not torch.equal(got.half().float(), got)
+    # O is not what the backward reads, so it may be written to; dO may have any strides
+    with torch.no_grad():
+        o.zero_()
+    again = torch.autograd.grad(o, (qg, kg, vg), do.transpose(1, 2).contiguous().transpose(1, 2), retain_graph=True)
+    expanded = torch.autograd.grad(o, (qg, kg, vg), torch.ones((1, 1, 1, 1), device=DEV).expand(B, H, T, D), retain_graph=True)
+    ones = torch.autograd.grad(o, (qg, kg, vg), torch.ones((B, H, T, D), device=DEV))
+    for x, y in list(zip(grads, again)) + list(zip(expanded, ones)):
+        assert float((x - y).norm()) <= (0.0 if deterministic else 1e-5) * float(y.norm())   # dQ's sums have no fixed order
