@@ -44,8 +44,9 @@ struct BwdCfg {
   static constexpr int THREADS = 128 + 256 * NSUB;    // four light warps + 2 * NSUB compute warpgroups
   static constexpr int REGS_COMPUTE = KD_REGS_COMPUTE_BWD;
   static constexpr int STAGE_WORDS = 2 * 32 * CPT;                 // per warp (dK/dV kernel): 32*CPT x {lse, delta}
-  static constexpr int SMEM_ACT = SMEM_STAGE + 8 * NSUB * STAGE_WORDS * 4;  // compacted entry list
-  static constexpr int SMEM_TOTAL = SMEM_ACT + 128 * 2;
+  static constexpr int NITEM = 4;                     // ring of item headers and lists
+  static constexpr int SMEM_ACT = SMEM_STAGE + 8 * NSUB * STAGE_WORDS * 4;  // NITEM x <= 128 list entries
+  static constexpr int SMEM_TOTAL = SMEM_ACT + NITEM * 128 * 2;
   static constexpr int SMEM_ALLOC = SMEM_TOTAL + 1024;
   // TMEM columns
   // buffer j: scores at 128*j, dP at 128*j + 64; accumulators behind the buffers
@@ -60,6 +61,7 @@ enum : uint32_t {
   W_Q_ACCFULL = 0x206, W_Q_M2ISSUED = 0x207, W_Q_FIXEMPTY = 0x208, W_Q_ACCFREE = 0x209,
   W_K_FIXFULL = 0x301, W_K_RINGEMPTY = 0x302, W_K_RINGFULL = 0x303, W_K_PFULL = 0x304, W_K_SFULL = 0x305,
   W_K_ACCFULL = 0x306, W_K_M2ISSUED = 0x307, W_K_FIXEMPTY = 0x308, W_K_ACCFREE = 0x309,
+  W_Q_ITEMFULL = 0x20A, W_Q_ITEMEMPTY = 0x20B, W_Q_CLC = 0x20C, W_K_ITEMFULL = 0x30A, W_K_ITEMEMPTY = 0x30B, W_K_CLC = 0x30C,
 };
 
 // =========================================================================================
@@ -123,11 +125,192 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
 }
 
 // =========================================================================================
-// dQ kernel: one CTA per (b, group of heads, query tile); streams = key halves of the current key
+// What the two kernels below share: barriers, items and the producer warp.
+//
+// A work item is one tile of one (batch, head). The grid has a CTA per item, but a CTA that is running takes further items by cancelling CTAs that have not been launched yet
+// (clusterlaunchcontrol), as in the forward and the fused backward: the rings, the issuers and the compute warps run on into the
+// next item, and the start and drain of a CTA (launch, TMEM, first loads, pipeline fill, last products: 12,000 cycles) is paid once
+// per SM instead of once per item, which has some ten tiles of 2,200-2,800 cycles. Both kernels together, before (a CTA per tile and one
+// or more heads) and with this, bf16 (us): hierarchical 4 x 16 x 2048 x 64 114 -> 108, 16 x 16 x 4096 x 64 1570 -> 1500; causal 8 x 16 x
+// 1000 x 64 146 -> 127, 8 x 16 x 2048 x 128 723 -> 685; no mask 4 x 16 x 2048 x 64 383 -> 331; causal 1 x 8 x 173 x 64 14.6 -> 11.7.
+// =========================================================================================
+template <typename C>
+struct BwdShared {
+  uint64_t fix_full[C::NFIX], fix_empty[C::NFIX], ring_full[C::STAGES], ring_empty[C::STAGES], s_full[C::NBUF], p_full[C::NBUF],
+      m2_issued[C::NBUF], acc_full, acc_free, item_full[C::NITEM], item_empty[C::NITEM], clc;
+  __align__(16) int4 items[C::NITEM];   // {batch, head, tile, entries}; entries < 0: there is no further item
+  __align__(16) uint8_t answer[16];     // of a cancellation
+  uint32_t tmem_base;
+  AbortFlag abortf;
+};
+
+template <typename C>
+__device__ __forceinline__ void bwd_init(BwdShared<C>& sh) {   // one thread
+  sh.abortf.v = 0;
+  for (int f = 0; f < C::NFIX; ++f) {
+    mbar_init(smem_u32(&sh.fix_full[f]), 1);
+    mbar_init(smem_u32(&sh.fix_empty[f]), 2);  // both M1 issuers are done with the item's resident tiles
+  }
+  for (int s = 0; s < C::STAGES; ++s) {
+    mbar_init(smem_u32(&sh.ring_full[s]), 1);
+    mbar_init(smem_u32(&sh.ring_empty[s]), 1);
+  }
+  for (int i = 0; i < C::NBUF; ++i) {
+    mbar_init(smem_u32(&sh.s_full[i]), 2);     // one commit from each of the two M1 issuers
+    mbar_init(smem_u32(&sh.p_full[i]), 4 * C::NSUB);   // one arrival per warp of the warpgroups that share the unit
+    mbar_init(smem_u32(&sh.m2_issued[i]), 1);
+  }
+  mbar_init(smem_u32(&sh.acc_full), 1);
+  mbar_init(smem_u32(&sh.acc_free), 8 * C::NSUB);      // every compute warp has read its part of the accumulators
+  for (int i = 0; i < C::NITEM; ++i) {
+    mbar_init(smem_u32(&sh.item_full[i]), 1);
+    mbar_init(smem_u32(&sh.item_empty[i]), 3 + 8 * C::NSUB);   // the three issuers and every compute warp
+  }
+  mbar_init(smem_u32(&sh.clc), 1);
+  fence_barrier_init();
+}
+
+// header of the CTA's k-th item for a single thread, which needs no list; false: an abort
+template <typename C>
+__device__ __forceinline__ bool bwd_header(BwdShared<C>& sh, int k, uint32_t site, int4& it) {
+  const int slot = k % C::NITEM;
+  if (!mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, site)) return false;
+  it = sh.items[slot];
+  mbar_arrive(smem_u32(&sh.item_empty[slot]));
+  return true;
+}
+
+// warp-uniform for the compiler
+__device__ __forceinline__ int4 uniform(const int4& v) {
+  return make_int4(__reduce_max_sync(0xffffffffu, v.x), __reduce_max_sync(0xffffffffu, v.y), __reduce_max_sync(0xffffffffu, v.z), __reduce_max_sync(0xffffffffu, v.w));
+}
+
+// The producer warp of the dQ kernel (kQ: items are query tiles; Q and dO resident, K and V streamed) and of the dK/dV kernel (key tiles;
+// K and V resident, Q and dO streamed). wait_ahead: the plan may be read now, the tensors only behind pdl_wait().
+template <int HD, bool kQ>
+__device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CUtensorMap& tmFix1, const CUtensorMap& tmRing0, const CUtensorMap& tmRing1,
+                                             const BwdArgs& a, uint32_t sFix, uint32_t sRing, uint16_t* lists, BwdShared<BwdCfg<HD>>& sh, int lane,
+                                             bool wait_ahead) {
+  using C = BwdCfg<HD>;
+  constexpr uint32_t FIXEMPTY = kQ ? W_Q_FIXEMPTY : W_K_FIXEMPTY, RINGEMPTY = kQ ? W_Q_RINGEMPTY : W_K_RINGEMPTY,
+                     ITEMEMPTY = kQ ? W_Q_ITEMEMPTY : W_K_ITEMEMPTY, CLC = kQ ? W_Q_CLC : W_K_CLC;
+  if (lane == 0) {
+    tma_prefetch_desc(&tmFix0);
+    tma_prefetch_desc(&tmFix1);
+    tma_prefetch_desc(&tmRing0);
+    tma_prefetch_desc(&tmRing1);
+  }
+  auto wait = [&](const uint64_t& bar, uint32_t parity, uint32_t site) -> bool {
+    return __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar), parity, &sh.abortf, site));
+  };
+  const uint32_t below = (1u << lane) - 1u;
+  uint32_t lst[4];   // the decoded item's list, 32 entries per register: tile | class << 8, zeros where an entry is another tile's
+  auto decode = [&](int idx) -> int4 {
+    int bh, rank;
+    a.order_of.decode(idx, a.NT, bh, rank);
+    int4 it;
+    it.x = bh / a.H;
+    it.y = bh - it.x * a.H;
+    it.z = __ldcg(a.order + ((size_t)it.x * 3 + (kQ ? 1 : 2)) * a.NT + rank);   // longest lists first
+    const int row = kQ ? it.z >> 1 : it.z;   // (query tiles: the list of the pair)
+    const uint16_t* list = kQ ? a.fwd_list + ((size_t)it.x * a.NP + row) * a.NT : a.bwd_list + ((size_t)it.x * a.NT + row) * a.NT;
+    const int n = __ldcg(kQ ? a.fwd_cnt + it.x * a.NP + row : a.bwd_cnt + it.x * a.NT + row);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
+    it.w = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (r * 32 + lane >= n) lst[r] = 0u;
+      if (kQ) {
+        const uint32_t cls = (lst[r] >> (8 + 2 * (it.z & 1))) & 3u;
+        lst[r] = cls != 0u ? (lst[r] & 0xFFu) | (cls << 8) : 0u;
+      }
+      it.w += __popc(__ballot_sync(0xffffffffu, lst[r] != 0u));
+    }
+    return it;
+  };
+  int k = 0, asked = 0, issued = 0, fixed = 0;   // items published, cancellations asked for, ring entries and resident pairs requested
+  bool ok = true, pending = false;
+  // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), as in the other kernels.
+  auto ask = [&]() {
+    if (lane == 0) {
+      fence_proxy_async_smem();   // the previous response has been read
+      mbar_arrive_expect_tx(smem_u32(&sh.clc), 16);
+      clc_try_cancel(smem_u32(sh.answer), smem_u32(&sh.clc));
+    }
+    ++asked;
+    pending = true;
+  };
+  auto take_next = [&](int4& nx) -> bool {
+    if (!wait(sh.clc, (asked - 1) & 1, CLC)) return false;
+    pending = false;
+    const int idx = clc_first_ctaid_x(smem_u32(sh.answer));
+    __syncwarp();   // every lane has read the response that the next request overwrites
+    nx.w = -1;
+    if (idx >= 0) {
+      nx = decode(idx);
+      if (nx.w <= 2) ask();
+    }
+    return true;
+  };
+  auto load_pair = [&](const CUtensorMap& t0, const CUtensorMap& t1, uint32_t dst, const uint64_t& full, int tile, int h, int b) {
+    if (lane != 0) return;
+    const uint32_t bar = smem_u32(&full);
+    mbar_arrive_expect_tx(bar, 2 * C::TILE_BYTES);
+    for (int kb = 0; kb < C::KBLK; ++kb) {
+      tma_load_4d(dst + kb * 16384, &t0, bar, kb * 64, tile * KD_TILE, h, b);
+      tma_load_4d(dst + C::TILE_BYTES + kb * 16384, &t1, bar, kb * 64, tile * KD_TILE, h, b);
+    }
+  };
+  int4 it = decode(blockIdx.x);
+  if (it.w <= 2) ask();
+  while (ok) {
+    const int slot = k % C::NITEM, b = it.x, h = it.y, n = it.w;
+    if (!(ok = wait(sh.item_empty[slot], ((k / C::NITEM) & 1) ^ 1, ITEMEMPTY))) break;
+    uint16_t* list = lists + slot * 128;
+    int at = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t has = __ballot_sync(0xffffffffu, lst[r] != 0u);
+      if (n > 0 && lst[r] != 0u) list[at + __popc(has & below)] = static_cast<uint16_t>(lst[r]);
+      at += __popc(has);
+    }
+    if (lane == 0) sh.items[slot] = it;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sh.item_full[slot]));
+    if (n < 0) break;
+    if (k == 0 && wait_ahead) pdl_wait();
+    ++k;
+    int4 nx = it;
+#pragma unroll 1
+    for (int e = 0; e < max(n, 1); ++e) {
+      if (n > 2 && e == n - 3) ask();
+      if (e >= n - 1 && !(ok = take_next(nx))) break;   // its list is looked up while this item's last tiles wait for slots
+      if (n == 0) break;
+      if (e == 0) {   // the item's resident tiles: into the buffer of the item before the last (NFIX = 2)
+        const int f = fixed % C::NFIX;
+        if (!(ok = wait(sh.fix_empty[f], ((fixed / C::NFIX) & 1) ^ 1, FIXEMPTY))) break;
+        load_pair(tmFix0, tmFix1, sFix + f * 2 * C::TILE_BYTES, sh.fix_full[f], it.z, h, b);
+        ++fixed;
+      }
+      const int st = issued % C::STAGES;
+      if (!(ok = wait(sh.ring_empty[st], ((issued / C::STAGES) & 1) ^ 1, RINGEMPTY))) break;
+      load_pair(tmRing0, tmRing1, sRing + st * 2 * C::TILE_BYTES, sh.ring_full[st], list[e] & 0xFF, h, b);
+      ++issued;
+    }
+    it = nx;
+  }
+  if (lane == 0 && sh.abortf.v != 0) {   // let the copies in flight land before the CTA exits
+    for (int e = max(0, issued - C::STAGES); e < issued; ++e) drain_wait(smem_u32(&sh.ring_full[e % C::STAGES]), (e / C::STAGES) & 1);
+    for (int f = max(0, fixed - C::NFIX); f < fixed; ++f) drain_wait(smem_u32(&sh.fix_full[f % C::NFIX]), (f / C::NFIX) & 1);
+    if (pending) drain_wait(smem_u32(&sh.clc), (asked - 1) & 1);
+  }
+}
+
+// =========================================================================================
+// dQ kernel: items are query tiles; streams = key halves of the current key
 // tile.   M1(i): S_i = Q K_i^T, dP_i = dO V_i^T      M2(i): dQ += dS_i K_i
-// The heads of the group are handled one after the other: they share the work list, the barriers
-// and the TMEM allocation, and the producer and the issuers run on into the next head while the
-// compute warps finish the current one, so the pipeline fill and drain are paid once per CTA.
+// The producer and the issuers run on into the next item while the compute warps finish the current one.
 // =========================================================================================
 template <int HD, bool kBf16>
 __global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
@@ -140,128 +323,46 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t sFix = smem_u32(smem + C::SMEM_FIX);    // buffer f: Q at +0, dO at +TILE_BYTES
   const uint32_t sRing = smem_u32(smem + C::SMEM_RING);  // stage s: K at +0, V at +TILE_BYTES
   uint32_t* sStage = reinterpret_cast<uint32_t*>(smem + C::SMEM_STAGE);
-  uint16_t* sAct = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
-
-  __shared__ __align__(8) uint64_t bar_fix_full[C::NFIX], bar_fix_empty[C::NFIX], bar_ring_full[C::STAGES],
-      bar_ring_empty[C::STAGES], bar_s_full[C::NBUF], bar_p_full[C::NBUF], bar_m2_issued[C::NBUF], bar_acc_full, bar_acc_free;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int n_act_s;
-  __shared__ AbortFlag abortf;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
+  __shared__ BwdShared<C> sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // With the delta kernel ahead the plan may be read before the wait, past L1: the start of a kernel that overlaps another
-  // need not have cleaned it, and a plan's memory may have held another one.
-  if (!a.plan_ready) pdl_wait();
-  const int h0 = blockIdx.x * a.G, b = blockIdx.y;
-  const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
-  const int qt = __ldcg(a.order + ((size_t)b * 3 + 1) * a.NT + blockIdx.z);   // longest lists first
-  const int pair = qt >> 1, ip = qt & 1;
-
-  if (tid == 0) {
-    abortf.v = 0;
-    for (int f = 0; f < C::NFIX; ++f) {
-      mbar_init(smem_u32(&bar_fix_full[f]), 1);
-      mbar_init(smem_u32(&bar_fix_empty[f]), 2);  // both M1 issuers are done with the head's Q and dO
-    }
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(smem_u32(&bar_ring_full[s]), 1);
-      mbar_init(smem_u32(&bar_ring_empty[s]), 1);
-    }
-    for (int i = 0; i < C::NBUF; ++i) {
-      mbar_init(smem_u32(&bar_s_full[i]), 2);     // one commit from each of the two M1 issuers
-      mbar_init(smem_u32(&bar_p_full[i]), 4 * C::NSUB);   // one arrival per warp of the warpgroups that share the unit
-      mbar_init(smem_u32(&bar_m2_issued[i]), 1);
-    }
-    mbar_init(smem_u32(&bar_acc_full), 1);
-    mbar_init(smem_u32(&bar_acc_free), 8 * C::NSUB);      // every compute warp has read its part of dQ
-    fence_barrier_init();
-  }
+  if (tid == 0) bwd_init<C>(sh);
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(&sh.tmem_base), 512);
     tmem_relinquish();
-  }
-  if (warp == 2) {
-    // compact the pair's list down to the entries that are non-empty for this query tile
-    const int n = __ldcg(a.fwd_cnt + b * a.NP + pair);
-    const uint16_t* list = a.fwd_list + ((size_t)b * a.NP + pair) * a.NT;
-    int na = 0;
-    for (int base = 0; base < n; base += 32) {
-      const int e = base + lane;
-      const uint32_t ent = e < n ? __ldcg(list + e) : 0u;
-      const uint32_t cls = (ent >> (8 + 2 * ip)) & 3u;
-      const uint32_t bal = __ballot_sync(0xffffffffu, cls != 0u);
-      if (cls != 0u) sAct[na + __popc(bal & ((1u << lane) - 1u))] = static_cast<uint16_t>((ent & 0xFFu) | (cls << 8));
-      na += __popc(bal);
-    }
-    if (lane == 0) n_act_s = na;
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  pdl_wait();
-  pdl_launch_dependents();
-  const uint32_t tbase = tmem_base_s;
-  const int na = n_act_s;
+  // With the delta kernel ahead the plan may be read before the wait, past L1: the start of a kernel that overlaps another
+  // need not have cleaned it, and a plan's memory may have held another one.
+  const bool wait_ahead = a.plan_ready != 0;
+  if (!wait_ahead) pdl_wait();
+  const uint32_t tbase = sh.tmem_base;
 
   if (warp < 4) {
     reg_dealloc<KD_REGS_ISSUE>();
-    if (warp == 0 && lane == 0 && na > 0) {
-      // ------------------------------ TMA producer ------------------------------
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmDO);
-      int issued = 0, fix_issued = 0;   // ring entries / resident pairs requested so far, over all heads
-      bool ok = true;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const int h = h0 + hh, fb = hh % C::NFIX;
-        if (hh >= C::NFIX) {   // the buffer's previous head must have been consumed by both M1 issuers
-          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, W_Q_FIXEMPTY);
-          if (!ok) break;
-        }
-        mbar_arrive_expect_tx(smem_u32(&bar_fix_full[fb]), 2 * C::TILE_BYTES);
-        for (int kb = 0; kb < C::KBLK; ++kb) {
-          tma_load_4d(sFix + fb * 2 * C::TILE_BYTES + kb * 16384, &tmQ, smem_u32(&bar_fix_full[fb]), kb * 64, qt * KD_TILE, h, b);
-          tma_load_4d(sFix + fb * 2 * C::TILE_BYTES + C::TILE_BYTES + kb * 16384, &tmDO, smem_u32(&bar_fix_full[fb]), kb * 64, qt * KD_TILE, h, b);
-        }
-        fix_issued = hh + 1;
-        for (int e = 0; e < na; ++e) {
-          const int s = issued % C::STAGES;
-          const uint32_t ph = (issued / C::STAGES) & 1;
-          const int kt = sAct[e] & 0xFF;
-          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, W_Q_RINGEMPTY);
-          if (!ok) break;
-          mbar_arrive_expect_tx(smem_u32(&bar_ring_full[s]), 2 * C::TILE_BYTES);
-          const uint32_t dst = sRing + s * 2 * C::TILE_BYTES;
-          for (int kb = 0; kb < C::KBLK; ++kb) {
-            tma_load_4d(dst + kb * 16384, &tmK, smem_u32(&bar_ring_full[s]), kb * 64, kt * KD_TILE, h, b);
-            tma_load_4d(dst + C::TILE_BYTES + kb * 16384, &tmV, smem_u32(&bar_ring_full[s]), kb * 64, kt * KD_TILE, h, b);
-          }
-          ++issued;
-        }
-      }
-      if (abortf.v != 0) {   // let the copies in flight land before the CTA exits
-        for (int e = max(0, issued - C::STAGES); e < issued; ++e)
-          for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&bar_ring_full[e % C::STAGES]), (e / C::STAGES) & 1); ++spin) {}
-        for (int f = max(0, fix_issued - C::NFIX); f < fix_issued; ++f)
-          for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&bar_fix_full[f % C::NFIX]), (f / C::NFIX) & 1); ++spin) {}
-      }
-    } else if ((warp == 3 || warp == 2) && lane == 0 && na > 0) {
+    if (warp == 0) {
+      bwd_producer<HD, true>(tmQ, tmDO, tmK, tmV, a, sFix, sRing, lists, sh, lane, wait_ahead);
+    } else if ((warp == 3 || warp == 2) && lane == 0) {
       // ------------------------------ M1 issuers: warp 3: S_u = Q K_u^T; warp 2: dP_u = dO V_u^T ------------------------------
       const bool dp_part = (warp == 2);
       const uint32_t idesc_m1 = make_idesc_f16(kBf16, 0, 0, KD_TILE, 64);   // N = 64 keys
       const uint32_t hi = desc_hi_sw128();
       const uint32_t loRingK = desc_lo_kmajor(sRing);
-      const int U = 2 * na;
       bool ok = true;
-      int buf = 0, round = 0, stage = 0;   // run on across the heads
+      int buf = 0, round = 0, stage = 0, item = 0;   // run on across the items; item: of those with entries
       uint32_t ring_parity = 0;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const int fb = hh % C::NFIX;
-        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, W_Q_FIXFULL);
+      int4 it;
+      for (int k = 0; ok && bwd_header<C>(sh, k, W_Q_ITEMFULL, it) && it.w >= 0; ++k) {
+        if (it.w == 0) continue;
+        const int U = 2 * it.w, fb = item % C::NFIX;
+        ok = mbar_wait(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_Q_FIXFULL);
+        ++item;
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // dO or Q
-        uint64_t adesc[HD / 16];   // A descriptors of the head's k-steps
+        uint64_t adesc[HD / 16];   // A descriptors of the item's k-steps
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) adesc[kk] = desc64(loA + koff_kmajor(kk), hi);
         for (int u = 0; u < U && ok; ++u) {
@@ -274,36 +375,38 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, W_Q_M2ISSUED);
+            ok = mbar_wait(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_Q_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its K and V tiles must have landed
-            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, W_Q_RINGFULL);
+            ok = mbar_wait(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_Q_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
           mma_ss64<false>(dst, adesc[0], bdesc[0], idesc_m1);
 #pragma unroll
           for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(dst, adesc[kk], bdesc[kk], idesc_m1);
-          mma_commit(smem_u32(&bar_s_full[buf]));
+          mma_commit(smem_u32(&sh.s_full[buf]));
           if (++buf == C::NBUF) { buf = 0; ++round; }
           if (i == 1 && ++stage == C::STAGES) { stage = 0; ring_parity ^= 1; }
         }
-        if (ok) mma_commit(smem_u32(&bar_fix_empty[fb]));   // this issuer's products of the head no longer read Q / dO
+        if (ok) mma_commit(smem_u32(&sh.fix_empty[fb]));   // this issuer's products of the item no longer read Q / dO
       }
-    } else if (warp == 1 && lane == 0 && na > 0) {
+    } else if (warp == 1 && lane == 0) {
       // ------------------------------ M2 issuer: dQ += dS_u K_u ------------------------------
       const uint32_t idesc_m2 = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);   // B = K rows, MN-major
       const uint32_t tAcc = tbase + C::TM_ACC0;
       const uint32_t hi = desc_hi_sw128();
       const uint32_t loRingMN = desc_lo_mnmajor(sRing);
-      const int U = 2 * na;
       bool ok = true;
-      int buf = 0, stage = 0;
+      int buf = 0, stage = 0, item = 0;
       uint32_t round_parity = 0;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        if (hh > 0) {   // the previous head's dQ must have been read out of the accumulator
-          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, W_Q_ACCFREE);
+      int4 it;
+      for (int k = 0; ok && bwd_header<C>(sh, k, W_Q_ITEMFULL, it) && it.w >= 0; ++k) {
+        if (it.w == 0) continue;
+        const int U = 2 * it.w;
+        if (item++ > 0) {   // the previous item's dQ must have been read out of the accumulator
+          ok = mbar_wait(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_Q_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -318,19 +421,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             bdesc[kk] = desc64(kb + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_Q_PFULL);
+          ok = mbar_wait(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_Q_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           mma_ts64_p(tAcc, aop[0], bdesc[0], idesc_m2, u > 0 ? 1u : 0u);
 #pragma unroll
           for (int kk = 1; kk < 4; ++kk) mma_ts64<true>(tAcc, aop[kk], bdesc[kk], idesc_m2);
-          if (i == 1) mma_commit(smem_u32(&bar_ring_empty[stage]));
+          if (i == 1) mma_commit(smem_u32(&sh.ring_empty[stage]));
           tc_fence_before_sync();
-          mbar_arrive(smem_u32(&bar_m2_issued[buf]));
+          mbar_arrive(smem_u32(&sh.m2_issued[buf]));
           if (++buf == C::NBUF) { buf = 0; round_parity ^= 1; }
           if (i == 1 && ++stage == C::STAGES) stage = 0;
         }
-        if (ok) mma_commit(smem_u32(&bar_acc_full));
+        if (ok) mma_commit(smem_u32(&sh.acc_full));
       }
     }
   } else {
@@ -342,14 +445,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int c0 = (g % C::NSUB) * CPT;   // first 32-key chunk of that half handled here
     const int wq = warp & 3;
     const int row = wq * 32 + lane;
-    const int qi = qt * KD_TILE + row;
-    const bool q_valid = qi < a.T;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float c = a.scale_log2;
-    const uint32_t qd = a.desc[(size_t)b * a.Tpad + qi];
     const int tbw = 2 * i + c0;      // first word of this thread's chunks in the 128-bit class masks of a key tile
     bool ok = true;
 
+    int4 it = make_int4(0, 0, 0, 0);   // the item in hand; behind its last unit the next one
     // key descriptors of PARTIAL tiles are fetched one entry ahead into registers
     uint32_t kd_pre[CPT];
     uint32_t tb_pre[3][CPT];   // key-side class masks of the chunks: is_prefix, context, in_span
@@ -358,34 +459,49 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     auto prefetch_kd = [&](uint32_t entry) {
       if ((entry >> 8) == KD_TILE_PARTIAL) {
         const uint32_t ktile = entry & 0xFFu;
-        const uint32_t* tbp = a.tilebits + ((size_t)b * a.NT + ktile) * 32;
+        const uint32_t* tbp = a.tilebits + ((size_t)it.x * a.NT + ktile) * 32;
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
-          kd_pre[cc] = a.desc[(size_t)b * a.Tpad + (size_t)ktile * KD_TILE + i * 64 + (c0 + cc) * 32 + lane];
-          tb_pre[0][cc] = tbp[4 * TB_PRE + tbw + cc];
-          tb_pre[1][cc] = tbp[4 * TB_CTX + tbw + cc];
-          tb_pre[2][cc] = tbp[4 * TB_INS + tbw + cc];
+          kd_pre[cc] = __ldcg(a.desc + (size_t)it.x * a.Tpad + (size_t)ktile * KD_TILE + i * 64 + (c0 + cc) * 32 + lane);
+          tb_pre[0][cc] = __ldcg(tbp + 4 * TB_PRE + tbw + cc);
+          tb_pre[1][cc] = __ldcg(tbp + 4 * TB_CTX + tbw + cc);
+          tb_pre[2][cc] = __ldcg(tbp + 4 * TB_INS + tbw + cc);
         }
       }
     };
-    uint32_t ent_next = na > 0 ? sAct[0] : 0u;
-    if (na > 0) prefetch_kd(ent_next);
-    // per-row scalars of the next head are fetched while the current head is processed
-    float nxt_delta = q_valid ? a.delta[((size_t)b * a.H + h0) * a.T + qi] : 0.f;
-    float nxt_lse = q_valid ? a.lse[((size_t)b * a.H + h0) * a.T + qi] : 0.f;
-    // this stream's next unit, counted over all heads, as (unit / NBUF, unit % NBUF)
+    // The next item's header, query descriptor, first entry and scalars are fetched before the epilogue.
+    uint32_t ent_next = 0u, qd = 0u;
+    float delta = 0.f, lse = 0.f;
+    const uint16_t* list = lists;
+    auto open_item = [&](int k) -> bool {
+      const int slot = k % C::NITEM;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_Q_ITEMFULL))) return false;
+      it = uniform(sh.items[slot]);
+      if (it.w < 0) return false;
+      qd = __ldcg(a.desc + (size_t)it.x * a.Tpad + it.z * KD_TILE + row);
+      list = lists + slot * 128;
+      if (it.w > 0) {
+        ent_next = list[0];
+        prefetch_kd(ent_next);
+        const int qi = it.z * KD_TILE + row;
+        const size_t at = ((size_t)it.x * a.H + it.y) * a.T + min(qi, a.T - 1);   // (rows beyond the last have descriptor 0: hidden)
+        delta = __ldcg(a.delta + at);
+        lse = __ldcg(a.lse + at);
+      }
+      return true;
+    };
+    if (wait_ahead) pdl_wait();
+    if (warp == 4) pdl_launch_dependents();
+    int n_acc = 0;   // items with units so far
+    // this stream's next unit, counted over all items, as (unit / NBUF, unit % NBUF)
     int buf = i % C::NBUF;
     uint32_t rnd = i / C::NBUF;
-    const uint32_t sfull0 = smem_u32(&bar_s_full[0]), pfull0 = smem_u32(&bar_p_full[0]);
+    const uint32_t sfull0 = smem_u32(&sh.s_full[0]), pfull0 = smem_u32(&sh.p_full[0]);
     const uint32_t tcol = tbase + lane_base + c0 * 32;   // this thread's first chunk inside a buffer
 
-    for (int hh = 0; hh < nh && ok; ++hh) {
-      const int h = h0 + hh;
-      const float delta = nxt_delta, neg_lse = -nxt_lse;
-      if (hh + 1 < nh && q_valid) {
-        nxt_delta = a.delta[((size_t)b * a.H + h + 1) * a.T + qi];
-        nxt_lse = a.lse[((size_t)b * a.H + h + 1) * a.T + qi];
-      }
+    bool have = open_item(0);
+    for (int k = 0; have && ok; ++k) {
+      const int b = it.x, h = it.y, na = it.w, qi = it.z * KD_TILE + row;
       for (int e = 0; e < na; ++e) {
         const uint32_t ent = ent_next;
         const uint32_t cls = ent >> 8;
@@ -413,13 +529,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             todo &= ~__ballot_sync(0xffffffffu, mine);
           }
         }
-        // the next entry: of this head or, at the end of the list, the first one again for the next head
-        if (e + 1 < na || hh + 1 < nh) {
-          ent_next = sAct[e + 1 < na ? e + 1 : 0];
+        if (e + 1 < na) {
+          ent_next = list[e + 1];
           prefetch_kd(ent_next);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, W_Q_SFULL);
+        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_Q_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -434,15 +549,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (cls != KD_TILE_PARTIAL) {   // warp-uniform: the common case carries no mask code at all
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
-              const float p0 = fast_exp2(fmaf(__uint_as_float(rs[j]), c, neg_lse));
-              const float p1 = fast_exp2(fmaf(__uint_as_float(rs[j + 1]), c, neg_lse));
+              const float p0 = fast_exp2(fmaf(__uint_as_float(rs[j]), c, -lse));
+              const float p1 = fast_exp2(fmaf(__uint_as_float(rs[j + 1]), c, -lse));
               pk[j / 2] = pack2<kBf16>(p0 * (__uint_as_float(rp[j]) - delta), p1 * (__uint_as_float(rp[j + 1]) - delta));
             }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
-              float p0 = fast_exp2(fmaf(__uint_as_float(rs[j]), c, neg_lse));
-              float p1 = fast_exp2(fmaf(__uint_as_float(rs[j + 1]), c, neg_lse));
+              float p0 = fast_exp2(fmaf(__uint_as_float(rs[j]), c, -lse));
+              float p1 = fast_exp2(fmaf(__uint_as_float(rs[j + 1]), c, -lse));
               if ((mk[cc] & (1u << j)) == 0u) p0 = 0.f;
               if ((mk[cc] & (2u << j)) == 0u) p1 = 0.f;
               pk[j / 2] = pack2<kBf16>(p0 * (__uint_as_float(rp[j]) - delta), p1 * (__uint_as_float(rp[j + 1]) - delta));
@@ -460,9 +575,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
       if (!ok) break;
 
-      // epilogue of this head: warpgroup g stores EC columns of dQ from column g * EC
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.item_empty[k % C::NITEM]));
+      have = open_item(k + 1);
+      // epilogue of this item: warpgroup g stores EC columns of dQ from column g * EC
       if (na > 0) {
-        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, W_Q_ACCFULL);
+        ok = mbar_wait(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_Q_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -480,14 +598,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_wait_ld();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_acc_free));   // the next head's first product may overwrite the accumulator
+        if (lane == 0) mbar_arrive(smem_u32(&sh.acc_free));   // the next item's first product may overwrite the accumulator
       } else {
 #pragma unroll
         for (int cb = 0; cb < EC / ECH; ++cb)
 #pragma unroll
           for (int j = 0; j < ECH; ++j) r[cb][j] = 0u;
       }
-      if (q_valid) {
+      if (qi < a.T) {
 #pragma unroll
         for (int cb = 0; cb < EC / ECH; ++cb) {
           const int col = g * EC + cb * ECH;
@@ -502,19 +620,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
         }
       }
-    }
+    }  // items
   }
 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tbase, 512);
-  if (tid == 0) report_abort(&abortf, a.status);
+  if (tid == 0) report_abort(&sh.abortf, a.status);
 }
 
 // =========================================================================================
-// dK/dV kernel: one CTA per (b, group of heads, key tile); streams = query halves of the current
+// dK/dV kernel: items are key tiles; streams = query halves of the current
 // query tile.   M1(i): S^T_i = K Q_i^T, dP^T_i = V dO_i^T     M2(i): dV += P^T_i dO_i,  dK += dS^T_i Q_i
-// Heads are handled one after the other as in the dQ kernel.
 // =========================================================================================
 template <int HD, bool kBf16>
 __global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
@@ -527,114 +644,48 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t sFix = smem_u32(smem + C::SMEM_FIX);    // buffer f: K at +0, V at +TILE_BYTES
   const uint32_t sRing = smem_u32(smem + C::SMEM_RING);  // stage s: Q at +0, dO at +TILE_BYTES
   uint32_t* sStage = reinterpret_cast<uint32_t*>(smem + C::SMEM_STAGE);
-  uint16_t* sList = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
-
-  __shared__ __align__(8) uint64_t bar_fix_full[C::NFIX], bar_fix_empty[C::NFIX], bar_ring_full[C::STAGES],
-      bar_ring_empty[C::STAGES], bar_s_full[C::NBUF], bar_p_full[C::NBUF], bar_m2_issued[C::NBUF], bar_acc_full, bar_acc_free;
-  __shared__ uint32_t tmem_base_s;
-  __shared__ AbortFlag abortf;
+  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
+  __shared__ BwdShared<C> sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (!a.plan_ready) pdl_wait();   // reads ahead of the wait below go past L1, as in the dQ kernel
-  const int h0 = blockIdx.x * a.G, b = blockIdx.y;
-  const int nh = min(a.G, a.H - h0);   // this CTA handles heads h0 .. h0 + nh - 1
-  const int kt = __ldcg(a.order + ((size_t)b * 3 + 2) * a.NT + blockIdx.z);   // longest lists first
-  const int n = __ldcg(a.bwd_cnt + b * a.NT + kt);
-
-  if (tid == 0) {
-    abortf.v = 0;
-    for (int f = 0; f < C::NFIX; ++f) {
-      mbar_init(smem_u32(&bar_fix_full[f]), 1);
-      mbar_init(smem_u32(&bar_fix_empty[f]), 2);  // both M1 issuers are done with the head's K and V
-    }
-    for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(smem_u32(&bar_ring_full[s]), 1);
-      mbar_init(smem_u32(&bar_ring_empty[s]), 1);
-    }
-    for (int i = 0; i < C::NBUF; ++i) {
-      mbar_init(smem_u32(&bar_s_full[i]), 2);     // one commit from each of the two M1 issuers
-      mbar_init(smem_u32(&bar_p_full[i]), 4 * C::NSUB);   // one arrival per warp of the warpgroups that share the unit
-      mbar_init(smem_u32(&bar_m2_issued[i]), 1);
-    }
-    mbar_init(smem_u32(&bar_acc_full), 1);
-    mbar_init(smem_u32(&bar_acc_free), 8 * C::NSUB);      // every compute warp has read its part of dK and dV
-    fence_barrier_init();
-  }
+  if (tid == 0) bwd_init<C>(sh);
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_base_s), 512);
+    tmem_alloc(smem_u32(&sh.tmem_base), 512);
     tmem_relinquish();
-  }
-  if (warp == 2) {
-    const uint16_t* glist = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
-    for (int e = lane; e < n; e += 32) sList[e] = __ldcg(glist + e);
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  pdl_wait();
-  pdl_launch_dependents();
-  const uint32_t tbase = tmem_base_s;
-  const uint16_t* list = sList;
+  // Directly behind the dQ kernel of the same call there is nothing to wait for: that kernel lets this one start when it has itself waited
+  // for the delta kernel, and the last CTAs of the one overlap the first of the other (1 x 16 x 500 x 128 30 -> 22.5 us together). The
+  // dQ kernel's end is awaited at the end, so that whatever comes next finds both complete (what a successor reads ahead of its own wait
+  // is a plan, which no backward writes). Everything that this kernel reads is read past L1.
+  const bool wait_ahead = a.after_dq == 0 && a.plan_ready != 0;
+  if (a.after_dq == 0 && !wait_ahead) pdl_wait();
+  const uint32_t tbase = sh.tmem_base;
 
   if (warp < 4) {
     reg_dealloc<KD_REGS_ISSUE>();
-    if (warp == 0 && lane == 0 && n > 0) {
-      // ------------------------------ TMA producer ------------------------------
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
-      tma_prefetch_desc(&tmDO);
-      int issued = 0, fix_issued = 0;   // ring entries / resident pairs requested so far, over all heads
-      bool ok = true;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const int h = h0 + hh, fb = hh % C::NFIX;
-        if (hh >= C::NFIX) {
-          ok = mbar_wait(smem_u32(&bar_fix_empty[fb]), (hh / C::NFIX - 1) & 1, &abortf, W_K_FIXEMPTY);
-          if (!ok) break;
-        }
-        mbar_arrive_expect_tx(smem_u32(&bar_fix_full[fb]), 2 * C::TILE_BYTES);
-        for (int kb = 0; kb < C::KBLK; ++kb) {
-          tma_load_4d(sFix + fb * 2 * C::TILE_BYTES + kb * 16384, &tmK, smem_u32(&bar_fix_full[fb]), kb * 64, kt * KD_TILE, h, b);
-          tma_load_4d(sFix + fb * 2 * C::TILE_BYTES + C::TILE_BYTES + kb * 16384, &tmV, smem_u32(&bar_fix_full[fb]), kb * 64, kt * KD_TILE, h, b);
-        }
-        fix_issued = hh + 1;
-        for (int e = 0; e < n; ++e) {
-          const int s = issued % C::STAGES;
-          const uint32_t ph = (issued / C::STAGES) & 1;
-          const int qt = list[e] & 0xFF;
-          ok = mbar_wait(smem_u32(&bar_ring_empty[s]), ph ^ 1, &abortf, W_K_RINGEMPTY);
-          if (!ok) break;
-          mbar_arrive_expect_tx(smem_u32(&bar_ring_full[s]), 2 * C::TILE_BYTES);
-          const uint32_t dst = sRing + s * 2 * C::TILE_BYTES;
-          for (int kb = 0; kb < C::KBLK; ++kb) {
-            tma_load_4d(dst + kb * 16384, &tmQ, smem_u32(&bar_ring_full[s]), kb * 64, qt * KD_TILE, h, b);
-            tma_load_4d(dst + C::TILE_BYTES + kb * 16384, &tmDO, smem_u32(&bar_ring_full[s]), kb * 64, qt * KD_TILE, h, b);
-          }
-          ++issued;
-        }
-      }
-      if (abortf.v != 0) {   // let the copies in flight land before the CTA exits
-        for (int e = max(0, issued - C::STAGES); e < issued; ++e)
-          for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&bar_ring_full[e % C::STAGES]), (e / C::STAGES) & 1); ++spin) {}
-        for (int f = max(0, fix_issued - C::NFIX); f < fix_issued; ++f)
-          for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(smem_u32(&bar_fix_full[f % C::NFIX]), (f / C::NFIX) & 1); ++spin) {}
-      }
-    } else if ((warp == 3 || warp == 2) && lane == 0 && n > 0) {
+    if (warp == 0) {
+      bwd_producer<HD, false>(tmK, tmV, tmQ, tmDO, a, sFix, sRing, lists, sh, lane, wait_ahead);
+    } else if ((warp == 3 || warp == 2) && lane == 0) {
       // ------------------------------ M1 issuers: warp 3: S^T_u = K Q_u^T; warp 2: dP^T_u = V dO_u^T ------------------------------
       const bool dp_part = (warp == 2);
       const uint32_t idesc_m1 = make_idesc_f16(kBf16, 0, 0, KD_TILE, 64);   // N = 64 queries
       const uint32_t hi = desc_hi_sw128();
       const uint32_t loRingK = desc_lo_kmajor(sRing);
-      const int U = 2 * n;
       bool ok = true;
-      int buf = 0, round = 0, stage = 0;   // run on across the heads
+      int buf = 0, round = 0, stage = 0, item = 0;   // run on across the items; item: of those with entries
       uint32_t ring_parity = 0;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        const int fb = hh % C::NFIX;
-        ok = mbar_wait(smem_u32(&bar_fix_full[fb]), (hh / C::NFIX) & 1, &abortf, W_K_FIXFULL);
+      int4 it;
+      for (int k = 0; ok && bwd_header<C>(sh, k, W_K_ITEMFULL, it) && it.w >= 0; ++k) {
+        if (it.w == 0) continue;
+        const int U = 2 * it.w, fb = item % C::NFIX;
+        ok = mbar_wait(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_K_FIXFULL);
+        ++item;
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // V or K
-        uint64_t adesc[HD / 16];   // A descriptors of the head's k-steps
+        uint64_t adesc[HD / 16];   // A descriptors of the item's k-steps
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) adesc[kk] = desc64(loA + koff_kmajor(kk), hi);
         for (int u = 0; u < U && ok; ++u) {
@@ -647,36 +698,38 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&bar_m2_issued[buf]), (round - 1) & 1, &abortf, W_K_M2ISSUED);
+            ok = mbar_wait(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_K_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its Q and dO tiles must have landed
-            ok = mbar_wait(smem_u32(&bar_ring_full[stage]), ring_parity, &abortf, W_K_RINGFULL);
+            ok = mbar_wait(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_K_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
           mma_ss64<false>(dst, adesc[0], bdesc[0], idesc_m1);
 #pragma unroll
           for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(dst, adesc[kk], bdesc[kk], idesc_m1);
-          mma_commit(smem_u32(&bar_s_full[buf]));
+          mma_commit(smem_u32(&sh.s_full[buf]));
           if (++buf == C::NBUF) { buf = 0; ++round; }
           if (i == 1 && ++stage == C::STAGES) { stage = 0; ring_parity ^= 1; }
         }
-        if (ok) mma_commit(smem_u32(&bar_fix_empty[fb]));   // this issuer's products of the head no longer read K / V
+        if (ok) mma_commit(smem_u32(&sh.fix_empty[fb]));   // this issuer's products of the item no longer read K / V
       }
-    } else if (warp == 1 && lane == 0 && n > 0) {
+    } else if (warp == 1 && lane == 0) {
       // ------------------------------ M2 issuer: dV += P^T_u dO_u, dK += dS^T_u Q_u ------------------------------
       const uint32_t idesc_m2 = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);   // B = dO / Q rows, MN-major
       const uint32_t tDK = tbase + C::TM_ACC0, tDV = tbase + C::TM_ACC1;
       const uint32_t hi = desc_hi_sw128();
       const uint32_t loRingMN = desc_lo_mnmajor(sRing);
-      const int U = 2 * n;
       bool ok = true;
-      int buf = 0, stage = 0;
+      int buf = 0, stage = 0, item = 0;
       uint32_t round_parity = 0;
-      for (int hh = 0; hh < nh && ok; ++hh) {
-        if (hh > 0) {   // the previous head's dK and dV must have been read out of the accumulators
-          ok = mbar_wait(smem_u32(&bar_acc_free), (hh - 1) & 1, &abortf, W_K_ACCFREE);
+      int4 it;
+      for (int k = 0; ok && bwd_header<C>(sh, k, W_K_ITEMFULL, it) && it.w >= 0; ++k) {
+        if (it.w == 0) continue;
+        const int U = 2 * it.w;
+        if (item++ > 0) {   // the previous item's dK and dV must have been read out of the accumulators
+          ok = mbar_wait(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_K_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -694,7 +747,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             bdo[kk] = desc64(dob + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&bar_p_full[buf]), round_parity, &abortf, W_K_PFULL);
+          ok = mbar_wait(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_K_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           // dV += P^T_u dO_u   (P^T_u on top of S^T_u)
@@ -705,13 +758,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           mma_ts64_p(tDK, aop[0] + 64, bq[0], idesc_m2, u > 0 ? 1u : 0u);
 #pragma unroll
           for (int kk = 1; kk < 4; ++kk) mma_ts64<true>(tDK, aop[kk] + 64, bq[kk], idesc_m2);
-          if (i == 1) mma_commit(smem_u32(&bar_ring_empty[stage]));
+          if (i == 1) mma_commit(smem_u32(&sh.ring_empty[stage]));
           tc_fence_before_sync();
-          mbar_arrive(smem_u32(&bar_m2_issued[buf]));
+          mbar_arrive(smem_u32(&sh.m2_issued[buf]));
           if (++buf == C::NBUF) { buf = 0; round_parity ^= 1; }
           if (i == 1 && ++stage == C::STAGES) stage = 0;
         }
-        if (ok) mma_commit(smem_u32(&bar_acc_full));
+        if (ok) mma_commit(smem_u32(&sh.acc_full));
       }
     }
   } else {
@@ -724,15 +777,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int c0 = (g % C::NSUB) * CPT;   // first 32-query chunk of that half handled here
     const int wq = warp & 3;
     const int row = wq * 32 + lane;
-    const int kj = kt * KD_TILE + row;   // this thread's key
-    const bool k_valid = kj < a.T;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     uint32_t* st_buf = sStage + (size_t)(warp - 4) * C::STAGE_WORDS;  // [QW lse][QW delta]
     const float c = a.scale_log2;
-    const uint32_t kdesc = a.desc[(size_t)b * a.Tpad + kj];
     const int tbw = 2 * i + c0;      // first word of this thread's chunks in the 128-bit class masks of a query tile
     bool ok = true;
 
+    int4 it = make_int4(0, 0, 0, 0);   // the item in hand; behind its last unit the next one
     // LSE, delta and the descriptors of the next unit's queries are fetched one unit ahead
     // into registers and handed to the warp through its shared-memory staging buffer
     float pre_lse[CPT], pre_delta[CPT];
@@ -747,14 +798,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     }
     auto prefetch = [&](uint32_t entry, int h) {
       if ((entry >> 8) == KD_TILE_PARTIAL) {
-        const uint32_t* tbp = a.tilebits + ((size_t)b * a.NT + (entry & 0xFFu)) * 32;
+        const uint32_t* tbp = a.tilebits + ((size_t)it.x * a.NT + (entry & 0xFFu)) * 32;
 #pragma unroll
         for (int cc = 0; cc < CPT; ++cc) {
-          tb_pre[0][cc] = tbp[4 * TB_SEES_PRE + tbw + cc];
-          tb_pre[1][cc] = tbp[4 * TB_SEES_CTX + tbw + cc];
-          tb_pre[2][cc] = tbp[4 * TB_SEES_INS + tbw + cc];
-          tb_pre[3][cc] = tbp[4 * TB_CTX + tbw + cc];
-          tb_pre[4][cc] = tbp[4 * TB_SIDPOS + tbw + cc];
+          tb_pre[0][cc] = __ldcg(tbp + 4 * TB_SEES_PRE + tbw + cc);
+          tb_pre[1][cc] = __ldcg(tbp + 4 * TB_SEES_CTX + tbw + cc);
+          tb_pre[2][cc] = __ldcg(tbp + 4 * TB_SEES_INS + tbw + cc);
+          tb_pre[3][cc] = __ldcg(tbp + 4 * TB_CTX + tbw + cc);
+          tb_pre[4][cc] = __ldcg(tbp + 4 * TB_SIDPOS + tbw + cc);
         }
       }
       // a query at or beyond the sequence length reads the last row's scalars: its descriptor is 0,
@@ -762,22 +813,41 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
         const int q = (entry & 0xFF) * KD_TILE + i * 64 + (c0 + cc) * 32 + lane;
-        const size_t r = ((size_t)b * a.H + h) * a.T + min(q, a.T - 1);
-        pre_lse[cc] = a.lse[r];   // negated where it is used: a negation here would wait for the load
-        pre_delta[cc] = a.delta[r];
-        pre_desc[cc] = a.desc[(size_t)b * a.Tpad + q];
+        const size_t r = ((size_t)it.x * a.H + h) * a.T + min(q, a.T - 1);
+        pre_lse[cc] = __ldcg(a.lse + r);   // negated where it is used: a negation here would wait for the load
+        pre_delta[cc] = __ldcg(a.delta + r);
+        pre_desc[cc] = __ldcg(a.desc + (size_t)it.x * a.Tpad + q);
       }
     };
-    uint32_t ent_next = n > 0 ? list[0] : 0u;
-    if (n > 0) prefetch(ent_next, h0);
-    // this stream's next unit, counted over all heads, as (unit / NBUF, unit % NBUF)
+    // The next item's header, key descriptor and first unit's scalars are fetched before the epilogue.
+    uint32_t ent_next = 0u, kdesc = 0u;
+    const uint16_t* list = lists;
+    auto open_item = [&](int k) -> bool {
+      const int slot = k % C::NITEM;
+      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_K_ITEMFULL))) return false;
+      it = uniform(sh.items[slot]);
+      if (it.w < 0) return false;
+      kdesc = __ldcg(a.desc + (size_t)it.x * a.Tpad + it.z * KD_TILE + row);
+      list = lists + slot * 128;
+      if (it.w > 0) {
+        ent_next = list[0];
+        prefetch(ent_next, it.y);
+      }
+      return true;
+    };
+    if (wait_ahead) pdl_wait();
+    if (warp == 4) pdl_launch_dependents();
+    int n_acc = 0;   // items with units so far
+    // this stream's next unit, counted over all items, as (unit / NBUF, unit % NBUF)
     int buf = i % C::NBUF;
     uint32_t rnd = i / C::NBUF;
-    const uint32_t sfull0 = smem_u32(&bar_s_full[0]), pfull0 = smem_u32(&bar_p_full[0]);
+    const uint32_t sfull0 = smem_u32(&sh.s_full[0]), pfull0 = smem_u32(&sh.p_full[0]);
     const uint32_t tcol = tbase + lane_base + c0 * 32;   // this thread's first chunk inside a buffer
 
-    for (int hh = 0; hh < nh && ok; ++hh) {
-      const int h = h0 + hh;
+    bool have = open_item(0);
+    for (int k = 0; have && ok; ++k) {
+    const int4 now = it;
+      const int n = now.w;
       for (int e = 0; e < n; ++e) {
         const uint32_t ent = ent_next;
         const uint32_t cls = ent >> 8;
@@ -793,7 +863,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int cc = 0; cc < CPT; ++cc) mk[cc] = 0xFFFFFFFFu;
         if (cls == KD_TILE_PARTIAL) {
           const int i0 = (ent & 0xFF) * KD_TILE + i * 64 + c0 * 32;  // first query handled here
-          key_row_mask<CPT>(kdesc, kj, i0, tb_pre[0], tb_pre[1], tb_pre[2], tb_pre[3], mk);
+          key_row_mask<CPT>(kdesc, now.z * KD_TILE + row, i0, tb_pre[0], tb_pre[1], tb_pre[2], tb_pre[3], mk);
           uint32_t any_armed = 0u;
 #pragma unroll
           for (int cc = 0; cc < CPT; ++cc) any_armed |= tb_pre[4][cc];
@@ -812,16 +882,12 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             todo &= ~__ballot_sync(0xffffffffu, mine);
           }
         }
-        // the next entry: of this head or, at the end of the list, the first one again for the next head
         if (e + 1 < n) {
           ent_next = list[e + 1];
-          prefetch(ent_next, h);
-        } else if (hh + 1 < nh) {
-          ent_next = list[0];
-          prefetch(ent_next, h + 1);
+          prefetch(ent_next, now.y);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &abortf, W_K_SFULL);
+        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_K_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -881,9 +947,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       if (!ok) break;
 
-      // epilogue of this head: warpgroup g stores EC columns of dK and dV from column g * EC
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.item_empty[k % C::NITEM]));
+      have = open_item(k + 1);
+      // (the fields are taken here and not before: carried through the loop they cost the head-dim-64 kernel its last registers)
+      const int b = now.x, h = now.y, kj = now.z * KD_TILE + row;
+      // epilogue of this item: warpgroup g stores EC columns of dK and dV from column g * EC
       if (n > 0) {
-        ok = mbar_wait(smem_u32(&bar_acc_full), hh & 1, &abortf, W_K_ACCFULL);
+        ok = mbar_wait(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_K_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -907,14 +978,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           if (cb == EC / ECH - 1) {
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_acc_free));   // the next head's first products may overwrite the accumulators
+            if (lane == 0) mbar_arrive(smem_u32(&sh.acc_free));   // the next item's first products may overwrite the accumulators
           }
         } else {
 #pragma unroll
           for (int j = 0; j < ECH; ++j) { rk[j] = 0u; rv[j] = 0u; }
         }
         const int col = g * EC + cb * ECH;
-        if (k_valid && !kBf16 && a.grads_f32) {
+        if (kj < a.T && !kBf16 && a.grads_f32) {
           float* kw = static_cast<float*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st + col;
           float* vw = static_cast<float*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st + col;
           if constexpr (ECH == 16) {
@@ -924,7 +995,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             store_row32_f32_upto(kw, rk, a.sm_scale, col, a.d_real);
             store_row32_f32_upto(vw, rv, 1.0f, col, a.d_real);
           }
-        } else if (k_valid) {
+        } else if (kj < a.T) {
           if constexpr (ECH == 16) {
             store_row16_upto<kBf16>(krow + cb * ECH, rk, a.sm_scale, g * EC + cb * ECH, a.d_real);
             store_row16_upto<kBf16>(vrow + cb * ECH, rv, 1.0f, g * EC + cb * ECH, a.d_real);
@@ -934,13 +1005,14 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
         }
       }
-    }
+    }  // items
   }
 
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tbase, 512);
-  if (tid == 0) report_abort(&abortf, a.status);
+  if (tid == 0) report_abort(&sh.abortf, a.status);
+  if (a.after_dq != 0) pdl_wait();
 }
 
 template <int HD, bool kBf16>
@@ -957,7 +1029,6 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.d_real = p.D;
   a.scale_log2 = scale_log2_of(p.sm_scale);
   a.sm_scale = p.sm_scale;
-  a.G = heads_per_cta((long long)p.B * p.H, p.H, L.NT, p.heads_per_cta, sm_count());
   a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
   a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
@@ -965,6 +1036,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.lse = p.lse; a.delta = p.delta;
   // with the delta kernel ahead of them in this call, the plan was complete before the kernels may start
   a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
+  a.after_dq = 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
   a.grads_f32 = f32 != nullptr;
   a.zero_dq = f32 != nullptr && fused;
@@ -982,7 +1054,10 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   cudaError_t e = opt_in_q(kq, C::SMEM_ALLOC);
   if (e == cudaSuccess) e = opt_in_k(kk, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "bwd smem attribute: %s", cudaGetErrorString(e));
-  dim3 grid((p.H + a.G - 1) / a.G, p.B, L.NT);
+  const long long n_items = fused ? 0 : (long long)p.B * p.H * L.NT;
+  if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
+  const unsigned grid = static_cast<unsigned>(n_items);
+  a.order_of = ItemOrder::make(p.B * p.H, L.NT, (double)p.T * p.D * 2 * 5, 64e6);   // Q, K, V, dO and a gradient
   const int phases = (p.bwd_phases & 3) ? (p.bwd_phases & 3) : 3;
   if (phases & 1) {
     const size_t rows = (size_t)p.B * p.H * p.T;
@@ -998,6 +1073,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
     // bwd_phases 1: the delta kernel alone (it also zeroes dq_acc); 2: the fused kernel and the conversion
     if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, (phases & 1) != 0, stream);
   } else if ((phases & 2) && e == cudaSuccess) {
+    a.after_dq = phases & 1;
     e = launch(kk, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_bwd kernels launch: %s", cudaGetErrorString(e));

@@ -6,7 +6,8 @@ namespace kd {
 
 struct BwdArgs {
   int B, H, T, NT, NP, Tpad;
-  int G;             // heads per CTA
+  ItemOrder order_of;   // of the two-kernel backward's items
+  int after_dq;      // dK/dV kernel: the dQ kernel of the same call is the kernel before this one on the stream
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;

@@ -494,7 +494,7 @@ Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
 struct Options {
   double sm_scale;
   bool like_input, deterministic;
-  int heads_per_cta;   // of the deterministic backward
+  int heads_per_cta;   // kd_attn_params.heads_per_cta
 };
 
 // dQ, dK, dV of one flash_attention call. Saves the operands the kernels read: for float32 tensors their float16

@@ -18,16 +18,10 @@ namespace kd {
 // A call by itself gains in all of them or is level.
 inline int split_pairs(long long pairs, int tiles, int sms) { return tiles > 1 && (4 * pairs <= sms || (tiles >= 5 && 2 * pairs <= sms)) ? 1 : 0; }
 
-// Deterministic backward: heads that a CTA handles one after the other (they share the plan's work list, so the list staging, the TMEM
-// allocation and the pipeline fill are paid once). As many as keep six CTAs per SM, at most eight: fewer CTAs lose more to imbalance
-// between sequences of different section lengths than the shared fill saves. Up to twelve tiles per SM that is one; two pay where an item
-// is short against a CTA's start and drain (6 us), and long lists need more of them to balance. `tiles`: tiles of a head, also the longest list.
-// Time with two heads over time with one, D = 64, hierarchical | causal | no mask, for 5.2, 7.1, 9.1 tiles per SM (D = 128: within 0.06 of it):
-//   T = 1000  .87 .87 .84 | .91 .90 .88 | .96 .95 .94       T = 2048  .92 .91 .89 | .97 .94 .93 | .98 .97 .98
-//   T = 2600 1.02 .94 .91 | .98 .95 .94 | 1.02 1.00 1.00    T = 4096 1.26 1.00 .95 | 1.02 .97 .96 | 1.00 .99 .99
-//   T = 8192, 6.9 per SM: - | .98 | 1.10; 10.4: 1.01 | .98 | 1.07.   T = 16384, 5.2: - | 1.06 | -
-// Lists of equal length, which only calls without a mask have, still lose where the last wave is nearly empty (6.5 per SM: 1.03-1.09);
-// the lists are on the device.
+// Heads that a CTA of a grid with a CTA per (tile, group of heads) should handle one after the other: as many as keep six CTAs per SM, at
+// most eight, and two where lists are short against a CTA's start and drain. The kernels take single items dynamically now and ask
+// nobody (a grouped item costs balance and saves nothing: 16 x 16 x 4096 x 64 hierarchical, dQ kernel 699 us with groups, 598 without);
+// for hosts that size such a grid themselves. `tiles`: tiles of a head.
 inline int heads_per_cta(long long pairs, int heads, int tiles, int forced, int sms) {   // pairs: (batch, head) pairs
   if (forced >= 1) return forced < heads ? forced : heads;
   const long long ctas = pairs * tiles;

@@ -32,9 +32,7 @@ __all__ = ["flash_attention", "generate_hadamard_signs", "hadamard_transform"]
 _HADAMARD_DIMS = (16, 32, 64, 128)
 _DTYPES = {torch.float16: _capi.KD_F16, torch.bfloat16: _capi.KD_BF16}
 
-# Heads a CTA of the deterministic backward handles one after the other (kd_attn_params.heads_per_cta): 0 lets the library
-# choose from the grid size. Small problems get 1 by themselves, so the tests of the multi-head path set this. The forward
-# and the fused backward take their work items one by one and have no use for it.
+# kd_attn_params.heads_per_cta, which the library accepts and ignores: its kernels take tiles of single heads.
 HEADS_PER_CTA = 0
 
 

@@ -10,7 +10,6 @@ sys.path.insert(0, os.path.join(os.path.dirname(os.path.abspath(__file__)), "gol
 from cocktail_inputs import cocktail_rows, embeddings  # noqa: E402
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 from oracle import attention_oracle as ao  # noqa: E402
-from helpers import rand_inputs  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -212,6 +211,7 @@ def test_host_thread_without_a_cuda_context():
 def test_float32_results_are_not_rounded_to_16_bits(B, H, T, D, layout, deterministic):
     """float32 O, dQ, dK and dV are written by the attention kernels: rows and columns at the edges of tiles and boxes, memory orders,
     sequences that end early (rows without keys, key tiles without queries). Errors are those of the float16 operands alone."""
+    from tests.helpers import rand_inputs
     from kerneldev_b200 import flash_attention
     q, k, v, do = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.float32, seed=T + D))
     if layout == "bthd":
@@ -238,3 +238,23 @@ def test_float32_results_are_not_rounded_to_16_bits(B, H, T, D, layout, determin
     ones = torch.autograd.grad(o, (qg, kg, vg), torch.ones((B, H, T, D), device=DEV))
     for x, y in list(zip(grads, again)) + list(zip(expanded, ones)):
         assert float((x - y).norm()) <= (0.0 if deterministic else 1e-5) * float(y.norm())   # dQ's sums have no fixed order
+
+
+@pytest.mark.parametrize("B,H,T,D", [(6, 40, 300, 64), (6, 40, 300, 128), (40, 9, 129, 48), (3, 50, 513, 112)])
+def test_deterministic_backward_takes_further_items(B, H, T, D):
+    """More tiles than SMs, so that CTAs of both kernels run on into other heads, tiles and sequences; runs of tiles without entries
+    (sequences of no or few tokens) between those with some, longer than the ring of item headers. Twice the same bits."""
+    from tests.helpers import assert_close, rand_inputs
+    from kerneldev_b200 import flash_attention
+    q, k, v, do = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.bfloat16, seed=T + D))
+    lens = torch.tensor([(T, 0, 1, T // 2, T - 1, 128)[b % 6] for b in range(B)], dtype=torch.int32, device=DEV)
+    qg, kg, vg = (x.detach().requires_grad_() for x in (q, k, v))
+    o = flash_attention(qg, kg, vg, lens=lens, causal=True, deterministic=True)
+    one = torch.autograd.grad(o, (qg, kg, vg), do, retain_graph=True)
+    two = torch.autograd.grad(o, (qg, kg, vg), do)
+    assert all(torch.equal(x, y) for x, y in zip(one, two))
+    mask = ao.dense_mask(T, None, None, None, lens.cpu().numpy(), causal=True, B=B)
+    heads = [0, H // 2, H - 1]
+    _, _, *ref = ao.attention_fwd_bwd(*(x[:, heads].cpu() for x in (q, k, v, do)), mask)
+    for name, got, want in zip(("dQ", "dK", "dV"), one, ref):
+        assert_close(name, got[:, heads], want)
