@@ -105,3 +105,17 @@ def test_span_id_out_of_range_is_reported():
     ins = np.zeros((1, T), bool); ins[0, 5] = True
     with pytest.raises(ValueError, match="span_id"):
         _plan(T, ins, sid, None)
+
+
+# one CTA per sequence up to 1024 tokens and 16 sequences, two kernels beyond
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (2, 129), (16, 300), (17, 300), (16, 1024), (1, 1025), (17, 1024)])
+def test_both_forms_of_the_plan_kernels(B, T):
+    ins, sid, pre = random_meta(B + T, B, T, sid_range=(-1, 9))
+    lens = np.array([(T, 0, 1, T - 1, T // 2)[b % 5] for b in range(B)], np.int32)
+    _check(_plan(T, ins, sid, pre, lens), ao.dense_mask(T, ins, sid, pre, lens))
+    _check(_plan(T, ins, sid, pre, None), ao.dense_mask(T, ins, sid, pre, None))
+    # a span id that does not fit is reported from any sequence, and not from behind a sequence's end
+    sid[B - 1, T - 1] = -(1 << 23) - 1
+    with pytest.raises(ValueError, match="span_id"):
+        _plan(T, ins, sid, pre, None)
+    _plan(T, ins, sid, pre, np.full(B, T - 1, np.int32))
