@@ -256,7 +256,7 @@ typedef struct {
 } kd_cocktail;
 
 /* kd_span_index, which also writes the [SPAN] counts to counts_host (B int32 of pinned host memory; they are there once
- * the stream has been synchronised). */
+ * the stream has been synchronised, and a word that held -1 may be taken as soon as it does not). */
 int kd_cocktail_index(const int64_t* tokens, int64_t stride_b, int32_t B, int32_t T, int64_t tok_span, int64_t tok_es,
                       int64_t tok_mask, int32_t* starts, int32_t* ends, int32_t* n_starts, int32_t* n_ends,
                       int32_t* first_mask, int32_t* counts_host, void* stream);

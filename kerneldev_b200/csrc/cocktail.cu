@@ -63,6 +63,8 @@ span_index_kernel(const int64_t* __restrict__ tokens, int64_t stride_b, int T, i
     int p_span = c_span + __reduce_add_sync(0xffffffffu, lane < warp ? w_span : 0);
     int p_es = c_es + __reduce_add_sync(0xffffffffu, lane < warp ? w_es : 0);
     first = min(first, __reduce_min_sync(0xffffffffu, s_mask[lane]));
+    // the count is what the host waits for: it leaves as soon as it is known
+    if (counts_host != nullptr && threadIdx.x == 0 && base + SI_CHUNK >= T) *const_cast<volatile int32_t*>(counts_host + b) = c_span + tot_span;
 #pragma unroll
     for (int r = 0; r < SI_PER; ++r) {
       if ((bs[r] >> lane) & 1u) row_st[p_span + __popc(bs[r] & below)] = t0 + 32 * r;
@@ -80,7 +82,6 @@ span_index_kernel(const int64_t* __restrict__ tokens, int64_t stride_b, int T, i
     n_starts[b] = c_span;
     n_ends[b] = c_es;
     first_mask[b] = first < T ? first : -1;
-    if (counts_host != nullptr) counts_host[b] = c_span;
   }
 }
 

@@ -11,6 +11,7 @@
 #include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
@@ -18,6 +19,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 
 #include <atomic>
+#include <chrono>
 #include <deque>
 #include <list>
 #include <mutex>
@@ -30,6 +32,17 @@ using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 
 namespace {
+
+// Uninitialised device tensors from torch's CUDA allocator without the trip through the dispatcher, which is most of what at::empty
+// costs: a forward allocates two and a backward five (0.4 us each: a forward's host time without its launch 5.0 -> 4.3 us).
+Tensor empty_on(at::IntArrayRef sizes, at::ScalarType type, at::Device device) {
+  return Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
+}
+// in the memory order of a dense tensor, as at::empty_like
+Tensor empty_like_of(const Tensor& like, at::ScalarType type) {
+  if (!like.is_non_overlapping_and_dense()) return at::empty_like(like, like.options().dtype(type));
+  return Tensor(at::detail::empty_strided_cuda(like.sizes(), like.strides(), type, like.device()));
+}
 
 // ---- the library -----------------------------------------------------------------------------------------------
 
@@ -157,7 +170,7 @@ struct Plan {
       : B(B_), T(T_), device(dev), built_on(at::cuda::getCurrentCUDAStream(dev.index())) {
     check(lib.plan_layout_get(static_cast<int32_t>(B), static_cast<int32_t>(T), &layout));
     // the caching allocator returns 512-byte aligned blocks, which covers the 256 the ABI asks for
-    buf = at::empty({static_cast<int64_t>(layout.total)}, at::TensorOptions().dtype(at::kByte).device(dev));
+    buf = empty_on({static_cast<int64_t>(layout.total)}, at::kByte, dev);
     kd_meta meta{};
     meta.B = layout.B;
     meta.T = layout.T;
@@ -359,8 +372,7 @@ Tensor usable(const Tensor& t) { return tma_ready(t) ? t : t.contiguous(); }
 
 Tensor empty_out(const Tensor& like, bool like_input, at::ScalarType type) {
   // empty_like keeps the strides of a dense tensor, e.g. (B,T,H,D) memory seen as (B,H,T,D)
-  const auto options = like.options().dtype(type);
-  return like_input ? at::empty_like(like, options) : at::empty(like.sizes(), options);
+  return like_input ? empty_like_of(like, type) : empty_on(like.sizes(), type, like.device());
 }
 Tensor empty_out(const Tensor& like, bool like_input) { return empty_out(like, like_input, like.scalar_type()); }
 
@@ -393,7 +405,7 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Ten
     *o32 = empty_out(q, like_input, at::kFloat);
     f.o = desc(*o32);
   }
-  if (want_lse) lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
+  if (want_lse) lse = empty_on({q.size(0), q.size(1), q.size(2)}, at::kFloat, q.device());
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
@@ -416,7 +428,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   Tensor d_o;
   if (!f32 || d_o_.scalar_type() != at::kFloat) {
     d_o = usable(d_o_);
-  } else if (Tensor copy = at::empty_like(d_o_, d_o_.options().dtype(at::kHalf)); aligned(d_o_) && tma_ready(copy)) {
+  } else if (Tensor copy = empty_like_of(d_o_, at::kHalf); aligned(d_o_) && tma_ready(copy)) {
     d_o = copy;   // filled by the delta kernel
     f.d_o = desc(d_o_);
   } else {
@@ -428,11 +440,10 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
     dk = empty_out(k, like_input, type);
     dv = empty_out(v, like_input, type);
   }
-  const auto f32_options = q.options().dtype(at::kFloat);
-  if (!delta.defined()) delta = at::empty({q.size(0), q.size(1), q.size(2)}, f32_options);
+  if (!delta.defined()) delta = empty_on({q.size(0), q.size(1), q.size(2)}, at::kFloat, q.device());
   const bool fused = !deterministic;
   // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
-  if (fused && !f32 && !dq_acc.defined()) dq_acc = at::empty({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, f32_options);
+  if (fused && !f32 && !dq_acc.defined()) dq_acc = empty_on({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, at::kFloat, q.device());
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
   p.heads_per_cta = heads_per_cta;
   p.d_o = desc(d_o);
@@ -461,7 +472,7 @@ std::array<Tensor, KD_CAST_MAX> cast(std::initializer_list<Tensor> in, at::Scala
   int n = 0, slot = 0;
   const Tensor& first = *in.begin();
   for (const Tensor& x : in) {
-    Tensor y = at::empty_like(x, x.options().dtype(to));
+    Tensor y = empty_like_of(x, to);
     if (x.numel() > 0 && x.scalar_type() != to && aligned(x) && aligned(y)) {
       src[n] = desc(x);
       dst[n++] = desc(y);
@@ -480,7 +491,7 @@ std::array<Tensor, KD_CAST_MAX> cast(std::initializer_list<Tensor> in, at::Scala
 
 Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
   const Tensor x = usable(x_);
-  Tensor y = at::empty(x.sizes(), x.options());
+  Tensor y = empty_on(x.sizes(), x.scalar_type(), x.device());
   const kd_tensor xs = desc(x), ys = desc(y);
   c10::cuda::CUDAGuard guard(x.device());
   check(lib.hadamard(&xs, &ys, static_cast<int32_t>(x.size(0)), static_cast<int32_t>(x.size(1)), static_cast<int32_t>(x.size(2)),
@@ -627,9 +638,9 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
 std::tuple<Tensor, Tensor, Tensor> metadata_from_tokens(const Tensor& tokens_, int64_t tok_span, int64_t tok_es, int64_t tok_cls, int64_t tok_maskq) {
   const Tensor tokens = tokens_.stride(1) == 1 ? tokens_ : tokens_.contiguous();
   const int64_t B = tokens.size(0), T = tokens.size(1);
-  Tensor in_span = at::empty({B, T}, tokens.options().dtype(at::kBool));
-  Tensor span_id = at::empty({B, T}, tokens.options());
-  Tensor is_prefix = at::empty({B, T}, tokens.options().dtype(at::kBool));
+  Tensor in_span = empty_on({B, T}, at::kBool, tokens.device());
+  Tensor span_id = empty_on({B, T}, at::kLong, tokens.device());
+  Tensor is_prefix = empty_on({B, T}, at::kBool, tokens.device());
   c10::cuda::CUDAGuard guard(tokens.device());
   check(lib.metadata_from_tokens(tokens.data_ptr<int64_t>(), B > 1 ? tokens.stride(0) : std::max<int64_t>(T, 1), static_cast<int32_t>(B),
                                  static_cast<int32_t>(T), tok_span, tok_es, tok_cls, tok_maskq, static_cast<uint8_t*>(in_span.data_ptr()),
@@ -720,7 +731,7 @@ struct CocktailBackward : torch::autograd::Node {
     at::NoGradGuard no_grad;
     const Tensor ds = grads[0].defined() ? grads[0].contiguous() : at::zeros({p.B, p.S}, like.options());
     // without a span nothing reaches x, and there is no kernel to write the zeros
-    Tensor gx = p.S == 0 ? at::zeros({p.B, p.T, p.C}, like.options()) : at::empty({p.B, p.T, p.C}, like.options());
+    Tensor gx = p.S == 0 ? at::zeros({p.B, p.T, p.C}, like.options()) : empty_on({p.B, p.T, p.C}, like.scalar_type(), like.device());
     kd_cocktail q = p;
     ti = ti.contiguous();
     th = th.contiguous();
@@ -770,7 +781,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     at::AutoDispatchBelowADInplaceOrView below;
     const Tensor tokens = tokens_.stride(1) == 1 ? tokens_ : tokens_.contiguous();
     const Tensor x = x_.stride(2) == 1 ? x_ : x_.contiguous();
-    index = at::empty({index_words(B, T)}, tokens.options().dtype(at::kInt));
+    index = empty_on({index_words(B, T)}, at::kInt, tokens.device());
     p.B = static_cast<int32_t>(B);
     p.T = static_cast<int32_t>(T);
     p.C = static_cast<int32_t>(C);
@@ -778,6 +789,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     point_into_index(p, index);
     auto out = [](const int32_t* words) { return const_cast<int32_t*>(words); };
     Tensor counts = at::empty({B}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    std::fill_n(counts.data_ptr<int32_t>(), B, -1);   // not there yet
     c10::cuda::CUDAGuard guard(x.device());
     auto stream = at::cuda::getCurrentCUDAStream();
     const int64_t n_tokens = tokens.size(1);
@@ -786,11 +798,20 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
                              counts.data_ptr<int32_t>(), stream));
     int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
     if (B > 0 && n_tokens > 0) {
-      C10_CUDA_CHECK(cudaStreamSynchronize(stream));
-      for (int64_t b = 0; b < B; ++b) S = std::max(S, counts.data_ptr<int32_t>()[b]);
+      // The counts arrive while the kernel still writes the markers. A wait for the stream would add the rest of the kernel, its end and
+      // the wake-up (16 x 4096 x 1024, forward and backward 72.2 -> 61 us); it follows only where they take long, or never come.
+      volatile int32_t* words = counts.data_ptr<int32_t>();
+      const auto give_up = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+      int64_t b = 0;
+      for (; b < B; ++b) {
+        while (words[b] < 0 && std::chrono::steady_clock::now() < give_up) {}
+        if (words[b] < 0) break;
+      }
+      if (b < B) C10_CUDA_CHECK(cudaStreamSynchronize(stream));
+      for (b = 0; b < B; ++b) S = std::max(S, static_cast<int32_t>(words[b]));
     }
-    scores = C == 0 ? at::zeros({B, S}, x.options()) : at::empty({B, S}, x.options());
-    if (track) h = at::empty({B, S + 1, C}, x.options().dtype(at::kFloat));
+    scores = C == 0 ? at::zeros({B, S}, x.options()) : empty_on({B, S}, x.scalar_type(), x.device());
+    if (track) h = empty_on({B, S + 1, C}, at::kFloat, x.device());
     p.x = x.data_ptr();
     p.x_sb = x.stride(0);
     p.x_st = x.stride(1);
@@ -807,7 +828,7 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     node->p.C = p.C;
     node->p.S = p.S;
     node->p.dtype = p.dtype;
-    node->like = at::empty({0}, x_.options());
+    node->like = empty_on({0}, x_.scalar_type(), x_.device());
     torch::autograd::set_history(scores, node);
     node->h = torch::autograd::SavedVariable(h, false);
     node->index = torch::autograd::SavedVariable(index, false);
