@@ -99,7 +99,7 @@ struct FusedCfg {
                        B_QEMPTY = B_QFULL + QS, B_DOFULL = B_QEMPTY + QS, B_DOEMPTY = B_DOFULL + OS, B_SFULL = B_DOEMPTY + OS,
                        B_SFREE = B_SFULL + NH, B_PFULL = B_SFREE + NH, B_PFREE = B_PFULL + NH, B_DPFULL = B_PFREE + NH,
                        B_DSFULL = B_DPFULL + 1, B_DSFREE = B_DSFULL + 1, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
-                       B_ACCFULL = B_DQEMPTY + 1, B_ACCFREE = B_ACCFULL + 1, B_ITEMFULL = B_ACCFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
+                       B_ACCFULL = B_DQEMPTY + 1, B_ACCFREE = B_ACCFULL + 2, B_ITEMFULL = B_ACCFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
                        B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;
   static constexpr int ITEM_READERS = (HD == 64) ? 15 : 14;   // warps that read item headers
   static constexpr int SMEM_ALLOC = SMEM_BAR + NBAR * 8 + 16;   // + TMEM base, abort flag
@@ -171,7 +171,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (i >= C::B_DOEMPTY && i < C::B_SFULL) count = 2;        // dP^T and dV have read the tile
     if (i == C::B_DSFULL || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
     if (i == C::B_DQEMPTY) count = 4;                          // one per dQ warp
-    if (i == C::B_ACCFULL) count = 2;                          // the head's last dV and dK
     if (i == C::B_ACCFREE || i == C::B_ACCFREE + 1) count = 4; // dV, dK have been read out of TMEM
     if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = C::ITEM_READERS;
     mbar_init(bar(i), count);
@@ -496,7 +495,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             commit_uniform(bar(C::B_DSFREE));
             commit_uniform(bar(C::B_QEMPTY + q_stage));
             if (last) {
-              commit_uniform(bar(C::B_ACCFULL));
+              commit_uniform(bar(C::B_ACCFULL + 1));
               commit_uniform(bar(C::B_KEMPTY + (item & 1)));
             }
             if (++q_stage == C::QS) q_stage = 0;
@@ -595,7 +594,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             commit_uniform(bar(C::B_QEMPTY + q_stage));
             if (++q_stage == C::QS) q_stage = 0;
             if (last) {
-              commit_uniform(bar(C::B_ACCFULL));
+              commit_uniform(bar(C::B_ACCFULL + 1));
               if (!v_asked) {
                 advance();
                 if (have) {
@@ -909,16 +908,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * f);
       stage_box(buf, r);
     };
-    // Writes dV, then dK (the next item's first dV product comes first) of the item: 32 rows of a warp as boxes of 64 columns
-    // through the staging buffers and TMA stores. m: number of the item; kt: its key tile.
-    auto write_out = [&](int b, int h, int kt, int m) -> bool {
-      if (!wait(C::B_ACCFULL, m & 1, W_U_ACCFULL)) return false;
+    // Writes dV or dK (is_k) of the item: 32 rows of a warp as boxes of 64 columns through the staging buffers and TMA stores. m: number of
+    // the item; kt: its key tile. dV goes before the item's last dQ tile, which is formed an iteration after the last dV product: the next
+    // item's first dV product waits for its columns, and with it P^T of the tile after. (dV behind that dQ tile, together with dK: the
+    // second tile of an item took 2,300 cycles more than others.)
+    auto write_out = [&](bool is_k, int b, int h, int kt, int m) -> bool {
+      if (!wait(C::B_ACCFULL + (is_k ? 1 : 0), m & 1, W_U_ACCFULL)) return false;
       tc_fence_after_sync();
       const int key0 = kt * KD_TILE + wq * 32;
 #pragma unroll 1
-      for (int part = 0; part < 2 * HD / 64; ++part) {
-        const bool is_k = part >= HD / 64;
-        const int col = (part % (HD / 64)) * 64;
+      for (int part = 0; part < HD / 64; ++part) {
+        const int col = part * 64;
         const uint32_t buf = kF32 ? stg : stg + (part & 1) * 4096;   // 64 columns of float32 are two boxes
         const float f = is_k ? a.sm_scale : 1.0f;
         if (kF32 || (part & 1) == 0) {
@@ -963,10 +963,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const int bh = b * a.H + h;
       const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
       uint32_t ent_next = static_cast<uint32_t>(it.z) >> 16;
-      for (int e = 0; e < n; ++e, ++t) {
+      auto dq_tile = [&](int e) -> bool {
         const int q0 = (ent_next & 0xFF) * KD_TILE + wq * 32;
         if (e + 1 < n) ent_next = list[e + 1];
-        if (!(ok = wait(C::B_DQFULL, t & 1, W_U_DQFULL))) break;
+        if (!wait(C::B_DQFULL, t & 1, W_U_DQFULL)) return false;
         tc_fence_after_sync();
         const uint32_t tDQ = lane_base + C::TM_DQ;
         auto drained = [&]() {   // the tile is in registers: the columns may be overwritten
@@ -1021,8 +1021,21 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           stage(1, r[1]);
           reduce(1);
         }
-        if (e == n - 1 && !(ok = write_out(b, h, kt, m++))) break;
+        ++t;
+        return true;
+      };
+      // the item's dQ tiles; dV before the last, dK behind it
+      if constexpr (HD == 64) {
+        for (int e = 0; ok && e < n; ++e) {
+          const bool last = e == n - 1;
+          ok = (!last || write_out(false, b, h, kt, m)) && dq_tile(e) && (!last || write_out(true, b, h, kt, m));
+        }
+      } else {   // (two copies of write_out are 60 bytes of spills at this width, and 2 % of the kernel; one copy is 0.6 % slower at the other)
+#pragma unroll 1
+        for (int step = 0; ok && step < n + 2; ++step)
+          ok = (step == n - 1 || step == n + 1) ? write_out(step == n + 1, b, h, kt, m) : dq_tile(min(step, n - 1));
       }
+      ++m;
     }
     if (lane == 0) bulk_wait_group0();
   }
