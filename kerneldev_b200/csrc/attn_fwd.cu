@@ -71,7 +71,8 @@ struct FwdCfg {
   static constexpr int SMEM_Q = 0;
   static constexpr int SMEM_K = SMEM_Q + NQ * TILE_BYTES;
   static constexpr int SMEM_V = SMEM_K + KST * TILE_BYTES;
-  static constexpr int SMEM_LIST = SMEM_V + VST * TILE_BYTES;      // NITEM x <= 128 list entries
+  static constexpr int SMEM_O = SMEM_V + VST * TILE_BYTES;         // O on its way out: per softmax warp a box [32 rows][32 columns], 64-byte swizzle
+  static constexpr int SMEM_LIST = SMEM_O + 16 * 2048;             // NITEM x <= 128 list entries
   static constexpr int SMEM_ITEM = SMEM_LIST + NITEM * 128 * 2;    // NITEM x {batch, head, pair, entries | units of tile 0 << 8 | of tile 1 << 16 | the item's only tile + 1 << 24}
   static constexpr int SMEM_XCH = SMEM_ITEM + NITEM * 16;          // NXB x [query tile][half][row] fp32
   static constexpr int SMEM_CLC = SMEM_XCH + NXB * 4 * KD_TILE * 4;
@@ -90,13 +91,14 @@ struct FwdCfg {
   // TMEM columns: NBUF score buffers of 128, then O0 and O1 (HD each)
   static constexpr uint32_t TM_O0 = NBUF * 128, TM_O1 = NBUF * 128 + HD;
   static_assert(TM_O1 + HD <= 512, "TMEM budget");
+  static_assert(SMEM_O % 512 == 0, "a 64-byte swizzle repeats every 512 bytes");
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
 template <bool kBf16>
 __global__ void __launch_bounds__(FwdCfg::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdArgs a) {
   using C = FwdCfg;
   constexpr int HD = C::HD, TILE = C::TILE_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -579,13 +581,37 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           if (lane == 0) mbar_arrive(bar(C::B_OFREE + i));
         }
         const int col = half * (HD / 2) + cb * 32;
-        if (qi < a.T && (kBf16 || a.o != nullptr)) store_row32_upto<kBf16>(orow + col, r, inv_l, col, a.d_real);
+        if (a.o_tma != 0) {
+          const int row0 = __reduce_min_sync(0xffffffffu, qi);   // INT_MAX: written by the other item of the pair
+          if (row0 < a.T && col < a.d_real) {   // (both are the warp's)
+            const uint32_t box = s0 + C::SMEM_O + (warp - 4) * 2048;
+            if (lane == 0) bulk_wait_group_read0();   // the last item's rows have been read
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint32_t at = box + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4);
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at),
+                           "r"(pack2<kBf16>(__uint_as_float(r[8 * j + 0]) * inv_l, __uint_as_float(r[8 * j + 1]) * inv_l)),
+                           "r"(pack2<kBf16>(__uint_as_float(r[8 * j + 2]) * inv_l, __uint_as_float(r[8 * j + 3]) * inv_l)),
+                           "r"(pack2<kBf16>(__uint_as_float(r[8 * j + 4]) * inv_l, __uint_as_float(r[8 * j + 5]) * inv_l)),
+                           "r"(pack2<kBf16>(__uint_as_float(r[8 * j + 6]) * inv_l, __uint_as_float(r[8 * j + 7]) * inv_l))
+                           : "memory");
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {   // rows at or beyond T and columns at or beyond d_real are not written
+              tma_store_4d(&tmO, box, col, row0, h, b);
+              bulk_commit_group();
+            }
+          }
+        } else if (qi < a.T && (kBf16 || a.o != nullptr)) store_row32_upto<kBf16>(orow + col, r, inv_l, col, a.d_real);
         if (!kBf16 && qi < a.T && a.o32 != nullptr)
           store_row32_f32_upto(a.o32 + (size_t)b * a.o32_sb + (size_t)h * a.o32_sh + (size_t)qi * a.o32_st + col, r, inv_l, col, a.d_real);
       }
     }
     }  // items
     if (abortf->v != 0u) named_bar_arrive(pair_bar, 64);
+    if (lane == 0) bulk_wait_group0();
   }
 
   tc_fence_before_sync();
@@ -595,12 +621,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 template <bool kBf16>
-static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, cudaStream_t stream) {
+static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmO,
+                        cudaStream_t stream) {
   auto kern = attn_fwd_kernel<kBf16>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, FwdCfg::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
-  e = launch(kern, static_cast<unsigned>(n_items), FwdCfg::THREADS, FwdCfg::SMEM_ALLOC, stream, tmQ, tmK, tmV, a);
+  e = launch(kern, static_cast<unsigned>(n_items), FwdCfg::THREADS, FwdCfg::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmO, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_fwd_kernel launch: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -636,7 +663,13 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
 #endif
   // head dims below the tile width run on the next wider kernel: TMA zero-fills the missing columns
   if (p.D > 64) return launch_attn_fwd_wide(n_items, a, p.dtype, tmQ, tmK, tmV, stream);
-  return p.dtype == KD_BF16 ? launch_fwd_t<true>(n_items, a, tmQ, tmK, tmV, stream) : launch_fwd_t<false>(n_items, a, tmQ, tmK, tmV, stream);
+  // O through TMA stores: a thread's 16-byte stores to its own row are 32 lines an instruction, 1,240 cycles of an item's end with sixteen
+  // warps at it (short bursts: hierarchical 16 x 16 x 4096 x 64 416 -> 406 us, 8 x 16 x 2048 x 64 66.3 -> 64.5; causal 113.9 -> 111.1; no mask
+  // 187.6 -> 182.3). Not where a CTA has one item: its rows leave as soon either way, and the map costs the host time. (Nor for strides
+  // that a map cannot have: 0 or below.)
+  CUtensorMap tmO = tmQ;
+  a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, "o", 64) == 0 ? 1 : 0;
+  return p.dtype == KD_BF16 ? launch_fwd_t<true>(n_items, a, tmQ, tmK, tmV, tmO, stream) : launch_fwd_t<false>(n_items, a, tmQ, tmK, tmV, tmO, stream);
 }
 
 }  // namespace kd

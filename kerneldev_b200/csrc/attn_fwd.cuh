@@ -22,6 +22,7 @@ struct FwdArgs {
   int64_t o_sb, o_sh, o_st;
   float* o32;        // null, or O of a float32 call
   int64_t o32_sb, o32_sh, o32_st;
+  int o_tma;         // head dims up to 64: O leaves through shared memory and TMA stores
   float* lse;
 #ifdef KD_TEST_DROP_LOAD
   int test_drop_load;   // wait time-out test build: the producer of CTA 0 leaves out its first K tile load

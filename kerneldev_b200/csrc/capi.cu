@@ -47,9 +47,9 @@ static CUresult with_context(F encode) {
   return r;
 }
 
-// a box is 128 bytes wide, whatever D is
+// a box is 128 bytes wide, whatever D is (or 64), and swizzled over that width
 static int encode_4d(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, CUtensorMapDataType type, int es,
-                     int box_rows, const char* name) {
+                     int box_rows, const char* name, int box_bytes = 128) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return set_error(KD_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
   if (t.ptr == nullptr) return set_error(KD_ERR_ARG, "tensor %s is null", name);
@@ -65,16 +65,17 @@ static int encode_4d(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, 
   cuuint64_t strides[3] = {(cuuint64_t)st, (cuuint64_t)(H > 1 ? sh : st * T), (cuuint64_t)(B > 1 ? sb : (H > 1 ? sh * H : st * T))};
   for (int i = 0; i < 3; ++i)
     if (strides[i] & 15) strides[i] = (strides[i] + 15) & ~cuuint64_t(15);
-  cuuint32_t box[4] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows, 1, 1};
+  cuuint32_t box[4] = {(cuuint32_t)(box_bytes / es), (cuuint32_t)box_rows, 1, 1};
   cuuint32_t step[4] = {1, 1, 1, 1};
-  const CUresult r = with_context([&] { return enc(out, type, 4, t.ptr, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+  const CUresult r = with_context([&] { return enc(out, type, 4, t.ptr, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
   if (r != CUDA_SUCCESS) return set_error(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
   return 0;
 }
 
-int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype, int box_rows, const char* name) {
-  return encode_4d(out, t, B, H, T, D, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, box_rows, name);
+int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype, int box_rows, const char* name, int box_bytes) {
+  return encode_4d(out, t, B, H, T, D, dtype == KD_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, box_rows, name, box_bytes);
 }
 
 int encode_tensor_map_f32(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int box_rows, const char* name) {

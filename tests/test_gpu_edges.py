@@ -258,3 +258,19 @@ def test_deterministic_backward_takes_further_items(B, H, T, D):
     _, _, *ref = ao.attention_fwd_bwd(*(x[:, heads].cpu() for x in (q, k, v, do)), mask)
     for name, got, want in zip(("dQ", "dK", "dV"), one, ref):
         assert_close(name, got[:, heads], want)
+
+
+# more items than SMs: O leaves through boxes of 32 rows and 32 columns (head dims that end inside the first or the second box, last rows
+# of a tile of 1, 31, 32 and 97); 148 items and fewer: by the threads themselves
+@pytest.mark.parametrize("layout", ["bhtd", "bthd"])
+@pytest.mark.parametrize("B,H,T,D", [(15, 10, 129, 16), (15, 10, 159, 48), (19, 8, 160, 32), (38, 4, 225, 64), (37, 4, 225, 64)])
+def test_forward_output_boxes(B, H, T, D, layout):
+    from tests.helpers import assert_close, rand_inputs
+    from kerneldev_b200 import flash_attention
+    q, k, v, _ = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.float16, seed=D + T))
+    if layout == "bthd":
+        q, k, v = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in (q, k, v))
+    lens = torch.tensor([(T, T // 3, 0)[b % 3] for b in range(B)], dtype=torch.int32, device=DEV)
+    o = flash_attention(q, k, v, lens=lens, causal=True, out_layout="input" if layout == "bthd" else "contiguous")
+    mask = ao.dense_mask(T, None, None, None, lens.cpu().numpy(), causal=True, B=B)
+    assert_close("O", o, ao.attention_forward(q.float().cpu(), k.float().cpu(), v.float().cpu(), mask)[0])
