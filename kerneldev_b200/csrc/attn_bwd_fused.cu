@@ -84,10 +84,11 @@ struct FusedCfg {
   static constexpr int SMEM_DO = SMEM_Q + QS * TILE_BYTES;
   static constexpr int SMEM_DS = SMEM_DO + OS * TILE_BYTES;   // dS^T: two blocks [128 keys][64 queries]
   static constexpr int SMEM_STG = SMEM_DS + 2 * 16384;        // dQ staging: per dQ warp two boxes [32 rows][32 floats]
-  // per Q stage: LSE and delta of the 128 queries, the 32 mask words of the query tile and its list entry (4 words with
+  // per Q stage: LSE and delta of the 128 queries, the 32 mask words of the query tile, its list entry (4 words with
   // padding); HD = 64 also the queries' token descriptors (HD = 128 has no room: its compute warps fetch them)
   static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + 32, SIDE_DESC = SIDE_ENT + 4;
-  static constexpr int SIDE_WORDS = (HD == 64) ? SIDE_DESC + KD_TILE : SIDE_DESC;
+  static constexpr int SIDE_KDESC = SIDE_DESC + KD_TILE;   // and the keys'
+  static constexpr int SIDE_WORDS = (HD == 64) ? SIDE_KDESC + KD_TILE : SIDE_DESC;
   static constexpr int SMEM_SIDE = SMEM_STG + 4 * 2 * 4096;
   static constexpr int NITEM = 4;                    // ring of item headers
   static constexpr int SMEM_ITEM = SMEM_SIDE + QS * SIDE_WORDS * 4;   // NITEM x {batch, head, key tile | first entry << 16, entries}
@@ -101,7 +102,8 @@ struct FusedCfg {
                        B_DSFULL = B_DPFULL + 1, B_DSFREE = B_DSFULL + 1, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
                        B_ACCFULL = B_DQEMPTY + 1, B_ACCFREE = B_ACCFULL + 2, B_ITEMFULL = B_ACCFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
                        B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;
-  static constexpr int ITEM_READERS = (HD == 64) ? 15 : 14;   // warps that read item headers
+  static constexpr int ITEM_READERS = (HD == 64) ? 7 : 14;    // warps that read item headers
+  static constexpr uint32_t ENT_END = 0xFFFFFFFFu;            // HD = 64: in place of a list entry, behind the last tile
   static constexpr int SMEM_ALLOC = SMEM_BAR + NBAR * 8 + 16;   // + TMEM base, abort flag
   static constexpr int THREADS = 512;
   // TMEM columns
@@ -289,6 +291,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (n != 0) {   // (no other warp hears of an item without entries)
         const int slot = k % C::NITEM;
         if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_U_ITEMEMPTY))) break;
+        if (HD == 64 && n < 0) {   // the compute warps read no headers: the stage behind the last tile tells them
+          if (!(ok = wait(C::B_QEMPTY + qs, q_parity, W_U_QEMPTY))) break;
+          if (lane == 0) {
+            st_shared_u32(s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4) + C::SIDE_ENT * 4, C::ENT_END);
+            if (k == 0) {   // no tile at all, and so no product that would wake them
+              mbar_arrive(bar(C::B_SFULL));
+              mbar_arrive(bar(C::B_SFULL + 1));
+            }
+          }
+          __syncwarp();
+        }
         if (lane == 0) {
           items[slot] = it;
           mbar_arrive(bar(C::B_ITEMFULL + slot));
@@ -328,7 +341,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (!(ok = wait(C::B_QEMPTY + qs, q_parity, W_U_QEMPTY))) break;
           const uint32_t side = s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4);
           if (lane == 0) {
-            st_shared_u32(side + C::SIDE_ENT * 4, this_ent);   // published by the arrival that goes with the load
+            st_shared_u32(side + C::SIDE_ENT * 4, this_ent | (HD == 64 ? static_cast<uint32_t>(kt) << 16 : 0u));   // published by the arrival that goes with the load
             load_tile(&tmQ, sQ + qs * TILE, C::B_QFULL + qs, qt, h, b);
           }
           // the scalars of four queries and one mask word per lane, copied asynchronously: the barrier counts the lanes' copies
@@ -347,7 +360,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
           }
           cp_async4(side + (C::SIDE_BITS + lane) * 4, a.tilebits + ((size_t)b * a.NT + qt) * 32 + lane);
-          if constexpr (HD == 64) cp_async16(side + C::SIDE_DESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + q);   // padded to whole tiles
+          if constexpr (HD == 64) {   // padded to whole tiles
+            cp_async16(side + C::SIDE_DESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + q);
+            cp_async16(side + C::SIDE_KDESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + kt * KD_TILE + 4 * lane);
+          }
           cp_async_mbar_arrive(bar(C::B_QFULL + qs));
           ++q_tiles;
           if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
@@ -690,104 +706,103 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
       for (int j = 0; j < 32; ++j) { p[0][j] = 0u; p[1][j] = 0u; }
       const float* side_prev = sSide;
-      bool s_ready = false;
+      bool s_ready = true;
       // One body for all iterations: the first one's dS^T and the last one's P^T are computed from whatever is there and
-      // read by nobody.
-      for (int k = 0;;) {
-        const bool more = next_item(k++, it);
-        if (!more && t == 0) break;
-        const int b = it.x, kt = it.z & 0xFFFF, n = more ? it.w : 1;
-        const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
-        const uint32_t kdesc = more ? __ldcg(a.desc + (size_t)b * a.Tpad + kj) : 0u;
+      // read by nobody. What the warps need to know of a tile's item lies beside its scalars: a header read at the start of
+      // every item is code that the instruction cache has lost by then, and cost 900 cycles of it. (Read where PARTIAL tiles are masked;
+      // read ahead of the arithmetic the entry makes every tile 4 % longer.)
+      ok = wait(C::B_SFULL + w, 0, W_U_SFULL);
+      bool more = ok && reinterpret_cast<const uint32_t*>(sSide)[C::SIDE_ENT] != C::ENT_END;
 #pragma unroll 1
-        for (int e = 0; e < n; ++e, ++t) {
-          if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
-          tc_fence_after_sync();
-          const float* side = sSide + qs * C::SIDE_WORDS;
-          bool out_ready = false;
-          uint32_t pk_ds[2][16];
-          // 16 keys x 16 queries at a time, both halves of the keys for a group of queries. The next block is loaded while one is
-          // worked on: with two warps to a scheduler a TMEM load of some 150 cycles that is waited for at once is not covered. (Four
-          // blocks of 32 queries, each loaded and awaited: causal 8 x 16 x 1000 x 64 84.0 -> 80.7 us, 8 x 16 x 2048 241 -> 230.)
-          uint64_t lse[2], delta[2];
-          uint32_t sb[2][8], dpb[2][8];
-          auto load_block = [&](int c) {
-            tmem_ld16x256_x2(tS + (c & 1) * ROW16 + (c >> 1) * 16, sb[c & 1]);
-            tmem_ld16x256_x2(tDP + (c & 1) * ROW16 + (c >> 1) * 16, dpb[c & 1]);
-          };
-          auto load_scalars = [&](int g) {
+      for (; more; ++t) {
+        if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
+        tc_fence_after_sync();
+        const float* side = sSide + qs * C::SIDE_WORDS;
+        bool out_ready = false;
+        uint32_t pk_ds[2][16];
+        // 16 keys x 16 queries at a time, both halves of the keys for a group of queries. The next block is loaded while one is
+        // worked on: with two warps to a scheduler a TMEM load of some 150 cycles that is waited for at once is not covered. (Four
+        // blocks of 32 queries, each loaded and awaited: causal 8 x 16 x 1000 x 64 84.0 -> 80.7 us, 8 x 16 x 2048 241 -> 230.)
+        uint64_t lse[2], delta[2];
+        uint32_t sb[2][8], dpb[2][8];
+        auto load_block = [&](int c) {
+          tmem_ld16x256_x2(tS + (c & 1) * ROW16 + (c >> 1) * 16, sb[c & 1]);
+          tmem_ld16x256_x2(tDP + (c & 1) * ROW16 + (c >> 1) * 16, dpb[c & 1]);
+        };
+        auto load_scalars = [&](int g) {
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              lse[j] = ld_shared_pair(side + qcol + 16 * g + 8 * j);
-              delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 16 * g + 8 * j);
+          for (int j = 0; j < 2; ++j) {
+            lse[j] = ld_shared_pair(side + qcol + 16 * g + 8 * j);
+            delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 16 * g + 8 * j);
+          }
+        };
+        load_block(0);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int hf = c & 1, g = c >> 1;
+          if (hf == 0) load_scalars(g);
+          tmem_wait_ld();
+          if (c < 7) load_block(c + 1);
+          if (c == 7) {   // all loaded
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(C::B_SFREE + w));
+            // The barriers of the stores below, and of the next iteration further down, are tested ahead: a test takes some 150
+            // cycles under this load, and as a rule it finds the phase complete.
+            out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1) && mbar_test_wait(bar(C::B_DSFREE), t & 1);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              uint32_t& p0 = p[hf][8 * g + 4 * j + 2 * r];
+              uint32_t& p1 = p[hf][8 * g + 4 * j + 2 * r + 1];
+              const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dpb[hf][4 * j + 2 * r], dpb[hf][4 * j + 2 * r + 1]));
+              const uint64_t x = mul_f32x2(pack_u32x2(p0, p1), d);
+              pk_ds[hf][4 * g + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+              const uint64_t y = fma_f32x2(pack_u32x2(sb[hf][4 * j + 2 * r], sb[hf][4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
+              p0 = __float_as_uint(fast_exp2(-lo_f32x2(y)));
+              p1 = __float_as_uint(fast_exp2(-hi_f32x2(y)));
             }
-          };
-          load_block(0);
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const int hf = c & 1, g = c >> 1;
-            if (hf == 0) load_scalars(g);
-            tmem_wait_ld();
-            if (c < 7) load_block(c + 1);
-            if (c == 7) {   // all loaded
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(bar(C::B_SFREE + w));
-              // The barriers of the stores below, and of the next iteration further down, are tested ahead: a test takes some 150
-              // cycles under this load, and as a rule it finds the phase complete.
-              out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1) && mbar_test_wait(bar(C::B_DSFREE), t & 1);
-            }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-#pragma unroll
-              for (int r = 0; r < 2; ++r) {
-                uint32_t& p0 = p[hf][8 * g + 4 * j + 2 * r];
-                uint32_t& p1 = p[hf][8 * g + 4 * j + 2 * r + 1];
-                const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dpb[hf][4 * j + 2 * r], dpb[hf][4 * j + 2 * r + 1]));
-                const uint64_t x = mul_f32x2(pack_u32x2(p0, p1), d);
-                pk_ds[hf][4 * g + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
-                const uint64_t y = fma_f32x2(pack_u32x2(sb[hf][4 * j + 2 * r], sb[hf][4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
-                p0 = __float_as_uint(fast_exp2(-lo_f32x2(y)));
-                p1 = __float_as_uint(fast_exp2(-hi_f32x2(y)));
-              }
-            }
           }
-          const uint32_t* side_u = reinterpret_cast<const uint32_t*>(side);
-          const uint32_t ent = side_u[C::SIDE_ENT];
-          if (more && (ent >> 8) == KD_TILE_PARTIAL) {
-            uint32_t mk[2];
-            mask_words(side, kdesc, kj, (ent & 0xFF) * KD_TILE + w * 64, side_u[C::SIDE_DESC + w * 64 + lane], side_u[C::SIDE_DESC + w * 64 + 32 + lane], mk);
-            apply_mask(p[0], mk, 0);
-            apply_mask(p[1], mk, 1);
-          }
-          // (in the last iteration too: it must not complete a phase of PFULL ahead of the dV issuer)
-          if (!__all_sync(0xffffffffu, out_ready)) {
-            if (t > 0 && !(ok = wait(C::B_PFREE + w, (t - 1) & 1, W_U_PFREE))) break;
-            if (t > 1 && !(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
-          }
-          tc_fence_after_sync();
-          s_ready = mbar_test_wait(bar(C::B_SFULL + w), (t + 1) & 1);
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t pk[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(p[hf][2 * j]), __uint_as_float(p[hf][2 * j + 1]));
-            tmem_st16x128_x8(tP + hf * ROW16, pk);
-          }
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-            for (int j = 0; j < 8; j += 2)
-              stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(j) << 4) ^ ds_sw), pk_ds[hf][2 * j], pk_ds[hf][2 * j + 1], pk_ds[hf][2 * j + 2], pk_ds[hf][2 * j + 3]);
-          fence_proxy_async_smem();   // the dK and dQ products read dS^T through the async proxy
-          tmem_wait_st();
-          tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(C::B_PFULL + w));
-          side_prev = side;
-          if (++qs == C::QS) qs = 0;
         }
-        if (!ok || !more) break;
+        const uint32_t* side_u = reinterpret_cast<const uint32_t*>(side);
+        const uint32_t ent = side_u[C::SIDE_ENT];
+        more = ent != C::ENT_END;
+        if (more && ((ent >> 8) & 0xFFu) == KD_TILE_PARTIAL) {
+          const uint32_t kdesc = side_u[C::SIDE_KDESC + wq * 32 + lane];   // of the key whose mask words this lane forms
+          const int kj = static_cast<int>(ent >> 16) * KD_TILE + wq * 32 + lane;
+          uint32_t mk[2];
+          mask_words(side, kdesc, kj, (ent & 0xFF) * KD_TILE + w * 64, side_u[C::SIDE_DESC + w * 64 + lane], side_u[C::SIDE_DESC + w * 64 + 32 + lane], mk);
+          apply_mask(p[0], mk, 0);
+          apply_mask(p[1], mk, 1);
+        }
+        // (in the last iteration too: it must not complete a phase of PFULL ahead of the dV issuer)
+        if (!__all_sync(0xffffffffu, out_ready)) {
+          if (t > 0 && !(ok = wait(C::B_PFREE + w, (t - 1) & 1, W_U_PFREE))) break;
+          if (t > 1 && !(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
+        }
+        tc_fence_after_sync();
+        s_ready = mbar_test_wait(bar(C::B_SFULL + w), (t + 1) & 1);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(p[hf][2 * j]), __uint_as_float(p[hf][2 * j + 1]));
+          tmem_st16x128_x8(tP + hf * ROW16, pk);
+        }
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+          for (int j = 0; j < 8; j += 2)
+            stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(j) << 4) ^ ds_sw), pk_ds[hf][2 * j], pk_ds[hf][2 * j + 1], pk_ds[hf][2 * j + 2], pk_ds[hf][2 * j + 3]);
+        fence_proxy_async_smem();   // the dK and dQ products read dS^T through the async proxy
+        tmem_wait_st();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(C::B_PFULL + w));
+        side_prev = side;
+        if (++qs == C::QS) qs = 0;
       }
     } else {
     for (int k = 0; ok && next_item(k, it); ++k) {
