@@ -95,7 +95,9 @@ struct FwdCfg {
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
-template <bool kBf16>
+// kF32: of a float32 call: O goes to a float32 tensor, and to a 16-bit one where there will be a backward. (As a branch of the float16 kernels the
+// second store cost short lists above head dim 64 4 %.)
+template <bool kBf16, bool kF32>
 __global__ void __launch_bounds__(FwdCfg::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdArgs a) {
@@ -604,8 +606,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
               bulk_commit_group();
             }
           }
-        } else if (qi < a.T && (kBf16 || a.o != nullptr)) store_row32_upto<kBf16>(orow + col, r, inv_l, col, a.d_real);
-        if (!kBf16 && qi < a.T && a.o32 != nullptr)
+        } else if (qi < a.T && (!kF32 || a.o != nullptr)) store_row32_upto<kBf16>(orow + col, r, inv_l, col, a.d_real);
+        if (kF32 && qi < a.T)
           store_row32_f32_upto(a.o32 + (size_t)b * a.o32_sb + (size_t)h * a.o32_sh + (size_t)qi * a.o32_st + col, r, inv_l, col, a.d_real);
       }
     }
@@ -620,10 +622,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (tid == 0) report_abort(abortf, a.status);
 }
 
-template <bool kBf16>
+template <bool kBf16, bool kF32>
 static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmO,
                         cudaStream_t stream) {
-  auto kern = attn_fwd_kernel<kBf16>;
+  auto kern = attn_fwd_kernel<kBf16, kF32>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, FwdCfg::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
@@ -669,7 +671,8 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   // that a map cannot have: 0 or below.)
   CUtensorMap tmO = tmQ;
   a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, "o", 64) == 0 ? 1 : 0;
-  return p.dtype == KD_BF16 ? launch_fwd_t<true>(n_items, a, tmQ, tmK, tmV, tmO, stream) : launch_fwd_t<false>(n_items, a, tmQ, tmK, tmV, tmO, stream);
+  auto run = [&](auto launch_fn) { return launch_fn(n_items, a, tmQ, tmK, tmV, tmO, stream); };
+  return f32 ? run(launch_fwd_t<false, true>) : p.dtype == KD_BF16 ? run(launch_fwd_t<true, false>) : run(launch_fwd_t<false, false>);
 }
 
 }  // namespace kd

@@ -59,7 +59,8 @@ struct FwdWideCfg {
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
-template <bool kBf16>
+// kF32: of a float32 call (see attn_fwd.cu)
+template <bool kBf16, bool kF32>
 __global__ void __launch_bounds__(FwdWideCfg::THREADS, 1)
 attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
@@ -439,8 +440,8 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)qi * a.o_st;
 #pragma unroll
         for (int cb = 0; cb < HD / 32; ++cb) {
-          if (kBf16 || a.o != nullptr) store_row32_upto<kBf16>(orow + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
-          if (!kBf16 && a.o32 != nullptr)
+          if (!kF32 || a.o != nullptr) store_row32_upto<kBf16>(orow + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
+          if (kF32)
             store_row32_f32_upto(a.o32 + (size_t)b * a.o32_sb + (size_t)h * a.o32_sh + (size_t)qi * a.o32_st + cb * 32, r[cb], inv_l, cb * 32, a.d_real);
         }
         if (a.lse != nullptr) a.lse[((size_t)b * a.H + h) * a.T + qi] = (l > 0.f) ? (m * c + log2f(l)) : -INFINITY;
@@ -454,10 +455,10 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (tid == 0) report_abort(abortf, a.status);
 }
 
-template <bool kBf16>
+template <bool kBf16, bool kF32>
 static int launch_wide_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, cudaStream_t stream) {
   using C = FwdWideCfg;
-  auto kern = attn_fwd_wide_kernel<kBf16>;
+  auto kern = attn_fwd_wide_kernel<kBf16, kF32>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
@@ -479,7 +480,8 @@ static int launch_wide_t(long long n_items, const FwdArgs& a, const CUtensorMap&
 
 int launch_attn_fwd_wide(long long n_items, const FwdArgs& a, int dtype, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                          cudaStream_t stream) {
-  return dtype == KD_BF16 ? launch_wide_t<true>(n_items, a, tmQ, tmK, tmV, stream) : launch_wide_t<false>(n_items, a, tmQ, tmK, tmV, stream);
+  auto run = [&](auto launch_fn) { return launch_fn(n_items, a, tmQ, tmK, tmV, stream); };
+  return a.o32 != nullptr ? run(launch_wide_t<false, true>) : dtype == KD_BF16 ? run(launch_wide_t<true, false>) : run(launch_wide_t<false, false>);
 }
 
 }  // namespace kd
