@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
 #pragma unroll
     for (int d = TPR / 2; d >= 1; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
     if (live && sub == 0) a.delta[r] = acc;
-    if (live && a.dq_acc != nullptr) {
+    if (live && a.dq_acc != nullptr && sub * 8 < a.d_real) {   // the columns beyond are never read (zeroed too: causal 8 x 16 x 2048 x 80 370 us, 365 without)
       float4* z = reinterpret_cast<float4*>(a.dq_acc + r * HD + sub * 8);
       z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
       z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
