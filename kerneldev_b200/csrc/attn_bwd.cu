@@ -491,7 +491,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       return true;
     };
     if (wait_ahead) pdl_wait();
-    if (warp == 4) pdl_launch_dependents();
+    if (warp == 4) {
+      __threadfence();   // for the dK/dV kernel, which does not wait for the delta kernel itself
+      pdl_launch_dependents();
+    }
     int n_acc = 0;   // items with units so far
     // this stream's next unit, counted over all items, as (unit / NBUF, unit % NBUF)
     int buf = i % C::NBUF;
@@ -648,7 +651,13 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __shared__ BwdShared<C> sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) bwd_init<C>(sh);
+  if (tid == 0) {
+    bwd_init<C>(sh);
+    if (a.after_dq != 0) {   // see below
+      __threadfence();
+      fence_proxy_async_global();
+    }
+  }
   if (warp == 1) {
     tmem_alloc(smem_u32(&sh.tmem_base), 512);
     tmem_relinquish();
@@ -656,18 +665,22 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // Directly behind the dQ kernel of the same call there is nothing to wait for: that kernel lets this one start when it has itself waited
-  // for the delta kernel, and the last CTAs of the one overlap the first of the other (1 x 16 x 500 x 128 30 -> 22.5 us together). The
-  // dQ kernel's end is awaited at the end, so that whatever comes next finds both complete (what a successor reads ahead of its own wait
-  // is a plan, which no backward writes). Everything that this kernel reads is read past L1.
-  const bool wait_ahead = a.after_dq == 0 && a.plan_ready != 0;
-  if (a.after_dq == 0 && !wait_ahead) pdl_wait();
+  // Directly behind the dQ kernel of the same call there is nothing to wait for: that kernel writes nothing that this one reads, and lets it
+  // start when it has itself waited for the delta kernel. So the last CTAs of the one overlap the first of the other (both together, with
+  // the wait here instead: 1 x 16 x 500 x 128 31.5 us, 23 so; 4 x 16 x 2048 x 64 110.2, 108.2; unmasked 1 x 4 x 2048 x 64 51.5, 34).
+  // What orders delta, and the dO of a float32 call, before the reads here: CUDA promises visibility to the kernel that executes
+  // griddepcontrol.wait behind the writer, which is the dQ kernel, and none through launch_dependents alone. Hence a device-wide
+  // fence on both sides of that hand-over (there behind the wait, here ahead of the block's barrier, with one for the TMA loads); all reads
+  // go past L1. That a dependent kernel starts after launch_dependents has been executed is what remains to be relied on.
+  // The dQ kernel's end is awaited at this one's end, so that whatever comes next finds both complete (what a successor reads ahead of its
+  // own wait is a plan, which no backward writes).
+  if (a.after_dq == 0) pdl_wait();
   const uint32_t tbase = sh.tmem_base;
 
   if (warp < 4) {
     reg_dealloc<KD_REGS_ISSUE>();
     if (warp == 0) {
-      bwd_producer<HD, false>(tmK, tmV, tmQ, tmDO, a, sFix, sRing, lists, sh, lane, wait_ahead);
+      bwd_producer<HD, false>(tmK, tmV, tmQ, tmDO, a, sFix, sRing, lists, sh, lane, false);
     } else if ((warp == 3 || warp == 2) && lane == 0) {
       // ------------------------------ M1 issuers: warp 3: S^T_u = K Q_u^T; warp 2: dP^T_u = V dO_u^T ------------------------------
       const bool dp_part = (warp == 2);
@@ -835,7 +848,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       return true;
     };
-    if (wait_ahead) pdl_wait();
     if (warp == 4) pdl_launch_dependents();
     int n_acc = 0;   // items with units so far
     // this stream's next unit, counted over all items, as (unit / NBUF, unit % NBUF)

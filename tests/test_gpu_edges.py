@@ -274,3 +274,27 @@ def test_forward_output_boxes(B, H, T, D, layout):
     o = flash_attention(q, k, v, lens=lens, causal=True, out_layout="input" if layout == "bthd" else "contiguous")
     mask = ao.dense_mask(T, None, None, None, lens.cpu().numpy(), causal=True, B=B)
     assert_close("O", o, ao.attention_forward(q.float().cpu(), k.float().cpu(), v.float().cpu(), mask)[0])
+
+
+@pytest.mark.parametrize("B,H,T,D,dtype", [(1, 4, 300, 64, torch.bfloat16), (1, 8, 173, 128, torch.float16), (1, 3, 513, 64, torch.float32), (2, 2, 257, 128, torch.float32)])
+def test_deterministic_backward_behind_one_another(B, H, T, D, dtype):
+    """The dK/dV kernel starts beside the end of the dQ kernel and reads what the delta kernel of the same call has written. Calls without
+    a pause between them, whose scratch is the memory of earlier calls with other gradients, give the bits of calls one by one."""
+    from tests.helpers import assert_close, rand_inputs
+    from kerneldev_b200 import flash_attention
+    q, k, v, _ = (x.to(DEV).requires_grad_() for x in rand_inputs(B, H, T, D, dtype, seed=T + D))
+    g = torch.Generator(device=DEV).manual_seed(D)
+    dos = [(torch.randn((B, H, T, D), generator=g, device=DEV) * 2.0 ** (i % 5 - 2)).to(dtype) for i in range(24)]
+    o = flash_attention(q, k, v, deterministic=True)
+    torch.cuda.synchronize()
+    together = [torch.autograd.grad(o, (q, k, v), do, retain_graph=True) for do in dos]
+    torch.cuda.synchronize()
+    for i, do in enumerate(dos):
+        alone = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
+        torch.cuda.synchronize()
+        assert all(torch.equal(x, y) for x, y in zip(together[i], alone)), i
+    mask = ao.dense_mask(T, None, None, None, None, causal=True, B=B)
+    for i in (1, 13, 23):
+        _, _, *ref = ao.attention_fwd_bwd(*(x.detach().float().cpu() for x in (q, k, v, dos[i])), mask)
+        for name, got, want in zip(("dQ", "dK", "dV"), together[i], ref):
+            assert_close(name, got, want)   # P and dS are rounded to 16 bits: the repository's tolerance for that
