@@ -426,13 +426,12 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
   kd_attn_f32 f{};
   Tensor d_o;
-  if (!f32 || d_o_.scalar_type() != at::kFloat) {
-    d_o = usable(d_o_);
-  } else if (Tensor copy = empty_like_of(d_o_, at::kHalf); aligned(d_o_) && tma_ready(copy)) {
-    d_o = copy;   // filled by the delta kernel
-    f.d_o = desc(d_o_);
+  const bool rounds = f32 && d_o_.scalar_type() == at::kFloat && aligned(d_o_);
+  if (rounds) d_o = empty_like_of(d_o_, at::kHalf);
+  if (rounds && tma_ready(d_o)) {
+    f.d_o = desc(d_o_);   // the delta kernel fills d_o
   } else {
-    d_o = usable(d_o_.to(at::kHalf));
+    d_o = usable(f32 ? d_o_.to(at::kHalf) : d_o_);   // (the engine brings float32; a node that is called by hand may get another type)
   }
   if (!dq.defined()) {
     const auto type = f32 ? at::kFloat : q.scalar_type();

@@ -199,6 +199,19 @@ def test_undefined_gradients_count_as_zeros(dtype):
         assert g.shape == t.shape and g.dtype == dtype and not g.any()
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
+def test_node_of_a_float32_call_by_hand(dtype):
+    """The engine brings a gradient in the output's type, a caller of the node may not: it is converted, never read as what it is not."""
+    from kerneldev_b200 import flash_attention
+    g = torch.Generator(device=DEV).manual_seed(4)
+    q, k, v, do = (torch.randn((1, 2, 150, 64), generator=g, device=DEV) for _ in range(4))
+    do = do.bfloat16().float()   # converting it to any of the types and then to float16 rounds once
+    o = flash_attention(q.requires_grad_(), k.requires_grad_(), v.requires_grad_(), deterministic=True)
+    want = o.grad_fn(do)
+    for x, y in zip(o.grad_fn(do.to(dtype)), want):
+        assert x.dtype == torch.float32 and torch.equal(x, y)
+
+
 def test_other_threads_run_while_the_host_waits(monkeypatch):
     """KD_CHECK_STATUS=1 waits for the device in every call: here behind a busy stream."""
     import threading
