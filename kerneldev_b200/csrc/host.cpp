@@ -33,14 +33,23 @@ using OptTensor = std::optional<Tensor>;
 
 namespace {
 
-// Uninitialised device tensors from torch's CUDA allocator without the trip through the dispatcher, which is most of what at::empty
-// costs: a forward allocates two and a backward five (0.4 us each: a forward's host time without its launch 5.0 -> 4.3 us).
+// Whether at::empty would do more than allocate: a dispatch mode or a function transform of the caller's sees this thread's operators, or
+// torch fills new memory (deterministic algorithms).
+bool allocations_are_seen() {
+  const auto& context = at::globalContext();
+  return !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty() ||
+         (context.deterministicAlgorithms() && context.deterministicFillUninitializedMemory());
+}
+
+// Uninitialised device tensors from torch's CUDA allocator, where nothing sees them without the trip through the dispatcher, which is
+// most of what at::empty costs: a forward allocates two and a backward five (0.4 us each: a forward's host time without its launch 5.0 -> 4.3 us).
 Tensor empty_on(at::IntArrayRef sizes, at::ScalarType type, at::Device device) {
+  if (allocations_are_seen()) return at::empty(sizes, at::TensorOptions().dtype(type).device(device));
   return Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
 }
 // in the memory order of a dense tensor, as at::empty_like
 Tensor empty_like_of(const Tensor& like, at::ScalarType type) {
-  if (!like.is_non_overlapping_and_dense()) return at::empty_like(like, like.options().dtype(type));
+  if (!like.is_non_overlapping_and_dense() || allocations_are_seen()) return at::empty_like(like, like.options().dtype(type));
   return Tensor(at::detail::empty_strided_cuda(like.sizes(), like.strides(), type, like.device()));
 }
 

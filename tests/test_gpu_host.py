@@ -179,6 +179,50 @@ def test_tracing_is_refused():
             trace(lambda a: cocktail_scores(a, tokens), x)
 
 
+def test_allocations_are_seen_by_dispatch_modes():
+    """A mode of the caller's sees the tensors that a call allocates; one that hands out tensors without memory makes the call fail."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from kerneldev_b200 import cocktail_scores, flash_attention, metadata_from_tokens
+    seen = []
+
+    class Record(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            out = func(*args, **(kwargs or {}))
+            if func.overloadpacket in (torch.ops.aten.empty, torch.ops.aten.empty_like):
+                seen.append((tuple(out.shape), out.dtype))
+            return out
+
+    q = torch.randn((1, 2, 150, 64), device=DEV).bfloat16()
+    x, tokens = torch.randn((1, 64, 16), device=DEV), _span_tokens(1, 64)
+    want, want_wide = flash_attention(q, q, q, causal=True), flash_attention(q.float(), q.float(), q.float(), causal=True)
+    with Record():
+        o, lse = flash_attention(q, q, q, causal=True, return_lse=True)
+        wide = flash_attention(q.float(), q.float(), q.float(), causal=True)
+        scores = cocktail_scores(x, tokens)
+        in_span, _, _ = metadata_from_tokens(tokens)
+    assert torch.equal(o, want) and torch.equal(wide, want_wide)
+    for t in (o, lse, wide, scores, in_span):
+        assert (tuple(t.shape), t.dtype) in seen
+    with FakeTensorMode(allow_non_fake_inputs=True), pytest.raises(RuntimeError):
+        flash_attention(q, q, q, causal=True)
+
+
+def test_new_memory_is_filled_where_torch_fills_it():
+    """torch.utils.deterministic.fill_uninitialized_memory: what a call allocates and does not write (here dK and dV) reads as NaN."""
+    from kerneldev_b200.original_kernel import _backward, _forward
+    from kerneldev_b200.plan import AttentionPlan
+    q = torch.randn((1, 2, 150, 64), device=DEV).bfloat16()
+    plan = AttentionPlan(1, 150, torch.device(DEV))
+    o, lse = _forward(q, q, q, plan, 0.125)
+    torch.use_deterministic_algorithms(True)
+    try:
+        dq, dk, dv = _backward(q, q, q, o, lse, q, plan, 0.125, 1, deterministic=True)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert torch.isfinite(dq).all() and torch.isnan(dk).all() and torch.isnan(dv).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_undefined_gradients_count_as_zeros(dtype):
     from kerneldev_b200 import cocktail_scores, flash_attention
