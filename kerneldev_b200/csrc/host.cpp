@@ -440,7 +440,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   if (rounds && tma_ready(d_o)) {
     f.d_o = desc(d_o_);   // the delta kernel fills d_o
   } else {
-    d_o = usable(f32 ? d_o_.to(at::kHalf) : d_o_);   // (the engine brings float32; a node that is called by hand may get another type)
+    d_o = usable(f32 ? d_o_.to(at::kHalf) : d_o_);
   }
   if (!dq.defined()) {
     const auto type = f32 ? at::kFloat : q.scalar_type();
@@ -539,7 +539,12 @@ struct AttentionBackward : torch::autograd::Node {
     at::NoGradGuard no_grad;
     // a gradient that a later node left undefined counts as zeros, as for autograd.Function
     const bool direct = widen && !signs.has_value();   // the transform of dQ and dK works on 16-bit tensors
-    const Tensor d_o = !grads[0].defined() ? at::zeros_like(to) : widen && !direct ? cast({grads[0]}, at::kHalf)[0] : grads[0];
+    Tensor d_o = grads[0].defined() ? grads[0] : at::zeros_like(to);
+    // The engine brings a gradient like the output; a node that is called by hand may get any, which the kernels would read as what it is not.
+    KD_VALUE(d_o.sizes() == to.sizes() && d_o.device() == to.device(), "the gradient of an output of shape ", to.sizes(), " on ", to.device(), " has shape ",
+             d_o.sizes(), " on ", d_o.device());
+    if (grads[0].defined()) d_o = d_o.to(widen ? at::kFloat : to.scalar_type());
+    if (widen && !direct) d_o = cast({d_o}, at::kHalf)[0];
     auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
                                  opt.heads_per_cta, direct);
     if (signs.has_value()) {

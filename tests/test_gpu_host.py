@@ -243,17 +243,23 @@ def test_undefined_gradients_count_as_zeros(dtype):
         assert g.shape == t.shape and g.dtype == dtype and not g.any()
 
 
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float64])
-def test_node_of_a_float32_call_by_hand(dtype):
-    """The engine brings a gradient in the output's type, a caller of the node may not: it is converted, never read as what it is not."""
-    from kerneldev_b200 import flash_attention
+@pytest.mark.parametrize("signs", [False, True])
+@pytest.mark.parametrize("dtype,other", [(torch.float32, torch.bfloat16), (torch.float32, torch.float16), (torch.float32, torch.float64),
+                                         (torch.bfloat16, torch.float32), (torch.float16, torch.bool)])
+def test_node_called_by_hand(dtype, other, signs):
+    """The engine brings a gradient in the output's type and shape, a caller of the node may not: it is converted or refused, never
+    read as what it is not."""
+    from kerneldev_b200 import flash_attention, generate_hadamard_signs
     g = torch.Generator(device=DEV).manual_seed(4)
-    q, k, v, do = (torch.randn((1, 2, 150, 64), generator=g, device=DEV) for _ in range(4))
-    do = do.bfloat16().float()   # converting it to any of the types and then to float16 rounds once
-    o = flash_attention(q.requires_grad_(), k.requires_grad_(), v.requires_grad_(), deterministic=True)
+    q, k, v = (torch.randn((1, 2, 150, 64), generator=g, device=DEV).to(dtype).requires_grad_() for _ in range(3))
+    do = torch.randint(0, 2, (1, 2, 150, 64), generator=g, device=DEV).to(dtype)   # exact in every type
+    o = flash_attention(q, k, v, deterministic=True, hadamard_signs=generate_hadamard_signs(2, 64) if signs else None)
     want = o.grad_fn(do)
-    for x, y in zip(o.grad_fn(do.to(dtype)), want):
-        assert x.dtype == torch.float32 and torch.equal(x, y)
+    for x, y in zip(o.grad_fn(do.to(other)), want):
+        assert x.dtype == dtype and torch.equal(x, y)
+    for wrong in (do[:, :, :100], do[:, :1], do.cpu()):
+        with pytest.raises(ValueError, match="the gradient of an output"):
+            o.grad_fn(wrong)
 
 
 def test_other_threads_run_while_the_host_waits(monkeypatch):
