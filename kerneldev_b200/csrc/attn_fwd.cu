@@ -670,7 +670,7 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   // 187.6 -> 182.3). Not where a CTA has one item: its rows leave as soon either way, and the map costs the host time. (Nor for strides
   // that a map cannot have: 0 or below.)
   CUtensorMap tmO = tmQ;
-  a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, "o", 64) == 0 ? 1 : 0;
+  a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, nullptr, 64) == 0 ? 1 : 0;
   auto run = [&](auto launch_fn) { return launch_fn(n_items, a, tmQ, tmK, tmV, tmO, stream); };
   return f32 ? run(launch_fwd_t<false, true>) : p.dtype == KD_BF16 ? run(launch_fwd_t<true, false>) : run(launch_fwd_t<false, false>);
 }

@@ -47,17 +47,18 @@ static CUresult with_context(F encode) {
   return r;
 }
 
-// a box is 128 bytes wide, whatever D is (or 64), and swizzled over that width
+// a box is 128 bytes wide, whatever D is (or 64), and swizzled over that width. name NULL: a map that the call can do without, no message
 static int encode_4d(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, CUtensorMapDataType type, int es,
                      int box_rows, const char* name, int box_bytes = 128) {
+  auto refuse = [&](int code, const char* fmt, auto... args) { return name != nullptr ? set_error(code, fmt, args...) : code; };
   EncodeTiledFn enc = encode_fn();
-  if (!enc) return set_error(KD_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
-  if (t.ptr == nullptr) return set_error(KD_ERR_ARG, "tensor %s is null", name);
-  if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) != 0) return set_error(KD_ERR_ALIGN, "tensor %s: base pointer not 16-byte aligned", name);
+  if (!enc) return refuse(KD_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
+  if (t.ptr == nullptr) return refuse(KD_ERR_ARG, "tensor %s is null", name);
+  if ((reinterpret_cast<uintptr_t>(t.ptr) & 15u) != 0) return refuse(KD_ERR_ALIGN, "tensor %s: base pointer not 16-byte aligned", name);
   const int64_t sb = t.stride_b * es, sh = t.stride_h * es, st = t.stride_t * es;  // bytes
   if (st <= 0 || (st & 15) || (H > 1 && (sh <= 0 || (sh & 15))) || (B > 1 && (sb <= 0 || (sb & 15))))
-    return set_error(KD_ERR_ALIGN, "tensor %s: byte strides (%lld, %lld, %lld) must be positive multiples of 16",
-                     name, (long long)sb, (long long)sh, (long long)st);
+    return refuse(KD_ERR_ALIGN, "tensor %s: byte strides (%lld, %lld, %lld) must be positive multiples of 16",
+                  name, (long long)sb, (long long)sh, (long long)st);
   // For a D that is no multiple of the box (64 elements of 16 bits) the elements beyond the tensor are filled with zeros, which
   // leaves every product of the kernels unchanged, and not written by stores.
   cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)T, (cuuint64_t)H, (cuuint64_t)B};
@@ -70,7 +71,7 @@ static int encode_4d(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, 
   const CUresult r = with_context([&] { return enc(out, type, 4, t.ptr, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); });
-  if (r != CUDA_SUCCESS) return set_error(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
+  if (r != CUDA_SUCCESS) return refuse(KD_ERR_ARG, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", name, (int)r);
   return 0;
 }
 

@@ -73,7 +73,7 @@ inline cudaError_t launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
 int set_error(int code, const char* fmt, ...);
 
 // 4-D tensor map over a (B,H,T,D) tensor with box (64 elements along D, `box_rows` tokens),
-// 128-byte swizzle, zero fill outside the tensor. box_bytes = 64: half the width and swizzle.
+// 128-byte swizzle, zero fill outside the tensor. box_bytes = 64: half the width and swizzle. name = NULL: a refusal leaves no message.
 int encode_tensor_map(CUtensorMap* out, const kd_tensor& t, int B, int H, int T, int D, int dtype,
                       int box_rows, const char* name, int box_bytes = 128);
 

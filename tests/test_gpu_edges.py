@@ -298,3 +298,30 @@ def test_deterministic_backward_behind_one_another(B, H, T, D, dtype):
         _, _, *ref = ao.attention_fwd_bwd(*(x.detach().float().cpu() for x in (q, k, v, dos[i])), mask)
         for name, got, want in zip(("dQ", "dK", "dV"), together[i], ref):
             assert_close(name, got, want)   # P and dS are rounded to 16 bits: the repository's tolerance for that
+
+
+@pytest.mark.parametrize("D", [64, 80])
+def test_forward_into_rows_in_descending_order(D):
+    """O with a negative time stride, which no tensor map describes, in a call with more items than SMs: written row by row, and the
+    call, which succeeds, leaves no message of a refused map behind."""
+    import ctypes
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import _capi
+    from kerneldev_b200.original_kernel import _forward, _kd_tensor, _params
+    from kerneldev_b200.plan import AttentionPlan
+    B, H, T = 15, 10, 159
+    q, k, v, _ = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.bfloat16, seed=D))
+    plan = AttentionPlan(B, T, torch.device(DEV))
+    want, lse = _forward(q, k, v, plan, 0.125)
+    back = torch.empty_like(want)
+    lib = _capi.load()
+    p = _params(q, k, v, back, torch.empty_like(lse), plan, 0.125)
+    p.D = 7
+    assert lib.kd_attn_fwd(ctypes.byref(p), None) != 0
+    message = lib.kd_last_error()
+    p.D = D
+    p.o = _capi.KdTensor(back.data_ptr() + (T - 1) * D * 2, H * T * D, T * D, -D)
+    torch.cuda.synchronize()
+    assert lib.kd_attn_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
+    assert message and lib.kd_last_error() == message
+    assert torch.equal(back.flip(2), want)
