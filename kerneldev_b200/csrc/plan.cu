@@ -244,10 +244,8 @@ __global__ void __launch_bounds__(CL_THREADS) classify_kernel(PlanView pv) {
 // 3. short sequences: the whole plan of a sequence by one CTA, in one launch
 // ---------------------------------------------------------------------------------------
 // Nothing but latency: the descriptors, class masks and tile classes of up to 1024 tokens stay in shared memory between the steps, where
-// the two kernels above hand them over through global memory and a launch. Up to eight tiles a CTA's sixteen warps classify a
-// sequence's tiles in four rounds; beyond that (or with many sequences, whose span ids the first CTA checks) the CTA per list is faster.
-// 1 x 173 tokens: 1.9 + 6.0 us in two launches, 4.1 in one; a pass of eight forwards with a new plan 69.4 -> 66.1 us, most of it the launch.
-constexpr int PS_TILES = 8, PS_BATCH = 16, PS_THREADS = 512, PS_WARPS = PS_THREADS / 32;
+// the two kernels above hand them over through global memory and a launch. For which calls: see launch_classify.
+constexpr int PS_TILES = 8, PS_THREADS = 512, PS_WARPS = PS_THREADS / 32;
 __global__ void __launch_bounds__(PS_THREADS) plan_small_kernel(kd_meta m, PlanView pv) {
   __shared__ uint32_t s_desc[PS_TILES * KD_TILE], s_bits[PS_TILES * 32];
   __shared__ uint32_t s_or[PS_TILES * 4], s_and[PS_TILES * 4];
@@ -359,7 +357,15 @@ int launch_classify(const kd_meta& m, void* plan, cudaStream_t stream) {
   if (kd_plan_layout_get(m.B, m.T, &L) != 0) return KD_ERR_ARG;
   PlanView pv = make_plan_view(plan, L);
   cudaError_t e;
-  if (L.NT <= PS_TILES && m.B <= PS_BATCH) {
+  // One launch where it is the faster one whatever the metadata says. Time of a plan in a chain of them (us), two launches | one; sections
+  // of the model's layout, then flags and ids drawn for each token (every tile PARTIAL):
+  //   1 x 173 6.6 | 3.6, 7.7 | 4.2    8 x 173 6.8 | 5.8, 7.3 | 6.4     12 x 173 6.9 | 7.2, 7.6 | 7.4
+  //   1 x 512 5.7 | 3.9, 7.8 | 5.5    8 x 512 7.0 | 6.2, 7.6 | 7.5     12 x 512 7.1 | 7.6, 7.6 | 8.9
+  //   1 x 640 6.6 | 4.2, 7.9 | 7.8    4 x 640 7.3 | 5.2, 8.1 | 8.7     1 x 1024 7.1 | 5.7, 7.5 | 12.9    16 x 1024 8.4 | 11.1, 10.7 | 18.1
+  // Four tiles are one for each of the CTA's warps; with metadata the first CTA also looks at the span ids of one sequence after the other.
+  // Without metadata neither counts: 1 x 173 6.6 | 2.8, 16 x 173 6.6 | 2.6, 1 x 1024 6.1 | 4.2, 16 x 1024 6.7 | 4.2, with lengths 7.4 | 6.3.
+  const bool small = m.rules ? L.NT <= 4 && m.B <= 8 : L.NT <= PS_TILES && m.B <= 16;
+  if (small) {
     e = launch(plan_small_kernel, m.B, PS_THREADS, 0, stream, m, pv);
   } else {
     e = launch(pack_kernel, dim3(L.NT, m.B), KD_TILE, 0, stream, m, pv);

@@ -107,8 +107,8 @@ def test_span_id_out_of_range_is_reported():
         _plan(T, ins, sid, None)
 
 
-# one CTA per sequence up to 1024 tokens and 16 sequences, two kernels beyond
-@pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (2, 129), (16, 300), (17, 300), (16, 1024), (1, 1025), (17, 1024)])
+# one CTA per sequence up to 512 tokens and 8 sequences, two kernels beyond
+@pytest.mark.parametrize("B,T", [(1, 1), (1, 127), (2, 129), (8, 512), (9, 512), (8, 513), (16, 300), (17, 300), (16, 1024), (1, 1025), (17, 1024)])
 def test_both_forms_of_the_plan_kernels(B, T):
     ins, sid, pre = random_meta(B + T, B, T, sid_range=(-1, 9))
     lens = np.array([(T, 0, 1, T - 1, T // 2)[b % 5] for b in range(B)], np.int32)
@@ -119,3 +119,12 @@ def test_both_forms_of_the_plan_kernels(B, T):
     with pytest.raises(ValueError, match="span_id"):
         _plan(T, ins, sid, pre, None)
     _plan(T, ins, sid, pre, np.full(B, T - 1, np.int32))
+
+
+# without metadata one CTA per sequence up to 1024 tokens and 16 sequences
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("B,T", [(1, 1), (3, 640), (16, 1024), (17, 1024), (16, 1025)])
+def test_both_forms_of_the_plan_kernels_without_metadata(B, T, causal):
+    lens = np.array([(T, 0, 1, T - 1, T // 2)[b % 5] for b in range(B)], np.int32)
+    _check(_plan(T, lens=lens, causal=causal), ao.dense_mask(T, lens=lens, causal=causal))
+    _check(_plan(T, causal=causal, B=B), ao.dense_mask(T, causal=causal, B=B))
