@@ -72,7 +72,7 @@ enum : uint32_t {
 // =========================================================================================
 // A float32 call (kF32) leaves two more passes to it: dO is rounded to the 16-bit operand on the way, and dQ, into which the fused
 // backward then adds, is zeroed in place of a scratch.
-template <int HD, bool kBf16, bool kF32 = false>
+template <int HD, bool kBf16, bool kF32>
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
   constexpr int TPR = HD / 8;   // threads per row
   constexpr int RPB = 256 / TPR;   // rows per block and iteration
@@ -311,8 +311,9 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
 // dQ kernel: items are query tiles; streams = key halves of the current key
 // tile.   M1(i): S_i = Q K_i^T, dP_i = dO V_i^T      M2(i): dQ += dS_i K_i
 // The producer and the issuers run on into the next item while the compute warps finish the current one.
+// kF32: of a float32 call, whose gradients are float32. (As a branch of the float16 kernels: causal 8 x 16 x 2048 x 128 610.8 us, 609.4 so; level at head dim 64.)
 // =========================================================================================
-template <int HD, bool kBf16>
+template <int HD, bool kBf16, bool kF32>
 __global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -612,7 +613,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
         for (int cb = 0; cb < EC / ECH; ++cb) {
           const int col = g * EC + cb * ECH;
-          if (!kBf16 && a.grads_f32) {
+          if constexpr (kF32) {
             float* wide = static_cast<float*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + (size_t)qi * a.dq_st + col;
             if constexpr (ECH == 16) store_row16_f32_upto(wide, r[cb], a.sm_scale, col, a.d_real);
             else store_row32_f32_upto(wide, r[cb], a.sm_scale, col, a.d_real);
@@ -636,7 +637,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // dK/dV kernel: items are key tiles; streams = query halves of the current
 // query tile.   M1(i): S^T_i = K Q_i^T, dP^T_i = V dO_i^T     M2(i): dV += P^T_i dO_i,  dK += dS^T_i Q_i
 // =========================================================================================
-template <int HD, bool kBf16>
+template <int HD, bool kBf16, bool kF32>
 __global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -997,7 +998,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int j = 0; j < ECH; ++j) { rk[j] = 0u; rv[j] = 0u; }
         }
         const int col = g * EC + cb * ECH;
-        if (kj < a.T && !kBf16 && a.grads_f32) {
+        if (kF32 && kj < a.T) {
           float* kw = static_cast<float*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st + col;
           float* vw = static_cast<float*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st + col;
           if constexpr (ECH == 16) {
@@ -1027,7 +1028,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (a.after_dq != 0) pdl_wait();
 }
 
-template <int HD, bool kBf16>
+template <int HD, bool kBf16, bool kF32>
 static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
   using C = BwdCfg<HD>;
   CUtensorMap tmQ, tmK, tmV, tmDO;
@@ -1060,8 +1061,8 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.d_o32 = f32 ? static_cast<const float*>(f32->d_o.ptr) : nullptr;
   if (f32) { a.do32_sb = f32->d_o.stride_b; a.do32_sh = f32->d_o.stride_h; a.do32_st = f32->d_o.stride_t; }
  
-  auto kq = attn_bwd_dq_kernel<HD, kBf16>;
-  auto kk = attn_bwd_dkdv_kernel<HD, kBf16>;
+  auto kq = attn_bwd_dq_kernel<HD, kBf16, kF32>;
+  auto kk = attn_bwd_dkdv_kernel<HD, kBf16, kF32>;
   static SmemOptIn opt_in_q, opt_in_k;
   cudaError_t e = opt_in_q(kq, C::SMEM_ALLOC);
   if (e == cudaSuccess) e = opt_in_k(kk, C::SMEM_ALLOC);
@@ -1075,10 +1076,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
     const size_t rows = (size_t)p.B * p.H * p.T;
     const int rows_per_block = 256 / (HD / 8);
     const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-    if constexpr (!kBf16) {
-      if (f32) e = launch(attn_bwd_delta_kernel<HD, kBf16, true>, blocks, 256, 0, stream, a);
-    }
-    if (!f32) e = launch(attn_bwd_delta_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
+    e = launch(attn_bwd_delta_kernel<HD, kBf16, kF32>, blocks, 256, 0, stream, a);
     if (!fused && e == cudaSuccess) e = launch(kq, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
   if (fused && e == cudaSuccess) {
@@ -1138,8 +1136,11 @@ int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
   PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
   if (!p.d_o.ptr) return set_error(KD_ERR_ARG, "d_o is null");
-  if (p.D <= 64) return p.dtype == KD_BF16 ? launch_bwd_t<64, true>(p, f32, L, pv, stream) : launch_bwd_t<64, false>(p, f32, L, pv, stream);
-  return p.dtype == KD_BF16 ? launch_bwd_t<128, true>(p, f32, L, pv, stream) : launch_bwd_t<128, false>(p, f32, L, pv, stream);
+  auto run = [&](auto launch_fn) { return launch_fn(p, f32, L, pv, stream); };
+  const bool narrow = p.D <= 64;
+  if (f32) return narrow ? run(launch_bwd_t<64, false, true>) : run(launch_bwd_t<128, false, true>);
+  if (p.dtype == KD_BF16) return narrow ? run(launch_bwd_t<64, true, false>) : run(launch_bwd_t<128, true, false>);
+  return narrow ? run(launch_bwd_t<64, false, false>) : run(launch_bwd_t<128, false, false>);
 }
 
 }  // namespace kd
