@@ -41,7 +41,7 @@
 // Work items. An item is one (batch, head, key tile). The grid has a CTA per item, but a CTA that is running takes
 // further items by cancelling CTAs that have not been launched yet (clusterlaunchcontrol) and works on them without
 // draining its pipeline: the rings of Q and dO tiles run on into the next item, K has two buffers at HD = 64
-// (at HD = 128 shared memory holds one of each, and the next K takes V's, which is free first), and dK and dV of the finished item leave through the dQ warps while the
+// (shared memory holds one at HD = 128), and dK and dV of the finished item leave through the dQ warps while the
 // next item's first products run. Starting a CTA costs some 12,000 cycles (launch, TMEM, first loads, pipeline fill,
 // drain), and a (batch, head, key tile) has around ten tiles.
 // Items are numbered in chunks of heads whose scratch and operands fit L2 together (ItemOrder), inside a
@@ -78,7 +78,7 @@ struct FusedCfg {
   static constexpr int NK = (HD == 64) ? 2 : 1;      // K buffers (head hh in buffer hh % NK)
   static constexpr int QS = (HD == 64) ? 4 : 2;      // ring stages of Q tiles: held from S^T of a tile to its dK
   static constexpr int OS = (HD == 64) ? 2 : 1;      // ring stages of dO tiles: held from dP^T to dV
-  static constexpr int SMEM_K = 0;                   // HD = 128: K and V change buffers with every item (K of item m in buffer m & 1)
+  static constexpr int SMEM_K = 0;
   static constexpr int SMEM_V = SMEM_K + NK * TILE_BYTES;
   static constexpr int SMEM_Q = SMEM_V + TILE_BYTES;
   static constexpr int SMEM_DO = SMEM_Q + QS * TILE_BYTES;
@@ -541,14 +541,14 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // ---- issuing warp A: S^T and dV ----
         int q_stage = 0, do_stage = 0;
         uint32_t q_parity = 0, do_parity = 0;
-        auto issue_s = [&](int item) {
+        auto issue_s = [&]() {
           tc_fence_after_sync();
-          product_kmajor(C::TM_S, lo_k0 + (item & 1) * T16, lo_q0 + q_stage * T16);
+          product_kmajor(C::TM_S, lo_k0, lo_q0 + q_stage * T16);
           commit_uniform(bar(C::B_SFULL));
           if (++q_stage == C::QS) { q_stage = 0; q_parity ^= 1u; }
         };
         advance();
-        if (have && (ok = wait(C::B_KFULL, 0, W_U_KFULL) && wait(C::B_QFULL, 0, W_U_QFULL))) issue_s(0);
+        if (have && (ok = wait(C::B_KFULL, 0, W_U_KFULL) && wait(C::B_QFULL, 0, W_U_QFULL))) issue_s();
         while (have && ok) {
           const int n = it.w;
           for (int e = 0; e < n; ++e, ++t) {
@@ -566,7 +566,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (have) {   // S^T of the next tile over P^T, whose reader precedes it in the pipe
               if (last && !(ok = wait(C::B_KFULL, (m + 1) & 1, W_U_KFULL))) break;
               if (!(ok = wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL))) break;
-              issue_s(last ? m + 1 : m);
+              issue_s();
             }
           }
           ++m;
@@ -575,40 +575,34 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // ---- issuing warp B: dP^T, dK and dQ ----
         int q_stage = 0, do_stage = 0, k_loads = 1, v_loads = 1;
         uint32_t do_parity = 0;
-        auto issue_dp = [&](int item) {
+        auto issue_dp = [&]() {
           tc_fence_after_sync();
-          product_kmajor(C::TM_DP, lo_k0 + ((item & 1) ^ 1) * T16, lo_do0 + do_stage * T16);
+          product_kmajor(C::TM_DP, lo_v, lo_do0 + do_stage * T16);
           commit_uniform(bar(C::B_DPFULL));
           commit_uniform(bar(C::B_DOEMPTY + do_stage));
           if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
         };
         advance();
-        if (have && (ok = wait(C::B_VFULL, 0, W_U_VFULL) && wait(C::B_DOFULL, 0, W_U_DOFULL))) issue_dp(0);
+        if (have && (ok = wait(C::B_VFULL, 0, W_U_VFULL) && wait(C::B_DOFULL, 0, W_U_DOFULL))) issue_dp();
         while (have && ok) {
           const int n = it.w;
           for (int e = 0; e < n; ++e, ++t) {
             const bool last = (e == n - 1);
             if (e == 0 && m > 0 && !(ok = wait(C::B_ACCFREE + 1, (m - 1) & 1, W_U_ACCFREE))) break;
-            // V's last reader in this item, dP^T, is done when dS^T(t) is: the next item's K goes into its buffer then (before the products
-            // below if that item is known), and the next item's V into K's, when dQ(t) has read that. (Each into its own buffer: K, which the
-            // next S^T waits for, came 3,200 cycles late. V has the time that P^T takes. Asked for when dP^T(t) is done, K would come
-            // 1,300 cycles sooner, but the next dO then waits as much longer for V's dP^T; and dP^T(t) may be done before this
-            // item's K has landed, whose barrier must not be armed again before.)
-            bool k_asked = false;
-            auto request = [&](const CUtensorMap* tm, bool into_v, int full) {   // into_v: into the buffer that holds V now
-              if (elect_one()) load_tile(tm, sK + ((m & 1) ^ (into_v ? 1 : 0)) * TILE, full, it.z & 0xFFFF, it.y, it.x);
-            };
-            auto request_k = [&]() {
-              advance();
-              k_asked = true;
-              if (!have) return;
-              request(&tmK, true, C::B_KFULL);
-              ++k_loads;
-            };
             if (!(ok = wait(C::B_DSFULL, t & 1, W_U_DSFULL))) break;
-            if (last && __all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) request_k();
+            // V's last reader in this item, dP^T(t), is done: the next item's V goes into the same buffer, before the products
+            // below if that item is known
+            bool v_asked = false;
+            if (last && __all_sync(0xffffffffu, mbar_test_wait(bar(C::B_ITEMFULL + k % C::NITEM), (k / C::NITEM) & 1))) {
+              advance();
+              v_asked = true;
+              if (have) {
+                if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
+                ++v_loads;
+              }
+            }
             tc_fence_after_sync();
-            product_dq(k_mn0 + (m & 1) * T16);   // over dP^T(t), which dS^T(t) was made from
+            product_dq(k_mn0);   // over dP^T(t), which dS^T(t) was made from
             commit_uniform(bar(C::B_DQFULL));
 #pragma unroll 1
             for (int w = 0; w < 2; ++w) product_dk(w, q_mn0 + q_stage * T16, e == 0 && w == 0);
@@ -617,18 +611,24 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (++q_stage == C::QS) q_stage = 0;
             if (last) {
               commit_uniform(bar(C::B_ACCFULL + 1));
-              if (!k_asked) request_k();
-              if (have) {
-                if (!(ok = wait(C::B_DQFULL, t & 1, W_U_DQFULL))) break;
-                request(&tmV, false, C::B_VFULL);
-                ++v_loads;
+              if (!v_asked) {
+                advance();
+                if (have) {
+                  if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
+                  ++v_loads;
+                }
+              }
+              if (have) {   // one K buffer: the next item's K can only be requested when the products above are done
+                if (!(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
+                if (elect_one()) load_tile(&tmK, sK, C::B_KFULL, it.z & 0xFFFF, it.y, it.x);
+                ++k_loads;
               }
             }
             if (have) {
               if (!(ok = wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY))) break;
               if (last && !(ok = wait(C::B_VFULL, (m + 1) & 1, W_U_VFULL))) break;
               if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
-              issue_dp(last ? m + 1 : m);
+              issue_dp();
             }
           }
           ++m;
