@@ -75,7 +75,7 @@ struct FusedCfg {
   static constexpr int HD = HD_;
   static constexpr int KBLK = HD / 64;               // 64-element blocks along D
   static constexpr int TILE_BYTES = KD_TILE * HD * 2;
-  static constexpr int NK = (HD == 64) ? 2 : 1;      // K buffers (head hh in buffer hh % NK)
+  static constexpr int NK = (HD == 64) ? 2 : 1;      // K buffers (K of the CTA's item m in buffer m % NK)
   static constexpr int QS = (HD == 64) ? 4 : 2;      // ring stages of Q tiles: held from S^T of a tile to its dK
   static constexpr int OS = (HD == 64) ? 2 : 1;      // ring stages of dO tiles: held from dP^T to dV
   static constexpr int SMEM_K = 0;
