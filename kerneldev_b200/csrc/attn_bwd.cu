@@ -323,7 +323,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sFix = smem_u32(smem + C::SMEM_FIX);    // buffer f: Q at +0, dO at +TILE_BYTES
   const uint32_t sRing = smem_u32(smem + C::SMEM_RING);  // stage s: K at +0, V at +TILE_BYTES
-  uint32_t* sStage = reinterpret_cast<uint32_t*>(smem + C::SMEM_STAGE);
   uint16_t* lists = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
   __shared__ BwdShared<C> sh;
 

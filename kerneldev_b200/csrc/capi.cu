@@ -123,7 +123,7 @@ static int check_attn(const kd_attn_params* p, bool backward, const kd_attn_f32*
   if (p->T > 128 * KD_TILE) return set_error(KD_ERR_LIMIT, "T=%d exceeds the maximum of %d tokens", p->T, 128 * KD_TILE);
   if (p->H > 65535 || p->B > 65535) return set_error(KD_ERR_LIMIT, "B and H must not exceed 65535");
   if (!(p->sm_scale > 0.f) || !(p->sm_scale < 1e30f)) return set_error(KD_ERR_ARG, "sm_scale must be positive and finite");
-  if (p->heads_per_cta < 0) return set_error(KD_ERR_ARG, "heads_per_cta must be 0 (automatic) or positive");
+  if (p->heads_per_cta < 0) return set_error(KD_ERR_ARG, "heads_per_cta must not be negative");
   if (!p->plan) return set_error(KD_ERR_ARG, "plan is null (call kd_classify first)");
   if (backward && !p->lse) return set_error(KD_ERR_ARG, "lse is null");
   if (f32) {

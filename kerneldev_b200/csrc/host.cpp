@@ -430,8 +430,7 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Ten
 // `phases` selects a part of the backward (kd_attn_params.bwd_phases); defined tensors among dq .. dq_acc are reused.
 std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o, const Tensor& lse,
                                             const Tensor& d_o_, const PlanPtr& plan, double sm_scale, int phases, Tensor dq, Tensor dk,
-                                            Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic,
-                                            int heads_per_cta, bool f32 = false) {
+                                            Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic, bool f32 = false) {
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
   kd_attn_f32 f{};
   Tensor d_o;
@@ -453,7 +452,6 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   // rows as wide as the kernel's tile (kd_workspace_bytes_fused)
   if (fused && !f32 && !dq_acc.defined()) dq_acc = empty_on({q.size(0), q.size(1), q.size(2), q.size(3) <= 64 ? 64 : 128}, at::kFloat, q.device());
   kd_attn_params p = params(q, k, v, o, lse, *plan, sm_scale);
-  p.heads_per_cta = heads_per_cta;
   p.d_o = desc(d_o);
   (f32 ? f.dq : p.dq) = desc(dq);
   (f32 ? f.dk : p.dk) = desc(dk);
@@ -513,7 +511,6 @@ Tensor hadamard(const Tensor& x_, const OptTensor& signs, bool inverse) {
 struct Options {
   double sm_scale;
   bool like_input, deterministic;
-  int heads_per_cta;   // kd_attn_params.heads_per_cta
 };
 
 // dQ, dK, dV of one flash_attention call. Saves the operands the kernels read: for float32 tensors their float16
@@ -545,8 +542,7 @@ struct AttentionBackward : torch::autograd::Node {
              d_o.sizes(), " on ", d_o.device());
     if (grads[0].defined()) d_o = d_o.to(widen ? at::kFloat : to.scalar_type());
     if (widen && !direct) d_o = cast({d_o}, at::kHalf)[0];
-    auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic,
-                                 opt.heads_per_cta, direct);
+    auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic, direct);
     if (signs.has_value()) {
       // y = x diag(s) W / sqrt(D) with W symmetric, so dx = dy W / sqrt(D) diag(s)
       dq = hadamard(dq, signs, true);
@@ -600,7 +596,7 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v) {
 
 std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& lens, std::optional<double> sm_scale,
                                      bool causal, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix, bool rules,
-                                     const OptTensor& signs, bool like_input, bool deterministic, int heads_per_cta, bool return_lse) {
+                                     const OptTensor& signs, bool like_input, bool deterministic, bool return_lse) {
   check_inputs(q, k, v);
   refuse_forward_ad("flash_attention", q, k, v);
   refuse_tracing("flash_attention");
@@ -633,7 +629,7 @@ std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& k, const Ten
     auto node = std::shared_ptr<AttentionBackward>(new AttentionBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
     node->plan = std::move(plan);
-    node->opt = Options{scale, like_input, deterministic, heads_per_cta};
+    node->opt = Options{scale, like_input, deterministic};
     node->signs = signs;
     node->widen = f32;
     torch::autograd::set_history(o, node);
@@ -883,10 +879,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return forward(q, k, v, plan, sm_scale, like_input);
   }, NoGil());
   m.def("backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, const PlanPtr& plan,
-                       double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic, int heads_per_cta) {
+                       double sm_scale, int phases, const std::vector<Tensor>& bufs, bool like_input, bool deterministic) {
     Tensor b[5];
     for (size_t i = 0; i < bufs.size() && i < 5; ++i) b[i] = bufs[i];
-    return backward(q, k, v, o, lse, d_o, plan, sm_scale, phases, b[0], b[1], b[2], b[3], b[4], like_input, deterministic, heads_per_cta);
+    return backward(q, k, v, o, lse, d_o, plan, sm_scale, phases, b[0], b[1], b[2], b[3], b[4], like_input, deterministic);
   }, NoGil());
   m.def("hadamard", &hadamard, NoGil());
   m.def("attention", &attention, NoGil());

@@ -18,17 +18,4 @@ namespace kd {
 // A call by itself gains in all of them or is level.
 inline int split_pairs(long long pairs, int tiles, int sms) { return tiles > 1 && (4 * pairs <= sms || (tiles >= 5 && 2 * pairs <= sms)) ? 1 : 0; }
 
-// Heads that a CTA of a grid with a CTA per (tile, group of heads) should handle one after the other: as many as keep six CTAs per SM, at
-// most eight, and two where lists are short against a CTA's start and drain. The kernels take single items dynamically now and ask
-// nobody (a grouped item costs balance and saves nothing: 16 x 16 x 4096 x 64 hierarchical, dQ kernel 699 us with groups, 598 without);
-// for hosts that size such a grid themselves. `tiles`: tiles of a head.
-inline int heads_per_cta(long long pairs, int heads, int tiles, int forced, int sms) {   // pairs: (batch, head) pairs
-  if (forced >= 1) return forced < heads ? forced : heads;
-  const long long ctas = pairs * tiles;
-  long long g = ctas / (6LL * sms);
-  if (g < 2) g = (tiles <= 20 && ctas >= 5LL * sms) || (tiles <= 32 && ctas >= 7LL * sms) ? 2 : 1;
-  if (g > 8) g = 8;
-  return static_cast<int>(g < heads ? g : heads);
-}
-
 }  // namespace kd

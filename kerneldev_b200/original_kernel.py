@@ -32,9 +32,6 @@ __all__ = ["flash_attention", "generate_hadamard_signs", "hadamard_transform"]
 _HADAMARD_DIMS = (16, 32, 64, 128)
 _DTYPES = {torch.float16: _capi.KD_F16, torch.bfloat16: _capi.KD_BF16}
 
-# kd_attn_params.heads_per_cta, which the library accepts and ignores: its kernels take tiles of single heads.
-HEADS_PER_CTA = 0
-
 
 def _kd_tensor(t: torch.Tensor) -> _capi.KdTensor:
     return _capi.KdTensor(t.data_ptr(), t.stride(0), t.stride(1), t.stride(2))
@@ -49,7 +46,6 @@ def _params(q, k, v, o, lse, plan, sm_scale):
     p.q, p.k, p.v, p.o = _kd_tensor(q), _kd_tensor(k), _kd_tensor(v), _kd_tensor(o)
     p.lse = lse.data_ptr()
     p.plan = plan.ptr
-    p.heads_per_cta = HEADS_PER_CTA
     return p
 
 
@@ -65,7 +61,7 @@ def _backward(q, k, v, o, lse, d_o, plan: AttentionPlan, sm_scale: float, phases
     kd_attn_params.bwd_phases); ``bufs`` = (dq, dk, dv, delta[, dq_acc]) reuses buffers.
     ``deterministic=False`` selects the fused backward: one pass over the tiles instead of two, dQ accumulated
     with fp32 additions in a scratch (kd_workspace_bytes_fused)."""
-    return _ext.backward(q, k, v, o, lse, d_o, plan._core, sm_scale, phases, list(bufs or ()), like_input, deterministic, HEADS_PER_CTA)
+    return _ext.backward(q, k, v, o, lse, d_o, plan._core, sm_scale, phases, list(bufs or ()), like_input, deterministic)
 
 
 def _hadamard_call(x: torch.Tensor, signs, inverse: bool) -> torch.Tensor:
@@ -170,7 +166,7 @@ def flash_attention(
             raise ValueError("hadamard_signs needs a head_dim in {16, 32, 64, 128}")
         hadamard_signs = _check_signs(hadamard_signs, q.shape[1], q.shape[3], q.device)
     o, lse = _ext.attention(q, k, v, lens, sm_scale, bool(causal), in_span, span_id, is_prefix, rules, hadamard_signs,
-                            out_layout == "input", bool(deterministic), HEADS_PER_CTA, bool(return_lse))
+                            out_layout == "input", bool(deterministic), bool(return_lse))
 
     if return_attention_mask:
         B, H, T, _ = q.shape

@@ -179,21 +179,8 @@ static int split_rule() {   // mistakes
   return bad + split_pairs(1LL << 40, 128, 148);
 }
 
-static int heads_rule() {   // mistakes
-  int bad = 0;
-  for (int tiles = 1; tiles <= 128; ++tiles)
-    for (long long pairs = 1; pairs * tiles < 12 * 148; ++pairs) {
-      const int g = heads_per_cta(pairs, 16, tiles, 0, 148);
-      const long long ctas = pairs * tiles;
-      bad += g < 1 || g > 2 || (g == 2 && (ctas < 740 || tiles > 32 || (tiles > 20 && ctas < 1036)));
-      bad += g == 1 && tiles <= 20 && ctas >= 740;
-      bad += heads_per_cta(pairs, 1, tiles, 0, 148) != 1 || heads_per_cta(pairs, 16, tiles, 3, 148) != 3 || heads_per_cta(pairs, 2, tiles, 3, 148) != 2;
-    }
-  return bad + (heads_per_cta(1LL << 24, 16, 128, 0, 148) != 8);
-}
-
 int main() {
-  int bad = list_rules() + split_rule() + heads_rule(), found = 0;
+  int bad = list_rules() + split_rule(), found = 0;
   for (uint64_t seed = 1; seed <= 20000; ++seed) {
     const char* e = run<AsBuilt>(seed);
     if (e != nullptr && bad++ == 0) printf("seed %llu: %s\n", static_cast<unsigned long long>(seed), e);

@@ -50,10 +50,9 @@ def test_cocktail_scores_and_gradient(B, T, C, dtype):
 @pytest.mark.parametrize("deterministic", [False, True])
 @pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (128, torch.float16), (80, torch.bfloat16)])
 @pytest.mark.parametrize("T,n_full", [(513, 1), (895, 2), (1280, 5)])
-def test_many_items_per_cta_with_empty_ones_between(monkeypatch, T, n_full, D, dtype, deterministic):
+def test_many_items_per_cta_with_empty_ones_between(T, n_full, D, dtype, deterministic):
     from tests.helpers import assert_close, random_meta
-    from kerneldev_b200 import flash_attention, original_kernel
-    monkeypatch.setattr(original_kernel, "HEADS_PER_CTA", 4)   # the deterministic backward's items are tiles of a group of heads
+    from kerneldev_b200 import flash_attention
     B, H = 12, 23
     ins, sid, pre = random_meta(T + D, B, T)
     lens = np.array([T if b % (B // n_full) == 0 else (0, 3, 129)[b % 3] for b in range(B)], np.int32)
@@ -150,10 +149,10 @@ def test_forward_items_of_one_tile(B, H, T, D, dtype):
     assert_lse_close(lse, want_lse)
 
 
-# deterministic backward: one head per CTA up to 739 tiles, two from 740 (an odd number of heads leaves a CTA with one)
+# deterministic backward: 738 and 740 items, some five for each SM, of lists of one and two tiles
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,H", [(9, 41), (10, 37)])
-def test_deterministic_backward_heads_per_cta(B, H, D):
+def test_deterministic_backward_five_items_per_sm(B, H, D):
     from tests.helpers import assert_close, rand_inputs, random_meta
     from kerneldev_b200 import flash_attention
     T = 200
