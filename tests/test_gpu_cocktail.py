@@ -76,3 +76,28 @@ def test_batch_without_spans_and_bad_inputs():
         span_means(e.double(), x)
     with pytest.raises(RuntimeError):
         span_means(e.cpu(), x)
+
+
+def test_number_of_spans_behind_queued_work():
+    """The host reads the number of spans as the index kernel writes it, for 200 us, and waits for the stream where work ahead of the kernel takes
+    longer: the same scores and gradients behind an idle and a busy stream, for rows with more and fewer spans in turn."""
+    from kerneldev_b200 import cocktail_scores
+    tokens = [cocktail_rows(seed, 4, T, unbalanced=True).to(DEV) for seed, T in ((1, 300), (2, 5000), (3, 64), (4, 900))]
+    embeds = [embeddings(i, 4, x.shape[1], 24).to(DEV).requires_grad_() for i, x in enumerate(tokens)]
+
+    def run(cycles):
+        out = []
+        for x, e in zip(tokens, embeds):
+            if cycles:
+                torch.cuda._sleep(cycles)
+            s = cocktail_scores(e, x)
+            out.append((s.detach(), *torch.autograd.grad(s.sum(), e)))
+        torch.cuda.synchronize()
+        return out
+
+    idle = run(0)
+    want = [ao.cocktail_scores(e.detach().double().cpu(), x.cpu())[0].shape for x, e in zip(tokens, embeds)]
+    assert [s.shape for s, _ in idle] == want
+    for cycles in (100_000, 20_000_000):   # some 60 us, and 10 ms
+        for (s, g), (s2, g2) in zip(idle, run(cycles)):
+            assert torch.equal(s, s2) and torch.equal(g, g2)

@@ -324,3 +324,26 @@ def test_forward_into_rows_in_descending_order(D):
     assert lib.kd_attn_fwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0
     assert message and lib.kd_last_error() == message
     assert torch.equal(back.flip(2), want)
+
+
+# 312 pairs of query tiles and 468 key tiles (odd: 780 tiles, some of 1 token), more than SMs: CTAs of all float32 kernels run on into further items, among them runs
+# of tiles without keys or queries. O leaves as float32 beside the 16-bit O of the boxes, dK and dV through both staging boxes between dQ tiles
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("B,H,T,D", [(12, 13, 300, 48), (12, 13, 300, 64), (12, 13, 300, 80), (12, 13, 300, 128), (12, 13, 513, 64), (12, 13, 513, 128)])
+def test_float32_calls_with_many_items(B, H, T, D, deterministic):
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import flash_attention
+    q, k, v, do = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.float32, seed=T + D))
+    lens = torch.tensor([(T, 0, 0, 1, T // 2, T - 1)[b % 6] for b in range(B)], dtype=torch.int32, device=DEV)
+    qg, kg, vg = (x.detach().requires_grad_() for x in (q, k, v))
+    o = flash_attention(qg, kg, vg, lens=lens, causal=True, deterministic=deterministic)
+    got = (o.detach(), *torch.autograd.grad(o, (qg, kg, vg), do))
+    with torch.no_grad():   # no backward to come: no 16-bit O
+        assert torch.equal(flash_attention(q, k, v, lens=lens, causal=True), got[0])
+    heads = [0, 6, H - 1]
+    mask = ao.dense_mask(T, None, None, None, lens.cpu().numpy(), causal=True, B=B)
+    ro, _, *rg = ao.attention_fwd_bwd(*(x[:, heads].half().float().cpu() for x in (q, k, v, do)), mask)
+    for x, ref in zip(got, (ro, *rg)):
+        x = x[:, heads].cpu()
+        for b in range(B):   # the bound of test_float32_results_are_not_rounded_to_16_bits, sequence by sequence
+            assert float((x[b] - ref[b]).norm()) <= 4 * 2.0**-11 * float(ref[b].norm()) + D * 2.0**-22
