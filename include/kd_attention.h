@@ -16,7 +16,8 @@
  *  - Device-side problems (a bounded wait that ran out, an unsupported span_id value) are
  *    reported through the 32-bit status word at plan offset `off_status`; it stays 0 on success.
  *  - Tensors are (B, H, T, D) with arbitrary element strides for b, h and t and unit stride
- *    along D; base pointers and the byte strides must be multiples of 16.
+ *    along D; base pointers and the byte strides must be multiples of 16. Outputs and scratch of kd_attn_* share no
+ *    memory with inputs or one another: the kernels of a backward overlap.
  *  - dtype: KD_F16 or KD_BF16; D: a multiple of 16 from 16 to 128 (the reference accepts 16, 32, 64, 128 and
  *    256, original_kernel.py:1720). Head dims below 64 run on the 64-wide kernels and those from 80 to 112 on
  *    the 128-wide ones: TMA fills the missing tile columns with zeros, which changes no product.
@@ -123,7 +124,8 @@ typedef struct kd_attn_params {
                          with fp32 atomics (dQ then differs in the last bits from run to run). With
                          KD_BWD_FUSED, bwd_phases 1 runs the delta kernel alone and 2 the fused kernel. */
   float* dq_acc;      /* KD_BWD_FUSED: (B,H,T,W) contiguous fp32 scratch, W = 64 for D <= 64 and 128 above
-                         (kd_workspace_bytes_fused gives its size); the library zeroes it itself. Ignored otherwise. */
+                         (kd_workspace_bytes_fused gives its size); the library zeroes what it reads of it. Columns at or
+                         beyond D are unspecified after the call. Ignored otherwise. */
   int32_t heads_per_cta; /* >= 0. Ignored, kept for the layout: every kernel takes its work items, tiles of single heads, dynamically. */
   int32_t plan_ready;    /* 1: an earlier launch on the same stream has used this plan, which lets kd_attn_fwd look up its
                          work before the kernel ahead of it on the stream has finished. 0 is always correct. */

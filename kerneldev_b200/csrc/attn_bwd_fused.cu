@@ -185,9 +185,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // With the delta kernel directly before this one, everything but delta and the zeroed dQ scratch was complete before that
-  // kernel let this one start: the plan, Q, K, V, dO and LSE may be read, and dK and dV written, before the wait (plain reads
-  // past L1, which the start of a kernel that overlaps another need not have cleaned).
+  // With the delta kernel directly before this one, everything that it does not write itself was complete before it let this one start:
+  // the plan, Q, K, V and LSE may be read, and dK and dV written, before the wait (plain reads past L1, which the start of a kernel that
+  // overlaps another need not have cleaned). Not so delta, the zeros of the dQ scratch or of a float32 dQ, and dO, which in a float32 call
+  // the delta kernel rounds to 16 bits.
   if (!fa.after_delta) pdl_wait();
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
@@ -316,7 +317,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         if (k == 0) {
           if (lane == 0) load_tile(&tmV, sV, C::B_VFULL, kt, h, b);
-          pdl_wait();   // delta is read from here on
+          pdl_wait();   // delta and dO are read from here on
           pdl_launch_dependents();
         }
         ++k;
@@ -368,7 +369,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           ++q_tiles;
           if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
           if (!(ok = wait(C::B_DOEMPTY + os, do_parity, W_U_DOEMPTY))) break;
-          if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, qt, h, b);
+          if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, qt, h, b);   // (behind pdl_wait())
           ++do_tiles;
           if (++os == C::OS) { os = 0; do_parity ^= 1u; }
         }

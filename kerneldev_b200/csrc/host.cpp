@@ -808,7 +808,8 @@ Tensor cocktail_scores(const Tensor& x_, const Tensor& tokens_, int64_t tok_span
     int32_t S = 0;   // the width of the scores has to be known here: the one wait for the device
     if (B > 0 && n_tokens > 0) {
       // The counts arrive while the kernel still writes the markers. A wait for the stream would add the rest of the kernel, its end and
-      // the wake-up (16 x 4096 x 1024, forward and backward 72.2 -> 61 us); it follows only where they take long, or never come.
+      // the wake-up (16 x 4096 x 1024, forward and backward on an idle stream 72.2 -> 61 us). It follows only where they never come, or take
+      // long because of work queued ahead: such a call gains nothing, and its thread has turned for 200 us where the wait turns as well.
       volatile int32_t* words = counts.data_ptr<int32_t>();
       const auto give_up = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
       int64_t b = 0;
