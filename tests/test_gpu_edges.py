@@ -276,9 +276,10 @@ def test_forward_output_boxes(B, H, T, D, layout):
 
 
 @pytest.mark.parametrize("B,H,T,D,dtype", [(1, 4, 300, 64, torch.bfloat16), (1, 8, 173, 128, torch.float16), (1, 3, 513, 64, torch.float32), (2, 2, 257, 128, torch.float32)])
-def test_deterministic_backward_behind_one_another(B, H, T, D, dtype):
+def test_deterministic_backward_behind_one_another(monkeypatch, B, H, T, D, dtype):
     """The dK/dV kernel starts beside the end of the dQ kernel and reads what the delta kernel of the same call has written. Calls without
     a pause between them, whose scratch is the memory of earlier calls with other gradients, give the bits of calls one by one."""
+    monkeypatch.setenv("KD_CHECK_STATUS", "0")   # a check waits for the device
     from tests.helpers import assert_close, rand_inputs
     from kerneldev_b200 import flash_attention
     q, k, v, _ = (x.to(DEV).requires_grad_() for x in rand_inputs(B, H, T, D, dtype, seed=T + D))
@@ -347,3 +348,39 @@ def test_float32_calls_with_many_items(B, H, T, D, deterministic):
         x = x[:, heads].cpu()
         for b in range(B):   # the bound of test_float32_results_are_not_rounded_to_16_bits, sequence by sequence
             assert float((x[b] - ref[b]).norm()) <= 4 * 2.0**-11 * float(ref[b].norm()) + D * 2.0**-22
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("B,H,T,D,dtype", [(1, 4, 300, 64, torch.bfloat16), (2, 40, 257, 128, torch.float16), (1, 3, 300, 64, torch.float32), (2, 40, 257, 128, torch.float32)])
+def test_captured_forward_and_backward(monkeypatch, B, H, T, D, dtype, deterministic):
+    """A graph of a forward and backward, replayed without a pause on inputs that change in place, gives what the calls give."""
+    monkeypatch.setenv("KD_CHECK_STATUS", "0")   # a check waits for the device
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import flash_attention
+    sets = [[x.to(DEV) for x in rand_inputs(B, H, T, D, dtype, seed=T + D + i)] for i in range(4)]
+    q, k, v, do = (x.clone() for x in sets[0])
+    lens = torch.tensor([T] + [T // 2] * (B - 1), dtype=torch.int32, device=DEV)
+
+    def call(q, k, v, do):   # the node by hand: the engine's own streams have no place in a capture
+        o = flash_attention(*(x.detach().requires_grad_() for x in (q, k, v)), lens=lens, deterministic=deterministic)
+        return (o.detach(), *o.grad_fn(do))
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call(q, k, v, do)   # builds the plan
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            outs = call(q, k, v, do)
+        replayed = []
+        for xs in sets:
+            for x, y in zip((q, k, v, do), xs):
+                x.copy_(y)
+            graph.replay()
+            replayed.append([x.clone() for x in outs])
+        torch.cuda.synchronize()
+        for xs, got in zip(sets, replayed):
+            for x, y in zip(got, call(*xs)):
+                # fused dQ: fp32 sums in no fixed order, then a rounding to the type (2^-8 covers bf16's, of any element)
+                assert torch.equal(x, y) or (not deterministic and float((x - y).norm()) <= 2.0**-8 * float(y.norm()))
