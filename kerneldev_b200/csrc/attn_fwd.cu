@@ -667,7 +667,7 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   if (p.D > 64) return launch_attn_fwd_wide(n_items, a, p.dtype, tmQ, tmK, tmV, stream);
   // O through TMA stores: a thread's 16-byte stores to its own row are 32 lines an instruction, 1,240 cycles of an item's end with sixteen
   // warps at it (short bursts: hierarchical 16 x 16 x 4096 x 64 416 -> 406 us, 8 x 16 x 2048 x 64 66.3 -> 64.5; causal 113.9 -> 111.1; no mask
-  // 187.6 -> 182.3; long runs of 8 x 16 x 4096 x 64 are level, under the power limit). Not where a CTA has one item: its rows leave as soon either way, and the map costs the host time. (Nor for strides
+  // 187.6 -> 182.3; passes of 8 x 16 x 4096 x 64 one after the other 234 -> 229). Not where a CTA has one item: its rows leave as soon either way, and the map costs the host time. (Nor for strides
   // that a map cannot have: 0 or below.)
   CUtensorMap tmO = tmQ;
   a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, nullptr, 64) == 0 ? 1 : 0;
