@@ -447,30 +447,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int row = wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float c = a.scale_log2;
-    const int tbw = 2 * i + c0;      // first word of this thread's chunks in the 128-bit class masks of a key tile
+    const int first_word = 2 * i + c0;   // of this thread's chunks among the four of a key tile
     bool ok = true;
 
     int4 it = make_int4(0, 0, 0, 0);   // the item in hand; behind its last unit the next one
-    // key descriptors of PARTIAL tiles are fetched one entry ahead into registers
-    uint32_t kd_pre[CPT];
-    uint32_t tb_pre[3][CPT];   // key-side class masks of the chunks: is_prefix, context, in_span
+    // The visibility words of a PARTIAL tile (of the plan; bit j: key j of a chunk) are fetched one entry ahead into registers.
+    uint32_t mk_next[CPT];
+    const uint32_t* words = a.words;   // of this thread's query and chunks in the item's query tile
 #pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) { kd_pre[cc] = 0u; tb_pre[0][cc] = 0u; tb_pre[1][cc] = 0u; tb_pre[2][cc] = 0u; }
-    auto prefetch_kd = [&](uint32_t entry) {
-      if ((entry >> 8) == KD_TILE_PARTIAL) {
-        const uint32_t ktile = entry & 0xFFu;
-        const uint32_t* tbp = a.tilebits + ((size_t)it.x * a.NT + ktile) * 32;
+    for (int cc = 0; cc < CPT; ++cc) mk_next[cc] = 0u;
+    auto fetch_words = [&](uint32_t entry) {
+      if ((entry >> 8) != KD_TILE_PARTIAL) return;
+      const uint32_t* src = words + (entry & 0xFFu) * static_cast<uint32_t>(KD_WORDS);
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-          kd_pre[cc] = __ldcg(a.desc + (size_t)it.x * a.Tpad + (size_t)ktile * KD_TILE + i * 64 + (c0 + cc) * 32 + lane);
-          tb_pre[0][cc] = __ldcg(tbp + 4 * TB_PRE + tbw + cc);
-          tb_pre[1][cc] = __ldcg(tbp + 4 * TB_CTX + tbw + cc);
-          tb_pre[2][cc] = __ldcg(tbp + 4 * TB_INS + tbw + cc);
-        }
-      }
+      for (int cc = 0; cc < CPT; ++cc) mk_next[cc] = __ldcg(src + cc * KD_TILE);
     };
-    // The next item's header, query descriptor, first entry and scalars are fetched before the epilogue.
-    uint32_t ent_next = 0u, qd = 0u;
+    // The next item's header, first entry and scalars are fetched before the epilogue.
+    uint32_t ent_next = 0u;
     float delta = 0.f, lse = 0.f;
     const uint16_t* list = lists;
     auto open_item = [&](int k) -> bool {
@@ -478,13 +471,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_Q_ITEMFULL))) return false;
       it = uniform(sh.items[slot]);
       if (it.w < 0) return false;
-      qd = __ldcg(a.desc + (size_t)it.x * a.Tpad + it.z * KD_TILE + row);
       list = lists + slot * 128;
+      words = a.words + ((size_t)it.x * a.NT + it.z) * a.NT * KD_WORDS + first_word * KD_TILE + row;
       if (it.w > 0) {
         ent_next = list[0];
-        prefetch_kd(ent_next);
+        fetch_words(ent_next);
         const int qi = it.z * KD_TILE + row;
-        const size_t at = ((size_t)it.x * a.H + it.y) * a.T + min(qi, a.T - 1);   // (rows beyond the last have descriptor 0: hidden)
+        const size_t at = ((size_t)it.x * a.H + it.y) * a.T + min(qi, a.T - 1);   // (rows beyond the last see nothing)
         delta = __ldcg(a.delta + at);
         lse = __ldcg(a.lse + at);
       }
@@ -508,33 +501,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int e = 0; e < na; ++e) {
         const uint32_t ent = ent_next;
         const uint32_t cls = ent >> 8;
-        uint32_t mk[CPT];   // visibility of the chunks' keys for this query row
+        uint32_t mk[CPT];   // visibility of the chunks' keys for this query row, where the tile is PARTIAL
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) mk[cc] = 0xFFFFFFFFu;
-        if (cls == KD_TILE_PARTIAL) {
-          const int j0 = (ent & 0xFF) * KD_TILE + i * 64 + c0 * 32;  // first key handled here
-          query_row_mask<CPT>(qd, qi, j0, tb_pre[0], tb_pre[1], tb_pre[2], mk);
-          uint32_t any_ins = 0u;
-#pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) any_ins |= tb_pre[2][cc];
-          // "same span": one round per distinct span among the warp's 32 queries; a ballot over the lanes' key descriptors
-          // (lane L holds keys L, 32 + L, ... of the chunks) gives the keys of that span, 32 at a time
-          const uint32_t my_key = span_key_of_query(qd);
-          uint32_t todo = (any_ins != 0u) ? __ballot_sync(0xffffffffu, (qd & TD_SIDPOS) != 0u) : 0u;
-          while (todo != 0u) {
-            const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-            const bool mine = (my_key == kq);
-#pragma unroll
-            for (int cc = 0; cc < CPT; ++cc) {
-              const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd_pre[cc]) != 0u);
-              if (mine) mk[cc] |= hit;
-            }
-            todo &= ~__ballot_sync(0xffffffffu, mine);
-          }
-        }
+        for (int cc = 0; cc < CPT; ++cc) mk[cc] = mk_next[cc];
         if (e + 1 < na) {
           ent_next = list[e + 1];
-          prefetch_kd(ent_next);
+          fetch_words(ent_next);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
         ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_Q_SFULL);
@@ -793,54 +765,39 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     uint32_t* st_buf = sStage + (size_t)(warp - 4) * C::STAGE_WORDS;  // [QW lse][QW delta]
     const float c = a.scale_log2;
-    const int tbw = 2 * i + c0;      // first word of this thread's chunks in the 128-bit class masks of a query tile
     bool ok = true;
 
     int4 it = make_int4(0, 0, 0, 0);   // the item in hand; behind its last unit the next one
-    // LSE, delta and the descriptors of the next unit's queries are fetched one unit ahead
-    // into registers and handed to the warp through its shared-memory staging buffer
+    // LSE and delta of the next unit's queries are fetched one unit ahead into registers and handed to the warp through its shared-memory
+    // staging buffer, and with them, for a PARTIAL tile, the plan's words of these queries for the warp's 32 keys
     float pre_lse[CPT], pre_delta[CPT];
-    uint32_t pre_desc[CPT];
-    // query-side class masks of the next unit: sees-prefix, sees-context, sees-in_span, context, same-span armed
-    uint32_t tb_pre[5][CPT];
+    uint32_t pre_words[CPT];
 #pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) {
-      pre_lse[cc] = 0.f; pre_delta[cc] = 0.f; pre_desc[cc] = 0u;
-#pragma unroll
-      for (int j = 0; j < 5; ++j) tb_pre[j][cc] = 0u;
-    }
+    for (int cc = 0; cc < CPT; ++cc) { pre_lse[cc] = 0.f; pre_delta[cc] = 0.f; pre_words[cc] = 0u; }
     auto prefetch = [&](uint32_t entry, int h) {
       if ((entry >> 8) == KD_TILE_PARTIAL) {
-        const uint32_t* tbp = a.tilebits + ((size_t)it.x * a.NT + (entry & 0xFFu)) * 32;
+        const uint32_t* src = a.words + (((size_t)it.x * a.NT + (entry & 0xFFu)) * a.NT + it.z) * KD_WORDS + wq * KD_TILE + i * 64 + c0 * 32 + lane;
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-          tb_pre[0][cc] = __ldcg(tbp + 4 * TB_SEES_PRE + tbw + cc);
-          tb_pre[1][cc] = __ldcg(tbp + 4 * TB_SEES_CTX + tbw + cc);
-          tb_pre[2][cc] = __ldcg(tbp + 4 * TB_SEES_INS + tbw + cc);
-          tb_pre[3][cc] = __ldcg(tbp + 4 * TB_CTX + tbw + cc);
-          tb_pre[4][cc] = __ldcg(tbp + 4 * TB_SIDPOS + tbw + cc);
-        }
+        for (int cc = 0; cc < CPT; ++cc) pre_words[cc] = __ldcg(src + cc * 32);
       }
-      // a query at or beyond the sequence length reads the last row's scalars: its descriptor is 0,
-      // so the tile is PARTIAL and the mask removes it
+      // a query at or beyond the sequence length reads the last row's scalars: it sees nothing, so the tile is PARTIAL and the mask
+      // removes it
 #pragma unroll
       for (int cc = 0; cc < CPT; ++cc) {
         const int q = (entry & 0xFF) * KD_TILE + i * 64 + (c0 + cc) * 32 + lane;
         const size_t r = ((size_t)it.x * a.H + h) * a.T + min(q, a.T - 1);
         pre_lse[cc] = __ldcg(a.lse + r);   // negated where it is used: a negation here would wait for the load
         pre_delta[cc] = __ldcg(a.delta + r);
-        pre_desc[cc] = __ldcg(a.desc + (size_t)it.x * a.Tpad + q);
       }
     };
-    // The next item's header, key descriptor and first unit's scalars are fetched before the epilogue.
-    uint32_t ent_next = 0u, kdesc = 0u;
+    // The next item's header and first unit's scalars are fetched before the epilogue.
+    uint32_t ent_next = 0u;
     const uint16_t* list = lists;
     auto open_item = [&](int k) -> bool {
       const int slot = k % C::NITEM;
       if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_K_ITEMFULL))) return false;
       it = uniform(sh.items[slot]);
       if (it.w < 0) return false;
-      kdesc = __ldcg(a.desc + (size_t)it.x * a.Tpad + it.z * KD_TILE + row);
       list = lists + slot * 128;
       if (it.w > 0) {
         ent_next = list[0];
@@ -870,30 +827,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           st_buf[QW + cc * 32 + lane] = __float_as_uint(pre_delta[cc]);
         }
         __syncwarp();
-        uint32_t mk[CPT];   // visibility of this key for the chunks' queries
+        uint32_t mk[CPT];
 #pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) mk[cc] = 0xFFFFFFFFu;
-        if (cls == KD_TILE_PARTIAL) {
-          const int i0 = (ent & 0xFF) * KD_TILE + i * 64 + c0 * 32;  // first query handled here
-          key_row_mask<CPT>(kdesc, now.z * KD_TILE + row, i0, tb_pre[0], tb_pre[1], tb_pre[2], tb_pre[3], mk);
-          uint32_t any_armed = 0u;
-#pragma unroll
-          for (int cc = 0; cc < CPT; ++cc) any_armed |= tb_pre[4][cc];
-          // "same span": one round per distinct span among the warp's 32 keys; a ballot over the lanes' query descriptors
-          // (lane L holds queries L, 32 + L, ... of the chunks) gives the queries of that span, 32 at a time
-          const uint32_t my_key = span_key_of_key(kdesc);
-          uint32_t todo = (any_armed != 0u) ? __ballot_sync(0xffffffffu, (kdesc & TD_INS) != 0u) : 0u;
-          while (todo != 0u) {
-            const uint32_t kk = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-            const bool mine = (my_key == kk);
-#pragma unroll
-            for (int cc = 0; cc < CPT; ++cc) {
-              const uint32_t hit = __ballot_sync(0xffffffffu, span_match_query(kk, pre_desc[cc]) != 0u);
-              if (mine) mk[cc] |= hit;
-            }
-            todo &= ~__ballot_sync(0xffffffffu, mine);
-          }
-        }
+        for (int cc = 0; cc < CPT; ++cc) mk[cc] = pre_words[cc];
         if (e + 1 < n) {
           ent_next = list[e + 1];
           prefetch(ent_next, now.y);
@@ -910,6 +846,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           uint32_t rs[32], rp[32];
           tmem_ld32(tS + cc * 32, rs);
           tmem_ld32(tP + cc * 32, rp);
+          if (cls == KD_TILE_PARTIAL) mk[cc] = transpose_bits(mk[cc], lane);   // this key's visibility for the chunk's queries, while the scores are on their way
           tmem_wait_ld();
           if (cls != KD_TILE_PARTIAL) {   // warp-uniform: the common case carries no mask code at all
 #pragma unroll
@@ -1041,8 +978,8 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.d_real = p.D;
   a.scale_log2 = scale_log2_of(p.sm_scale);
   a.sm_scale = p.sm_scale;
-  a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
-  a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order; a.tilebits = pv.tilebits;
+  a.words = pv.words; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
+  a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.d_o = p.d_o.ptr; a.do_sb = p.d_o.stride_b; a.do_sh = p.d_o.stride_h; a.do_st = p.d_o.stride_t;
   a.lse = p.lse; a.delta = p.delta;

@@ -11,8 +11,7 @@ struct BwdArgs {
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
-  const uint32_t* desc;
-  const uint32_t* tilebits;   // [B][NT][8][4] class masks of every 128-token tile
+  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles
   const int32_t* fwd_cnt;
   const uint16_t* fwd_list;
   const int32_t* bwd_cnt;
@@ -38,6 +37,18 @@ struct BwdArgs {
   void* dv;
   int64_t dv_sb, dv_sh, dv_st;
 };
+
+// 32 x 32 bits across a warp: lane l gives word l and gets bit l of every lane's word, lane 0's in bit 0
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
+  constexpr uint32_t low[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+    const int d = 16 >> i;
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, d);
+    x = (lane & d) ? ((x & ~low[i]) | ((y & ~low[i]) >> d)) : ((x & low[i]) | ((y & low[i]) << d));
+  }
+  return x;
+}
 
 // Fused backward (attn_bwd_fused.cu): one key-tile-major kernel that forms S and dP once per tile, accumulates dK and
 // dV in TMEM and adds its dQ partials to a.dq_acc, then a conversion kernel.

@@ -48,8 +48,8 @@
 // chunk by decreasing list length, so that the CTAs on the machine at one time add to dQ lines that stay in L2 and
 // the last items are short.
 //
-// 512 threads: warp 0 takes items and streams Q and dO (lane 0 issues the TMA loads; all lanes copy LSE, delta, token
-// descriptors and mask words of the tile's 128 queries to shared memory); warps 1-3 as above; warps 4-11 are two compute
+// 512 threads: warp 0 takes items and streams Q and dO (lane 0 issues the TMA loads; all lanes copy LSE, delta
+// and a PARTIAL tile's visibility words to shared memory); warps 1-3 as above; warps 4-11 are two compute
 // warpgroups (64 query columns each); warps 12-15 move finished dQ tiles from TMEM to the scratch (each warp stages and
 // reduces its own 32 rows) and write dK and dV of finished items.
 //
@@ -84,11 +84,9 @@ struct FusedCfg {
   static constexpr int SMEM_DO = SMEM_Q + QS * TILE_BYTES;
   static constexpr int SMEM_DS = SMEM_DO + OS * TILE_BYTES;   // dS^T: two blocks [128 keys][64 queries]
   static constexpr int SMEM_STG = SMEM_DS + 2 * 16384;        // dQ staging: per dQ warp two boxes [32 rows][32 floats]
-  // per Q stage: LSE and delta of the 128 queries, the 32 mask words of the query tile, its list entry (4 words with
-  // padding); HD = 64 also the queries' token descriptors (HD = 128 has no room: its compute warps fetch them)
-  static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + 32, SIDE_DESC = SIDE_ENT + 4;
-  static constexpr int SIDE_KDESC = SIDE_DESC + KD_TILE;   // and the keys'
-  static constexpr int SIDE_WORDS = (HD == 64) ? SIDE_KDESC + KD_TILE : SIDE_DESC;
+  // per Q stage: LSE and delta of the 128 queries; HD = 64: the visibility words of a PARTIAL tile, [32 keys][query] (HD = 128 has no room: its
+  // compute warps fetch them); the tile's list entry (4 words with padding)
+  static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + (HD == 64 ? static_cast<int>(KD_WORDS) : 0), SIDE_WORDS = SIDE_ENT + 4;
   static constexpr int SMEM_SIDE = SMEM_STG + 4 * 2 * 4096;
   static constexpr int NITEM = 4;                    // ring of item headers
   static constexpr int SMEM_ITEM = SMEM_SIDE + QS * SIDE_WORDS * 4;   // NITEM x {batch, head, key tile | first entry << 16, entries}
@@ -342,12 +340,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (!(ok = wait(C::B_QEMPTY + qs, q_parity, W_U_QEMPTY))) break;
           const uint32_t side = s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4);
           if (lane == 0) {
-            st_shared_u32(side + C::SIDE_ENT * 4, this_ent | (HD == 64 ? static_cast<uint32_t>(kt) << 16 : 0u));   // published by the arrival that goes with the load
+            st_shared_u32(side + C::SIDE_ENT * 4, this_ent);   // published by the arrival that goes with the load
             load_tile(&tmQ, sQ + qs * TILE, C::B_QFULL + qs, qt, h, b);
           }
-          // the scalars of four queries and one mask word per lane, copied asynchronously: the barrier counts the lanes' copies
-          // (a query at or beyond the sequence length takes the last row's scalars: its descriptor is 0, so the tile is PARTIAL
-          // and the mask removes it)
+          // the scalars of four queries per lane, and a PARTIAL tile's words, copied asynchronously: the barrier counts the lanes' copies
+          // (a query at or beyond the sequence length takes the last row's scalars: it sees nothing, so the tile is PARTIAL and the
+          // mask removes it)
           const int q = qt * KD_TILE + 4 * lane;
           if (aligned && q + 3 < a.T) {
             cp_async16(side + 16 * lane, a.lse + row + q);
@@ -360,10 +358,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               cp_async4(side + KD_TILE * 4 + 16 * lane + 4 * j, a.delta + r);
             }
           }
-          cp_async4(side + (C::SIDE_BITS + lane) * 4, a.tilebits + ((size_t)b * a.NT + qt) * 32 + lane);
-          if constexpr (HD == 64) {   // padded to whole tiles
-            cp_async16(side + C::SIDE_DESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + q);
-            cp_async16(side + C::SIDE_KDESC * 4 + 16 * lane, a.desc + (size_t)b * a.Tpad + kt * KD_TILE + 4 * lane);
+          if (HD == 64 && (this_ent >> 8) == KD_TILE_PARTIAL) {
+            const uint32_t* src = a.words + (((size_t)b * a.NT + qt) * a.NT + kt) * KD_WORDS + 4 * lane;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) cp_async16(side + (C::SIDE_BITS + w * KD_TILE) * 4 + 16 * lane, src + w * KD_TILE);
           }
           cp_async_mbar_arrive(bar(C::B_QFULL + qs));
           ++q_tiles;
@@ -656,31 +654,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const uint32_t ds_sw = static_cast<uint32_t>((lane >> 4) ^ (lane & 7)) << 4;
     bool ok = true;
     int t = 0, qs = 0;
-    uint32_t q_parity = 0u;   // of the Q stage's "full" phase
     int4 it;
-    // visibility of this lane's key for the warpgroup's 64 queries
-    auto mask_words = [&](const float* side, uint32_t kdesc, int kj, int i0, uint32_t qd0, uint32_t qd1, uint32_t (&mk)[2]) {
-      const uint32_t* tb = reinterpret_cast<const uint32_t*>(side) + C::SIDE_BITS + 2 * w;   // words 2 w, 2 w + 1 of every mask
-      key_row_mask<2>(kdesc, kj, i0, tb + 4 * TB_SEES_PRE, tb + 4 * TB_SEES_CTX, tb + 4 * TB_SEES_INS, tb + 4 * TB_CTX, mk);
-      if ((tb[4 * TB_SIDPOS] | tb[4 * TB_SIDPOS + 1]) != 0u) {
-        // "same span": one round per distinct span among the warp's 32 keys, each a ballot over the queries
-        const uint32_t my_key = span_key_of_key(kdesc);
-        uint32_t todo = __ballot_sync(0xffffffffu, (kdesc & TD_INS) != 0u);
-        while (todo != 0u) {
-          const uint32_t kk = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-          const uint32_t hit0 = __ballot_sync(0xffffffffu, span_match_query(kk, qd0) != 0u);
-          const uint32_t hit1 = __ballot_sync(0xffffffffu, span_match_query(kk, qd1) != 0u);
-          const bool mine = (my_key == kk);
-          if (mine) { mk[0] |= hit0; mk[1] |= hit1; }
-          todo &= ~__ballot_sync(0xffffffffu, mine);
-        }
-      }
-    };
     // zeroes the hidden ones among this thread's 32 values of half hf
     auto apply_mask = [&](uint32_t (&p)[32], const uint32_t (&mk)[2], int hf) {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int src = hf * 16 + r * 8 + (lane >> 2);   // the lane that formed this key's mask
+        const int src = hf * 16 + r * 8 + (lane >> 2);   // the lane that holds this key's mask
         const uint32_t m0 = __shfl_sync(0xffffffffu, mk[0], src) >> (2 * (lane & 3));
         const uint32_t m1 = __shfl_sync(0xffffffffu, mk[1], src) >> (2 * (lane & 3));
         // A byte's top bit spread over a word by one permute, for the two queries of a byte: two instructions a value, where a test
@@ -771,12 +750,25 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const uint32_t ent = side_u[C::SIDE_ENT];
         more = ent != C::ENT_END;
         if (more && ((ent >> 8) & 0xFFu) == KD_TILE_PARTIAL) {
-          const uint32_t kdesc = side_u[C::SIDE_KDESC + wq * 32 + lane];   // of the key whose mask words this lane forms
-          const int kj = static_cast<int>(ent >> 16) * KD_TILE + wq * 32 + lane;
-          uint32_t mk[2];
-          mask_words(side, kdesc, kj, (ent & 0xFF) * KD_TILE + w * 64, side_u[C::SIDE_DESC + w * 64 + lane], side_u[C::SIDE_DESC + w * 64 + 32 + lane], mk);
-          apply_mask(p[0], mk, 0);
-          apply_mask(p[1], mk, 1);
+          // The words of this thread's queries, one pair after the other: a shift brings this thread's keys to the top bits of the
+          // bytes, and a byte's top bit spreads over a word by one permute. (Formed here from class masks and descriptors, key by
+          // key, before the plan held them: hierarchical 16 x 16 x 4096 x 64 backward 1072 -> 1025 us, 8 x 16 x 2048 x 64 167 -> 162,
+          // causal 8 x 16 x 1000 x 64 97.4 -> 94.5.)
+          const uint32_t* words = side_u + C::SIDE_BITS + wq * KD_TILE + qcol;
+          const int up = 7 - (lane >> 2);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint2 x = *reinterpret_cast<const uint2*>(words + 8 * j);
+            const uint32_t even = x.x << up, odd = x.y << up;
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const uint32_t sel = 0x8888u + 0x1111u * (2 * hf + r);
+                p[hf][4 * j + 2 * r] &= prmt_sign(even, sel);
+                p[hf][4 * j + 2 * r + 1] &= prmt_sign(odd, sel);
+              }
+          }
         }
         // (in the last iteration too: it must not complete a phase of PFULL ahead of the dV issuer)
         if (!__all_sync(0xffffffffu, out_ready)) {
@@ -808,32 +800,31 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     } else {
     for (int k = 0; ok && next_item(k, it); ++k) {
       const int b = it.x, kt = it.z & 0xFFFF, n = it.w;
-      const int kj = kt * KD_TILE + wq * 32 + lane;   // the key whose mask words this lane forms
-      const uint32_t kdesc = __ldcg(a.desc + (size_t)b * a.Tpad + kj);
       const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
       uint32_t ent_next = static_cast<uint32_t>(it.z) >> 16;
       for (int e = 0; e < n; ++e, ++t) {
         const uint32_t ent = ent_next;
         if (e + 1 < n) ent_next = __ldcg(list + e + 1);
         const bool partial = (ent >> 8) == KD_TILE_PARTIAL;
-        const int i0 = (ent & 0xFF) * KD_TILE + w * 64;
-        uint32_t qd0 = 0u, qd1 = 0u;
-        if (partial) {   // query descriptors for the same-span ballots, requested ahead of the wait
-          qd0 = __ldcg(a.desc + (size_t)b * a.Tpad + i0 + lane);
-          qd1 = __ldcg(a.desc + (size_t)b * a.Tpad + i0 + 32 + lane);
+        uint32_t mk[2] = {0u, 0u};   // of a PARTIAL tile: the words of queries 64 w + lane and + 32 for the warp's keys, requested ahead of the wait
+        if (partial) {
+          const uint32_t* src = a.words + (((size_t)b * a.NT + (ent & 0xFF)) * a.NT + kt) * KD_WORDS + wq * KD_TILE + w * 64 + lane;
+          mk[0] = __ldcg(src);
+          mk[1] = __ldcg(src + 32);
         }
-        // LSE, delta and mask words of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here
+        // LSE and delta of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here
         const float* side = sSide + qs * C::SIDE_WORDS;
         bool masked = false;
-        uint32_t mk[2] = {0u, 0u};
-        if (partial) {   // before the wait for the scores, from what came with the Q tile (many a block of such a tile is visible as a whole)
-          if (!(ok = wait(C::B_QFULL + qs, q_parity, W_U_QFULL))) break;
-          mask_words(side, kdesc, kj, i0, qd0, qd1, mk);
+        if (partial) {   // before the wait for the scores: a word for each key (many a block of such a tile is visible as a whole)
           masked = __any_sync(0xffffffffu, (mk[0] & mk[1]) != 0xFFFFFFFFu);
+          if (masked) {
+            mk[0] = transpose_bits(mk[0], lane);
+            mk[1] = transpose_bits(mk[1], lane);
+          }
         }
         if (!(ok = wait(C::B_SFULL, t & 1, W_U_SFULL))) break;
         tc_fence_after_sync();
-        if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
+        if (++qs == C::QS) qs = 0;
         uint32_t s[2][32];
         tmem_ld16x256_x8(tS, s[0]);
         uint64_t col[8];

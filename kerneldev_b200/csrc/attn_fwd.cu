@@ -138,7 +138,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after_sync();
   // A plan that an earlier launch on this stream has used was complete when the kernel before this one let it start (a kernel
-  // lets its successor start only when its own predecessors are complete): its lists and descriptors may be read before the
+  // lets its successor start only when its own predecessors are complete): its lists and words may be read before the
   // wait, which hides three dependent look-ups under the predecessor (in a stack of layers, 2 us of each kernel's 9 at T = 173).
   // They are read past L1, which the start of a kernel that overlaps another need not have cleaned.
   if (!a.plan_ready) pdl_wait();
@@ -369,11 +369,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const int c = pv_seen - back;
       return c < 0 || wait(C::B_PVDONE + 2 * i + (c & 1), (c >> 1) & 1, W_F_PVDONE);
     };
-    // The next item's header, query descriptor and first unit are fetched before the epilogue of the item in hand, which
+    // The next item's header and first unit are fetched before the epilogue of the item in hand, which
     // hides their latency (they took 2,000 cycles of an item, of 35,000 for one of nine tiles).
     int4 it = make_int4(0, 0, 0, 0);
     int n_next = 0, qi_next = 0, e = 0, buf_next = 0;
-    uint32_t qd_next = 0u, ent_next = 0u, fetched = 0u;   // fetched: entry e of the list, read one step ahead
+    uint32_t ent_next = 0u, fetched = 0u;   // fetched: entry e of the list, read one step ahead
     const uint16_t* list = sList;
     // this query tile's next unit, of which there is one: sets ent_next and, in buf_next, its buffer
     auto find_next = [&]() {
@@ -385,42 +385,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       buf_next = static_cast<int>(ent_next >> 12) + ((i == 1 && entry_class(ent_next, 0) != 0u) ? 1 : 0);
       if (buf_next >= C::NBUF) buf_next -= C::NBUF;
     };
-    // Key descriptors (lane L holds keys L, 32 + L, ...) and class masks of PARTIAL tiles are fetched one unit ahead
-    // into registers, so their global-memory latency overlaps the previous tile's softmax.
-    uint32_t kd_pre[NW];
-    uint32_t tb_pre[3][NW];   // key-side class masks of this thread's columns: is_prefix, context, in_span
+    // The visibility words of a PARTIAL tile (bit j: key j of 32) are fetched one unit ahead into registers, so that their latency overlaps
+    // the previous tile's softmax. They come with the plan: formed here, for every head anew, from class masks and descriptors they were
+    // half of what masking costs (us, before -> now: hierarchical 16 x 16 x 4096 x 64 397 -> 368, 8 x 16 x 2048 x 64 59.4 -> 54.4, causal
+    // 8 x 16 x 1000 x 64 38.0 -> 33.7, no mask 8 x 16 x 2048 x 64 level). Asked for behind the exchange of maxima; ahead of it or behind
+    // the exponentials +0.5-2.5 %.
+    uint32_t mk[NW] = {0u, 0u};
+    const uint32_t* words = a.words;   // of this thread's query in the item's query tile
+    auto fetch_words = [&](uint32_t ent) {
+      if (entry_class(ent, i) != KD_TILE_PARTIAL) return;
+      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-    for (int w = 0; w < NW; ++w) { kd_pre[w] = 0u; tb_pre[0][w] = 0u; tb_pre[1][w] = 0u; tb_pre[2][w] = 0u; }
-    auto prefetch_kd = [&](uint32_t ent) {
-      if (entry_class(ent, i) == KD_TILE_PARTIAL) {
-        const int kt = ent & 0xFF;
-        const uint32_t* src = a.desc + (size_t)it.x * a.Tpad + (size_t)kt * KD_TILE;
-        const uint2* tbp = reinterpret_cast<const uint2*>(a.tilebits + ((size_t)it.x * a.NT + kt) * 32);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) kd_pre[w] = __ldcg(src + half * CW + w * 32 + lane);
-        static_assert(NW == 2, "a class mask of half a tile is two words: one 8-byte load each");
-        constexpr int cls3[3] = {TB_PRE, TB_CTX, TB_INS};
-#pragma unroll
-        for (int k3 = 0; k3 < 3; ++k3) {
-          const uint2 m2 = __ldcg(tbp + cls3[k3] * 2 + half);
-          tb_pre[k3][0] = m2.x; tb_pre[k3][1] = m2.y;
-        }
-      }
+      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
     };
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
+      words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + half * NW * KD_TILE + row;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
       const int only = it.w >> 24;
       const bool mine = only == 0 || only == i + 1;
       qi_next = mine ? qtile * KD_TILE + row : INT_MAX;   // (written by the other item of the pair)
-      qd_next = mine && qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
       list = sList + (k % C::NITEM) * 128;
       e = 0;
       if (n_next > 0) {
         fetched = list[0];
         find_next();
-        prefetch_kd(ent_next);
+        fetch_words(ent_next);
       }
       return true;
     };
@@ -429,14 +420,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     pdl_wait();   // O and LSE are written from here on
     for (int k = 0; have; ++k) {
     const int b = it.x, h = it.y, n_own = n_next, qi = qi_next;   // qi: token index of this thread's query
-    const uint32_t qd = qd_next;
     float m = -INFINITY, l = 0.f;
     int nact = 0;
 #pragma unroll 1
     for (int u = 0; u < n_own; ++u) {
       const uint32_t ent = ent_next;
       const uint32_t cls = entry_class(ent, i);
-      const int kt = ent & 0xFF, sbuf = buf_next;
+      const int sbuf = buf_next;
       const uint32_t tS = lane_base + sbuf * 128 + half * CW;
       if (!(ok = wait(C::B_SFULL + 2 * sbuf + i, (sfull_par >> sbuf) & 1u, W_F_SFULL))) break;
       sfull_par ^= 1u << sbuf;
@@ -453,28 +443,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (u + 1 < n_own) find_next();   // while the scores are on their way
       tmem_wait_ld();
       if (cls == KD_TILE_PARTIAL) {
-        // The row's visibility mask comes from the tile's class masks with a few word-wide
-        // operations; only the "same span" term needs the individual key descriptors.
-        const int j0 = kt * KD_TILE + half * CW;
-        uint32_t mk[NW];
-        query_row_mask<NW>(qd, qi, j0, tb_pre[0], tb_pre[1], tb_pre[2], mk);
-        uint32_t any_ins = 0u;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) any_ins |= tb_pre[2][w];
-        // "same span": one round per distinct span among the warp's 32 queries; a ballot over the lanes' key descriptors
-        // gives the keys of that span, 32 at a time
-        const uint32_t my_key = span_key_of_query(qd);
-        uint32_t todo = (any_ins != 0u) ? __ballot_sync(0xffffffffu, (qd & TD_SIDPOS) != 0u) : 0u;
-        while (todo != 0u) {
-          const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-          const bool mine = (my_key == kq);
-#pragma unroll
-          for (int w = 0; w < NW; ++w) {
-            const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd_pre[w]) != 0u);
-            if (mine) mk[w] |= hit;
-          }
-          todo &= ~__ballot_sync(0xffffffffu, mine);
-        }
 #pragma unroll
         for (int w = 0; w < NW; ++w) {
           if (__all_sync(0xffffffffu, mk[w] == 0xFFFFFFFFu)) continue;   // all 32 keys visible to all 32 queries
@@ -483,7 +451,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             if ((mk[w] & (1u << j)) == 0u) sc[w * 32 + j] = -INFINITY;
         }
       }
-      if (u + 1 < n_own) prefetch_kd(ent_next);
       // four independent chains for the row maximum and for the row sum: a single chain of
       // dependent operations would be latency-bound
       float mx4[4] = {sc[0], sc[1], sc[2], sc[3]};
@@ -499,6 +466,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx_other;
       exchange(mx, mx_other);
+      if (u + 1 < n_own) fetch_words(ent_next);
       mx = fmaxf(mx, mx_other);
       // The running maximum is refreshed only when it would grow by more than 2^8 in the exponent (or is -inf: the difference is then
       // inf); until then the stale value is used consistently for P, l and O, which leaves the normalised result unchanged, skips
@@ -653,8 +621,8 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   // Q, K, V and O. (64 and 110 MB: no difference outside the noise)
   a.order_of = ItemOrder::make(p.B * p.H, L.NP << a.split, (double)p.T * p.D * 2 * 4, 64e6);
   a.plan_ready = p.plan_ready;
-  a.desc = pv.desc; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
-  a.order = pv.order; a.tilebits = pv.tilebits;
+  a.words = pv.words; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
+  a.order = pv.order;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.o32 = f32 ? static_cast<float*>(f32->o.ptr) : nullptr;
   if (f32) { a.o32_sb = f32->o.stride_b; a.o32_sh = f32->o.stride_h; a.o32_st = f32->o.stride_t; }

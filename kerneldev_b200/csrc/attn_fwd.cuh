@@ -10,8 +10,7 @@ struct FwdArgs {
   ItemOrder order_of;
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
-  const uint32_t* desc;
-  const uint32_t* tilebits;   // [B][NT][8][4] class masks of every 128-token tile
+  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles
   const int32_t* fwd_cnt;
   const uint16_t* fwd_list;
   const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length

@@ -258,54 +258,33 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int c = n_seen - back;
       return c < 0 || wait(C::B_PVDONE + 2 * i + (c & 1), (c >> 1) & 1, W_F_PVDONE);
     };
-    // The next item's header, query descriptor and first unit's mask are fetched before the epilogue of the item in hand, and for the first
+    // The next item's header and first unit's mask are fetched before the epilogue of the item in hand, and for the first
     // item before the wait for the kernel ahead, which hides their latency.
     int4 it = make_int4(0, 0, 0, 0);
     int n_next = 0, qi_next = 0;
-    uint32_t qd_next = 0u, ent_next = 0u;   // the query descriptor and the first (then: the next) unit's entry
+    uint32_t ent_next = 0u;   // the first (then: the next) unit's entry
     const uint16_t* list = sOwn;
-    // Visibility of the 128 keys of tile kt for this thread's query: a few word-wide operations on the tile's class masks, and for
-    // "same span" one round per distinct span among the warp's 32 queries, in which a ballot over the lanes' key descriptors (lane L
-    // holds keys L, 32 + L, ...) gives the keys of that span, 32 at a time.
-    auto row_mask = [&](int kt, uint32_t qd, int qi, uint32_t (&mk)[NW]) {
-      const uint32_t* src = a.desc + (size_t)it.x * a.Tpad + (size_t)kt * KD_TILE;
-      const uint4* tbp = reinterpret_cast<const uint4*>(a.tilebits + ((size_t)it.x * a.NT + kt) * 32);
-      uint32_t kd[NW], tb[3][NW];   // key-side class masks: is_prefix, context, in_span
+    // Visibility of the 128 keys of a PARTIAL tile for this thread's query, of the coming unit (from the plan, see attn_fwd.cu)
+    uint32_t mk[NW] = {0u, 0u, 0u, 0u};
+    const uint32_t* words = a.words;   // of this thread's query in the item's query tile
+    auto fetch_words = [&](uint32_t ent) {
+      if ((ent & 0x100u) == 0u) return;
+      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-      for (int w = 0; w < NW; ++w) kd[w] = __ldcg(src + w * 32 + lane);
-      constexpr int cls3[3] = {TB_PRE, TB_CTX, TB_INS};
-#pragma unroll
-      for (int k3 = 0; k3 < 3; ++k3) {
-        const uint4 m4 = __ldcg(tbp + cls3[k3]);
-        tb[k3][0] = m4.x; tb[k3][1] = m4.y; tb[k3][2] = m4.z; tb[k3][3] = m4.w;
-      }
-      query_row_mask<NW>(qd, qi, kt * KD_TILE, tb[0], tb[1], tb[2], mk);
-      const uint32_t my_key = span_key_of_query(qd);
-      uint32_t todo = (tb[2][0] | tb[2][1] | tb[2][2] | tb[2][3]) != 0u ? __ballot_sync(0xffffffffu, (qd & TD_SIDPOS) != 0u) : 0u;
-      while (todo != 0u) {
-        const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-        const bool mine = (my_key == kq);
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd[w]) != 0u);
-          if (mine) mk[w] |= hit;
-        }
-        todo &= ~__ballot_sync(0xffffffffu, mine);
-      }
+      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
     };
-    uint32_t mk[NW] = {0u, 0u, 0u, 0u};   // of the coming unit, where it is PARTIAL
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
+      words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + row;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
       const int only = it.w >> 24;
       const bool mine = only == 0 || only == i + 1;
       qi_next = mine ? qtile * KD_TILE + row : INT_MAX;   // (written by the other item of the pair)
-      qd_next = mine && qtile < a.NT ? __ldcg(a.desc + (size_t)it.x * a.Tpad + qi_next) : 0u;
       list = sOwn + (k % C::NITEM) * 256 + i * 128;
       if (n_next > 0) {
         ent_next = list[0];
-        if (ent_next & 0x100u) row_mask(ent_next & 0xFF, qd_next, qi_next, mk);
+        fetch_words(ent_next);
       }
       return true;
     };
@@ -314,7 +293,6 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     pdl_wait();   // O and LSE are written from here on
     for (int k = 0; have; ++k) {
       const int b = it.x, h = it.y, n_own = n_next, qi = qi_next;   // qi: token index of this thread's query
-      const uint32_t qd = qd_next;
       float m = -INFINITY, l = 0.f;
 #pragma unroll 1
       for (int u = 0; u < n_own; ++u) {
@@ -410,8 +388,7 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const uint64_t sum_pair = add_f32x2(sum2[0], sum2[1]);
         l += lo_f32x2(sum_pair) + hi_f32x2(sum_pair);
         ++n_seen;
-        // the mask of a PARTIAL tile is formed while its scores are: the tile's products take longer
-        if (u + 1 < n_own && (ent_next & 0x100u) != 0u) row_mask(ent_next & 0xFF, qd, qi, mk);
+        if (u + 1 < n_own) fetch_words(ent_next);   // while its scores are formed
       }
       if (!ok) break;
       item_done(k);

@@ -11,6 +11,10 @@
 
 namespace kd {
 
+// Visibility of a tile as bits: uint32 [4][128], bit k of word [w][q] = query q of the query tile sees key 32 w + k of the key tile. The last part of
+// a plan has room for every tile of a sequence, [B][query tile][key tile], and holds the PARTIAL ones'.
+constexpr size_t KD_WORDS = 4 * KD_TILE, KD_WORDS_BYTES = KD_WORDS * 4;
+
 // Typed pointers into a plan buffer (see kd_plan_layout for the contents).
 struct PlanView {
   int NT, NP, Tpad;
@@ -26,6 +30,7 @@ struct PlanView {
   uint32_t* stats;
   uint32_t* done;   // [B] CTAs of the classifier that have finished
   uint32_t* status;
+  uint32_t* words;
 };
 
 inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
@@ -46,6 +51,7 @@ inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
   v.stats = reinterpret_cast<uint32_t*>(base + L.off_stats);
   v.done = v.stats + 2 * (size_t)L.B;
   v.status = reinterpret_cast<uint32_t*>(base + L.off_status);
+  v.words = reinterpret_cast<uint32_t*>(base + L.total - (size_t)L.B * L.NT * L.NT * KD_WORDS_BYTES);
   return v;
 }
 

@@ -287,7 +287,9 @@ struct PlanKeyHash {
 
 class PlanCache {
  public:
-  static constexpr size_t kSize = 64;
+  // Plans kept: so many, and so many bytes of device memory (the visibility words of a plan are 16 bits for every 8 x 8 tokens and
+  // sequence: 2 MB at T = 4096), but never fewer than kLeast.
+  static constexpr size_t kSize = 64, kLeast = 4, kBytes = size_t(512) << 20;
   PlanPtr find(const PlanKey& key) {
     std::lock_guard<std::mutex> lock(m_);
     auto it = map_.find(key);
@@ -296,13 +298,15 @@ class PlanCache {
     return it->second->second;
   }
   void insert(const PlanKey& key, PlanPtr plan) {
-    PlanPtr evicted;   // destroyed after the lock is released
+    std::vector<PlanPtr> evicted;   // destroyed after the lock is released
     std::lock_guard<std::mutex> lock(m_);
     if (map_.count(key)) return;
+    bytes_ += plan->layout.total;
     order_.emplace_back(key, std::move(plan));
     map_[key] = std::prev(order_.end());
-    if (order_.size() > kSize) {
-      evicted = std::move(order_.front().second);
+    while (order_.size() > kSize || (bytes_ > kBytes && order_.size() > kLeast)) {
+      bytes_ -= order_.front().second->layout.total;
+      evicted.push_back(std::move(order_.front().second));
       map_.erase(order_.front().first);
       order_.pop_front();
     }
@@ -318,10 +322,12 @@ class PlanCache {
     std::lock_guard<std::mutex> lock(m_);
     map_.clear();
     gone.swap(order_);
+    bytes_ = 0;
   }
 
  private:
   std::mutex m_;
+  size_t bytes_ = 0;   // of the plans in the cache
   std::list<std::pair<PlanKey, PlanPtr>> order_;   // least recently used first
   std::unordered_map<PlanKey, std::list<std::pair<PlanKey, PlanPtr>>::iterator, PlanKeyHash> map_;
 };

@@ -99,11 +99,13 @@ __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
 // classified twice; in exchange the lists need no kernel of their own that walks the classes serially. The last CTA of a
 // sequence sorts its items. All of it is latency: a step on 8 x 2048 tokens spent 21 us in a memset and three kernels, of
 // which the serial lists took 8, and evaluating a tile pair by pair 5 (now a row's 128 bits are a few word operations).
+// The pairs' CTAs also write the bits of their PARTIAL tiles, which the attention kernels mask with (0.1-1.5 us of a plan; each kernel
+// and head formed them anew before, up to a tenth of a forward).
 constexpr int CL_THREADS = 512, CL_WARPS = CL_THREADS / 32;
 
 // exact class of tile (qt, kt) from all its pairs; one warp
-// (desc, tilebits: of the sequence)
-__device__ __forceinline__ int classify_exact(const uint32_t* desc, const uint32_t* tilebits, int qt, int kt, int lane) {
+// (desc, tilebits: of the sequence; words: null, or where a PARTIAL tile's bits go)
+__device__ __forceinline__ int classify_exact(const uint32_t* desc, const uint32_t* tilebits, int qt, int kt, int lane, uint32_t* words) {
   const uint32_t *dq = desc + qt * KD_TILE, *dk = desc + kt * KD_TILE, *tb = tilebits + kt * 32;
   uint32_t pre[4], ctx[4], ins[4], kd[4], qd[4];
   uint32_t any_ins = 0u;
@@ -116,10 +118,10 @@ __device__ __forceinline__ int classify_exact(const uint32_t* desc, const uint32
     kd[w] = dk[w * 32 + lane];
     qd[w] = dq[w * 32 + lane];
   }
-  uint32_t on = 0u, off = 0u;
+  uint32_t on = 0u, off = 0u, m[4][4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    uint32_t mk[4];
+    uint32_t (&mk)[4] = m[r];
     query_row_mask<4>(qd[r], qt * KD_TILE + r * 32 + lane, kt * KD_TILE, pre, ctx, ins, mk);
     // "same span": one round per distinct span among the 32 queries; a ballot gives the keys of that span
     const uint32_t my_key = span_key_of_query(qd[r]);
@@ -141,6 +143,12 @@ __device__ __forceinline__ int classify_exact(const uint32_t* desc, const uint32
     }
   }
   const bool w_on = __any_sync(0xffffffffu, on != 0u), w_off = __any_sync(0xffffffffu, off != 0u);
+  if (words != nullptr && w_on && w_off) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int w = 0; w < 4; ++w) words[w * KD_TILE + r * 32 + lane] = m[r][w];
+  }
   return w_on ? (w_off ? KD_TILE_PARTIAL : KD_TILE_FULL) : KD_TILE_EMPTY;
 }
 
@@ -189,7 +197,9 @@ __global__ void __launch_bounds__(CL_THREADS) classify_kernel(PlanView pv) {
     const int r = e / NT, c = e - r * NT;
     const int qt = is_pair ? 2 * item + r : c, kt = is_pair ? c : item - NP;
     int cls = classify_summary(s_sum[qt], s_sum[kt], qt, kt);
-    if (cls < 0) cls = classify_exact(pv.desc + (size_t)b * pv.Tpad, pv.tilebits + (size_t)b * NT * 32, qt, kt, lane);
+    if (cls < 0 || (is_pair && cls == KD_TILE_PARTIAL))   // (a pair's CTA writes the bits of its PARTIAL tiles)
+      cls = classify_exact(pv.desc + (size_t)b * pv.Tpad, pv.tilebits + (size_t)b * NT * 32, qt, kt, lane,
+                           is_pair ? pv.words + (((size_t)b * NT + qt) * NT + kt) * KD_WORDS : nullptr);
     if (lane == 0) {
       s_cls[r][c] = static_cast<uint8_t>(cls);
       if (is_pair) pv.cls[((size_t)b * NT + qt) * NT + kt] = static_cast<uint8_t>(cls);
@@ -292,7 +302,7 @@ __global__ void __launch_bounds__(PS_THREADS) plan_small_kernel(kd_meta m, PlanV
   for (int e = warp; e < NT * NT; e += PS_WARPS) {
     const int qt = e / NT, kt = e - qt * NT;
     int cls = classify_summary(s_sum[qt], s_sum[kt], qt, kt);
-    if (cls < 0) cls = classify_exact(s_desc, s_bits, qt, kt, lane);
+    if (cls < 0 || cls == KD_TILE_PARTIAL) cls = classify_exact(s_desc, s_bits, qt, kt, lane, pv.words + ((size_t)b * NT * NT + e) * KD_WORDS);
     if (lane == 0) {
       s_cls[qt][kt] = static_cast<uint8_t>(cls);
       pv.cls[(size_t)b * NT * NT + e] = static_cast<uint8_t>(cls);

@@ -128,3 +128,21 @@ def test_both_forms_of_the_plan_kernels_without_metadata(B, T, causal):
     lens = np.array([(T, 0, 1, T - 1, T // 2)[b % 5] for b in range(B)], np.int32)
     _check(_plan(T, lens=lens, causal=causal), ao.dense_mask(T, lens=lens, causal=causal))
     _check(_plan(T, causal=causal, B=B), ao.dense_mask(T, causal=causal, B=B))
+
+
+@pytest.mark.parametrize("B,T,rules", [(1, 1, False), (2, 129, True), (3, 513, True), (9, 300, True), (2, 640, True), (2, 1025, False), (2, 1100, True)])
+def test_visibility_words_of_partial_tiles(B, T, rules):
+    """The bits the attention kernels mask with, of both plan forms (one launch and two): those of the dense mask, zero beyond T."""
+    meta = random_meta(T, B, T) if rules else (None, None, None)
+    lens = np.maximum(1, T - 37 * np.arange(B)).astype(np.int32)
+    plan = _plan(T, *meta, lens, rules=rules)
+    mask = ao.dense_mask(T, *meta, lens) if rules else ao.dense_mask(T, *(np.zeros((B, T), x) for x in (bool, np.int64, bool)), lens)
+    NT = plan.NT
+    padded = np.zeros((B, NT * 128, NT * 128), bool)
+    padded[:, :T, :T] = mask
+    tiles = padded.reshape(B, NT, 128, NT, 128).transpose(0, 1, 3, 2, 4)   # [b][query tile][key tile][query][key]
+    bits = np.packbits(tiles.reshape(B, NT, NT, 128, 4, 32), axis=-1, bitorder="little").view(np.uint32)[..., 0].swapaxes(-1, -2)
+    words = plan.buf[-B * NT * NT * 2048:].cpu().numpy().view(np.uint32).reshape(B, NT, NT, 4, 128)
+    partial = ao.tile_classes(mask) == ao.PARTIAL
+    assert partial.any()
+    assert np.array_equal(words[partial], bits[partial])
