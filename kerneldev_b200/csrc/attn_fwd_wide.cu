@@ -107,7 +107,8 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   // header of this CTA's k-th item; false: there is none. The slot stays taken until item_done.
   auto next_item = [&](int k, int4& it) -> bool {
     const int slot = k % C::NITEM;
-    if (!wait(C::B_ITEMFULL + slot, (k / C::NITEM) & 1, W_F_ITEMFULL)) return false;
+    // (Twice the limit: warps without work wait here for as long as the others wait for what is late, and those are to say what it is.)
+    if (!__all_sync(0xffffffffu, mbar_wait(bar(C::B_ITEMFULL + slot), (k / C::NITEM) & 1, abortf, W_F_ITEMFULL, 2u * KD_WAIT_LIMIT_CYCLES))) return false;
     const int4 v = items[slot];
     it.x = __reduce_max_sync(0xffffffffu, v.x);   // warp-uniform for the compiler
     it.y = __reduce_max_sync(0xffffffffu, v.y);

@@ -147,12 +147,12 @@ __device__ __forceinline__ void raise_abort(AbortFlag* abort_flag, uint32_t site
 // another role has aborted. This is inlined dozens of times per kernel, between hot loops that compete for the
 // instruction cache, so the slow path is a few instructions: a 32-bit cycle count, and the status word is left to the
 // end of the kernel (with the reporting inlined here the fused backward was 120 KB of code).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFlag* abort_flag, uint32_t site) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, AbortFlag* abort_flag, uint32_t site, uint32_t limit = KD_WAIT_LIMIT_CYCLES) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint32_t t0 = clock32();
   while (!mbar_try_wait_suspend(bar, parity, 20000u)) {
     if (abort_flag->v != 0u) return false;
-    if (clock32() - t0 > KD_WAIT_LIMIT_CYCLES) {
+    if (clock32() - t0 > limit) {
       raise_abort(abort_flag, site);
       return false;
     }
