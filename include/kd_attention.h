@@ -127,7 +127,7 @@ typedef struct kd_attn_params {
                          KD_BWD_FUSED, bwd_phases 1 runs the delta kernel alone and 2 the fused kernel. */
   float* dq_acc;      /* KD_BWD_FUSED: (B,H,T,W) contiguous fp32 scratch, W = 64 for D <= 64 and 128 above
                          (kd_workspace_bytes_fused gives its size); the library zeroes what it reads of it. Columns at or
-                         beyond D are unspecified after the call. Ignored otherwise. */
+                         beyond D and rows of padding are unspecified after the call. Ignored otherwise. */
   int32_t heads_per_cta; /* >= 0. Ignored, kept for the layout: every kernel takes its work items, tiles of single heads, dynamically. */
   int32_t plan_ready;    /* 1: an earlier launch on the same stream has used this plan, which lets kd_attn_fwd look up its
                          work before the kernel ahead of it on the stream has finished. 0 is always correct. */

@@ -72,55 +72,62 @@ enum : uint32_t {
 // =========================================================================================
 // A float32 call (kF32) leaves two more passes to it: dO is rounded to the 16-bit operand on the way, and dQ, into which the fused
 // backward then adds, is zeroed in place of a scratch.
+// Rows of padding see nothing: neither their O and dO are read nor their scratch zeroed (the conversion writes zeros there without a look at it).
 template <int HD, bool kBf16, bool kF32>
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
-  constexpr int TPR = HD / 8;   // threads per row
-  constexpr int RPB = 256 / TPR;   // rows per block and iteration
-  const size_t rows = (size_t)a.B * a.H * a.T;
-  const int sub = threadIdx.x % TPR;
+  using R = RowBlocks<HD>;
+  const int sub = threadIdx.x % R::TPR;
+  const int b = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * R::ROWS;
+  if (a.len_ready == 0) pdl_wait();
+  const int len = __ldcg(a.len + b);
   pdl_wait();
   pdl_launch_dependents();
-  // the loop bound is the same for every thread of the block: the shuffles below need full warps
-  for (size_t base = (size_t)blockIdx.x * RPB; base < rows; base += (size_t)gridDim.x * RPB) {
-    const size_t r = base + threadIdx.x / TPR;
-    const bool live = r < rows;
-    float acc = 0.f;
-    if (live && sub * 8 < a.d_real) {
-      const int t = static_cast<int>(r % a.T);
-      const int h = static_cast<int>((r / a.T) % a.H);
-      const int b = static_cast<int>(r / ((size_t)a.T * a.H));
-      const uint4 ov = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)t * a.o_st + sub * 8);
-      uint4* dp = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.d_o) + (size_t)b * a.do_sb + (size_t)h * a.do_sh + (size_t)t * a.do_st + sub * 8);
-      uint4 dv;
+  const size_t row0 = ((size_t)b * a.H + h) * a.T;
+  uint16_t* d_o = reinterpret_cast<uint16_t*>(a.d_o) + (size_t)b * a.do_sb + (size_t)h * a.do_sh + sub * 8;
+  // the loops' bounds are the same for every thread of the block: the shuffles below need full warps
+  uint4 ov[R::STEPS], dv[R::STEPS];
+#pragma unroll
+  for (int i = 0; i < R::STEPS; ++i) {   // all loads ahead of the stores
+    const int t = t0 + i * R::RPB + threadIdx.x / R::TPR;
+    ov[i] = dv[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (t < len && sub * 8 < a.d_real) {
+      ov[i] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.o) + (size_t)b * a.o_sb + (size_t)h * a.o_sh + (size_t)t * a.o_st + sub * 8);
       if (kF32 && a.d_o32 != nullptr) {
         const float4* src = reinterpret_cast<const float4*>(a.d_o32 + (size_t)b * a.do32_sb + (size_t)h * a.do32_sh + (size_t)t * a.do32_st + sub * 8);
         const float4 x = src[0], y = src[1];
-        dv = make_uint4(pack2<kBf16>(x.x, x.y), pack2<kBf16>(x.z, x.w), pack2<kBf16>(y.x, y.y), pack2<kBf16>(y.z, y.w));
-        *dp = dv;
+        dv[i] = make_uint4(pack2<kBf16>(x.x, x.y), pack2<kBf16>(x.z, x.w), pack2<kBf16>(y.x, y.y), pack2<kBf16>(y.z, y.w));
       } else {
-        dv = *dp;
+        dv[i] = *reinterpret_cast<const uint4*>(d_o + (size_t)t * a.do_st);
       }
-      if (kF32 && a.zero_dq) {
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R::STEPS; ++i) {
+    const int t = t0 + i * R::RPB + threadIdx.x / R::TPR;
+    float acc = 0.f;
+    const uint32_t ow[4] = {ov[i].x, ov[i].y, ov[i].z, ov[i].w}, dw[4] = {dv[i].x, dv[i].y, dv[i].z, dv[i].w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 x = unpack2<kBf16>(ow[k]), y = unpack2<kBf16>(dw[k]);
+      acc = fmaf(x.x, y.x, acc);
+      acc = fmaf(x.y, y.y, acc);
+    }
+    if (!kF32 && a.dq_acc != nullptr && t < len && sub * 8 < a.d_real) {   // the columns beyond are never read (zeroed too: causal 8 x 16 x 2048 x 80 370 us, 365 without)
+      float4* z = reinterpret_cast<float4*>(a.dq_acc + (row0 + t) * HD + sub * 8);
+      z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+      z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if (kF32 && t < a.T && sub * 8 < a.d_real) {
+      if (a.d_o32 != nullptr) *reinterpret_cast<uint4*>(d_o + (size_t)t * a.do_st) = dv[i];   // of padding too (zeros): the fused kernel reads whole tiles
+      if (a.zero_dq) {
         float4* z = reinterpret_cast<float4*>(static_cast<float*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + (size_t)t * a.dq_st + sub * 8);
         z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
         z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, dw[4] = {dv.x, dv.y, dv.z, dv.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float2 x = unpack2<kBf16>(ow[k]), y = unpack2<kBf16>(dw[k]);
-        acc = fmaf(x.x, y.x, acc);
-        acc = fmaf(x.y, y.y, acc);
-      }
     }
 #pragma unroll
-    for (int d = TPR / 2; d >= 1; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-    if (live && sub == 0) a.delta[r] = acc;
-    if (live && a.dq_acc != nullptr && sub * 8 < a.d_real) {   // the columns beyond are never read (zeroed too: causal 8 x 16 x 2048 x 80 370 us, 365 without)
-      float4* z = reinterpret_cast<float4*>(a.dq_acc + r * HD + sub * 8);
-      z[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-      z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    for (int d = R::TPR / 2; d >= 1; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (t < a.T && sub == 0) a.delta[row0 + t] = acc;
   }
 }
 
@@ -978,13 +985,14 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.d_real = p.D;
   a.scale_log2 = scale_log2_of(p.sm_scale);
   a.sm_scale = p.sm_scale;
-  a.words = pv.words; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
+  a.words = pv.words; a.len = pv.len; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
   a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.d_o = p.d_o.ptr; a.do_sb = p.d_o.stride_b; a.do_sh = p.d_o.stride_h; a.do_st = p.d_o.stride_t;
   a.lse = p.lse; a.delta = p.delta;
   // with the delta kernel ahead of them in this call, the plan was complete before the kernels may start
   a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
+  a.len_ready = p.plan_ready;
   a.after_dq = 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
   a.grads_f32 = f32 != nullptr;
@@ -1009,10 +1017,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   a.order_of = ItemOrder::make(p.B * p.H, L.NT, (double)p.T * p.D * 2 * 5, 64e6);   // Q, K, V, dO and a gradient (32 and 128 MB: within 1 %; no chunks: up to 6 % slower)
   const int phases = (p.bwd_phases & 3) ? (p.bwd_phases & 3) : 3;
   if (phases & 1) {
-    const size_t rows = (size_t)p.B * p.H * p.T;
-    const int rows_per_block = 256 / (HD / 8);
-    const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-    e = launch(attn_bwd_delta_kernel<HD, kBf16, kF32>, blocks, 256, 0, stream, a);
+    e = launch(attn_bwd_delta_kernel<HD, kBf16, kF32>, RowBlocks<HD>::grid(p.B, p.H, p.T), 256, 0, stream, a);
     if (!fused && e == cudaSuccess) e = launch(kq, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
   }
   if (fused && e == cudaSuccess) {

@@ -36,6 +36,20 @@ struct BwdArgs {
   int64_t dk_sb, dk_sh, dk_st;
   void* dv;
   int64_t dv_sb, dv_sh, dv_st;
+  const int32_t* len;   // [B] tokens that are not padding (at the end: the fused kernel of head dim 64 is 2 % slower with its other arguments elsewhere)
+  int len_ready;     // the plan may be read by the delta kernel before the wait for the kernel ahead
+};
+
+// How the delta and the conversion kernel (256 threads) divide the rows: a block per ROWS rows of a head, HD / 8 threads to a row, three rows to a
+// thread, all of whose loads are under way together. Both are bound by HBM traffic, and leave the rows of padding alone (delta kernel,
+// hierarchical 16 x 16 x 4096 x 64 with a third of padding 84 -> 56 us; whole backward 1070 -> 1020, 8 x 16 x 2048 x 64 163 -> 151, 4 x 16 x 2048 x
+// 128 140 -> 129). The block index gives head and sequence: with a flat row index, three 64-bit divisions a row and the length looked up for each
+// the kernels lost 2 % of the backward without padding (causal 8 x 16 x 2048 x 64), with the length fetched a row ahead 10 %. One row to a thread
+// 288 -> 303 us there, two 293, four 294.
+template <int HD>
+struct RowBlocks {
+  static constexpr int TPR = HD / 8, RPB = 256 / TPR, STEPS = 3, ROWS = RPB * STEPS;
+  static dim3 grid(int B, int H, int T) { return dim3((T + ROWS - 1) / ROWS, H, B); }
 };
 
 // 32 x 32 bits across a warp: lane l gives word l and gets bit l of every lane's word, lane 0's in bit 0

@@ -1056,24 +1056,35 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 // dq[b, h, t, :] = dq_acc[b, h, t, :] * sm_scale in the output dtype; HD / 8 threads per row, 32 bytes in and 16 out each
 template <int HD, bool kBf16>
 __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs a) {
-  constexpr int TPR = HD / 8;
-  const size_t rows = (size_t)a.B * a.H * a.T;
-  const int sub = threadIdx.x % TPR;
+  using R = RowBlocks<HD>;
+  const int sub = threadIdx.x % R::TPR;
+  const int b = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * R::ROWS;
+  const int len = __ldcg(a.len + b);   // (the plan was complete before the fused kernel let this one start)
   pdl_wait();
   pdl_launch_dependents();
-  for (size_t r = (size_t)blockIdx.x * (256 / TPR) + threadIdx.x / TPR; r < rows; r += (size_t)gridDim.x * (256 / TPR)) {
-    const int t = static_cast<int>(r % a.T);
-    const int h = static_cast<int>((r / a.T) % a.H);
-    const int b = static_cast<int>(r / ((size_t)a.T * a.H));
-    if (sub * 8 >= a.d_real) continue;
-    const float4* src = reinterpret_cast<const float4*>(a.dq_acc + r * HD + sub * 8);
-    const float4 x = src[0], y = src[1];
+  if (sub * 8 >= a.d_real) return;
+  const size_t row0 = ((size_t)b * a.H + h) * a.T;
+  uint16_t* out = reinterpret_cast<uint16_t*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + sub * 8;
+  float4 x[R::STEPS], y[R::STEPS];
+#pragma unroll
+  for (int i = 0; i < R::STEPS; ++i) {
+    const int t = t0 + i * R::RPB + threadIdx.x / R::TPR;
+    x[i] = y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (t < len) {   // (the scratch of padding has not been zeroed)
+      const float4* src = reinterpret_cast<const float4*>(a.dq_acc + (row0 + t) * HD + sub * 8);
+      x[i] = src[0];
+      y[i] = src[1];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < R::STEPS; ++i) {
+    const int t = t0 + i * R::RPB + threadIdx.x / R::TPR;
     uint4 v;
-    v.x = pack2<kBf16>(x.x * a.sm_scale, x.y * a.sm_scale);
-    v.y = pack2<kBf16>(x.z * a.sm_scale, x.w * a.sm_scale);
-    v.z = pack2<kBf16>(y.x * a.sm_scale, y.y * a.sm_scale);
-    v.w = pack2<kBf16>(y.z * a.sm_scale, y.w * a.sm_scale);
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.dq) + (size_t)b * a.dq_sb + (size_t)h * a.dq_sh + (size_t)t * a.dq_st + sub * 8) = v;
+    v.x = pack2<kBf16>(x[i].x * a.sm_scale, x[i].y * a.sm_scale);
+    v.y = pack2<kBf16>(x[i].z * a.sm_scale, x[i].w * a.sm_scale);
+    v.z = pack2<kBf16>(y[i].x * a.sm_scale, y[i].y * a.sm_scale);
+    v.w = pack2<kBf16>(y[i].z * a.sm_scale, y[i].w * a.sm_scale);
+    if (t < a.T) *reinterpret_cast<uint4*>(out + (size_t)t * a.dq_st) = v;
   }
 }
 
@@ -1112,10 +1123,7 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   }
   if (launch_regs < C::REGS_LAUNCH) return set_error(KD_ERR_DEVICE, "fused bwd was built with %d registers per thread, needs %d", launch_regs, C::REGS_LAUNCH);
   e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
-  const size_t rows = (size_t)a.B * a.H * a.T;
-  const int rows_per_block = 256 / (HD / 8);
-  const int blocks = static_cast<int>(std::min<size_t>((rows + rows_per_block - 1) / rows_per_block, size_t(148) * 32));
-  if (e == cudaSuccess && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, blocks, 256, 0, stream, a);
+  if (e == cudaSuccess && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, RowBlocks<HD>::grid(a.B, a.H, a.T), 256, 0, stream, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }

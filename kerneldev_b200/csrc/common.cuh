@@ -29,6 +29,7 @@ struct PlanView {
   uint8_t* order;
   uint32_t* stats;
   uint32_t* done;   // [B] CTAs of the classifier that have finished
+  int32_t* len;     // [B] tokens of each sequence that are not padding
   uint32_t* status;
   uint32_t* words;
 };
@@ -50,6 +51,7 @@ inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
   v.order = reinterpret_cast<uint8_t*>(base + L.off_order);
   v.stats = reinterpret_cast<uint32_t*>(base + L.off_stats);
   v.done = v.stats + 2 * (size_t)L.B;
+  v.len = reinterpret_cast<int32_t*>(v.stats + 3 * (size_t)L.B);
   v.status = reinterpret_cast<uint32_t*>(base + L.off_status);
   v.words = reinterpret_cast<uint32_t*>(base + L.total - (size_t)L.B * L.NT * L.NT * KD_WORDS_BYTES);
   return v;

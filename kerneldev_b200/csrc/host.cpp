@@ -471,6 +471,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
+  p.plan_ready = plan->ready_on(stream) ? 1 : 0;
   check(f32 ? lib.attn_bwd_f32(&p, &f, stream) : lib.attn_bwd(&p, stream));
   plan->after_launch();
   return {dq, dk, dv};

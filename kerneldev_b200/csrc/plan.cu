@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(KD_TILE) pack_kernel(kd_meta m, PlanView pv) {
       pv.stats[b * 2 + 0] = 0;
       pv.stats[b * 2 + 1] = 0;
       pv.done[b] = 0;
+      pv.len[b] = tokens_of(m, b);
     }
   }
 }
@@ -268,6 +269,7 @@ __global__ void __launch_bounds__(PS_THREADS) plan_small_kernel(kd_meta m, PlanV
   pdl_wait();
   pdl_launch_dependents();
   const int n_b = tokens_of(m, b);
+  if (tid == 0) pv.len[b] = n_b;
   for (int w = warp; w < 4 * NT; w += PS_WARPS) {   // 32 tokens: word w & 3 of tile w >> 2
     bool bad_id = false;
     const uint32_t d = describe(m, b, 32 * w + lane, n_b, bad_id);

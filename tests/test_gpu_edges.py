@@ -45,6 +45,31 @@ def test_cocktail_scores_and_gradient(B, T, C, dtype):
     assert bool((err <= 2 * eps * e_ref.grad.abs() + (S + T + 8) * 2.0**-24 * top).all())
 
 
+# Rows of padding are left alone by the delta and conversion kernels: garbage in every buffer they are given must not come through. T and lens at the
+# edges of their blocks (96 rows at head dims up to 64, 48 above) and of tiles
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (16, torch.float16), (128, torch.bfloat16), (80, torch.float16)])
+@pytest.mark.parametrize("T,lens", [(95, (95, 0, 1)), (97, (96, 97, 48)), (300, (47, 289, 128)), (192, (192, 191, 129))])
+def test_padding_is_left_out_of_delta_and_conversion(T, lens, D, dtype):
+    from tests.helpers import assert_close, rand_inputs
+    from kerneldev_b200.original_kernel import _backward, _forward
+    from kerneldev_b200.plan import AttentionPlan
+    B, H = len(lens), 3
+    q, k, v, do = rand_inputs(B, H, T, D, dtype, T + D)
+    lens = torch.tensor(lens, dtype=torch.int32)
+    plan = AttentionPlan(B, T, DEV, lens=lens.to(DEV), causal=True)
+    dev = [x.to(DEV) for x in (q, k, v, do)]
+    o, lse = _forward(*dev[:3], plan, D ** -0.5)
+    bufs = [torch.full_like(dev[0], float("nan")) for _ in range(3)]
+    bufs += [torch.full((B, H, T, *w), float("nan"), device=DEV) for w in ((), (64 if D <= 64 else 128,))]
+    got = _backward(*dev[:3], o, lse, dev[3], plan, D ** -0.5, 0, bufs)
+    mask = ao.dense_mask(T, lens=lens, causal=True)
+    ref = ao.attention_fwd_bwd(*(x.float() for x in (q, k, v, do)), mask, D ** -0.5)[2:]
+    beyond = torch.arange(T)[None, None, :, None] >= lens[:, None, None, None]
+    for name, g, want in zip(("dQ", "dK", "dV"), got, ref):
+        assert_close(name, g, want)
+        assert not g.cpu()[beyond.expand_as(g)].any()
+
+
 # More items than SMs, so that CTAs take several one after the other; chunks of heads of equal and (at T = 1280) unequal size. `lens` makes runs of empty items longer than the ring of
 # item headers between items with work (both tile widths; an odd number of query tiles; a last tile of 1 and of 127 tokens)
 @pytest.mark.parametrize("deterministic", [False, True])
