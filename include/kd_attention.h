@@ -130,7 +130,8 @@ typedef struct kd_attn_params {
                          beyond D and rows of padding are unspecified after the call. Ignored otherwise. */
   int32_t heads_per_cta; /* >= 0. Ignored, kept for the layout: every kernel takes its work items, tiles of single heads, dynamically. */
   int32_t plan_ready;    /* 1: an earlier launch on the same stream has used this plan, which lets kd_attn_fwd look up its
-                         work before the kernel ahead of it on the stream has finished. 0 is always correct. */
+                         work, and the first kernel of kd_attn_bwd the sequences' lengths, before the kernel ahead of it
+                         on the stream has finished. 0 is always correct. */
 } kd_attn_params;
 
 /* Size and layout of a plan for B sequences of T tokens. */

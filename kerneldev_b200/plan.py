@@ -5,8 +5,8 @@ A plan holds the packed token descriptors, the class (EMPTY / FULL / PARTIAL) of
 metadata (``in_span``, ``span_id``, ``is_prefix``, ``lens``, ``causal``), not on the head, so one
 plan serves all heads and -- because ``model.GPTModel`` passes the same three metadata tensors
 to every layer (model.py:243-244) -- all layers of a step. Plans are cached on the identity and
-version of the metadata tensors (the cache keeps those tensors alive, so an address cannot be
-reused while its plan is cached). Metadata rewritten in place through raw pointers -- by
+version of the metadata tensors (the cache keeps their memory alive, so an address cannot be
+reused while its plan is cached; a plan whose metadata nobody else holds any more leaves the cache with the next new plan). Metadata rewritten in place through raw pointers -- by
 kd_metadata_from_tokens into preallocated buffers, or through ``.data`` -- does not change a tensor's
 version: call ``clear_plan_cache()`` after such a write.
 

@@ -359,3 +359,36 @@ def test_second_derivatives_of_the_cocktail_scores(through_ds):
     (want,) = torch.autograd.grad(penalty(ao.cocktail_scores(y, tokens.cpu())[0], y, w0.double()), y)
     assert (want - 2 * y).abs().max() > 0.1
     assert torch.allclose(got.double().cpu(), want, rtol=4 * (T + C) * 2.0**-24, atol=4 * (T + C) * 2.0**-24 * float(want.abs().max()))
+
+
+def test_cached_plans_whose_metadata_is_gone_leave_the_cache():
+    """A plan is kept as long as somebody could ask for it again: as long as the caller holds its metadata, or a tensor that the metadata is a
+    view of, and not when a new batch has taken its place."""
+    from kerneldev_b200 import clear_plan_cache
+    from kerneldev_b200.plan import _CACHE, get_plan
+    B, T = 2, 300
+    dev = torch.device(DEV)
+
+    def new(more=0):
+        ids = torch.zeros((B, T + more), dtype=torch.int64, device=DEV)
+        return ids > 0, ids
+
+    def plan_of(ins, sid):
+        return get_plan(B, T, dev, ins, sid, None, None, True, True)._core
+
+    def plan_of_views(ins, sid):
+        return plan_of(ins[:, :T], sid[:, :T].to(torch.int32))
+
+    clear_plan_cache()
+    held = [(ins, sid.to(torch.int32)) for ins, sid in (new(20) for _ in range(3))]   # (converted for the kernels)
+    first = [plan_of_views(*h) for h in held]
+    span = torch.ones((B, T), dtype=torch.bool, device=DEV)   # no view, and alone
+    alone = get_plan(B, T, dev, span, None, None, None, True, True)._core
+    plain = get_plan(B, T, dev, None, None, None, None, True, False)._core
+    for _ in range(20):
+        plan_of(*new())
+    assert len(_CACHE) <= len(first) + 2 + 1
+    assert all(plan_of_views(*h) is f for h, f in zip(held, first))
+    assert get_plan(B, T, dev, span, None, None, None, True, True)._core is alone
+    assert get_plan(B, T, dev, None, None, None, None, True, False)._core is plain
+    clear_plan_cache()
