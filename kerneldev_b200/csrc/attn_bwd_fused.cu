@@ -259,11 +259,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       auto write_zeros = [&](const int4& z) {
         using Out = std::conditional_t<kF32, float, uint16_t>;
         constexpr int per = 16 / sizeof(Out);   // elements of a 16-byte chunk
-        const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0), cpr = a.d_real / per;
+        constexpr int CPR = HD / per;           // chunks of a tile's row
+        const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0);
         Out* dk = reinterpret_cast<Out*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
         Out* dv = reinterpret_cast<Out*>(a.dv) + (size_t)z.x * a.dv_sb + (size_t)z.y * a.dv_sh;
-        for (int i = lane; i < rows * cpr; i += 32) {
-          const int r = i / cpr, c = (i - r * cpr) * per;
+        // (Items without entries come last, and nothing hides them there. With a division by the real width for each chunk: hierarchical
+        // 4 x 16 x 2048 x 64 88.5 us, 87.5 now, 8 x 16 x 2048 x 64 163 -> 161, 8 x 8 x 1000 x 64 33.4 -> 32.5.)
+        for (int i = lane; i < rows * CPR; i += 32) {
+          const int r = i / CPR, c = i % CPR * per;
+          if (c >= a.d_real) continue;
           *reinterpret_cast<uint4*>(dk + (size_t)(row0 + r) * a.dk_st + c) = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(dv + (size_t)(row0 + r) * a.dv_st + c) = make_uint4(0u, 0u, 0u, 0u);
         }
