@@ -157,6 +157,11 @@ int kd_attn_fwd(const kd_attn_params* p, void* stream);
  * with its dQ and dK/dV workers (:713-838, :1173-1525). */
 int kd_attn_bwd(const kd_attn_params* p, void* stream);
 
+/* kd_attn_bwd (KD_BWD_FUSED, all phases) on Q and K that kd_hadamard has transformed with these signs: dQ and dK come back for the tensors
+ * they were made from. As kd_attn_bwd and kd_hadamard(inverse = 1) on dQ and dK, with dQ rounded once and two passes over memory fewer.
+ * D 16, 32, 64 or 128; signs: (H,D) contiguous, 16-byte aligned. */
+int kd_attn_bwd_hadamard(const kd_attn_params* p, const float* signs, void* stream);
+
 /* float32 tensors of a call whose operands are float16 copies (p->dtype KD_F16; see kd_cast): what the kernels of the call read or
  * write of them directly, in place of a conversion before or behind. Pointers and byte strides multiples of 16. No counterpart in the
  * reference, whose float32 path multiplies in tf32. */

@@ -24,7 +24,7 @@ LIB_PATH = Path(os.environ.get("KD_LIB_PATH") or Path(__file__).resolve().parent
 
 EXPORTS = (
     "kd_version", "kd_last_error", "kd_plan_layout_get", "kd_classify", "kd_mask_dense",
-    "kd_attn_fwd", "kd_attn_bwd", "kd_attn_fwd_f32", "kd_attn_bwd_f32", "kd_attn_bwd_static", "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard",
+    "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_hadamard", "kd_attn_fwd_f32", "kd_attn_bwd_f32", "kd_attn_bwd_static", "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard",
     "kd_metadata_from_tokens", "kd_span_index", "kd_span_mean",
     "kd_cocktail_index", "kd_cocktail_scores", "kd_cocktail_grad",
     "kd_cast",
@@ -92,6 +92,7 @@ def load() -> ctypes.CDLL:
     lib.kd_mask_dense.argtypes = [c_void_p, c_int32, c_int32, c_void_p, c_void_p]
     lib.kd_attn_fwd.argtypes = [POINTER(KdAttnParams), c_void_p]
     lib.kd_attn_bwd.argtypes = [POINTER(KdAttnParams), c_void_p]
+    lib.kd_attn_bwd_hadamard.argtypes = [POINTER(KdAttnParams), c_void_p, c_void_p]
     lib.kd_attn_bwd_static.argtypes = [POINTER(KdAttnParams), c_void_p]
     lib.kd_workspace_bytes.argtypes = [c_int32, c_int32, c_int32, c_int32, POINTER(c_size_t)]
     lib.kd_workspace_bytes_fused.argtypes = [c_int32, c_int32, c_int32, c_int32, POINTER(c_size_t)]
@@ -103,7 +104,7 @@ def load() -> ctypes.CDLL:
                                  c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.kd_metadata_from_tokens.argtypes = [c_void_p, c_int64, c_int32, c_int32, c_int64, c_int64, c_int64, c_int64,
                                             c_void_p, c_void_p, c_void_p, c_void_p]
-    for name in ("kd_plan_layout_get", "kd_classify", "kd_mask_dense", "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_static",
+    for name in ("kd_plan_layout_get", "kd_classify", "kd_mask_dense", "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_hadamard", "kd_attn_bwd_static",
                  "kd_workspace_bytes", "kd_workspace_bytes_fused", "kd_hadamard", "kd_metadata_from_tokens", "kd_span_index", "kd_span_mean"):
         getattr(lib, name).restype = c_int32
     _lib = lib

@@ -14,7 +14,7 @@ import torch  # noqa: F401  (the extension links against libtorch)
 from . import _capi
 from .build import HOST_PATH
 
-_ENTRY_POINTS = ("kd_plan_layout_get", "kd_classify", "kd_attn_fwd", "kd_attn_bwd", "kd_attn_fwd_f32", "kd_attn_bwd_f32", "kd_hadamard", "kd_metadata_from_tokens",
+_ENTRY_POINTS = ("kd_plan_layout_get", "kd_classify", "kd_attn_fwd", "kd_attn_bwd", "kd_attn_bwd_hadamard", "kd_attn_fwd_f32", "kd_attn_bwd_f32", "kd_hadamard", "kd_metadata_from_tokens",
                  "kd_cocktail_index", "kd_cocktail_scores", "kd_cocktail_grad", "kd_cast",
                  "kd_last_error")
 

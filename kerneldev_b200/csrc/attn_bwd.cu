@@ -972,7 +972,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 template <int HD, bool kBf16, bool kF32>
-static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
+static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const float* signs, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
   using C = BwdCfg<HD>;
   CUtensorMap tmQ, tmK, tmV, tmDO;
   int rc;
@@ -993,6 +993,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const k
   // with the delta kernel ahead of them in this call, the plan was complete before the kernels may start
   a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
   a.len_ready = p.plan_ready;
+  a.signs = signs;
   a.after_dq = 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
   a.grads_f32 = f32 != nullptr;
@@ -1072,12 +1073,12 @@ int static_delta_address(size_t rows_needed, float** out) {
   return 0;
 }
 
-int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream) {
+int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, const float* signs, cudaStream_t stream) {
   kd_plan_layout L;
   if (kd_plan_layout_get(p.B, p.T, &L) != 0) return KD_ERR_ARG;
   PlanView pv = make_plan_view(const_cast<void*>(p.plan), L);
   if (!p.d_o.ptr) return set_error(KD_ERR_ARG, "d_o is null");
-  auto run = [&](auto launch_fn) { return launch_fn(p, f32, L, pv, stream); };
+  auto run = [&](auto launch_fn) { return launch_fn(p, f32, signs, L, pv, stream); };
   const bool narrow = p.D <= 64;
   if (f32) return narrow ? run(launch_bwd_t<64, false, true>) : run(launch_bwd_t<128, false, true>);
   if (p.dtype == KD_BF16) return narrow ? run(launch_bwd_t<64, true, false>) : run(launch_bwd_t<128, true, false>);

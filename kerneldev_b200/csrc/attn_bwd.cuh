@@ -37,6 +37,7 @@ struct BwdArgs {
   void* dv;
   int64_t dv_sb, dv_sh, dv_st;
   const int32_t* len;   // [B] tokens that are not padding (at the end: the fused kernel of head dim 64 is 2 % slower with its other arguments elsewhere)
+  const float* signs;   // null, or Q and K are Hadamard transforms with these signs, and dQ and dK are wanted of what they were made from
   int len_ready;     // the plan may be read by the delta kernel before the wait for the kernel ahead
 };
 

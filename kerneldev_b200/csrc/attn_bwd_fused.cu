@@ -1127,6 +1127,8 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   }
   if (launch_regs < C::REGS_LAUNCH) return set_error(KD_ERR_DEVICE, "fused bwd was built with %d registers per thread, needs %d", launch_regs, C::REGS_LAUNCH);
   e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
+  if (e == cudaSuccess && !kF32 && a.signs != nullptr)
+    return launch_grad_transform(a.dq_acc, HD, a.sm_scale, a.len, a.signs, dq, dk, a.B, a.H, a.T, a.d_real, dtype, stream);
   if (e == cudaSuccess && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, RowBlocks<HD>::grid(a.B, a.H, a.T), 256, 0, stream, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;

@@ -217,7 +217,18 @@ int kd_attn_bwd(const kd_attn_params* p, void* stream) {
   int rc = check_attn(p, true);
   if (rc) return rc;
   if ((rc = check_device()) != 0) return rc;
-  return launch_attn_bwd(*p, nullptr, static_cast<cudaStream_t>(stream));
+  return launch_attn_bwd(*p, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+}
+
+int kd_attn_bwd_hadamard(const kd_attn_params* p, const float* signs, void* stream) {
+  int rc = check_attn(p, true);
+  if (rc) return rc;
+  if (!signs || (reinterpret_cast<uintptr_t>(signs) & 15u)) return set_error(KD_ERR_ARG, "signs is null or not 16-byte aligned");
+  if (p->D != 16 && p->D != 32 && p->D != 64 && p->D != 128) return set_error(KD_ERR_ARG, "head dim %d not supported (16, 32, 64 or 128)", p->D);
+  if (p->bwd_mode != KD_BWD_FUSED || (p->bwd_phases & 3) == 1 || (p->bwd_phases & 3) == 2)
+    return set_error(KD_ERR_ARG, "the transform of the gradients is part of all phases of the fused backward");
+  if ((rc = check_device()) != 0) return rc;
+  return launch_attn_bwd(*p, nullptr, signs, static_cast<cudaStream_t>(stream));
 }
 
 int kd_attn_fwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream) {
@@ -233,7 +244,7 @@ int kd_attn_bwd_f32(const kd_attn_params* p, const kd_attn_f32* f, void* stream)
   int rc = check_attn(p, true, f);
   if (rc) return rc;
   if ((rc = check_device()) != 0) return rc;
-  return launch_attn_bwd(*p, f, static_cast<cudaStream_t>(stream));
+  return launch_attn_bwd(*p, f, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int kd_attn_bwd_static(const kd_attn_params* p, void* stream) {
@@ -249,7 +260,7 @@ int kd_attn_bwd_static(const kd_attn_params* p, void* stream) {
   q.delta = scratch;
   q.bwd_mode = KD_BWD_SPLIT;   // the fused backward needs a second, much larger scratch
   if ((rc = check_attn(&q, true)) != 0) return rc;
-  return launch_attn_bwd(q, nullptr, static_cast<cudaStream_t>(stream));
+  return launch_attn_bwd(q, nullptr, nullptr, static_cast<cudaStream_t>(stream));
 }
 
 int kd_workspace_bytes(int32_t B, int32_t H, int32_t T, int32_t D, size_t* bytes) {

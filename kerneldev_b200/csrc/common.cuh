@@ -96,10 +96,14 @@ int launch_classify(const kd_meta& m, void* plan, cudaStream_t stream);
 int launch_mask_dense(const void* plan, int B, int T, uint8_t* out, cudaStream_t stream);
 // f32: NULL, or the call's float32 tensors (kd_attn_f32)
 int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream);
-int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_t stream);
+// signs: NULL, or of transformed Q and K (kd_attn_bwd_hadamard)
+int launch_attn_bwd(const kd_attn_params& p, const kd_attn_f32* f32, const float* signs, cudaStream_t stream);
 int static_delta_address(size_t rows_needed, float** out);
 int launch_hadamard(const kd_tensor& x, const kd_tensor& y, int B, int H, int T, int D, int dtype,
                     const float* signs, int inverse, cudaStream_t stream);
+
+int launch_grad_transform(const float* acc, int width, float scale, const int32_t* len, const float* signs, const kd_tensor& dq, const kd_tensor& dk,
+                          int B, int H, int T, int D, int dtype, cudaStream_t stream);
 
 int launch_cast(const kd_tensor* src, const kd_tensor* dst, int n, int B, int H, int T, int D, bool widen, cudaStream_t stream);
 

@@ -8,6 +8,54 @@
 
 namespace kd {
 
+// Unnormalised transform of rows of 8 CH TPR elements, in place. Element index = 8 * (sub + TPR * i) + k of v[i][k]: the bits of k and of i are
+// butterflied in registers, the bits of `sub` with warp shuffles (all lanes call it).
+template <int CH, int TPR>
+__device__ __forceinline__ void walsh_hadamard(float (&v)[CH][8], int sub) {
+  // inside a chunk
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+#pragma unroll
+    for (int s = 1; s < 8; s <<= 1) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if ((k & s) == 0) {
+          const float a0 = v[i][k], a1 = v[i][k | s];
+          v[i][k] = a0 + a1;
+          v[i][k | s] = a0 - a1;
+        }
+      }
+    }
+  }
+  // across the threads of the row
+#pragma unroll
+  for (int s = 1; s < TPR; s <<= 1) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float other = __shfl_xor_sync(0xffffffffu, v[i][k], s);
+        v[i][k] = (sub & s) ? (other - v[i][k]) : (v[i][k] + other);
+      }
+    }
+  }
+  // between this thread's chunks
+#pragma unroll
+  for (int s = 1; s < CH; s <<= 1) {
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      if ((i & s) == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float a0 = v[i][k], a1 = v[i | s][k];
+          v[i][k] = a0 + a1;
+          v[i | s][k] = a0 - a1;
+        }
+      }
+    }
+  }
+}
+
 // TPR = min(4, HD/8) threads share a token row; thread `sub` holds the 16-byte chunks sub, sub + TPR, ... of the
 // row (CH = HD/8/TPR chunks of 8 elements), so that a warp-wide load covers 64 contiguous bytes per row.
 // Element index = 8 * (sub + TPR * i) + k: index bits 0-2 (k) and the bits of i are butterflied in registers,
@@ -55,48 +103,7 @@ __global__ void __launch_bounds__(256) hadamard_kernel(const uint16_t* x, int64_
         v[i][4] *= s1.x; v[i][5] *= s1.y; v[i][6] *= s1.z; v[i][7] *= s1.w;
       }
     }
-    // index bits 0-2: inside a chunk
-#pragma unroll
-    for (int i = 0; i < CH; ++i) {
-#pragma unroll
-      for (int s = 1; s < 8; s <<= 1) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if ((k & s) == 0) {
-            const float a0 = v[i][k], a1 = v[i][k | s];
-            v[i][k] = a0 + a1;
-            v[i][k | s] = a0 - a1;
-          }
-        }
-      }
-    }
-    // the bits of `sub`: across the threads of the row
-#pragma unroll
-    for (int s = 1; s < TPR; s <<= 1) {
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float other = __shfl_xor_sync(0xffffffffu, v[i][k], s);
-          v[i][k] = (sub & s) ? (other - v[i][k]) : (v[i][k] + other);
-        }
-      }
-    }
-    // the bits of the chunk counter i: between this thread's chunks
-#pragma unroll
-    for (int s = 1; s < CH; s <<= 1) {
-#pragma unroll
-      for (int i = 0; i < CH; ++i) {
-        if ((i & s) == 0) {
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float a0 = v[i][k], a1 = v[i | s][k];
-            v[i][k] = a0 + a1;
-            v[i | s][k] = a0 - a1;
-          }
-        }
-      }
-    }
+    walsh_hadamard<CH, TPR>(v, sub);
 #pragma unroll
     for (int i = 0; i < CH; ++i) {
       float f[8];
@@ -117,6 +124,91 @@ __global__ void __launch_bounds__(256) hadamard_kernel(const uint16_t* x, int64_
       }
     }
   }
+}
+
+// The last pass of a fused backward on transformed Q and K: dQ from the fp32 scratch, scaled, and dK, both times the transform's transpose. One
+// launch in the place of the conversion to 16 bits and two transforms (fp16 4 x 32 x 8192 x 128 with a fifth of padding 172 + 2 x 128 us -> 307, bf16
+// 8 x 16 x 2048 x 64 18 + 2 x 20 -> 32), which write and read dQ once more, and dQ is rounded once. Rows of padding: dQ is 0 and its scratch not
+// read; dK is 0 already. By the bytes it would take 175 us (hadamard_kernel: 82 of 128): shuffles and butterflies are half of its issue slots. Pieces of
+// 4 floats, so that a load takes whole sectors: 317; five or six blocks to an SM 325 and 394 (registers).
+// blockIdx.x: 2 * (block of rows) + (0: dQ, 1: dK).
+struct GradTransformArgs {
+  const float* acc;
+  const int32_t* len;
+  const float* signs;
+  kd_tensor dq, dk;
+  int H, T, width;   // width: of the scratch's rows
+  float scale;
+};
+template <int HD, bool kBf16>
+__global__ void __launch_bounds__(256) grad_transform_kernel(const GradTransformArgs a) {
+  constexpr int TPR = (HD / 8 < 4) ? HD / 8 : 4, CH = HD / 8 / TPR, RPB = 256 / TPR;
+  const int sub = threadIdx.x % TPR, b = blockIdx.z, h = blockIdx.y, t = static_cast<int>(blockIdx.x >> 1) * RPB + threadIdx.x / TPR;
+  const bool is_k = (blockIdx.x & 1) != 0;
+  const int len = __ldcg(a.len + b);   // (the plan was complete before the fused kernel let this one start)
+  pdl_wait();
+  pdl_launch_dependents();
+  const kd_tensor& out = is_k ? a.dk : a.dq;
+  uint16_t* row = static_cast<uint16_t*>(out.ptr) + (size_t)b * out.stride_b + (size_t)h * out.stride_h + (size_t)t * out.stride_t;
+  float v[CH][8];
+#pragma unroll
+  for (int i = 0; i < CH; ++i)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[i][k] = 0.f;
+  const float norm = rsqrtf(static_cast<float>(HD)) * (is_k ? 1.0f : a.scale);
+  if (t < len) {
+    if (is_k) {
+      uint4 in[CH];
+#pragma unroll
+      for (int i = 0; i < CH; ++i) in[i] = *reinterpret_cast<const uint4*>(row + (sub + TPR * i) * 8);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const uint32_t w[4] = {in[i].x, in[i].y, in[i].z, in[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = unpack2<kBf16>(w[k]);
+          v[i][2 * k] = f.x; v[i][2 * k + 1] = f.y;
+        }
+      }
+    } else {
+      const float* src = a.acc + (((size_t)b * a.H + h) * a.T + t) * a.width;
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(src + (sub + TPR * i) * 8), y = *reinterpret_cast<const float4*>(src + (sub + TPR * i) * 8 + 4);
+        v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+        v[i][4] = y.x; v[i][5] = y.y; v[i][6] = y.z; v[i][7] = y.w;
+      }
+    }
+  }
+  walsh_hadamard<CH, TPR>(v, sub);
+  if (t >= (is_k ? len : a.T)) return;
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const float* sg = a.signs + h * HD + (sub + TPR * i) * 8;
+    const float4 s0 = *reinterpret_cast<const float4*>(sg), s1 = *reinterpret_cast<const float4*>(sg + 4);
+    uint4 w;
+    w.x = pack2<kBf16>(v[i][0] * norm * s0.x, v[i][1] * norm * s0.y);
+    w.y = pack2<kBf16>(v[i][2] * norm * s0.z, v[i][3] * norm * s0.w);
+    w.z = pack2<kBf16>(v[i][4] * norm * s1.x, v[i][5] * norm * s1.y);
+    w.w = pack2<kBf16>(v[i][6] * norm * s1.z, v[i][7] * norm * s1.w);
+    *reinterpret_cast<uint4*>(row + (sub + TPR * i) * 8) = w;
+  }
+}
+
+int launch_grad_transform(const float* acc, int width, float scale, const int32_t* len, const float* signs, const kd_tensor& dq, const kd_tensor& dk,
+                          int B, int H, int T, int D, int dtype, cudaStream_t stream) {
+  const GradTransformArgs a = {acc, len, signs, dq, dk, H, T, width, scale};
+  const int rows_per_block = 256 / (D / 8 < 4 ? D / 8 : 4);
+  const dim3 grid(2 * ((T + rows_per_block - 1) / rows_per_block), H, B);
+  auto run = [&](auto kernel) { return launch(kernel, grid, 256, 0, stream, a); };
+  const bool bf16 = dtype == KD_BF16;
+  cudaError_t e;
+  if (D == 16) e = bf16 ? run(grad_transform_kernel<16, true>) : run(grad_transform_kernel<16, false>);
+  else if (D == 32) e = bf16 ? run(grad_transform_kernel<32, true>) : run(grad_transform_kernel<32, false>);
+  else if (D == 64) e = bf16 ? run(grad_transform_kernel<64, true>) : run(grad_transform_kernel<64, false>);
+  else e = bf16 ? run(grad_transform_kernel<128, true>) : run(grad_transform_kernel<128, false>);
+  if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "grad_transform_kernel launch: %s", cudaGetErrorString(e));
+  return 0;
 }
 
 int launch_hadamard(const kd_tensor& x, const kd_tensor& y, int B, int H, int T, int D, int dtype,

@@ -61,6 +61,7 @@ struct Library {
   decltype(&kd_classify) classify = nullptr;
   decltype(&kd_attn_fwd) attn_fwd = nullptr;
   decltype(&kd_attn_bwd) attn_bwd = nullptr;
+  decltype(&kd_attn_bwd_hadamard) attn_bwd_hadamard = nullptr;
   decltype(&kd_attn_fwd_f32) attn_fwd_f32 = nullptr;
   decltype(&kd_attn_bwd_f32) attn_bwd_f32 = nullptr;
   decltype(&kd_hadamard) hadamard = nullptr;
@@ -83,6 +84,7 @@ void bind(const py::dict& a) {
   take(lib.classify, a, "kd_classify");
   take(lib.attn_fwd, a, "kd_attn_fwd");
   take(lib.attn_bwd, a, "kd_attn_bwd");
+  take(lib.attn_bwd_hadamard, a, "kd_attn_bwd_hadamard");
   take(lib.attn_fwd_f32, a, "kd_attn_fwd_f32");
   take(lib.attn_bwd_f32, a, "kd_attn_bwd_f32");
   take(lib.hadamard, a, "kd_hadamard");
@@ -456,10 +458,12 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Ten
 }
 
 // f32: of a float32 call; dO may be float32, and dQ, dK and dV are.
+// signs: q and k are transforms with these, and dQ and dK are wanted of what they were made from (not deterministic).
 // `phases` selects a part of the backward (kd_attn_params.bwd_phases); defined tensors among dq .. dq_acc are reused.
 std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const Tensor& o, const Tensor& lse,
                                             const Tensor& d_o_, const PlanPtr& plan, double sm_scale, int phases, Tensor dq, Tensor dk,
-                                            Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic, bool f32 = false) {
+                                            Tensor dv, Tensor delta, Tensor dq_acc, bool like_input, bool deterministic, bool f32 = false,
+                                            const float* signs = nullptr) {
   const Tensor q = usable(q_), k = usable(k_), v = usable(v_);
   kd_attn_f32 f{};
   Tensor d_o;
@@ -495,7 +499,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   p.plan_ready = plan->ready_on(stream) ? 1 : 0;
-  check(f32 ? lib.attn_bwd_f32(&p, &f, stream) : lib.attn_bwd(&p, stream));
+  check(f32 ? lib.attn_bwd_f32(&p, &f, stream) : signs != nullptr ? lib.attn_bwd_hadamard(&p, signs, stream) : lib.attn_bwd(&p, stream));
   plan->after_launch();
   return {dq, dk, dv};
 }
@@ -572,8 +576,10 @@ struct AttentionBackward : torch::autograd::Node {
              d_o.sizes(), " on ", d_o.device());
     if (grads[0].defined()) d_o = d_o.to(widen ? at::kFloat : to.scalar_type());
     if (widen && !direct) d_o = cast({d_o}, at::kHalf)[0];
-    auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic, direct);
-    if (signs.has_value()) {
+    const bool with_gradients = signs.has_value() && !opt.deterministic;
+    auto [dq, dk, dv] = backward(tq, tk, tv, to, tlse, d_o, plan, opt.sm_scale, 0, {}, {}, {}, {}, {}, opt.like_input, opt.deterministic, direct,
+                                 with_gradients ? signs->data_ptr<float>() : nullptr);
+    if (signs.has_value() && !with_gradients) {
       // y = x diag(s) W / sqrt(D) with W symmetric, so dx = dy W / sqrt(D) diag(s)
       dq = hadamard(dq, signs, true);
       dk = hadamard(dk, signs, true);

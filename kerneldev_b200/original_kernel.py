@@ -94,7 +94,8 @@ def generate_hadamard_signs(n_heads: int, head_dim: int, seed: int = 0, device="
 def _check_signs(signs: torch.Tensor, n_heads: int, head_dim: int, device) -> torch.Tensor:
     if signs.shape != (n_heads, head_dim):
         raise ValueError("signs must have shape (heads, head_dim)")
-    return signs.to(device=device, dtype=torch.float32).contiguous()
+    signs = signs.to(device=device, dtype=torch.float32).contiguous()
+    return signs if signs.data_ptr() % 16 == 0 else signs.clone()   # the kernels read four at a time
 
 
 def hadamard_transform(x: torch.Tensor, signs: torch.Tensor | None = None) -> torch.Tensor:

@@ -70,6 +70,33 @@ def test_padding_is_left_out_of_delta_and_conversion(T, lens, D, dtype):
         assert not g.cpu()[beyond.expand_as(g)].any()
 
 
+# dQ and dK of transformed Q and K, transformed back by the last pass of the fused backward, against the transform's own backward. T and lens at the
+# edges of its blocks (128 rows at head dim 16, 64 above)
+@pytest.mark.parametrize("D,dtype", [(16, torch.bfloat16), (32, torch.float16), (64, torch.bfloat16), (128, torch.float16)])
+@pytest.mark.parametrize("T,lens", [(63, (63, 1, 0)), (129, (64, 129, 65)), (200, (128, 127, 193))])
+def test_gradients_of_transformed_tensors(T, lens, D, dtype):
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import flash_attention, generate_hadamard_signs, hadamard_transform
+    B, H = len(lens), 3
+    q, k, v, do = rand_inputs(B, H, T, D, dtype, T + D, DEV)
+    lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    signs = torch.cat([torch.ones(1, device=DEV), generate_hadamard_signs(H, D).flatten()])[1:].view(H, D)   # not on 16 bytes
+    for x in (q, k, v):
+        x.requires_grad_()
+    got = torch.autograd.grad(flash_attention(q, k, v, lens=lens, hadamard_signs=signs), (q, k, v), do)
+    qt, kt = hadamard_transform(q, signs), hadamard_transform(k, signs)
+    o = flash_attention(qt, kt, v, lens=lens)
+    dqt, = torch.autograd.grad(o, qt, do, retain_graph=True)
+    want = torch.autograd.grad(o, (q, k, v), do)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    # A rounding to p bits moves a number by u = 2^-p of it at most (bfloat16 p = 8, float16 p = 11). The second path rounds dQ before the
+    # transform as well, which is orthogonal: the elements' errors move a result by u times the row's 2-norm at most. Both round the result, by u
+    # of it each; 1.01 for the products of these, and for the sums of up to two key tiles, which may come in another order (1e-6)
+    u = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    bound = 1.01 * u * (dqt.float().norm(dim=-1, keepdim=True) + 2 * want[0].float().abs()) + 1e-6
+    assert bool(((got[0].float() - want[0].float()).abs() <= bound).all())
+
+
 # More items than SMs, so that CTAs take several one after the other; chunks of heads of equal and (at T = 1280) unequal size. `lens` makes runs of empty items longer than the ring of
 # item headers between items with work (both tile widths; an odd number of query tiles; a last tile of 1 and of 127 tokens)
 @pytest.mark.parametrize("deterministic", [False, True])
