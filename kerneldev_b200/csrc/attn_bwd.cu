@@ -181,7 +181,7 @@ __device__ __forceinline__ void bwd_init(BwdShared<C>& sh) {   // one thread
 template <typename C>
 __device__ __forceinline__ bool bwd_header(BwdShared<C>& sh, int k, uint32_t site, int4& it) {
   const int slot = k % C::NITEM;
-  if (!mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, site)) return false;
+  if (!mbar_wait<true>(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, site)) return false;
   it = sh.items[slot];
   mbar_arrive(smem_u32(&sh.item_empty[slot]));
   return true;
@@ -208,7 +208,7 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
     tma_prefetch_desc(&tmRing1);
   }
   auto wait = [&](const uint64_t& bar, uint32_t parity, uint32_t site) -> bool {
-    return __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar), parity, &sh.abortf, site));
+    return __all_sync(0xffffffffu, mbar_wait<true>(smem_u32(&bar), parity, &sh.abortf, site));
   };
   const uint32_t below = (1u << lane) - 1u;
   uint32_t lst[4];   // the decoded item's list, 32 entries per register: tile | class << 8, zeros where an entry is another tile's
@@ -365,7 +365,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int k = 0; ok && bwd_header<C>(sh, k, W_Q_ITEMFULL, it) && it.w >= 0; ++k) {
         if (it.w == 0) continue;
         const int U = 2 * it.w, fb = item % C::NFIX;
-        ok = mbar_wait(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_Q_FIXFULL);
+        ok = mbar_wait<true>(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_Q_FIXFULL);
         ++item;
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // dO or Q
@@ -382,11 +382,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_Q_M2ISSUED);
+            ok = mbar_wait<true>(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_Q_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its K and V tiles must have landed
-            ok = mbar_wait(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_Q_RINGFULL);
+            ok = mbar_wait<true>(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_Q_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -413,7 +413,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         if (it.w == 0) continue;
         const int U = 2 * it.w;
         if (item++ > 0) {   // the previous item's dQ must have been read out of the accumulator
-          ok = mbar_wait(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_Q_ACCFREE);
+          ok = mbar_wait<true>(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_Q_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -428,7 +428,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             bdesc[kk] = desc64(kb + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_Q_PFULL);
+          ok = mbar_wait<true>(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_Q_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           mma_ts64_p(tAcc, aop[0], bdesc[0], idesc_m2, u > 0 ? 1u : 0u);
@@ -475,7 +475,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint16_t* list = lists;
     auto open_item = [&](int k) -> bool {
       const int slot = k % C::NITEM;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_Q_ITEMFULL))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait<true>(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_Q_ITEMFULL))) return false;
       it = uniform(sh.items[slot]);
       if (it.w < 0) return false;
       list = lists + slot * 128;
@@ -516,7 +516,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           fetch_words(ent_next);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_Q_SFULL);
+        ok = mbar_wait<true>(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_Q_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -562,7 +562,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       have = open_item(k + 1);
       // epilogue of this item: warpgroup g stores EC columns of dQ from column g * EC
       if (na > 0) {
-        ok = mbar_wait(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_Q_ACCFULL);
+        ok = mbar_wait<true>(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_Q_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }
@@ -673,7 +673,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       for (int k = 0; ok && bwd_header<C>(sh, k, W_K_ITEMFULL, it) && it.w >= 0; ++k) {
         if (it.w == 0) continue;
         const int U = 2 * it.w, fb = item % C::NFIX;
-        ok = mbar_wait(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_K_FIXFULL);
+        ok = mbar_wait<true>(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_K_FIXFULL);
         ++item;
         if (!ok) break;
         const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // V or K
@@ -690,11 +690,11 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
           const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
           if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_K_M2ISSUED);
+            ok = mbar_wait<true>(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_K_M2ISSUED);
             if (!ok) break;
           }
           if (i == 0) {      // first unit of a new entry: its Q and dO tiles must have landed
-            ok = mbar_wait(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_K_RINGFULL);
+            ok = mbar_wait<true>(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_K_RINGFULL);
             if (!ok) break;
           }
           tc_fence_after_sync();
@@ -721,7 +721,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (it.w == 0) continue;
         const int U = 2 * it.w;
         if (item++ > 0) {   // the previous item's dK and dV must have been read out of the accumulators
-          ok = mbar_wait(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_K_ACCFREE);
+          ok = mbar_wait<true>(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_K_ACCFREE);
           if (!ok) break;
         }
         for (int u = 0; u < U && ok; ++u) {
@@ -739,7 +739,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             bdo[kk] = desc64(dob + koff_mnmajor(kk), hi);
             aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
           }
-          ok = mbar_wait(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_K_PFULL);
+          ok = mbar_wait<true>(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_K_PFULL);
           if (!ok) break;
           tc_fence_after_sync();
           // dV += P^T_u dO_u   (P^T_u on top of S^T_u)
@@ -802,7 +802,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint16_t* list = lists;
     auto open_item = [&](int k) -> bool {
       const int slot = k % C::NITEM;
-      if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_K_ITEMFULL))) return false;
+      if (!__all_sync(0xffffffffu, mbar_wait<true>(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_K_ITEMFULL))) return false;
       it = uniform(sh.items[slot]);
       if (it.w < 0) return false;
       list = lists + slot * 128;
@@ -842,7 +842,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           prefetch(ent_next, now.y);
         }
         const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_K_SFULL);
+        ok = mbar_wait<true>(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_K_SFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after_sync();
@@ -910,7 +910,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int b = now.x, h = now.y, kj = now.z * KD_TILE + row;
       // epilogue of this item: warpgroup g stores EC columns of dK and dV from column g * EC
       if (n > 0) {
-        ok = mbar_wait(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_K_ACCFULL);
+        ok = mbar_wait<true>(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_K_ACCFULL);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
       }

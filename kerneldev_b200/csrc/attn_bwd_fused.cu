@@ -25,7 +25,12 @@
 //    through stmatrix without bank conflicts. Arithmetic on column pairs uses the packed f32x2 instructions.
 //  * The instruction cache: sixteen warps in six roles run different loops at the same time. With the waits' time-out
 //    code inlined and more unrolling this kernel was 120 KB and took 5,600 cycles a tile (a loop back-edge cost 580);
-//    at 75 KB the same schedule took 3,600. Loops of the issuing and dQ warps are therefore rolled where they can be.
+//    at 75 KB the same schedule took 3,600. Loops of the issuing and dQ warps are therefore rolled where they can be, and
+//    the waits are as short as they can be (mbar_wait_short): a first test ahead of the loop, a look at the flag that
+//    another role has given up, and the raising of that flag at each wait made 64 KB at HD = 64 where it is 52 now; without
+//    them the backward of 16 x 16 x 4096 x 64 hierarchical takes 954 us where it took 1093, of 8 x 16 x 2048 x 64 causal 278
+//    where it took 301, of 8 x 16 x 2048 x 128 causal 485 where it took 492. Suspending the waiting threads for longer (20 us)
+//    gives 2 % of it back, the test ahead of the loop 4 %.
 //  * The products are issued by whole warps with warp-uniform operands (mma_ss_uniform).
 //
 // Schedule at HD = 64. The compute warps form P^T of tile t and dS^T of tile t - 1 in one instruction stream (see there).
@@ -188,9 +193,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // overlaps another need not have cleaned). Not so delta, the zeros of the dQ scratch or of a float32 dQ, and dO, which in a float32 call
   // the delta kernel rounds to 16 bits.
   if (!fa.after_delta) pdl_wait();
+  // The site of this warp's wait that ran out, 0 while none has. There is no wait after it: every role ends at its first, with
+  // its copies drained, and raises the flag where all roles meet. All waits of this kernel are such waits (there is no named
+  // barrier), so a role whose partner has ended waits for its own limit and ends too.
+  uint32_t gave_up = 0u;
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
   auto wait = [&](int i, uint32_t parity, uint32_t site) -> bool {
-    return __all_sync(0xffffffffu, mbar_wait(bar(i), parity, abortf, site));
+    const bool there = __all_sync(0xffffffffu, mbar_wait_short(bar(i), parity));
+    if (!there) gave_up = site;
+    return there;
   };
   // two barriers of which both are complete as a rule: their tests overlap
   auto wait2 = [&](int i, uint32_t pi, uint32_t site_i, int j, uint32_t pj, uint32_t site_j) -> bool {
@@ -377,7 +388,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         it = nx;
       }
-      if (lane == 0 && abortf->v != 0) {   // let the copies in flight land before the CTA exits
+      if (lane == 0 && (gave_up != 0u || abortf->v != 0u)) {   // let the copies in flight land before the CTA exits
         for (int f = max(0, k_loads - C::NK); f < k_loads; ++f) drain_wait(bar(C::B_KFULL + f % C::NK), (f / C::NK) & 1);
         if (k > 0) drain_wait(bar(C::B_VFULL), 0);
         for (int f = max(0, q_tiles - C::QS); f < q_tiles; ++f) drain_wait(bar(C::B_QFULL + f % C::QS), (f / C::QS) & 1);
@@ -469,7 +480,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               e = 0;
             }
           }
-          if (lane == 0 && abortf->v != 0 && v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
+          if (lane == 0 && (gave_up != 0u || abortf->v != 0u) && v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
         } else if (warp == 3) {
           // ---- dV, a half at a time ----
           int do_stage = 0;
@@ -636,7 +647,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           ++m;
         }
-        if (lane == 0 && abortf->v != 0) {   // let this warp's own copies in flight land before the CTA exits
+        if (lane == 0 && (gave_up != 0u || abortf->v != 0u)) {   // let this warp's own copies in flight land before the CTA exits
           if (k_loads > 1) drain_wait(bar(C::B_KFULL), (k_loads - 1) & 1);
           if (v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
         }
@@ -1051,6 +1062,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (lane == 0) bulk_wait_group0();
   }
 
+  if (gave_up != 0u) raise_abort(abortf, gave_up);
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) tmem_dealloc(0, 512);
