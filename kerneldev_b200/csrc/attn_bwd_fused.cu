@@ -92,7 +92,9 @@ struct FusedCfg {
   // per Q stage: LSE and delta of the 128 queries; HD = 64: the visibility words of a PARTIAL tile, [32 keys][query] (HD = 128 has no room: its
   // compute warps fetch them); the tile's list entry (4 words with padding)
   static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + (HD == 64 ? static_cast<int>(KD_WORDS) : 0), SIDE_WORDS = SIDE_ENT + 4;
-  static constexpr int SMEM_SIDE = SMEM_STG + 4 * 2 * 4096;
+  static constexpr int SMEM_ZERO = SMEM_STG + 4 * 2 * 4096;   // HD = 64: a box of zeros, what items without entries are written from
+  static constexpr int ZERO_BYTES = (HD == 64) ? 4096 : 0;
+  static constexpr int SMEM_SIDE = SMEM_ZERO + ZERO_BYTES;
   static constexpr int NITEM = 4;                    // ring of item headers
   static constexpr int SMEM_ITEM = SMEM_SIDE + QS * SIDE_WORDS * 4;   // NITEM x {batch, head, key tile | first entry << 16, entries}
   static constexpr int SMEM_CLC = SMEM_ITEM + NITEM * 16;             // response of a cancellation
@@ -240,6 +242,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tma_prefetch_desc(&tmK);
         tma_prefetch_desc(&tmV);
       }
+      for (int i = lane; i < C::ZERO_BYTES / 16; i += 32) st_shared_v4(s0 + C::SMEM_ZERO + 16 * i, 0u, 0u, 0u, 0u);
+      if (C::ZERO_BYTES > 0) fence_proxy_async_smem();
+      __syncwarp();
       int q_tiles = 0, do_tiles = 0, k_loads = 0, k = 0;   // Q / dO / K tiles requested and items published so far
       bool ok = true, pending = false;
       // decodes item number `idx` of the launch
@@ -269,13 +274,26 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // dK = dV = 0 for an item without entries
       auto write_zeros = [&](const int4& z) {
         using Out = std::conditional_t<kF32, float, uint16_t>;
+        if constexpr (HD == 64) {
+          // Items without entries come last and nothing hides them there: 14,500 of the 87,000 cycles of a CTA of hierarchical 4 x 16 x 2048
+          // x 64 lie behind its last tile. So they leave through the copy engine, a lane per 32 rows, and cost this warp no more than
+          // the look-up (stores by the lanes before: that backward 71.1 -> 67.8 us, 8 x 16 x 2048 x 64 141.7 -> 132.5, 16 x 16 x 4096 x 64
+          // 978 -> 947, 8 x 8 x 1000 x 64 29.4 -> 28.5). At HD = 128 there is no room for the box; made in a Q stage that
+          // is empty, it gives 1 to 4 % of longer hierarchical calls, and 3 x 6 x 1357 x 80 is 3.5 % slower for the longer code.
+          if (lane < 4 && (z.z & 0xFFFF) * KD_TILE + lane * 32 < a.T) {   // rows at or beyond T and columns at or beyond d_real are not written
+            for (int col = 0; col < a.d_real; col += 128 / static_cast<int>(sizeof(Out))) {
+              tma_store_4d(&tmDK, s0 + C::SMEM_ZERO, col, (z.z & 0xFFFF) * KD_TILE + lane * 32, z.y, z.x);
+              tma_store_4d(&tmDV, s0 + C::SMEM_ZERO, col, (z.z & 0xFFFF) * KD_TILE + lane * 32, z.y, z.x);
+            }
+            bulk_commit_group();
+          }
+          return;
+        }
         constexpr int per = 16 / sizeof(Out);   // elements of a 16-byte chunk
         constexpr int CPR = HD / per;           // chunks of a tile's row
         const int row0 = (z.z & 0xFFFF) * KD_TILE, rows = min(KD_TILE, a.T - row0);
         Out* dk = reinterpret_cast<Out*>(a.dk) + (size_t)z.x * a.dk_sb + (size_t)z.y * a.dk_sh;
         Out* dv = reinterpret_cast<Out*>(a.dv) + (size_t)z.x * a.dv_sb + (size_t)z.y * a.dv_sh;
-        // (Items without entries come last, and nothing hides them there. With a division by the real width for each chunk: hierarchical
-        // 4 x 16 x 2048 x 64 88.5 us, 87.5 now, 8 x 16 x 2048 x 64 163 -> 161, 8 x 8 x 1000 x 64 33.4 -> 32.5.)
         for (int i = lane; i < rows * CPR; i += 32) {
           const int r = i / CPR, c = i % CPR * per;
           if (c >= a.d_real) continue;
@@ -388,6 +406,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         it = nx;
       }
+      if (C::ZERO_BYTES > 0) bulk_wait_group_read0();   // the box of zeros has been read
       if (lane == 0 && (gave_up != 0u || abortf->v != 0u)) {   // let the copies in flight land before the CTA exits
         for (int f = max(0, k_loads - C::NK); f < k_loads; ++f) drain_wait(bar(C::B_KFULL + f % C::NK), (f / C::NK) & 1);
         if (k > 0) drain_wait(bar(C::B_VFULL), 0);

@@ -70,6 +70,37 @@ def test_padding_is_left_out_of_delta_and_conversion(T, lens, D, dtype):
         assert not g.cpu()[beyond.expand_as(g)].any()
 
 
+# Key tiles that no query sees: their dK and dV are written from a box of 32 zeroed rows. Every element of theirs and nothing beside it: ragged last
+# boxes and widths below the tile's, in gradients that are slices of a wider tensor
+@pytest.mark.parametrize("D", [16, 48, 64])
+@pytest.mark.parametrize("T,lens", [(129, (128, 1)), (161, (0, 100)), (287, (129, 60)), (384, (3, 256))])
+def test_empty_key_tiles_are_written_as_zeros(T, lens, D):
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import flash_attention
+    from kerneldev_b200.original_kernel import _backward, _forward
+    from kerneldev_b200.plan import AttentionPlan
+    B, H = len(lens), 3
+    q, k, v, do = rand_inputs(B, H, T, D, torch.bfloat16, T + D, DEV)
+    lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    beyond = (torch.arange(T, device=DEV)[None, None, :, None] >= (lens[:, None, None, None] + 127) // 128 * 128).expand(B, H, T, D)
+    plan = AttentionPlan(B, T, DEV, lens=lens, causal=True)
+    o, lse = _forward(q, k, v, plan, D ** -0.5)
+    wide = [torch.full((B, T, H, D + 16), float("nan"), device=DEV, dtype=q.dtype) for _ in range(3)]
+    bufs = [w[..., 8:8 + D].transpose(1, 2) for w in wide]
+    bufs += [torch.full((B, H, T, *w), float("nan"), device=DEV) for w in ((), (64,))]
+    got = _backward(q, k, v, o, lse, do, plan, D ** -0.5, 0, bufs)
+    for g, w in zip(got, wide):
+        assert g.data_ptr() == w[..., 8:].data_ptr() and not g[beyond].any()
+        assert bool(w[..., :8].isnan().all()) and bool(w[..., 8 + D:].isnan().all())
+    # a float32 call, whose boxes are of 32 columns: freed memory that its gradients are likely to be made in holds no zeros
+    x32 = [x.float().requires_grad_() for x in (q, k, v)]
+    out = flash_attention(*x32, lens=lens)
+    spoilt = [torch.full((B, H, T, D), float("nan"), device=DEV) for _ in range(8)]
+    del spoilt
+    for g in torch.autograd.grad(out, x32, do.float()):
+        assert not g[beyond].any() and not g.isnan().any()
+
+
 # dQ and dK of transformed Q and K, transformed back by the last pass of the fused backward, against the transform's own backward. T and lens at the
 # edges of its blocks (128 rows at head dim 16, 64 above)
 @pytest.mark.parametrize("D,dtype", [(16, torch.bfloat16), (32, torch.float16), (64, torch.bfloat16), (128, torch.float16)])
