@@ -34,7 +34,7 @@
 //  * The products are issued by whole warps with warp-uniform operands (mma_ss_uniform).
 //
 // Schedule at HD = 64. The compute warps form P^T of tile t and dS^T of tile t - 1 in one instruction stream (see there).
-//   warp 1   S^T(t), dP^T(t - 1) as soon as S^T(t - 1) and dP^T(t - 2) have been loaded; also requests the next item's V
+//   warp 1   S^T(t), dP^T(t - 1) as soon as S^T(t - 1) and dP^T(t - 2) have been loaded
 //   warp 3   dV += P^T(t) dO, a half of 64 queries at a time
 //   warp 2   dK += dS^T(t - 1) Q by halves, dQ(t - 1)
 // TMEM: S^T 128, dP^T 128, dV 64, dK 64, dQ 64, P^T 64 columns.
@@ -45,8 +45,9 @@
 //
 // Work items. An item is one (batch, head, key tile). The grid has a CTA per item, but a CTA that is running takes
 // further items by cancelling CTAs that have not been launched yet (clusterlaunchcontrol) and works on them without
-// draining its pipeline: the rings of Q and dO tiles run on into the next item, K has two buffers at HD = 64
-// (shared memory holds one at HD = 128), and dK and dV of the finished item leave through the dQ warps while the
+// draining its pipeline: the rings of Q and dO tiles run on into the next item, K and V have two buffers at HD = 64
+// (shared memory holds one at HD = 128; at HD = 64 the second V buffer takes the place of half of the dQ staging, which costs
+// nothing), and dK and dV of the finished item leave through the dQ warps while the
 // next item's first products run. Starting a CTA costs some 12,000 cycles (launch, TMEM, first loads, pipeline fill,
 // drain), and a (batch, head, key tile) has around ten tiles.
 // Items are numbered in chunks of heads whose scratch and operands fit L2 together (ItemOrder), inside a
@@ -84,15 +85,17 @@ struct FusedCfg {
   static constexpr int QS = (HD == 64) ? 4 : 2;      // ring stages of Q tiles: held from S^T of a tile to its dK
   static constexpr int OS = (HD == 64) ? 2 : 1;      // ring stages of dO tiles: held from dP^T to dV
   static constexpr int SMEM_K = 0;
+  static constexpr int NV = NK;                      // V buffers, as K's
   static constexpr int SMEM_V = SMEM_K + NK * TILE_BYTES;
-  static constexpr int SMEM_Q = SMEM_V + TILE_BYTES;
+  static constexpr int SMEM_Q = SMEM_V + NV * TILE_BYTES;
   static constexpr int SMEM_DO = SMEM_Q + QS * TILE_BYTES;
   static constexpr int SMEM_DS = SMEM_DO + OS * TILE_BYTES;   // dS^T: two blocks [128 keys][64 queries]
-  static constexpr int SMEM_STG = SMEM_DS + 2 * 16384;        // dQ staging: per dQ warp two boxes [32 rows][32 floats]
+  static constexpr int SMEM_STG = SMEM_DS + 2 * 16384;        // dQ staging: per dQ warp NSTG boxes [32 rows][32 floats]
+  static constexpr int NSTG = (HD == 64) ? 1 : 2;
   // per Q stage: LSE and delta of the 128 queries; HD = 64: the visibility words of a PARTIAL tile, [32 keys][query] (HD = 128 has no room: its
   // compute warps fetch them); the tile's list entry (4 words with padding)
   static constexpr int SIDE_BITS = 2 * KD_TILE, SIDE_ENT = SIDE_BITS + (HD == 64 ? static_cast<int>(KD_WORDS) : 0), SIDE_WORDS = SIDE_ENT + 4;
-  static constexpr int SMEM_ZERO = SMEM_STG + 4 * 2 * 4096;   // HD = 64: a box of zeros, what items without entries are written from
+  static constexpr int SMEM_ZERO = SMEM_STG + 4 * NSTG * 4096;   // HD = 64: a box of zeros, what items without entries are written from
   static constexpr int ZERO_BYTES = (HD == 64) ? 4096 : 0;
   static constexpr int SMEM_SIDE = SMEM_ZERO + ZERO_BYTES;
   static constexpr int NITEM = 4;                    // ring of item headers
@@ -101,7 +104,7 @@ struct FusedCfg {
   static constexpr int SMEM_BAR = SMEM_CLC + 16;
   // barriers (8 bytes each)
   static constexpr int NH = (HD == 64) ? 2 : 1;      // halves of 64 queries with barriers of their own
-  static constexpr int B_KFULL = 0, B_KEMPTY = B_KFULL + NK, B_VFULL = B_KEMPTY + NK, B_VEMPTY = B_VFULL + 1, B_QFULL = B_VEMPTY + 1,
+  static constexpr int B_KFULL = 0, B_KEMPTY = B_KFULL + NK, B_VFULL = B_KEMPTY + NK, B_VEMPTY = B_VFULL + NV, B_QFULL = B_VEMPTY + NV,
                        B_QEMPTY = B_QFULL + QS, B_DOFULL = B_QEMPTY + QS, B_DOEMPTY = B_DOFULL + OS, B_SFULL = B_DOEMPTY + OS,
                        B_SFREE = B_SFULL + NH, B_PFULL = B_SFREE + NH, B_PFREE = B_PFULL + NH, B_DPFULL = B_PFREE + NH,
                        B_DSFULL = B_DPFULL + 1, B_DSFREE = B_DSFULL + 1, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
@@ -245,19 +248,20 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int i = lane; i < C::ZERO_BYTES / 16; i += 32) st_shared_v4(s0 + C::SMEM_ZERO + 16 * i, 0u, 0u, 0u, 0u);
       if (C::ZERO_BYTES > 0) fence_proxy_async_smem();
       __syncwarp();
-      int q_tiles = 0, do_tiles = 0, k_loads = 0, k = 0;   // Q / dO / K tiles requested and items published so far
+      int q_tiles = 0, do_tiles = 0, k_loads = 0, v_loads = 0, k = 0;   // Q / dO / K tiles requested and items published so far
       bool ok = true, pending = false;
       // decodes item number `idx` of the launch
-      auto decode = [&](int idx) -> int4 {
+      auto find_tile = [&](int idx, int4& it) {
         int bh, rank;
         fa.order_of.decode(idx, a.NT, bh, rank);
-        int4 it;
         it.x = bh / a.H;
         it.y = bh - it.x * a.H;
-        const int kt = __ldcg(a.order + ((size_t)it.x * 3 + 2) * a.NT + rank);   // longest lists first
-        it.w = __ldcg(a.bwd_cnt + it.x * a.NT + kt);
-        it.z = kt | (static_cast<int>(__ldcg(a.bwd_list + ((size_t)it.x * a.NT + kt) * a.NT)) << 16);
-        return it;
+        it.z = __ldcg(a.order + ((size_t)it.x * 3 + 2) * a.NT + rank);   // longest lists first
+        it.w = 0;
+      };
+      auto find_list = [&](int4& it, int& first) {
+        first = __ldcg(a.bwd_list + ((size_t)it.x * a.NT + it.z) * a.NT);
+        it.w = __ldcg(a.bwd_cnt + it.x * a.NT + it.z);
       };
       int asked = 0;   // cancellations asked for
       // The next item is asked for three tiles before the end of this one (for a shorter one: when it is taken), which hides the
@@ -302,24 +306,49 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       };
       // the answer (nx.w < 0: there is no further item)
-      auto take_next = [&](int4& nx) -> bool {
+      // Takes the next item in three steps between the loads of this one's last tiles, which hide the look-ups (a round trip to L2 each):
+      // the answer and the key tile (nx.w < 0: there is no further item), its list's length and first entry, and the header. At HD = 64
+      // a tile lasts no longer than these: taken in one step ahead of the last tile's Q, that tile's S^T came 1,100 cycles late and the
+      // next item's first, whose K was requested behind it, 600. With the steps, the next item's header, K and V ahead of the last
+      // dO, and a second V buffer (one: the next item's second S^T waits for V, 600 cycles) backward us: causal 8 x 16 x 2048 x 64 280 -> 274,
+      // 8 x 16 x 1000 x 64 90.2 -> 88.8, hierarchical 8 x 16 x 2048 x 64 132.2 -> 131.5, 16 x 16 x 4096 x 64 940 -> 937. Level at HD = 128.
+      int first_entry = 0;
+      auto next_tile = [&](int4& nx) -> bool {
         if (!wait(C::B_CLC, (asked - 1) & 1, W_U_CLC)) return false;
         pending = false;
         const int idx = clc_first_ctaid_x(s0 + C::SMEM_CLC);
         __syncwarp();   // every lane has read the response that the next request overwrites
         nx.w = -1;
-        if (idx >= 0) {
-          nx = decode(idx);
-          if (nx.w <= 2) ask();
-        }
+        if (idx >= 0) find_tile(idx, nx);
         return true;
       };
-      int4 it = decode(blockIdx.x);
-      if (it.w <= 2) ask();
+      auto next_list = [&](int4& nx) {
+        if (nx.w >= 0) find_list(nx, first_entry);
+      };
+      auto next_header = [&](int4& nx) {
+        nx.z |= first_entry << 16;
+        if (nx.w >= 0 && nx.w <= 2) ask();
+      };
+      int4 it;
+      find_tile(blockIdx.x, it);
+      next_list(it);
+      next_header(it);
       int qs = 0, os = 0;
       uint32_t q_parity = 1u, do_parity = 1u;   // of the stages' "empty" phases
+      // dO of a tile is requested after its Q; at HD = 64 that of an item's last tile behind the next item's header, K and V, none of which waits for it
+      int do_tile = -1, do_h = 0, do_b = 0;
+      auto load_do = [&]() -> bool {
+        if (do_tile < 0) return true;
+        if (!wait(C::B_DOEMPTY + os, do_parity, W_U_DOEMPTY)) return false;
+        if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, do_tile, do_h, do_b);   // (behind pdl_wait())
+        ++do_tiles;
+        if (++os == C::OS) { os = 0; do_parity ^= 1u; }
+        do_tile = -1;
+        return true;
+      };
       while (ok) {
         const int b = it.x, h = it.y, kt = it.z & 0xFFFF, n = it.w;
+        if (HD == 64 && n <= 0 && !(ok = load_do())) break;
         if (n != 0) {   // (no other warp hears of an item without entries)
         const int slot = k % C::NITEM;
         if (!(ok = wait(C::B_ITEMEMPTY + slot, ((k / C::NITEM) & 1) ^ 1, W_U_ITEMEMPTY))) break;
@@ -346,12 +375,17 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if (lane == 0) load_tile(&tmK, sK + (k % C::NK) * TILE, C::B_KFULL + k % C::NK, kt, h, b);
           ++k_loads;
         }
+        if (HD == 64 || k == 0) {
+          if (!(ok = wait(C::B_VEMPTY + k % C::NV, ((k / C::NV) & 1) ^ 1, W_U_VEMPTY))) break;
+          if (lane == 0) load_tile(&tmV, sV + (k % C::NV) * TILE, C::B_VFULL + k % C::NV, kt, h, b);
+          ++v_loads;
+        }
         if (k == 0) {
-          if (lane == 0) load_tile(&tmV, sV, C::B_VFULL, kt, h, b);
           pdl_wait();   // delta and dO are read from here on
           pdl_launch_dependents();
         }
         ++k;
+        if (HD == 64 && !(ok = load_do())) break;
         }
         const uint16_t* list = a.bwd_list + ((size_t)b * a.NT + kt) * a.NT;
         const size_t row = ((size_t)b * a.H + h) * a.T;
@@ -362,7 +396,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
         for (int e = 0; e < max(n, 1); ++e) {
           if (n > 2 && e == n - 3) ask();
-          if (e >= n - 1 && !(ok = take_next(nx))) break;   // its list is looked up while this item's last tile waits for a slot
+          const bool last = e >= n - 1;
+          if ((HD == 64 && n > 2 ? e == n - 2 : last) && !(ok = next_tile(nx))) break;
+          if (last) next_list(nx);
+          if (HD == 128 ? last : n == 0) next_header(nx);
           if (n == 0) {
             write_zeros(it);
             break;
@@ -399,17 +436,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           cp_async_mbar_arrive(bar(C::B_QFULL + qs));
           ++q_tiles;
           if (++qs == C::QS) { qs = 0; q_parity ^= 1u; }
-          if (!(ok = wait(C::B_DOEMPTY + os, do_parity, W_U_DOEMPTY))) break;
-          if (lane == 0) load_tile(&tmDO, sDO + os * TILE, C::B_DOFULL + os, qt, h, b);   // (behind pdl_wait())
-          ++do_tiles;
-          if (++os == C::OS) { os = 0; do_parity ^= 1u; }
+          do_tile = qt;
+          do_h = h;
+          do_b = b;
+          if (HD == 64 && last) next_header(nx);
+          if ((HD == 128 || !last) && !(ok = load_do())) break;
         }
         it = nx;
       }
       if (C::ZERO_BYTES > 0) bulk_wait_group_read0();   // the box of zeros has been read
       if (lane == 0 && (gave_up != 0u || abortf->v != 0u)) {   // let the copies in flight land before the CTA exits
         for (int f = max(0, k_loads - C::NK); f < k_loads; ++f) drain_wait(bar(C::B_KFULL + f % C::NK), (f / C::NK) & 1);
-        if (k > 0) drain_wait(bar(C::B_VFULL), 0);
+        for (int f = max(0, v_loads - C::NV); f < v_loads; ++f) drain_wait(bar(C::B_VFULL + f % C::NV), (f / C::NV) & 1);
         for (int f = max(0, q_tiles - C::QS); f < q_tiles; ++f) drain_wait(bar(C::B_QFULL + f % C::QS), (f / C::QS) & 1);
         for (int f = max(0, do_tiles - C::OS); f < do_tiles; ++f) drain_wait(bar(C::B_DOFULL + f % C::OS), (f / C::OS) & 1);
         if (pending) drain_wait(bar(C::B_CLC), (asked - 1) & 1);
@@ -456,7 +494,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           uint32_t q_parity = 0, do_parity = 0;
           advance();
           bool p_first = false, p_last = false;   // tile t - 1 is its item's first / last
-          int e = 0, v_loads = 1;
+          int e = 0;
           while (ok) {
             const bool s_there = have, dp_there = t > 0;
             if (!s_there && !dp_there) break;
@@ -465,14 +503,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (e == 0 && !(ok = wait(C::B_KFULL + (m & 1), (m >> 1) & 1, W_U_KFULL))) break;
               if (!(ok = wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL))) break;
             }
-            if (dp_there) {   // V of tile t - 1's item: waited for at the item's first dP^T
-              if (p_first && !(ok = wait(C::B_VFULL, ((s_there && e > 0) ? m : m - 1) & 1, W_U_VFULL))) break;
+            const int mp = (s_there && e > 0) ? m : m - 1;   // tile t - 1's item
+            if (dp_there) {   // its V is waited for at the item's first dP^T
+              if (p_first && !(ok = wait(C::B_VFULL + (mp & 1), (mp >> 1) & 1, W_U_VFULL))) break;
               if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
             }
             if (dp_there && !(ok = wait2(C::B_SFREE, (t - 1) & 1, W_U_SFREE, C::B_SFREE + 1, (t - 1) & 1, W_U_SFREE))) break;
             tc_fence_after_sync();
             if (s_there) product_kmajor(C::TM_S, lo_k0 + (m & 1) * T16, lo_q0 + q_stage * T16);
-            if (dp_there) product_kmajor(C::TM_DP, lo_v, lo_do0 + do_stage * T16);
+            if (dp_there) product_kmajor(C::TM_DP, lo_v + (mp & 1) * T16, lo_do0 + do_stage * T16);
             commit_uniform(bar(C::B_SFULL));
             commit_uniform(bar(C::B_SFULL + 1));
             if (dp_there) {
@@ -480,14 +519,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
             }
             if (!s_there) break;   // that was the last dP^T
-            if (dp_there && p_last) {
-              // That was V's last reader in its item: the next item's V goes into the same buffer. This warp has nothing else to
-              // do before the next S^T can be formed, and the load has an iteration to land.
-              commit_uniform(bar(C::B_VEMPTY));
-              if (!(ok = wait(C::B_VEMPTY, (m - 1) & 1, W_U_VEMPTY))) break;
-              if (elect_one()) load_tile(&tmV, sV, C::B_VFULL, it.z & 0xFFFF, it.y, it.x);
-              v_loads = m + 1;
-            }
+            if (dp_there && p_last) commit_uniform(bar(C::B_VEMPTY + (mp & 1)));   // that was V's last reader in its item
             if (++q_stage == C::QS) { q_stage = 0; q_parity ^= 1u; }
             p_first = e == 0;
             p_last = last;
@@ -499,7 +531,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               e = 0;
             }
           }
-          if (lane == 0 && (gave_up != 0u || abortf->v != 0u) && v_loads > 1) drain_wait(bar(C::B_VFULL), (v_loads - 1) & 1);
         } else if (warp == 3) {
           // ---- dV, a half at a time ----
           int do_stage = 0;
@@ -930,7 +961,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     pdl_wait();   // the scratch has been zeroed
     const int wq = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    const uint32_t stg = s0 + C::SMEM_STG + wq * 8192, st_row = static_cast<uint32_t>(lane) * 128u, st_sw = static_cast<uint32_t>(lane & 7);
+    const uint32_t stg = s0 + C::SMEM_STG + wq * (C::NSTG * 4096), st_row = static_cast<uint32_t>(lane) * 128u, st_sw = static_cast<uint32_t>(lane & 7);
     if (lane == 0) {
       tma_prefetch_desc(&tmAcc);
       tma_prefetch_desc(&tmDK);
@@ -976,7 +1007,21 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + (is_k ? 1 : 0)));
           }
-          if constexpr (kF32) {
+          if constexpr (kF32 && C::NSTG == 1) {   // a box at a time
+            if (half == 1) {
+              if (lane == 0) bulk_wait_group_read0();
+              __syncwarp();
+            }
+            stage_scaled(0, r, f);
+            if (half == 0) {
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0 && key0 < a.T) {
+                tma_store_4d(is_k ? &tmDK : &tmDV, stg, col, key0, h, b);
+                bulk_commit_group();
+              }
+            }
+          } else if constexpr (kF32) {
             stage_scaled(half, r, f);
           } else {
             uint32_t pk[16];
@@ -990,8 +1035,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && key0 < a.T && col < a.d_real) {
-          tma_store_4d(is_k ? &tmDK : &tmDV, buf, col, key0, h, b);
-          if (kF32 && col + 32 < a.d_real) tma_store_4d(is_k ? &tmDK : &tmDV, buf + 4096, col + 32, key0, h, b);
+          if (kF32 && C::NSTG == 1) {
+            if (col + 32 < a.d_real) tma_store_4d(is_k ? &tmDK : &tmDV, buf, col + 32, key0, h, b);
+          } else {
+            tma_store_4d(is_k ? &tmDK : &tmDV, buf, col, key0, h, b);
+          }
+          if (kF32 && C::NSTG == 2 && col + 32 < a.d_real) tma_store_4d(is_k ? &tmDK : &tmDV, buf + 4096, col + 32, key0, h, b);
           bulk_commit_group();
         }
       }
@@ -1019,21 +1068,19 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           if constexpr (kF32) stage_scaled(buf, r, a.sm_scale);
           else stage_box(buf, r);
         };
+        auto add = [&](uint32_t src, int col) {
+          if constexpr (kF32) tma_reduce_add_4d(&tmAcc, src, col, q0, h, b);
+          else tma_reduce_add_3d(&tmAcc, src, col, q0, bh);
+        };
         auto reduce = [&](int g) {   // both boxes: columns 64 g .. 64 g + 63
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && q0 < a.T) {
-            auto add = [&](uint32_t src, int col) {
-              if constexpr (kF32) tma_reduce_add_4d(&tmAcc, src, col, q0, h, b);
-              else tma_reduce_add_3d(&tmAcc, src, col, q0, bh);
-            };
             if (g * 2 < np) add(stg, g * 64);
             if (g * 2 + 1 < np) add(stg + 4096, g * 64 + 32);
             bulk_commit_group();
           }
         };
-        if (lane == 0) bulk_wait_group_read0();   // the staging buffers have been read
-        __syncwarp();
         if constexpr (HD == 64) {
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
@@ -1041,14 +1088,23 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             tmem_ld32(tDQ + p * 32, r);
             tmem_wait_ld();
             if (p == 1) drained();
-            stage(p, r);
+            if (lane == 0) bulk_wait_group_read0();   // the staging buffer has been read
+            __syncwarp();
+            stage(0, r);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0 && q0 < a.T) {
+              if (p < np) add(stg, p * 32);
+              bulk_commit_group();
+            }
           }
-          reduce(0);
         } else {   // the next dP^T waits for these columns: the second half goes into registers before the first leaves
           uint32_t r[2][32];
           tmem_ld32(tDQ, r[0]);
           tmem_ld32(tDQ + 32, r[1]);
           tmem_wait_ld();
+          if (lane == 0) bulk_wait_group_read0();   // the staging buffers have been read
+          __syncwarp();
           stage(0, r[0]);
           stage(1, r[1]);
           tmem_ld32(tDQ + 64, r[0]);
