@@ -33,8 +33,8 @@
 //    gives 2 % of it back, the test ahead of the loop 4 %.
 //  * The products are issued by whole warps with warp-uniform operands (mma_ss_uniform).
 //
-// Schedule at HD = 64. The compute warps form P^T of tile t and dS^T of tile t - 1 in one instruction stream (see there).
-//   warp 1   S^T(t), dP^T(t - 1) as soon as S^T(t - 1) and dP^T(t - 2) have been loaded
+// Schedule at HD = 64. The compute warps form dS^T of tile t - 1 and P^T of tile t in one instruction stream (see there).
+//   warp 1   dP^T(t) as soon as dP^T(t - 1) has been loaded, S^T(t + 1) as soon as S^T(t) has
 //   warp 3   dV += P^T(t) dO, a half of 64 queries at a time
 //   warp 2   dK += dS^T(t - 1) Q by halves, dQ(t - 1)
 // TMEM: S^T 128, dP^T 128, dV 64, dK 64, dQ 64, P^T 64 columns.
@@ -106,8 +106,8 @@ struct FusedCfg {
   static constexpr int NH = (HD == 64) ? 2 : 1;      // halves of 64 queries with barriers of their own
   static constexpr int B_KFULL = 0, B_KEMPTY = B_KFULL + NK, B_VFULL = B_KEMPTY + NK, B_VEMPTY = B_VFULL + NV, B_QFULL = B_VEMPTY + NV,
                        B_QEMPTY = B_QFULL + QS, B_DOFULL = B_QEMPTY + QS, B_DOEMPTY = B_DOFULL + OS, B_SFULL = B_DOEMPTY + OS,
-                       B_SFREE = B_SFULL + NH, B_PFULL = B_SFREE + NH, B_PFREE = B_PFULL + NH, B_DPFULL = B_PFREE + NH,
-                       B_DSFULL = B_DPFULL + 1, B_DSFREE = B_DSFULL + 1, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
+                       B_SFREE = B_SFULL + NH, B_PFULL = B_SFREE + NH, B_PFREE = B_PFULL + NH, B_DPFULL = B_PFREE + NH, B_DPFREE = B_DPFULL + NH,
+                       B_DSFULL = B_DPFREE + NH, B_DSFREE = B_DSFULL + NH, B_DQFULL = B_DSFREE + 1, B_DQEMPTY = B_DQFULL + 1,
                        B_ACCFULL = B_DQEMPTY + 1, B_ACCFREE = B_ACCFULL + 2, B_ITEMFULL = B_ACCFREE + 2, B_ITEMEMPTY = B_ITEMFULL + NITEM,
                        B_CLC = B_ITEMEMPTY + NITEM, NBAR = B_CLC + 1;
   static constexpr int ITEM_READERS = (HD == 64) ? 7 : 14;    // warps that read item headers
@@ -130,7 +130,7 @@ enum : uint32_t {
   W_U_KFULL = 0x401, W_U_VFULL = 0x402, W_U_QFULL = 0x403, W_U_DOFULL = 0x404, W_U_QEMPTY = 0x405, W_U_DOEMPTY = 0x406, W_U_ITEMEMPTY = 0x407,
   W_U_SFULL = 0x408, W_U_SFREE = 0x409, W_U_PFULL = 0x40A, W_U_PFREE = 0x40B, W_U_DPFULL = 0x40C, W_U_DSFULL = 0x40D,
   W_U_DSFREE = 0x40E, W_U_DQFULL = 0x40F, W_U_DQEMPTY = 0x410, W_U_ACCFULL = 0x411, W_U_ACCFREE = 0x412, W_U_ALIGN = 0x413,
-  W_U_ITEMFULL = 0x414, W_U_CLC = 0x415, W_U_KEMPTY = 0x416, W_U_VEMPTY = 0x417,
+  W_U_ITEMFULL = 0x414, W_U_CLC = 0x415, W_U_KEMPTY = 0x416, W_U_VEMPTY = 0x417, W_U_DPFREE = 0x418,
 };
 
 __device__ __forceinline__ void st_shared_v4(uint32_t saddr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
@@ -179,7 +179,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     uint32_t count = 1;
     if (i >= C::B_QFULL && i < C::B_QEMPTY) count = 33;        // the TMA load and the producer lanes' own copies
     if (i >= C::B_DOEMPTY && i < C::B_SFULL) count = 2;        // dP^T and dV have read the tile
-    if (i == C::B_DSFULL || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
+    if ((i >= C::B_DPFREE && i < C::B_DSFREE) || (i >= C::B_SFREE && i < C::B_PFREE)) count = 8 / C::NH;   // one arrival per compute warp
     if (i == C::B_DQEMPTY) count = 4;                          // one per dQ warp
     if (i == C::B_ACCFREE || i == C::B_ACCFREE + 1) count = 4; // dV, dK have been read out of TMEM
     if (i >= C::B_ITEMEMPTY && i < C::B_CLC) count = C::ITEM_READERS;
@@ -489,47 +489,43 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       };
       if constexpr (HD == 64) {
         if (warp == 1) {
-          // ---- S^T(t) and dP^T(t - 1), a half at a time, as soon as the half's S^T(t - 1) and dP^T(t - 2) have been loaded ----
-          int q_stage = 0, do_stage = 0;
+          // ---- dP^T(t) when dP^T(t - 1) has been loaded, S^T(t + 1) when S^T(t) has ----
+          int q_stage = 0, do_stage = 0, e = 0;
           uint32_t q_parity = 0, do_parity = 0;
-          advance();
-          bool p_first = false, p_last = false;   // tile t - 1 is its item's first / last
-          int e = 0;
-          while (ok) {
-            const bool s_there = have, dp_there = t > 0;
-            if (!s_there && !dp_there) break;
-            const bool last = e == it.w - 1;
-            if (s_there) {
-              if (e == 0 && !(ok = wait(C::B_KFULL + (m & 1), (m >> 1) & 1, W_U_KFULL))) break;
-              if (!(ok = wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL))) break;
+          auto issue_s = [&]() -> bool {   // of tile t + 1, the item's e-th; behind the last tile only the signal
+            if (have) {
+              if (e == 0 && !wait(C::B_KFULL + (m & 1), (m >> 1) & 1, W_U_KFULL)) return false;
+              if (!wait(C::B_QFULL + q_stage, q_parity, W_U_QFULL)) return false;
             }
-            const int mp = (s_there && e > 0) ? m : m - 1;   // tile t - 1's item
-            if (dp_there) {   // its V is waited for at the item's first dP^T
-              if (p_first && !(ok = wait(C::B_VFULL + (mp & 1), (mp >> 1) & 1, W_U_VFULL))) break;
-              if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
-            }
-            if (dp_there && !(ok = wait2(C::B_SFREE, (t - 1) & 1, W_U_SFREE, C::B_SFREE + 1, (t - 1) & 1, W_U_SFREE))) break;
+            if (t >= 0 && !wait2(C::B_SFREE, t & 1, W_U_SFREE, C::B_SFREE + 1, t & 1, W_U_SFREE)) return false;
             tc_fence_after_sync();
-            if (s_there) product_kmajor(C::TM_S, lo_k0 + (m & 1) * T16, lo_q0 + q_stage * T16);
-            if (dp_there) product_kmajor(C::TM_DP, lo_v + (mp & 1) * T16, lo_do0 + do_stage * T16);
+            if (have) product_kmajor(C::TM_S, lo_k0 + (m & 1) * T16, lo_q0 + q_stage * T16);
             commit_uniform(bar(C::B_SFULL));
             commit_uniform(bar(C::B_SFULL + 1));
-            if (dp_there) {
-              commit_uniform(bar(C::B_DOEMPTY + do_stage));
-              if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
-            }
-            if (!s_there) break;   // that was the last dP^T
-            if (dp_there && p_last) commit_uniform(bar(C::B_VEMPTY + (mp & 1)));   // that was V's last reader in its item
             if (++q_stage == C::QS) { q_stage = 0; q_parity ^= 1u; }
-            p_first = e == 0;
-            p_last = last;
             ++t;
-            ++e;
-            if (last) {
+            return true;
+          };
+          advance();
+          t = -1;
+          if (have) ok = issue_s();
+          while (have && ok) {
+            if (e == 0 && !(ok = wait(C::B_VFULL + (m & 1), (m >> 1) & 1, W_U_VFULL))) break;
+            if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
+            if (t > 0 && !(ok = wait2(C::B_DPFREE, (t - 1) & 1, W_U_DPFREE, C::B_DPFREE + 1, (t - 1) & 1, W_U_DPFREE))) break;
+            tc_fence_after_sync();
+            product_kmajor(C::TM_DP, lo_v + (m & 1) * T16, lo_do0 + do_stage * T16);
+            commit_uniform(bar(C::B_DPFULL));
+            commit_uniform(bar(C::B_DPFULL + 1));
+            commit_uniform(bar(C::B_DOEMPTY + do_stage));
+            if (++do_stage == C::OS) { do_stage = 0; do_parity ^= 1u; }
+            if (++e == it.w) {
+              commit_uniform(bar(C::B_VEMPTY + (m & 1)));   // that was V's last reader in its item
               advance();
               ++m;
               e = 0;
             }
+            ok = issue_s();
           }
         } else if (warp == 3) {
           // ---- dV, a half at a time ----
@@ -557,14 +553,14 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (ok) advance();
           }
         } else {
-          // ---- dK(t - 1), a half at a time, and dQ(t - 1), as dS^T(t - 1) is written in the compute warps' iteration t ----
+          // ---- dK(t - 1), a half at a time, and dQ(t - 1) ----
           int q_stage = 0;
           bool first = false, last = false;   // of tile t - 1
           auto accumulate = [&](int item) -> bool {
             if (first && item > 0 && !wait(C::B_ACCFREE + 1, (item - 1) & 1, W_U_ACCFREE)) return false;
 #pragma unroll 1
             for (int w = 0; w < 2; ++w) {
-              if (!wait(C::B_PFULL + w, t & 1, W_U_PFULL)) return false;
+              if (!wait(C::B_DSFULL + w, (t - 1) & 1, W_U_DSFULL)) return false;
               tc_fence_after_sync();
               product_dk(w, q_mn0 + q_stage * T16, first && w == 0);
             }
@@ -584,11 +580,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           int e = 0;
           advance();
           while (have || t > 0) {
-            if (t == 0) {
-              if (!(ok = wait(C::B_PFULL, 0, W_U_PFULL) && wait(C::B_PFULL + 1, 0, W_U_PFULL))) break;
-            } else if (!(ok = accumulate((have && e > 0) ? m : m - 1))) {
-              break;
-            }
+            if (t > 0 && !(ok = accumulate((have && e > 0) ? m : m - 1))) break;
             if (!have) break;   // that was the last tile
             first = e == 0;
             last = e == it.w - 1;
@@ -739,82 +731,106 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
     };
     if constexpr (HD == 64) {
-      // Iteration t forms P^T of tile t and dS^T of tile t - 1 in one instruction stream: the exponentials' special-function
-      // pipe and the multiply-adds, conversions and stores of dS^T overlap, and neither product is ever waited for in a
-      // chain: S^T(t + 1) and dP^T(t) are issued as soon as S^T(t) and dP^T(t - 1) have been loaded. The two warpgroups
+      // Iteration t forms dS^T of tile t - 1 and, LAG blocks behind it in the same instruction stream, P^T of tile t. Each product is issued as
+      // soon as its predecessor has been loaded; dP^T(t) then has the P^T blocks behind the dS^T blocks' end, the masks and the stores
+      // to be formed under, S^T(t + 1) the first LAG blocks of the next iteration. (Side by side from one barrier for both, every
+      // iteration waits some 250 cycles for its products. Backward us, lag 0 / 2 / 5 / 6 / 7 / 8: causal 8 x 16 x 1000 x 64 93.6 / 91.7 / 90.6 / 89.2 / 89.6 / 91.7,
+      // 8 x 16 x 2048 280 / 290 / 281 / 273 / 276 / 281, hierarchical 8 x 16 x 2048 x 64 139.4 / 139.3 / 138.5 / 135.8 / 136.8 / 140.7, 16 x 16 x 4096 x 64 948 / 981 /
+      // 966 / 930 / 943 / 983. The exponentials and the multiply-adds of one warp overlap less, so both want to be kept.) The two warpgroups
       // have barriers of their own and drift apart, so that one does arithmetic while the other waits, loads or stores:
-      //   SFULL  S^T(t) and dP^T(t - 1) of the half are there      SFREE   they have been loaded
-      //   PFULL  its P^T(t) and dS^T(t - 1) have been written      PFREE   dV has read P^T(t);  DSFREE  dK and dQ have read dS^T(t)
-      // P^T stays in registers as fp32 for a tile; results are stored at the end of the iteration, when the products that
-      // read their predecessors are done.
+      //   SFULL, DPFULL  the half of S^T, dP^T is there       SFREE, DPFREE  it has been loaded
+      //   PFULL, DSFULL  its P^T, dS^T has been written       PFREE  dV has read P^T;  DSFREE  dK and dQ have read dS^T
+      // P^T stays in registers as fp32 for a tile.
       uint32_t p[2][32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) { p[0][j] = 0u; p[1][j] = 0u; }
+      for (int j = 0; j < 32; ++j) p[0][j] = p[1][j] = 0u;
+      constexpr int LAG = 6;
+      bool dp_ready = true;
       const float* side_prev = sSide;
-      bool s_ready = true;
-      // One body for all iterations: the first one's dS^T and the last one's P^T are computed from whatever is there and
-      // read by nobody. What the warps need to know of a tile's item lies beside its scalars: a header read at the start of
-      // every item is code that the instruction cache has lost by then, and cost 900 cycles of it. (Read where PARTIAL tiles are masked;
-      // read ahead of the arithmetic the entry makes every tile 4 % longer.)
-      ok = wait(C::B_SFULL + w, 0, W_U_SFULL);
-      bool more = ok && reinterpret_cast<const uint32_t*>(sSide)[C::SIDE_ENT] != C::ENT_END;
+      // What the warps need to know of a tile's item lies beside its scalars: a header read at the start of every item is code that the
+      // instruction cache has lost by then, and cost 900 cycles of it. (Read where PARTIAL tiles are masked; read ahead of the arithmetic the
+      // entry makes every tile 4 % longer.) Behind the last tile, P^T is computed from whatever is there and read by nobody.
 #pragma unroll 1
-      for (; more; ++t) {
-        if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
-        tc_fence_after_sync();
+      for (;; ++t) {
         const float* side = sSide + qs * C::SIDE_WORDS;
-        bool out_ready = false;
-        uint32_t pk_ds[2][16];
         // 16 keys x 16 queries at a time, both halves of the keys for a group of queries. The next block is loaded while one is
         // worked on: with two warps to a scheduler a TMEM load of some 150 cycles that is waited for at once is not covered. (Four
         // blocks of 32 queries, each loaded and awaited: causal 8 x 16 x 1000 x 64 84.0 -> 80.7 us, 8 x 16 x 2048 241 -> 230.)
+        // (In the first iteration dS^T is computed from whatever is there, and read by nobody.)
+        uint32_t sb[2][8], db[2][8];
         uint64_t lse[2], delta[2];
-        uint32_t sb[2][8], dpb[2][8];
-        auto load_block = [&](int c) {
-          tmem_ld16x256_x2(tS + (c & 1) * ROW16 + (c >> 1) * 16, sb[c & 1]);
-          tmem_ld16x256_x2(tDP + (c & 1) * ROW16 + (c >> 1) * 16, dpb[c & 1]);
-        };
-        auto load_scalars = [&](int g) {
+        bool s_ready = false, out_ready = false;   // barriers are tested ahead: a test takes some 150 cycles under this load, and as a rule it finds the phase complete
+        if (!__all_sync(0xffffffffu, dp_ready)) {
+          if (t > 0 && !(ok = wait(C::B_DPFULL + w, (t - 1) & 1, W_U_DPFULL))) break;
+          if (t > 1 && !(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
+        }
+        tc_fence_after_sync();
+        tmem_ld16x256_x2(tDP, db[0]);
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            lse[j] = ld_shared_pair(side + qcol + 16 * g + 8 * j);
-            delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 16 * g + 8 * j);
+        for (int c = 0; c < 8 + LAG; ++c) {
+          const int hf = c & 1, g = c >> 1, cp = c - LAG, gp = cp >> 1, hp = cp & 1;
+          if (c < 8 && hf == 0) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) delta[j] = ld_shared_pair(side_prev + KD_TILE + qcol + 16 * g + 8 * j);
           }
-        };
-        load_block(0);
+          if (cp >= 0 && hp == 0) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const int hf = c & 1, g = c >> 1;
-          if (hf == 0) load_scalars(g);
+            for (int j = 0; j < 2; ++j) lse[j] = ld_shared_pair(side + qcol + 16 * gp + 8 * j);
+          }
+          if (c == LAG - 2) s_ready = mbar_test_wait(bar(C::B_SFULL + w), t & 1);
+          if (c == LAG - 1) {
+            if (!__all_sync(0xffffffffu, s_ready) && !(ok = wait(C::B_SFULL + w, t & 1, W_U_SFULL))) break;
+            tc_fence_after_sync();
+          }
           tmem_wait_ld();
-          if (c < 7) load_block(c + 1);
-          if (c == 7) {   // all loaded
+          if (c < 7) tmem_ld16x256_x2(tDP + ((c + 1) & 1) * ROW16 + ((c + 1) >> 1) * 16, db[(c + 1) & 1]);
+          if (cp >= -1 && cp < 7) tmem_ld16x256_x2(tS + ((cp + 1) & 1) * ROW16 + ((cp + 1) >> 1) * 16, sb[(cp + 1) & 1]);
+          if (c == 7) {
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0 && t > 0) mbar_arrive(bar(C::B_DPFREE + w));
+          }
+          if (cp == 7) {
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::B_SFREE + w));
-            // The barriers of the stores below, and of the next iteration further down, are tested ahead: a test takes some 150
-            // cycles under this load, and as a rule it finds the phase complete.
-            out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1) && mbar_test_wait(bar(C::B_DSFREE), t & 1);
+            out_ready = mbar_test_wait(bar(C::B_PFREE + w), (t - 1) & 1);
           }
+          if (c < 8) {
+            uint32_t pk[4];
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
+            for (int j = 0; j < 2; ++j) {
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-              uint32_t& p0 = p[hf][8 * g + 4 * j + 2 * r];
-              uint32_t& p1 = p[hf][8 * g + 4 * j + 2 * r + 1];
-              const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(dpb[hf][4 * j + 2 * r], dpb[hf][4 * j + 2 * r + 1]));
-              const uint64_t x = mul_f32x2(pack_u32x2(p0, p1), d);
-              pk_ds[hf][4 * g + 2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
-              const uint64_t y = fma_f32x2(pack_u32x2(sb[hf][4 * j + 2 * r], sb[hf][4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
-              p0 = __float_as_uint(fast_exp2(-lo_f32x2(y)));
-              p1 = __float_as_uint(fast_exp2(-hi_f32x2(y)));
+              for (int r = 0; r < 2; ++r) {
+                const uint64_t d = fma_f32x2(delta[j], minus1, pack_u32x2(db[hf][4 * j + 2 * r], db[hf][4 * j + 2 * r + 1]));
+                const uint64_t x = mul_f32x2(pack_u32x2(p[hf][8 * g + 4 * j + 2 * r], p[hf][8 * g + 4 * j + 2 * r + 1]), d);
+                pk[2 * j + r] = pack2<kBf16>(lo_f32x2(x), hi_f32x2(x));
+              }
+            }
+            stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(2 * g) << 4) ^ ds_sw), pk[0], pk[1], pk[2], pk[3]);
+          }
+          if (cp >= 0) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+#pragma unroll
+              for (int r = 0; r < 2; ++r) {
+                const uint64_t y = fma_f32x2(pack_u32x2(sb[hp][4 * j + 2 * r], sb[hp][4 * j + 2 * r + 1]), nc2, lse[j]);   // LSE - c S
+                p[hp][8 * gp + 4 * j + 2 * r] = __float_as_uint(fast_exp2(-lo_f32x2(y)));
+                p[hp][8 * gp + 4 * j + 2 * r + 1] = __float_as_uint(fast_exp2(-hi_f32x2(y)));
+              }
             }
           }
+          if (c == 7) {
+            fence_proxy_async_smem();   // the dK and dQ products read dS^T through the async proxy
+            __syncwarp();
+            if (lane == 0 && t > 0) mbar_arrive(bar(C::B_DSFULL + w));
+          }
         }
+        if (!ok) break;
         const uint32_t* side_u = reinterpret_cast<const uint32_t*>(side);
         const uint32_t ent = side_u[C::SIDE_ENT];
-        more = ent != C::ENT_END;
-        if (more && ((ent >> 8) & 0xFFu) == KD_TILE_PARTIAL) {
+        if (ent == C::ENT_END) break;
+        if ((ent >> 8) == KD_TILE_PARTIAL) {
           // The words of this thread's queries, one pair after the other: a shift brings this thread's keys to the top bits of the
           // bytes, and a byte's top bit spreads over a word by one permute. (Formed here from class masks and descriptors, key by
           // key, before the plan held them: hierarchical 16 x 16 x 4096 x 64 backward 1072 -> 1025 us, 8 x 16 x 2048 x 64 167 -> 162,
@@ -835,13 +851,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               }
           }
         }
-        // (in the last iteration too: it must not complete a phase of PFULL ahead of the dV issuer)
-        if (!__all_sync(0xffffffffu, out_ready)) {
-          if (t > 0 && !(ok = wait(C::B_PFREE + w, (t - 1) & 1, W_U_PFREE))) break;
-          if (t > 1 && !(ok = wait(C::B_DSFREE, t & 1, W_U_DSFREE))) break;
-        }
+        if (!__all_sync(0xffffffffu, out_ready) && t > 0 && !(ok = wait(C::B_PFREE + w, (t - 1) & 1, W_U_PFREE))) break;
         tc_fence_after_sync();
-        s_ready = mbar_test_wait(bar(C::B_SFULL + w), (t + 1) & 1);
+        dp_ready = mbar_test_wait(bar(C::B_DPFULL + w), t & 1) && mbar_test_wait(bar(C::B_DSFREE), (t + 1) & 1);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t pk[16];
@@ -849,12 +861,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           for (int j = 0; j < 16; ++j) pk[j] = pack2<kBf16>(__uint_as_float(p[hf][2 * j]), __uint_as_float(p[hf][2 * j + 1]));
           tmem_st16x128_x8(tP + hf * ROW16, pk);
         }
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf)
-#pragma unroll
-          for (int j = 0; j < 8; j += 2)
-            stmatrix_x4(ds_row + hf * 2048u + ((static_cast<uint32_t>(j) << 4) ^ ds_sw), pk_ds[hf][2 * j], pk_ds[hf][2 * j + 1], pk_ds[hf][2 * j + 2], pk_ds[hf][2 * j + 3]);
-        fence_proxy_async_smem();   // the dK and dQ products read dS^T through the async proxy
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
