@@ -1,13 +1,15 @@
-// Backward kernels for sm_100a: dQ (query-tile major) and dK/dV (key-tile major).
+// Backward for sm_100a: the delta kernel, the deterministic backward's dQ kernel (query-tile major), and the launches of both backwards.
 //
-// Both kernels recompute P = exp2(S*scale*log2e - LSE) from Q, K and the saved base-2 LSE and
-// form dS = P * (dP - delta), as the reference's two backward workers do
-// (_flash_attn_bwd_dq, original_kernel.py:1173-1336; _flash_attn_bwd_dkdv, :1339-1525), but
-// walk only the non-empty tiles of the plan and apply the rule only on PARTIAL tiles.
+// The dQ kernel recomputes P = exp2(S*scale*log2e - LSE) from Q, K and the saved base-2 LSE and
+// forms dS = P * (dP - delta), as the reference's dQ worker does (_flash_attn_bwd_dq, original_kernel.py:1173-1336), but
+// walks only the non-empty tiles of the plan and applies the rule only on PARTIAL tiles.
 // delta = rowsum(O * dO) (the reference's _flash_attn_bwd_precompute, :629-710) is produced
-// by a small bandwidth-bound kernel ahead of the other two.
+// by a small bandwidth-bound kernel ahead of it. dK and dV (the reference's _flash_attn_bwd_dkdv, :1339-1525) come from the fused kernel
+// without its dQ (attn_bwd_fused.cu), which forms them in a fixed order. (A kernel of the structure below in its place, all key-tile
+// work in units of 64 queries: deterministic backward, us, before and with the fused kernel: hierarchical 4 x 16 x 2048 x 64 96.7 -> 82.8,
+// 16 x 16 x 4096 x 64 1378 -> 1202, 4 x 16 x 2048 x 128 177 -> 154, 3 x 6 x 1357 x 80 37.4 -> 28.9, causal 8 x 16 x 1000 x 64 124 -> 113.)
 //
-// Shared structure (640 threads): warp 0 = TMA producer, warps 1-3 = MMA issuers, warps 4-19 =
+// Structure of the dQ kernel (640 threads): warp 0 = TMA producer, warps 1-3 = MMA issuers, warps 4-19 =
 // four compute warpgroups. The backward needs no row reductions, so a 128-column score tile is
 // split by columns: a "unit" u = 2*entry + half is one 64-column half, and two warpgroups share a
 // unit, 32 columns each, so that sixteen warps (four per scheduler) hide one another's
@@ -38,30 +40,25 @@ struct BwdCfg {
   static constexpr int NFIX = (HD == 64) ? 2 : 1;     // buffers for the per-head resident tile pair
   static constexpr int SMEM_FIX = 0;                               // NFIX x two resident tiles
   static constexpr int SMEM_RING = SMEM_FIX + NFIX * 2 * TILE_BYTES;  // STAGES x two streamed tiles
-  static constexpr int SMEM_STAGE = SMEM_RING + STAGES * 2 * TILE_BYTES;  // per-warp staging
   static constexpr int NSUB = 2;                      // warpgroups that share a 64-column unit
   static constexpr int CPT = 2 / NSUB;                // 32-column chunks per compute thread and unit
   static constexpr int THREADS = 128 + 256 * NSUB;    // four light warps + 2 * NSUB compute warpgroups
   static constexpr int REGS_COMPUTE = KD_REGS_COMPUTE_BWD;
-  static constexpr int STAGE_WORDS = 2 * 32 * CPT;                 // per warp (dK/dV kernel): 32*CPT x {lse, delta}
   static constexpr int NITEM = 4;                     // ring of item headers and lists
-  static constexpr int SMEM_ACT = SMEM_STAGE + 8 * NSUB * STAGE_WORDS * 4;  // NITEM x <= 128 list entries
+  static constexpr int SMEM_ACT = SMEM_RING + STAGES * 2 * TILE_BYTES;  // NITEM x <= 128 list entries
   static constexpr int SMEM_TOTAL = SMEM_ACT + NITEM * 128 * 2;
   static constexpr int SMEM_ALLOC = SMEM_TOTAL + 1024;
   // TMEM columns
-  // buffer j: scores at 128*j, dP at 128*j + 64; accumulators behind the buffers
-  static constexpr uint32_t TM_ACC0 = NBUF * 128;        // dQ, or dK
-  static constexpr uint32_t TM_ACC1 = NBUF * 128 + HD;   // dV
-  static_assert(TM_ACC1 + HD <= 512, "TMEM budget");
+  // buffer j: scores at 128*j, dP at 128*j + 64; the accumulator behind the buffers
+  static constexpr uint32_t TM_ACC0 = NBUF * 128;        // dQ
+  static_assert(TM_ACC0 + HD <= 512, "TMEM budget");
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
 enum : uint32_t {
   W_Q_FIXFULL = 0x201, W_Q_RINGEMPTY = 0x202, W_Q_RINGFULL = 0x203, W_Q_PFULL = 0x204, W_Q_SFULL = 0x205,
   W_Q_ACCFULL = 0x206, W_Q_M2ISSUED = 0x207, W_Q_FIXEMPTY = 0x208, W_Q_ACCFREE = 0x209,
-  W_K_FIXFULL = 0x301, W_K_RINGEMPTY = 0x302, W_K_RINGFULL = 0x303, W_K_PFULL = 0x304, W_K_SFULL = 0x305,
-  W_K_ACCFULL = 0x306, W_K_M2ISSUED = 0x307, W_K_FIXEMPTY = 0x308, W_K_ACCFREE = 0x309,
-  W_Q_ITEMFULL = 0x20A, W_Q_ITEMEMPTY = 0x20B, W_Q_CLC = 0x20C, W_K_ITEMFULL = 0x30A, W_K_ITEMEMPTY = 0x30B, W_K_CLC = 0x30C,
+  W_Q_ITEMFULL = 0x20A, W_Q_ITEMEMPTY = 0x20B, W_Q_CLC = 0x20C,
 };
 
 // =========================================================================================
@@ -132,12 +129,12 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const BwdArgs a) {
 }
 
 // =========================================================================================
-// What the two kernels below share: barriers, items and the producer warp.
+// The dQ kernel's barriers, items and producer warp.
 //
 // A work item is one tile of one (batch, head). The grid has a CTA per item, but a CTA that is running takes further items by cancelling CTAs that have not been launched yet
 // (clusterlaunchcontrol), as in the forward and the fused backward: the rings, the issuers and the compute warps run on into the
 // next item, and the start and drain of a CTA (launch, TMEM, first loads, pipeline fill, last products: 12,000 cycles) is paid once
-// per SM instead of once per item, which has some ten tiles of 2,200-2,800 cycles. Both kernels together, before (a CTA per tile and one
+// per SM instead of once per item, which has some ten tiles of 2,200-2,800 cycles. This kernel and one alike for dK and dV, before (a CTA per tile and one
 // or more heads) and with this, bf16 (us): hierarchical 4 x 16 x 2048 x 64 114 -> 108, 16 x 16 x 4096 x 64 1570 -> 1500; causal 8 x 16 x
 // 1000 x 64 146 -> 127, 8 x 16 x 2048 x 128 723 -> 685; no mask 4 x 16 x 2048 x 64 383 -> 331; causal 1 x 8 x 173 x 64 14.6 -> 11.7.
 // =========================================================================================
@@ -192,15 +189,12 @@ __device__ __forceinline__ int4 uniform(const int4& v) {
   return make_int4(__reduce_max_sync(0xffffffffu, v.x), __reduce_max_sync(0xffffffffu, v.y), __reduce_max_sync(0xffffffffu, v.z), __reduce_max_sync(0xffffffffu, v.w));
 }
 
-// The producer warp of the dQ kernel (kQ: items are query tiles; Q and dO resident, K and V streamed) and of the dK/dV kernel (key tiles;
-// K and V resident, Q and dO streamed). wait_ahead: the plan may be read now, the tensors only behind pdl_wait().
-template <int HD, bool kQ>
+// The producer warp: items are query tiles; Q and dO resident, K and V streamed. wait_ahead: the plan may be read now, the tensors only behind pdl_wait().
+template <int HD>
 __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CUtensorMap& tmFix1, const CUtensorMap& tmRing0, const CUtensorMap& tmRing1,
                                              const BwdArgs& a, uint32_t sFix, uint32_t sRing, uint16_t* lists, BwdShared<BwdCfg<HD>>& sh, int lane,
                                              bool wait_ahead) {
   using C = BwdCfg<HD>;
-  constexpr uint32_t FIXEMPTY = kQ ? W_Q_FIXEMPTY : W_K_FIXEMPTY, RINGEMPTY = kQ ? W_Q_RINGEMPTY : W_K_RINGEMPTY,
-                     ITEMEMPTY = kQ ? W_Q_ITEMEMPTY : W_K_ITEMEMPTY, CLC = kQ ? W_Q_CLC : W_K_CLC;
   if (lane == 0) {
     tma_prefetch_desc(&tmFix0);
     tma_prefetch_desc(&tmFix1);
@@ -218,20 +212,18 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
     int4 it;
     it.x = bh / a.H;
     it.y = bh - it.x * a.H;
-    it.z = __ldcg(a.order + ((size_t)it.x * 3 + (kQ ? 1 : 2)) * a.NT + rank);   // longest lists first
-    const int row = kQ ? it.z >> 1 : it.z;   // (query tiles: the list of the pair)
-    const uint16_t* list = kQ ? a.fwd_list + ((size_t)it.x * a.NP + row) * a.NT : a.bwd_list + ((size_t)it.x * a.NT + row) * a.NT;
-    const int n = __ldcg(kQ ? a.fwd_cnt + it.x * a.NP + row : a.bwd_cnt + it.x * a.NT + row);
+    it.z = __ldcg(a.order + ((size_t)it.x * 3 + 1) * a.NT + rank);   // longest lists first
+    const int row = it.z >> 1;   // the list of the pair
+    const uint16_t* list = a.fwd_list + ((size_t)it.x * a.NP + row) * a.NT;
+    const int n = __ldcg(a.fwd_cnt + it.x * a.NP + row);
 #pragma unroll
     for (int r = 0; r < 4; ++r) lst[r] = r * 32 + lane < a.NT ? __ldcg(list + r * 32 + lane) : 0u;   // does not wait for the count
     it.w = 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       if (r * 32 + lane >= n) lst[r] = 0u;
-      if (kQ) {
-        const uint32_t cls = (lst[r] >> (8 + 2 * (it.z & 1))) & 3u;
-        lst[r] = cls != 0u ? (lst[r] & 0xFFu) | (cls << 8) : 0u;
-      }
+      const uint32_t cls = (lst[r] >> (8 + 2 * (it.z & 1))) & 3u;
+      lst[r] = cls != 0u ? (lst[r] & 0xFFu) | (cls << 8) : 0u;
       it.w += __popc(__ballot_sync(0xffffffffu, lst[r] != 0u));
     }
     return it;
@@ -249,7 +241,7 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
     pending = true;
   };
   auto take_next = [&](int4& nx) -> bool {
-    if (!wait(sh.clc, (asked - 1) & 1, CLC)) return false;
+    if (!wait(sh.clc, (asked - 1) & 1, W_Q_CLC)) return false;
     pending = false;
     const int idx = clc_first_ctaid_x(smem_u32(sh.answer));
     __syncwarp();   // every lane has read the response that the next request overwrites
@@ -273,7 +265,7 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
   if (it.w <= 2) ask();
   while (ok) {
     const int slot = k % C::NITEM, b = it.x, h = it.y, n = it.w;
-    if (!(ok = wait(sh.item_empty[slot], ((k / C::NITEM) & 1) ^ 1, ITEMEMPTY))) break;
+    if (!(ok = wait(sh.item_empty[slot], ((k / C::NITEM) & 1) ^ 1, W_Q_ITEMEMPTY))) break;
     uint16_t* list = lists + slot * 128;
     int at = 0;
 #pragma unroll
@@ -296,12 +288,12 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
       if (n == 0) break;
       if (e == 0) {   // the item's resident tiles: into the buffer of the item before the last (NFIX = 2)
         const int f = fixed % C::NFIX;
-        if (!(ok = wait(sh.fix_empty[f], ((fixed / C::NFIX) & 1) ^ 1, FIXEMPTY))) break;
+        if (!(ok = wait(sh.fix_empty[f], ((fixed / C::NFIX) & 1) ^ 1, W_Q_FIXEMPTY))) break;
         load_pair(tmFix0, tmFix1, sFix + f * 2 * C::TILE_BYTES, sh.fix_full[f], it.z, h, b);
         ++fixed;
       }
       const int st = issued % C::STAGES;
-      if (!(ok = wait(sh.ring_empty[st], ((issued / C::STAGES) & 1) ^ 1, RINGEMPTY))) break;
+      if (!(ok = wait(sh.ring_empty[st], ((issued / C::STAGES) & 1) ^ 1, W_Q_RINGEMPTY))) break;
       load_pair(tmRing0, tmRing1, sRing + st * 2 * C::TILE_BYTES, sh.ring_full[st], list[e] & 0xFF, h, b);
       ++issued;
     }
@@ -351,7 +343,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (warp < 4) {
     reg_dealloc<KD_REGS_ISSUE>();
     if (warp == 0) {
-      bwd_producer<HD, true>(tmQ, tmDO, tmK, tmV, a, sFix, sRing, lists, sh, lane, wait_ahead);
+      bwd_producer<HD>(tmQ, tmDO, tmK, tmV, a, sFix, sRing, lists, sh, lane, wait_ahead);
     } else if ((warp == 3 || warp == 2) && lane == 0) {
       // ------------------------------ M1 issuers: warp 3: S_u = Q K_u^T; warp 2: dP_u = dO V_u^T ------------------------------
       const bool dp_part = (warp == 2);
@@ -492,7 +484,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     };
     if (wait_ahead) pdl_wait();
     if (warp == 4) {
-      __threadfence();   // for the dK/dV kernel, which does not wait for the delta kernel itself
+      __threadfence();   // for the kernel behind it, which does not wait for the delta kernel itself
       pdl_launch_dependents();
     }
     int n_acc = 0;   // items with units so far
@@ -611,366 +603,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (tid == 0) report_abort(&sh.abortf, a.status);
 }
 
-// =========================================================================================
-// dK/dV kernel: items are key tiles; streams = query halves of the current
-// query tile.   M1(i): S^T_i = K Q_i^T, dP^T_i = V dO_i^T     M2(i): dV += P^T_i dO_i,  dK += dS^T_i Q_i
-// =========================================================================================
-template <int HD, bool kBf16, bool kF32>
-__global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
-attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                     const BwdArgs a) {
-  using C = BwdCfg<HD>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t sFix = smem_u32(smem + C::SMEM_FIX);    // buffer f: K at +0, V at +TILE_BYTES
-  const uint32_t sRing = smem_u32(smem + C::SMEM_RING);  // stage s: Q at +0, dO at +TILE_BYTES
-  uint32_t* sStage = reinterpret_cast<uint32_t*>(smem + C::SMEM_STAGE);
-  uint16_t* lists = reinterpret_cast<uint16_t*>(smem + C::SMEM_ACT);
-  __shared__ BwdShared<C> sh;
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    bwd_init<C>(sh);
-    if (a.after_dq != 0) {   // see below
-      __threadfence();
-      fence_proxy_async_global();
-    }
-  }
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&sh.tmem_base), 512);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  // Directly behind the dQ kernel of the same call there is nothing to wait for: that kernel writes nothing that this one reads, and lets it
-  // start when it has itself waited for the delta kernel. So the last CTAs of the one overlap the first of the other (both together, with
-  // the wait here instead: 1 x 16 x 500 x 128 31.5 us, 23 so; 4 x 16 x 2048 x 64 110.2, 108.2; unmasked 1 x 4 x 2048 x 64 51.5, 34).
-  // What orders delta, and the dO of a float32 call, before the reads here: CUDA promises visibility to the kernel that executes
-  // griddepcontrol.wait behind the writer, which is the dQ kernel, and none through launch_dependents alone. Hence a device-wide
-  // fence on both sides of that hand-over (there behind the wait, here ahead of the block's barrier, with one for the TMA loads); all reads
-  // go past L1. That a dependent kernel starts after launch_dependents has been executed is what remains to be relied on.
-  // The dQ kernel's end is awaited at this one's end, so that whatever comes next finds both complete (what a successor reads ahead of its
-  // own wait is a plan, which no backward writes).
-  if (a.after_dq == 0) pdl_wait();
-  const uint32_t tbase = sh.tmem_base;
-
-  if (warp < 4) {
-    reg_dealloc<KD_REGS_ISSUE>();
-    if (warp == 0) {
-      bwd_producer<HD, false>(tmK, tmV, tmQ, tmDO, a, sFix, sRing, lists, sh, lane, false);
-    } else if ((warp == 3 || warp == 2) && lane == 0) {
-      // ------------------------------ M1 issuers: warp 3: S^T_u = K Q_u^T; warp 2: dP^T_u = V dO_u^T ------------------------------
-      const bool dp_part = (warp == 2);
-      const uint32_t idesc_m1 = make_idesc_f16(kBf16, 0, 0, KD_TILE, 64);   // N = 64 queries
-      const uint32_t hi = desc_hi_sw128();
-      const uint32_t loRingK = desc_lo_kmajor(sRing);
-      bool ok = true;
-      int buf = 0, round = 0, stage = 0, item = 0;   // run on across the items; item: of those with entries
-      uint32_t ring_parity = 0;
-      int4 it;
-      for (int k = 0; ok && bwd_header<C>(sh, k, W_K_ITEMFULL, it) && it.w >= 0; ++k) {
-        if (it.w == 0) continue;
-        const int U = 2 * it.w, fb = item % C::NFIX;
-        ok = mbar_wait<true>(smem_u32(&sh.fix_full[fb]), (item / C::NFIX) & 1, &sh.abortf, W_K_FIXFULL);
-        ++item;
-        if (!ok) break;
-        const uint32_t loA = desc_lo_kmajor(sFix + fb * 2 * C::TILE_BYTES + (dp_part ? C::TILE_BYTES : 0));   // V or K
-        uint64_t adesc[HD / 16];   // A descriptors of the item's k-steps
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) adesc[kk] = desc64(loA + koff_kmajor(kk), hi);
-        for (int u = 0; u < U && ok; ++u) {
-          const int i = u & 1;
-          // operands of the unit, formed ahead of the waits
-          // query rows 64i.. of Q (scores) or dO (dP)
-          const uint32_t blo = loRingK + stage * (2 * C::TILE_BYTES >> 4) + i * (64 * 128 >> 4) + (dp_part ? (C::TILE_BYTES >> 4) : 0);
-          uint64_t bdesc[HD / 16];
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk) bdesc[kk] = desc64(blo + koff_kmajor(kk), hi);
-          const uint32_t dst = tbase + buf * 128 + (dp_part ? 64 : 0);
-          if (round > 0) {   // buffer free once M2 of its previous unit has been issued
-            ok = mbar_wait<true>(smem_u32(&sh.m2_issued[buf]), (round - 1) & 1, &sh.abortf, W_K_M2ISSUED);
-            if (!ok) break;
-          }
-          if (i == 0) {      // first unit of a new entry: its Q and dO tiles must have landed
-            ok = mbar_wait<true>(smem_u32(&sh.ring_full[stage]), ring_parity, &sh.abortf, W_K_RINGFULL);
-            if (!ok) break;
-          }
-          tc_fence_after_sync();
-          mma_ss64<false>(dst, adesc[0], bdesc[0], idesc_m1);
-#pragma unroll
-          for (int kk = 1; kk < HD / 16; ++kk) mma_ss64<true>(dst, adesc[kk], bdesc[kk], idesc_m1);
-          mma_commit(smem_u32(&sh.s_full[buf]));
-          if (++buf == C::NBUF) { buf = 0; ++round; }
-          if (i == 1 && ++stage == C::STAGES) { stage = 0; ring_parity ^= 1; }
-        }
-        if (ok) mma_commit(smem_u32(&sh.fix_empty[fb]));   // this issuer's products of the item no longer read K / V
-      }
-    } else if (warp == 1 && lane == 0) {
-      // ------------------------------ M2 issuer: dV += P^T_u dO_u, dK += dS^T_u Q_u ------------------------------
-      const uint32_t idesc_m2 = make_idesc_f16(kBf16, 0, 1, KD_TILE, HD);   // B = dO / Q rows, MN-major
-      const uint32_t tDK = tbase + C::TM_ACC0, tDV = tbase + C::TM_ACC1;
-      const uint32_t hi = desc_hi_sw128();
-      const uint32_t loRingMN = desc_lo_mnmajor(sRing);
-      bool ok = true;
-      int buf = 0, stage = 0, item = 0;
-      uint32_t round_parity = 0;
-      int4 it;
-      for (int k = 0; ok && bwd_header<C>(sh, k, W_K_ITEMFULL, it) && it.w >= 0; ++k) {
-        if (it.w == 0) continue;
-        const int U = 2 * it.w;
-        if (item++ > 0) {   // the previous item's dK and dV must have been read out of the accumulators
-          ok = mbar_wait<true>(smem_u32(&sh.acc_free), item & 1, &sh.abortf, W_K_ACCFREE);
-          if (!ok) break;
-        }
-        for (int u = 0; u < U && ok; ++u) {
-          const int i = u & 1;
-          // operands of the unit, formed ahead of the wait
-          const uint32_t qb = loRingMN + stage * (2 * C::TILE_BYTES >> 4) + i * (64 * 128 >> 4);
-          const uint32_t dob = qb + (C::TILE_BYTES >> 4);
-          const uint32_t aS = tbase + buf * 128;
-          // 16-bit operands: queries 0-31 of the unit at columns [0,16) of their buffer half, queries 32-63 at [32,48)
-          uint64_t bq[4], bdo[4];
-          uint32_t aop[4];
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            bq[kk] = desc64(qb + koff_mnmajor(kk), hi);
-            bdo[kk] = desc64(dob + koff_mnmajor(kk), hi);
-            aop[kk] = aS + (kk >> 1) * 32 + (kk & 1) * 8;
-          }
-          ok = mbar_wait<true>(smem_u32(&sh.p_full[buf]), round_parity, &sh.abortf, W_K_PFULL);
-          if (!ok) break;
-          tc_fence_after_sync();
-          // dV += P^T_u dO_u   (P^T_u on top of S^T_u)
-          mma_ts64_p(tDV, aop[0], bdo[0], idesc_m2, u > 0 ? 1u : 0u);
-#pragma unroll
-          for (int kk = 1; kk < 4; ++kk) mma_ts64<true>(tDV, aop[kk], bdo[kk], idesc_m2);
-          // dK += dS^T_u Q_u   (dS^T_u on top of dP^T_u, 64 columns further)
-          mma_ts64_p(tDK, aop[0] + 64, bq[0], idesc_m2, u > 0 ? 1u : 0u);
-#pragma unroll
-          for (int kk = 1; kk < 4; ++kk) mma_ts64<true>(tDK, aop[kk] + 64, bq[kk], idesc_m2);
-          if (i == 1) mma_commit(smem_u32(&sh.ring_empty[stage]));
-          tc_fence_before_sync();
-          mbar_arrive(smem_u32(&sh.m2_issued[buf]));
-          if (++buf == C::NBUF) { buf = 0; round_parity ^= 1; }
-          if (i == 1 && ++stage == C::STAGES) stage = 0;
-        }
-        if (ok) mma_commit(smem_u32(&sh.acc_full));
-      }
-    }
-  } else {
-    reg_alloc<C::REGS_COMPUTE>();
-    // ------------------------------ compute warpgroups ------------------------------
-    constexpr int CPT = C::CPT;      // 32-column chunks of a unit this thread handles
-    constexpr int QW = 32 * CPT;     // queries of a unit handled by this warp
-    const int g = (warp - 4) >> 2;   // warpgroup
-    const int i = g / C::NSUB;       // stream: query half (64 queries) of each query tile
-    const int c0 = (g % C::NSUB) * CPT;   // first 32-query chunk of that half handled here
-    const int wq = warp & 3;
-    const int row = wq * 32 + lane;
-    const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
-    uint32_t* st_buf = sStage + (size_t)(warp - 4) * C::STAGE_WORDS;  // [QW lse][QW delta]
-    const float c = a.scale_log2;
-    bool ok = true;
-
-    int4 it = make_int4(0, 0, 0, 0);   // the item in hand; behind its last unit the next one
-    // LSE and delta of the next unit's queries are fetched one unit ahead into registers and handed to the warp through its shared-memory
-    // staging buffer, and with them, for a PARTIAL tile, the plan's words of these queries for the warp's 32 keys
-    float pre_lse[CPT], pre_delta[CPT];
-    uint32_t pre_words[CPT];
-#pragma unroll
-    for (int cc = 0; cc < CPT; ++cc) { pre_lse[cc] = 0.f; pre_delta[cc] = 0.f; pre_words[cc] = 0u; }
-    auto prefetch = [&](uint32_t entry, int h) {
-      if ((entry >> 8) == KD_TILE_PARTIAL) {
-        const uint32_t* src = a.words + (((size_t)it.x * a.NT + (entry & 0xFFu)) * a.NT + it.z) * KD_WORDS + wq * KD_TILE + i * 64 + c0 * 32 + lane;
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) pre_words[cc] = __ldcg(src + cc * 32);
-      }
-      // a query at or beyond the sequence length reads the last row's scalars: it sees nothing, so the tile is PARTIAL and the mask
-      // removes it
-#pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) {
-        const int q = (entry & 0xFF) * KD_TILE + i * 64 + (c0 + cc) * 32 + lane;
-        const size_t r = ((size_t)it.x * a.H + h) * a.T + min(q, a.T - 1);
-        pre_lse[cc] = __ldcg(a.lse + r);   // negated where it is used: a negation here would wait for the load
-        pre_delta[cc] = __ldcg(a.delta + r);
-      }
-    };
-    // The next item's header and first unit's scalars are fetched before the epilogue.
-    uint32_t ent_next = 0u;
-    const uint16_t* list = lists;
-    auto open_item = [&](int k) -> bool {
-      const int slot = k % C::NITEM;
-      if (!__all_sync(0xffffffffu, mbar_wait<true>(smem_u32(&sh.item_full[slot]), (k / C::NITEM) & 1, &sh.abortf, W_K_ITEMFULL))) return false;
-      it = uniform(sh.items[slot]);
-      if (it.w < 0) return false;
-      list = lists + slot * 128;
-      if (it.w > 0) {
-        ent_next = list[0];
-        prefetch(ent_next, it.y);
-      }
-      return true;
-    };
-    if (warp == 4) pdl_launch_dependents();
-    int n_acc = 0;   // items with units so far
-    // this stream's next unit, counted over all items, as (unit / NBUF, unit % NBUF)
-    int buf = i % C::NBUF;
-    uint32_t rnd = i / C::NBUF;
-    const uint32_t sfull0 = smem_u32(&sh.s_full[0]), pfull0 = smem_u32(&sh.p_full[0]);
-    const uint32_t tcol = tbase + lane_base + c0 * 32;   // this thread's first chunk inside a buffer
-
-    bool have = open_item(0);
-    for (int k = 0; have && ok; ++k) {
-    const int4 now = it;
-      const int n = now.w;
-      for (int e = 0; e < n; ++e) {
-        const uint32_t ent = ent_next;
-        const uint32_t cls = ent >> 8;
-        __syncwarp();
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-          st_buf[cc * 32 + lane] = __float_as_uint(pre_lse[cc]);
-          st_buf[QW + cc * 32 + lane] = __float_as_uint(pre_delta[cc]);
-        }
-        __syncwarp();
-        uint32_t mk[CPT];
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) mk[cc] = pre_words[cc];
-        if (e + 1 < n) {
-          ent_next = list[e + 1];
-          prefetch(ent_next, now.y);
-        }
-        const uint32_t tS = tcol + buf * 128, tP = tS + 64;
-        ok = mbar_wait<true>(sfull0 + buf * 8, rnd & 1u, &sh.abortf, W_K_SFULL);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after_sync();
-
-#pragma unroll
-        for (int cc = 0; cc < CPT; ++cc) {
-          uint32_t pk_p[16], pk_ds[16];
-          uint32_t rs[32], rp[32];
-          tmem_ld32(tS + cc * 32, rs);
-          tmem_ld32(tP + cc * 32, rp);
-          if (cls == KD_TILE_PARTIAL) mk[cc] = transpose_bits(mk[cc], lane);   // this key's visibility for the chunk's queries, while the scores are on their way
-          tmem_wait_ld();
-          if (cls != KD_TILE_PARTIAL) {   // warp-uniform: the common case carries no mask code at all
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 l4 = *reinterpret_cast<const float4*>(st_buf + cc * 32 + j);        // LSE of 4 queries
-              const float4 d4 = *reinterpret_cast<const float4*>(st_buf + QW + cc * 32 + j);   // delta of 4 queries
-              const float lw[4] = {l4.x, l4.y, l4.z, l4.w}, dw[4] = {d4.x, d4.y, d4.z, d4.w};
-              float pv[4], ds[4];
-#pragma unroll
-              for (int u2 = 0; u2 < 4; ++u2) pv[u2] = fast_exp2(fmaf(__uint_as_float(rs[j + u2]), c, -lw[u2]));
-#pragma unroll
-              for (int u2 = 0; u2 < 4; ++u2) ds[u2] = pv[u2] * (__uint_as_float(rp[j + u2]) - dw[u2]);
-              pk_p[j / 2] = pack2<kBf16>(pv[0], pv[1]);
-              pk_p[j / 2 + 1] = pack2<kBf16>(pv[2], pv[3]);
-              pk_ds[j / 2] = pack2<kBf16>(ds[0], ds[1]);
-              pk_ds[j / 2 + 1] = pack2<kBf16>(ds[2], ds[3]);
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 l4 = *reinterpret_cast<const float4*>(st_buf + cc * 32 + j);
-              const float4 d4 = *reinterpret_cast<const float4*>(st_buf + QW + cc * 32 + j);
-              const float lw[4] = {l4.x, l4.y, l4.z, l4.w}, dw[4] = {d4.x, d4.y, d4.z, d4.w};
-              float pv[4], ds[4];
-#pragma unroll
-              for (int u2 = 0; u2 < 4; ++u2) {
-                pv[u2] = fast_exp2(fmaf(__uint_as_float(rs[j + u2]), c, -lw[u2]));
-                if ((mk[cc] & (1u << (j + u2))) == 0u) pv[u2] = 0.f;
-              }
-#pragma unroll
-              for (int u2 = 0; u2 < 4; ++u2) ds[u2] = pv[u2] * (__uint_as_float(rp[j + u2]) - dw[u2]);
-              pk_p[j / 2] = pack2<kBf16>(pv[0], pv[1]);
-              pk_p[j / 2 + 1] = pack2<kBf16>(pv[2], pv[3]);
-              pk_ds[j / 2] = pack2<kBf16>(ds[0], ds[1]);
-              pk_ds[j / 2 + 1] = pack2<kBf16>(ds[2], ds[3]);
-            }
-          }
-          tmem_st16(tS + cc * 32, pk_p);    // P^T of the chunk over the start of the scores it was made from
-          tmem_st16(tP + cc * 32, pk_ds);   // dS^T of the chunk over the start of its dP^T
-        }
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(pfull0 + buf * 8);
-        buf += 2;
-        if (buf >= C::NBUF) { buf -= C::NBUF; ++rnd; }
-      }
-      if (!ok) break;
-
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sh.item_empty[k % C::NITEM]));
-      have = open_item(k + 1);
-      // (the fields are taken here and not before: carried through the loop they cost the head-dim-64 kernel its last registers)
-      const int b = now.x, h = now.y, kj = now.z * KD_TILE + row;
-      // epilogue of this item: warpgroup g stores EC columns of dK and dV from column g * EC
-      if (n > 0) {
-        ok = mbar_wait<true>(smem_u32(&sh.acc_full), n_acc++ & 1, &sh.abortf, W_K_ACCFULL);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-      }
-      tc_fence_after_sync();
-      constexpr int EC = HD / (2 * C::NSUB);
-      constexpr int ECH = EC < 32 ? EC : 32;   // columns per TMEM load
-      uint16_t* krow = reinterpret_cast<uint16_t*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st + g * EC;
-      uint16_t* vrow = reinterpret_cast<uint16_t*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st + g * EC;
-#pragma unroll
-      for (int cb = 0; cb < EC / ECH; ++cb) {
-        uint32_t rk[ECH], rv[ECH];
-        if (n > 0) {
-          if constexpr (ECH == 16) {
-            tmem_ld16(tbase + lane_base + C::TM_ACC0 + g * EC + cb * ECH, rk);
-            tmem_ld16(tbase + lane_base + C::TM_ACC1 + g * EC + cb * ECH, rv);
-          } else {
-            tmem_ld32(tbase + lane_base + C::TM_ACC0 + g * EC + cb * ECH, rk);
-            tmem_ld32(tbase + lane_base + C::TM_ACC1 + g * EC + cb * ECH, rv);
-          }
-          tmem_wait_ld();
-          if (cb == EC / ECH - 1) {
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh.acc_free));   // the next item's first products may overwrite the accumulators
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < ECH; ++j) { rk[j] = 0u; rv[j] = 0u; }
-        }
-        const int col = g * EC + cb * ECH;
-        if (kF32 && kj < a.T) {
-          float* kw = static_cast<float*>(a.dk) + (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)kj * a.dk_st + col;
-          float* vw = static_cast<float*>(a.dv) + (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)kj * a.dv_st + col;
-          if constexpr (ECH == 16) {
-            store_row16_f32_upto(kw, rk, a.sm_scale, col, a.d_real);
-            store_row16_f32_upto(vw, rv, 1.0f, col, a.d_real);
-          } else {
-            store_row32_f32_upto(kw, rk, a.sm_scale, col, a.d_real);
-            store_row32_f32_upto(vw, rv, 1.0f, col, a.d_real);
-          }
-        } else if (kj < a.T) {
-          if constexpr (ECH == 16) {
-            store_row16_upto<kBf16>(krow + cb * ECH, rk, a.sm_scale, g * EC + cb * ECH, a.d_real);
-            store_row16_upto<kBf16>(vrow + cb * ECH, rv, 1.0f, g * EC + cb * ECH, a.d_real);
-          } else {
-            store_row32_upto<kBf16>(krow + cb * ECH, rk, a.sm_scale, g * EC + cb * ECH, a.d_real);
-            store_row32_upto<kBf16>(vrow + cb * ECH, rv, 1.0f, g * EC + cb * ECH, a.d_real);
-          }
-        }
-      }
-    }  // items
-  }
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc(tbase, 512);
-  if (tid == 0) report_abort(&sh.abortf, a.status);
-  if (a.after_dq != 0) pdl_wait();
-}
-
 template <int HD, bool kBf16, bool kF32>
 static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const float* signs, const kd_plan_layout& L, const PlanView& pv, cudaStream_t stream) {
   using C = BwdCfg<HD>;
@@ -1007,10 +639,8 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const f
   if (f32) { a.do32_sb = f32->d_o.stride_b; a.do32_sh = f32->d_o.stride_h; a.do32_st = f32->d_o.stride_t; }
  
   auto kq = attn_bwd_dq_kernel<HD, kBf16, kF32>;
-  auto kk = attn_bwd_dkdv_kernel<HD, kBf16, kF32>;
-  static SmemOptIn opt_in_q, opt_in_k;
-  cudaError_t e = opt_in_q(kq, C::SMEM_ALLOC);
-  if (e == cudaSuccess) e = opt_in_k(kk, C::SMEM_ALLOC);
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in(kq, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "bwd smem attribute: %s", cudaGetErrorString(e));
   const long long n_items = fused ? 0 : (long long)p.B * p.H * L.NT;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
@@ -1026,7 +656,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const f
     if (phases & 2) return launch_bwd_fused(tmQ, tmK, tmV, tmDO, a, p.dtype, (phases & 1) != 0, stream);
   } else if ((phases & 2) && e == cudaSuccess) {
     a.after_dq = phases & 1;
-    e = launch(kk, grid, C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, a);
+    return launch_bwd_dkdv(tmQ, tmK, tmV, tmDO, a, p.dtype, stream);
   }
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "attn_bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;

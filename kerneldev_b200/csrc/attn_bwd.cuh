@@ -7,7 +7,7 @@ namespace kd {
 struct BwdArgs {
   int B, H, T, NT, NP, Tpad;
   ItemOrder order_of;   // of the two-kernel backward's items
-  int after_dq;      // dK/dV kernel: the dQ kernel of the same call is the kernel before this one on the stream
+  int after_dq;      // fused kernel without dQ: the dQ kernel of the same call is the kernel before this one on the stream
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
@@ -69,5 +69,9 @@ __device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
 // dV in TMEM and adds its dQ partials to a.dq_acc, then a conversion kernel.
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                      const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream);
+
+// The same kernel without dQ: dK and dV of the deterministic backward, behind a kernel for dQ (attn_bwd.cu).
+int launch_bwd_dkdv(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
+                    const BwdArgs& a, int dtype, cudaStream_t stream);
 
 }  // namespace kd

@@ -149,7 +149,9 @@ __device__ __forceinline__ uint64_t ld_shared_pair(const float* p) {
 
 // kF32: dQ, dK and dV are float32 tensors (of a float32 call). The dQ tiles are then scaled and added into dQ itself, which the delta kernel
 // has zeroed: no scratch and no conversion (2 x 4 x 256 x 64: forward and backward 8 launches -> 4, 105 -> 86 us).
-template <int HD_, bool kBf16, bool kF32>
+// kDq: false in the deterministic backward, which forms dQ in a kernel of its own (attn_bwd.cu). What is left here adds in a fixed order: the
+// products of a key tile follow one another in the order of its list.
+template <int HD_, bool kBf16, bool kF32, bool kDq>
 __global__ void __launch_bounds__(FusedCfg<HD_>::THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -186,6 +188,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(bar(i), count);
     fence_barrier_init();
   }
+  if (!kDq && tid == 0 && a.after_dq != 0) {   // see below
+    __threadfence();
+    fence_proxy_async_global();
+  }
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_base_s), 512);
     tmem_relinquish();
@@ -197,7 +203,16 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // the plan, Q, K, V and LSE may be read, and dK and dV written, before the wait (plain reads past L1, which the start of a kernel that
   // overlaps another need not have cleaned). Not so delta, the zeros of the dQ scratch or of a float32 dQ, and dO, which in a float32 call
   // the delta kernel rounds to 16 bits.
-  if (!fa.after_delta) pdl_wait();
+  // Without dQ, directly behind the dQ kernel of the same call, there is nothing to wait for at all: that kernel writes nothing that this one
+  // reads, and lets it start when it has itself waited for the delta kernel. So the last CTAs of the one overlap the first of the other (both
+  // together, with the wait here instead: 1 x 16 x 500 x 128 31.5 us, 23 so; 4 x 16 x 2048 x 64 110.2, 108.2; unmasked 1 x 4 x 2048 x 64 51.5, 34).
+  // What orders delta, and the dO of a float32 call, before the reads here: CUDA promises visibility to the kernel that executes
+  // griddepcontrol.wait behind the writer, which is the dQ kernel, and none through launch_dependents alone. Hence a device-wide
+  // fence on both sides of that hand-over (there behind the wait, here ahead of the block's barrier, with one for the TMA loads); all reads
+  // go past L1. That a dependent kernel starts after launch_dependents has been executed is what remains to be relied on.
+  // The dQ kernel's end is awaited at this one's end, so that whatever comes next finds both complete (what a successor reads ahead of its
+  // own wait is a plan, which no backward writes).
+  if (kDq ? fa.after_delta == 0 : a.after_dq == 0) pdl_wait();
   // The site of this warp's wait that ran out, 0 while none has. There is no wait after it: every role ends at its first, with
   // its copies drained, and raises the flag where all roles meet. All waits of this kernel are such waits (there is no named
   // barrier), so a role whose partner has ended waits for its own limit and ends too.
@@ -381,7 +396,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           ++v_loads;
         }
         if (k == 0) {
-          pdl_wait();   // delta and dO are read from here on
+          if (kDq) pdl_wait();   // delta and dO are read from here on
           pdl_launch_dependents();
         }
         ++k;
@@ -405,7 +420,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             break;
           }
           const uint32_t this_ent = ent;
-          if (e + 1 < n) ent = list[e + 1];
+          if (e + 1 < n) ent = __ldcg(list + e + 1);
           const int qt = this_ent & 0xFF;
           if (!(ok = wait(C::B_QEMPTY + qs, q_parity, W_U_QEMPTY))) break;
           const uint32_t side = s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4);
@@ -421,11 +436,27 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             cp_async16(side + 16 * lane, a.lse + row + q);
             cp_async16(side + KD_TILE * 4 + 16 * lane, a.delta + row + q);
           } else {
+            if (kDq) {
 #pragma unroll 1
-            for (int j = 0; j < 4; ++j) {
-              const size_t r = row + min(q + j, a.T - 1);
-              cp_async4(side + 16 * lane + 4 * j, a.lse + r);
-              cp_async4(side + KD_TILE * 4 + 16 * lane + 4 * j, a.delta + r);
+              for (int j = 0; j < 4; ++j) {
+                const size_t r = row + min(q + j, a.T - 1);
+                cp_async4(side + 16 * lane + 4 * j, a.lse + r);
+                cp_async4(side + KD_TILE * 4 + 16 * lane + 4 * j, a.delta + r);
+              }
+            } else {   // (copies of 4 bytes go through L1, which may hold delta of before the kernel ahead: see above)
+              float l[4], d[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const size_t r = row + min(q + j, a.T - 1);
+                l[j] = __ldcg(a.lse + r);
+                d[j] = __ldcg(a.delta + r);
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                st_shared_u32(side + 16 * lane + 4 * j, __float_as_uint(l[j]));
+                st_shared_u32(side + KD_TILE * 4 + 16 * lane + 4 * j, __float_as_uint(d[j]));
+              }
+              __threadfence_block();   // the arrival below is ordered behind the asynchronous copies alone
             }
           }
           if (HD == 64 && (this_ent >> 8) == KD_TILE_PARTIAL) {
@@ -564,10 +595,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               tc_fence_after_sync();
               product_dk(w, q_mn0 + q_stage * T16, first && w == 0);
             }
-            if (t > 1 && !wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY)) return false;
-            tc_fence_after_sync();
-            product_dq(k_mn0 + (item & 1) * T16);
-            commit_uniform(bar(C::B_DQFULL));
+            if constexpr (kDq) {
+              if (t > 1 && !wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY)) return false;
+              tc_fence_after_sync();
+              product_dq(k_mn0 + (item & 1) * T16);
+              commit_uniform(bar(C::B_DQFULL));
+            }
             commit_uniform(bar(C::B_DSFREE));
             commit_uniform(bar(C::B_QEMPTY + q_stage));
             if (last) {
@@ -658,8 +691,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               }
             }
             tc_fence_after_sync();
-            product_dq(k_mn0);   // over dP^T(t), which dS^T(t) was made from
-            commit_uniform(bar(C::B_DQFULL));
+            if (kDq) {
+              product_dq(k_mn0);   // over dP^T(t), which dS^T(t) was made from
+              commit_uniform(bar(C::B_DQFULL));
+            }
 #pragma unroll 1
             for (int w = 0; w < 2; ++w) product_dk(w, q_mn0 + q_stage * T16, e == 0 && w == 0);
             commit_uniform(bar(C::B_DSFREE));
@@ -681,7 +716,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               }
             }
             if (have) {
-              if (!(ok = wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY))) break;
+              if (kDq && !(ok = wait(C::B_DQEMPTY, t & 1, W_U_DQEMPTY))) break;
               if (last && !(ok = wait(C::B_VFULL, (m + 1) & 1, W_U_VFULL))) break;
               if (!(ok = wait(C::B_DOFULL + do_stage, do_parity, W_U_DOFULL))) break;
               issue_dp();
@@ -964,7 +999,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   } else {
     reg_dealloc<C::REGS_DQ>();
     // ------------------------------ dQ warps: TMEM -> shared memory -> bulk reduction into the fp32 scratch ------------------------------
-    pdl_wait();   // the scratch has been zeroed
+    if (kDq) pdl_wait();   // the scratch has been zeroed
     const int wq = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t stg = s0 + C::SMEM_STG + wq * (C::NSTG * 4096), st_row = static_cast<uint32_t>(lane) * 128u, st_sw = static_cast<uint32_t>(lane & 7);
@@ -1128,7 +1163,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         return true;
       };
       // the item's dQ tiles; dV before the last, dK behind it
-      if constexpr (HD == 64) {
+      if constexpr (!kDq) {
+#pragma unroll 1
+        for (int step = 0; ok && step < 2; ++step) ok = write_out(step == 1, b, h, kt, m);
+      } else if constexpr (HD == 64) {
         for (int e = 0; ok && e < n; ++e) {
           const bool last = e == n - 1;
           ok = (!last || write_out(false, b, h, kt, m)) && dq_tile(e) && (!last || write_out(true, b, h, kt, m));
@@ -1148,6 +1186,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   if (warp == 1) tmem_dealloc(0, 512);
   if (tid == 0) report_abort(abortf, a.status);
+  if (!kDq && a.after_dq != 0) pdl_wait();
 }
 
 // dq[b, h, t, :] = dq_acc[b, h, t, :] * sm_scale in the output dtype; HD / 8 threads per row, 32 bytes in and 16 out each
@@ -1185,7 +1224,7 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
   }
 }
 
-template <int HD, bool kBf16, bool kF32>
+template <int HD, bool kBf16, bool kF32, bool kDq>
 static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                           const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   using C = FusedCfg<HD>;
@@ -1194,8 +1233,9 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   auto encode_out = [&](CUtensorMap* tm, const kd_tensor& t, const char* name) {
     return kF32 ? encode_tensor_map_f32(tm, t, a.B, a.H, a.T, a.d_real, 32, name) : encode_tensor_map(tm, t, a.B, a.H, a.T, a.d_real, dtype, 32, name);
   };
-  int rc = kF32 ? encode_out(&tmAcc, dq, "dq") : encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
-  if (rc == 0) rc = encode_out(&tmDK, dk, "dk");
+  int rc = encode_out(&tmDK, dk, "dk");
+  if (!kDq) tmAcc = tmDK;   // not used
+  else if (rc == 0) rc = kF32 ? encode_out(&tmAcc, dq, "dq") : encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
   if (rc == 0) rc = encode_out(&tmDV, dv, "dv");
   if (rc != 0) return rc;
   const long long n_items = (long long)a.B * a.H * a.NT;
@@ -1203,9 +1243,9 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   FusedArgs fa;
   fa.b = a;
   fa.after_delta = after_delta;
-  // Q, K, V, dO and the dQ scratch. (64 MB: hier T = 8192, D = 128 2470 us instead of 2409; without chunks 3540)
-  fa.order_of = ItemOrder::make(a.B * a.H, a.NT, (double)a.T * (4.0 * a.d_real * 2 + HD * 4.0), 90e6);
-  auto kern = attn_bwd_fused_kernel<HD, kBf16, kF32>;
+  // Q, K, V, dO and, if there is one, the dQ scratch. (64 MB: hier T = 8192, D = 128 2470 us instead of 2409; without chunks 3540)
+  fa.order_of = ItemOrder::make(a.B * a.H, a.NT, (double)a.T * (4.0 * a.d_real * 2 + (kDq ? HD * 4.0 : 0.0)), 90e6);
+  auto kern = attn_bwd_fused_kernel<HD, kBf16, kF32, kDq>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd smem attribute: %s", cudaGetErrorString(e));
@@ -1220,20 +1260,31 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   }
   if (launch_regs < C::REGS_LAUNCH) return set_error(KD_ERR_DEVICE, "fused bwd was built with %d registers per thread, needs %d", launch_regs, C::REGS_LAUNCH);
   e = launch(kern, static_cast<unsigned>(n_items), C::THREADS, C::SMEM_ALLOC, stream, tmQ, tmK, tmV, tmDO, tmAcc, tmDK, tmDV, fa);
-  if (e == cudaSuccess && !kF32 && a.signs != nullptr)
+  if (e == cudaSuccess && kDq && !kF32 && a.signs != nullptr)
     return launch_grad_transform(a.dq_acc, HD, a.sm_scale, a.len, a.signs, dq, dk, a.B, a.H, a.T, a.d_real, dtype, stream);
-  if (e == cudaSuccess && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, RowBlocks<HD>::grid(a.B, a.H, a.T), 256, 0, stream, a);
+  if (e == cudaSuccess && kDq && !kF32) e = launch(attn_bwd_dq_convert_kernel<HD, kBf16>, RowBlocks<HD>::grid(a.B, a.H, a.T), 256, 0, stream, a);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd kernels launch: %s", cudaGetErrorString(e));
   return 0;
 }
 
-int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
-                     const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
+template <bool kDq>
+static int launch_one_pass(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
+                           const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   auto run = [&](auto launch_fn) { return launch_fn(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream); };
   const bool narrow = a.d_real <= 64;
-  if (a.grads_f32) return narrow ? run(launch_fused_t<64, false, true>) : run(launch_fused_t<128, false, true>);
-  if (dtype == KD_BF16) return narrow ? run(launch_fused_t<64, true, false>) : run(launch_fused_t<128, true, false>);
-  return narrow ? run(launch_fused_t<64, false, false>) : run(launch_fused_t<128, false, false>);
+  if (a.grads_f32) return narrow ? run(launch_fused_t<64, false, true, kDq>) : run(launch_fused_t<128, false, true, kDq>);
+  if (dtype == KD_BF16) return narrow ? run(launch_fused_t<64, true, false, kDq>) : run(launch_fused_t<128, true, false, kDq>);
+  return narrow ? run(launch_fused_t<64, false, false, kDq>) : run(launch_fused_t<128, false, false, kDq>);
+}
+
+int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
+                     const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
+  return launch_one_pass<true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
+}
+
+int launch_bwd_dkdv(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
+                    const BwdArgs& a, int dtype, cudaStream_t stream) {
+  return launch_one_pass<false>(tmQ, tmK, tmV, tmDO, a, dtype, false, stream);
 }
 
 }  // namespace kd

@@ -101,6 +101,25 @@ def test_empty_key_tiles_are_written_as_zeros(T, lens, D):
         assert not g[beyond].any() and not g.isnan().any()
 
 
+# dK and dV of the deterministic backward come from the fused kernel without its dQ: the same sums in the same order. T at the edges of tiles, and lengths at
+# which the rows of a head do not begin on 16 bytes; calls behind one another, whose kernels overlap
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (48, torch.float32), (128, torch.float16), (80, torch.float32)])
+@pytest.mark.parametrize("T,lens", [(64, (64, 1)), (128, (128, 70)), (131, (131, 129)), (385, (0, 385)), (1022, (900, 257))])
+def test_both_backwards_give_the_same_dk_and_dv(T, lens, D, dtype):
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import flash_attention
+    B, H = len(lens), 5
+    lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    for seed in range(3):
+        q, k, v, do = (x.to(dtype) for x in rand_inputs(B, H, T, D, torch.float16, T + D + seed, DEV))
+        x = [t.requires_grad_() for t in (q, k, v)]
+        want = torch.autograd.grad(flash_attention(*x, lens=lens), x, do)
+        got = torch.autograd.grad(flash_attention(*x, lens=lens, deterministic=True), x, do)
+        again = torch.autograd.grad(flash_attention(*x, lens=lens, deterministic=True), x, do)
+        assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+        assert all(torch.equal(a, b) for a, b in zip(got, again))
+
+
 # dQ and dK of transformed Q and K, transformed back by the last pass of the fused backward, against the transform's own backward. T and lens at the
 # edges of its blocks (128 rows at head dim 16, 64 above)
 @pytest.mark.parametrize("D,dtype", [(16, torch.bfloat16), (32, torch.float16), (64, torch.bfloat16), (128, torch.float16)])
