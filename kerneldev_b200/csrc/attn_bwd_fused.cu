@@ -74,6 +74,7 @@ struct FusedArgs {
   BwdArgs b;
   ItemOrder order_of;
   int after_delta;   // the delta kernel of the same call is the kernel before this one on the stream
+  int direct;        // without dQ: dK or dV has strides that no tensor map describes, and is written row by row
 };
 
 template <int HD_>
@@ -293,7 +294,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // dK = dV = 0 for an item without entries
       auto write_zeros = [&](const int4& z) {
         using Out = std::conditional_t<kF32, float, uint16_t>;
-        if constexpr (HD == 64) {
+        if (HD == 64 && (kDq || fa.direct == 0)) {
           // Items without entries come last and nothing hides them there: 14,500 of the 87,000 cycles of a CTA of hierarchical 4 x 16 x 2048
           // x 64 lie behind its last tile. So they leave through the copy engine, a lane per 32 rows, and cost this warp no more than
           // the look-up (stores by the lanes before: that backward 71.1 -> 67.8 us, 8 x 16 x 2048 x 64 141.7 -> 132.5, 16 x 16 x 4096 x 64
@@ -1048,6 +1049,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(C::B_ACCFREE + (is_k ? 1 : 0)));
           }
+          if (!kDq && fa.direct != 0) {
+            if (key0 + lane < a.T) {
+              const size_t at = is_k ? (size_t)b * a.dk_sb + (size_t)h * a.dk_sh + (size_t)(key0 + lane) * a.dk_st : (size_t)b * a.dv_sb + (size_t)h * a.dv_sh + (size_t)(key0 + lane) * a.dv_st;
+              void* out = is_k ? a.dk : a.dv;
+              if constexpr (kF32) store_row32_f32_upto(static_cast<float*>(out) + at + col + half * 32, r, f, col + half * 32, a.d_real);
+              else store_row32_upto<kBf16>(static_cast<uint16_t*>(out) + at + col + half * 32, r, f, col + half * 32, a.d_real);
+            }
+            continue;
+          }
           if constexpr (kF32 && C::NSTG == 1) {   // a box at a time
             if (half == 1) {
               if (lane == 0) bulk_wait_group_read0();
@@ -1075,7 +1085,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && key0 < a.T && col < a.d_real) {
+        if (lane == 0 && key0 < a.T && col < a.d_real && (kDq || fa.direct == 0)) {
           if (kF32 && C::NSTG == 1) {
             if (col + 32 < a.d_real) tma_store_4d(is_k ? &tmDK : &tmDV, buf, col + 32, key0, h, b);
           } else {
@@ -1233,14 +1243,21 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   auto encode_out = [&](CUtensorMap* tm, const kd_tensor& t, const char* name) {
     return kF32 ? encode_tensor_map_f32(tm, t, a.B, a.H, a.T, a.d_real, 32, name) : encode_tensor_map(tm, t, a.B, a.H, a.T, a.d_real, dtype, 32, name);
   };
-  int rc = encode_out(&tmDK, dk, "dk");
-  if (!kDq) tmAcc = tmDK;   // not used
-  else if (rc == 0) rc = kF32 ? encode_out(&tmAcc, dq, "dq") : encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
-  if (rc == 0) rc = encode_out(&tmDV, dv, "dv");
+  FusedArgs fa;
+  fa.direct = 0;
+  int rc = 0;
+  if (!kDq) {
+    fa.direct = encode_out(&tmDK, dk, nullptr) != 0 || encode_out(&tmDV, dv, nullptr) != 0;
+    if (fa.direct) tmDK = tmDV = tmQ;   // not used
+    tmAcc = tmDK;                       // nor is this
+  } else {
+    rc = kF32 ? encode_out(&tmAcc, dq, "dq") : encode_tensor_map_f32_rows(&tmAcc, a.dq_acc, a.B * a.H, a.T, HD, 32, "dq_acc");
+    if (rc == 0) rc = encode_out(&tmDK, dk, "dk");
+    if (rc == 0) rc = encode_out(&tmDV, dv, "dv");
+  }
   if (rc != 0) return rc;
   const long long n_items = (long long)a.B * a.H * a.NT;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");
-  FusedArgs fa;
   fa.b = a;
   fa.after_delta = after_delta;
   // Q, K, V, dO and, if there is one, the dQ scratch. (64 MB: hier T = 8192, D = 128 2470 us instead of 2409; without chunks 3540)

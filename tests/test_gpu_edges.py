@@ -429,6 +429,32 @@ def test_forward_into_rows_in_descending_order(D):
     assert torch.equal(back.flip(2), want)
 
 
+# dK and dV of the deterministic backward with strides that no tensor map describes: written row by row, key tiles that no query sees too
+@pytest.mark.parametrize("T,lens", [(159, (159, 100)), (385, (385, 129))])
+@pytest.mark.parametrize("D", [48, 64, 80])
+def test_deterministic_backward_into_rows_in_descending_order(T, lens, D):
+    import ctypes
+    from tests.helpers import rand_inputs
+    from kerneldev_b200 import _capi
+    from kerneldev_b200.original_kernel import _backward, _forward, _kd_tensor, _params
+    from kerneldev_b200.plan import AttentionPlan
+    B, H = 2, 7
+    q, k, v, do = (x.to(DEV) for x in rand_inputs(B, H, T, D, torch.bfloat16, seed=T + D))
+    plan = AttentionPlan(B, T, torch.device(DEV), lens=torch.tensor(lens, dtype=torch.int32, device=DEV), causal=True)
+    o, lse = _forward(q, k, v, plan, 0.125)
+    want = _backward(q, k, v, o, lse, do, plan, 0.125, deterministic=True)
+    dq, dk, dv = (torch.full_like(q, float("nan")) for _ in range(3))
+    delta = torch.empty_like(lse)
+    p = _params(q, k, v, o, lse, plan, 0.125)
+    p.d_o, p.dq, p.delta, p.bwd_mode = _kd_tensor(do), _kd_tensor(dq), delta.data_ptr(), 0
+    p.dk, p.dv = (_capi.KdTensor(x.data_ptr() + (T - 1) * D * 2, H * T * D, T * D, -D) for x in (dk, dv))
+    lib = _capi.load()
+    torch.cuda.synchronize()
+    assert lib.kd_attn_bwd(ctypes.byref(p), torch.cuda.current_stream().cuda_stream) == 0, lib.kd_last_error()
+    for got, ref in zip((dq, dk.flip(2), dv.flip(2)), want):
+        assert torch.equal(got, ref)
+
+
 # 312 pairs of query tiles and 468 key tiles (odd: 780 tiles, some of 1 token), more than SMs: CTAs of all float32 kernels run on into further items, among them runs
 # of tiles without keys or queries. O leaves as float32 beside the 16-bit O of the boxes, dK and dV through both staging boxes between dQ tiles
 @pytest.mark.parametrize("deterministic", [False, True])
