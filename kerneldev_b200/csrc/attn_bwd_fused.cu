@@ -16,9 +16,11 @@
 // the scratch to the output dtype afterwards. The delta kernel, which runs first anyway, zeroes the
 // scratch.
 //
-// What bounds it. No single unit. Per tile at HD = 64 (cycles of an SM): products 1,540, exponentials 1,024, shared
+// What bounds it. Per tile at HD = 64 (cycles of an SM): products 1,540, exponentials 1,024, shared
 // memory 2,450 of its 128 bytes a cycle (1,408 of them the products' operands), instruction issue 1,350 of each
-// scheduler; a tile takes 3,000 with full lists. Taking any one of these out of the kernel changes it by 3 to 8 %.
+// scheduler; a tile takes 2,500 with full lists, so it is shared memory's rate that is left (3,000 when long waits and late products
+// came on top), and 2,700-2,800 with lists of 4 to 9 tiles. At HD = 128 a tile takes 3,900, and 3,300 without the additions of
+// dQ, for which the L2 needs 3,200 from all SMs at once.
 //  * Shared memory is kept free by the layout of the compute warps' registers: they read S^T and dP^T from TMEM in the
 //    16x256b shape, in which a thread owns four key rows and a quarter of the columns, as in an mma fragment, so that a
 //    warp needs LSE and delta of a column once and not 32 times; P^T goes back in the 16x128b shape and dS^T leaves
@@ -63,6 +65,7 @@
 // thread, sixteen compute warps and heads per CTA (HD = 64) and the two-kernel form (HD = 128):
 //   bf16 B16 H16 T4096 D64 hierarchical 1291 -> 1175-1230    bf16 B8 H16 T2048 D64 causal 338 -> 284
 //   bf16 B8 H16 T2048 D128 causal 644 -> 415                 fp16 B4 H32 T8192 D128 hierarchical 3944 -> 2420
+// The first is 890-950 now, the second 250-270.
 #include <algorithm>
 #include <type_traits>
 
