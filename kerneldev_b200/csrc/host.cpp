@@ -23,6 +23,7 @@
 #include <chrono>
 #include <deque>
 #include <list>
+#include <memory>
 #include <mutex>
 #include <unordered_map>
 
@@ -148,6 +149,18 @@ bool check_every_launch() {
   return e != nullptr && e[0] == '1' && e[1] == 0;
 }
 
+// Whether a stream is being captured, and into which graph.
+struct Capture {
+  bool active;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  explicit Capture(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    active = cudaStreamGetCaptureInfo_v2(stream, &status, &id, &graph) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+    if (status != cudaStreamCaptureStatusActive) graph = nullptr;
+  }
+};
+
 struct Plan {
   int64_t B, T;
   at::Device device;
@@ -169,15 +182,12 @@ struct Plan {
   at::cuda::CUDAEvent built;
   std::atomic<cudaStream_t> used_on{reinterpret_cast<cudaStream_t>(-1)};   // the stream of the plan's last eager launch
 
-  // kd_attn_params.plan_ready for a launch on `stream`. A captured launch says nothing about the stream it was captured from.
-  bool ready_on(cudaStream_t stream) const {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    return used_on.load() == stream && cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-  }
-  void launched_on(cudaStream_t stream) {
-    if (used_on.load() == stream) return;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) used_on.store(stream);
+  std::atomic<unsigned long long> held_by{0};   // the last capture whose graph has been given this plan to hold
+
+  // kd_attn_params.plan_ready for a launch. A captured launch says nothing about the stream it was captured from.
+  bool ready_on(cudaStream_t stream, const Capture& capture) const { return !capture.active && used_on.load() == stream; }
+  void launched_on(cudaStream_t stream, const Capture& capture) {
+    if (!capture.active && used_on.load() != stream) used_on.store(stream);
   }
 
   Plan(int64_t B_, int64_t T_, at::Device dev, const OptTensor& in_span, const OptTensor& span_id, const OptTensor& is_prefix,
@@ -276,6 +286,49 @@ struct Plan {
   }
 };
 using PlanPtr = std::shared_ptr<Plan>;
+
+// Plans that graphs have let go of. The driver runs a graph's destructors on a thread of its own, where no CUDA call may be made, and a plan
+// that goes frees memory and an event: the next look-up of a plan does.
+class LetGo {
+ public:
+  void add(PlanPtr plan) {
+    std::lock_guard<std::mutex> lock(m_);
+    plans_.push_back(std::move(plan));
+    any_.store(true);
+  }
+  void clear() {
+    if (!any_.load()) return;
+    std::vector<PlanPtr> gone;   // destroyed after the lock is released
+    std::lock_guard<std::mutex> lock(m_);
+    gone.swap(plans_);
+    any_.store(false);
+  }
+
+ private:
+  std::mutex m_;
+  std::vector<PlanPtr> plans_;
+  std::atomic<bool> any_{false};
+};
+LetGo& let_go() {
+  static LetGo* l = new LetGo;   // never destroyed: graphs outlive the statics of this file
+  return *l;
+}
+
+// A captured launch has the plan's address and nothing else, and the cache may drop the plan: the graph keeps it, as do the graphs made from it.
+void hold_for_graph(const PlanPtr& plan, const Capture& capture) {
+  if (capture.graph == nullptr || plan->held_by.load() == capture.id) return;
+  auto held = std::make_unique<PlanPtr>(plan);
+  cudaUserObject_t object;
+  C10_CUDA_CHECK(cudaUserObjectCreate(&object, held.get(), [](void* p) {
+    std::unique_ptr<PlanPtr> h(static_cast<PlanPtr*>(p));
+    let_go().add(std::move(*h));
+  }, 1, cudaUserObjectNoDestructorSync));
+  held.release();
+  const cudaError_t e = cudaGraphRetainUserObject(capture.graph, object, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) cudaUserObjectRelease(object, 1);
+  C10_CUDA_CHECK(e);
+  plan->held_by.store(capture.id);
+}
 
 // The cache key: identity, version and geometry of the metadata tensors (the plan keeps their memory alive, so an address
 // cannot be reused while its plan is cached) and the flags of the mask.
@@ -376,6 +429,7 @@ bool fill_slot(PlanKey::Slot& s, const OptTensor& t) {
 PlanPtr get_plan(int64_t B, int64_t T, at::Device device, const OptTensor& in_span, const OptTensor& span_id,
                  const OptTensor& is_prefix, const OptTensor& lens, bool causal, bool rules) {
   if (!device.has_index()) device = at::Device(device.type(), at::cuda::current_device());
+  let_go().clear();
   PlanKey key{B, T, device.index(), (causal ? 1 : 0) | (rules ? 2 : 0), {}};
   const bool keyed = fill_slot(key.slot[0], in_span) && fill_slot(key.slot[1], span_id) && fill_slot(key.slot[2], is_prefix) &&
                      fill_slot(key.slot[3], lens);
@@ -450,9 +504,11 @@ std::tuple<Tensor, Tensor> forward(const Tensor& q_, const Tensor& k_, const Ten
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-  p.plan_ready = plan->ready_on(stream) ? 1 : 0;
+  const Capture capture(stream);
+  hold_for_graph(plan, capture);
+  p.plan_ready = plan->ready_on(stream, capture) ? 1 : 0;
   check(o32 != nullptr ? lib.attn_fwd_f32(&p, &f, stream) : lib.attn_fwd(&p, stream));
-  plan->launched_on(stream);
+  plan->launched_on(stream, capture);
   plan->after_launch();
   return {o, lse};
 }
@@ -498,7 +554,9 @@ std::tuple<Tensor, Tensor, Tensor> backward(const Tensor& q_, const Tensor& k_, 
   plan->poll();
   c10::cuda::CUDAGuard guard(q.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
-  p.plan_ready = plan->ready_on(stream) ? 1 : 0;
+  const Capture capture(stream);
+  hold_for_graph(plan, capture);
+  p.plan_ready = plan->ready_on(stream, capture) ? 1 : 0;
   check(f32 ? lib.attn_bwd_f32(&p, &f, stream) : signs != nullptr ? lib.attn_bwd_hadamard(&p, signs, stream) : lib.attn_bwd(&p, stream));
   plan->after_launch();
   return {dq, dk, dv};

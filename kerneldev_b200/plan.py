@@ -6,7 +6,8 @@ metadata (``in_span``, ``span_id``, ``is_prefix``, ``lens``, ``causal``), not on
 plan serves all heads and -- because ``model.GPTModel`` passes the same three metadata tensors
 to every layer (model.py:243-244) -- all layers of a step. Plans are cached on the identity and
 version of the metadata tensors (the cache keeps their memory alive, so an address cannot be
-reused while its plan is cached; a plan whose metadata nobody else holds any more leaves the cache with the next new plan). Metadata rewritten in place through raw pointers -- by
+reused while its plan is cached; a plan whose metadata nobody else holds any more leaves the cache with the next new plan). A CUDA
+graph keeps the plans that its launches read, whatever becomes of the cache. Metadata rewritten in place through raw pointers -- by
 kd_metadata_from_tokens into preallocated buffers, or through ``.data`` -- does not change a tensor's
 version: call ``clear_plan_cache()`` after such a write.
 

@@ -392,3 +392,72 @@ def test_cached_plans_whose_metadata_is_gone_leave_the_cache():
     assert get_plan(B, T, dev, span, None, None, None, True, True)._core is alone
     assert get_plan(B, T, dev, None, None, None, None, True, False)._core is plain
     clear_plan_cache()
+
+
+@pytest.mark.parametrize("gone", ["metadata", "cache"])
+@pytest.mark.parametrize("grad", [False, True])
+def test_graphs_keep_the_plans_they_read(monkeypatch, grad, gone):
+    """A captured launch has the address of its plan: the memory stays the plan's when its metadata is gone and newer plans come, or when the
+    cache is cleared, and is given back when the graph goes."""
+    monkeypatch.setenv("KD_CHECK_STATUS", "0")   # a check waits for the device
+    import gc
+    import time
+    from kerneldev_b200 import clear_plan_cache, flash_attention
+    from kerneldev_b200.plan import _CACHE
+    B, H, T, D = 2, 3, 700, 64
+    q, k, v, do = (torch.randn((B, H, T, D), device=DEV, dtype=torch.bfloat16) for _ in range(4))
+
+    def plain_plan(length):
+        flash_attention(q, k, v, lens=torch.tensor([length] * B, dtype=torch.int32, device=DEV))
+
+    def call(lens):
+        if not grad:
+            with torch.no_grad():
+                return (flash_attention(q, k, v, lens=lens),)
+        o = flash_attention(*(x.detach().requires_grad_() for x in (q, k, v)), lens=lens, deterministic=True)
+        return (o.detach(), *o.grad_fn(do))
+
+    clear_plan_cache()
+    lens = torch.tensor([T, 430], dtype=torch.int32, device=DEV)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = [x.clone() for x in call(lens)]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            outs = call(lens)
+    torch.cuda.synchronize()
+    (plan,) = _CACHE.values()
+    first, nbytes = plan.ptr, plan.layout.total
+    del plan
+    if gone == "metadata":
+        del lens
+    else:
+        clear_plan_cache()
+    with torch.cuda.stream(side):   # whose allocations the plan's memory would go to
+        for length in range(1, 9):
+            plain_plan(length)
+        blocks = [torch.full((nbytes,), 255, dtype=torch.uint8, device=DEV) for _ in range(16)]
+    torch.cuda.synchronize()
+    # (before the replay: on memory that is not the plan's any more it would read anything)
+    for p in [p.ptr for p in _CACHE.values()] + [x.data_ptr() for x in blocks]:
+        assert p + nbytes <= first or first + nbytes <= p
+    for x in outs:
+        x.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(outs, want))
+    # the graph's end gives the plan back (its destructors run on a thread of the driver's)
+    del blocks, outs, want
+    clear_plan_cache()
+    plain_plan(9)
+    held = torch.cuda.memory_allocated()
+    del graph
+    gc.collect()
+    deadline = time.time() + 10
+    while torch.cuda.memory_allocated() > held - nbytes and time.time() < deadline:
+        plain_plan(9)
+        clear_plan_cache()
+        time.sleep(0.05)
+    assert torch.cuda.memory_allocated() <= held - nbytes
