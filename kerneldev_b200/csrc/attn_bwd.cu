@@ -311,8 +311,9 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
 // tile.   M1(i): S_i = Q K_i^T, dP_i = dO V_i^T      M2(i): dQ += dS_i K_i
 // The producer and the issuers run on into the next item while the compute warps finish the current one.
 // kF32: of a float32 call, whose gradients are float32. (As a branch of the float16 kernels: causal 8 x 16 x 2048 x 128 610.8 us, 609.4 so; level at head dim 64.)
+// kWords: the plan has the PARTIAL tiles' bits (see KD_WORDS_LIMIT).
 // =========================================================================================
-template <int HD, bool kBf16, bool kF32>
+template <int HD, bool kBf16, bool kF32, bool kWords>
 __global__ void __launch_bounds__(BwdCfg<HD>::THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -457,9 +458,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     for (int cc = 0; cc < CPT; ++cc) mk_next[cc] = 0u;
     auto fetch_words = [&](uint32_t entry) {
       if ((entry >> 8) != KD_TILE_PARTIAL) return;
-      const uint32_t* src = words + (entry & 0xFFu) * static_cast<uint32_t>(KD_WORDS);
+      if constexpr (kWords) {
+        const uint32_t* src = words + (entry & 0xFFu) * static_cast<uint32_t>(KD_WORDS);
 #pragma unroll
-      for (int cc = 0; cc < CPT; ++cc) mk_next[cc] = __ldcg(src + cc * KD_TILE);
+        for (int cc = 0; cc < CPT; ++cc) mk_next[cc] = __ldcg(src + cc * KD_TILE);
+      } else {
+        form_words<CPT>(a.desc + (size_t)it.x * a.Tpad, a.tilebits + (size_t)it.x * a.NT * 32, it.z * KD_TILE + row, entry & 0xFFu, first_word, lane, mk_next);
+      }
     };
     // The next item's header, first entry and scalars are fetched before the epilogue.
     uint32_t ent_next = 0u;
@@ -471,7 +476,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       it = uniform(sh.items[slot]);
       if (it.w < 0) return false;
       list = lists + slot * 128;
-      words = a.words + ((size_t)it.x * a.NT + it.z) * a.NT * KD_WORDS + first_word * KD_TILE + row;
+      if (kWords) words = a.words + ((size_t)it.x * a.NT + it.z) * a.NT * KD_WORDS + first_word * KD_TILE + row;
       if (it.w > 0) {
         ent_next = list[0];
         fetch_words(ent_next);
@@ -619,6 +624,7 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const f
   a.sm_scale = p.sm_scale;
   a.words = pv.words; a.len = pv.len; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list;
   a.bwd_cnt = pv.bwd_cnt; a.bwd_list = pv.bwd_list; a.status = pv.status; a.order = pv.order;
+  a.desc = pv.desc; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.d_o = p.d_o.ptr; a.do_sb = p.d_o.stride_b; a.do_sh = p.d_o.stride_h; a.do_st = p.d_o.stride_t;
   a.lse = p.lse; a.delta = p.delta;
@@ -638,9 +644,9 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const f
   a.d_o32 = f32 ? static_cast<const float*>(f32->d_o.ptr) : nullptr;
   if (f32) { a.do32_sb = f32->d_o.stride_b; a.do32_sh = f32->d_o.stride_h; a.do32_st = f32->d_o.stride_t; }
  
-  auto kq = attn_bwd_dq_kernel<HD, kBf16, kF32>;
-  static SmemOptIn opt_in;
-  cudaError_t e = opt_in(kq, C::SMEM_ALLOC);
+  auto kq = pv.words != nullptr ? attn_bwd_dq_kernel<HD, kBf16, kF32, true> : attn_bwd_dq_kernel<HD, kBf16, kF32, false>;
+  static SmemOptIn opt_in[2];
+  cudaError_t e = opt_in[pv.words != nullptr](kq, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "bwd smem attribute: %s", cudaGetErrorString(e));
   const long long n_items = fused ? 0 : (long long)p.B * p.H * L.NT;
   if (n_items > 0x7FFFFFFF) return set_error(KD_ERR_LIMIT, "B * H * ceil(T / 128) exceeds 2^31 - 1");

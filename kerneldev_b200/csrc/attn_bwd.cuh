@@ -11,7 +11,7 @@ struct BwdArgs {
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
   float sm_scale;
-  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles
+  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles, or null
   const int32_t* fwd_cnt;
   const uint16_t* fwd_list;
   const int32_t* bwd_cnt;
@@ -39,6 +39,8 @@ struct BwdArgs {
   const int32_t* len;   // [B] tokens that are not padding (at the end: the fused kernel of head dim 64 is 2 % slower with its other arguments elsewhere)
   const float* signs;   // null, or Q and K are Hadamard transforms with these signs, and dQ and dK are wanted of what they were made from
   int len_ready;     // the plan may be read by the delta kernel before the wait for the kernel ahead
+  const uint32_t* desc;       // for kernels without words: the tokens' descriptors,
+  const uint32_t* tilebits;   // [B][NT][8][4] class masks of every tile
 };
 
 // How the delta and the conversion kernel (256 threads) divide the rows: a block per ROWS rows of a head, HD / 8 threads to a row, three rows to a

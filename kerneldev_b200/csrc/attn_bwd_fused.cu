@@ -155,7 +155,8 @@ __device__ __forceinline__ uint64_t ld_shared_pair(const float* p) {
 // has zeroed: no scratch and no conversion (2 x 4 x 256 x 64: forward and backward 8 launches -> 4, 105 -> 86 us).
 // kDq: false in the deterministic backward, which forms dQ in a kernel of its own (attn_bwd.cu). What is left here adds in a fixed order: the
 // products of a key tile follow one another in the order of its list.
-template <int HD_, bool kBf16, bool kF32, bool kDq>
+// kWords: the plan has the PARTIAL tiles' bits (see KD_WORDS_LIMIT); without them they are formed where they would be read.
+template <int HD_, bool kBf16, bool kF32, bool kDq, bool kWords>
 __global__ void __launch_bounds__(FusedCfg<HD_>::THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -464,9 +465,20 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
           }
           if (HD == 64 && (this_ent >> 8) == KD_TILE_PARTIAL) {
-            const uint32_t* src = a.words + (((size_t)b * a.NT + qt) * a.NT + kt) * KD_WORDS + 4 * lane;
+            if constexpr (kWords) {
+              const uint32_t* src = a.words + (((size_t)b * a.NT + qt) * a.NT + kt) * KD_WORDS + 4 * lane;
 #pragma unroll
-            for (int w = 0; w < 4; ++w) cp_async16(side + (C::SIDE_BITS + w * KD_TILE) * 4 + 16 * lane, src + w * KD_TILE);
+              for (int w = 0; w < 4; ++w) cp_async16(side + (C::SIDE_BITS + w * KD_TILE) * 4 + 16 * lane, src + w * KD_TILE);
+            } else {
+#pragma unroll 1
+              for (int r = 0; r < 4; ++r) {   // 32 queries at a time
+                uint32_t mk[4];
+                form_words<4>(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, qt * KD_TILE + r * 32 + lane, kt, 0, lane, mk);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) st_shared_u32(side + (C::SIDE_BITS + w * KD_TILE + r * 32 + lane) * 4, mk[w]);
+              }
+              __threadfence_block();   // (as above)
+            }
           }
           cp_async_mbar_arrive(bar(C::B_QFULL + qs));
           ++q_tiles;
@@ -918,9 +930,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const bool partial = (ent >> 8) == KD_TILE_PARTIAL;
         uint32_t mk[2] = {0u, 0u};   // of a PARTIAL tile: the words of queries 64 w + lane and + 32 for the warp's keys, requested ahead of the wait
         if (partial) {
-          const uint32_t* src = a.words + (((size_t)b * a.NT + (ent & 0xFF)) * a.NT + kt) * KD_WORDS + wq * KD_TILE + w * 64 + lane;
-          mk[0] = __ldcg(src);
-          mk[1] = __ldcg(src + 32);
+          if constexpr (kWords) {
+            const uint32_t* src = a.words + (((size_t)b * a.NT + (ent & 0xFF)) * a.NT + kt) * KD_WORDS + wq * KD_TILE + w * 64 + lane;
+            mk[0] = __ldcg(src);
+            mk[1] = __ldcg(src + 32);
+          } else {
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+              form_words<1>(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, static_cast<int>(ent & 0xFF) * KD_TILE + w * 64 + r * 32 + lane, kt, wq, lane, mk + r);
+          }
         }
         // LSE and delta of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here
         const float* side = sSide + qs * C::SIDE_WORDS;
@@ -1237,7 +1255,7 @@ __global__ void __launch_bounds__(256) attn_bwd_dq_convert_kernel(const BwdArgs 
   }
 }
 
-template <int HD, bool kBf16, bool kF32, bool kDq>
+template <int HD, bool kBf16, bool kF32, bool kDq, bool kWords>
 static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                           const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   using C = FusedCfg<HD>;
@@ -1265,7 +1283,7 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   fa.after_delta = after_delta;
   // Q, K, V, dO and, if there is one, the dQ scratch. (64 MB: hier T = 8192, D = 128 2470 us instead of 2409; without chunks 3540)
   fa.order_of = ItemOrder::make(a.B * a.H, a.NT, (double)a.T * (4.0 * a.d_real * 2 + (kDq ? HD * 4.0 : 0.0)), 90e6);
-  auto kern = attn_bwd_fused_kernel<HD, kBf16, kF32, kDq>;
+  auto kern = attn_bwd_fused_kernel<HD, kBf16, kF32, kDq, kWords>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fused bwd smem attribute: %s", cudaGetErrorString(e));
@@ -1287,24 +1305,26 @@ static int launch_fused_t(const CUtensorMap& tmQ, const CUtensorMap& tmK, const 
   return 0;
 }
 
-template <bool kDq>
+template <bool kDq, bool kWords>
 static int launch_one_pass(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                            const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
   auto run = [&](auto launch_fn) { return launch_fn(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream); };
   const bool narrow = a.d_real <= 64;
-  if (a.grads_f32) return narrow ? run(launch_fused_t<64, false, true, kDq>) : run(launch_fused_t<128, false, true, kDq>);
-  if (dtype == KD_BF16) return narrow ? run(launch_fused_t<64, true, false, kDq>) : run(launch_fused_t<128, true, false, kDq>);
-  return narrow ? run(launch_fused_t<64, false, false, kDq>) : run(launch_fused_t<128, false, false, kDq>);
+  if (a.grads_f32) return narrow ? run(launch_fused_t<64, false, true, kDq, kWords>) : run(launch_fused_t<128, false, true, kDq, kWords>);
+  if (dtype == KD_BF16) return narrow ? run(launch_fused_t<64, true, false, kDq, kWords>) : run(launch_fused_t<128, true, false, kDq, kWords>);
+  return narrow ? run(launch_fused_t<64, false, false, kDq, kWords>) : run(launch_fused_t<128, false, false, kDq, kWords>);
 }
 
 int launch_bwd_fused(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                      const BwdArgs& a, int dtype, bool after_delta, cudaStream_t stream) {
-  return launch_one_pass<true>(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
+  const auto run = a.words != nullptr ? launch_one_pass<true, true> : launch_one_pass<true, false>;
+  return run(tmQ, tmK, tmV, tmDO, a, dtype, after_delta, stream);
 }
 
 int launch_bwd_dkdv(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                     const BwdArgs& a, int dtype, cudaStream_t stream) {
-  return launch_one_pass<false>(tmQ, tmK, tmV, tmDO, a, dtype, false, stream);
+  const auto run = a.words != nullptr ? launch_one_pass<false, true> : launch_one_pass<false, false>;
+  return run(tmQ, tmK, tmV, tmDO, a, dtype, false, stream);
 }
 
 }  // namespace kd

@@ -27,6 +27,25 @@ namespace kd {
 // score and of a row maximum without keys (-inf both); raised to FLT_MIN it leaves every exponential at 1, as the smaller one would.
 inline float scale_log2_of(float sm_scale) { return std::max(sm_scale * 1.4426950408889634f, FLT_MIN); }
 
+// Words w0 .. w0 + W - 1 of key tile kt for the query rows of a warp, of which this lane has row qi: what a plan's words hold of a PARTIAL tile, for
+// plans without them. desc, tilebits: the sequence's.
+template <int W>
+__device__ __forceinline__ void form_words(const uint32_t* desc, const uint32_t* tilebits, int qi, int kt, int w0, int lane, uint32_t* m) {
+  const uint32_t qd = __ldcg(desc + qi);
+  const uint32_t* tb = tilebits + kt * 32 + w0;
+  uint32_t kd[W], pre[W], ctx[W], ins[W], any = 0u;
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    kd[w] = __ldcg(desc + kt * KD_TILE + (w0 + w) * 32 + lane);
+    pre[w] = __ldcg(tb + 4 * TB_PRE + w);
+    ctx[w] = __ldcg(tb + 4 * TB_CTX + w);
+    ins[w] = __ldcg(tb + 4 * TB_INS + w);
+    any |= ins[w];
+  }
+  query_row_mask<W>(qd, qi, kt * KD_TILE + w0 * 32, pre, ctx, ins, m);
+  add_same_span<W>(qd, any != 0u, kd, m);
+}
+
 // High words of the two descriptor kinds used here (layout, version, stride byte offset 1024);
 // the low word carries the start address and the leading byte offset.
 __device__ __forceinline__ uint32_t desc_hi_sw128() {

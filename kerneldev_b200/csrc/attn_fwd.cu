@@ -97,7 +97,8 @@ struct FwdCfg {
 
 // kF32: of a float32 call: O goes to a float32 tensor, and to a 16-bit one where there will be a backward. (As a branch of the float16 kernels the
 // second store cost short lists above head dim 64 4 %.)
-template <bool kBf16, bool kF32>
+// kWords: the plan has the PARTIAL tiles' bits (see KD_WORDS_LIMIT).
+template <bool kBf16, bool kF32, bool kWords>
 __global__ void __launch_bounds__(FwdCfg::THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const FwdArgs a) {
@@ -395,14 +396,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t* words = a.words;   // of this thread's query in the item's query tile
     auto fetch_words = [&](uint32_t ent) {
       if (entry_class(ent, i) != KD_TILE_PARTIAL) return;
-      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
+      if constexpr (kWords) {
+        const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
+        for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
+      } else {
+        form_words<NW>(a.desc + (size_t)it.x * a.Tpad, a.tilebits + (size_t)it.x * a.NT * 32, (2 * it.z + i) * KD_TILE + row, ent & 0xFF, half * NW, lane, mk);
+      }
     };
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
-      words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + half * NW * KD_TILE + row;
+      if (kWords) words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + half * NW * KD_TILE + row;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
       const int only = it.w >> 24;
       const bool mine = only == 0 || only == i + 1;
@@ -591,10 +596,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (tid == 0) report_abort(abortf, a.status);
 }
 
-template <bool kBf16, bool kF32>
+template <bool kBf16, bool kF32, bool kWords>
 static int launch_fwd_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmO,
                         cudaStream_t stream) {
-  auto kern = attn_fwd_kernel<kBf16, kF32>;
+  auto kern = attn_fwd_kernel<kBf16, kF32, kWords>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, FwdCfg::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
@@ -623,7 +628,7 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   a.order_of = ItemOrder::make(p.B * p.H, L.NP << a.split, (double)p.T * p.D * 2 * 4, 64e6);
   a.plan_ready = p.plan_ready;
   a.words = pv.words; a.fwd_cnt = pv.fwd_cnt; a.fwd_list = pv.fwd_list; a.status = pv.status;
-  a.order = pv.order;
+  a.order = pv.order; a.desc = pv.desc; a.tilebits = pv.tilebits;
   a.o = p.o.ptr; a.o_sb = p.o.stride_b; a.o_sh = p.o.stride_h; a.o_st = p.o.stride_t;
   a.o32 = f32 ? static_cast<float*>(f32->o.ptr) : nullptr;
   if (f32) { a.o32_sb = f32->o.stride_b; a.o32_sh = f32->o.stride_h; a.o32_st = f32->o.stride_t; }
@@ -641,7 +646,8 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   CUtensorMap tmO = tmQ;
   a.o_tma = n_items > sm_count() && p.o.ptr != nullptr && encode_tensor_map(&tmO, p.o, p.B, p.H, p.T, p.D, p.dtype, 32, nullptr, 64) == 0 ? 1 : 0;
   auto run = [&](auto launch_fn) { return launch_fn(n_items, a, tmQ, tmK, tmV, tmO, stream); };
-  return f32 ? run(launch_fwd_t<false, true>) : p.dtype == KD_BF16 ? run(launch_fwd_t<true, false>) : run(launch_fwd_t<false, false>);
+  if (a.words == nullptr) return f32 ? run(launch_fwd_t<false, true, false>) : p.dtype == KD_BF16 ? run(launch_fwd_t<true, false, false>) : run(launch_fwd_t<false, false, false>);
+  return f32 ? run(launch_fwd_t<false, true, true>) : p.dtype == KD_BF16 ? run(launch_fwd_t<true, false, true>) : run(launch_fwd_t<false, false, true>);
 }
 
 }  // namespace kd

@@ -10,7 +10,7 @@ struct FwdArgs {
   ItemOrder order_of;
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)
-  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles
+  const uint32_t* words;   // [B][NT][NT][4][128] visibility bits of the PARTIAL tiles, or null
   const int32_t* fwd_cnt;
   const uint16_t* fwd_list;
   const uint8_t* order;   // [B][3][NT]; row 0 = pairs sorted by decreasing list length
@@ -23,6 +23,8 @@ struct FwdArgs {
   int64_t o32_sb, o32_sh, o32_st;
   int o_tma;         // head dims up to 64: O leaves through shared memory and TMA stores
   float* lse;
+  const uint32_t* desc;       // for kernels without words: the tokens' descriptors,
+  const uint32_t* tilebits;   // [B][NT][8][4] class masks of every tile
 #ifdef KD_TEST_DROP_LOAD
   int test_drop_load;   // wait time-out test build: the producer of CTA 0 leaves out its first K tile load
 #endif

@@ -59,8 +59,8 @@ struct FwdWideCfg {
   static_assert(SMEM_ALLOC <= 232448, "shared memory budget");
 };
 
-// kF32: of a float32 call (see attn_fwd.cu)
-template <bool kBf16, bool kF32>
+// kF32: of a float32 call; kWords: the plan has the PARTIAL tiles' bits (see attn_fwd.cu)
+template <bool kBf16, bool kF32, bool kWords>
 __global__ void __launch_bounds__(FwdWideCfg::THREADS, 1)
 attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const FwdArgs a) {
@@ -270,14 +270,18 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t* words = a.words;   // of this thread's query in the item's query tile
     auto fetch_words = [&](uint32_t ent) {
       if ((ent & 0x100u) == 0u) return;
-      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
+      if constexpr (kWords) {
+        const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
+        for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
+      } else {
+        form_words<NW>(a.desc + (size_t)it.x * a.Tpad, a.tilebits + (size_t)it.x * a.NT * 32, (2 * it.z + i) * KD_TILE + row, ent & 0xFF, 0, lane, mk);
+      }
     };
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
-      words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + row;
+      if (kWords) words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + row;
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
       const int only = it.w >> 24;
       const bool mine = only == 0 || only == i + 1;
@@ -433,10 +437,10 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (tid == 0) report_abort(abortf, a.status);
 }
 
-template <bool kBf16, bool kF32>
+template <bool kBf16, bool kF32, bool kWords>
 static int launch_wide_t(long long n_items, const FwdArgs& a, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, cudaStream_t stream) {
   using C = FwdWideCfg;
-  auto kern = attn_fwd_wide_kernel<kBf16, kF32>;
+  auto kern = attn_fwd_wide_kernel<kBf16, kF32, kWords>;
   static SmemOptIn opt_in;
   cudaError_t e = opt_in(kern, C::SMEM_ALLOC);
   if (e != cudaSuccess) return set_error(KD_ERR_DEVICE, "fwd smem attribute: %s", cudaGetErrorString(e));
@@ -459,7 +463,8 @@ static int launch_wide_t(long long n_items, const FwdArgs& a, const CUtensorMap&
 int launch_attn_fwd_wide(long long n_items, const FwdArgs& a, int dtype, const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV,
                          cudaStream_t stream) {
   auto run = [&](auto launch_fn) { return launch_fn(n_items, a, tmQ, tmK, tmV, stream); };
-  return a.o32 != nullptr ? run(launch_wide_t<false, true>) : dtype == KD_BF16 ? run(launch_wide_t<true, false>) : run(launch_wide_t<false, false>);
+  if (a.words == nullptr) return a.o32 != nullptr ? run(launch_wide_t<false, true, false>) : dtype == KD_BF16 ? run(launch_wide_t<true, false, false>) : run(launch_wide_t<false, false, false>);
+  return a.o32 != nullptr ? run(launch_wide_t<false, true, true>) : dtype == KD_BF16 ? run(launch_wide_t<true, false, true>) : run(launch_wide_t<false, false, true>);
 }
 
 }  // namespace kd

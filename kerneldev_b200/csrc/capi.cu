@@ -183,7 +183,7 @@ int kd_plan_layout_get(int32_t B, int32_t T, kd_plan_layout* out) {
   out->off_order = off;    off = up(off + (size_t)B * 3 * NT);
   out->off_stats = off;    off = up(off + (size_t)B * 4 * 4);   // and a counter and the length of each sequence behind the documented words
   out->off_status = off;   off = up(off + 16);
-  off += (size_t)B * NT * NT * KD_WORDS_BYTES;   // visibility words of the tiles (plan_words)
+  off += words_bytes(B, NT);   // visibility words of the tiles
   out->total = off;
   return 0;
 }

@@ -14,6 +14,14 @@ namespace kd {
 // Visibility of a tile as bits: uint32 [4][128], bit k of word [w][q] = query q of the query tile sees key 32 w + k of the key tile. The last part of
 // a plan has room for every tile of a sequence, [B][query tile][key tile], and holds the PARTIAL ones'.
 constexpr size_t KD_WORDS = 4 * KD_TILE, KD_WORDS_BYTES = KD_WORDS * 4;
+// ... if that is no more than KD_WORDS_LIMIT for the batch: a bit for each pair of tokens grows with the square of the length (8 x 16384 tokens 256 MB),
+// whatever the heads and the head dim are, and would take the place of tensors. Beyond it the plan has no such part, and the kernels form the
+// bits of a PARTIAL tile for every head (form_words), in instantiations of their own (kWords false). At the limit: 4 x 16384 tokens, 64 x 4096.
+constexpr size_t KD_WORDS_LIMIT = size_t(128) << 20;
+inline size_t words_bytes(size_t B, size_t NT) {
+  const size_t n = B * NT * NT * KD_WORDS_BYTES;
+  return n <= KD_WORDS_LIMIT ? n : 0;
+}
 
 // Typed pointers into a plan buffer (see kd_plan_layout for the contents).
 struct PlanView {
@@ -31,7 +39,7 @@ struct PlanView {
   uint32_t* done;   // [B] CTAs of the classifier that have finished
   int32_t* len;     // [B] tokens of each sequence that are not padding
   uint32_t* status;
-  uint32_t* words;
+  uint32_t* words;   // null: see KD_WORDS_LIMIT
 };
 
 inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
@@ -53,7 +61,8 @@ inline PlanView make_plan_view(void* plan, const kd_plan_layout& L) {
   v.done = v.stats + 2 * (size_t)L.B;
   v.len = reinterpret_cast<int32_t*>(v.stats + 3 * (size_t)L.B);
   v.status = reinterpret_cast<uint32_t*>(base + L.off_status);
-  v.words = reinterpret_cast<uint32_t*>(base + L.total - (size_t)L.B * L.NT * L.NT * KD_WORDS_BYTES);
+  const size_t words = words_bytes(L.B, L.NT);
+  v.words = words > 0 ? reinterpret_cast<uint32_t*>(base + L.total - words) : nullptr;
   return v;
 }
 

@@ -360,9 +360,9 @@ struct PlanKeyHash {
 
 class PlanCache {
  public:
-  // Plans kept: so many, and so many bytes of device memory (the visibility words of a plan are 16 bits for every 8 x 8 tokens and
-  // sequence: 2 MB at T = 4096), but never fewer than kLeast.
-  static constexpr size_t kSize = 64, kLeast = 4, kBytes = size_t(512) << 20;
+  // Plans kept: so many, and so many bytes of device memory with the newest (the visibility words of a plan are a bit for each pair of tokens, up to
+  // 128 MB), but the newest always.
+  static constexpr size_t kSize = 64, kBytes = size_t(512) << 20;
   PlanPtr find(const PlanKey& key) {
     std::lock_guard<std::mutex> lock(m_);
     auto it = map_.find(key);
@@ -380,7 +380,7 @@ class PlanCache {
     bytes_ += plan->layout.total;
     order_.emplace_back(key, std::move(plan));
     map_[key] = std::prev(order_.end());
-    while (order_.size() > kSize || (bytes_ > kBytes && order_.size() > kLeast)) drop(order_.begin(), evicted);
+    while (order_.size() > kSize || (bytes_ > kBytes && order_.size() > 1)) drop(order_.begin(), evicted);
   }
   std::vector<PlanPtr> values() {
     std::lock_guard<std::mutex> lock(m_);

@@ -128,4 +128,25 @@ __host__ __device__ __forceinline__ uint32_t span_match_query(uint32_t key, uint
   return ((qd & TD_SPAN_QUERY_BITS) == key) ? 1u : 0u;
 }
 
+// The "same span" term: 32 query rows (a lane each, descriptor qd) against W words of keys, adds what they see to m. kd: lane l's W keys, l, 32 + l, ...
+// One round per distinct span among the queries; a ballot gives the keys of that span, 32 at a time. any: whether any of the keys
+// is in a span (warp-uniform).
+#ifdef __CUDACC__
+template <int W>
+__device__ __forceinline__ void add_same_span(uint32_t qd, bool any, const uint32_t* kd, uint32_t* m) {
+  const uint32_t my_key = span_key_of_query(qd);
+  uint32_t todo = any ? __ballot_sync(0xffffffffu, (qd & TD_SIDPOS) != 0u) : 0u;
+  while (todo != 0u) {
+    const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
+    const bool mine = my_key == kq;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd[w]) != 0u);
+      if (mine) m[w] |= hit;
+    }
+    todo &= ~__ballot_sync(0xffffffffu, mine);
+  }
+}
+#endif
+
 }  // namespace kd

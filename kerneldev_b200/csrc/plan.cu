@@ -124,19 +124,7 @@ __device__ __forceinline__ int classify_exact(const uint32_t* desc, const uint32
   for (int r = 0; r < 4; ++r) {
     uint32_t (&mk)[4] = m[r];
     query_row_mask<4>(qd[r], qt * KD_TILE + r * 32 + lane, kt * KD_TILE, pre, ctx, ins, mk);
-    // "same span": one round per distinct span among the 32 queries; a ballot gives the keys of that span
-    const uint32_t my_key = span_key_of_query(qd[r]);
-    uint32_t todo = any_ins != 0u ? __ballot_sync(0xffffffffu, (qd[r] & TD_SIDPOS) != 0u) : 0u;
-    while (todo != 0u) {
-      const uint32_t kq = __shfl_sync(0xffffffffu, my_key, __ffs(todo) - 1);
-      const bool mine = my_key == kq;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const uint32_t hit = __ballot_sync(0xffffffffu, span_match_key(kq, kd[w]) != 0u);
-        if (mine) mk[w] |= hit;
-      }
-      todo &= ~__ballot_sync(0xffffffffu, mine);
-    }
+    add_same_span<4>(qd[r], any_ins != 0u, kd, mk);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       on |= mk[w];
@@ -198,9 +186,10 @@ __global__ void __launch_bounds__(CL_THREADS) classify_kernel(PlanView pv) {
     const int r = e / NT, c = e - r * NT;
     const int qt = is_pair ? 2 * item + r : c, kt = is_pair ? c : item - NP;
     int cls = classify_summary(s_sum[qt], s_sum[kt], qt, kt);
-    if (cls < 0 || (is_pair && cls == KD_TILE_PARTIAL))   // (a pair's CTA writes the bits of its PARTIAL tiles)
+    const bool writes = is_pair && pv.words != nullptr;   // a pair's CTA writes the bits of its PARTIAL tiles, where the plan has room for them
+    if (cls < 0 || (writes && cls == KD_TILE_PARTIAL))
       cls = classify_exact(pv.desc + (size_t)b * pv.Tpad, pv.tilebits + (size_t)b * NT * 32, qt, kt, lane,
-                           is_pair ? pv.words + (((size_t)b * NT + qt) * NT + kt) * KD_WORDS : nullptr);
+                           writes ? pv.words + (((size_t)b * NT + qt) * NT + kt) * KD_WORDS : nullptr);
     if (lane == 0) {
       s_cls[r][c] = static_cast<uint8_t>(cls);
       if (is_pair) pv.cls[((size_t)b * NT + qt) * NT + kt] = static_cast<uint8_t>(cls);

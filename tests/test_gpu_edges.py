@@ -147,6 +147,38 @@ def test_gradients_of_transformed_tensors(T, lens, D, dtype):
     assert bool(((got[0].float() - want[0].float()).abs() <= bound).all())
 
 
+# 1,025 sequences of eight tiles are more than a plan holds the bits of PARTIAL tiles for: the kernels form them, and the results are those of
+# two calls on parts of the batch, whose plans have them. Rules with spans, prefix and [MASKQ] strewn over all tiles; causal
+@pytest.mark.parametrize("rules", [True, False])
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (48, torch.float32), (128, torch.float16), (80, torch.float32)])
+def test_batches_without_mask_bits_in_the_plan(D, dtype, rules):
+    from kerneldev_b200 import _capi, clear_plan_cache, flash_attention
+    B, H, T = 1025, 1, 1000
+    assert _capi.plan_layout(B, T).total < 8 << 20 < 64 << 20 < _capi.plan_layout(513, T).total
+    g = torch.Generator(device=DEV).manual_seed(D)
+    q, k, v, do = (torch.randn((B, H, T, D), generator=g, device=DEV).to(dtype) for _ in range(4))
+    options = {"lens": torch.randint(1, T + 1, (B,), generator=g, device=DEV).clamp_min(T // 2).to(torch.int32)}
+    if rules:   # runs of 1 to 200 tokens: prefix, context or one of four spans; a [MASKQ] in every tile
+        t = torch.arange(T, device=DEV)
+        run = t // torch.randint(1, 201, (B, 1), generator=g, device=DEV)
+        kind = torch.randint(-3, 5, (B, T), generator=g, device=DEV).gather(1, run)
+        options.update(in_span=kind > 0, span_id=torch.where(t % 128 == 77, -1, kind.clamp_min(0)), is_prefix=kind == 0)
+
+    def call(lo, hi, deterministic):
+        x = [y[lo:hi].detach().requires_grad_() for y in (q, k, v)]
+        o, lse = flash_attention(*x, return_lse=True, deterministic=deterministic, **{n: y[lo:hi] for n, y in options.items()})
+        return (o.detach(), lse, *torch.autograd.grad(o, x, do[lo:hi]))
+
+    for deterministic in (False, True):
+        whole, parts = call(0, B, deterministic), zip(call(0, 513, deterministic), call(513, B, deterministic))
+        for n, (got, want) in enumerate(zip(whole, map(torch.cat, parts))):
+            # fused dQ: fp32 sums in no fixed order, then a rounding to the type (2^-8 covers bf16's, of any element)
+            assert torch.equal(got, want) or (n == 2 and not deterministic and float((got - want).norm()) <= 2.0**-8 * float(want.norm()))
+    clear_plan_cache()
+    del q, k, v, do, options, whole, parts, got, want
+    torch.cuda.empty_cache()   # later tests' plans would hold on to segments of this size
+
+
 # More items than SMs, so that CTAs take several one after the other; chunks of heads of equal and (at T = 1280) unequal size. `lens` makes runs of empty items longer than the ring of
 # item headers between items with work (both tile widths; an odd number of query tiles; a last tile of 1 and of 127 tokens)
 @pytest.mark.parametrize("deterministic", [False, True])
