@@ -94,7 +94,7 @@ typedef struct kd_plan_layout {
                                                  pairs, [1] dQ q tiles, [2] dK/dV k tiles */
   size_t off_stats;      /* uint32 [B][2]        number of FULL and of PARTIAL tiles */
   size_t off_status;     /* uint32               device status word (0 = ok); at +8 the address of its host mirror */
-  size_t total;          /* bytes the caller must provide (256-byte aligned base). If B * NT * NT * 2048 is at most 2^27, that
+  size_t total;          /* bytes the caller must provide (256-byte aligned base). If B * NT * NT * 2048 is at most 2^28, that
                             many at the end are uint32 [B][NT][NT][4][128], bit k of word [b][q_tile][k_tile][w][q] =
                             query q of the tile sees key 32 w + k, written for PARTIAL tiles alone. Larger batches have no such
                             part, and the kernels form the bits for every head */

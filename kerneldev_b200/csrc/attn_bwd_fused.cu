@@ -470,10 +470,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
               for (int w = 0; w < 4; ++w) cp_async16(side + (C::SIDE_BITS + w * KD_TILE) * 4 + 16 * lane, src + w * KD_TILE);
             } else {
+              const uint32_t* desc = a.desc + (size_t)b * a.Tpad;
+              const KeyRun<4> keys(desc, a.tilebits + (size_t)b * a.NT * 32, kt, 0, lane);
+              uint32_t qd[4];
+#pragma unroll
+              for (int r = 0; r < 4; ++r) qd[r] = __ldcg(desc + qt * KD_TILE + r * 32 + lane);
 #pragma unroll 1
               for (int r = 0; r < 4; ++r) {   // 32 queries at a time
                 uint32_t mk[4];
-                form_words<4>(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, qt * KD_TILE + r * 32 + lane, kt, 0, lane, mk);
+                keys.words(r < 2 ? (r == 0 ? qd[0] : qd[1]) : (r == 2 ? qd[2] : qd[3]), qt * KD_TILE + r * 32 + lane, mk);
 #pragma unroll
                 for (int w = 0; w < 4; ++w) st_shared_u32(side + (C::SIDE_BITS + w * KD_TILE + r * 32 + lane) * 4, mk[w]);
               }
@@ -935,9 +940,12 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             mk[0] = __ldcg(src);
             mk[1] = __ldcg(src + 32);
           } else {
+            const uint32_t* desc = a.desc + (size_t)b * a.Tpad;
+            const int qi = static_cast<int>(ent & 0xFF) * KD_TILE + w * 64 + lane;
+            const uint32_t qd[2] = {__ldcg(desc + qi), __ldcg(desc + qi + 32)};
+            const KeyRun<1> keys(desc, a.tilebits + (size_t)b * a.NT * 32, kt, wq, lane);
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-              form_words<1>(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, static_cast<int>(ent & 0xFF) * KD_TILE + w * 64 + r * 32 + lane, kt, wq, lane, mk + r);
+            for (int r = 0; r < 2; ++r) keys.words(qd[r], qi + 32 * r, mk + r);
           }
         }
         // LSE and delta of the stage were copied by the producer warp, which the stage's barrier counts and for which the issuing warp waited before the product awaited here

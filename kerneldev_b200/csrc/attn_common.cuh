@@ -27,23 +27,44 @@ namespace kd {
 // score and of a row maximum without keys (-inf both); raised to FLT_MIN it leaves every exponential at 1, as the smaller one would.
 inline float scale_log2_of(float sm_scale) { return std::max(sm_scale * 1.4426950408889634f, FLT_MIN); }
 
-// Words w0 .. w0 + W - 1 of key tile kt for the query rows of a warp, of which this lane has row qi: what a plan's words hold of a PARTIAL tile, for
-// plans without them. desc, tilebits: the sequence's.
+// What a plan's words hold of a PARTIAL tile, for plans without them. KeyRun: of 32 W keys of key tile kt from word w0 on, what words are formed from
+// (w0 is a multiple of W). words(): those of the query rows of a warp, of which this lane has row qi. desc, tilebits: the sequence's.
+template <int W>
+struct KeyRun {
+  uint32_t kd[W], pre[W], ctx[W], ins[W];
+  int j0;
+  __device__ __forceinline__ KeyRun(const uint32_t* desc, const uint32_t* tilebits, int kt, int w0, int lane) : j0(kt * KD_TILE + w0 * 32) {
+    const uint32_t* tb = tilebits + kt * 32 + w0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) kd[w] = __ldcg(desc + j0 + w * 32 + lane);
+    load(pre, tb + 4 * TB_PRE);
+    load(ctx, tb + 4 * TB_CTX);
+    load(ins, tb + 4 * TB_INS);
+  }
+  static __device__ __forceinline__ void load(uint32_t (&m)[W], const uint32_t* src) {
+    if constexpr (W == 4) {
+      const uint4 x = __ldcg(reinterpret_cast<const uint4*>(src));
+      m[0] = x.x; m[1] = x.y; m[2] = x.z; m[3] = x.w;
+    } else if constexpr (W == 2) {
+      const uint2 x = __ldcg(reinterpret_cast<const uint2*>(src));
+      m[0] = x.x; m[1] = x.y;
+    } else {
+      static_assert(W == 1, "1, 2 or 4 words");
+      m[0] = __ldcg(src);
+    }
+  }
+  __device__ __forceinline__ void words(uint32_t qd, int qi, uint32_t* m) const {
+    query_row_mask<W>(qd, qi, j0, pre, ctx, ins, m);
+    uint32_t any = 0u;
+#pragma unroll
+    for (int w = 0; w < W; ++w) any |= ins[w];
+    add_same_span<W>(qd, any != 0u, kd, m);
+  }
+};
 template <int W>
 __device__ __forceinline__ void form_words(const uint32_t* desc, const uint32_t* tilebits, int qi, int kt, int w0, int lane, uint32_t* m) {
   const uint32_t qd = __ldcg(desc + qi);
-  const uint32_t* tb = tilebits + kt * 32 + w0;
-  uint32_t kd[W], pre[W], ctx[W], ins[W], any = 0u;
-#pragma unroll
-  for (int w = 0; w < W; ++w) {
-    kd[w] = __ldcg(desc + kt * KD_TILE + (w0 + w) * 32 + lane);
-    pre[w] = __ldcg(tb + 4 * TB_PRE + w);
-    ctx[w] = __ldcg(tb + 4 * TB_CTX + w);
-    ins[w] = __ldcg(tb + 4 * TB_INS + w);
-    any |= ins[w];
-  }
-  query_row_mask<W>(qd, qi, kt * KD_TILE + w0 * 32, pre, ctx, ins, m);
-  add_same_span<W>(qd, any != 0u, kd, m);
+  KeyRun<W>(desc, tilebits, kt, w0, lane).words(qd, qi, m);
 }
 
 // High words of the two descriptor kinds used here (layout, version, stride byte offset 1024);

@@ -395,14 +395,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     uint32_t mk[NW] = {0u, 0u};
     const uint32_t* words = a.words;   // of this thread's query in the item's query tile
     auto fetch_words = [&](uint32_t ent) {
-      if (entry_class(ent, i) != KD_TILE_PARTIAL) return;
-      if constexpr (kWords) {
-        const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
+      if (!kWords || entry_class(ent, i) != KD_TILE_PARTIAL) return;
+      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
-      } else {
-        form_words<NW>(a.desc + (size_t)it.x * a.Tpad, a.tilebits + (size_t)it.x * a.NT * 32, (2 * it.z + i) * KD_TILE + row, ent & 0xFF, half * NW, lane, mk);
-      }
+      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
     };
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
@@ -433,6 +429,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t ent = ent_next;
       const uint32_t cls = entry_class(ent, i);
       const int sbuf = buf_next;
+      if (!kWords && cls == KD_TILE_PARTIAL)
+        form_words<NW>(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, qi, ent & 0xFF, half * NW, lane, mk);
       const uint32_t tS = lane_base + sbuf * 128 + half * CW;
       if (!(ok = wait(C::B_SFULL + 2 * sbuf + i, (sfull_par >> sbuf) & 1u, W_F_SFULL))) break;
       sfull_par ^= 1u << sbuf;

@@ -268,20 +268,18 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // Visibility of the 128 keys of a PARTIAL tile for this thread's query, of the coming unit (from the plan, see attn_fwd.cu)
     uint32_t mk[NW] = {0u, 0u, 0u, 0u};
     const uint32_t* words = a.words;   // of this thread's query in the item's query tile
+    uint32_t qd_next = 0u;             // without words: its descriptor
     auto fetch_words = [&](uint32_t ent) {
-      if ((ent & 0x100u) == 0u) return;
-      if constexpr (kWords) {
-        const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
+      if (!kWords || (ent & 0x100u) == 0u) return;
+      const uint32_t* src = words + (ent & 0xFF) * static_cast<int>(KD_WORDS);
 #pragma unroll
-        for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
-      } else {
-        form_words<NW>(a.desc + (size_t)it.x * a.Tpad, a.tilebits + (size_t)it.x * a.NT * 32, (2 * it.z + i) * KD_TILE + row, ent & 0xFF, 0, lane, mk);
-      }
+      for (int w = 0; w < NW; ++w) mk[w] = __ldcg(src + w * KD_TILE);
     };
     auto open_item = [&](int k) -> bool {
       if (!next_item(k, it)) return false;
       const int qtile = 2 * it.z + i;
       if (kWords) words = a.words + ((size_t)it.x * a.NT + qtile) * a.NT * KD_WORDS + row;
+      else if (qtile < a.NT) qd_next = __ldcg(a.desc + (size_t)it.x * a.Tpad + qtile * KD_TILE + row);
       n_next = (it.w >> (8 + 8 * i)) & 0xFF;
       const int only = it.w >> 24;
       const bool mine = only == 0 || only == i + 1;
@@ -298,11 +296,16 @@ attn_fwd_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     pdl_wait();   // O and LSE are written from here on
     for (int k = 0; have; ++k) {
       const int b = it.x, h = it.y, n_own = n_next, qi = qi_next;   // qi: token index of this thread's query
+      const uint32_t qd = qd_next;
       float m = -INFINITY, l = 0.f;
 #pragma unroll 1
       for (int u = 0; u < n_own; ++u) {
         const uint32_t ent = ent_next;
         if (u + 1 < n_own) ent_next = list[u + 1];
+        if (!kWords && (ent & 0x100u) != 0u) {   // (here, where no scores are held in registers: behind the exponentials every unit is 9 % longer)
+          const KeyRun<NW> keys(a.desc + (size_t)b * a.Tpad, a.tilebits + (size_t)b * a.NT * 32, ent & 0xFF, 0, lane);
+          keys.words(qd, qi, mk);
+        }
         if (!(ok = wait(C::B_SFULL + i, n_seen & 1, W_F_SFULL))) break;
         tc_fence_after_sync();
         float sc[KD_TILE];

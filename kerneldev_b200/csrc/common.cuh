@@ -14,10 +14,12 @@ namespace kd {
 // Visibility of a tile as bits: uint32 [4][128], bit k of word [w][q] = query q of the query tile sees key 32 w + k of the key tile. The last part of
 // a plan has room for every tile of a sequence, [B][query tile][key tile], and holds the PARTIAL ones'.
 constexpr size_t KD_WORDS = 4 * KD_TILE, KD_WORDS_BYTES = KD_WORDS * 4;
-// ... if that is no more than KD_WORDS_LIMIT for the batch: a bit for each pair of tokens grows with the square of the length (8 x 16384 tokens 256 MB),
+// ... if that is no more than KD_WORDS_LIMIT for the batch: a bit for each pair of tokens grows with the square of the length (64 x 16384 tokens 2 GB),
 // whatever the heads and the head dim are, and would take the place of tensors. Beyond it the plan has no such part, and the kernels form the
-// bits of a PARTIAL tile for every head (form_words), in instantiations of their own (kWords false). At the limit: 4 x 16384 tokens, 64 x 4096.
-constexpr size_t KD_WORDS_LIMIT = size_t(128) << 20;
+// bits of a PARTIAL tile for every head (form_words), in instantiations of their own (kWords false). At the limit: 8 x 16384 tokens, 128 x 4096. Passes beyond it, us, with the bits in a
+// plan of any size and so: hierarchical forward 9 x 4 x 16384 x 64 660 | 705, x 128 905 | 918, with the backward 2,050 | 2,220 and 3,215 | 3,230; deterministic 2,450 | 2,660;
+// causal 2100 x 2 x 1000 x 64 with the backward 3,460 | 3,800.
+constexpr size_t KD_WORDS_LIMIT = size_t(256) << 20;
 inline size_t words_bytes(size_t B, size_t NT) {
   const size_t n = B * NT * NT * KD_WORDS_BYTES;
   return n <= KD_WORDS_LIMIT ? n : 0;

@@ -361,7 +361,7 @@ struct PlanKeyHash {
 class PlanCache {
  public:
   // Plans kept: so many, and so many bytes of device memory with the newest (the visibility words of a plan are a bit for each pair of tokens, up to
-  // 128 MB), but the newest always.
+  // 256 MB), but the newest always.
   static constexpr size_t kSize = 64, kBytes = size_t(512) << 20;
   PlanPtr find(const PlanKey& key) {
     std::lock_guard<std::mutex> lock(m_);

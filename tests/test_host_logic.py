@@ -34,9 +34,9 @@ def test_plan_layout_is_consistent():
             L.off_tilebits, L.off_order, L.off_stats, L.off_status, L.total]
     assert offs == sorted(offs) and all(o % 256 == 0 for o in offs)
     assert L.off_summary - L.off_desc >= 16 * 32 * 128 * 4
-    # masks as bits, 2 KB a tile, where they are at most 128 MB: beyond, a plan grows as its lists do
-    assert _capi.plan_layout(1024, 1000).total - _capi.plan_layout(1024, 1000).off_status == 256 + (128 << 20)
-    for B, T in ((1025, 1000), (65, 4096), (5, 16384), (1024, 16384), (65535, 16384)):
+    # masks as bits, 2 KB a tile, where they are at most 256 MB: beyond, a plan grows as its lists do
+    assert _capi.plan_layout(32, 8100).total - _capi.plan_layout(32, 8100).off_status == 256 + (256 << 20)
+    for B, T in ((2049, 1000), (129, 4096), (33, 8100), (9, 16384), (1024, 16384), (65535, 16384)):
         L = _capi.plan_layout(B, T)
         assert L.total <= B * (4.5 * L.NT ** 2 + 700 * L.NT + 16) + 12 * 256
     L = _capi.plan_layout(1, 200)
