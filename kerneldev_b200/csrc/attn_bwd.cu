@@ -25,6 +25,9 @@
 // that none of them is on the critical path of the other.
 #include <algorithm>
 #include <mutex>
+#ifdef KD_TEST_DROP_LOAD
+#include <stdlib.h>
+#endif
 
 #include "attn_bwd.cuh"
 
@@ -294,7 +297,7 @@ __device__ __forceinline__ void bwd_producer(const CUtensorMap& tmFix0, const CU
       }
       const int st = issued % C::STAGES;
       if (!(ok = wait(sh.ring_empty[st], ((issued / C::STAGES) & 1) ^ 1, W_Q_RINGEMPTY))) break;
-      load_pair(tmRing0, tmRing1, sRing + st * 2 * C::TILE_BYTES, sh.ring_full[st], list[e] & 0xFF, h, b);
+      if (!(test_drops(a, 2) && issued == 0)) load_pair(tmRing0, tmRing1, sRing + st * 2 * C::TILE_BYTES, sh.ring_full[st], list[e] & 0xFF, h, b);
       ++issued;
     }
     it = nx;
@@ -632,6 +635,10 @@ static int launch_bwd_t(const kd_attn_params& p, const kd_attn_f32* f32, const f
   a.plan_ready = ((p.bwd_phases & 3) == 0 || (p.bwd_phases & 1)) ? 1 : 0;
   a.len_ready = p.plan_ready;
   a.signs = signs;
+#ifdef KD_TEST_DROP_LOAD
+  const char* drop = getenv("KD_TEST_DROP_LOAD");
+  a.test_drop = drop != nullptr ? atoi(drop) : 0;
+#endif
   a.after_dq = 0;
   const bool fused = (p.bwd_mode == KD_BWD_FUSED);
   a.grads_f32 = f32 != nullptr;

@@ -41,7 +41,20 @@ struct BwdArgs {
   int len_ready;     // the plan may be read by the delta kernel before the wait for the kernel ahead
   const uint32_t* desc;       // for kernels without words: the tokens' descriptors,
   const uint32_t* tilebits;   // [B][NT][8][4] class masks of every tile
+#ifdef KD_TEST_DROP_LOAD
+  int test_drop;     // wait time-out test build: what the producer of CTA 0 leaves out
+#endif
 };
+
+// Wait time-out test build: whether the producer of this CTA leaves something out, so that waits run out and the CTA has to unwind. 2: the dQ kernel's
+// first pair of K and V; the fused kernel's 3: first Q, 4: second header. Nothing is requested and no bytes are expected, so that nothing is in flight.
+__device__ __forceinline__ bool test_drops(const BwdArgs& a, int what) {
+#ifdef KD_TEST_DROP_LOAD
+  return a.test_drop == what && blockIdx.x == 0;
+#else
+  return false;
+#endif
+}
 
 // How the delta and the conversion kernel (256 threads) divide the rows: a block per ROWS rows of a head, HD / 8 threads to a row, three rows to a
 // thread, all of whose loads are under way together. Both are bound by HBM traffic, and leave the rows of padding alone (delta kernel,

@@ -218,8 +218,10 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // The dQ kernel's end is awaited at this one's end, so that whatever comes next finds both complete (what a successor reads ahead of its
   // own wait is a plan, which no backward writes).
   if (kDq ? fa.after_delta == 0 : a.after_dq == 0) pdl_wait();
-  // The site of this warp's wait that ran out, 0 while none has. There is no wait after it: every role ends at its first, with
-  // its copies drained, and raises the flag where all roles meet. All waits of this kernel are such waits (there is no named
+  // The site of this warp's wait that ran out, 0 while none has. There is no wait or product after it: every role ends at its first, with
+  // its copies drained, and raises the flag where all roles meet. One exception: at HD = 64 the warp that issues S^T takes a header that stays out
+  // for the end of the items and gives the signal that goes behind the last tile (another look at gave_up in its loop costs
+  // the backward 3 %). The compute warps may then form a P^T that is no tile's; nobody reads it, for the other issuers wait for the same header. All waits of this kernel are such waits (there is no named
   // barrier), so a role whose partner has ended waits for its own limit and ends too.
   uint32_t gave_up = 0u;
   // the whole of TMEM is allocated, so the allocation starts at column 0 and the addresses below are constants
@@ -270,6 +272,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       __syncwarp();
       int q_tiles = 0, do_tiles = 0, k_loads = 0, v_loads = 0, k = 0;   // Q / dO / K tiles requested and items published so far
       bool ok = true, pending = false;
+      auto drops = [&](int what, bool here) -> bool { return test_drops(a, what) && here; };
       // decodes item number `idx` of the launch
       auto find_tile = [&](int idx, int4& it) {
         int bh, rank;
@@ -383,7 +386,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           __syncwarp();
         }
-        if (lane == 0) {
+        if (lane == 0 && !drops(4, k == 1)) {
           items[slot] = it;
           mbar_arrive(bar(C::B_ITEMFULL + slot));
         }
@@ -431,7 +434,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           const uint32_t side = s0 + C::SMEM_SIDE + qs * (C::SIDE_WORDS * 4);
           if (lane == 0) {
             st_shared_u32(side + C::SIDE_ENT * 4, this_ent);   // published by the arrival that goes with the load
-            load_tile(&tmQ, sQ + qs * TILE, C::B_QFULL + qs, qt, h, b);
+            if (!drops(3, q_tiles == 0)) load_tile(&tmQ, sQ + qs * TILE, C::B_QFULL + qs, qt, h, b);
           }
           // the scalars of four queries per lane, and a PARTIAL tile's words, copied asynchronously: the barrier counts the lanes' copies
           // (a query at or beyond the sequence length takes the last row's scalars: it sees nothing, so the tile is PARTIAL and the
@@ -609,6 +612,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           int q_stage = 0;
           bool first = false, last = false;   // of tile t - 1
           auto accumulate = [&](int item) -> bool {
+            if (gave_up != 0u) return false;   // (a header stays out)
             if (first && item > 0 && !wait(C::B_ACCFREE + 1, (item - 1) & 1, W_U_ACCFREE)) return false;
 #pragma unroll 1
             for (int w = 0; w < 2; ++w) {

@@ -284,10 +284,8 @@ struct SmemOptIn {
   }
 };
 
-// bounded wait used while unwinding after an abort: lets a TMA copy that is already in flight land
-__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) {
-  for (int spin = 0; spin < (1 << 20) && !mbar_try_wait(bar, parity); ++spin) {
-  }
-}
+// used while unwinding after an abort: lets a TMA copy that is already in flight land, with the limit of the other waits (a number of tests is
+// no limit in time, for the hardware may suspend each of them)
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity) { mbar_wait_short(bar, parity); }
 
 }  // namespace kd

@@ -633,7 +633,7 @@ int launch_attn_fwd(const kd_attn_params& p, const kd_attn_f32* f32, cudaStream_
   a.lse = p.lse;
 #ifdef KD_TEST_DROP_LOAD
   const char* drop = getenv("KD_TEST_DROP_LOAD");
-  a.test_drop_load = (drop != nullptr && atoi(drop) != 0) ? 1 : 0;
+  a.test_drop_load = (drop != nullptr && atoi(drop) == 1) ? 1 : 0;
 #endif
   // head dims below the tile width run on the next wider kernel: TMA zero-fills the missing columns
   if (p.D > 64) return launch_attn_fwd_wide(n_items, a, p.dtype, tmQ, tmK, tmV, stream);

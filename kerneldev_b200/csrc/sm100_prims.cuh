@@ -143,7 +143,7 @@ __device__ __forceinline__ void raise_abort(AbortFlag* abort_flag, uint32_t site
   atomicCAS(const_cast<uint32_t*>(&abort_flag->v), 0u, KD_DEV_TIMEOUT | site);
 }
 // Waits for the phase with the given parity. Returns true when the phase completed, false when the limit ran out. A role
-// ends at its first false, so what the others wait for in turn stays out and each of them ends at its own limit, a few
+// ends at its first false (in the forward and the dQ kernel behind the item in hand, where it is the next header that stays out), so what the others wait for in turn stays out and each of them ends at its own limit, a few
 // limits after the first at the latest. This is inlined dozens of times per kernel, between hot loops that compete for the
 // instruction cache, so it is kept to a few instructions: a 32-bit cycle count, the status word is left to the end of the
 // kernel (with the reporting inlined here the fused backward was 120 KB of code), and another role's time-out is not

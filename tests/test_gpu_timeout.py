@@ -3,7 +3,7 @@ reports it, the Python layer raises, and the next launch on the same device is c
 
 The failure is made in the allowed form only. A TEST BUILD of the library (-DKD_TEST_DROP_LOAD, wait limit
 20 ms instead of 0.4 s) lets the TMA producer of one CTA leave out one K tile load when the environment
-variable KD_TEST_DROP_LOAD=1 is set at launch: no copy is issued and no bytes are expected, so nothing is in
+variable KD_TEST_DROP_LOAD=1 is set at launch (2 to 4: what the backward's producers leave out, see attn_bwd.cuh): no copy is issued and no bytes are expected, so nothing is in
 flight for that stage. The first wait on the starved chain (the S issuer's for the tile, or a softmax warp's for
 the scores) runs out after 20 ms, records
 KD_STATUS_TIMEOUT | wait site in the plan's status word, raises the CTA's abort flag, and every role returns
@@ -70,6 +70,65 @@ def test_wait_timeout_unwinds_reports_and_recovers(shape):
     env = dict(os.environ, KD_LIB_PATH=str(lib))
     env.pop("KD_CHECK_STATUS", None)     # the default, asynchronous reporting is what is under test
     r = subprocess.run([sys.executable, "-c", CHILD % {"root": ROOT, "shape": shape}], env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0 and "unwound and recovered" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+CHILD_BACKWARD = r"""
+import os, sys
+sys.path.insert(0, %(root)r)
+import torch
+from kerneldev_b200 import _capi, flash_attention
+from kerneldev_b200 import plan as plan_module
+assert "waittest" in str(_capi.LIB_PATH)
+dev = torch.device("cuda:0")
+B, H, T, D = %(shape)s
+q, k, v, do = (torch.randn((B, H, T, D), device=dev).to(torch.bfloat16) for _ in range(4))
+x = [t.requires_grad_() for t in (q, k, v)]
+os.environ["KD_TEST_DROP_LOAD"] = "0"
+
+def gradients(deterministic, drop=0):
+    o = flash_attention(*x, causal=True, deterministic=deterministic)
+    os.environ["KD_TEST_DROP_LOAD"] = str(drop)
+    try:
+        return torch.autograd.grad(o, x, do)
+    finally:
+        os.environ["KD_TEST_DROP_LOAD"] = "0"
+
+def same(a, b):   # fused dQ: fp32 sums in no fixed order, then a rounding (2^-8 covers bf16's, of any element)
+    return all(torch.equal(s, t) or float((s.float() - t.float()).norm()) <= 2.0**-8 * float(t.float().norm()) for s, t in zip(a, b))
+
+want = [gradients(det) for det in (False, True)]
+torch.cuda.synchronize()
+(plan,) = plan_module._CACHE.values()
+assert plan.status() == 0
+# what is left out, in which backward, and the kernel whose waits run out
+for drop, deterministic, kernel in ((3, False, 0x400), (4, False, 0x400), (3, True, 0x400), (4, True, 0x400), (2, True, 0x200)):
+    gradients(deterministic, drop)                     # returns: the failure is on the device
+    torch.cuda.synchronize()                           # the kernel ended by itself
+    raw = int(plan._status_host[0]) & 0xFFFFFFFF
+    assert raw & _capi.KD_STATUS_TIMEOUT and (raw & 0xFF00) == kernel, (drop, deterministic, hex(raw))
+    try:
+        gradients(deterministic)                       # the next call on the plan raises, without a sync of its own
+        raise SystemExit("no exception")
+    except RuntimeError as e:
+        assert "timed out" in str(e), str(e)
+    assert plan.status() == 0                          # reported once, then cleared on the device too
+    for det in (False, True):                          # and the device is still usable and correct
+        got = gradients(det)
+        torch.cuda.synchronize()
+        assert plan.status() == 0 and same(got, want[det]), (drop, deterministic, det)
+print("unwound and recovered")
+"""
+
+
+# the fused backward with and without its dQ, and the dQ kernel, at both tile widths; CTAs of one item (6 key tiles) and of several (320)
+@pytest.mark.parametrize("shape", [(1, 2, 384, 64), (2, 40, 512, 64), (1, 2, 384, 128), (2, 40, 512, 128)])
+def test_wait_timeout_in_the_backward(shape):
+    from kerneldev_b200.build import build
+    lib = build(name="waittest", extra_flags=WAITTEST_FLAGS)
+    env = dict(os.environ, KD_LIB_PATH=str(lib))
+    env.pop("KD_CHECK_STATUS", None)
+    r = subprocess.run([sys.executable, "-c", CHILD_BACKWARD % {"root": ROOT, "shape": shape}], env=env, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "unwound and recovered" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
 
 
