@@ -168,12 +168,14 @@ struct Plan {
   Tensor buf;
   struct Mirror {                  // the status word's copy in host memory
     StatusWords::Word word = status_words().take();
+    volatile uint32_t* const at = reinterpret_cast<volatile uint32_t*>(word.first.data_ptr<int32_t>() + word.second);
     ~Mirror() { status_words().give_back(std::move(word)); }
-  } mirror;
-  volatile uint32_t* host_word;
+  };
+  std::shared_ptr<Mirror> mirror = std::make_shared<Mirror>();   // (the cache looks at those of plans that it has dropped)
+  volatile uint32_t* host_word = mirror->at;
   // the status word and its mirror as tensors: views cost more than a launch, and only reports and tests want them
   Tensor status_dev() const { return buf.narrow(0, static_cast<int64_t>(layout.off_status), 4).view(at::kInt); }
-  Tensor status_host() const { return mirror.word.first.narrow(0, mirror.word.second, 1); }
+  Tensor status_host() const { return mirror->word.first.narrow(0, mirror->word.second, 1); }
   // Memory of the caller's metadata, then of its converted copies, alive as long as the plan is cached. (Not the tensors: with a Python object one
   // counts as held by somebody for good.)
   std::vector<c10::Storage> keep;
@@ -214,7 +216,6 @@ struct Plan {
     }
     meta.causal = causal;
     meta.rules = rules;
-    host_word = reinterpret_cast<volatile uint32_t*>(mirror.word.first.data_ptr<int32_t>() + mirror.word.second);
     meta.status_mirror = const_cast<uint32_t*>(host_word);
     c10::cuda::CUDAGuard guard(dev);
     check(lib.classify(&meta, buf.data_ptr(), built_on.stream()));
@@ -272,6 +273,10 @@ struct Plan {
     // both copies are cleared, so that one event is reported once and later launches start clean
     status_dev().zero_();
     *host_word = 0;
+    raise_status(s);
+  }
+
+  [[noreturn]] static void raise_status(uint32_t s) {
     TORCH_CHECK_VALUE((s & kStatusSpanRange) == 0, "span_id values must fit in 24 signed bits (|span_id| < 2**23)");
     char hex[16], site[16];
     snprintf(hex, sizeof hex, "0x%08x", s);
@@ -370,17 +375,10 @@ class PlanCache {
     order_.splice(order_.end(), order_, it->second);
     return it->second->second;
   }
+  // Raises if a launch of a plan that an earlier insertion has dropped, or this one drops, has reported a status.
   void insert(const PlanKey& key, PlanPtr plan) {
     std::vector<PlanPtr> evicted;   // destroyed after the lock is released
-    std::lock_guard<std::mutex> lock(m_);
-    if (map_.count(key)) return;
-    // Plans that no call can ask for any more go back to the allocator at once: a training step's plan has the memory of the last
-    // one's, and not a new block until the cache is full (a first pass at 3 x 1357 tokens 175 us, 158 with this).
-    for (auto it = order_.begin(); it != order_.end();) it = it->second->orphaned() ? drop(it, evicted) : std::next(it);
-    bytes_ += plan->layout.total;
-    order_.emplace_back(key, std::move(plan));
-    map_[key] = std::prev(order_.end());
-    while (order_.size() > kSize || (bytes_ > kBytes && order_.size() > 1)) drop(order_.begin(), evicted);
+    if (const uint32_t s = add(key, std::move(plan), evicted)) Plan::raise_status(s);
   }
   std::vector<PlanPtr> values() {
     std::lock_guard<std::mutex> lock(m_);
@@ -398,6 +396,29 @@ class PlanCache {
 
  private:
   using Entries = std::list<std::pair<PlanKey, PlanPtr>>;
+  uint32_t add(const PlanKey& key, PlanPtr plan, std::vector<PlanPtr>& evicted) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (map_.count(key)) return 0;
+    // Plans that no call can ask for any more go back to the allocator at once: a training step's plan has the memory of the last
+    // one's, and not a new block until the cache is full (a first pass at 3 x 1357 tokens 175 us, 158 with this).
+    for (auto it = order_.begin(); it != order_.end();) it = it->second->orphaned() ? drop(it, evicted) : std::next(it);
+    bytes_ += plan->layout.total;
+    order_.emplace_back(key, std::move(plan));
+    map_[key] = std::prev(order_.end());
+    while (order_.size() > kSize || (bytes_ > kBytes && order_.size() > 1)) drop(order_.begin(), evicted);
+    // Their launches may still run, and no call looks at these plans any more: the last backward of a step would report to nobody.
+    for (const PlanPtr& p : evicted) dropped_.push_back(p->mirror);
+    while (dropped_.size() > kSize) dropped_.pop_front();
+    for (auto it = dropped_.begin(); it != dropped_.end(); ++it) {
+      volatile uint32_t* const word = (*it)->at;
+      const uint32_t s = *word;
+      if (s == 0) continue;
+      *word = 0;
+      dropped_.erase(it);
+      return s;
+    }
+    return 0;
+  }
   Entries::iterator drop(Entries::iterator it, std::vector<PlanPtr>& gone) {
     bytes_ -= it->second->layout.total;
     gone.push_back(std::move(it->second));
@@ -407,6 +428,7 @@ class PlanCache {
   std::mutex m_;
   size_t bytes_ = 0;   // of the plans in the cache
   Entries order_;   // least recently used first
+  std::deque<std::shared_ptr<Plan::Mirror>> dropped_;   // status words of the last kSize plans that left for others
   std::unordered_map<PlanKey, Entries::iterator, PlanKeyHash> map_;
 };
 PlanCache& cache() {

@@ -17,7 +17,9 @@ of them from Python.
 Device status. Kernels report problems (a bounded wait that ran out, a span id out of range) in the
 plan's status word and, in the same breath, in a pinned host mirror whose address the plan carries; the
 next call that uses the plan (or ``poll()``) looks at the mirror without synchronising and raises, so a
-failed launch surfaces one call later at the latest -- normally at the backward of the same step. A
+failed launch surfaces one call later at the latest -- normally at the backward of the same step. The
+words of the last 64 plans that left the cache for newer ones are looked at whenever a plan is made for it: what the
+last launch of a step reports surfaces with a later step's new metadata. A
 launch that succeeds costs no copy. ``KD_CHECK_STATUS=1`` makes every call synchronise and check at once.
 """
 from __future__ import annotations

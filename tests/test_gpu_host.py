@@ -302,6 +302,32 @@ def test_a_live_plan_keeps_its_status_word():
     assert len({p._status_host.data_ptr() for p in live + [plan]}) == 1101
 
 
+@pytest.mark.parametrize("late", [False, True])
+def test_a_plan_that_leaves_the_cache_still_reports(late):
+    """What the last launch of a step reports, before its plan makes room for the next step's or behind that (the host is ahead of the
+    device), is raised once, by a call with new metadata, which then works."""
+    from kerneldev_b200 import _capi, clear_plan_cache
+    from kerneldev_b200.plan import _CACHE, get_plan
+    new = lambda: torch.tensor([100], dtype=torch.int32, device=DEV)
+    plan_of = lambda lens: get_plan(1, 128, DEV, lens=lens)
+    clear_plan_cache()
+    lens = new()
+    words = [plan_of(lens)._status_host]
+    lens, held = new(), [new()]   # (all at once: no two have the same memory)
+    if late:
+        plan_of(held[0])   # the first plan goes here
+    words[0].fill_(_capi.KD_STATUS_TIMEOUT | 0x104)
+    lens = new()
+    with pytest.raises(RuntimeError, match="timed out.*0x104"):
+        plan_of(lens)
+    assert int(words[0]) == 0 and len(_CACHE) == 1 + late
+    plan = plan_of(lens)
+    held.append(new())
+    plan_of(held[-1])
+    assert plan_of(lens) is plan and len(_CACHE) == 2 + late
+    clear_plan_cache()
+
+
 def test_one_row_may_have_more_embeddings_than_tokens():
     from kerneldev_b200 import cocktail_scores
     T, more, C = 130, 37, 24
