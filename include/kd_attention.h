@@ -159,7 +159,7 @@ int kd_attn_fwd(const kd_attn_params* p, void* stream);
 int kd_attn_bwd(const kd_attn_params* p, void* stream);
 
 /* kd_attn_bwd (KD_BWD_FUSED, all phases) on Q and K that kd_hadamard has transformed with these signs: dQ and dK come back for the tensors
- * they were made from. As kd_attn_bwd and kd_hadamard(inverse = 1) on dQ and dK, with dQ rounded once and two passes over memory fewer.
+ * they were made from. As kd_attn_bwd and kd_hadamard(inverse = 1) on dQ and dK, with dQ rounded once, and written and read once less.
  * D 16, 32, 64 or 128; signs: (H,D) contiguous, 16-byte aligned. */
 int kd_attn_bwd_hadamard(const kd_attn_params* p, const float* signs, void* stream);
 

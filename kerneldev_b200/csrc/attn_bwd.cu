@@ -16,8 +16,8 @@
 // tensor-memory, barrier and special-function latencies. A unit owns TMEM buffer u % NBUF
 // (64 columns of scores + 64 of dP) and the issuers run NBUF units ahead, so that a warpgroup
 // finishing unit u finds its next unit's scores already in TMEM:
-//   M1(u): S_u, dP_u  (smem x smem -> TMEM, N = 64)      compute(u): P_u / dS_u -> TMEM (16 bit)
-//   M2(u): accumulators += (P_u | dS_u) x smem operand   (A from TMEM);   then M1(u + NBUF)
+//   M1(u): S_u, dP_u  (smem x smem -> TMEM, N = 64)      compute(u): dS_u -> TMEM (16 bit)
+//   M2(u): dQ += dS_u K  (A from TMEM);   then M1(u + NBUF)
 // Each warpgroup writes its 16 packed columns over the start of the 32 fp32 columns it has just
 // read, so the 16-bit operand of a unit sits at columns [0,16) and [32,48) of the buffer.
 // The tensor pipe executes in issue order, so M1(u + NBUF) may overwrite the buffer M2(u) read.

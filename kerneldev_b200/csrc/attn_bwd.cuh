@@ -6,7 +6,7 @@ namespace kd {
 
 struct BwdArgs {
   int B, H, T, NT, NP, Tpad;
-  ItemOrder order_of;   // of the two-kernel backward's items
+  ItemOrder order_of;   // of the dQ kernel's items
   int after_dq;      // fused kernel without dQ: the dQ kernel of the same call is the kernel before this one on the stream
   int d_real;        // head dim of the tensors (a multiple of 16, <= HD); TMA zero-fills the tile columns beyond it
   float scale_log2;  // sm_scale * log2(e)

@@ -16,11 +16,12 @@
 // the scratch to the output dtype afterwards. The delta kernel, which runs first anyway, zeroes the
 // scratch.
 //
-// What bounds it. Per tile at HD = 64 (cycles of an SM): products 1,540, exponentials 1,024, shared
-// memory 2,450 of its 128 bytes a cycle (1,408 of them the products' operands), instruction issue 1,350 of each
-// scheduler; a tile takes 2,500 with full lists, so it is shared memory's rate that is left (3,000 when long waits and late products
-// came on top), and 2,700-2,800 with lists of 4 to 9 tiles. At HD = 128 a tile takes 3,900, and 3,300 without the additions of
-// dQ, for which the L2 needs 3,200 from all SMs at once.
+// What bounds it. Counters, cycles of an SM per tile: at HD = 64 (causal 8 x 16 x 2048, 2,790 a tile) 1,273 wavefronts of the threads in shared
+// memory and 1,408 of the products' operands, tensor pipe 1,280, exponentials 1,030, instruction issue 1,280 of each scheduler; at HD = 128
+// (hierarchical 1 x 32 x 8192, 4,290) 1,491 and 2,304, 2,560, 1,030, 1,330. So shared memory is the most loaded, and what is taken off it
+// comes out of the time in part: timing-only builds that read the A operands of S^T and dP^T from TMEM (256 wavefronts of a tile less, 512 at HD
+// = 128) took 3.5 % off the backward of causal 8 x 16 x 2048 x 64 and 6.5 % x 128, with dK's (384, 768) 5.5 % and 7.5 %: four to six tenths of
+// those cycles. The rest is latency of the chain from scores to dS and hand-overs. Without the additions of dQ a tile at HD = 128 took 3,300 cycles for 3,900.
 //  * Shared memory is kept free by the layout of the compute warps' registers: they read S^T and dP^T from TMEM in the
 //    16x256b shape, in which a thread owns four key rows and a quarter of the columns, as in an mma fragment, so that a
 //    warp needs LSE and delta of a column once and not 32 times; P^T goes back in the 16x128b shape and dS^T leaves
@@ -65,7 +66,7 @@
 // thread, sixteen compute warps and heads per CTA (HD = 64) and the two-kernel form (HD = 128):
 //   bf16 B16 H16 T4096 D64 hierarchical 1291 -> 1175-1230    bf16 B8 H16 T2048 D64 causal 338 -> 284
 //   bf16 B8 H16 T2048 D128 causal 644 -> 415                 fp16 B4 H32 T8192 D128 hierarchical 3944 -> 2420
-// The first is 890-950 now, the second 250-270.
+// The first is 890-950 now, the second 230-280 (boxes differ, and the power limit's state).
 #include <algorithm>
 #include <type_traits>
 
@@ -794,7 +795,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // Iteration t forms dS^T of tile t - 1 and, LAG blocks behind it in the same instruction stream, P^T of tile t. Each product is issued as
       // soon as its predecessor has been loaded; dP^T(t) then has the P^T blocks behind the dS^T blocks' end, the masks and the stores
       // to be formed under, S^T(t + 1) the first LAG blocks of the next iteration. (Side by side from one barrier for both, every
-      // iteration waits some 250 cycles for its products. Backward us, lag 0 / 2 / 5 / 6 / 7 / 8: causal 8 x 16 x 1000 x 64 93.6 / 91.7 / 90.6 / 89.2 / 89.6 / 91.7,
+      // iteration waits some 250 cycles for its products. Backward us on one box, lag 0 / 2 / 5 / 6 / 7 / 8: causal 8 x 16 x 1000 x 64 93.6 / 91.7 / 90.6 / 89.2 / 89.6 / 91.7,
       // 8 x 16 x 2048 280 / 290 / 281 / 273 / 276 / 281, hierarchical 8 x 16 x 2048 x 64 139.4 / 139.3 / 138.5 / 135.8 / 136.8 / 140.7, 16 x 16 x 4096 x 64 948 / 981 /
       // 966 / 930 / 943 / 983. The exponentials and the multiply-adds of one warp overlap less, so both want to be kept.) The two warpgroups
       // have barriers of their own and drift apart, so that one does arithmetic while the other waits, loads or stores:

@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(256) hadamard_kernel(const uint16_t* x, int64_
 // The last pass of a fused backward on transformed Q and K: dQ from the fp32 scratch, scaled, and dK, both times the transform's transpose. One
 // launch in the place of the conversion to 16 bits and two transforms (fp16 4 x 32 x 8192 x 128 with a fifth of padding 172 + 2 x 128 us -> 307, bf16
 // 8 x 16 x 2048 x 64 18 + 2 x 20 -> 32), which write and read dQ once more, and dQ is rounded once. Rows of padding: dQ is 0 and its scratch not
-// read; dK is 0 already. By the bytes it would take 175 us (hadamard_kernel: 82 of 128): shuffles and butterflies are half of its issue slots. Pieces of
-// 4 floats, so that a load takes whole sectors: 317; five or six blocks to an SM 325 and 394 (registers).
+// read; dK is 0 already. By the bytes it would take 175 us (hadamard_kernel: 82 of 128): the pipe that loads, stores and shuffles share is busy for 81 % of the
+// cycles (73 %), issue slots for 61 % (74 %). Pieces of 4 floats, so that a load takes whole sectors: 317; five or six blocks to an SM 325 and 394 (registers).
 // blockIdx.x: 2 * (block of rows) + (0: dQ, 1: dK).
 struct GradTransformArgs {
   const float* acc;
