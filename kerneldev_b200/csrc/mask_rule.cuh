@@ -89,7 +89,8 @@ __host__ __device__ __forceinline__ void query_row_mask(uint32_t qd, int i, int 
 }
 
 // Key row with descriptor kd at index j against W words of query-side masks of the queries
-// i0 .. i0 + 32 W - 1: every term of the rule except "same span".
+// i0 .. i0 + 32 W - 1: every term of the rule except "same span". (For users of the plan's query-side masks: the kernels
+// here mask with words of query rows in either order of the tiles.)
 template <int W>
 __host__ __device__ __forceinline__ void key_row_mask(uint32_t kdesc, int j, int i0, const uint32_t* q_sees_pre,
                                                       const uint32_t* q_sees_ctx, const uint32_t* q_sees_ins,
@@ -119,7 +120,7 @@ __host__ __device__ __forceinline__ uint32_t span_key_of_query(uint32_t qd) {
 __host__ __device__ __forceinline__ uint32_t span_match_key(uint32_t key, uint32_t kdesc) {
   return ((kdesc & TD_SPAN_KEY_BITS) == key) ? 1u : 0u;
 }
-// key of a KEY row matched against QUERY descriptors: query needs the rule armed and the same id
+// key of a KEY row matched against QUERY descriptors (beside key_row_mask): query needs the rule armed and the same id
 constexpr uint32_t TD_SPAN_QUERY_BITS = 0xFFFFFF00u | TD_SIDPOS;
 __host__ __device__ __forceinline__ uint32_t span_key_of_key(uint32_t kdesc) {
   return (kdesc & TD_INS) ? ((kdesc & 0xFFFFFF00u) | TD_SIDPOS) : 0x00000001u;
